@@ -5,15 +5,18 @@
 //             dz_j = g_row * (exp(z_j - lse) - (1 - alpha) * [j == t] - alpha / V).
 // As framework operations this is a log-softmax, a gather, a mean and their backward passes over an array of
 // [tokens, vocabulary] f32 (8.6 GB at 32768 x 65536): six passes and three arrays of that size.  Here the forward kernel
-// reads the logits once from HBM (one CTA per row; the second read of the row, for the sum of exponentials, comes from
-// L2) and the backward kernel reads them once more and writes dz: HBM-bound, 4 + 8 bytes per logit.
+// reads the logits once (one CTA per row, every thread with a running maximum of its own) and the backward kernel reads them
+// once more and writes dz: HBM-bound, 4 + 8 bytes per logit.
 #include "common.cuh"
 
 namespace pb {
 namespace {
 
-constexpr int kLossThreads = 256;
+// Threads per row: 256, six rows at a time on an SM (40 registers); 1024 where there are too few rows for that (wide_rows).
+constexpr int kLossThreads = 256, kWideThreads = 1024;
+constexpr int kLoads = 4;             // 16-byte loads that a thread has in flight
 
+template <int THREADS>
 __device__ __forceinline__ float block_reduce(float v, bool take_max, float* red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -23,50 +26,81 @@ __device__ __forceinline__ float block_reduce(float v, bool take_max, float* red
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   float r = red[0];
-  for (int w = 1; w < kLossThreads / 32; ++w) r = take_max ? fmaxf(r, red[w]) : r + red[w];
+  for (int w = 1; w < THREADS / 32; ++w) r = take_max ? fmaxf(r, red[w]) : r + red[w];
   __syncthreads();
   return r;
 }
 
-// row_loss[r] = weight[r] * loss_row, lse[r] kept for the backward pass.  One CTA per row: the row's maximum and sum first,
-// then the sum of exp(z - max) on a second read that comes from L2 (a row of 65536 logits is 256 KB).
-__global__ void __launch_bounds__(kLossThreads) smoothed_xent_fwd_kernel(const float* logits, const int64_t* target, const float* weight,
-                                                                        float* row_loss, float* lse, int64_t vocab, float alpha) {
-  __shared__ float red[kLossThreads / 32];
-  const int64_t row = blockIdx.x;
-  const float* z = logits + row * vocab;
-  float m = -INFINITY, zs = 0.0f;
-  for (int64_t j = (int64_t)threadIdx.x * 4; j < vocab; j += kLossThreads * 4) {
-    const float4 v = *reinterpret_cast<const float4*>(z + j);
-    m = fmaxf(fmaxf(m, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
+// A thread's maximum, sum of exp(z - maximum) and sum of z.  While the maximum is -inf (nothing but -inf seen) the
+// exponentials are taken from 0, so that -inf - -inf does not make a NaN of a logit that only weighs nothing.
+struct RowTerms {
+  float m = -INFINITY, s = 0.0f, zs = 0.0f;
+  __device__ __forceinline__ void raise(float top) {
+    const float m2 = fmaxf(m, top);
+    if (m2 > m) {
+      s *= expf(m - m2);               // m = -inf: 0 * 0
+      m = m2;
+    }
+  }
+  __device__ __forceinline__ void add(const float4& v) {
+    const float base = m == -INFINITY ? 0.0f : m;
+    s += (expf(v.x - base) + expf(v.y - base)) + (expf(v.z - base) + expf(v.w - base));
     zs += (v.x + v.y) + (v.z + v.w);
   }
-  m = block_reduce(m, true, red);
-  zs = block_reduce(zs, false, red);
-  float s = 0.0f;
-  for (int64_t j = (int64_t)threadIdx.x * 4; j < vocab; j += kLossThreads * 4) {
-    const float4 v = *reinterpret_cast<const float4*>(z + j);
-    s += (expf(v.x - m) + expf(v.y - m)) + (expf(v.z - m) + expf(v.w - m));
+};
+__device__ __forceinline__ float top4(const float4& v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); }
+
+// row_loss[r] = weight[r] * loss_row, lse[r] kept for the backward pass.  One CTA per row, one read of it: a thread keeps a
+// running maximum and rescales its sum of exponentials where the maximum rises; the threads' terms meet at the end.
+// Bound by the 4 bytes per logit.  The form before read the row twice, maximum and sum of z first and the exponentials on
+// a second read from L2, with one 16-byte load of a thread in flight:
+// 4096 x 65536 logits 0.316 ms, now 0.17 ms (6.3 TB/s; the loss and its gradient 0.684 -> 0.537 ms).
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) smoothed_xent_fwd_kernel(const float* logits, const int64_t* target, const float* weight,
+                                                                   float* row_loss, float* lse, int64_t vocab, float alpha) {
+  __shared__ float red[THREADS / 32];
+  const int64_t row = blockIdx.x;
+  const float4* z4 = reinterpret_cast<const float4*>(logits + row * vocab);
+  const int64_t quads = vocab / 4, whole = quads - quads % (THREADS * kLoads);
+  RowTerms t;
+  for (int64_t j = threadIdx.x; j < whole; j += THREADS * kLoads) {
+    float4 v[kLoads];
+#pragma unroll
+    for (int k = 0; k < kLoads; ++k) v[k] = __ldg(z4 + j + k * THREADS);
+    float top = top4(v[0]);
+#pragma unroll
+    for (int k = 1; k < kLoads; ++k) top = fmaxf(top, top4(v[k]));
+    t.raise(top);
+#pragma unroll
+    for (int k = 0; k < kLoads; ++k) t.add(v[k]);
   }
-  s = block_reduce(s, false, red);
+  for (int64_t j = whole + threadIdx.x; j < quads; j += THREADS) {
+    const float4 v = __ldg(z4 + j);
+    t.raise(top4(v));
+    t.add(v);
+  }
+  const float m = block_reduce<THREADS>(t.m, true, red);
+  const float s = block_reduce<THREADS>(t.s * expf(t.m - m), false, red);       // a row of -inf only: NaN, as its softmax is
+  const float zs = block_reduce<THREADS>(t.zs, false, red);
   if (threadIdx.x == 0) {
     const float l = m + logf(s);
     lse[row] = l;
-    row_loss[row] = weight[row] * (l - (1.0f - alpha) * z[target[row]] - alpha * (zs / (float)vocab));
+    row_loss[row] = weight[row] * (l - (1.0f - alpha) * logits[row * vocab + target[row]] - alpha * (zs / (float)vocab));
   }
 }
 
 // dz[r][j] = g[r] * (exp(z - lse) - (1 - alpha) * [j == t] - alpha / V), g[r] = upstream * weight[r] / denominator
-__global__ void __launch_bounds__(kLossThreads) smoothed_xent_bwd_kernel(const float* logits, const int64_t* target, const float* weight,
-                                                                        const float* lse, const float* upstream, float inv_denominator,
-                                                                        float* dlogits, int64_t vocab, float alpha) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) smoothed_xent_bwd_kernel(const float* logits, const int64_t* target, const float* weight,
+                                                                   const float* lse, const float* upstream, float inv_denominator,
+                                                                   float* dlogits, int64_t vocab, float alpha) {
   const int64_t row = blockIdx.x;
   const float* z = logits + row * vocab;
   float* dz = dlogits + row * vocab;
   const float g = upstream[0] * weight[row] * inv_denominator, l = lse[row];
   const int64_t t = target[row];
   const float smooth = alpha / (float)vocab;
-  for (int64_t j = (int64_t)threadIdx.x * 4; j < vocab; j += kLossThreads * 4) {
+  for (int64_t j = (int64_t)threadIdx.x * 4; j < vocab; j += THREADS * 4) {
     const float4 v = *reinterpret_cast<const float4*>(z + j);
     float4 d = make_float4(expf(v.x - l) - smooth, expf(v.y - l) - smooth, expf(v.z - l) - smooth, expf(v.w - l) - smooth);
     if (t >= j && t < j + 4) {
@@ -76,6 +110,9 @@ __global__ void __launch_bounds__(kLossThreads) smoothed_xent_bwd_kernel(const f
     *reinterpret_cast<float4*>(dz + j) = make_float4(g * d.x, g * d.y, g * d.z, g * d.w);
   }
 }
+
+// Fewer rows than the SMs hold at 256 threads each: four times the threads per row, where a row has loads for them.
+bool wide_rows(int64_t rows, int64_t vocab) { return rows < (int64_t)sm_count() * 6 && vocab >= kWideThreads * 4; }
 
 }  // namespace
 }  // namespace pb
@@ -88,7 +125,11 @@ extern "C" int pb_smoothed_xent(const float* logits, const int64_t* target, cons
   if (rows <= 0 || vocab <= 0 || vocab % 4 != 0 || rows > 0x7fffffffll)
     return fail(PB_ERR_BAD_SHAPE, "pb_smoothed_xent: rows=%lld vocab=%lld (vocab must be a multiple of 4)", (long long)rows, (long long)vocab);
   if (reinterpret_cast<uintptr_t>(logits) & 15) return fail(PB_ERR_MISALIGNED, "pb_smoothed_xent: logits must be 16-byte aligned");
-  smoothed_xent_fwd_kernel<<<(unsigned)rows, kLossThreads, 0, static_cast<cudaStream_t>(stream)>>>(logits, target, weight, row_loss, lse, vocab, alpha);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (wide_rows(rows, vocab))
+    smoothed_xent_fwd_kernel<kWideThreads><<<(unsigned)rows, kWideThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
+  else
+    smoothed_xent_fwd_kernel<kLossThreads><<<(unsigned)rows, kLossThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
   PB_LAUNCH_CHECK("smoothed_xent_fwd_kernel");
   return PB_OK;
 }
@@ -100,8 +141,11 @@ extern "C" int pb_smoothed_xent_bwd(const float* logits, const int64_t* target, 
     return fail(PB_ERR_BAD_SHAPE, "pb_smoothed_xent_bwd: rows=%lld vocab=%lld denominator=%g", (long long)rows, (long long)vocab, (double)denominator);
   if ((reinterpret_cast<uintptr_t>(logits) & 15) || (reinterpret_cast<uintptr_t>(dlogits) & 15))
     return fail(PB_ERR_MISALIGNED, "pb_smoothed_xent_bwd: logits and dlogits must be 16-byte aligned");
-  smoothed_xent_bwd_kernel<<<(unsigned)rows, kLossThreads, 0, static_cast<cudaStream_t>(stream)>>>(logits, target, weight, lse, upstream,
-                                                                                                1.0f / denominator, dlogits, vocab, alpha);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (wide_rows(rows, vocab))
+    smoothed_xent_bwd_kernel<kWideThreads><<<(unsigned)rows, kWideThreads, 0, st>>>(logits, target, weight, lse, upstream, 1.0f / denominator, dlogits, vocab, alpha);
+  else
+    smoothed_xent_bwd_kernel<kLossThreads><<<(unsigned)rows, kLossThreads, 0, st>>>(logits, target, weight, lse, upstream, 1.0f / denominator, dlogits, vocab, alpha);
   PB_LAUNCH_CHECK("smoothed_xent_bwd_kernel");
   return PB_OK;
 }
