@@ -1074,29 +1074,45 @@ __device__ __forceinline__ int64_t flat_block(const PrepParams& q, int r, int kb
   return q.transposed ? (int64_t)kb * (q.rows / q.grid_a) + r / q.grid_a : (int64_t)(r / q.grid_a) * q.KB + kb;
 }
 
-__global__ void __launch_bounds__(256) gemm_prep_kernel(PrepParams q) {
-  const int atoms_per_kg = q.tiles * q.atoms_per_tile;
-  const int64_t n_sf = (int64_t)q.KG * atoms_per_kg * 512;
+// Both operands in one launch: blocks [0, first) work on q[0], the others on q[1] (a call that needs one operand gives it all).
+// Bound by launch and memory latency, not bytes: a thread writes the four bytes of one row and four k-blocks at a time.
+// A launch per operand and a thread per byte: 22 us of a 2048 x 2048 training step on 16384 tokens (six launches), now 11.7 (three).
+struct PrepPair {
+  PrepParams q[2];
+  unsigned first;
+};
+
+__global__ void __launch_bounds__(256) gemm_prep_kernel(const __grid_constant__ PrepPair pair) {
+  const bool second = blockIdx.x >= pair.first;
+  const PrepParams& q = pair.q[second];
+  const unsigned block = second ? blockIdx.x - pair.first : blockIdx.x, blocks = second ? gridDim.x - pair.first : pair.first;
+  const uint32_t atoms_per_kg = (uint32_t)(q.tiles * q.atoms_per_tile);
+  const int64_t n_sf = (int64_t)q.KG * atoms_per_kg * 128;      // words of four bytes
   const int64_t n_f = (int64_t)q.rows_pad * q.nchunks;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_sf + n_f; i += stride) {
+  const int64_t stride = (int64_t)blocks * blockDim.x;
+  for (int64_t i = (int64_t)block * blockDim.x + threadIdx.x; i < n_sf + n_f; i += stride) {
     if (i < n_sf) {
-      // i enumerates the destination bytes in order: kg, tile, atom, then the 512 bytes of the atom
-      const int within = (int)(i & 511);
-      const int64_t atom_global = i >> 9;
-      const int kg = (int)(atom_global / atoms_per_kg), rem = (int)(atom_global % atoms_per_kg);
-      const int tile = rem / q.atoms_per_tile, atom = rem % q.atoms_per_tile;
-      const int local = atom * 128 + ((within >> 2) & 3) * 32 + (within >> 4);
-      const int r = tile * q.tile_rows + local;
-      const int kb = kg * 4 + (within & 3);
-      uint8_t v = 0;
-      if (local < q.tile_rows && r < q.rows && kb < q.KB) v = q.sc8[flat_block(q, r, kb)];
-      q.sf[i] = v;
+      // i enumerates the destination words in order: kg, tile, atom, then the 128 words of the atom
+      const int within = (int)(i & 127);
+      const uint32_t atom_global = (uint32_t)(i >> 7);
+      const uint32_t kg = atom_global / atoms_per_kg, rem = atom_global - kg * atoms_per_kg;
+      const uint32_t tile = rem / (uint32_t)q.atoms_per_tile, atom = rem - tile * (uint32_t)q.atoms_per_tile;
+      const int local = (int)atom * 128 + (within & 3) * 32 + (within >> 2);
+      const int r = (int)tile * q.tile_rows + local;
+      uint32_t v = 0;
+      if (local < q.tile_rows && r < q.rows) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int kb = (int)kg * 4 + k;
+          if (kb < q.KB) v |= (uint32_t)__ldg(q.sc8 + flat_block(q, r, kb)) << (8 * k);
+        }
+      }
+      reinterpret_cast<uint32_t*>(q.sf)[i] = v;
     } else {
       const int64_t j = i - n_sf;
-      const int r = (int)(j % q.rows_pad), c = (int)(j / q.rows_pad);
+      const int c = (int)(j / q.rows_pad), r = (int)(j - (int64_t)c * q.rows_pad);
       float v = 0.0f;
-      if (r < q.rows) v = q.sc32[flat_block(q, r, c * q.P) / q.Ksg] * 0.0078125f;
+      if (r < q.rows) v = __ldg(q.sc32 + flat_block(q, r, c * q.P) / q.Ksg) * 0.0078125f;
       q.f[j] = v;
     }
   }
@@ -1287,14 +1303,20 @@ int make_plan(const pb_operand* a, const pb_operand* b, GemmPlan* gp) {
   return PB_OK;
 }
 
-int launch_prep(const pb_operand* o, const OperandPlan& op, const GemmPlan& gp, int rows_pad, int tile_rows, int tiles, int atoms_per_tile,
-                uint8_t* sf, float* f, cudaStream_t st) {
-  PrepParams q{o->sc8, o->sc32, sf, f, (int)o->rows, rows_pad, gp.KB, gp.KG, gp.P, gp.nchunks, tile_rows, tiles, atoms_per_tile,
-               o->grid_a, o->transposed_blocks, op.Ksg};
-  const int64_t items = (int64_t)gp.KG * tiles * atoms_per_tile * 512 + (int64_t)rows_pad * gp.nchunks;
-  const int64_t need = (items + 255) / 256;
-  const int grid = (int)(need < (int64_t)sm_count() * 8 ? need : (int64_t)sm_count() * 8);
-  gemm_prep_kernel<<<grid, 256, 0, st>>>(q);
+PrepParams prep_params(const pb_operand* o, const OperandPlan& op, const GemmPlan& gp, int rows_pad, int tile_rows, int tiles, int atoms_per_tile,
+                       uint8_t* sf, float* f) {
+  return PrepParams{o->sc8, o->sc32, sf, f, (int)o->rows, rows_pad, gp.KB, gp.KG, gp.P, gp.nchunks, tile_rows, tiles, atoms_per_tile,
+                    o->grid_a, o->transposed_blocks, op.Ksg};
+}
+unsigned prep_blocks(const PrepParams& q) {
+  const int64_t items = (int64_t)q.KG * q.tiles * q.atoms_per_tile * 128 + (int64_t)q.rows_pad * q.nchunks;
+  const int64_t need = (items + 255) / 256, cap = (int64_t)sm_count() * 8;
+  return (unsigned)(need < cap ? need : cap);
+}
+// `a`, `b`: the operands to prepare; either may be null, not both
+int launch_prep(const PrepParams* a, const PrepParams* b, cudaStream_t st) {
+  PrepPair pair{{a ? *a : *b, b ? *b : *a}, a ? prep_blocks(*a) : 0u};
+  gemm_prep_kernel<<<pair.first + (b ? prep_blocks(*b) : 0u), 256, 0, st>>>(pair);
   PB_LAUNCH_CHECK("gemm_prep_kernel");
   return PB_OK;
 }
@@ -1409,10 +1431,12 @@ extern "C" int pb_gemm_tn_ex(const pb_operand* a, const pb_operand* b, void* d, 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
 
-  if (!(flags & PB_GEMM_A_PREPARED))
-    if (int s = launch_prep(a, gp.pa, gp, gp.Mpad, 128, gp.tiles_m, 1, ws + gp.off_sfa, reinterpret_cast<float*>(ws + gp.off_fa), st)) return s;
-  if (!(flags & PB_GEMM_B_PREPARED))
-    if (int s = launch_prep(b, gp.pb, gp, gp.Npad, gp.BN, gp.tiles_n, gp.atoms_b, ws + gp.off_sfb, reinterpret_cast<float*>(ws + gp.off_fb), st)) return s;
+  const bool prep_a = !(flags & PB_GEMM_A_PREPARED), prep_b = !(flags & PB_GEMM_B_PREPARED);
+  if (prep_a || prep_b) {
+    const PrepParams pa = prep_params(a, gp.pa, gp, gp.Mpad, 128, gp.tiles_m, 1, ws + gp.off_sfa, reinterpret_cast<float*>(ws + gp.off_fa));
+    const PrepParams pb = prep_params(b, gp.pb, gp, gp.Npad, gp.BN, gp.tiles_n, gp.atoms_b, ws + gp.off_sfb, reinterpret_cast<float*>(ws + gp.off_fb));
+    if (int s = launch_prep(prep_a ? &pa : nullptr, prep_b ? &pb : nullptr, st)) return s;
+  }
 
   CUtensorMap ma, mb;
   if (int s = make_operand_map(&ma, a->q, a->rows, a->depth, BM)) return s;
