@@ -218,6 +218,10 @@ PB_API int pb_quantize_for_gemm(const void* x, int x_dtype, int64_t rows, int64_
  * super-groups of eight blocks only; anything else returns PB_ERR_UNSUPPORTED (use the two calls). */
 PB_API int pb_fake_quantize(const void* x, int x_dtype, int64_t batch, int64_t rows, int64_t cols, int a, int b,
                      int out_format, void* out, int out_dtype, void* stream);
+/* The same with the scales of the triple in between, which the backward pass of a Linear needs of its output
+ * (dequantize_impl_bwd, pratchya/_qualia/_qarr.py:575-601): sc8 and sc32 as pb_quantize writes them. */
+PB_API int pb_fake_quantize_scales(const void* x, int x_dtype, int64_t batch, int64_t rows, int64_t cols, int a, int b,
+                            int out_format, void* out, int out_dtype, uint8_t* sc8, float* sc32, void* stream);
 /* Reads (and clears) the device status words of the kernels that wait on mbarriers (the GEMM kernels and the
  * persistent transposed quantizer) launched on this device; synchronises `stream`.  Every such wait is bounded
  * (a few seconds at most); a wait that runs out makes its kernel return early and is reported here:

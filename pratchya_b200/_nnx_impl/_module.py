@@ -199,9 +199,8 @@ class _LinearFn(torch.autograd.Function):
         else:
             ctx.have_xt = False
         if fake_quant_output:
-            yq = _ops.quantize_impl(y, (1, b))
-            y = _ops.dequantize_impl(*yq, x.dtype, (1, b))
-            saved += [yq[1], yq[2]]
+            y, y_sc8, y_sc32 = _ops.fake_quantize_scales_impl(y, (1, b), x.dtype)
+            saved += [y_sc8, y_sc32]
         else:
             y = y.to(x.dtype)
         ctx.save_for_backward(*saved)

@@ -170,25 +170,50 @@ def dequantize_impl(x_fp8: torch.Tensor, sc_fp8: torch.Tensor, sc_fp32: torch.Te
     return out if kernel_dtype == dtype else out.to(dtype)
 
 
+def _fake_quantize_fused(x: torch.Tensor, tgrid, dtype) -> bool:
+    """Whether one kernel fake-quantizes x: f32 on the (1,128) grid with whole 8-block super-groups."""
+    if not (x.dtype == torch.float32 and dtype in _DENSE_CODE and (int(tgrid[0]), int(tgrid[1])) == (1, 128) and x.numel() > 0):
+        return False
+    rows, cols = _as_2d(tuple(x.shape))[-2:]
+    return group_geometry(rows, cols, (1, 128))[1] == 8
+
+
 def fake_quantize_impl(x: torch.Tensor, tgrid, dtype, out_format: str = "e4m3") -> torch.Tensor:
     """dequantize_impl(*quantize_impl(x, tgrid), dtype, tgrid) -- QArrayImpl(x, tgrid).astype(dtype),
     _qarr.py:29 and :339-342 -- in one pass where the library has a fused kernel (f32 input on the
     (1,128) grid with whole 8-block super-groups), otherwise by the two calls.  Same bits either way."""
     _require_cuda(x, "fake_quantize_impl input")
+    if not _fake_quantize_fused(x, tgrid, dtype):
+        return dequantize_impl(*quantize_impl(x, tgrid, out_format), dtype, tgrid)
     lib = _lib.load()
     shape = _as_2d(tuple(x.shape))
-    a, b = int(tgrid[0]), int(tgrid[1])
-    rows, cols = shape[-2], shape[-1]
-    fused = (x.dtype == torch.float32 and dtype in _DENSE_CODE and (a, b) == (1, 128) and x.numel() > 0
-             and group_geometry(rows, cols, (a, b))[1] == 8)
-    if not fused:
-        return dequantize_impl(*quantize_impl(x, tgrid, out_format), dtype, tgrid)
     x = x.contiguous()
     with torch.cuda.device(x.device):
         out = torch.empty(tuple(x.shape), dtype=dtype, device=x.device)
-        check(lib.pb_fake_quantize(x.data_ptr(), _DENSE_CODE[x.dtype], math.prod(shape[:-2]), rows, cols, a, b,
+        check(lib.pb_fake_quantize(x.data_ptr(), _DENSE_CODE[x.dtype], math.prod(shape[:-2]), shape[-2], shape[-1], 1, 128,
                                    _FMT_CODE[out_format], out.data_ptr(), _DENSE_CODE[dtype], _stream(x)))
     return out
+
+
+def fake_quantize_scales_impl(x: torch.Tensor, tgrid, dtype):
+    """(fake_quantize_impl(x, tgrid, dtype), sc_fp8, sc_fp32): the value a Linear returns and the scales of its triple, which the
+    cotangent rule of that value needs (_qarr.py:575-601); the fp8 bytes in between are not written where one kernel does it."""
+    _require_cuda(x, "fake_quantize_scales_impl input")
+    if not _fake_quantize_fused(x, tgrid, dtype):
+        q, sc8, sc32 = quantize_impl(x, tgrid)
+        return dequantize_impl(q, sc8, sc32, dtype, tgrid), sc8, sc32
+    lib = _lib.load()
+    shape = _as_2d(tuple(x.shape))
+    lead, (m, k) = shape[:-2], group_geometry(shape[-2], shape[-1], (1, 128))
+    x = x.contiguous()
+    dev = x.device
+    with torch.cuda.device(dev):
+        out = torch.empty(tuple(x.shape), dtype=dtype, device=dev)
+        sc8 = torch.empty((*lead, m, k), dtype=E8M0, device=dev)
+        sc32 = torch.empty((*lead, m, 1, 1), dtype=torch.float32, device=dev)
+        check(lib.pb_fake_quantize_scales(x.data_ptr(), PB_F32, math.prod(lead), shape[-2], shape[-1], 1, 128, PB_E4M3,
+                                          out.data_ptr(), _DENSE_CODE[dtype], sc8.data_ptr(), sc32.data_ptr(), _stream(x)))
+    return out, sc8, sc32
 
 
 def relu2_requantize_impl(y: torch.Tensor):

@@ -349,9 +349,11 @@ template <> struct Out4<__nv_bfloat16> {
   static __device__ __forceinline__ vec make(float a, float b, float c, float d) { return make_uint2(pack_bf16x2(a, b), pack_bf16x2(c, d)); }
 };
 
-template <int FMT, typename OutT>
+// SCALES: the triple's scales leave as well (the fp8 bytes never do).
+template <int FMT, typename OutT, bool SCALES>
 __global__ void __launch_bounds__(kRowThreads)
-fake_quantize_row128_f32_kernel(const float4* __restrict__ x, typename Out4<OutT>::vec* __restrict__ out, int64_t n_groups) {
+fake_quantize_row128_f32_kernel(const float4* __restrict__ x, typename Out4<OutT>::vec* __restrict__ out, uint8_t* __restrict__ sc8,
+                                float* __restrict__ sc32, int64_t n_groups) {
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * (kRowThreads / 32);
   for (int64_t g = (int64_t)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); g < n_groups; g += warps_total) {
@@ -373,6 +375,10 @@ fake_quantize_row128_f32_kernel(const float4* __restrict__ x, typename Out4<OutT
     block_scale(m[0], Mj, sb, D);
     const float r = __frcp_rn(D);
     const float x_sc = __fmul_rn(e8m0_to_f32(sb), Mj);       // the dequantizer's multiplier: raw amax, no floor
+    if (SCALES) {
+      if (lane < 8) sc8[g * 8 + bitrev<3>(lane)] = (uint8_t)sb;
+      if (lane == 0) sc32[g] = Mj;
+    }
 
     typename Out4<OutT>::vec* dst = out + g * (kGroupElems / 4);
 #pragma unroll
@@ -1226,8 +1232,8 @@ extern "C" int pb_shift_lerp_quantize(const float* x, const float* state, const 
   return PB_OK;
 }
 
-extern "C" int pb_fake_quantize(const void* x, int x_dtype, int64_t batch, int64_t rows, int64_t cols, int a, int b,
-                                int out_format, void* out, int out_dtype, void* stream) {
+static int fake_quantize_entry(const void* x, int x_dtype, int64_t batch, int64_t rows, int64_t cols, int a, int b,
+                               int out_format, void* out, int out_dtype, uint8_t* sc8, float* sc32, void* stream) {
   if (!x || !out) return fail(PB_ERR_NULL_POINTER, "pb_fake_quantize: x and out must be non-null");
   if (batch <= 0) return fail(PB_ERR_BAD_SHAPE, "pb_fake_quantize: batch=%lld must be positive", (long long)batch);
   if (out_format != PB_E4M3 && out_format != PB_E5M2) return fail(PB_ERR_BAD_DTYPE, "pb_fake_quantize: out_format %d is neither PB_E4M3 nor PB_E5M2", out_format);
@@ -1242,15 +1248,32 @@ extern "C" int pb_fake_quantize(const void* x, int x_dtype, int64_t batch, int64
   const int64_t n_groups = batch * g.M;
   const int grid = grid_for(n_groups * 32, kRowThreads, 8);
   const bool e4 = out_format == PB_E4M3;
+#define PB_FAKE_LAUNCH(FMT, OT, VT)                                                                                                              \
+  do {                                                                                                                                           \
+    if (sc8) fake_quantize_row128_f32_kernel<FMT, OT, true><<<grid, kRowThreads, 0, st>>>((const float4*)x, (VT*)out, sc8, sc32, n_groups);       \
+    else     fake_quantize_row128_f32_kernel<FMT, OT, false><<<grid, kRowThreads, 0, st>>>((const float4*)x, (VT*)out, nullptr, nullptr, n_groups); \
+  } while (0)
   if (out_dtype == PB_F32) {
-    if (e4) fake_quantize_row128_f32_kernel<PB_E4M3, float><<<grid, kRowThreads, 0, st>>>((const float4*)x, (float4*)out, n_groups);
-    else    fake_quantize_row128_f32_kernel<PB_E5M2, float><<<grid, kRowThreads, 0, st>>>((const float4*)x, (float4*)out, n_groups);
+    if (e4) PB_FAKE_LAUNCH(PB_E4M3, float, float4);
+    else    PB_FAKE_LAUNCH(PB_E5M2, float, float4);
   } else {
-    if (e4) fake_quantize_row128_f32_kernel<PB_E4M3, __nv_bfloat16><<<grid, kRowThreads, 0, st>>>((const float4*)x, (uint2*)out, n_groups);
-    else    fake_quantize_row128_f32_kernel<PB_E5M2, __nv_bfloat16><<<grid, kRowThreads, 0, st>>>((const float4*)x, (uint2*)out, n_groups);
+    if (e4) PB_FAKE_LAUNCH(PB_E4M3, __nv_bfloat16, uint2);
+    else    PB_FAKE_LAUNCH(PB_E5M2, __nv_bfloat16, uint2);
   }
+#undef PB_FAKE_LAUNCH
   PB_LAUNCH_CHECK("fake_quantize_row128_f32_kernel");
   return PB_OK;
+}
+
+extern "C" int pb_fake_quantize(const void* x, int x_dtype, int64_t batch, int64_t rows, int64_t cols, int a, int b,
+                                int out_format, void* out, int out_dtype, void* stream) {
+  return fake_quantize_entry(x, x_dtype, batch, rows, cols, a, b, out_format, out, out_dtype, nullptr, nullptr, stream);
+}
+
+extern "C" int pb_fake_quantize_scales(const void* x, int x_dtype, int64_t batch, int64_t rows, int64_t cols, int a, int b,
+                                       int out_format, void* out, int out_dtype, uint8_t* sc8, float* sc32, void* stream) {
+  if (!sc8 || !sc32) return fail(PB_ERR_NULL_POINTER, "pb_fake_quantize_scales: sc8 and sc32 must be non-null");
+  return fake_quantize_entry(x, x_dtype, batch, rows, cols, a, b, out_format, out, out_dtype, sc8, sc32, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -1,8 +1,11 @@
-"""The byte transpose of a weight: its 16-byte form and the other."""
+"""Small kernels around a Linear's products: the byte transpose of a weight (16-byte form and the other), and the fake quantization
+that also leaves its scales, against the calls they stand for."""
 import pytest
 import torch
 
+from helpers import synth, to_torch
 from pratchya_b200._qualia import _ops
+from pratchya_b200._qualia import dequantize_impl, quantize_impl
 
 pytestmark = pytest.mark.gpu
 
@@ -11,3 +14,13 @@ pytestmark = pytest.mark.gpu
 def test_transpose_bytes(built_lib, rows, cols):
     q = torch.randint(0, 256, (rows, cols), device="cuda", dtype=torch.uint8).view(torch.float8_e4m3fn)
     assert torch.equal(_ops.transpose_bytes(q).view(torch.uint8), q.view(torch.uint8).t())
+
+
+@pytest.mark.parametrize("shape,dtype", [((1, 1024), torch.float32), ((3, 2048), torch.bfloat16), ((8, 128), torch.float32), ((2, 5, 1024), torch.float32),
+                                         ((3, 128), torch.float32), ((4, 384), torch.bfloat16)])
+def test_fake_quantize_with_its_scales(built_lib, shape, dtype):
+    x = to_torch(synth(shape, seed=shape[-1]))
+    out, sc8, sc32 = _ops.fake_quantize_scales_impl(x, (1, 128), dtype)
+    q, want8, want32 = quantize_impl(x, (1, 128))
+    assert torch.equal(out, dequantize_impl(q, want8, want32, dtype, (1, 128)))
+    assert torch.equal(sc8.view(torch.uint8), want8.view(torch.uint8)) and torch.equal(sc32, want32) and sc8.shape == want8.shape
