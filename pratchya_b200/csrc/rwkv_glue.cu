@@ -137,6 +137,10 @@ __global__ void __launch_bounds__(kGlueThreads) reduce_partials_kernel(const flo
 // ---- TimeMix between its linears and the scan ----------------------------------------------------------------
 // One warp per (token, head); lane l holds channels l and l + 32 of the head: the two halves that the rotary
 // embedding pairs (_module.py:275-283: x * cos + cat(-x2, x1) * sin, the same angle for both halves).
+// Bound by their 14 and 20 passes over [tokens, channels].  Every input is read through __ldg, so that a row's loads are all
+// under way before its first store (and, backward, the next row's before this one's last): as plain loads they wait for the
+// stores in front of them, which might be to the same arrays for all the compiler knows.  8 x 1024 tokens of 2048
+// channels: forward 195 -> 166 us, backward 381 -> 216 us (6.2 TB/s).
 struct PrepareParams {
   const float* r_raw; const float* k_raw; const float* d; const float* iclr_raw; const float* v_prime;
   const float* v0; const float* nu_raw;                      // null in the first layer (v = v_prime)
@@ -162,18 +166,19 @@ __global__ void __launch_bounds__(kGlueThreads) wkv_prepare_fwd_kernel(const Pre
     const int c1 = n * kGlueH + lane, c2 = c1 + 32;
     const size_t i1 = (size_t)row * C + c1, i2 = i1 + 32;
     const float cs = __ldg(p.cos_tab + t * 32 + lane), sn = __ldg(p.sin_tab + t * 32 + lane);
-    const float ra = p.r_raw[i1], rb = p.r_raw[i2], ka = p.k_raw[i1], kb = p.k_raw[i2];
+    const float ra = __ldg(p.r_raw + i1), rb = __ldg(p.r_raw + i2), ka = __ldg(p.k_raw + i1), kb = __ldg(p.k_raw + i2);
+    const float ar1 = __ldg(p.iclr_raw + i1), ar2 = __ldg(p.iclr_raw + i2), d1 = __ldg(p.d + i1), d2 = __ldg(p.d + i2);
+    float v1 = __ldg(p.v_prime + i1), v2 = __ldg(p.v_prime + i2);
     const float r1 = __fadd_rn(__fmul_rn(ra, cs), __fmul_rn(-rb, sn)), r2 = __fadd_rn(__fmul_rn(rb, cs), __fmul_rn(ra, sn));
     const float k1 = __fadd_rn(__fmul_rn(ka, cs), __fmul_rn(-kb, sn)), k2 = __fadd_rn(__fmul_rn(kb, cs), __fmul_rn(ka, sn));
-    const float a1 = sigmoid_rn(p.iclr_raw[i1]), a2 = sigmoid_rn(p.iclr_raw[i2]);
-    float v1 = p.v_prime[i1], v2 = p.v_prime[i2];
+    const float a1 = sigmoid_rn(ar1), a2 = sigmoid_rn(ar2);
     if (p.v0) {
-      v1 = lerp_rn(v1, p.v0[i1], sigmoid_rn(p.nu_raw[i1]));
-      v2 = lerp_rn(v2, p.v0[i2], sigmoid_rn(p.nu_raw[i2]));
+      v1 = lerp_rn(v1, __ldg(p.v0 + i1), sigmoid_rn(__ldg(p.nu_raw + i1)));
+      v2 = lerp_rn(v2, __ldg(p.v0 + i2), sigmoid_rn(__ldg(p.nu_raw + i2)));
     }
     const float u1 = __fmul_rn(k1, __ldg(p.rk_mult + c1)), u2 = __fmul_rn(k2, __ldg(p.rk_mult + c2));
     const float nrm = sqrtf(__fadd_rn(warp_sum(__fadd_rn(__fmul_rn(u1, u1), __fmul_rn(u2, u2))), 1e-12f));
-    p.decay[i1] = expf(-expf(p.d[i1])); p.decay[i2] = expf(-expf(p.d[i2]));
+    p.decay[i1] = expf(-expf(d1)); p.decay[i2] = expf(-expf(d2));
     p.iclr[i1] = a1; p.iclr[i2] = a2;
     p.removal_k[i1] = __fdiv_rn(u1, nrm); p.removal_k[i2] = __fdiv_rn(u2, nrm);
     p.replacement_k[i1] = lerp_rn(k1, __fmul_rn(k1, a1), __ldg(p.mix_amt + c1));
@@ -210,38 +215,44 @@ __global__ void __launch_bounds__(kGlueThreads) wkv_prepare_bwd_kernel(const Pre
     const int t = (int)(row % f.T);
     const size_t i1 = (size_t)row * C + c1, i2 = i1 + 32;
     const float cs = __ldg(f.cos_tab + t * 32 + lane), sn = __ldg(f.sin_tab + t * 32 + lane);
-    const float ka = f.k_raw[i1], kb = f.k_raw[i2];
+    const float ka = __ldg(f.k_raw + i1), kb = __ldg(f.k_raw + i2);
+    const float ar1 = __ldg(f.iclr_raw + i1), ar2 = __ldg(f.iclr_raw + i2), gq1 = __ldg(p.g_removal_k + i1), gq2 = __ldg(p.g_removal_k + i2);
+    const float gp1 = __ldg(p.g_replacement_k + i1), gp2 = __ldg(p.g_replacement_k + i2), gk1 = __ldg(p.g_k + i1), gk2 = __ldg(p.g_k + i2);
+    const float gi1 = __ldg(p.g_iclr + i1), gi2 = __ldg(p.g_iclr + i2), gr1 = __ldg(p.g_r + i1), gr2 = __ldg(p.g_r + i2);
+    const float d1 = __ldg(f.d + i1), d2 = __ldg(f.d + i2), gd1 = __ldg(p.g_decay + i1), gd2 = __ldg(p.g_decay + i2);
+    const float gv1 = __ldg(p.g_v + i1), gv2 = __ldg(p.g_v + i2);
+    float nr1 = 0.f, nr2 = 0.f, vd1 = 0.f, vd2 = 0.f;      // nu_raw, v0 - v_prime
+    if (f.v0) {
+      nr1 = __ldg(f.nu_raw + i1); nr2 = __ldg(f.nu_raw + i2);
+      vd1 = __ldg(f.v0 + i1) - __ldg(f.v_prime + i1); vd2 = __ldg(f.v0 + i2) - __ldg(f.v_prime + i2);
+    }
     const float k1 = __fadd_rn(__fmul_rn(ka, cs), __fmul_rn(-kb, sn)), k2 = __fadd_rn(__fmul_rn(kb, cs), __fmul_rn(ka, sn));
-    const float a1 = sigmoid_fast(f.iclr_raw[i1]), a2 = sigmoid_fast(f.iclr_raw[i2]);
+    const float a1 = sigmoid_fast(ar1), a2 = sigmoid_fast(ar2);
     // removal_k = u / nrm, u = k * m: d_u = (g - removal_k * sum(g * removal_k)) / nrm
     const float u1 = __fmul_rn(k1, m1), u2 = __fmul_rn(k2, m2);
     const float inv_nrm = rsqrtf(warp_sum(u1 * u1 + u2 * u2) + 1e-12f);
     const float q1 = u1 * inv_nrm, q2 = u2 * inv_nrm;
-    const float gq1 = p.g_removal_k[i1], gq2 = p.g_removal_k[i2];
     const float dot = warp_sum(gq1 * q1 + gq2 * q2);
     const float du1 = (gq1 - q1 * dot) * inv_nrm, du2 = (gq2 - q2 * dot) * inv_nrm;
     dm1 = fmaf(du1, k1, dm1); dm2 = fmaf(du2, k2, dm2);
     // replacement_k = k + (k * a - k) * x
-    const float gp1 = p.g_replacement_k[i1], gp2 = p.g_replacement_k[i2];
     dx1 = fmaf(gp1, k1 * a1 - k1, dx1); dx2 = fmaf(gp2, k2 * a2 - k2, dx2);
-    const float dk1 = p.g_k[i1] + du1 * m1 + gp1 * (1.0f + (a1 - 1.0f) * x1);
-    const float dk2 = p.g_k[i2] + du2 * m2 + gp2 * (1.0f + (a2 - 1.0f) * x2);
-    const float da1 = p.g_iclr[i1] + gp1 * k1 * x1, da2 = p.g_iclr[i2] + gp2 * k2 * x2;
+    const float dk1 = gk1 + du1 * m1 + gp1 * (1.0f + (a1 - 1.0f) * x1);
+    const float dk2 = gk2 + du2 * m2 + gp2 * (1.0f + (a2 - 1.0f) * x2);
+    const float da1 = gi1 + gp1 * k1 * x1, da2 = gi2 + gp2 * k2 * x2;
     p.d_iclr_raw[i1] = da1 * a1 * (1.0f - a1); p.d_iclr_raw[i2] = da2 * a2 * (1.0f - a2);
     // rotary: out1 = x1 cos - x2 sin, out2 = x2 cos + x1 sin
     p.d_k_raw[i1] = dk1 * cs + dk2 * sn; p.d_k_raw[i2] = dk2 * cs - dk1 * sn;
-    const float gr1 = p.g_r[i1], gr2 = p.g_r[i2];
     p.d_r_raw[i1] = gr1 * cs + gr2 * sn; p.d_r_raw[i2] = gr2 * cs - gr1 * sn;
     // decay = exp(-e), e = exp(d)
-    const float e1 = __expf(f.d[i1]), e2 = __expf(f.d[i2]);
-    p.d_d[i1] = -p.g_decay[i1] * __expf(-e1) * e1; p.d_d[i2] = -p.g_decay[i2] * __expf(-e2) * e2;
-    const float gv1 = p.g_v[i1], gv2 = p.g_v[i2];
+    const float e1 = __expf(d1), e2 = __expf(d2);
+    p.d_d[i1] = -gd1 * __expf(-e1) * e1; p.d_d[i2] = -gd2 * __expf(-e2) * e2;
     if (f.v0) {
-      const float nu1 = sigmoid_fast(f.nu_raw[i1]), nu2 = sigmoid_fast(f.nu_raw[i2]);
+      const float nu1 = sigmoid_fast(nr1), nu2 = sigmoid_fast(nr2);
       p.d_v_prime[i1] = gv1 - gv1 * nu1; p.d_v_prime[i2] = gv2 - gv2 * nu2;
       p.d_v0[i1] = gv1 * nu1; p.d_v0[i2] = gv2 * nu2;
-      p.d_nu_raw[i1] = gv1 * (f.v0[i1] - f.v_prime[i1]) * nu1 * (1.0f - nu1);
-      p.d_nu_raw[i2] = gv2 * (f.v0[i2] - f.v_prime[i2]) * nu2 * (1.0f - nu2);
+      p.d_nu_raw[i1] = gv1 * vd1 * nu1 * (1.0f - nu1);
+      p.d_nu_raw[i2] = gv2 * vd2 * nu2 * (1.0f - nu2);
     } else {
       p.d_v_prime[i1] = gv1; p.d_v_prime[i2] = gv2;
     }
