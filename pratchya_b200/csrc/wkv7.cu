@@ -11,17 +11,10 @@
 //     y_i   = sum_j S[i][j] * r_j                           (:199)
 // All arithmetic is fp32, as in the reference (its inputs are cast to f32 before the scan).
 //
-// Two layouts of the state over the threads of a CTA (one CTA per (b, n), H = 64).
-// Forward: one row per thread (64 threads).  Both dot products of a timestep run inside the thread, so the recurrence
-// holds no shuffle; the price is that every thread reads every input vector in full, and although those reads are
-// same-address broadcasts a 16-byte load still returns 512 bytes per warp to the registers: at 128 bytes per clock
-// and SM that traffic is what bounds the kernel.
-// Backward: 2-D tiles (128 threads).  Warp q owns rows 16q .. 16q+15; its 32 lanes form a 4 x 8 grid (ti, tj) and
-// lane (ti, tj) keeps the 4 x 8 tile of rows 16q + 4ti .. +3 and columns 4tj .. +3 and 32 + 4tj .. +3 (as float2 pairs
-// along the columns).  A lane reads 8 elements of each vector per timestep, not 64, which the backward pass needs:
-// kept per row and per column it moved four times the forward pass's vector bytes.  Sums along a row end with three
-// xor-shuffles across tj and never leave the warp; sums along a column are outputs, not part of the recurrence: two
-// butterfly shuffle levels across ti, then the warps' parts meet in shared memory.
+// Both kernels keep the state in 2-D register tiles (H = 64), so that a lane reads a part of each vector per timestep: what
+// those reads return to the registers, 128 bytes per clock and SM, is what a whole row per thread was bound by.  Sums along a
+// row stay inside a warp (shuffles); sums along a column, which only the backward pass has and which are outputs, not part of
+// the recurrence, meet in shared memory.
 // The input vectors of a timestep arrive by cp.async ahead of time.  HBM traffic is the algorithmic minimum: every
 // input read once, every output written once, the state once per sequence, plus what the backward pass needs when
 // one follows (below).
@@ -31,19 +24,10 @@ namespace pb {
 namespace {
 
 constexpr int kH = 64;            // head size
-constexpr int kR = 4;             // rows of a lane's tile (measured: 4 beats 8 and 2 on batch 8 x 32 heads x 4096 timesteps)
-constexpr int kWarps = 16 / kR;   // a warp owns 4 * kR rows
+constexpr int kWarps = 4;         // of the backward kernel: a warp owns 16 rows
 constexpr int kThreads = 32 * kWarps;      // per head
-constexpr int kPairs = 4;         // forward ring depth in pairs of timesteps: eight timesteps of input in flight
 constexpr int kVecs = 6;          // decay, iclr, removal_k, replacement_k, v, r
 constexpr int kCk = 8;            // spacing of the state checkpoints the backward pass restarts from
-#ifndef PB_WKV_FWD_ROWS
-#define PB_WKV_FWD_ROWS 1
-#endif
-// State rows per thread of the forward kernel (64 / kFwdRows threads per head).  Two rows per thread halve the vector bytes a
-// timestep pulls from shared memory, but the one warp left per head then runs twice the arithmetic in sequence: measured 2.67 ms
-// against 1.88 ms for one row per thread (batch 8 x 32 heads x 4096 timesteps).
-constexpr int kFwdRows = PB_WKV_FWD_ROWS;
 constexpr int kSub = 4;           // timesteps whose recomputed states the backward pass keeps at once
 constexpr int kBwdVecs = kVecs + 2;      // the six inputs, dy and sa
 constexpr int kTileQuads = kH * kH / 4;  // float4 per state
@@ -61,96 +45,26 @@ __device__ __forceinline__ void ld8(const float* p, float2 (&out)[4]) {
   const float4 lo = *reinterpret_cast<const float4*>(p), hi = *reinterpret_cast<const float4*>(p + 32);
   out[0] = make_float2(lo.x, lo.y); out[1] = make_float2(lo.z, lo.w); out[2] = make_float2(hi.x, hi.y); out[3] = make_float2(hi.z, hi.w);
 }
-// kR consecutive floats
-__device__ __forceinline__ void ldr(const float* p, float (&out)[kR]) {
-  if constexpr (kR == 8) {
-    const float4 lo = *reinterpret_cast<const float4*>(p), hi = *reinterpret_cast<const float4*>(p + 4);
-    out[0] = lo.x; out[1] = lo.y; out[2] = lo.z; out[3] = lo.w; out[4] = hi.x; out[5] = hi.y; out[6] = hi.z; out[7] = hi.w;
-  } else if constexpr (kR == 4) {
-    const float4 lo = *reinterpret_cast<const float4*>(p);
-    out[0] = lo.x; out[1] = lo.y; out[2] = lo.z; out[3] = lo.w;
-  } else {
-    const float2 lo = *reinterpret_cast<const float2*>(p);
-    out[0] = lo.x; out[1] = lo.y;
-  }
-}
-
-// every lane's v[a] becomes the sum over the eight lanes that share ti (lane bits 0..2)
-__device__ __forceinline__ void row_allreduce(float (&v)[kR]) {
-#pragma unroll
-  for (int m = 1; m < 8; m <<= 1) {
-#pragma unroll
-    for (int a = 0; a < kR; ++a) v[a] += __shfl_xor_sync(0xffffffffu, v[a], m);
-  }
-}
-// four column sums over the four lanes that share tj (lane bits 3, 4): lane ti ends up with column ti of the four
-__device__ __forceinline__ float col_reduce_scatter(const float2 (&v)[2], int ti) {
-  bool up = ti & 2;
-  const float2 keep = up ? v[1] : v[0], send = up ? v[0] : v[1];
-  const float2 w2 = make_float2(keep.x + __shfl_xor_sync(0xffffffffu, send.x, 16), keep.y + __shfl_xor_sync(0xffffffffu, send.y, 16));
-  up = ti & 1;
-  return (up ? w2.y : w2.x) + __shfl_xor_sync(0xffffffffu, up ? w2.x : w2.y, 8);
-}
-__device__ __forceinline__ float pick(const float (&v)[kR], int a) {
-  float r = v[0];
-#pragma unroll
-  for (int k = 1; k < kR; ++k) r = a == k ? v[k] : r;
-  return r;
-}
-
-// Where lane (ti, tj) of warp q sits: rows row0 .. row0 + kR - 1, columns col0 .. col0+3 and 32 + col0 .. +3 (so that the
-// eight lanes of a tile row read 128 contiguous bytes of a vector with each 16-byte load: no bank conflicts).
-struct Tile {
-  int tid, ti, tj, row0, col0;
-  __device__ Tile() {
-    tid = threadIdx.x;
-    const int lane = tid & 31;
-    ti = lane >> 3; tj = lane & 7;
-    row0 = 4 * kR * (tid >> 5) + kR * ti; col0 = 4 * tj;
-  }
-};
-
-// the 8 x 8 tile of a row-major H x H matrix in global memory
-__device__ __forceinline__ void load_tile_rowmajor(const float* m, const Tile& tl, float2 (&S)[kR][4]) {
-#pragma unroll
-  for (int a = 0; a < kR; ++a) {
-    const float4 lo = __ldg(reinterpret_cast<const float4*>(m + (tl.row0 + a) * kH + tl.col0));
-    const float4 hi = __ldg(reinterpret_cast<const float4*>(m + (tl.row0 + a) * kH + tl.col0 + 32));
-    S[a][0] = make_float2(lo.x, lo.y); S[a][1] = make_float2(lo.z, lo.w); S[a][2] = make_float2(hi.x, hi.y); S[a][3] = make_float2(hi.z, hi.w);
-  }
-}
-__device__ __forceinline__ void store_tile_rowmajor(float* m, const Tile& tl, const float2 (&S)[kR][4]) {
-#pragma unroll
-  for (int a = 0; a < kR; ++a) {
-    *reinterpret_cast<float4*>(m + (tl.row0 + a) * kH + tl.col0) = make_float4(S[a][0].x, S[a][0].y, S[a][1].x, S[a][1].y);
-    *reinterpret_cast<float4*>(m + (tl.row0 + a) * kH + tl.col0 + 32) = make_float4(S[a][2].x, S[a][2].y, S[a][3].x, S[a][3].y);
-  }
-}
-// The tile in the kernels' own layout, [2 kR quarters][threads] float4: consecutive threads, consecutive 16 bytes
-// (checkpoints in global memory, recomputed states in shared memory).
-template <typename Ptr>
-__device__ __forceinline__ void store_tile_private(Ptr base, const Tile& tl, const float2 (&S)[kR][4]) {
-#pragma unroll
-  for (int a = 0; a < kR; ++a) {
-    base[(2 * a) * kThreads + tl.tid] = make_float4(S[a][0].x, S[a][0].y, S[a][1].x, S[a][1].y);
-    base[(2 * a + 1) * kThreads + tl.tid] = make_float4(S[a][2].x, S[a][2].y, S[a][3].x, S[a][3].y);
-  }
-}
-template <typename Ptr>
-__device__ __forceinline__ void load_tile_private(Ptr base, const Tile& tl, float2 (&S)[kR][4]) {
-#pragma unroll
-  for (int a = 0; a < kR; ++a) {
-    const float4 lo = base[(2 * a) * kThreads + tl.tid], hi = base[(2 * a + 1) * kThreads + tl.tid];
-    S[a][0] = make_float2(lo.x, lo.y); S[a][1] = make_float2(lo.z, lo.w); S[a][2] = make_float2(hi.x, hi.y); S[a][3] = make_float2(hi.z, hi.w);
-  }
-}
+// A state in the kernels' own layout (checkpoints in global memory, kept states in shared memory): 1024 quads, a quad the
+// rows 2P, 2P + 1 of the columns 2Q, 2Q + 1 as ((2P, 2Q), (2P+1, 2Q), (2P, 2Q+1), (2P+1, 2Q+1)).  Backward thread
+// 16 * (P >> 2) + (Q >> 1) keeps it as its quad 2 * (P & 3) + (Q & 1): consecutive threads, consecutive 16 bytes.
+__device__ __forceinline__ int ckpt_quad(int P, int Q) { return (2 * (P & 3) + (Q & 1)) * kThreads + 16 * (P >> 2) + (Q >> 1); }
 
 // ---- forward ---------------------------------------------------------------------------------------------------
-// The forward pass keeps one state ROW per thread (64 threads per head): both dot products of a timestep run inside the
-// thread on four independent partial sums, with no shuffle anywhere in the recurrence, and every vector is read as a
-// same-address broadcast.  That makes it bound by the bytes those reads return to the registers (80 16-byte loads per
-// thread and timestep), and still a fifth faster than a forward pass on the backward pass's tiles (measured: 1.66 ms
-// against 2.04 ms on batch 8 x 32 heads x 4096 timesteps), whose three shuffle levels sit inside the recurrence.
+// The rows of a head's state are independent of one another given the timestep's vectors, so a head's 64 rows are cut over
+// warps, and where there are few heads over CTAs as well.  A warp owns 4 * ROWS rows on the backward pass's 4 x 8 lane grid:
+// a lane keeps ROWS rows x 8 columns, a row's two dot products end in three xor-shuffles (the state's one only delays the
+// warp, the output's one nothing).  No barrier inside a chunk of eight timesteps: the chunk's vectors arrive by cp.async two
+// chunks ahead, a step's are in registers one step ahead, and S * w + v kt^T is formed while sa's shuffles are under way.
+// What bounds it: with few heads the latency of a timestep (dot product, three shuffles, update: 310 cycles); with many the
+// f32x2 products, three cycles each where their operands are three different registers, and the 4 * (40 + ROWS) bytes per lane
+// and timestep that the vector reads return, which more rows per lane spread over more of them.
+// 1024 timesteps, against one row per thread and both dot products inside it: 32 heads 377 -> 174 us, 64 heads 379 -> 181,
+// 128 heads 379 -> 236, 256 heads 437 -> 370 (with sa and checkpoints 494 -> 457).  y reduced in its own timestep, behind sa's
+// shuffles, cost a fifth: 219 us with 32 heads.
+constexpr int kFwdChunk = 8;      // timesteps between barriers
+constexpr int kFwdBufs = 3;       // chunks in shared memory
+
 struct WkvParams {
   const float* in[kVecs];
   const float* state_in;          // [B, N, H, H] or null (zeros)
@@ -161,164 +75,213 @@ struct WkvParams {
   int T, N;                       // timesteps, heads
 };
 
-// One timestep for ROWS rows of S (rows i, i + kH / ROWS, ...): every vector load serves all of the thread's rows.
-// `buf` holds the step's decay, iclr, removal_k, replacement_k, v, r; `bk` = iclr * removal_k.
+// a lane's share of one timestep's vectors
 template <int ROWS>
-__device__ __forceinline__ void wkv_step(float2 (&S)[ROWS][32], const float (*buf)[kH], const float* bk, int i, float (&y_out)[ROWS], float (&sa_out)[ROWS]) {
-  // sa_i = sum_j S[i][j] * kap_j, four partial sums per row
-  float2 acc[ROWS][4];
-#pragma unroll
-  for (int a = 0; a < ROWS; ++a)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[a][q] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const float4 k4 = *reinterpret_cast<const float4*>(&buf[2][4 * j]);
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) {
-      acc[a][(2 * j) & 3] = __ffma2_rn(S[a][2 * j], make_float2(k4.x, k4.y), acc[a][(2 * j) & 3]);
-      acc[a][(2 * j + 1) & 3] = __ffma2_rn(S[a][2 * j + 1], make_float2(k4.z, k4.w), acc[a][(2 * j + 1) & 3]);
+struct StepVecs {
+  float2 w[4], b[4], kap[4], kt[4], r[4];
+  float v[ROWS];
+  __device__ __forceinline__ void load(const float (*buf)[kH], int col0, int row0) {
+    ld8(buf[2] + col0, kap);
+    ld8(buf[0] + col0, w);
+    ld8(buf[3] + col0, kt);
+    ld8(buf[1] + col0, b);
+    ld8(buf[5] + col0, r);
+    if constexpr (ROWS == 4) {
+      const float4 t = *reinterpret_cast<const float4*>(buf[4] + row0);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+      const float2 t = *reinterpret_cast<const float2*>(buf[4] + row0);
+      v[0] = t.x; v[1] = t.y;
     }
   }
-  float2 nsa2[ROWS], vi2[ROWS], y[ROWS][4];
+};
+
+// The sums over the eight lanes of a tile row that a timestep ends with: sa for every lane (the state's update waits for it),
+// and the output of the timestep BEFORE, each lane ending with row own_row(tj): that one's shuffles run beside sa's instead of
+// behind them.
+template <int ROWS>
+__device__ __forceinline__ float reduce_rows(float (&sa)[ROWS], const float (&y)[ROWS], int tj) {
+  const bool hi = tj & 4;
+  float y_row;
+  if constexpr (ROWS == 4) {
+    const bool mid = tj & 2;
+    const float s0 = hi ? y[0] : y[2], s1 = hi ? y[1] : y[3];
+    float k0 = hi ? y[2] : y[0], k1 = hi ? y[3] : y[1];
 #pragma unroll
-  for (int a = 0; a < ROWS; ++a) {
-    const float sa = ((acc[a][0].x + acc[a][0].y) + (acc[a][1].x + acc[a][1].y)) + ((acc[a][2].x + acc[a][2].y) + (acc[a][3].x + acc[a][3].y));
-    sa_out[a] = sa;
-    const float vi = buf[4][i + a * (kH / ROWS)];
-    nsa2[a] = make_float2(-sa, -sa); vi2[a] = make_float2(vi, vi);
+    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 1);
+    k0 += __shfl_xor_sync(0xffffffffu, s0, 4);
+    k1 += __shfl_xor_sync(0xffffffffu, s1, 4);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) y[a][q] = make_float2(0.f, 0.f);
+    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 2);
+    y_row = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, 2);
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 4);
+    y_row += __shfl_xor_sync(0xffffffffu, y_row, 1);
+  } else {
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 1);
+    y_row = (hi ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, hi ? y[0] : y[1], 4);
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 2);
+    y_row += __shfl_xor_sync(0xffffffffu, y_row, 2);
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 4);
+    y_row += __shfl_xor_sync(0xffffffffu, y_row, 1);
   }
+  return y_row;
+}
+template <int ROWS>
+__device__ __forceinline__ float pick_row(const float (&v)[ROWS], int a) {
+  float r = v[0];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const float4 w4 = *reinterpret_cast<const float4*>(&buf[0][4 * j]);
-    const float4 b4 = *reinterpret_cast<const float4*>(&bk[4 * j]);
-    const float4 kt4 = *reinterpret_cast<const float4*>(&buf[3][4 * j]);
-    const float4 r4 = *reinterpret_cast<const float4*>(&buf[5][4 * j]);
+  for (int k = 1; k < ROWS; ++k) r = a == k ? v[k] : r;
+  return r;
+}
+// sum over a lane's columns of S * x, row by row.  Loops over columns outside, rows inside: consecutive products share x.
+template <int ROWS>
+__device__ __forceinline__ void row_dots(const float2 (&S)[ROWS][4], const float2 (&x)[4], float (&out)[ROWS]) {
+  float2 p[ROWS], q[ROWS];
 #pragma unroll
-    for (int a = 0; a < ROWS; ++a) {
-      float2 s0 = __ffma2_rn(nsa2[a], make_float2(b4.x, b4.y), __fmul2_rn(S[a][2 * j], make_float2(w4.x, w4.y)));
-      float2 s1 = __ffma2_rn(nsa2[a], make_float2(b4.z, b4.w), __fmul2_rn(S[a][2 * j + 1], make_float2(w4.z, w4.w)));
-      s0 = __ffma2_rn(vi2[a], make_float2(kt4.x, kt4.y), s0);
-      s1 = __ffma2_rn(vi2[a], make_float2(kt4.z, kt4.w), s1);
-      S[a][2 * j] = s0; S[a][2 * j + 1] = s1;
-      y[a][(2 * j) & 3] = __ffma2_rn(s0, make_float2(r4.x, r4.y), y[a][(2 * j) & 3]);
-      y[a][(2 * j + 1) & 3] = __ffma2_rn(s1, make_float2(r4.z, r4.w), y[a][(2 * j + 1) & 3]);
-    }
-  }
+  for (int a = 0; a < ROWS; ++a) p[a] = __fmul2_rn(S[a][0], x[0]);
 #pragma unroll
-  for (int a = 0; a < ROWS; ++a)
-    y_out[a] = ((y[a][0].x + y[a][0].y) + (y[a][1].x + y[a][1].y)) + ((y[a][2].x + y[a][2].y) + (y[a][3].x + y[a][3].y));
+  for (int a = 0; a < ROWS; ++a) q[a] = __fmul2_rn(S[a][2], x[2]);
+#pragma unroll
+  for (int a = 0; a < ROWS; ++a) p[a] = __ffma2_rn(S[a][1], x[1], p[a]);
+#pragma unroll
+  for (int a = 0; a < ROWS; ++a) q[a] = __ffma2_rn(S[a][3], x[3], q[a]);
+#pragma unroll
+  for (int a = 0; a < ROWS; ++a) out[a] = (p[a].x + p[a].y) + (q[a].x + q[a].y);
 }
 
+// One timestep on a lane's tile.  In: y of the timestep before, unsummed.  Out: this one's, and the finished row of that one.
 template <int ROWS>
-__global__ void __launch_bounds__(kH / ROWS)
-wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
-  constexpr int kFwdThreads = kH / ROWS;
-  __shared__ __align__(16) float ring[kPairs][2][kVecs][kH];      // [pair slot][step of the pair][vector][channel]
-  __shared__ __align__(16) float bk[2][kH];                       // iclr * removal_k of the two steps of the current pair
-  __shared__ __align__(16) float stage[kH * kH];                  // a checkpoint on its way out
-  const int n = blockIdx.x % p.N, b = blockIdx.x / p.N;
-  const int C = p.N * kH;
-  const int i = threadIdx.x;                                      // this thread's rows: i + a * kFwdThreads
-  const size_t head_base = (size_t)b * p.T * C + (size_t)n * kH;      // element (b, t = 0, channel n*H)
-
-  // a pair of timesteps is 2 x 6 vectors x 16 chunks of 16 bytes = 192 chunks: 3 * ROWS per thread
-  auto issue = [&](int pair) {
+__device__ __forceinline__ float wkv_step(float2 (&S)[ROWS][4], StepVecs<ROWS>& x, int tj, float (&y)[ROWS], float (&sa)[ROWS]) {
+  row_dots<ROWS>(S, x.kap, sa);
+  const float y_before = reduce_rows<ROWS>(sa, y, tj);
 #pragma unroll
-    for (int c = 0; c < 3 * ROWS; ++c) {
-      const int id = c * kFwdThreads + i;                // 0 .. 191
-      const int step = id / (kVecs * (kH / 4)), vec = (id / (kH / 4)) % kVecs, chunk = id % (kH / 4);
-      const int t = 2 * pair + step;
-      if (t < p.T)
-        cp_async16((uint32_t)__cvta_generic_to_shared(&ring[pair % kPairs][step][vec][chunk * 4]),
-                   p.in[vec] + head_base + (size_t)t * C + chunk * 4);
+  for (int k = 0; k < 4; ++k) x.b[k] = __fmul2_rn(x.b[k], x.kap[k]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) S[a][k] = __fmul2_rn(S[a][k], x.w[k]);
+#pragma unroll
+  for (int a = 0; a < ROWS; ++a)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) S[a][k] = __ffma2_rn(dup(x.v[a]), x.kt[k], S[a][k]);
+#pragma unroll
+  for (int a = 0; a < ROWS; ++a) {
+    const float2 nsa = dup(-sa[a]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) S[a][k] = __ffma2_rn(nsa, x.b[k], S[a][k]);
+  }
+  row_dots<ROWS>(S, x.r, y);
+  return y_before;
+}
+
+// SAVE: checkpoints and sa are wanted (a backward pass follows).
+template <int ROWS, int WARPS, bool SAVE>
+__global__ void __launch_bounds__(32 * WARPS)
+wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
+  constexpr int kFwdThreads = 32 * WARPS;
+  constexpr int kCtaRows = 4 * ROWS * WARPS, kCtasPerHead = kH / kCtaRows;
+  __shared__ __align__(16) float ring[kFwdBufs][kFwdChunk][kVecs][kH];
+  const int head = blockIdx.x / kCtasPerHead;
+  const int n = head % p.N, b = head / p.N;
+  const int C = p.N * kH;
+  const int tid = threadIdx.x, lane = tid & 31, ti = lane >> 3, tj = lane & 7;
+  const int row0 = (blockIdx.x % kCtasPerHead) * kCtaRows + 4 * ROWS * (tid >> 5) + ROWS * ti, col0 = 4 * tj;
+  const size_t head_base = (size_t)b * p.T * C + (size_t)n * kH;      // element (b, t = 0, channel n*H)
+  const int n_chunks = (p.T + kFwdChunk - 1) / kFwdChunk;
+
+  // a chunk is 8 x 6 vectors of 16 quarters of 16 bytes; every thread commits one (possibly empty) group per call
+  auto issue = [&](int chunk) {
+    constexpr int kStepsAtOnce = kFwdThreads / 16;
+#pragma unroll
+    for (int s0 = 0; s0 < kFwdChunk; s0 += kStepsAtOnce) {
+      const int s = s0 + (tid >> 4), t = chunk * kFwdChunk + s;
+      if (t < p.T) {
+        const size_t at = head_base + (size_t)t * C + (tid & 15) * 4;
+#pragma unroll
+        for (int v = 0; v < kVecs; ++v)
+          cp_async16((uint32_t)__cvta_generic_to_shared(&ring[chunk % kFwdBufs][s][v][(tid & 15) * 4]), p.in[v] + at);
+      }
     }
-    cp_async_commit();            // every thread commits a (possibly empty) group per pair: the counts stay aligned
+    cp_async_commit();
   };
 
-  float2 S[ROWS][32];             // this thread's rows of the head's state
-  const size_t shead = ((size_t)b * p.N + n) * kH * kH;
+  float2 S[ROWS][4];
+  const size_t shead = (size_t)head * kH * kH;
 #pragma unroll
   for (int a = 0; a < ROWS; ++a) {
     if (p.state_in) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float4 s4 = __ldg(reinterpret_cast<const float4*>(p.state_in + shead + (size_t)(i + a * kFwdThreads) * kH) + j);
-        S[a][2 * j] = make_float2(s4.x, s4.y); S[a][2 * j + 1] = make_float2(s4.z, s4.w);
-      }
+      const float4 lo = __ldg(reinterpret_cast<const float4*>(p.state_in + shead + (row0 + a) * kH + col0));
+      const float4 hi = __ldg(reinterpret_cast<const float4*>(p.state_in + shead + (row0 + a) * kH + col0 + 32));
+      S[a][0] = make_float2(lo.x, lo.y); S[a][1] = make_float2(lo.z, lo.w); S[a][2] = make_float2(hi.x, hi.y); S[a][3] = make_float2(hi.z, hi.w);
     } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) S[a][j] = make_float2(0.0f, 0.0f);
+      for (int k = 0; k < 4; ++k) S[a][k] = make_float2(0.0f, 0.0f);
     }
   }
+  // of the lanes that end up with a row's y one stores it, and its neighbour sa, both a timestep late
+  constexpr int kSame = 8 / ROWS;              // lanes with the same row
+  const int own = tj / kSame, part = tj % kSame;
+  float* const out = part == 0 ? p.y : (SAVE && part == 1 ? p.sa : nullptr);
+  float* dst = out ? out + head_base + row0 + own : nullptr;
+  float y[ROWS], sa[ROWS], sa_before = 0.0f;
+#pragma unroll
+  for (int a = 0; a < ROWS; ++a) y[a] = 0.0f;
 
-  const int n_pairs = (p.T + 1) >> 1;
-  for (int pr = 0; pr < kPairs - 1; ++pr) issue(pr);
-  float* yp = p.y + head_base + i;
-  for (int pr = 0; pr < n_pairs; ++pr) {
-    cp_async_wait<kPairs - 2>();      // this thread's copies for this pair have landed
-    __syncthreads();                  // ... and everyone's; every thread is also done with the previous pair (ring slot and bk)
-    issue(pr + kPairs - 1);           // into the slot the previous pair used
-    const float (*step0)[kH] = ring[pr % kPairs][0];
-    const float (*step1)[kH] = ring[pr % kPairs][1];
+  issue(0);
+  issue(1);
+  for (int c = 0; c < n_chunks; ++c) {
+    cp_async_wait<1>();               // this thread's copies for this chunk have landed
+    __syncthreads();                  // ... and everyone's; every warp is also done with the chunk before this one
+    issue(c + 2);                     // into the buffer that chunk used
+    const float (*buf)[kVecs][kH] = ring[c % kFwdBufs];
+    if (SAVE && p.ckpt) {             // the state before the chunk (kCk == kFwdChunk), in the backward kernel's layout
+      float4* ck = p.ckpt + ((size_t)head * n_chunks + c) * kTileQuads;
 #pragma unroll
-    for (int a = 0; a < ROWS; ++a) {
-      const int r = i + a * kFwdThreads;
-      bk[0][r] = step0[1][r] * step0[2][r];
-      bk[1][r] = step1[1][r] * step1[2][r];
+      for (int a = 0; a < ROWS; a += 2)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          ck[ckpt_quad((row0 + a) >> 1, (col0 >> 1) + (k & 1) + 16 * (k >> 1))] = make_float4(S[a][k].x, S[a + 1][k].x, S[a][k].y, S[a + 1][k].y);
     }
-    __syncthreads();
-    const int t = 2 * pr;
-    if (p.ckpt && (t & (kCk - 1)) == 0) {
-      // the state before timestep t, in the backward kernel's tile layout.  A row would store 16 bytes every 2 KB; the rows
-      // go through shared memory (16-byte groups of row i at group ^ (i & 15): conflict-free) and leave in the layout's
-      // order, consecutive threads consecutive 16 bytes.
+    const int steps = min(kFwdChunk, p.T - c * kFwdChunk);
+    StepVecs<ROWS> cur;
+    cur.load(buf[0], col0, row0);
 #pragma unroll
-      for (int a = 0; a < ROWS; ++a) {
-        const int r = i + a * kFwdThreads;
-#pragma unroll
-        for (int g = 0; g < 16; ++g)
-          *reinterpret_cast<float4*>(&stage[r * kH + ((g ^ (r & 15)) << 2)]) = make_float4(S[a][2 * g].x, S[a][2 * g].y, S[a][2 * g + 1].x, S[a][2 * g + 1].y);
+    for (int s = 0; s < kFwdChunk; ++s) {
+      if (s >= steps) break;
+      StepVecs<ROWS> next;
+      if (s + 1 < kFwdChunk) next.load(buf[s + 1], col0, row0);
+      const float y_before = wkv_step<ROWS>(S, cur, tj, y, sa);
+      if (dst && (s > 0 || c > 0)) {
+        *dst = SAVE && part != 0 ? sa_before : y_before;
+        dst += C;
       }
-      __syncthreads();
-      float4* dst = p.ckpt + (((size_t)b * p.N + n) * ((p.T + kCk - 1) / kCk) + t / kCk) * kTileQuads;
-#pragma unroll
-      for (int k = 0; k < kTileQuads / kFwdThreads; ++k) {
-        const int d = k * kFwdThreads + i;              // quarter q of backward thread bt
-        const int q = d / kThreads, bt = d % kThreads;
-        const int row = 4 * kR * (bt >> 5) + kR * ((bt & 31) >> 3) + (q >> 1);
-        const int g = (bt & 7) + 8 * (q & 1);
-        dst[d] = *reinterpret_cast<const float4*>(&stage[row * kH + ((g ^ (row & 15)) << 2)]);
-      }
-      // the next write of `stage` is eight timesteps and several barriers away
-    }
-    float y0[ROWS], sa0[ROWS];
-    wkv_step<ROWS>(S, step0, bk[0], i, y0, sa0);
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) {
-      yp[(size_t)t * C + a * kFwdThreads] = y0[a];
-      if (p.sa) p.sa[head_base + (size_t)t * C + i + a * kFwdThreads] = sa0[a];
-    }
-    if (t + 1 < p.T) {
-      wkv_step<ROWS>(S, step1, bk[1], i, y0, sa0);
-#pragma unroll
-      for (int a = 0; a < ROWS; ++a) {
-        yp[(size_t)(t + 1) * C + a * kFwdThreads] = y0[a];
-        if (p.sa) p.sa[head_base + (size_t)(t + 1) * C + i + a * kFwdThreads] = sa0[a];
-      }
+      if (SAVE) sa_before = pick_row<ROWS>(sa, own);
+      if (s + 1 < kFwdChunk) cur = next;
     }
   }
+  const float y_last = reduce_rows<ROWS>(sa, y, tj);
+  if (dst) *dst = SAVE && part != 0 ? sa_before : y_last;
   cp_async_wait<0>();
   if (p.state_out) {
 #pragma unroll
-    for (int a = 0; a < ROWS; ++a)
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        reinterpret_cast<float4*>(p.state_out + shead + (size_t)(i + a * kFwdThreads) * kH)[j] =
-            make_float4(S[a][2 * j].x, S[a][2 * j].y, S[a][2 * j + 1].x, S[a][2 * j + 1].y);
+    for (int a = 0; a < ROWS; ++a) {
+      *reinterpret_cast<float4*>(p.state_out + shead + (row0 + a) * kH + col0) = make_float4(S[a][0].x, S[a][0].y, S[a][1].x, S[a][1].y);
+      *reinterpret_cast<float4*>(p.state_out + shead + (row0 + a) * kH + col0 + 32) = make_float4(S[a][2].x, S[a][2].y, S[a][3].x, S[a][3].y);
+    }
   }
+}
+
+template <int ROWS, int WARPS>
+int launch_forward(const WkvParams& p, int64_t heads, cudaStream_t st) {
+  const unsigned grid = (unsigned)(heads * (kH / (4 * ROWS * WARPS)));
+  if (p.ckpt || p.sa) wkv7_forward_kernel<ROWS, WARPS, true><<<grid, 32 * WARPS, 0, st>>>(p);
+  else                wkv7_forward_kernel<ROWS, WARPS, false><<<grid, 32 * WARPS, 0, st>>>(p);
+  PB_LAUNCH_CHECK("wkv7_forward_kernel");
+  return PB_OK;
 }
 
 // ---- backward of the scan ------------------------------------------------------------------------------------
@@ -326,19 +289,23 @@ wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
 //     dr_t   = S_t^T dy_t                    dv_t  = G_t kt_t                 dkt_t = G_t^T v_t
 //     dsa_t  = -G_t b_t   (b = a * kap)      db_t  = -G_t^T sa_t              dw_t  = sum_i G_t[i][:] * S_{t-1}[i][:]
 //     dkap_t = S_{t-1}^T dsa_t + db_t * a_t  da_t  = db_t * kap_t             dS_{t-1} = G_t diag(w_t) + dsa_t kap_t^T
-// Each lane keeps its tile of dS and, within a timestep, of S_{t-1}.  dsa is a row sum (needed at once: three
-// xor-shuffles); dv a row sum that is only written out; the other five are column sums that are only written out:
-// two shuffle levels inside the warp, then the warps' parts go to shared memory and are added after the
-// timestep's one block barrier (two buffers, by the parity of t).
+// Warp q owns rows 16q .. 16q+15; its lanes form a 2 x 16 grid and a lane keeps 8 rows (as float2 row pairs) x 4 columns of dS
+// and of S_{t-1}: per timestep it reads 4 elements of five vectors and 8 of three, and a column's sum needs one shuffle.  dsa,
+// the only sum that the recurrence waits for, is reduced first (a reduce-scatter over the sixteen lanes and eight
+// broadcasts), and everything that only leaves the kernel is formed behind it.  dr_t takes no S_t: it is
+// w o (S_{t-1}^T dy) - b (sa . dy) + kt (v . dy), a column sum of the state at hand and two dot products per timestep.
 //
 // S_{t-1} is needed for every t and is not stored by the forward pass; inverting the recurrence would divide by the
 // decay, which the reference lets go to zero.  The forward pass writes a checkpoint every kCk = 8 timesteps and
 // sa_t for every t; with sa_t known the recurrence is element-wise, so every lane recomputes its own tile of the
-// states from the checkpoint with no sums and no exchange: first the states before the chunk's last four
-// timesteps into four shared-memory slots (the lane's private 64 floats of each), those four timesteps run
-// backwards, then the states before the first four into the same slots, and those run backwards.  The chunk's
-// eight vectors per timestep arrive by cp.async one chunk ahead, and the checkpoint that the next recomputation
-// starts from by cp.async into the first slot that the timesteps before it have emptied.
+// states from the checkpoint with no sums and no exchange: first to the state before timestep 4, from where the
+// chunk's last four timesteps run backwards with three of their states in registers, then again for the first four.  The
+// column sums of four timesteps wait in shared memory for one block barrier.  The chunk's eight vectors per timestep
+// arrive by cp.async one chunk ahead, and the next checkpoint into the slot that the upper half has emptied.
+//
+// Bound by the bytes its shared-memory reads and shuffles return and by its f32x2 products, both near 1300 of the 2100 cycles
+// a timestep takes with two heads on an SM.  8 x 32 heads x 1024 timesteps 1580 -> 1121 us, 32 heads 1037 -> 646 us, against
+// 4 x 8 tiles with every state in shared memory and a barrier per timestep.
 struct WkvBwdParams {
   const float* in[kVecs];
   const float* dy;                // [B, T, C]
@@ -351,212 +318,306 @@ struct WkvBwdParams {
 };
 
 struct WkvBwdSmem {
-  float4 slot[kSub][kTileQuads];            // recomputed states, every lane its own tile
+  float4 slot[2][kTileQuads];               // every thread its own quads: the chunk's checkpoint, and the state before its timestep 4
   float vec[2][kCk][kBwdVecs][kH];          // the chunk's vectors, two chunks
-  float col_part[2][kWarps][5][kH];         // [parity of t][warp][dr, dkt, sum G sa, dw, S^T dsa][column]
+  float col_part[2][kSub][kWarps][5][kH];   // two halves of a chunk: [timestep][warp][S^T dy, dkt, sum G sa, dw, S^T dsa][column]
+  float dots[2][kCk][2];                    // of the chunk's timesteps: sa . dy and v . dy
 };
 
-__global__ void __launch_bounds__(kThreads)
+// A lane's tile: the row pairs rp of rows row0 + 2 rp, + 1 by the columns col0 + c.
+using BwdTile = float2[4][4];
+
+__device__ __forceinline__ void load_quads(const float4* base, int tid, BwdTile& S) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float4 t = base[q * kThreads + tid];
+    S[q >> 1][2 * (q & 1)] = make_float2(t.x, t.y); S[q >> 1][2 * (q & 1) + 1] = make_float2(t.z, t.w);
+  }
+}
+__device__ __forceinline__ void store_quads(float4* base, int tid, const BwdTile& S) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float2 l = S[q >> 1][2 * (q & 1)], r = S[q >> 1][2 * (q & 1) + 1];
+    base[q * kThreads + tid] = make_float4(l.x, l.y, r.x, r.y);
+  }
+}
+// eight rows' values as row pairs
+__device__ __forceinline__ void ld_rows(const float* p, float2 (&out)[4]) {
+  const float4 lo = *reinterpret_cast<const float4*>(p), hi = *reinterpret_cast<const float4*>(p + 4);
+  out[0] = make_float2(lo.x, lo.y); out[1] = make_float2(lo.z, lo.w); out[2] = make_float2(hi.x, hi.y); out[3] = make_float2(hi.z, hi.w);
+}
+// Eight row values over the sixteen lanes of a tile row: lane tj ends with the sum of row tj >> 1.
+__device__ __forceinline__ float rows_reduce_scatter(const float2 (&v)[4], int tj) {
+  const bool b3 = tj & 8, b2 = tj & 4, b1 = tj & 2;
+  float2 k0 = b3 ? v[2] : v[0], k1 = b3 ? v[3] : v[1];
+  const float2 s0 = b3 ? v[0] : v[2], s1 = b3 ? v[1] : v[3];
+  k0.x += __shfl_xor_sync(0xffffffffu, s0.x, 8); k0.y += __shfl_xor_sync(0xffffffffu, s0.y, 8);
+  k1.x += __shfl_xor_sync(0xffffffffu, s1.x, 8); k1.y += __shfl_xor_sync(0xffffffffu, s1.y, 8);
+  float2 k = b2 ? k1 : k0;
+  const float2 s = b2 ? k0 : k1;
+  k.x += __shfl_xor_sync(0xffffffffu, s.x, 4); k.y += __shfl_xor_sync(0xffffffffu, s.y, 4);
+  float r = (b1 ? k.y : k.x) + __shfl_xor_sync(0xffffffffu, b1 ? k.x : k.y, 2);
+  return r + __shfl_xor_sync(0xffffffffu, r, 1);
+}
+// Four column sums (each still as a row pair) over the two lanes of a tile column: lane ti ends with columns 2 ti, 2 ti + 1.
+__device__ __forceinline__ float2 cols_reduce_scatter(const float2 (&v)[4], int ti) {
+  const float c0 = v[0].x + v[0].y, c1 = v[1].x + v[1].y, c2 = v[2].x + v[2].y, c3 = v[3].x + v[3].y;
+  return make_float2((ti ? c2 : c0) + __shfl_xor_sync(0xffffffffu, ti ? c0 : c2, 16), (ti ? c3 : c1) + __shfl_xor_sync(0xffffffffu, ti ? c1 : c3, 16));
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
 wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
   extern __shared__ __align__(16) unsigned char wkv_bwd_smem[];
   WkvBwdSmem& sm = *reinterpret_cast<WkvBwdSmem*>(wkv_bwd_smem);
-  const Tile tl;
-  const int warp = tl.tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int ti = lane >> 4, tj = lane & 15, row0 = 16 * warp + 8 * ti, col0 = 4 * tj;
   const int n = blockIdx.x % p.N, b = blockIdx.x / p.N;
   const int C = p.N * kH;
   const size_t head_base = (size_t)b * p.T * C + (size_t)n * kH;
   const size_t head = (size_t)b * p.N + n;
   const int n_ck = (p.T + kCk - 1) / kCk;
 
-  float2 dS[kR][4];
-  if (p.dstate_out) {
-    load_tile_rowmajor(p.dstate_out + head * kH * kH, tl, dS);
-  } else {
+  BwdTile dS;
 #pragma unroll
-    for (int a = 0; a < kR; ++a)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) dS[a][k] = make_float2(0.0f, 0.0f);
+  for (int rp = 0; rp < 4; ++rp) {
+    float4 e = make_float4(0.f, 0.f, 0.f, 0.f), o = e;
+    if (p.dstate_out) {
+      e = __ldg(reinterpret_cast<const float4*>(p.dstate_out + head * kH * kH + (row0 + 2 * rp) * kH + col0));
+      o = __ldg(reinterpret_cast<const float4*>(p.dstate_out + head * kH * kH + (row0 + 2 * rp + 1) * kH + col0));
+    }
+    dS[rp][0] = make_float2(e.x, o.x); dS[rp][1] = make_float2(e.y, o.y); dS[rp][2] = make_float2(e.z, o.z); dS[rp][3] = make_float2(e.w, o.w);
   }
 
   // the eight vectors of every timestep of chunk ck -> vec[ck & 1]; every thread commits one group per call
   auto issue_vec = [&](int ck) {
     if (ck >= 0) {
-      const int t0 = ck * kCk, steps = min(kCk, p.T - t0);
-      for (int e = tl.tid; e < steps * kBwdVecs * (kH / 4); e += kThreads) {
-        const int s = e / (kBwdVecs * (kH / 4)), rem = e % (kBwdVecs * (kH / 4)), v = rem / (kH / 4), c4 = rem % (kH / 4);
-        const float* src = (v < kVecs ? p.in[v] : (v == kVecs ? p.dy : p.sa)) + head_base + (size_t)(t0 + s) * C + c4 * 4;
-        cp_async16((uint32_t)__cvta_generic_to_shared(&sm.vec[ck & 1][s][v][c4 * 4]), src);
+      const int s = tid >> 4, t = ck * kCk + s;              // a timestep per sixteen threads
+      if (t < p.T) {
+        const size_t at = head_base + (size_t)t * C + (tid & 15) * 4;
+#pragma unroll
+        for (int v = 0; v < kBwdVecs; ++v)
+          cp_async16((uint32_t)__cvta_generic_to_shared(&sm.vec[ck & 1][s][v][(tid & 15) * 4]), (v < kVecs ? p.in[v] : (v == kVecs ? p.dy : p.sa)) + at);
       }
     }
     cp_async_commit();
   };
-
-  float2 S[kR][4];                // the tile being recomputed, or S_{t-1} within a timestep
-  // The checkpoint a recomputation starts from is copied (this thread's 16 quarters of it) into a slot the walk has
-  // just emptied, well before it is needed; the thread that copies is the thread that reads, so its own
-  // cp.async wait is all the ordering this needs.
+  // checkpoint ck -> slot; the thread that copies is the thread that reads, so its own cp.async wait is all the ordering this needs
   auto prefetch_ckpt = [&](int ck, int slot) {
     if (ck >= 0) {
       const float4* src = p.ckpt + (head * n_ck + ck) * kTileQuads;
 #pragma unroll
-      for (int q = 0; q < 2 * kR; ++q)
-        cp_async16((uint32_t)__cvta_generic_to_shared(&sm.slot[slot][q * kThreads + tl.tid]), src + q * kThreads + tl.tid);
+      for (int q = 0; q < 8; ++q)
+        cp_async16((uint32_t)__cvta_generic_to_shared(&sm.slot[slot][q * kThreads + tid]), src + q * kThreads + tid);
     }
     cp_async_commit();
   };
-  // S <- S * w - sa b^T + v kt^T on the tile
-  auto update = [&](const float (*buf)[kH]) {
-    float2 kap[4], w[4], bb[4], kt[4];
-    float v[kR], sa[kR];
-    ld8(buf[2] + tl.col0, kap); ld8(buf[1] + tl.col0, bb); ld8(buf[0] + tl.col0, w); ld8(buf[3] + tl.col0, kt);
-    ldr(buf[4] + tl.row0, v); ldr(buf[kVecs + 1] + tl.row0, sa);
+  // to = from * w - sa b^T + v kt^T on the tile
+  auto update = [&](const float (*buf)[kH], const BwdTile& from, BwdTile& to) {
+    const float4 w4 = *reinterpret_cast<const float4*>(buf[0] + col0), a4 = *reinterpret_cast<const float4*>(buf[1] + col0);
+    const float4 k4 = *reinterpret_cast<const float4*>(buf[2] + col0), t4 = *reinterpret_cast<const float4*>(buf[3] + col0);
+    const float2 w[4] = {dup(w4.x), dup(w4.y), dup(w4.z), dup(w4.w)}, kt[4] = {dup(t4.x), dup(t4.y), dup(t4.z), dup(t4.w)};
+    const float2 nb[4] = {dup(-(a4.x * k4.x)), dup(-(a4.y * k4.y)), dup(-(a4.z * k4.z)), dup(-(a4.w * k4.w))};
+    float2 v[4], sa[4];
+    ld_rows(buf[4] + row0, v); ld_rows(buf[kVecs + 1] + row0, sa);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) bb[k] = __fmul2_rn(bb[k], kap[k]);
+    for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int a = 0; a < kR; ++a) {
-      const float2 nsa2 = dup(-sa[a]), v2 = dup(v[a]);
+      for (int rp = 0; rp < 4; ++rp) to[rp][c] = __fmul2_rn(from[rp][c], w[c]);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) S[a][k] = __ffma2_rn(v2, kt[k], __ffma2_rn(nsa2, bb[k], __fmul2_rn(S[a][k], w[k])));
+    for (int rp = 0; rp < 4; ++rp)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) to[rp][c] = __ffma2_rn(v[rp], kt[c], to[rp][c]);
+#pragma unroll
+    for (int rp = 0; rp < 4; ++rp)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) to[rp][c] = __ffma2_rn(sa[rp], nb[c], to[rp][c]);
+  };
+  // one timestep backwards, S the state before it
+  auto back = [&](const float (*buf)[kH], const BwdTile& S, float (*part)[kH], size_t out) {
+    float2 nb[4], kap[4], dy[4], rds[4];
+    {
+      const float4 a4 = *reinterpret_cast<const float4*>(buf[1] + col0), k4 = *reinterpret_cast<const float4*>(buf[2] + col0);
+      const float4 r4 = *reinterpret_cast<const float4*>(buf[5] + col0);
+      kap[0] = dup(k4.x); kap[1] = dup(k4.y); kap[2] = dup(k4.z); kap[3] = dup(k4.w);
+      nb[0] = dup(-(a4.x * k4.x)); nb[1] = dup(-(a4.y * k4.y)); nb[2] = dup(-(a4.z * k4.z)); nb[3] = dup(-(a4.w * k4.w));
+      const float2 r[4] = {dup(r4.x), dup(r4.y), dup(r4.z), dup(r4.w)};
+      ld_rows(buf[kVecs] + row0, dy);
+      // G = dS + dy r^T, and dsa = -G b: the only sum the recurrence waits for, so it goes first
+#pragma unroll
+      for (int rp = 0; rp < 4; ++rp)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) dS[rp][c] = __ffma2_rn(dy[rp], r[c], dS[rp][c]);
+#pragma unroll
+      for (int rp = 0; rp < 4; ++rp) rds[rp] = __fmul2_rn(dS[rp][0], nb[0]);
+#pragma unroll
+      for (int c = 1; c < 4; ++c)
+#pragma unroll
+        for (int rp = 0; rp < 4; ++rp) rds[rp] = __ffma2_rn(dS[rp][c], nb[c], rds[rp]);
+    }
+    const float dsa_row = rows_reduce_scatter(rds, tj);
+    float2 dsa[4];
+#pragma unroll
+    for (int rp = 0; rp < 4; ++rp) {
+      dsa[rp].x = __shfl_sync(0xffffffffu, dsa_row, (lane & 16) + 4 * rp);
+      dsa[rp].y = __shfl_sync(0xffffffffu, dsa_row, (lane & 16) + 4 * rp + 2);
+    }
+    const int col = col0 + 2 * ti;
+    // the sums that only leave: dv along the rows, the others along the columns
+    {
+      float2 v[4], sum[4], dvp[4];
+      ld_rows(buf[4] + row0, v);
+      const float4 t4 = *reinterpret_cast<const float4*>(buf[3] + col0);
+      const float2 kt[4] = {dup(t4.x), dup(t4.y), dup(t4.z), dup(t4.w)};
+#pragma unroll
+      for (int rp = 0; rp < 4; ++rp) dvp[rp] = __fmul2_rn(dS[rp][0], kt[0]);
+#pragma unroll
+      for (int c = 1; c < 4; ++c)
+#pragma unroll
+        for (int rp = 0; rp < 4; ++rp) dvp[rp] = __ffma2_rn(dS[rp][c], kt[c], dvp[rp]);
+      const float dv = rows_reduce_scatter(dvp, tj);
+      if (!(tj & 1)) p.din[4][out + row0 + (tj >> 1)] = dv;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(dS[0][c], v[0]);
+#pragma unroll
+      for (int rp = 1; rp < 4; ++rp)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(dS[rp][c], v[rp], sum[c]);
+      *reinterpret_cast<float2*>(part[1] + col) = cols_reduce_scatter(sum, ti);
+    }
+    {
+      float2 sa[4], sum[4];
+      ld_rows(buf[kVecs + 1] + row0, sa);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(dS[0][c], sa[0]);
+#pragma unroll
+      for (int rp = 1; rp < 4; ++rp)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(dS[rp][c], sa[rp], sum[c]);
+      *reinterpret_cast<float2*>(part[2] + col) = cols_reduce_scatter(sum, ti);
+    }
+    {
+      float2 sum[4], dw[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(S[0][c], dy[0]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) dw[c] = __fmul2_rn(S[0][c], dS[0][c]);
+#pragma unroll
+      for (int rp = 1; rp < 4; ++rp) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(S[rp][c], dy[rp], sum[c]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) dw[c] = __ffma2_rn(S[rp][c], dS[rp][c], dw[c]);
+      }
+      *reinterpret_cast<float2*>(part[0] + col) = cols_reduce_scatter(sum, ti);
+      *reinterpret_cast<float2*>(part[3] + col) = cols_reduce_scatter(dw, ti);
+    }
+    {
+      const float4 w4 = *reinterpret_cast<const float4*>(buf[0] + col0);
+      const float2 w[4] = {dup(w4.x), dup(w4.y), dup(w4.z), dup(w4.w)};
+      float2 sum[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int rp = 0; rp < 4; ++rp) dS[rp][c] = __fmul2_rn(dS[rp][c], w[c]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(S[0][c], dsa[0]);
+#pragma unroll
+      for (int rp = 0; rp < 4; ++rp) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) dS[rp][c] = __ffma2_rn(dsa[rp], kap[c], dS[rp][c]);
+        if (rp > 0) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(S[rp][c], dsa[rp], sum[c]);
+        }
+      }
+      *reinterpret_cast<float2*>(part[4] + col) = cols_reduce_scatter(sum, ti);
     }
   };
-
-  // Timesteps hi-1 .. lo of the chunk at t0 backwards; the state before local timestep s is in slot (s - lo + shift) & 3.
-  // The slot of the first timestep is free as soon as its tile is in registers: checkpoint `next_ck` goes there.
-  auto run_backwards = [&](const float (*V)[kBwdVecs][kH], int t0, int lo, int hi, int shift, int next_ck) {
-    for (int s = hi - 1; s >= lo; --s) {
-      const float (*buf)[kH] = V[s];
-      const int slot = (s - lo + shift) & (kSub - 1);
-      load_tile_private(sm.slot[slot], tl, S);
-      if (s == hi - 1) prefetch_ckpt(next_ck, slot);
-      float dy[kR], v[kR], sa[kR];
-      ldr(buf[kVecs] + tl.row0, dy); ldr(buf[4] + tl.row0, v); ldr(buf[kVecs + 1] + tl.row0, sa);
-      float dvp[kR], dsp[kR];
+  // The column sums of the half chunk's timesteps [lo, hi): every warp's part is in shared memory behind the barrier.  (The
+  // other buffer is written by the next half, and this one again only behind that half's barrier.)
+  auto finish_columns = [&](const float (*V)[kBwdVecs][kH], const float (*dots)[2], const float (*part)[kWarps][5][kH], int t0, int lo, int hi) {
+    __syncthreads();
+    const int j = tid & (kH - 1);
+    for (int s = lo + (tid >> 6); s < hi; s += 2) {
+      float sum[5];
 #pragma unroll
-      for (int a = 0; a < kR; ++a) { dvp[a] = 0.f; dsp[a] = 0.f; }
-      const int par = (t0 + s) & 1;
-      float (*cp)[kH] = sm.col_part[par][warp];
-      // first pass over the tile, four columns at a time: G, the row sums' parts, four of the five column sums
+      for (int q = 0; q < 5; ++q) {
+        sum[q] = part[s - lo][0][q][j];
 #pragma unroll
-      for (int hc = 0; hc < 2; ++hc) {
-        float2 w[2], bb[2], kap[2], kt[2], r[2];
-        {
-          const int c = tl.col0 + 32 * hc;
-          const float4 w4 = *reinterpret_cast<const float4*>(buf[0] + c), a4 = *reinterpret_cast<const float4*>(buf[1] + c);
-          const float4 k4 = *reinterpret_cast<const float4*>(buf[2] + c), kt4 = *reinterpret_cast<const float4*>(buf[3] + c);
-          const float4 r4 = *reinterpret_cast<const float4*>(buf[5] + c);
-          w[0] = make_float2(w4.x, w4.y); w[1] = make_float2(w4.z, w4.w);
-          kap[0] = make_float2(k4.x, k4.y); kap[1] = make_float2(k4.z, k4.w);
-          bb[0] = __fmul2_rn(make_float2(a4.x, a4.y), kap[0]); bb[1] = __fmul2_rn(make_float2(a4.z, a4.w), kap[1]);
-          kt[0] = make_float2(kt4.x, kt4.y); kt[1] = make_float2(kt4.z, kt4.w);
-          r[0] = make_float2(r4.x, r4.y); r[1] = make_float2(r4.z, r4.w);
-        }
-        float2 dr[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, dkt[2] = {dr[0], dr[0]}, db[2] = {dr[0], dr[0]}, dw[2] = {dr[0], dr[0]};
-#pragma unroll
-        for (int a = 0; a < kR; ++a) {
-          const float2 dy2 = dup(dy[a]), v2 = dup(v[a]), sa2 = dup(sa[a]), nsa2 = dup(-sa[a]);
-          float2 rdv = make_float2(0.f, 0.f), rds = rdv;
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const float2 sp = S[a][2 * hc + k];
-            const float2 g = __ffma2_rn(dy2, r[k], dS[a][2 * hc + k]);
-            dS[a][2 * hc + k] = g;
-            rdv = __ffma2_rn(g, kt[k], rdv);
-            rds = __ffma2_rn(g, bb[k], rds);
-            const float2 st = __ffma2_rn(v2, kt[k], __ffma2_rn(nsa2, bb[k], __fmul2_rn(sp, w[k])));
-            dr[k] = __ffma2_rn(st, dy2, dr[k]);
-            dkt[k] = __ffma2_rn(g, v2, dkt[k]);
-            db[k] = __ffma2_rn(g, sa2, db[k]);
-            dw[k] = __ffma2_rn(g, sp, dw[k]);
-          }
-          dvp[a] += rdv.x + rdv.y;
-          dsp[a] += rds.x + rds.y;
-        }
-        const int col = tl.col0 + 32 * hc + tl.ti;
-        cp[0][col] = col_reduce_scatter(dr, tl.ti);
-        cp[1][col] = col_reduce_scatter(dkt, tl.ti);
-        cp[2][col] = col_reduce_scatter(db, tl.ti);
-        cp[3][col] = col_reduce_scatter(dw, tl.ti);
+        for (int w = 1; w < kWarps; ++w) sum[q] += part[s - lo][w][q][j];
       }
-      row_allreduce(dsp);         // dsp[a] = sum_j G b of row row0 + a; dsa = -dsp
-      const size_t out = head_base + (size_t)(t0 + s) * C;
-      row_allreduce(dvp);
-      if (tl.tj < kR) p.din[4][out + tl.row0 + tl.tj] = pick(dvp, tl.tj);
-      // second pass: S_{t-1}^T dsa and dS_{t-1}
-#pragma unroll
-      for (int hc = 0; hc < 2; ++hc) {
-        const int c = tl.col0 + 32 * hc;
-        const float4 w4 = *reinterpret_cast<const float4*>(buf[0] + c), k4 = *reinterpret_cast<const float4*>(buf[2] + c);
-        const float2 w[2] = {make_float2(w4.x, w4.y), make_float2(w4.z, w4.w)};
-        const float2 kap[2] = {make_float2(k4.x, k4.y), make_float2(k4.z, k4.w)};
-        float2 dk[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-        for (int a = 0; a < kR; ++a) {
-          const float2 dsa2 = dup(-dsp[a]);
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            dk[k] = __ffma2_rn(S[a][2 * hc + k], dsa2, dk[k]);
-            dS[a][2 * hc + k] = __ffma2_rn(dsa2, kap[k], __fmul2_rn(dS[a][2 * hc + k], w[k]));
-          }
-        }
-        cp[4][c + tl.ti] = col_reduce_scatter(dk, tl.ti);
-      }
-      // the five column sums of this timestep: each warp's half is in shared memory after the barrier; thread j adds column j.
-      // (The buffer of the other parity is written by the next timestep, and this one again only after the next barrier.)
-      const int j = tl.tid & (kH - 1);
-      const float kap_j = buf[2][j], a_j = buf[1][j];
-      __syncthreads();
-      if (tl.tid < kH) {
-        float sum[5];
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-          sum[q] = sm.col_part[par][0][q][j];
-#pragma unroll
-          for (int w = 1; w < kWarps; ++w) sum[q] += sm.col_part[par][w][q][j];
-        }
-        p.din[5][out + j] = sum[0];
-        p.din[3][out + j] = sum[1];
-        p.din[0][out + j] = sum[3];
-        p.din[1][out + j] = -sum[2] * kap_j;
-        p.din[2][out + j] = sum[4] - sum[2] * a_j;
-      }
+      const size_t out = head_base + (size_t)(t0 + s) * C + j;
+      const float w = V[s][0][j], a = V[s][1][j], kap = V[s][2][j], kt = V[s][3][j];
+      p.din[5][out] = fmaf(kt, dots[s][1], fmaf(-(a * kap), dots[s][0], w * sum[0]));      // S_t^T dy with S_t = S_{t-1} w - sa b^T + v kt^T
+      p.din[3][out] = sum[1];
+      p.din[0][out] = sum[3];
+      p.din[1][out] = -sum[2] * kap;
+      p.din[2][out] = sum[4] - sum[2] * a;
     }
+  };
+  // Timesteps lo .. lo + count - 1 backwards, `first` holding the state before lo; the later ones' states stay in registers.
+  auto run_half = [&](const float (*V)[kBwdVecs][kH], const float4* first, int t0, int lo, int count, int half, BwdTile& S1) {
+    float (*part)[kWarps][5][kH] = sm.col_part[half];
+    const size_t out = head_base + (size_t)(t0 + lo) * C;
+    BwdTile S2, S3;                   // S1 comes as the state before lo
+    if (count > 1) update(V[lo], S1, S1);
+    if (count > 2) update(V[lo + 1], S1, S2);
+    if (count > 3) {
+      update(V[lo + 2], S2, S3);
+      back(V[lo + 3], S3, part[3][warp], out + 3 * (size_t)C);
+    }
+    if (count > 2) back(V[lo + 2], S2, part[2][warp], out + 2 * (size_t)C);
+    if (count > 1) back(V[lo + 1], S1, part[1][warp], out + (size_t)C);
+    load_quads(first, tid, S1);
+    back(V[lo], S1, part[0][warp], out);
   };
 
   issue_vec(n_ck - 1);
-  int pre_slot = 0;               // the slot that holds the checkpoint the next recomputation starts from
-  prefetch_ckpt(n_ck - 1, pre_slot);
+  int ck_slot = 0;                // the slot of the current chunk's checkpoint; the other takes the state before timestep 4
+  prefetch_ckpt(n_ck - 1, ck_slot);
   for (int ck = n_ck - 1; ck >= 0; --ck) {
     const int t0 = ck * kCk, steps = min(kCk, p.T - t0);
-    const int lo = steps > kSub ? kSub : 0;      // the chunk runs as [lo, steps) and then, if lo > 0, [0, lo)
     __syncthreads();              // everyone is done with the vectors of the chunk after this one
     issue_vec(ck - 1);            // into the buffer that chunk used
     cp_async_wait<1>();           // this thread's copies of chunk ck, and of its checkpoint, have landed
     __syncthreads();              // ... and everyone's vectors
     const float (*V)[kBwdVecs][kH] = sm.vec[ck & 1];
-    load_tile_private(sm.slot[pre_slot], tl, S);
-    for (int s = 0; s < steps; ++s) {            // the states before timesteps lo .. steps-1 -> slots 0 ..
-      if (s >= lo) store_tile_private(sm.slot[s - lo], tl, S);
-      if (s + 1 < steps) update(V[s]);
+    float (*dots)[2] = sm.dots[ck & 1];
+    {                             // sa . dy and v . dy of the eight timesteps, eight threads each (of a timestep past the end: never read)
+      const int d = tid >> 3, s = d >> 1, e = (tid & 7) * 8;
+      const float* l = V[s][d & 1 ? 4 : kVecs + 1] + e;
+      const float* r = V[s][kVecs] + e;
+      float sum = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum = fmaf(l[k], r[k], sum);
+#pragma unroll
+      for (int m = 1; m < 8; m <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+      if ((tid & 7) == 0) dots[s][d & 1] = sum;
     }
-    if (lo > 0) {
-      run_backwards(V, t0, lo, steps, 0, ck);    // its first timestep empties slot steps-1-lo: this chunk's checkpoint goes there again
-      pre_slot = steps - 1 - lo;
-      cp_async_wait<0>();
-      load_tile_private(sm.slot[pre_slot], tl, S);
-      // the states before timesteps 0 .. lo-1 -> slots pre_slot, pre_slot+1, ... (mod 4): the first is there already
-      for (int s = 0; s + 1 < lo; ++s) {
-        update(V[s]);
-        store_tile_private(sm.slot[(s + 1 + pre_slot) & (kSub - 1)], tl, S);
-      }
-      run_backwards(V, t0, 0, lo, pre_slot, ck - 1);
-      pre_slot = (lo - 1 + pre_slot) & (kSub - 1);
-    } else {
-      run_backwards(V, t0, 0, steps, 0, ck - 1);
-      pre_slot = steps - 1;
+    BwdTile S;
+    load_quads(sm.slot[ck_slot], tid, S);
+    if (steps > kSub) {
+#pragma unroll
+      for (int s = 0; s < kSub; ++s) update(V[s], S, S);
+      store_quads(sm.slot[ck_slot ^ 1], tid, S);
+      run_half(V, sm.slot[ck_slot ^ 1], t0, kSub, steps - kSub, 1, S);
+      finish_columns(V, dots, sm.col_part[1], t0, kSub, steps);
+      load_quads(sm.slot[ck_slot], tid, S);
     }
+    prefetch_ckpt(ck - 1, ck_slot ^ 1);       // that slot's state has been read
+    run_half(V, sm.slot[ck_slot], t0, 0, min(steps, kSub), 0, S);
+    finish_columns(V, dots, sm.col_part[0], t0, 0, min(steps, kSub));
+    ck_slot ^= 1;
   }
   cp_async_wait<0>();
-  if (p.dstate_in) store_tile_rowmajor(p.dstate_in + head * kH * kH, tl, dS);
+  if (p.dstate_in) {
+#pragma unroll
+    for (int rp = 0; rp < 4; ++rp) {
+      float* m = p.dstate_in + head * kH * kH + (row0 + 2 * rp) * kH + col0;
+      *reinterpret_cast<float4*>(m) = make_float4(dS[rp][0].x, dS[rp][1].x, dS[rp][2].x, dS[rp][3].x);
+      *reinterpret_cast<float4*>(m + kH) = make_float4(dS[rp][0].y, dS[rp][1].y, dS[rp][2].y, dS[rp][3].y);
+    }
+  }
 }
 
 }  // namespace
@@ -577,9 +638,12 @@ extern "C" int pb_wkv7_forward(const float* decay, const float* iclr, const floa
   for (const void* ptr : ptrs)
     if (reinterpret_cast<uintptr_t>(ptr) & 15) return fail(PB_ERR_MISALIGNED, "pb_wkv7_forward: every array must be 16-byte aligned");
   WkvParams p{{decay, iclr, removal_k, replacement_k, v, r}, state_in, y, state_out, reinterpret_cast<float4*>(checkpoints), sa, (int)steps, (int)heads};
-  wkv7_forward_kernel<kFwdRows><<<(unsigned)(batch * heads), kH / kFwdRows, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  PB_LAUNCH_CHECK("wkv7_forward_kernel");
-  return PB_OK;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // 16, 32 or 64 rows of a head per CTA: as many CTAs as there are SMs, and no more of them on one (each reads the head's vectors)
+  const int64_t n = batch * heads;
+  if (4 * n <= sm_count()) return launch_forward<2, 2>(p, n, st);
+  if (2 * n <= sm_count()) return launch_forward<2, 4>(p, n, st);
+  return launch_forward<4, 4>(p, n, st);
 }
 
 extern "C" size_t pb_wkv7_checkpoint_floats(int64_t batch, int64_t steps, int64_t heads, int head_dim) {

@@ -1,0 +1,43 @@
+"""The scan's two forward layouts (16 rows of a head per CTA for few heads, a whole head for many) and the backward kernel's half
+chunks, over lengths around the chunk of eight, against the recurrence in 64 bits."""
+import pytest
+import torch
+
+from pratchya_b200._nnx_impl._wkv7 import wkv_state_scan
+
+pytestmark = pytest.mark.gpu
+
+
+def _recurrence(state, ins, n):
+    b, t, c = ins[0].shape
+    w, a, kap, kt, v, r = (x.reshape(b, t, n, 64) for x in ins)
+    ys = []
+    for i in range(t):
+        sa = torch.einsum("bnij,bnj->bni", state, kap[:, i])
+        state = state * w[:, i].unsqueeze(-2) - sa.unsqueeze(-1) * (a[:, i] * kap[:, i]).unsqueeze(-2) + v[:, i].unsqueeze(-1) * kt[:, i].unsqueeze(-2)
+        ys.append(torch.einsum("bnij,bnj->bni", state, r[:, i]))
+    return state, torch.stack(ys, 1).reshape(b, t, c)
+
+
+@pytest.mark.parametrize("batch,steps,heads", [(1, 1, 1), (1, 2, 3), (2, 8, 2), (1, 9, 2), (1, 17, 5), (3, 24, 32), (4, 12, 33), (1, 13, 130)])
+@pytest.mark.parametrize("with_grad", [False, True])
+def test_scan_against_the_recurrence(built_lib, batch, steps, heads, with_grad):
+    g = torch.Generator(device="cuda").manual_seed(steps * 100 + heads)
+    rn = lambda: torch.randn(batch, steps, heads * 64, generator=g, device="cuda")
+    k = rn()
+    kap = torch.nn.functional.normalize(k.view(batch, steps, heads, 64), dim=-1).reshape(k.shape)
+    ins = [torch.exp(-torch.exp(rn() - 2)), torch.sigmoid(rn()), kap, k, rn(), rn()]
+    state = torch.randn(batch, heads, 64, 64, generator=g, device="cuda") * 0.3
+    leaves = [t.clone().requires_grad_(with_grad) for t in (state, *ins)]
+    s_out, y = wkv_state_scan(leaves[0], *leaves[1:], heads)
+    ref = [t.double().requires_grad_(with_grad) for t in (state, *ins)]
+    s_ref, y_ref = _recurrence(ref[0], ref[1:], heads)
+    # 64-term f32 sums of values of this size, their errors carried over `steps` contracting updates: 1e-7 observed, 64 * 2^-24 allowed
+    close = lambda got, want: (got.double() - want).abs().max() <= 4e-6 * want.abs().max()
+    assert close(s_out.detach(), s_ref.detach()) and close(y.detach(), y_ref.detach())
+    if with_grad:
+        gy, gs = rn(), torch.randn_like(state)
+        got = torch.autograd.grad((y, s_out), leaves, (gy, gs))
+        want = torch.autograd.grad((y_ref, s_ref), ref, (gy.double(), gs.double()))
+        for name, u, v in zip(("state", "decay", "iclr", "removal_k", "replacement_k", "v", "r"), got, want):
+            assert (u.double() - v).abs().max() <= 2e-5 * v.abs().max(), name
