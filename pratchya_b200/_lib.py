@@ -5,8 +5,11 @@ usable, the ops raise.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 from pathlib import Path
+
+import torch
 
 _LIB_PATH = Path(__file__).resolve().parent / "csrc" / "libpratchya_b200.so"
 _DIAG_LIB_PATH = Path(__file__).resolve().parent / "csrc" / "libpratchya_b200_diag.so"
@@ -132,6 +135,19 @@ def load_diagnostics():
     if _diag_lib is None:
         _diag_lib = _open(_DIAG_LIB_PATH, {**_SIGNATURES, **_DIAG_SIGNATURES})
     return _diag_lib
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def on_device(device):
+    """`torch.cuda.device(device)` where that is not the current device already: the usual case costs a comparison."""
+    return _SAME_DEVICE if torch._C._cuda_getDevice() == device.index else torch.cuda.device(device)
+
+
+def current_stream(device) -> int:
+    """The current torch stream of a CUDA tensor's device, as the C ABI takes it (no Stream object in between)."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
 
 
 def check(status: int):

@@ -17,7 +17,7 @@ def _f32c(t):
 
 
 def _stream(dev):
-    return torch.cuda.current_stream(dev).cuda_stream
+    return _lib.current_stream(dev)
 
 
 class _ShiftLerpFn(torch.autograd.Function):
@@ -27,7 +27,7 @@ class _ShiftLerpFn(torch.autograd.Function):
         bsz, steps, chans = x.shape
         n_mix = mu.shape[0]
         out = torch.empty((n_mix, bsz, steps, chans), dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
+        with _lib.on_device(x.device):
             check(lib.pb_token_shift_lerp(x.data_ptr(), state.data_ptr() if state is not None else None, mu.data_ptr(),
                                           bsz, steps, chans, n_mix, out.data_ptr(), _stream(x.device)))
         ctx.save_for_backward(x, state, mu)
@@ -40,7 +40,7 @@ class _ShiftLerpFn(torch.autograd.Function):
         bsz, steps, chans = x.shape
         n_mix = mu.shape[0]
         dev = x.device
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             gs = [_f32c(g) if g is not None else torch.zeros_like(x) for g in gs]
             g_ptrs = (C.c_void_p * n_mix)(*[g.data_ptr() for g in gs])
             dx = torch.empty_like(x)
@@ -93,7 +93,7 @@ class _ShiftLerpQuantFn(torch.autograd.Function):
         n_t = bin(mask).count("1")
         dev = x.device
         groups = rows * chans // 1024
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             q = torch.empty((n_mix, rows, chans), dtype=torch.float8_e4m3fn, device=dev)
             sc8 = torch.empty((n_mix, groups, 8), dtype=torch.float8_e8m0fnu, device=dev)
             sc32 = torch.empty((n_mix, groups, 1, 1), dtype=torch.float32, device=dev)
@@ -159,7 +159,7 @@ class _WkvPrepareFn(torch.autograd.Function):
         lib = _lib.load()
         bsz, steps, chans = r_raw.shape
         outs = [torch.empty_like(r_raw) for _ in range(7)]
-        with torch.cuda.device(r_raw.device):
+        with _lib.on_device(r_raw.device):
             check(lib.pb_wkv_prepare(r_raw.data_ptr(), k_raw.data_ptr(), d.data_ptr(), iclr_raw.data_ptr(), v_prime.data_ptr(),
                                      v0.data_ptr() if v0 is not None else None, nu_raw.data_ptr() if nu_raw is not None else None,
                                      cos_tab.data_ptr(), sin_tab.data_ptr(), rk_mult.data_ptr(), mix_amt.data_ptr(),
@@ -175,7 +175,7 @@ class _WkvPrepareFn(torch.autograd.Function):
         bsz, steps, chans = r_raw.shape
         n_head = ctx.n_head
         dev = r_raw.device
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             gs = [_f32c(g) if g is not None else torch.zeros_like(r_raw) for g in grads]
             douts = [torch.empty_like(r_raw) for _ in range(5)]
             d_v0 = torch.empty_like(r_raw) if v0 is not None else None
@@ -221,7 +221,7 @@ class _RmsNormFn(torch.autograd.Function):
         rows = x.numel() // chans
         y = torch.empty_like(x)
         inv = torch.empty(rows, dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
+        with _lib.on_device(x.device):
             check(lib.pb_rms_norm(x.data_ptr(), scale.data_ptr(), rows, chans, eps, y.data_ptr(), inv.data_ptr(), _stream(x.device)))
         ctx.save_for_backward(x, scale, inv)
         return y
@@ -234,7 +234,7 @@ class _RmsNormFn(torch.autograd.Function):
         rows = x.numel() // chans
         dy = _f32c(dy)
         dev = x.device
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             dx, dscale = torch.empty_like(x), torch.empty_like(scale)
             ws_bytes = lib.pb_rms_norm_bwd_workspace_size(rows, chans)
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
@@ -258,7 +258,7 @@ class _Relu2Fn(torch.autograd.Function):
     def forward(ctx, x):
         lib = _lib.load()
         y = torch.empty_like(x)
-        with torch.cuda.device(x.device):
+        with _lib.on_device(x.device):
             check(lib.pb_relu2(x.data_ptr(), x.numel(), y.data_ptr(), _stream(x.device)))
         ctx.save_for_backward(x)
         return y
@@ -269,7 +269,7 @@ class _Relu2Fn(torch.autograd.Function):
         lib = _lib.load()
         g = _f32c(g)
         dx = torch.empty_like(x)
-        with torch.cuda.device(x.device):
+        with _lib.on_device(x.device):
             check(lib.pb_relu2_bwd(g.data_ptr(), x.data_ptr(), x.numel(), dx.data_ptr(), _stream(x.device)))
         return dx
 
@@ -289,7 +289,7 @@ class _Relu2QuantFn(torch.autograd.Function):
         rows = k.numel() // cols
         groups = rows * cols // 1024
         dev = k.device
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             q = torch.empty((rows, cols), dtype=torch.float8_e4m3fn, device=dev)
             sc8 = torch.empty((groups, 8), dtype=torch.float8_e8m0fnu, device=dev)
             sc32 = torch.empty((groups, 1, 1), dtype=torch.float32, device=dev)
@@ -333,7 +333,7 @@ class _WkvFinishFn(torch.autograd.Function):
         dev = y.device
         out = torch.empty_like(y)
         stats = torch.empty((bsz * n_head, 2), dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             ws_bytes = lib.pb_wkv_finish_workspace_size(bsz, steps, n_head, chans // n_head)
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
             check(lib.pb_wkv_finish(y.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), gate.data_ptr(), gn_scale.data_ptr(),
@@ -351,7 +351,7 @@ class _WkvFinishFn(torch.autograd.Function):
         n_head = ctx.n_head
         dev = y.device
         g = _f32c(g)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             d_y, d_r, d_k, d_v, d_gate = (torch.empty_like(y) for _ in range(5))
             d_gs, d_gb, d_bm = torch.empty_like(gn_scale), torch.empty_like(gn_bias), torch.empty_like(bonus_mult)
             ws_bytes = lib.pb_wkv_finish_bwd_workspace_size(bsz, steps, n_head, chans // n_head)
@@ -386,7 +386,7 @@ class _SmoothedXentFn(torch.autograd.Function):
         dev = logits.device
         row_loss = torch.empty(rows, dtype=torch.float32, device=dev)
         lse = torch.empty(rows, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             check(lib.pb_smoothed_xent(logits.data_ptr(), target.data_ptr(), weight.data_ptr(), rows, vocab, alpha,
                                        row_loss.data_ptr(), lse.data_ptr(), _stream(dev)))
         ctx.save_for_backward(logits, target, weight, lse)
@@ -402,7 +402,7 @@ class _SmoothedXentFn(torch.autograd.Function):
         g = g.to(torch.float32).reshape(1).contiguous()
         # every element of the cotangent depends on its own logit only: with reuse_logits it is written over the logits
         dlogits = logits if ctx.reuse_logits else torch.empty_like(logits)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             check(lib.pb_smoothed_xent_bwd(logits.data_ptr(), target.data_ptr(), weight.data_ptr(), lse.data_ptr(), g.data_ptr(),
                                            ctx.denominator, rows, vocab, ctx.alpha, dlogits.data_ptr(), _stream(dev)))
         return dlogits, None, None, None, None, None

@@ -37,7 +37,7 @@ def momentum_update(g: QArrayImpl, m: QArrayImpl, beta1: float, beta2: float):
     g8, g32 = g.sc_fp8.contiguous(), g.sc_fp32.contiguous()
     m8, m32 = m.sc_fp8.contiguous(), m.sc_fp32.contiguous()
     f32 = lambda v: float(np.float32(v))
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         c = torch.empty(shape, dtype=torch.float32, device=dev)
         nq = torch.empty(shape, dtype=torch.float8_e4m3fn, device=dev)
         n8 = torch.empty_like(m8)
@@ -47,7 +47,7 @@ def momentum_update(g: QArrayImpl, m: QArrayImpl, beta1: float, beta2: float):
         check(lib.pb_momentum_update(gq.data_ptr(), g8.data_ptr(), g32.data_ptr(), mq.data_ptr(), m8.data_ptr(), m32.data_ptr(),
                                      batch, rows, cols, a, b, f32(beta1), f32(1.0 - beta1), f32(beta2), f32(1.0 - beta2),
                                      c.data_ptr(), nq.data_ptr(), n8.data_ptr(), n32.data_ptr(), ws.data_ptr(), ws_bytes,
-                                     torch.cuda.current_stream(dev).cuda_stream))
+                                     _lib.current_stream(dev)))
     return c, QArrayImpl.from_triple(nq, n8, n32, (a, b))
 
 
@@ -75,7 +75,7 @@ def momentum_update_stacked(g: QArrayImpl, m: QArrayImpl, beta1: float, beta2: f
     dev = mq.device
     g8, g32 = g.sc_fp8.contiguous(), g.sc_fp32.contiguous()
     m8, m32 = m.sc_fp8.contiguous(), m.sc_fp32.contiguous()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         c = torch.empty((layers, rows, cols), dtype=torch.bfloat16, device=dev)
         nq = torch.empty((layers, rows, cols), dtype=torch.float8_e4m3fn, device=dev)
         n8 = torch.empty_like(m8)
@@ -86,7 +86,7 @@ def momentum_update_stacked(g: QArrayImpl, m: QArrayImpl, beta1: float, beta2: f
                                              layers, rows, cols, a, b, _bf16_scalar(beta1), _bf16_scalar(1.0 - beta1),
                                              _bf16_scalar(beta2), _bf16_scalar(1.0 - beta2),
                                              c.data_ptr(), nq.data_ptr(), n8.data_ptr(), n32.data_ptr(), ws.data_ptr(), ws_bytes,
-                                             torch.cuda.current_stream(dev).cuda_stream))
+                                             _lib.current_stream(dev)))
     return c, QArrayImpl.from_triple(nq, n8, n32, (a, b))
 
 

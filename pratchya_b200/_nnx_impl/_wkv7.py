@@ -27,7 +27,7 @@ def _forward(state_in, ins, n_head, want_checkpoints):
     head_dim = chans // n_head
     dev = ins[0].device
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         out = torch.empty((bsz, steps, chans), dtype=torch.float32, device=dev)
         state_out = torch.empty((bsz, n_head, head_dim, head_dim), dtype=torch.float32, device=dev)
         ckpt = sa = None
@@ -40,7 +40,7 @@ def _forward(state_in, ins, n_head, want_checkpoints):
         check(lib.pb_wkv7_forward(*[t.data_ptr() for t in ins], state_in.data_ptr() if state_in is not None else None,
                                   bsz, steps, n_head, head_dim, out.data_ptr(), state_out.data_ptr(),
                                   ckpt.data_ptr() if ckpt is not None else None, sa.data_ptr() if sa is not None else None,
-                                  torch.cuda.current_stream(dev).cuda_stream))
+                                  _lib.current_stream(dev)))
     return state_out, out, ckpt, sa
 
 
@@ -61,7 +61,7 @@ class _WkvScanFn(torch.autograd.Function):
         head_dim = chans // n_head
         dev = ins[0].device
         lib = _lib.load()
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             d_out = d_out.to(torch.float32).contiguous() if d_out is not None else torch.zeros_like(ins[0])
             d_state = d_state_out.to(torch.float32).contiguous() if d_state_out is not None else None
             grads = [torch.empty_like(ins[0]) for _ in range(6)]
@@ -70,7 +70,7 @@ class _WkvScanFn(torch.autograd.Function):
                                        d_state.data_ptr() if d_state is not None else None,
                                        bsz, steps, n_head, head_dim, *[g.data_ptr() for g in grads],
                                        d_state_in.data_ptr() if d_state_in is not None else None,
-                                       torch.cuda.current_stream(dev).cuda_stream))
+                                       _lib.current_stream(dev)))
         return (d_state_in, *grads, None)
 
 

@@ -35,7 +35,7 @@ def group_geometry(rows: int, cols: int, tgrid) -> Tuple[int, int]:
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _lib.current_stream(t.device)
 
 
 def _require_cuda(t: torch.Tensor, what: str):
@@ -75,7 +75,7 @@ def quantize_impl(x: torch.Tensor, tgrid=(128, 128), out_format: str = "e4m3"):
     lead = shape[:-2]
     batch = math.prod(lead)
     x = _dense_input(x)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         q = torch.empty(orig_shape, dtype=_FMT_DTYPE[out_format], device=x.device)
         sc8 = torch.empty((*lead, m, k), dtype=E8M0, device=x.device)
         sc32 = torch.empty((*lead, m, 1, 1), dtype=torch.float32, device=x.device)
@@ -101,7 +101,7 @@ def quantize_transposed_impl(x: torch.Tensor, b: int = 128, out_format: str = "e
     batch = math.prod(lead)
     m, k = group_geometry(cols, rows, (1, b))
     x = _dense_input(x)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         q = torch.empty((*lead, cols, rows), dtype=_FMT_DTYPE[out_format], device=x.device)
         sc8 = torch.empty((*lead, m, k), dtype=E8M0, device=x.device)
         sc32 = torch.empty((*lead, m, 1, 1), dtype=torch.float32, device=x.device)
@@ -132,7 +132,7 @@ def quantize_dual_impl(x: torch.Tensor, out_format: str = "e4m3"):
     mt, kt = group_geometry(cols, rows, (1, 128))
     x = x.contiguous()
     dev = x.device
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         fmt = _FMT_DTYPE[out_format]
         q = torch.empty(tuple(x.shape), dtype=fmt, device=dev)
         sc8 = torch.empty((*lead, m, k), dtype=E8M0, device=dev)
@@ -162,7 +162,7 @@ def dequantize_impl(x_fp8: torch.Tensor, sc_fp8: torch.Tensor, sc_fp32: torch.Te
     batch = math.prod(shape[:-2])
     kernel_dtype = dtype if dtype in _DENSE_CODE else torch.float32
     x_fp8, sc_fp8, sc_fp32 = x_fp8.contiguous(), sc_fp8.contiguous(), sc_fp32.contiguous()
-    with torch.cuda.device(x_fp8.device):
+    with _lib.on_device(x_fp8.device):
         out = torch.empty(orig_shape, dtype=kernel_dtype, device=x_fp8.device)
         if out.numel():
             check(lib.pb_dequantize(x_fp8.data_ptr(), _DTYPE_FMT[x_fp8.dtype], sc_fp8.data_ptr(), sc_fp32.data_ptr(),
@@ -188,7 +188,7 @@ def fake_quantize_impl(x: torch.Tensor, tgrid, dtype, out_format: str = "e4m3") 
     lib = _lib.load()
     shape = _as_2d(tuple(x.shape))
     x = x.contiguous()
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x.device):
         out = torch.empty(tuple(x.shape), dtype=dtype, device=x.device)
         check(lib.pb_fake_quantize(x.data_ptr(), _DENSE_CODE[x.dtype], math.prod(shape[:-2]), shape[-2], shape[-1], 1, 128,
                                    _FMT_CODE[out_format], out.data_ptr(), _DENSE_CODE[dtype], _stream(x)))
@@ -207,7 +207,7 @@ def fake_quantize_scales_impl(x: torch.Tensor, tgrid, dtype):
     lead, (m, k) = shape[:-2], group_geometry(shape[-2], shape[-1], (1, 128))
     x = x.contiguous()
     dev = x.device
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         out = torch.empty(tuple(x.shape), dtype=dtype, device=dev)
         sc8 = torch.empty((*lead, m, k), dtype=E8M0, device=dev)
         sc32 = torch.empty((*lead, m, 1, 1), dtype=torch.float32, device=dev)
@@ -228,7 +228,7 @@ def relu2_requantize_impl(y: torch.Tensor):
     y = y.contiguous()
     cols = y.shape[-1]
     rows = y.numel() // cols
-    with torch.cuda.device(y.device):
+    with _lib.on_device(y.device):
         q = torch.empty((rows, cols), dtype=E4M3, device=y.device)
         sc8 = torch.empty((rows * cols // 1024, 8), dtype=E8M0, device=y.device)
         sc32 = torch.empty((rows * cols // 1024, 1, 1), dtype=torch.float32, device=y.device)
@@ -248,7 +248,7 @@ def dequantize_impl_bwd(sc_fp8: torch.Tensor, sc_fp32: torch.Tensor, g_out: torc
     batch = math.prod(shape[:-2])
     g = g_out if g_out.dtype in _DENSE_CODE else g_out.to(torch.float32)
     g = g.contiguous()
-    with torch.cuda.device(g.device):
+    with _lib.on_device(g.device):
         out = torch.empty_like(g)
         if out.numel():
             check(lib.pb_dequantize_bwd(g.data_ptr(), _DENSE_CODE[g.dtype], sc_fp8.contiguous().data_ptr(),
@@ -269,7 +269,7 @@ def dequantize_bwd_quantize_dual_impl(sc_fp8: torch.Tensor, sc_fp32: torch.Tenso
     g = g_out.contiguous()
     groups = rows * cols // 1024
     dev = g.device
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         q = torch.empty((rows, cols), dtype=_FMT_DTYPE[out_format], device=dev)
         sc8 = torch.empty((groups, 8), dtype=E8M0, device=dev)
         sc32 = torch.empty((groups, 1, 1), dtype=torch.float32, device=dev)
@@ -321,7 +321,7 @@ def transpose_bytes(q: torch.Tensor) -> torch.Tensor:
     lib = _lib.load()
     rows, cols = q.shape
     q = q.contiguous()
-    with torch.cuda.device(q.device):
+    with _lib.on_device(q.device):
         out = torch.empty((cols, rows), dtype=q.dtype, device=q.device)
         check(lib.pb_transpose_bytes(q.data_ptr(), rows, cols, out.data_ptr(), _stream(q)))
     return out
@@ -335,12 +335,12 @@ def _operand(q, sc8, sc32, rows, depth, grid, transposed_blocks=0) -> Operand:
 def gemm_tn(a: Operand, b: Operand, out_dtype, device, keep_alive=()) -> torch.Tensor:
     """D[m, n] = sum_k dq(A)[m, k] * dq(B)[n, k] on the tcgen05 kernel."""
     lib = _lib.load()
-    with torch.cuda.device(device):
+    with _lib.on_device(device):
         d = torch.empty((a.rows, b.rows), dtype=out_dtype, device=device)
         ws_bytes = lib.pb_gemm_workspace_size(a, b)
         ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=device)
         check(lib.pb_gemm_tn(a, b, d.data_ptr(), _DENSE_CODE[out_dtype], b.rows, ws.data_ptr(), ws_bytes,
-                             torch.cuda.current_stream(device).cuda_stream))
+                             _lib.current_stream(device)))
     return d
 
 
@@ -370,7 +370,7 @@ class LinearStep:
         self.b = _operand(w_t, self._keep[1], self._keep[2], self.n, self.k, (128, 128), transposed_blocks=1)
         lib = _lib.load()
         dev = w_t.device
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             # the workspace size depends on the shapes and grids only: a placeholder A describes them
             ph = torch.empty(16, dtype=torch.uint8, device=dev)
             a = Operand(ph.data_ptr(), ph.data_ptr(), ph.data_ptr(), self.rows, self.k, 1, 128, _FMT_CODE[out_format], 0)
@@ -395,7 +395,7 @@ class LinearStep:
         if x.numel() != self.rows * self.k or x.shape[-1] != self.k:
             raise ValueError(f"LinearStep was planned for [{self.rows}, {self.k}], got {tuple(x.shape)}")
         dev = x.device
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             if triple is None:
                 q = torch.empty((self.rows, self.k), dtype=_FMT_DTYPE[self.out_format], device=dev)
                 sc8 = torch.empty((self.rows * self.k // 1024, 8), dtype=E8M0, device=dev)
@@ -403,7 +403,7 @@ class LinearStep:
             else:
                 q, sc8, sc32 = triple
             d = out if out is not None else torch.empty((self.rows, self.n), dtype=self.out_dtype, device=dev)
-            st = torch.cuda.current_stream(dev).cuda_stream
+            st = _lib.current_stream(dev)
             if relu2_of_fake_quantized:
                 check(lib.pb_relu2_requantize(x.data_ptr(), self.rows, self.k, _FMT_CODE[self.out_format],
                                               q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), self.b,
@@ -589,7 +589,7 @@ def make_elementwise_impl(op):
             shape = _as_2d(tuple(x_fp8.shape))
             a, b = int(tgrid[0]), int(tgrid[1])
             xs = [t.contiguous() for t in (x_fp8, x_sc8, x_sc32, y_fp8, y_sc8, y_sc32)]
-            with torch.cuda.device(x_fp8.device):
+            with _lib.on_device(x_fp8.device):
                 out = torch.empty(tuple(x_fp8.shape), dtype=torch.float32, device=x_fp8.device)
                 check(lib.pb_elementwise(code, xs[0].data_ptr(), _DTYPE_FMT[x_fp8.dtype], xs[1].data_ptr(), xs[2].data_ptr(),
                                          xs[3].data_ptr(), _DTYPE_FMT[y_fp8.dtype], xs[4].data_ptr(), xs[5].data_ptr(),
