@@ -154,7 +154,7 @@ class _LinearFn(torch.autograd.Function):
     recipe "fp8" (default): dY is quantized on (1,128) for dgrad, and both X^T and dY^T are
     quantized on (1,128) along the tokens for wgrad (the operands of fp8_matmul_bwd, :784-789);
     the reference's matmul_impl_bwd keeps dY in f32, which no tensor-core K-block can consume.
-    recipe "reference": the literal f32 dots on dequantized operands (library matmul).
+    recipe "reference": the literal f32 dots on dequantized operands (`literal_dots`).
     In both, dX is quantized on (1,a) and dequantized again, and dW is quantized on the weight's
     grid, as the reference returns them (:637-640, :522-526)."""
 
@@ -231,11 +231,7 @@ class _LinearFn(torch.autograd.Function):
             gx = _ops.gemm_tn(op(gq[0], gq[1], gq[2], m, n, (1, 128)), op(wq[0], wq[1], wq[2], k, n, (128, 128)), torch.float32, g.device)
             gw = _ops.gemm_tn(op(xt[0], xt[1], xt[2], k, m, (1, 128)), op(gt[0], gt[1], gt[2], n, m, (1, 128)), torch.float32, g.device)
         else:
-            x_hat = _ops.dequantize_impl(*xq, torch.float32, (1, a))
-            w_hat = _ops.dequantize_impl(*wq, torch.float32, ctx.grid)
-            g32 = g.to(torch.float32)
-            gx = _ops._matmul_f32(g32, w_hat.t())
-            gw = _ops._matmul_f32(x_hat.t(), g32)
+            gx, gw = _ops.literal_dots(xq, wq, (1, a), ctx.grid, g)
         gx = _ops.fake_quantize_impl(gx, (1, a), torch.float32)                                  # :637 then :522-526
         gw = _ops.dequantize_impl(*_ops.quantize_impl(gw, ctx.grid), torch.float32, ctx.grid)    # :638; the optimizer dequantizes it
         return gx.reshape(ctx.x_shape).to(ctx.x_dtype), gw.to(ctx.w_dtype), None, None, None, None, None, None, None

@@ -471,6 +471,38 @@ def _matmul_f32(x, y):
         torch.backends.cuda.matmul.allow_tf32 = prev
 
 
+def _dense_dot(tokens: int, q, sc8, sc32, grid, g: torch.Tensor):
+    """g @ dq(Q)^T (`tokens` 0) or dq(Q)^T @ g (`tokens` 1) of a 2-D e4m3 triple and a contiguous f32 g on pb_dense_dot."""
+    lib = _lib.load()
+    rows, cols = q.shape
+    free = g.shape[0] if tokens == 0 else g.shape[1]
+    q, sc8, sc32 = q.contiguous(), sc8.contiguous(), sc32.contiguous()
+    with _lib.on_device(g.device):
+        out = torch.empty((free, rows) if tokens == 0 else (cols, free), dtype=torch.float32, device=g.device)
+        ws_bytes = lib.pb_dense_dot_workspace_size(tokens, rows, cols, grid[0], grid[1], free)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=g.device) if ws_bytes else None
+        check(lib.pb_dense_dot(tokens, q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), rows, cols, grid[0], grid[1], g.data_ptr(), free,
+                               out.data_ptr(), ws.data_ptr() if ws is not None else None, ws_bytes, _stream(g)))
+    return out
+
+
+def literal_dots(xq, wq, grid_x, grid_w, g: torch.Tensor):
+    """(g @ w^T, x^T @ g) of matmul_impl_bwd (_qarr.py:620-621) as f32 dots for 2-D triples x [m, k], w [k, n] and a dense
+    cotangent g [m, n].  (1,128) activations against a (128,128) or (128,1) weight run on pb_dense_dot, straight from the
+    triples; other grids, widths that are no multiple of 16, and the "tf32" precision dequantize and take the library matmul."""
+    _require_cuda(g, "literal_dots cotangent")
+    g = g.to(torch.float32).contiguous()
+    m, k = xq[0].shape
+    n = wq[0].shape[1]
+    if (tuple(grid_x) == (1, 128) and tuple(grid_w) in ((128, 128), (128, 1)) and n % 16 == 0 and min(m, k, n) > 0 and not _LITERAL_DOT_TF32
+            and xq[0].dtype == E4M3 and wq[0].dtype == E4M3
+            and all(t.data_ptr() % 16 == 0 and t.is_contiguous() for t in (xq[0], wq[0], g))):
+        return _dense_dot(0, *wq, grid_w, g), _dense_dot(1, *xq, grid_x, g)
+    x = dequantize_impl(*xq, torch.float32, grid_x)
+    w = dequantize_impl(*wq, torch.float32, grid_w)
+    return _matmul_f32(g, w.t()), _matmul_f32(x.t(), g)
+
+
 def matmul_mixed_impl(x_fp8, x_sc8, x_sc32, y_f32, block_grid_x):
     """_qarr.py:645-647."""
     x = dequantize_impl(x_fp8, x_sc8, x_sc32, torch.float32, block_grid_x)

@@ -1506,7 +1506,10 @@ extern "C" int pb_gemm_tn_ex(const pb_operand* a, const pb_operand* b, void* d, 
   return launch_gemm_uni<224, false>(ma, mb, md, p, st);
 }
 
-namespace pb { int transposed_status_fetch(unsigned int* out); }   // transpose_quantize.cu
+namespace pb {
+int transposed_status_fetch(unsigned int* out);   // transpose_quantize.cu
+int dense_dot_status_fetch(unsigned int* out);    // dense_dot.cu
+}
 
 extern "C" int pb_gemm_check(void* stream) {
   PB_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));

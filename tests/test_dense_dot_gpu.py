@@ -1,0 +1,56 @@
+"""pb_dense_dot (an fp8 triple against a dense f32 cotangent) against 64-bit products of the dequantized operands: tiles with one row
+or column, a contraction shorter than a stage, parts of it on several CTAs, and every grid it takes."""
+import pytest
+import torch
+
+from pratchya_b200._qualia import _ops
+from pratchya_b200._qualia import dequantize_impl, quantize_impl
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(a, b):
+    """Per element: |a| @ |b| times the roundings an f32 dot of this kernel can make -- one of the scaled operand (2^-24; the three
+    bf16 terms keep it to 2^-26), the tensor core's within 32 of the contraction (six additions of at most 2^-23) and one
+    addition per 32 of it."""
+    depth = a.shape[1]
+    return (a.abs() @ b.abs()) * 2.0 ** -24 * (14 + (depth + 31) // 32)
+
+
+@pytest.mark.parametrize("m,k,n,grid", [(1, 128, 16, (128, 1)), (5, 128, 128, (128, 128)), (129, 256, 48, (128, 1)), (64, 1024, 2048, (128, 1)),
+                                        (31, 128, 1024, (128, 128)), (130, 384, 640, (128, 128)), (1000, 2048, 128, (128, 1)), (3000, 128, 256, (128, 1))])
+def test_dense_dot_matches_64_bits(built_lib, m, k, n, grid):
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    x = torch.randn(m, k, generator=g, device="cuda") * torch.randn(1, k, generator=g, device="cuda").exp()
+    w = torch.randn(k, n, generator=g, device="cuda") * 0.02
+    dy = torch.randn(m, n, generator=g, device="cuda") * torch.randn(m, 1, generator=g, device="cuda").exp() * 1e-3
+    dy[0, 0] = 0.0
+    xq, wq = quantize_impl(x, (1, 128)), quantize_impl(w, grid)
+    xh, wh = dequantize_impl(*xq, torch.float32, (1, 128)).double(), dequantize_impl(*wq, torch.float32, grid).double()
+    gx, gw = _ops.literal_dots(xq, wq, (1, 128), grid, dy)
+    assert gx.shape == (m, k) and gw.shape == (k, n)
+    dy64 = dy.double()
+    assert ((gx.double() - dy64 @ wh.t()).abs() <= _bound(dy64, wh.t()) + 1e-30).all()
+    assert ((gw.double() - xh.t() @ dy64).abs() <= _bound(xh.t(), dy64) + 1e-30).all()
+    again = _ops.literal_dots(xq, wq, (1, 128), grid, dy)
+    assert torch.equal(gx, again[0]) and torch.equal(gw, again[1])
+
+
+def test_infinities_and_nans_spread_as_in_an_f32_dot(built_lib):
+    xq, wq = quantize_impl(torch.ones(64, 128, device="cuda"), (1, 128)), quantize_impl(torch.ones(128, 128, device="cuda"), (128, 128))
+    dy = torch.ones(64, 128, device="cuda")
+    dy[3, 5], dy[9, 7] = float("inf"), float("nan")
+    gx, gw = _ops.literal_dots(xq, wq, (1, 128), (128, 128), dy)
+    assert torch.isinf(gx[3]).all() and torch.isnan(gx[9]).all() and torch.isfinite(gx[[r for r in range(64) if r not in (3, 9)]]).all()
+    assert torch.isinf(gw[:, 5]).all() and torch.isnan(gw[:, 7]).all() and torch.isfinite(gw[:, :5]).all()
+
+
+def test_other_shapes_take_the_library_route(built_lib):
+    """A width that is no multiple of 16, a grid the kernel does not take, a cotangent off the 16-byte alignment."""
+    for m, k, n, gx_, gw_ in [(32, 64, 24, (1, 64), (64, 1)), (32, 128, 24, (1, 128), (128, 1)), (32, 128, 128, (1, 128), (128, 128))]:
+        x, w = torch.randn(m, k, device="cuda"), torch.randn(k, n, device="cuda")
+        dy = torch.randn(m * n + 1, device="cuda")[1:].view(m, n)
+        xq, wq = quantize_impl(x, gx_), quantize_impl(w, gw_)
+        gx, gw = _ops.literal_dots(xq, wq, gx_, gw_, dy)
+        xh, wh = dequantize_impl(*xq, torch.float32, gx_).double(), dequantize_impl(*wq, torch.float32, gw_).double()
+        assert (gx.double() - dy.double() @ wh.t()).abs().max() <= 1e-4 and (gw.double() - xh.t() @ dy.double()).abs().max() <= 1e-4
