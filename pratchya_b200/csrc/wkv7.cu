@@ -303,8 +303,8 @@ int launch_forward(const WkvParams& p, int64_t heads, cudaStream_t st) {
 // column sums of four timesteps wait in shared memory for one block barrier.  The chunk's eight vectors per timestep
 // arrive by cp.async one chunk ahead, and the next checkpoint into the slot that the upper half has emptied.
 //
-// Bound by the bytes its shared-memory reads and shuffles return and by its f32x2 products, both near 1300 of the 2100 cycles
-// a timestep takes with two heads on an SM.  8 x 32 heads x 1024 timesteps 1580 -> 1121 us, 32 heads 1037 -> 646 us, against
+// Bound by the bytes its shared-memory reads and shuffles return and by its f32x2 products, both near 1300 of the 1950 cycles
+// a timestep takes with two heads on an SM.  8 x 32 heads x 1024 timesteps 1577 -> 1045 us, 32 heads 1035 -> 675 us, against
 // 4 x 8 tiles with every state in shared memory and a barrier per timestep.
 struct WkvBwdParams {
   const float* in[kVecs];
@@ -594,19 +594,24 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
       for (int m = 1; m < 8; m <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
       if ((tid & 7) == 0) dots[s][d & 1] = sum;
     }
-    BwdTile S;
-    load_quads(sm.slot[ck_slot], tid, S);
-    if (steps > kSub) {
-#pragma unroll
-      for (int s = 0; s < kSub; ++s) update(V[s], S, S);
-      store_quads(sm.slot[ck_slot ^ 1], tid, S);
-      run_half(V, sm.slot[ck_slot ^ 1], t0, kSub, steps - kSub, 1, S);
-      finish_columns(V, dots, sm.col_part[1], t0, kSub, steps);
+    // The upper half chunk, then the lower one, through the same instructions: written out for each, they are twice what the
+    // instruction cache holds (a tenth of the warps' stalls were for instructions): 256 heads x
+    // 1024 timesteps 1121 -> 1045 us, 128 heads 799 -> 716; 32 heads, whose four warps an SM hide less, 646 -> 675.
+#pragma unroll 1
+    for (int half = steps > kSub; half >= 0; --half) {
+      BwdTile S;
       load_quads(sm.slot[ck_slot], tid, S);
+      if (half) {
+#pragma unroll 1
+        for (int s = 0; s < kSub; ++s) update(V[s], S, S);
+        store_quads(sm.slot[ck_slot ^ 1], tid, S);
+      } else {
+        prefetch_ckpt(ck - 1, ck_slot ^ 1);    // the state in that slot has been read
+      }
+      const int lo = half * kSub, hi = min(steps, lo + kSub);
+      run_half(V, sm.slot[half ? ck_slot ^ 1 : ck_slot], t0, lo, hi - lo, half, S);
+      finish_columns(V, dots, sm.col_part[half], t0, lo, hi);
     }
-    prefetch_ckpt(ck - 1, ck_slot ^ 1);       // that slot's state has been read
-    run_half(V, sm.slot[ck_slot], t0, 0, min(steps, kSub), 0, S);
-    finish_columns(V, dots, sm.col_part[0], t0, 0, min(steps, kSub));
     ck_slot ^= 1;
   }
   cp_async_wait<0>();
