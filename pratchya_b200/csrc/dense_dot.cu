@@ -11,16 +11,17 @@
 // tensor core's own additions do not round to nearest), so the sums are no worse than an f32 dot's: 2-norm
 // errors of 1.0e-7 to 3.1e-7 against 64 bits for contractions of 37 to 8192, where the library's SGEMM has 1.1e-7 to 1.6e-6.
 //
-// A CTA makes a 128 x 128 tile of out: eight warps convert (global loads a stage ahead in registers, scale, split, 128-byte
+// A CTA makes a 128 x 128 tile of out: eight warps convert (global loads into registers, scale, split, 128-byte
 // swizzled K-major tiles in shared memory; where i and j are the contiguous dimensions the eight c of a 16-byte chunk come from
-// eight rows, so the transpose is in the loads), eight warps empty one accumulator while
-// the other fills, and one lane of theirs issues tcgen05.mma.  Where the tiles do not fill the SMs the contraction is cut, and the parts are added in order by a second
-// kernel.
+// eight rows, so the transpose is in the loads), eight warps empty one pair of accumulators
+// while the other fills, and one lane of theirs issues tcgen05.mma.  Where the tiles do not fill the SMs the contraction is
+// cut, and the parts are added in order by a second kernel.
 //
-// What bounds it: the converting warps' own latency.  A stage takes 3000 cycles, of which the tensor core works 768; with the
-// split left out dX takes 17 % less, with the loads 14, with the emptying 13, with eleven of the twelve products 8 (dW: 28, 40,
-// 11, 5).  Against the library's SGEMM alone (the dequantization of both operands came on top), 3000 tokens, 2048 x 2048:
-// dX 488 -> 158 us, dW 430 -> 221; 8192 tokens, 2048 x 128: 100 -> 67 and 124 -> 48; 64 tokens, 1024 x 1024: 22 -> 24, 16 -> 16.
+// What bounds it: no one part.  A stage takes 2800 cycles, of which the tensor core works 768; before the loads moved behind the
+// fence, dX took 17 % less with the split left out, 14 with the loads, 13 with the emptying, 8 with eleven of the twelve
+// products (dW: 28, 40, 11, 5), and sixteen converting warps were no faster than eight.  Against the library's SGEMM alone (the
+// dequantization of both operands came on top), 3000 tokens, 2048 x 2048: dX 488 -> 155 us, dW 430 -> 202; 8192 tokens,
+// 2048 x 128: 100 -> 67 and 124 -> 45; 64 tokens, 1024 x 1024: 22 -> 25, 16 -> 16.
 #include <algorithm>
 
 #include "common.cuh"
@@ -126,7 +127,7 @@ __device__ __forceinline__ void split_chunk(const float (&g)[8], const float (&s
 // byte offset of the 16-byte chunk (eight c) of a row in a swizzled tile
 __device__ __forceinline__ uint32_t chunk_at(int row, int chunk) { return (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4); }
 __device__ __forceinline__ void st_chunk(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d));      // ordered by the fence at the stage's end
 }
 
 // What a converting thread holds of a stage: four chunks (eight c each) of g for rows j, its share of q, the scales of its c.
@@ -237,16 +238,18 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
         }
       }
     };
-    load_scales(0);
-    load_q(0);
+    auto load_stage = [&](int st) {
+      load_scales(st);
+      load_q(st);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) load_g(0, k);
+      for (int k = 0; k < 4; ++k) load_g(st, k);
+    };
+    load_stage(0);
     for (int st = 0; st < n_stages; ++st) {
       const int buf = st % kStages;
       if (!bar_wait(empty(buf), ((st / kStages) & 1) ^ 1)) break;
       const uint32_t base = tiles_base + buf * kStageBytes;
       const bool more = st + 1 < n_stages;
-      // every piece of the next stage is asked for as soon as its registers are free
       if constexpr (TOKENS) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -268,7 +271,6 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
           st_chunk(base + chunk_at(tid >> 1, 4 * (tid & 1) + h), o[0], o[1], o[2], o[3]);
         }
       }
-      if (more) load_q(st + 1);
       float s[8];
       auto scale = [](uint32_t e8, float e32) { return __fmul_rn(__fmul_rn(e8m0_to_f32(e8), e32), 0.0078125f); };
       if constexpr (TOKENS) {
@@ -280,12 +282,10 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
 #pragma unroll
         for (int e = 1; e < 8; ++e) s[e] = p.per_column ? scale(r.e8[e], r.e32[e]) : s[0];
       }
-      if (more) load_scales(st + 1);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         uint32_t hi[4], mid[4], lo[4];
         split_chunk(r.g[k], s, hi, mid, lo);
-        if (more) load_g(st + 1, k);
         const uint32_t at = base + chunk_at(row_of(k), chunk);
         st_chunk(at + kOpBytes, lo[0], lo[1], lo[2], lo[3]);
         st_chunk(at + 2 * kOpBytes, mid[0], mid[1], mid[2], mid[3]);
@@ -294,6 +294,9 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the tensor core reads what was stored
       __syncwarp();
       if (lane == 0) bar_arrive(full(buf));
+      // The next stage's loads go behind the fence, which waits for the thread's accesses that are under way: asked for as
+      // their registers became free, they held every stage up at its fence (dX 155 -> 150 us, dW 174 -> 160, 2368 tokens).
+      if (more) load_stage(st + 1);
     }
   } else {
     const int quad = warp & 3, half = (warp - kConvWarps) >> 2;      // rows 32 quad .., columns 64 half ..
