@@ -1379,7 +1379,7 @@ int launch_gemm_pair_uni(const CUtensorMap& ma, const CUtensorMap& mb, const CUt
 // the row quantizer that writes them directly.  The quantizer covers one super-group of eight
 // k-blocks per warp, so the plan must promote in chunks of eight.
 int gemm_a_prep_location(const pb_operand* a, const pb_operand* b, void* workspace, size_t workspace_bytes,
-                         uint8_t** sf, float** f, uint32_t* tiles, uint32_t* Mpad, void* stream) {
+                         uint8_t** sf, float** f, uint32_t* tiles, uint32_t* Mpad) {
   GemmPlan gp;
   if (int s = make_plan(a, b, &gp)) return s;
   if (gp.P != kMaxChunk)
@@ -1388,11 +1388,8 @@ int gemm_a_prep_location(const pb_operand* a, const pb_operand* b, void* workspa
     return fail(PB_ERR_WORKSPACE_TOO_SMALL, "pb_quantize_for_gemm: needs %zu bytes of GEMM workspace, got %zu", gp.total, workspace_bytes);
   if (reinterpret_cast<uintptr_t>(workspace) & 255) return fail(PB_ERR_MISALIGNED, "pb_quantize_for_gemm: workspace must be 256-byte aligned");
   uint8_t* ws = static_cast<uint8_t*>(workspace);
-  if (gp.Mpad != a->rows) {      // rows of padding are never written by the quantizer: give them zeros
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    PB_CUDA_TRY(cudaMemsetAsync(ws + gp.off_sfa, 0, (size_t)gp.KG * gp.tiles_m * 512, st));
-    PB_CUDA_TRY(cudaMemsetAsync(ws + gp.off_fa, 0, (size_t)gp.nchunks * gp.Mpad * 4, st));
-  }
+  // Rows of padding are never written: what stands there scales rows of the tile that no store takes (two memsets gave them
+  // zeros before: 6 us of a ChannelMix of 1000 rows, and two launches of every step whose rows are no multiple of 256).
   *sf = ws + gp.off_sfa;
   *f = reinterpret_cast<float*>(ws + gp.off_fa);
   *tiles = (uint32_t)gp.tiles_m;

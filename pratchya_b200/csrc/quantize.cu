@@ -1010,7 +1010,7 @@ extern "C" size_t pb_quantize_workspace_size(int64_t batch, int64_t rows, int64_
 namespace pb {
 // defined in gemm_sm100.cu: where the A operand's prepared scales live inside a GEMM workspace
 int gemm_a_prep_location(const pb_operand* a, const pb_operand* b, void* workspace, size_t workspace_bytes,
-                         uint8_t** sf, float** f, uint32_t* tiles, uint32_t* Mpad, void* stream);
+                         uint8_t** sf, float** f, uint32_t* tiles, uint32_t* Mpad);
 }
 
 static int quantize_entry(const void* x, int x_dtype, int64_t batch, int64_t rows, int64_t cols,
@@ -1104,7 +1104,7 @@ extern "C" int pb_quantize_for_gemm(const void* x, int x_dtype, int64_t rows, in
   pb_operand a_op;
   a_op.q = q; a_op.sc8 = sc8; a_op.sc32 = sc32; a_op.rows = rows; a_op.depth = cols;
   a_op.grid_a = 1; a_op.grid_b = 128; a_op.format = out_format; a_op.transposed_blocks = 0;
-  if (int s = pb::gemm_a_prep_location(&a_op, b, gemm_workspace, gemm_workspace_bytes, &prep.sf, &prep.f, &prep.tiles, &prep.Mpad, stream)) return s;
+  if (int s = pb::gemm_a_prep_location(&a_op, b, gemm_workspace, gemm_workspace_bytes, &prep.sf, &prep.f, &prep.tiles, &prep.Mpad)) return s;
   return quantize_entry(x, x_dtype, 1, rows, cols, 1, 128, out_format, q, sc8, sc32, nullptr, 0, stream, prep);
 }
 
@@ -1122,7 +1122,7 @@ extern "C" int pb_relu2_requantize(const void* y, int64_t rows, int64_t cols, in
     pb_operand a_op;
     a_op.q = q; a_op.sc8 = sc8; a_op.sc32 = sc32; a_op.rows = rows; a_op.depth = cols;
     a_op.grid_a = 1; a_op.grid_b = 128; a_op.format = out_format; a_op.transposed_blocks = 0;
-    if (int s = pb::gemm_a_prep_location(&a_op, b, gemm_workspace, gemm_workspace_bytes, &prep.sf, &prep.f, &prep.tiles, &prep.Mpad, stream)) return s;
+    if (int s = pb::gemm_a_prep_location(&a_op, b, gemm_workspace, gemm_workspace_bytes, &prep.sf, &prep.f, &prep.tiles, &prep.Mpad)) return s;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t n_groups = rows * (cols / 1024);
