@@ -222,6 +222,11 @@ PB_API int pb_fake_quantize(const void* x, int x_dtype, int64_t batch, int64_t r
  * (dequantize_impl_bwd, pratchya/_qualia/_qarr.py:575-601): sc8 and sc32 as pb_quantize writes them. */
 PB_API int pb_fake_quantize_scales(const void* x, int x_dtype, int64_t batch, int64_t rows, int64_t cols, int a, int b,
                             int out_format, void* out, int out_dtype, uint8_t* sc8, float* sc32, void* stream);
+/* The same for a weight's gradient on its own grid (matmul_impl_bwd quantizes it there and it is read back, :637-640, :522-526):
+ * f32 in and out, e4m3, blocks of 64 rows or more that are one column wide or 4, 8, ... 128 columns, x 16-byte aligned and
+ * cols a multiple of 4; anything else PB_ERR_UNSUPPORTED.  Workspace: 4 bytes per block. */
+PB_API int pb_fake_quantize_blocks(const float* x, int64_t batch, int64_t rows, int64_t cols, int a, int b, float* out,
+                            void* workspace, size_t workspace_bytes, void* stream);
 /* Reads (and clears) the device status words of the kernels that wait on mbarriers (the GEMM kernels and the
  * persistent transposed quantizer) launched on this device; synchronises `stream`.  Every such wait is bounded
  * (a few seconds at most); a wait that runs out makes its kernel return early and is reported here:

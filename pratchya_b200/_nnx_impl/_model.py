@@ -55,10 +55,10 @@ class FakeQuant(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, tgrid, dtype):
-        q, sc8, sc32 = _ops.quantize_impl(x, tgrid)
+        out, sc8, sc32 = _ops.fake_quantize_scales_impl(x, tgrid, dtype)
         ctx.save_for_backward(sc8, sc32)
         ctx.tgrid, ctx.x_dtype = tgrid, x.dtype
-        return _ops.dequantize_impl(q, sc8, sc32, dtype, tgrid)
+        return out
 
     @staticmethod
     def backward(ctx, g):

@@ -233,7 +233,7 @@ class _LinearFn(torch.autograd.Function):
         else:
             gx, gw = _ops.literal_dots(xq, wq, (1, a), ctx.grid, g)
         gx = _ops.fake_quantize_impl(gx, (1, a), torch.float32)                                  # :637 then :522-526
-        gw = _ops.dequantize_impl(*_ops.quantize_impl(gw, ctx.grid), torch.float32, ctx.grid)    # :638; the optimizer dequantizes it
+        gw = _ops.fake_quantize_impl(gw, ctx.grid, torch.float32)                                # :638; the optimizer dequantizes it
         return gx.reshape(ctx.x_shape).to(ctx.x_dtype), gw.to(ctx.w_dtype), None, None, None, None, None, None, None
 
 

@@ -180,12 +180,24 @@ def _fake_quantize_fused(x: torch.Tensor, tgrid, dtype) -> bool:
 
 def fake_quantize_impl(x: torch.Tensor, tgrid, dtype, out_format: str = "e4m3") -> torch.Tensor:
     """dequantize_impl(*quantize_impl(x, tgrid), dtype, tgrid) -- QArrayImpl(x, tgrid).astype(dtype),
-    _qarr.py:29 and :339-342 -- in one pass where the library has a fused kernel (f32 input on the
-    (1,128) grid with whole 8-block super-groups), otherwise by the two calls.  Same bits either way."""
+    _qarr.py:29 and :339-342 -- in one call where the library has one (f32 input on the (1,128) grid with
+    whole 8-block super-groups, or f32 in and out on a weight's grid), otherwise by the two calls.  Same bits either way."""
     _require_cuda(x, "fake_quantize_impl input")
-    if not _fake_quantize_fused(x, tgrid, dtype):
-        return dequantize_impl(*quantize_impl(x, tgrid, out_format), dtype, tgrid)
     lib = _lib.load()
+    if not _fake_quantize_fused(x, tgrid, dtype):
+        a, b = int(tgrid[0]), int(tgrid[1])
+        # a weight's gradient on its own grid: the tall-block kernels, without the triple in between
+        if (a >= 64 and (b == 1 or b in (4, 8, 16, 32, 64, 128)) and x.dim() >= 2 and x.dtype == torch.float32 and dtype == torch.float32
+                and out_format == "e4m3" and x.numel() > 0 and x.shape[-1] % 4 == 0 and x.shape[-2] % a == 0 and x.shape[-1] % b == 0
+                and x.is_contiguous() and x.data_ptr() % 16 == 0):
+            rows, cols = x.shape[-2:]
+            with _lib.on_device(x.device):
+                out = torch.empty_like(x)
+                ws = torch.empty(x.numel() // (a * b), dtype=torch.float32, device=x.device)
+                check(lib.pb_fake_quantize_blocks(x.data_ptr(), math.prod(x.shape[:-2]), rows, cols, a, b, out.data_ptr(),
+                                                  ws.data_ptr(), ws.numel() * 4, _stream(x)))
+            return out
+        return dequantize_impl(*quantize_impl(x, tgrid, out_format), dtype, tgrid)
     shape = _as_2d(tuple(x.shape))
     x = x.contiguous()
     with _lib.on_device(x.device):
@@ -452,9 +464,9 @@ _LITERAL_DOT_TF32 = False
 
 
 def set_literal_dot_precision(precision: str) -> None:
-    """Precision of the library f32 matmul behind the grids the block-scaled kernel cannot take (the reference's
-    literal recipe there: dequantize, then an f32 dot).  "f32" (default) keeps full f32 products; "tf32" lets the
-    library round the operands to 10 mantissa bits, which is what an f32 dot gets on a GPU under XLA's default
+    """Precision of the f32 dots behind the grids the block-scaled kernel cannot take (the reference's literal recipe
+    there: dequantize, then an f32 dot).  "f32" (default) keeps full f32 products (`literal_dots`: on the tensor cores
+    where it can, else the library matmul); "tf32" lets the library round the operands to 10 mantissa bits, which is what an f32 dot gets on a GPU under XLA's default
     precision, and is several times faster."""
     global _LITERAL_DOT_TF32
     if precision not in ("f32", "tf32"):

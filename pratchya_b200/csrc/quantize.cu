@@ -1,11 +1,13 @@
 // Block quantizers (sm_100a).  Replace quantize_impl, pratchya/_qualia/_qarr.py:458-506.
 //
-// Two implementations, identical results:
+// Three implementations, identical results:
 //   * row128: grid (1,128) with 8-block super-groups.  With a == 1 the row-major
 //     block order is the memory order, so a super-group is 1024 contiguous
 //     elements; one warp owns one super-group, keeps it in registers between the
 //     amax pass and the cast, and touches HBM once (read x, write q + scales).
 //     No scratch memory.
+//   * tall: blocks of 64 rows or more on whole vectors of columns (weights).  Two
+//     kernels around a scratch buffer of the blocks' maxima.
 //   * generic: any grid.  Three small kernels around a scratch buffer
 //     (per-block amax bits, then per-block divisors).
 #include <mutex>
@@ -840,13 +842,14 @@ tall_amax_kernel(const InT* __restrict__ x, float* __restrict__ amax, const Tall
   }
 }
 
-template <typename InT, bool PER_COLUMN, int FMT>
+// FAKE (f32 in and out): the values read back from the fp8 bytes instead of the triple, with the dequantizer's arithmetic.
+template <typename InT, bool PER_COLUMN, int FMT, bool FAKE>
 __global__ void __launch_bounds__(32 * kTallWarps)
 tall_apply_kernel(const InT* __restrict__ x, const float* __restrict__ amax, uint8_t* __restrict__ q,
-                  uint8_t* __restrict__ sc8, float* __restrict__ sc32, const TallDims d) {
+                  uint8_t* __restrict__ sc8, float* __restrict__ sc32, float* __restrict__ fake, const TallDims d) {
   constexpr int N = TallVec<InT>::kN;
   constexpr int kMost = PER_COLUMN ? 32 * N : 32;      // blocks of a CTA
-  __shared__ float divisor[kMost];
+  __shared__ float divisor[kMost], multiplier[FAKE ? kMost : 1];
   __shared__ float red[kTallWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t br = blockIdx.x / d.col_groups, cg = blockIdx.x - br * d.col_groups;
@@ -858,8 +861,12 @@ tall_apply_kernel(const InT* __restrict__ x, const float* __restrict__ amax, uin
     uint32_t sb; float D;
     block_scale(amax[blk], Mj, sb, D);
     divisor[i] = D;
-    sc8[blk] = (uint8_t)sb;
-    if (blk % d.K == 0) sc32[blk / d.K] = Mj;
+    if constexpr (FAKE) {
+      multiplier[i] = __fmul_rn(e8m0_to_f32(sb), Mj);  // raw amax, no floor
+    } else {
+      sc8[blk] = (uint8_t)sb;
+      if (blk % d.K == 0) sc32[blk / d.K] = Mj;
+    }
   };
   if (d.K <= 32) {
     for (int i = threadIdx.x; i < have; i += 32 * kTallWarps) {
@@ -915,7 +922,15 @@ tall_apply_kernel(const InT* __restrict__ x, const float* __restrict__ amax, uin
       o[k] = bf16x2_to_fp8x2<FMT>(div_hoisted_pack2(v[4 * k], v[4 * k + 1], nD2[k0], r2[k0])) |
              (bf16x2_to_fp8x2<FMT>(div_hoisted_pack2(v[4 * k + 2], v[4 * k + 3], nD2[k1], r2[k1])) << 16);
     }
-    if constexpr (N == 4) __stcs(reinterpret_cast<uint32_t*>(q + at), o[0]);
+    if constexpr (FAKE) {
+      const float2 a = fp8x2_to_f32x2<FMT>((uint16_t)(o[0] & 0xffffu)), b = fp8x2_to_f32x2<FMT>((uint16_t)(o[0] >> 16));
+      float m[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) m[k] = multiplier[PER_COLUMN ? lane * N + k : lane / (d.b / N)];
+      const float k128 = 0.0078125f;
+      __stcs(reinterpret_cast<float4*>(fake + at), make_float4(__fmul_rn(__fmul_rn(a.x, m[0]), k128), __fmul_rn(__fmul_rn(a.y, m[1]), k128),
+                                                               __fmul_rn(__fmul_rn(b.x, m[2]), k128), __fmul_rn(__fmul_rn(b.y, m[3]), k128)));
+    } else if constexpr (N == 4) __stcs(reinterpret_cast<uint32_t*>(q + at), o[0]);
     else                  __stcs(reinterpret_cast<uint2*>(q + at), make_uint2(o[0], o[1]));
   }
 }
@@ -941,13 +956,32 @@ int launch_tall(const InT* x, const Geometry& g, int64_t batch, int fmt, uint8_t
   if (g.b == 1) {
     tall_amax_kernel<InT, true><<<grid, threads, 0, st>>>(x, amax, d);
     PB_LAUNCH_CHECK("tall_amax_kernel");
-    if (fmt == PB_E4M3) tall_apply_kernel<InT, true, PB_E4M3><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, d);
-    else                tall_apply_kernel<InT, true, PB_E5M2><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, d);
+    if (fmt == PB_E4M3) tall_apply_kernel<InT, true, PB_E4M3, false><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, nullptr, d);
+    else                tall_apply_kernel<InT, true, PB_E5M2, false><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, nullptr, d);
   } else {
     tall_amax_kernel<InT, false><<<grid, threads, 0, st>>>(x, amax, d);
     PB_LAUNCH_CHECK("tall_amax_kernel");
-    if (fmt == PB_E4M3) tall_apply_kernel<InT, false, PB_E4M3><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, d);
-    else                tall_apply_kernel<InT, false, PB_E5M2><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, d);
+    if (fmt == PB_E4M3) tall_apply_kernel<InT, false, PB_E4M3, false><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, nullptr, d);
+    else                tall_apply_kernel<InT, false, PB_E5M2, false><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, nullptr, d);
+  }
+  PB_LAUNCH_CHECK("tall_apply_kernel");
+  return PB_OK;
+}
+
+// x read back from its e4m3 triple, f32 to f32
+int launch_tall_fake(const float* x, const Geometry& g, int64_t batch, float* out, void* workspace, cudaStream_t st) {
+  float* amax = static_cast<float*>(workspace);
+  const TallDims d{g.cols, (uint32_t)((g.cols + 127) / 128), (uint32_t)g.nbc, g.a, g.b, (int)g.K};
+  const unsigned grid = (unsigned)(batch * g.nbr * d.col_groups);
+  const int threads = 32 * kTallWarps;
+  if (g.b == 1) {
+    tall_amax_kernel<float, true><<<grid, threads, 0, st>>>(x, amax, d);
+    PB_LAUNCH_CHECK("tall_amax_kernel");
+    tall_apply_kernel<float, true, PB_E4M3, true><<<grid, threads, 0, st>>>(x, amax, nullptr, nullptr, nullptr, out, d);
+  } else {
+    tall_amax_kernel<float, false><<<grid, threads, 0, st>>>(x, amax, d);
+    PB_LAUNCH_CHECK("tall_amax_kernel");
+    tall_apply_kernel<float, false, PB_E4M3, true><<<grid, threads, 0, st>>>(x, amax, nullptr, nullptr, nullptr, out, d);
   }
   PB_LAUNCH_CHECK("tall_apply_kernel");
   return PB_OK;
@@ -1276,6 +1310,22 @@ extern "C" int pb_fake_quantize_scales(const void* x, int x_dtype, int64_t batch
   return fake_quantize_entry(x, x_dtype, batch, rows, cols, a, b, out_format, out, out_dtype, sc8, sc32, stream);
 }
 
+extern "C" int pb_fake_quantize_blocks(const float* x, int64_t batch, int64_t rows, int64_t cols, int a, int b, float* out,
+                                       void* workspace, size_t workspace_bytes, void* stream) {
+  if (!x || !out) return fail(PB_ERR_NULL_POINTER, "pb_fake_quantize_blocks: x and out must be non-null");
+  if (batch <= 0) return fail(PB_ERR_BAD_SHAPE, "pb_fake_quantize_blocks: batch=%lld must be positive", (long long)batch);
+  Geometry g;
+  if (int s = make_geometry(rows, cols, a, b, &g)) return s;
+  if (reinterpret_cast<uintptr_t>(out) & 15) return fail(PB_ERR_MISALIGNED, "pb_fake_quantize_blocks: out must be 16-byte aligned");
+  if (!tall_eligible(x, static_cast<const uint8_t*>(nullptr), g, batch))
+    return fail(PB_ERR_UNSUPPORTED, "pb_fake_quantize_blocks: grid (%d,%d) on [%lld, %lld]: use pb_quantize + pb_dequantize", a, b, (long long)rows, (long long)cols);
+  const size_t need = (size_t)(batch * g.Nb) * 4;
+  if (!workspace || workspace_bytes < need)
+    return fail(PB_ERR_WORKSPACE_TOO_SMALL, "pb_fake_quantize_blocks: needs %zu bytes of workspace, got %zu", need, workspace_bytes);
+  if (reinterpret_cast<uintptr_t>(workspace) & 3) return fail(PB_ERR_MISALIGNED, "pb_fake_quantize_blocks: workspace must be 4-byte aligned");
+  return launch_tall_fake(x, g, batch, out, workspace, static_cast<cudaStream_t>(stream));
+}
+
 // ---------------------------------------------------------------------------------------------
 // Quantize without any caller-provided or library-allocated scratch.
 //
@@ -1326,8 +1376,8 @@ extern "C" int pb_quantize_static(const void* x, int x_dtype, int64_t batch, int
                 (long long)(batch * g.Nb), (long long)kStaticScratchBlocks);
   void* scratch = nullptr;
   if (int s = static_scratch_address(&scratch)) return s;
-  // pb_quantize clears the amax half of the scratch itself (cudaMemsetAsync on `stream`), so
-  // whatever the previous call left behind is never read.
+  // pb_quantize clears the amax half of the scratch itself (cudaMemsetAsync on `stream`), or writes every
+  // maximum that it reads (tall blocks), so whatever the previous call left behind is never read.
   return pb_quantize(x, x_dtype, batch, rows, cols, a, b, out_format, q, sc8, sc32, scratch,
                      (size_t)kStaticScratchBlocks * 8, stream);
 }

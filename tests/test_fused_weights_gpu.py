@@ -24,3 +24,13 @@ def test_fake_quantize_with_its_scales(built_lib, shape, dtype):
     q, want8, want32 = quantize_impl(x, (1, 128))
     assert torch.equal(out, dequantize_impl(q, want8, want32, dtype, (1, 128)))
     assert torch.equal(sc8.view(torch.uint8), want8.view(torch.uint8)) and torch.equal(sc32, want32) and sc8.shape == want8.shape
+
+
+@pytest.mark.parametrize("shape,grid", [((128, 128), (128, 128)), ((384, 640), (128, 128)), ((2048, 128), (128, 1)), ((128, 132), (128, 1)),
+                                        ((192, 320), (64, 64)), ((3, 128, 272), (128, 16)), ((64, 260), (64, 4)), ((100, 256), (50, 128)), ((128, 6), (128, 1))])
+def test_fake_quantize_on_a_weights_grid(built_lib, shape, grid):
+    x = to_torch(synth(shape, seed=shape[-1], scale=1e-3))
+    x.view(-1)[::41] = -0.0
+    x.view(-1)[: shape[-1]] = 0.0
+    got, want = _ops.fake_quantize_impl(x, grid, torch.float32), dequantize_impl(*quantize_impl(x, grid), torch.float32, grid)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
