@@ -484,7 +484,8 @@ def _matmul_f32(x, y):
 
 
 def _dense_dot(tokens: int, q, sc8, sc32, grid, g: torch.Tensor):
-    """g @ dq(Q)^T (`tokens` 0) or dq(Q)^T @ g (`tokens` 1) of a 2-D e4m3 triple and a contiguous f32 g on pb_dense_dot."""
+    """g @ dq(Q)^T (`tokens` 0) or dq(Q)^T @ g (`tokens` 1) of a 2-D e4m3 triple and a contiguous f32 or bf16 g
+    on pb_dense_dot."""
     lib = _lib.load()
     rows, cols = q.shape
     free = g.shape[0] if tokens == 0 else g.shape[1]
@@ -493,7 +494,7 @@ def _dense_dot(tokens: int, q, sc8, sc32, grid, g: torch.Tensor):
         out = torch.empty((free, rows) if tokens == 0 else (cols, free), dtype=torch.float32, device=g.device)
         ws_bytes = lib.pb_dense_dot_workspace_size(tokens, rows, cols, grid[0], grid[1], free)
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=g.device) if ws_bytes else None
-        check(lib.pb_dense_dot(tokens, q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), rows, cols, grid[0], grid[1], g.data_ptr(), free,
+        check(lib.pb_dense_dot(tokens, q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), rows, cols, grid[0], grid[1], g.data_ptr(), _DENSE_CODE[g.dtype], free,
                                out.data_ptr(), ws.data_ptr() if ws is not None else None, ws_bytes, _stream(g)))
     return out
 
@@ -503,7 +504,7 @@ def literal_dots(xq, wq, grid_x, grid_w, g: torch.Tensor):
     cotangent g [m, n].  (1,128) activations against a (128,128) or (128,1) weight run on pb_dense_dot, straight from the
     triples; other grids, widths that are no multiple of 16, and the "tf32" precision dequantize and take the library matmul."""
     _require_cuda(g, "literal_dots cotangent")
-    g = g.to(torch.float32).contiguous()
+    g = (g if g.dtype in _DENSE_CODE else g.to(torch.float32)).contiguous()
     m, k = xq[0].shape
     n = wq[0].shape[1]
     if (tuple(grid_x) == (1, 128) and tuple(grid_w) in ((128, 128), (128, 1)) and n % 16 == 0 and min(m, k, n) > 0 and not _LITERAL_DOT_TF32
@@ -512,6 +513,7 @@ def literal_dots(xq, wq, grid_x, grid_w, g: torch.Tensor):
         return _dense_dot(0, *wq, grid_w, g), _dense_dot(1, *xq, grid_x, g)
     x = dequantize_impl(*xq, torch.float32, grid_x)
     w = dequantize_impl(*wq, torch.float32, grid_w)
+    g = g.to(torch.float32)
     return _matmul_f32(g, w.t()), _matmul_f32(x.t(), g)
 
 

@@ -21,8 +21,10 @@
 // fence, dX took 17 % less with the split left out, 14 with the loads, 13 with the emptying, 8 with eleven of the twelve
 // products (dW: 28, 40, 11, 5), and sixteen converting warps were no faster than eight.  Against the library's SGEMM alone (the
 // dequantization of both operands came on top), 3000 tokens, 2048 x 2048: dX 488 -> 155 us, dW 430 -> 202; 8192 tokens,
-// 2048 x 128: 100 -> 67 and 124 -> 45; 64 tokens, 1024 x 1024: 22 -> 25, 16 -> 16.
+// 2048 x 128: 100 -> 67 and 124 -> 45; 64 tokens, 1024 x 1024: 22 -> 25, 16 -> 16.  A bf16 g is read as it is: 146 and 186 us for the
+// 3000 tokens, and no f32 copy of it.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -45,7 +47,7 @@ __device__ unsigned int g_dot_status; // 0, or PB_ERR_DEVICE_TIMEOUT once a boun
 
 struct DotParams {
   const uint8_t* q; const uint8_t* sc8; const float* sc32;
-  const float* g;
+  const void* g;                      // f32 or bf16
   float* out;                         // or the parts, [splits][out]
   int64_t ldq, ldg, ldo, part;        // row strides in elements; elements of out
   int I, J, C;                        // extents: i and j of out, and the contraction
@@ -131,15 +133,24 @@ __device__ __forceinline__ void st_chunk(uint32_t addr, uint32_t a, uint32_t b, 
 }
 
 // What a converting thread holds of a stage: four chunks (eight c each) of g for rows j, its share of q, the scales of its c.
-template <bool TOKENS>
+template <bool TOKENS, typename G>
 struct StageRegs {
-  float g[4][8];
+  static constexpr int kWords = sizeof(G) == 4 || TOKENS ? 8 : 4;
+  uint32_t g[4][kWords];              // as loaded: f32, or a bf16 in the low half, or two bf16
+  __device__ __forceinline__ void chunk(int k, float (&f)[8]) const {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if constexpr (sizeof(G) == 4) f[e] = __uint_as_float(g[k][e]);
+      else if constexpr (TOKENS) f[e] = __uint_as_float(g[k][e] << 16);
+      else f[e] = __uint_as_float(e & 1 ? g[k][e / 2] & 0xffff0000u : g[k][e / 2] << 16);
+    }
+  }
   uint32_t q[TOKENS ? 16 : 8];        // TOKENS: [half][c] two i each; else 32 bytes of a row
   uint32_t e8[TOKENS ? 1 : 8];        // TOKENS: lanes 0-7 a c each, handed round; else this thread's
   float e32[TOKENS ? 1 : 8];
 };
 
-template <bool TOKENS>
+template <bool TOKENS, typename G>
 __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_constant__ DotParams p) {
   extern __shared__ unsigned char dot_smem[];
   __shared__ __align__(8) uint64_t bars[2 * kStages + 4];
@@ -171,7 +182,7 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
 
   if (warp < kConvWarps) {
     const int chunk = TOKENS ? warp : tid & 7;              // this thread's eight c of a stage
-    StageRegs<TOKENS> r;
+    StageRegs<TOKENS, G> r;
     auto row_of = [&](int k) { return TOKENS ? 32 * k + lane : 32 * k + (tid >> 3); };
     // Offsets from a stage's first element, the same for every stage: one add per load.  Rows past J are read again from the
     // last one: what they make is never stored.  c past the end are zeros (only a last stage has them: `whole`).
@@ -187,16 +198,19 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
       const int c0 = c_begin + st * kDepth;
       const bool whole = c0 + kDepth <= c_end;
       if constexpr (TOKENS) {
-        const float* src = p.g + (int64_t)c0 * p.ldg + j0;
+        const G* src = static_cast<const G*>(p.g) + (int64_t)c0 * p.ldg + j0;
+        using Word = typename std::conditional<sizeof(G) == 4, uint32_t, uint16_t>::type;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) r.g[k][e] = (whole || c0 + 8 * chunk + e < c_end) ? __ldg(src + (8 * chunk + e) * ldg + g_row[k]) : 0.0f;
+        for (int e = 0; e < 8; ++e)
+          r.g[k][e] = (whole || c0 + 8 * chunk + e < c_end) ? (uint32_t)__ldg(reinterpret_cast<const Word*>(src) + (8 * chunk + e) * ldg + g_row[k]) : 0u;
       } else {
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-        if (whole || c0 + 8 * chunk < c_end) {              // C is a multiple of 16: a chunk is in or out together
-          const float* src = p.g + (int64_t)j0 * p.ldg + c0 + g_row[k];
-          a = __ldg(reinterpret_cast<const float4*>(src)); b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+        const bool in = whole || c0 + 8 * chunk < c_end;    // C is a multiple of 16: a chunk is in or out together
+        const uint4* src = reinterpret_cast<const uint4*>(static_cast<const G*>(p.g) + (int64_t)j0 * p.ldg + c0 + g_row[k]);
+#pragma unroll
+        for (int h = 0; h < StageRegs<TOKENS, G>::kWords / 4; ++h) {
+          const uint4 v = in ? __ldg(src + h) : make_uint4(0, 0, 0, 0);
+          r.g[k][4 * h] = v.x; r.g[k][4 * h + 1] = v.y; r.g[k][4 * h + 2] = v.z; r.g[k][4 * h + 3] = v.w;
         }
-        r.g[k][0] = a.x; r.g[k][1] = a.y; r.g[k][2] = a.z; r.g[k][3] = a.w; r.g[k][4] = b.x; r.g[k][5] = b.y; r.g[k][6] = b.z; r.g[k][7] = b.w;
       }
     };
     auto load_q = [&](int st) {
@@ -285,7 +299,9 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         uint32_t hi[4], mid[4], lo[4];
-        split_chunk(r.g[k], s, hi, mid, lo);
+        float g[8];
+        r.chunk(k, g);
+        split_chunk(g, s, hi, mid, lo);
         const uint32_t at = base + chunk_at(row_of(k), chunk);
         st_chunk(at + kOpBytes, lo[0], lo[1], lo[2], lo[3]);
         st_chunk(at + 2 * kOpBytes, mid[0], mid[1], mid[2], mid[3]);
@@ -394,6 +410,14 @@ DotPlan make_plan(int tokens, int64_t rows, int64_t cols, int64_t g_free) {
   return d;
 }
 
+template <bool TOKENS, typename G>
+int launch_dot(const DotParams& p, unsigned grid, cudaStream_t st) {
+  PB_CUDA_TRY(cudaFuncSetAttribute(dense_dot_kernel<TOKENS, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDotSmem));      // per device
+  dense_dot_kernel<TOKENS, G><<<grid, kDotThreads, kDotSmem, st>>>(p);
+  PB_LAUNCH_CHECK("dense_dot_kernel");
+  return PB_OK;
+}
+
 bool dot_shape_ok(int tokens, int64_t rows, int64_t cols, int a, int b, int64_t g_free) {
   if (rows <= 0 || cols <= 0 || g_free <= 0 || rows > 0x7fffff00ll || cols > 0x7fffff00ll || g_free > 0x7fffff00ll) return false;
   if (tokens) return a == 1 && b == 128 && cols % 128 == 0 && g_free % 4 == 0;
@@ -420,11 +444,12 @@ extern "C" size_t pb_dense_dot_workspace_size(int tokens, int64_t rows, int64_t 
 }
 
 extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, const float* sc32, int64_t rows, int64_t cols, int a, int b,
-                            const float* g, int64_t g_free, float* out, void* workspace, size_t workspace_bytes, void* stream) {
+                            const void* g, int g_dtype, int64_t g_free, float* out, void* workspace, size_t workspace_bytes, void* stream) {
   if (!q || !sc8 || !sc32 || !g || !out) return fail(PB_ERR_NULL_POINTER, "pb_dense_dot: q, sc8, sc32, g and out must be non-null");
   if (!dot_shape_ok(tokens, rows, cols, a, b, g_free))
     return fail(PB_ERR_UNSUPPORTED, "pb_dense_dot: a [%lld, %lld] triple on (%d,%d) against %lld (see the header for what it takes)",
                 (long long)rows, (long long)cols, a, b, (long long)g_free);
+  if (g_dtype != PB_F32 && g_dtype != PB_BF16) return fail(PB_ERR_BAD_DTYPE, "pb_dense_dot: g_dtype %d is neither PB_F32 nor PB_BF16", g_dtype);
   Geometry geo;
   if (int s = make_geometry(rows, cols, a, b, &geo)) return s;
   const DotPlan d = make_plan(tokens, rows, cols, g_free);
@@ -444,14 +469,9 @@ extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, co
   DotParams p{q, sc8, sc32, g, dst, cols, tokens ? g_free : cols, tokens ? g_free : (int64_t)d.I, out_elems, d.I, d.J, d.C,
               (uint32_t)geo.nbc, log2_K, b == 1, d.i_tiles, d.tiles, d.split_depth};
   const unsigned grid = (unsigned)(d.tiles * d.splits);
-  if (tokens) {
-    PB_CUDA_TRY(cudaFuncSetAttribute(dense_dot_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDotSmem));
-    dense_dot_kernel<true><<<grid, kDotThreads, kDotSmem, st>>>(p);
-  } else {
-    PB_CUDA_TRY(cudaFuncSetAttribute(dense_dot_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDotSmem));
-    dense_dot_kernel<false><<<grid, kDotThreads, kDotSmem, st>>>(p);
-  }
-  PB_LAUNCH_CHECK("dense_dot_kernel");
+  const int status = tokens ? (g_dtype == PB_F32 ? launch_dot<true, float>(p, grid, st) : launch_dot<true, __nv_bfloat16>(p, grid, st))
+                            : (g_dtype == PB_F32 ? launch_dot<false, float>(p, grid, st) : launch_dot<false, __nv_bfloat16>(p, grid, st));
+  if (status) return status;
   if (d.splits > 1) {
     const int64_t n4 = out_elems / 4;                 // I is a multiple of 128
     add_parts_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4*>(dst), reinterpret_cast<float4*>(out), n4, d.splits);

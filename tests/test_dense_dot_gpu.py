@@ -19,12 +19,14 @@ def _bound(a, b):
 
 @pytest.mark.parametrize("m,k,n,grid", [(1, 128, 16, (128, 1)), (5, 128, 128, (128, 128)), (129, 256, 48, (128, 1)), (64, 1024, 2048, (128, 1)),
                                         (31, 128, 1024, (128, 128)), (130, 384, 640, (128, 128)), (1000, 2048, 128, (128, 1)), (3000, 128, 256, (128, 1))])
-def test_dense_dot_matches_64_bits(built_lib, m, k, n, grid):
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_dense_dot_matches_64_bits(built_lib, m, k, n, grid, dtype):
     g = torch.Generator(device="cuda").manual_seed(m + n)
     x = torch.randn(m, k, generator=g, device="cuda") * torch.randn(1, k, generator=g, device="cuda").exp()
     w = torch.randn(k, n, generator=g, device="cuda") * 0.02
     dy = torch.randn(m, n, generator=g, device="cuda") * torch.randn(m, 1, generator=g, device="cuda").exp() * 1e-3
     dy[0, 0] = 0.0
+    dy = dy.to(dtype)
     xq, wq = quantize_impl(x, (1, 128)), quantize_impl(w, grid)
     xh, wh = dequantize_impl(*xq, torch.float32, (1, 128)).double(), dequantize_impl(*wq, torch.float32, grid).double()
     gx, gw = _ops.literal_dots(xq, wq, (1, 128), grid, dy)
