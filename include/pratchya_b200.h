@@ -227,10 +227,10 @@ PB_API int pb_fake_quantize_scales(const void* x, int x_dtype, int64_t batch, in
  * cols a multiple of 4; anything else PB_ERR_UNSUPPORTED.  Workspace: 4 bytes per block. */
 PB_API int pb_fake_quantize_blocks(const float* x, int64_t batch, int64_t rows, int64_t cols, int a, int b, float* out,
                             void* workspace, size_t workspace_bytes, void* stream);
-/* Reads (and clears) the device status words of the kernels that wait on mbarriers (the GEMM kernels and the
- * persistent transposed quantizer) launched on this device; synchronises `stream`.  Every such wait is bounded
- * (a few seconds at most); a wait that runs out makes its kernel return early and is reported here:
- * PB_OK or PB_ERR_DEVICE_TIMEOUT. */
+/* Reads (and clears) the device status words of the kernels that wait on mbarriers (the GEMM kernels, the
+ * persistent transposed quantizer and the dense dots) launched on this device; synchronises `stream`.  Every such wait
+ * is bounded (a few seconds at most); a wait that runs out makes its kernel return early, its outputs unfinished, and is
+ * reported here: PB_OK or PB_ERR_DEVICE_TIMEOUT.  All the words are cleared by one call. */
 PB_API int pb_gemm_check(void* stream);
 
 /* The middle of ChannelMix (pratchya/_nnx_impl/_module.py:246-251) on the f32 product y[rows, cols] of

@@ -99,6 +99,7 @@ _DIAG_SIGNATURES = {
     "pb_debug_division_check": (_int, [C.c_uint64, C.c_uint64, _ptr, _ptr]),
     "pb_debug_gemm_profile": (_int, [C.POINTER(C.c_uint64), _ptr]),
     "pb_debug_gemm_control": (_int, [C.c_uint, _int]),
+    "pb_debug_dot_control": (_int, [C.c_uint, _int]),
 }
 
 # every symbol include/pratchya_b200.h declares (checked by the CPU test-suite)

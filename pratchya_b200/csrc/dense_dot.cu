@@ -24,6 +24,7 @@
 // 2048 x 128: 100 -> 67 and 124 -> 45; 64 tokens, 1024 x 1024: 22 -> 25, 16 -> 16.  A bf16 g is read as it is: 146 and 186 us for the
 // 3000 tokens, and no f32 copy of it.
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -54,14 +55,23 @@ struct DotParams {
   uint32_t nbc, log2_K;               // blocks per block row of the triple; blocks per super-group, a power of two
   int per_column;                     // tokens == 0: the blocks are (128,1), not (128,128)
   int i_tiles, tiles, split_depth;
+#ifdef PB_DIAGNOSTICS
+  uint32_t polls;                     // poll budget of every wait
+  int withhold;                       // the first stage is filled and never announced: every role runs out of patience
+#endif
 };
+#ifdef PB_DIAGNOSTICS
+__device__ __forceinline__ uint32_t wait_polls(const DotParams& p) { return p.polls; }
+#else
+__device__ __forceinline__ uint32_t wait_polls(const DotParams&) { return kWaitPolls; }
+#endif
 
 __device__ __forceinline__ uint32_t dot_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
 __device__ __forceinline__ void bar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // Bounded: false, and the status word set, when the poll budget ran out.
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-  for (uint32_t n = 0; n < kWaitPolls; ++n) {
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, uint32_t polls) {
+  for (uint32_t n = 0; n < polls; ++n) {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 2000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
@@ -261,7 +271,7 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
     load_stage(0);
     for (int st = 0; st < n_stages; ++st) {
       const int buf = st % kStages;
-      if (!bar_wait(empty(buf), ((st / kStages) & 1) ^ 1)) break;
+      if (!bar_wait(empty(buf), ((st / kStages) & 1) ^ 1, wait_polls(p))) break;
       const uint32_t base = tiles_base + buf * kStageBytes;
       const bool more = st + 1 < n_stages;
       if constexpr (TOKENS) {
@@ -309,7 +319,11 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the tensor core reads what was stored
       __syncwarp();
+#ifdef PB_DIAGNOSTICS
+      if (lane == 0 && !(p.withhold && st == 0)) bar_arrive(full(buf));
+#else
       if (lane == 0) bar_arrive(full(buf));
+#endif
       // The next stage's loads go behind the fence, which waits for the thread's accesses that are under way: asked for as
       // their registers became free, they held every stage up at its fence (dX 155 -> 150 us, dW 174 -> 160, 2368 tokens).
       if (more) load_stage(st + 1);
@@ -319,7 +333,7 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
     // The first of these warps has one lane issue a stage's products, always a stage ahead of the one the warp empties.
     auto issue = [&](int st) {
       const int buf = st % kStages, ab = st & 1;
-      if (!bar_wait(full(buf), (st / kStages) & 1) || !bar_wait(acc_empty(ab), ((st >> 1) & 1) ^ 1)) return false;
+      if (!bar_wait(full(buf), (st / kStages) & 1, wait_polls(p)) || !bar_wait(acc_empty(ab), ((st >> 1) & 1) ^ 1, wait_polls(p))) return false;
       tc_after();
       const uint64_t a = tile_desc(tiles_base + buf * kStageBytes);
 #pragma unroll
@@ -341,7 +355,7 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
       const int ab = st & 1;
       if (issuing && st + 1 < n_stages) issuing = issue(st + 1);
       __syncwarp();
-      if (!bar_wait(acc_full(ab), (st >> 1) & 1)) break;
+      if (!bar_wait(acc_full(ab), (st >> 1) & 1, wait_polls(p))) break;
       tc_after();
       const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + 2 * ab * kTile + half * 64;
       uint32_t v[2][16];
@@ -410,6 +424,11 @@ DotPlan make_plan(int tokens, int64_t rows, int64_t cols, int64_t g_free) {
   return d;
 }
 
+#ifdef PB_DIAGNOSTICS
+std::atomic<uint32_t> g_dot_polls{kWaitPolls};
+std::atomic<int> g_dot_withhold{0};
+#endif
+
 template <bool TOKENS, typename G>
 int launch_dot(const DotParams& p, unsigned grid, cudaStream_t st) {
   PB_CUDA_TRY(cudaFuncSetAttribute(dense_dot_kernel<TOKENS, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDotSmem));      // per device
@@ -468,6 +487,10 @@ extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, co
   float* dst = d.splits > 1 ? static_cast<float*>(workspace) : out;
   DotParams p{q, sc8, sc32, g, dst, cols, tokens ? g_free : cols, tokens ? g_free : (int64_t)d.I, out_elems, d.I, d.J, d.C,
               (uint32_t)geo.nbc, log2_K, b == 1, d.i_tiles, d.tiles, d.split_depth};
+#ifdef PB_DIAGNOSTICS
+  p.polls = g_dot_polls.load();
+  p.withhold = g_dot_withhold.load();
+#endif
   const unsigned grid = (unsigned)(d.tiles * d.splits);
   const int status = tokens ? (g_dtype == PB_F32 ? launch_dot<true, float>(p, grid, st) : launch_dot<true, __nv_bfloat16>(p, grid, st))
                             : (g_dtype == PB_F32 ? launch_dot<false, float>(p, grid, st) : launch_dot<false, __nv_bfloat16>(p, grid, st));
@@ -479,3 +502,13 @@ extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, co
   }
   return PB_OK;
 }
+
+#ifdef PB_DIAGNOSTICS
+// Diagnostics build only (not part of the reference's surface, not in the product library).  Sets the poll budget of the
+// waits (0 restores the default) and whether the first stage of the launches that follow is withheld.
+extern "C" PB_API int pb_debug_dot_control(unsigned int polls, int withhold) {
+  g_dot_polls.store(polls ? polls : kWaitPolls);
+  g_dot_withhold.store(withhold);
+  return PB_OK;
+}
+#endif

@@ -1510,14 +1510,16 @@ int dense_dot_status_fetch(unsigned int* out);    // dense_dot.cu
 
 extern "C" int pb_gemm_check(void* stream) {
   PB_CUDA_TRY(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
-  unsigned int v = 0, zero = 0;
-  PB_CUDA_TRY(cudaMemcpyFromSymbol(&v, g_gemm_status, sizeof(v)));
-  if (v != 0) {
-    PB_CUDA_TRY(cudaMemcpyToSymbol(g_gemm_status, &zero, sizeof(zero)));
-    return fail((int)v, "a bounded device-side wait in the GEMM kernel ran out");
-  }
-  if (int s = transposed_status_fetch(&v)) return s;
-  if (v != 0) return fail((int)v, "a bounded device-side wait in the transposed quantizer ran out");
+  // all three words are read and cleared before any of them is reported
+  unsigned int gemm = 0, transposed = 0, dots = 0;
+  const unsigned int zero = 0;
+  PB_CUDA_TRY(cudaMemcpyFromSymbol(&gemm, g_gemm_status, sizeof(gemm)));
+  if (gemm != 0) PB_CUDA_TRY(cudaMemcpyToSymbol(g_gemm_status, &zero, sizeof(zero)));
+  if (int s = transposed_status_fetch(&transposed)) return s;
+  if (int s = dense_dot_status_fetch(&dots)) return s;
+  if (gemm != 0) return fail((int)gemm, "a bounded device-side wait in the GEMM kernel ran out");
+  if (transposed != 0) return fail((int)transposed, "a bounded device-side wait in the transposed quantizer ran out");
+  if (dots != 0) return fail((int)dots, "a bounded device-side wait in the dense-dot kernel ran out");
   return PB_OK;
 }
 

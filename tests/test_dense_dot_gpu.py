@@ -36,6 +36,7 @@ def test_dense_dot_matches_64_bits(built_lib, m, k, n, grid, dtype):
     assert ((gw.double() - xh.t() @ dy64).abs() <= _bound(xh.t(), dy64) + 1e-30).all()
     again = _ops.literal_dots(xq, wq, (1, 128), grid, dy)
     assert torch.equal(gx, again[0]) and torch.equal(gw, again[1])
+    assert built_lib.pb_gemm_check(torch.cuda.current_stream().cuda_stream) == 0
 
 
 def test_infinities_and_nans_spread_as_in_an_f32_dot(built_lib):
