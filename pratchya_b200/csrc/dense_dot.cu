@@ -11,6 +11,14 @@
 // tensor core's own additions do not round to nearest), so the sums are no worse than an f32 dot's: 2-norm
 // errors of 1.0e-7 to 3.1e-7 against 64 bits for contractions of 37 to 8192, where the library's SGEMM has 1.1e-7 to 1.6e-6.
 //
+// The ends of the f32 range.  bf16's exponents are f32's, so below 2^-110 the three terms of an f would run into its subnormals,
+// and scaling the cotangent before it meets a small fp8 value can pass f32's largest number where their product does not.  So
+// f carries an exact factor of 2^40, which moves the first below anything that f32 holds, and the second to |g scale| near
+// 2^87, where it shows: an f without a finite bf16 makes every sum that it enters infinite or NaN.  A thread whose sums
+// are not all finite makes them again with f32 products of dequantized values, one after the other (infinite cotangents among them:
+// their infinities and NaNs are then an f32 dot's).  The look at the sums is free, behind their stores; ranges kept by
+// the converting warps instead cost 5 % (3000 tokens, 2048 x 2048, f32: dW 173 -> 182 us).
+//
 // A CTA makes a 128 x 128 tile of out: eight warps convert (global loads into registers, scale, split, 128-byte
 // swizzled K-major tiles in shared memory; where i and j are the contiguous dimensions the eight c of a 16-byte chunk come from
 // eight rows, so the transpose is in the loads), eight warps empty one pair of accumulators
@@ -42,6 +50,7 @@ constexpr int kOpBytes = kTile * kDepth * 2;            // one bf16 operand tile
 constexpr int kStageBytes = 4 * kOpBytes;               // q, then f's lo, mid and hi
 constexpr int kDotSmem = kStages * kStageBytes + 1024 + 128;      // 1024: the tiles start on a swizzle atom
 constexpr uint32_t kAccCols = 4 * kTile;                // tensor memory: two stages of two accumulators, each of half a stage's c
+constexpr float kScaleUp = 0x1p40f, kScaleDown = 0x1p-40f;      // of f, and of its sums (see above)
 constexpr uint32_t kWaitPolls = 1u << 21;               // a poll parks for up to 2 us: about four seconds at most
 
 __device__ unsigned int g_dot_status; // 0, or PB_ERR_DEVICE_TIMEOUT once a bounded wait ran out
@@ -109,8 +118,7 @@ __device__ __forceinline__ uint32_t fp8x2_to_bf16x2(uint32_t v) {
   const float2 f = fp8x2_to_f32x2<PB_E4M3>((uint16_t)v);
   return pack_bf16x2(f.x, f.y);
 }
-// f = hi + mid + lo, two elements at a time.  An infinite f (or one that rounds to an infinity) leaves infinite or NaN rests:
-// split_chunk makes them nothing.
+// f = hi + mid + lo, two elements at a time.  An f that is no finite bf16 leaves NaN rests, and its sums are made again.
 __device__ __forceinline__ void split3(float2 f, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   hi = pack_bf16x2(f.x, f.y);
   const float2 minus = make_float2(-1.0f, -1.0f);
@@ -119,22 +127,10 @@ __device__ __forceinline__ void split3(float2 f, uint32_t& hi, uint32_t& mid, ui
   const float2 t = __ffma2_rn(make_float2(__uint_as_float(mid << 16), __uint_as_float(mid & 0xffff0000u)), minus, r);
   lo = pack_bf16x2(t.x, t.y);
 }
-__device__ __forceinline__ uint32_t keep_finite(uint32_t of_hi, uint32_t v) {       // the halves of v whose hi is finite
-  return ((of_hi & 0x7f80u) == 0x7f80u ? 0u : v & 0xffffu) | ((of_hi & 0x7f800000u) == 0x7f800000u ? 0u : v & 0xffff0000u);
-}
 // eight f of one chunk
 __device__ __forceinline__ void split_chunk(const float (&g)[8], const float (&s)[8], uint32_t (&hi)[4], uint32_t (&mid)[4], uint32_t (&lo)[4]) {
-  float top = 0.0f;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float2 f = __fmul2_rn(make_float2(g[2 * e], g[2 * e + 1]), make_float2(s[2 * e], s[2 * e + 1]));
-    top = fmaxf(top, fmaxf(fabsf(f.x), fabsf(f.y)));
-    split3(f, hi[e], mid[e], lo[e]);
-  }
-  if (top > 3.38e38f) {               // below bf16's largest number: nothing rounded to an infinity
-#pragma unroll
-    for (int e = 0; e < 4; ++e) { mid[e] = keep_finite(hi[e], mid[e]); lo[e] = keep_finite(hi[e], lo[e]); }
-  }
+  for (int e = 0; e < 4; ++e) split3(__fmul2_rn(make_float2(g[2 * e], g[2 * e + 1]), make_float2(s[2 * e], s[2 * e + 1])), hi[e], mid[e], lo[e]);
 }
 // byte offset of the 16-byte chunk (eight c) of a row in a swizzled tile
 __device__ __forceinline__ uint32_t chunk_at(int row, int chunk) { return (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4); }
@@ -159,6 +155,39 @@ struct StageRegs {
   uint32_t e8[TOKENS ? 1 : 8];        // TOKENS: lanes 0-7 a c each, handed round; else this thread's
   float e32[TOKENS ? 1 : 8];
 };
+
+// what dequantizing multiplies a block's values by, before the exact 1/128
+__device__ __forceinline__ float block_multiplier(uint32_t e8, float e32) { return __fmul_rn(e8m0_to_f32(e8), e32); }
+
+// One emptying thread's 64 sums (row i, columns from jb) made and stored one f32 product after the other: the rare ones whose
+// scaled cotangent has no finite bf16.  A call of its own, sixteen sums at a time, to leave the kernel's registers alone; the
+// cotangents of a c are the same for a whole warp.
+template <bool TOKENS, typename G>
+__device__ __noinline__ void plain_dots(const DotParams& p, float* out, int i, int jb, int it, int c_begin, int c_end) {
+  const G* g = static_cast<const G*>(p.g);
+#pragma unroll 1
+  for (int j0 = jb; j0 < jb + 64 && j0 < p.J; j0 += 16) {
+    float acc[16];
+#pragma unroll
+    for (int n = 0; n < 16; ++n) acc[n] = 0.0f;
+#pragma unroll 1
+    for (int c = c_begin; c < c_end; ++c) {
+      const uint8_t q = __ldg(p.q + (TOKENS ? (int64_t)c * p.ldq + i : (int64_t)i * p.ldq + c));
+      const uint32_t id = TOKENS ? (uint32_t)c * p.nbc + it : (uint32_t)it * p.nbc + (p.per_column ? c : c / 128);
+      const float x_sc = block_multiplier(__ldg(p.sc8 + id), __ldg(p.sc32 + (id >> p.log2_K)));
+      const float x = __fmul_rn(__fmul_rn(fp8x2_to_f32x2<PB_E4M3>((uint16_t)q).x, x_sc), 0.0078125f);
+      const G* at = g + (TOKENS ? (int64_t)c * p.ldg + j0 : (int64_t)j0 * p.ldg + c);
+#pragma unroll
+      for (int n = 0; n < 16; ++n) {
+        const int k = min(n, p.J - 1 - j0);
+        acc[n] = fmaf(Elem<G>::to_f32(at[TOKENS ? (int64_t)k : k * p.ldg]), x, acc[n]);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 16; ++n)
+      if (j0 + n < p.J) out[TOKENS ? (int64_t)i * p.ldo + j0 + n : (int64_t)(j0 + n) * p.ldo + i] = acc[n];
+  }
+}
 
 template <bool TOKENS, typename G>
 __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_constant__ DotParams p) {
@@ -296,7 +325,7 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
         }
       }
       float s[8];
-      auto scale = [](uint32_t e8, float e32) { return __fmul_rn(__fmul_rn(e8m0_to_f32(e8), e32), 0.0078125f); };
+      auto scale = [](uint32_t e8, float e32) { return __fmul_rn(block_multiplier(e8, e32), kScaleUp * 0.0078125f); };
       if constexpr (TOKENS) {
         const float own = scale(r.e8[0], r.e32[0]);
 #pragma unroll
@@ -380,12 +409,17 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
 #pragma unroll
       for (int n = 0; n < 64; n += 4)
         if (jb + n < p.J)             // J is a multiple of 4
-          *reinterpret_cast<float4*>(out + (int64_t)i * p.ldo + jb + n) = make_float4(acc[n], acc[n + 1], acc[n + 2], acc[n + 3]);
+          *reinterpret_cast<float4*>(out + (int64_t)i * p.ldo + jb + n) =
+              make_float4(acc[n] * kScaleDown, acc[n + 1] * kScaleDown, acc[n + 2] * kScaleDown, acc[n + 3] * kScaleDown);
     } else {
 #pragma unroll
       for (int n = 0; n < 64; ++n)
-        if (jb + n < p.J) out[(int64_t)(jb + n) * p.ldo + i] = acc[n];
+        if (jb + n < p.J) out[(int64_t)(jb + n) * p.ldo + i] = acc[n] * kScaleDown;
     }
+    uint32_t most = 0;                // twice the largest magnitude's bits
+#pragma unroll
+    for (int n = 0; n < 64; ++n) most = max(most, __float_as_uint(acc[n]) << 1);
+    if (most >= 2 * 0x7f800000u) plain_dots<TOKENS, G>(p, out, i, jb, it, c_begin, c_end);
   }
   tc_before();
   __syncthreads();

@@ -48,6 +48,50 @@ def test_infinities_and_nans_spread_as_in_an_f32_dot(built_lib):
     assert torch.isinf(gw[:, 5]).all() and torch.isnan(gw[:, 7]).all() and torch.isfinite(gw[:, :5]).all()
 
 
+def _f32_dot_bound(a, b):
+    """As _bound for sums made one f32 product after the other: two roundings of the operand and one addition each, of numbers that
+    may be subnormal (2^-149)."""
+    return (a.abs() @ b.abs()) * 2.0 ** -24 * (a.shape[1] + 4) + a.shape[1] * 2.0 ** -149
+
+
+@pytest.mark.parametrize("x_amp,w_amp,g_amp", [(1.0, 0.02, 1e-32), (1.0, 0.02, 1e-35), (1.0, 0.02, 1e-38), (1e-4, 1e-4, 1e-32), (1e-37, 1e-37, 1.0), (1e-30, 1e-30, 1e30),
+                                               (1.0, 0.02, 1e34)])
+@pytest.mark.parametrize("m,k,n,grid", [(130, 384, 640, (128, 128)), (300, 1024, 48, (128, 1))])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_cotangents_and_scales_far_from_one(built_lib, x_amp, w_amp, g_amp, m, k, n, grid, dtype):
+    """Cotangents, scales or both at the ends of the f32 range: as an f32 dot."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x, w = torch.randn(m, k, generator=g, device="cuda") * x_amp, torch.randn(k, n, generator=g, device="cuda") * w_amp
+    dy = (torch.randn(m, n, generator=g, device="cuda") * g_amp).to(dtype)
+    dy[5] = 0.0
+    xq, wq = quantize_impl(x, (1, 128)), quantize_impl(w, grid)
+    xh, wh = dequantize_impl(*xq, torch.float32, (1, 128)).double(), dequantize_impl(*wq, torch.float32, grid).double()
+    gx, gw = _ops.literal_dots(xq, wq, (1, 128), grid, dy)
+    dy64 = dy.double()
+    assert ((gx.double() - dy64 @ wh.t()).abs() <= _f32_dot_bound(dy64, wh.t())).all()
+    assert ((gw.double() - xh.t() @ dy64).abs() <= _f32_dot_bound(xh.t(), dy64)).all()
+
+
+def test_products_that_are_finite_though_the_scaled_cotangent_is_not(built_lib):
+    """3e38 against a block of amplitude 300: the block's small values make finite products, its large ones infinities."""
+    m, k, n = 64, 256, 128
+    w = torch.full((k, n), 1e-3, device="cuda")
+    w[7] = 300.0                                         # one row of dX's columns in either block row
+    w[200] = -300.0
+    x = torch.full((m, k), 1e-3, device="cuda")
+    x[:, 9] = 300.0
+    dy = torch.zeros(m, n, device="cuda")
+    dy[3, 5], dy[11, 6], dy[20, 100] = 3e38, -3.39e38, 1.0
+    xq, wq = quantize_impl(x, (1, 128)), quantize_impl(w, (128, 128))
+    xh, wh = dequantize_impl(*xq, torch.float32, (1, 128)).double(), dequantize_impl(*wq, torch.float32, (128, 128)).double()
+    gx, gw = _ops.literal_dots(xq, wq, (1, 128), (128, 128), dy)
+    for got, a, b in ((gx, dy.double(), wh.t()), (gw, xh.t(), dy.double())):
+        want = a @ b
+        finite = want.abs() < 3.3e38
+        assert finite.any() and (~finite).any()
+        assert ((got.double() - want).abs() <= _f32_dot_bound(a, b))[finite].all() and torch.isinf(got[~finite]).all()
+
+
 def test_other_shapes_take_the_library_route(built_lib):
     """A width that is no multiple of 16, a grid the kernel does not take, a cotangent off the 16-byte alignment."""
     for m, k, n, gx_, gw_ in [(32, 64, 24, (1, 64), (64, 1)), (32, 128, 24, (1, 128), (128, 1)), (32, 128, 128, (1, 128), (128, 128))]:
