@@ -15,9 +15,9 @@
 // those reads return to the registers, 128 bytes per clock and SM, is what a whole row per thread was bound by.  Sums along a
 // row stay inside a warp (shuffles); sums along a column, which only the backward pass has and which are outputs, not part of
 // the recurrence, meet in shared memory.
-// The input vectors of a timestep arrive by cp.async ahead of time.  HBM traffic is the algorithmic minimum: every
-// input read once, every output written once, the state once per sequence, plus what the backward pass needs when
-// one follows (below).
+// The input vectors of a timestep arrive by cp.async ahead of time.  HBM traffic is near the algorithmic minimum: every
+// input read once (where several CTAs share a head each reads its vectors, at about the same time: all but one from L2), every
+// output written once, the state once per sequence, plus what the backward pass needs when one follows (below).
 #include "common.cuh"
 
 namespace pb {
@@ -55,13 +55,14 @@ __device__ __forceinline__ int ckpt_quad(int P, int Q) { return (2 * (P & 3) + (
 // warps, and where there are few heads over CTAs as well.  A warp owns 4 * ROWS rows on the backward pass's 4 x 8 lane grid:
 // a lane keeps ROWS rows x 8 columns, a row's two dot products end in three xor-shuffles (the state's one only delays the
 // warp, the output's one nothing).  No barrier inside a chunk of eight timesteps: the chunk's vectors arrive by cp.async two
-// chunks ahead, a step's are in registers one step ahead, and S * w + v kt^T is formed while sa's shuffles are under way.
+// chunks ahead, a step's are in registers one step ahead, and S * w is formed while sa's shuffles are under way.  v kt^T comes
+// last: added to a state that is about to be erased, its low bits would go with it.
 // What bounds it: with few heads the latency of a timestep (dot product, three shuffles, update: 310 cycles); with many the
 // f32x2 products, three cycles each where their operands are three different registers, and the 4 * (40 + ROWS) bytes per lane
 // and timestep that the vector reads return, which more rows per lane spread over more of them.
-// 1024 timesteps, against one row per thread and both dot products inside it: 32 heads 377 -> 174 us, 64 heads 379 -> 181,
-// 128 heads 379 -> 236, 256 heads 437 -> 370 (with sa and checkpoints 494 -> 457).  y reduced in its own timestep, behind sa's
-// shuffles, cost a fifth: 219 us with 32 heads.
+// 1024 timesteps, against one row per thread and both dot products inside it: 32 heads 377 -> 172 us, 64 heads 379 -> 188,
+// 128 heads 379 -> 246, 256 heads 437 -> 387 (with sa and checkpoints 490 -> 474).  y reduced in its own timestep, behind sa's
+// shuffles, cost a fifth with 32 heads; v kt^T formed into the state before sa was known saved a twentieth with 64 heads and more.
 constexpr int kFwdChunk = 8;      // timesteps between barriers
 constexpr int kFwdBufs = 3;       // chunks in shared memory
 
@@ -165,15 +166,15 @@ __device__ __forceinline__ float wkv_step(float2 (&S)[ROWS][4], StepVecs<ROWS>& 
 #pragma unroll
     for (int a = 0; a < ROWS; ++a) S[a][k] = __fmul2_rn(S[a][k], x.w[k]);
 #pragma unroll
-  for (int a = 0; a < ROWS; ++a)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) S[a][k] = __ffma2_rn(dup(x.v[a]), x.kt[k], S[a][k]);
-#pragma unroll
   for (int a = 0; a < ROWS; ++a) {
     const float2 nsa = dup(-sa[a]);
 #pragma unroll
     for (int k = 0; k < 4; ++k) S[a][k] = __ffma2_rn(nsa, x.b[k], S[a][k]);
   }
+#pragma unroll
+  for (int a = 0; a < ROWS; ++a)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) S[a][k] = __ffma2_rn(dup(x.v[a]), x.kt[k], S[a][k]);
   row_dots<ROWS>(S, x.r, y);
   return y_before;
 }
@@ -292,8 +293,9 @@ int launch_forward(const WkvParams& p, int64_t heads, cudaStream_t st) {
 // Warp q owns rows 16q .. 16q+15; its lanes form a 2 x 16 grid and a lane keeps 8 rows (as float2 row pairs) x 4 columns of dS
 // and of S_{t-1}: per timestep it reads 4 elements of five vectors and 8 of three, and a column's sum needs one shuffle.  dsa,
 // the only sum that the recurrence waits for, is reduced first (a reduce-scatter over the sixteen lanes and eight
-// broadcasts), and everything that only leaves the kernel is formed behind it.  dr_t takes no S_t: it is
-// w o (S_{t-1}^T dy) - b (sa . dy) + kt (v . dy), a column sum of the state at hand and two dot products per timestep.
+// broadcasts), and everything that only leaves the kernel is formed behind it.  dr_t = S_t^T dy_t is formed a timestep later
+// in the walk, where S_t is the state at hand: put together from S_{t-1} instead, w o (S_{t-1}^T dy) - b (sa . dy) + kt (v . dy),
+// it loses what a timestep writes where it has just erased something larger.
 //
 // S_{t-1} is needed for every t and is not stored by the forward pass; inverting the recurrence would divide by the
 // decay, which the reference lets go to zero.  The forward pass writes a checkpoint every kCk = 8 timesteps and
@@ -304,7 +306,7 @@ int launch_forward(const WkvParams& p, int64_t heads, cudaStream_t st) {
 // arrive by cp.async one chunk ahead, and the next checkpoint into the slot that the upper half has emptied.
 //
 // Bound by the bytes its shared-memory reads and shuffles return and by its f32x2 products, both near 1300 of the 1950 cycles
-// a timestep takes with two heads on an SM.  8 x 32 heads x 1024 timesteps 1577 -> 1045 us, 32 heads 1035 -> 675 us, against
+// a timestep takes with two heads on an SM.  8 x 32 heads x 1024 timesteps 1577 -> 1030 us, 32 heads 1035 -> 698 us, against
 // 4 x 8 tiles with every state in shared memory and a barrier per timestep.
 struct WkvBwdParams {
   const float* in[kVecs];
@@ -320,8 +322,9 @@ struct WkvBwdParams {
 struct WkvBwdSmem {
   float4 slot[2][kTileQuads];               // every thread its own quads: the chunk's checkpoint, and the state before its timestep 4
   float vec[2][kCk][kBwdVecs][kH];          // the chunk's vectors, two chunks
-  float col_part[2][kSub][kWarps][5][kH];   // two halves of a chunk: [timestep][warp][S^T dy, dkt, sum G sa, dw, S^T dsa][column]
-  float dots[2][kCk][2];                    // of the chunk's timesteps: sa . dy and v . dy
+  float col_part[2][kSub][kWarps][5][kH];   // two halves of a chunk: [timestep][warp][S^T dy of the timestep before, dkt, sum G sa, dw, S^T dsa][column]
+  float dy_before[2][kH];                   // dy of the timestep before the chunk, two chunks (the first has none: what it reads is dropped)
+  float last_part[kWarps][kH];              // S^T dy of the last timestep, a warp's rows each
 };
 
 // A lane's tile: the row pairs rp of rows row0 + 2 rp, + 1 by the columns col0 + c.
@@ -397,6 +400,7 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
 #pragma unroll
         for (int v = 0; v < kBwdVecs; ++v)
           cp_async16((uint32_t)__cvta_generic_to_shared(&sm.vec[ck & 1][s][v][(tid & 15) * 4]), (v < kVecs ? p.in[v] : (v == kVecs ? p.dy : p.sa)) + at);
+        if (s == 0 && t > 0) cp_async16((uint32_t)__cvta_generic_to_shared(&sm.dy_before[ck & 1][(tid & 15) * 4]), p.dy + at - C);
       }
     }
     cp_async_commit();
@@ -426,22 +430,23 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
 #pragma unroll
     for (int rp = 0; rp < 4; ++rp)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) to[rp][c] = __ffma2_rn(v[rp], kt[c], to[rp][c]);
+      for (int c = 0; c < 4; ++c) to[rp][c] = __ffma2_rn(sa[rp], nb[c], to[rp][c]);
 #pragma unroll
     for (int rp = 0; rp < 4; ++rp)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) to[rp][c] = __ffma2_rn(sa[rp], nb[c], to[rp][c]);
+      for (int c = 0; c < 4; ++c) to[rp][c] = __ffma2_rn(v[rp], kt[c], to[rp][c]);
   };
-  // one timestep backwards, S the state before it
-  auto back = [&](const float (*buf)[kH], const BwdTile& S, float (*part)[kH], size_t out) {
-    float2 nb[4], kap[4], dy[4], rds[4];
+  float2 dy[4];                     // of the timestep that goes backwards next
+  // one timestep backwards, S the state before it, which is also the one after the timestep before: dr of that one, whose dy
+  // is at `dy_below`
+  auto back = [&](const float (*buf)[kH], const float* dy_below, const BwdTile& S, float (*part)[kH], size_t out) {
+    float2 nb[4], kap[4], rds[4];
     {
       const float4 a4 = *reinterpret_cast<const float4*>(buf[1] + col0), k4 = *reinterpret_cast<const float4*>(buf[2] + col0);
       const float4 r4 = *reinterpret_cast<const float4*>(buf[5] + col0);
       kap[0] = dup(k4.x); kap[1] = dup(k4.y); kap[2] = dup(k4.z); kap[3] = dup(k4.w);
       nb[0] = dup(-(a4.x * k4.x)); nb[1] = dup(-(a4.y * k4.y)); nb[2] = dup(-(a4.z * k4.z)); nb[3] = dup(-(a4.w * k4.w));
       const float2 r[4] = {dup(r4.x), dup(r4.y), dup(r4.z), dup(r4.w)};
-      ld_rows(buf[kVecs] + row0, dy);
       // G = dS + dy r^T, and dsa = -G b: the only sum the recurrence waits for, so it goes first
 #pragma unroll
       for (int rp = 0; rp < 4; ++rp)
@@ -497,6 +502,7 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
     }
     {
       float2 sum[4], dw[4];
+      ld_rows(dy_below + row0, dy);
 #pragma unroll
       for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(S[0][c], dy[0]);
 #pragma unroll
@@ -535,7 +541,7 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
   };
   // The column sums of the half chunk's timesteps [lo, hi): every warp's part is in shared memory behind the barrier.  (The
   // other buffer is written by the next half, and this one again only behind that half's barrier.)
-  auto finish_columns = [&](const float (*V)[kBwdVecs][kH], const float (*dots)[2], const float (*part)[kWarps][5][kH], int t0, int lo, int hi) {
+  auto finish_columns = [&](const float (*V)[kBwdVecs][kH], const float (*part)[kWarps][5][kH], int t0, int lo, int hi) {
     __syncthreads();
     const int j = tid & (kH - 1);
     for (int s = lo + (tid >> 6); s < hi; s += 2) {
@@ -547,8 +553,8 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
         for (int w = 1; w < kWarps; ++w) sum[q] += part[s - lo][w][q][j];
       }
       const size_t out = head_base + (size_t)(t0 + s) * C + j;
-      const float w = V[s][0][j], a = V[s][1][j], kap = V[s][2][j], kt = V[s][3][j];
-      p.din[5][out] = fmaf(kt, dots[s][1], fmaf(-(a * kap), dots[s][0], w * sum[0]));      // S_t^T dy with S_t = S_{t-1} w - sa b^T + v kt^T
+      const float a = V[s][1][j], kap = V[s][2][j];
+      if (t0 + s > 0) p.din[5][out - C] = sum[0];
       p.din[3][out] = sum[1];
       p.din[0][out] = sum[3];
       p.din[1][out] = -sum[2] * kap;
@@ -556,7 +562,7 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
     }
   };
   // Timesteps lo .. lo + count - 1 backwards, `first` holding the state before lo; the later ones' states stay in registers.
-  auto run_half = [&](const float (*V)[kBwdVecs][kH], const float4* first, int t0, int lo, int count, int half, BwdTile& S1) {
+  auto run_half = [&](const float (*V)[kBwdVecs][kH], const float* dy_below, const float4* first, int t0, int lo, int count, int half, BwdTile& S1) {
     float (*part)[kWarps][5][kH] = sm.col_part[half];
     const size_t out = head_base + (size_t)(t0 + lo) * C;
     BwdTile S2, S3;                   // S1 comes as the state before lo
@@ -564,12 +570,12 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
     if (count > 2) update(V[lo + 1], S1, S2);
     if (count > 3) {
       update(V[lo + 2], S2, S3);
-      back(V[lo + 3], S3, part[3][warp], out + 3 * (size_t)C);
+      back(V[lo + 3], V[lo + 2][kVecs], S3, part[3][warp], out + 3 * (size_t)C);
     }
-    if (count > 2) back(V[lo + 2], S2, part[2][warp], out + 2 * (size_t)C);
-    if (count > 1) back(V[lo + 1], S1, part[1][warp], out + (size_t)C);
+    if (count > 2) back(V[lo + 2], V[lo + 1][kVecs], S2, part[2][warp], out + 2 * (size_t)C);
+    if (count > 1) back(V[lo + 1], V[lo][kVecs], S1, part[1][warp], out + (size_t)C);
     load_quads(first, tid, S1);
-    back(V[lo], S1, part[0][warp], out);
+    back(V[lo], dy_below, S1, part[0][warp], out);
   };
 
   issue_vec(n_ck - 1);
@@ -582,17 +588,27 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
     cp_async_wait<1>();           // this thread's copies of chunk ck, and of its checkpoint, have landed
     __syncthreads();              // ... and everyone's vectors
     const float (*V)[kBwdVecs][kH] = sm.vec[ck & 1];
-    float (*dots)[2] = sm.dots[ck & 1];
-    {                             // sa . dy and v . dy of the eight timesteps, eight threads each (of a timestep past the end: never read)
-      const int d = tid >> 3, s = d >> 1, e = (tid & 7) * 8;
-      const float* l = V[s][d & 1 ? 4 : kVecs + 1] + e;
-      const float* r = V[s][kVecs] + e;
-      float sum = 0.0f;
+    if (ck == n_ck - 1) {         // the last timestep's dr takes the final state
+      BwdTile S;
+      load_quads(sm.slot[ck_slot], tid, S);
+#pragma unroll 1
+      for (int s = 0; s < steps; ++s) update(V[s], S, S);
+      ld_rows(V[steps - 1][kVecs] + row0, dy);
+      float2 sum[4];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) sum = fmaf(l[k], r[k], sum);
+      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(S[0][c], dy[0]);
 #pragma unroll
-      for (int m = 1; m < 8; m <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
-      if ((tid & 7) == 0) dots[s][d & 1] = sum;
+      for (int rp = 1; rp < 4; ++rp)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(S[rp][c], dy[rp], sum[c]);
+      *reinterpret_cast<float2*>(sm.last_part[warp] + col0 + 2 * ti) = cols_reduce_scatter(sum, ti);
+      __syncthreads();
+      if (tid < kH) {
+        float r = sm.last_part[0][tid];
+#pragma unroll
+        for (int w = 1; w < kWarps; ++w) r += sm.last_part[w][tid];
+        p.din[5][head_base + (size_t)(p.T - 1) * C + tid] = r;
+      }
     }
     // The upper half chunk, then the lower one, through the same instructions: written out for each, they are twice what the
     // instruction cache holds (a tenth of the warps' stalls were for instructions): 256 heads x
@@ -609,8 +625,8 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
         prefetch_ckpt(ck - 1, ck_slot ^ 1);    // the state in that slot has been read
       }
       const int lo = half * kSub, hi = min(steps, lo + kSub);
-      run_half(V, sm.slot[half ? ck_slot ^ 1 : ck_slot], t0, lo, hi - lo, half, S);
-      finish_columns(V, dots, sm.col_part[half], t0, lo, hi);
+      run_half(V, half ? V[kSub - 1][kVecs] : sm.dy_before[ck & 1], sm.slot[half ? ck_slot ^ 1 : ck_slot], t0, lo, hi - lo, half, S);
+      finish_columns(V, sm.col_part[half], t0, lo, hi);
     }
     ck_slot ^= 1;
   }

@@ -41,3 +41,31 @@ def test_scan_against_the_recurrence(built_lib, batch, steps, heads, with_grad):
         want = torch.autograd.grad((y_ref, s_ref), ref, (gy.double(), gs.double()))
         for name, u, v in zip(("state", "decay", "iclr", "removal_k", "replacement_k", "v", "r"), got, want):
             assert (u.double() - v).abs().max() <= 2e-5 * v.abs().max(), name
+
+
+@pytest.mark.parametrize("heads,steps", [(1, 5), (2, 64), (40, 13), (130, 24)])
+def test_what_a_timestep_writes_where_it_erases_something_larger(built_lib, heads, steps):
+    """w = a = 1 and unit keys: every timestep erases a column of a state near 1e4 exactly and writes v there, of size one.  The
+    column and the output are v to the last bit, and dr = S_t^T dy is as accurate as a sum of that column (64 products and
+    additions), none of which survives where the write meets the old state before the erasure does."""
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    shape = (1, steps, heads * 64)
+    unit = torch.zeros(1, steps, heads, 64, device="cuda")
+    for t in range(steps):
+        unit[:, t, :, (5 * t) % 64] = 1.0
+    unit = unit.reshape(shape)
+    ones, v = torch.ones(shape, device="cuda"), torch.randn(shape, generator=g, device="cuda")
+    state = 1e4 * torch.randn(1, heads, 64, 64, generator=g, device="cuda")
+    leaves = [t.clone().requires_grad_(True) for t in (state, ones, ones, unit, unit, v, unit)]
+    s_out, y = wkv_state_scan(leaves[0], *leaves[1:], heads)
+    assert torch.equal(y, v)
+    want = state.clone()
+    for t in range(steps):
+        want[..., (5 * t) % 64] = v.view(1, steps, heads, 64)[:, t]
+    assert torch.equal(s_out, want)
+    dy = torch.randn(shape, generator=g, device="cuda")
+    dr = torch.autograd.grad(y, leaves[6], dy)[0].view(1, steps, heads, 64).double()
+    v64, dy64 = v.view(1, steps, heads, 64).double(), dy.view(1, steps, heads, 64).double()
+    for t in range(steps):
+        got = dr[:, t, :, (5 * t) % 64]
+        assert ((got - (v64[:, t] * dy64[:, t]).sum(-1)).abs() <= 65 * 2.0 ** -24 * (v64[:, t] * dy64[:, t]).abs().sum(-1)).all(), t
