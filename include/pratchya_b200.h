@@ -71,7 +71,8 @@ PB_API int pb_group_geometry(int64_t rows, int64_t cols, int a, int b, int64_t* 
  *      Non-finite inputs are where this library knowingly departs from the reference: jnp.max propagates a
  *      NaN, so one NaN makes the reference's whole super-group (its fp32 amax, every scale and byte) NaN; the
  *      amax reductions here drop NaNs (fmaxf / __hmax2 / integer max on the bits), so only the NaN element
- *      itself becomes the fp8 NaN byte and its neighbours keep finite scales.  An Inf input gives an Inf amax
+ *      itself becomes the fp8 NaN byte and its neighbours keep finite scales, whatever the grid and the
+ *      alignment (a block of nothing but NaNs has the scale byte 255).  An Inf input gives an Inf amax
  *      in both.  Finite inputs are bit-exact. */
 PB_API size_t pb_quantize_workspace_size(int64_t batch, int64_t rows, int64_t cols, int a, int b);
 PB_API int pb_quantize(const void* x, int x_dtype, int64_t batch, int64_t rows, int64_t cols,

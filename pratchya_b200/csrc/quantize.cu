@@ -640,13 +640,13 @@ __device__ __forceinline__ void load_vec(const InT* p, float (&v)[VEC]) {
 
 template <typename InT, int VEC>
 __global__ void __launch_bounds__(256)
-generic_amax_kernel(const InT* __restrict__ x, uint32_t* __restrict__ amax_bits, GenericDims d) {
+generic_amax_kernel(const InT* __restrict__ x, int* __restrict__ amax_bits, GenericDims d) {
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; ; i += stride) {
     // whole warps leave together: lane 0 holds the warp's smallest index
     const bool active = i < d.total_vecs;
     if (__all_sync(0xffffffffu, !active)) break;
-    uint32_t bits = 0;
+    int bits = -1;                        // no magnitude: less than any, and as a float a NaN
     uint32_t blk = 0xffffffffu;
     if (active) {
       float v[VEC];
@@ -654,12 +654,12 @@ generic_amax_kernel(const InT* __restrict__ x, uint32_t* __restrict__ amax_bits,
       float m = fabsf(v[0]);
 #pragma unroll
       for (int j = 1; j < VEC; ++j) m = fmaxf(m, fabsf(v[j]));
-      bits = __float_as_uint(m);          // non-negative floats order like unsigned ints
+      if (m == m) bits = __float_as_int(m);      // non-negative floats order like integers; a vector of NaNs adds nothing
       blk = d.idx.block_of(i);
     }
     const uint32_t blk0 = __shfl_sync(0xffffffffu, blk, 0);
     if (__all_sync(0xffffffffu, blk == blk0)) {
-      const uint32_t mx = __reduce_max_sync(0xffffffffu, bits);
+      const int mx = __reduce_max_sync(0xffffffffu, bits);
       if ((threadIdx.x & 31) == 0) atomicMax(amax_bits + blk0, mx);
     } else if (active) {
       atomicMax(amax_bits + blk, bits);
@@ -784,14 +784,6 @@ struct TallDims {
   int K;
 };
 
-// The larger of two magnitudes.  Across columns NaNs are dropped (fmaxf; a block of nothing else keeps one); a one-column
-// block keeps its own (the order of the bit patterns), as the three-kernel form does.
-template <bool PER_COLUMN>
-__device__ __forceinline__ float larger(float a, float b) {
-  if constexpr (PER_COLUMN) return __uint_as_float(max(__float_as_uint(a), __float_as_uint(b)));
-  else return fmaxf(a, b);
-}
-
 // PER_COLUMN: b == 1, every column of the block row is a block.  Otherwise b is a power-of-two number of vectors, at most 32.
 template <typename InT, bool PER_COLUMN>
 __global__ void __launch_bounds__(32 * kTallWarps)
@@ -801,9 +793,9 @@ tall_amax_kernel(const InT* __restrict__ x, float* __restrict__ amax, const Tall
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t br = blockIdx.x / d.col_groups, cg = blockIdx.x - br * d.col_groups;
   const int64_t col = ((int64_t)cg * 32 + lane) * N;
-  float m[N];
+  float m[N];                         // NaNs are dropped (fmaxf): a block of nothing else keeps one
 #pragma unroll
-  for (int k = 0; k < N; ++k) m[k] = PER_COLUMN ? 0.0f : __uint_as_float(0x7fffffffu);
+  for (int k = 0; k < N; ++k) m[k] = __uint_as_float(0x7fffffffu);
   if (col < d.cols) {
     const InT* p = x + (int64_t)br * d.a * d.cols + col;
 #pragma unroll 8
@@ -811,7 +803,7 @@ tall_amax_kernel(const InT* __restrict__ x, float* __restrict__ amax, const Tall
       float v[N];
       TallVec<InT>::load(p + (int64_t)r * d.cols, v);
 #pragma unroll
-      for (int k = 0; k < N; ++k) m[k] = larger<PER_COLUMN>(m[k], fabsf(v[k]));
+      for (int k = 0; k < N; ++k) m[k] = fmaxf(m[k], fabsf(v[k]));
     }
   }
   if constexpr (PER_COLUMN) {
@@ -823,7 +815,7 @@ tall_amax_kernel(const InT* __restrict__ x, float* __restrict__ amax, const Tall
       if (gc >= d.cols) break;
       float t = red[0][c];
 #pragma unroll
-      for (int w = 1; w < kTallWarps; ++w) t = larger<PER_COLUMN>(t, red[w][c]);
+      for (int w = 1; w < kTallWarps; ++w) t = fmaxf(t, red[w][c]);
       amax[(int64_t)br * d.nbc + gc] = t;
     }
   } else {
@@ -1004,9 +996,9 @@ int launch_generic(const InT* x, const Geometry& g, int64_t batch, int fmt, uint
   if (total / VEC > kMaxIndexed || batch * g.rows > kMaxIndexed)
     return fail(PB_ERR_UNSUPPORTED, "pb_quantize: %lld elements exceed the 31-bit index range of the generic kernels", (long long)total);
   GenericDims d{VecIndexer(g.cols, g.a, g.b, VEC), (uint32_t)(total / VEC)};
-  PB_CUDA_TRY(cudaMemsetAsync(amax_bits, 0, nblk * sizeof(uint32_t), st));
+  PB_CUDA_TRY(cudaMemsetAsync(amax_bits, 0xff, nblk * sizeof(uint32_t), st));      // -1: a block of nothing but NaNs keeps it
   const int grid = grid_for(d.total_vecs, 256, 8);
-  generic_amax_kernel<InT, VEC><<<grid, 256, 0, st>>>(x, amax_bits, d);
+  generic_amax_kernel<InT, VEC><<<grid, 256, 0, st>>>(x, reinterpret_cast<int*>(amax_bits), d);
   PB_LAUNCH_CHECK("generic_amax_kernel");
   if (int s = launch_group_scales(amax_bits, divisor, sc8, sc32, batch * g.M, g.K, st)) return s;
   if (fmt == PB_E4M3) generic_apply_kernel<InT, VEC, PB_E4M3><<<grid, 256, 0, st>>>(x, divisor, q, d);

@@ -44,3 +44,29 @@ def test_views_off_the_vector_alignment(built_lib):
     base = to_torch(synth((128 * 256 + 1,), seed=9))
     x = base[1:].view(128, 256)                        # four bytes off sixteen: the scalar form of the three-kernel path
     assert_triple_equal(quantize_impl(x, (128, 128)), oracle.quantize_impl(x.cpu().numpy(), (128, 128)), "offset view")
+
+
+@pytest.mark.parametrize("shape,grid", [((128, 256), (128, 128)), ((256, 256), (128, 1)), ((128, 128), (64, 16)), ((130, 256), (65, 4)), ((32, 256), (4, 64)), ((16, 1024), (2, 512))])
+@pytest.mark.parametrize("dtype", [np.float32, BF16])
+def test_nans_are_dropped_on_every_route(built_lib, shape, grid, dtype):
+    """A row, a column and single elements of NaN: everything else has the scales and bytes that it has beside zeros, and a copy off
+    the vector alignment has those of the aligned array.  A block of nothing but NaNs keeps the scale byte 255."""
+    x = synth(shape, seed=grid[1], dtype=np.float32)
+    nan = np.zeros(shape, bool)
+    nan[5] = True
+    nan[: grid[0], 8 * grid[1] % shape[1] : 8 * grid[1] % shape[1] + grid[1]] = True      # one whole block
+    nan[:, 3] = True
+    nan[7, 9] = nan[11, 40] = True
+    clean, x = np.where(nan, 0, x).astype(dtype), np.where(nan, np.nan, x).astype(dtype)
+    got, want = quantize_impl(to_torch(x), grid), quantize_impl(to_torch(clean), grid)
+    q, wq = bytes_of(got[0]), bytes_of(want[0])
+    assert (q[nan] & 0x7F == 0x7F).all() and np.array_equal(q[~nan], wq[~nan])
+    whole = nan.reshape(shape[0] // grid[0], grid[0], shape[1] // grid[1], grid[1]).all(axis=(1, 3)).reshape(-1)
+    sc8, wsc8 = bytes_of(got[1]).reshape(-1), bytes_of(want[1]).reshape(-1)
+    assert whole.any() and (sc8[whole] == 255).all() and np.array_equal(sc8[~whole], wsc8[~whole])
+    assert torch.equal(got[2], want[2])
+    t = to_torch(x)
+    base = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+    off = base[1:].view(shape)
+    off.copy_(t)
+    assert all(np.array_equal(bytes_of(a), bytes_of(b)) for a, b in zip(quantize_impl(off, grid)[:2], got[:2]))
