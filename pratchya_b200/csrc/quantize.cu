@@ -868,23 +868,22 @@ tall_apply_kernel(const InT* __restrict__ x, const float* __restrict__ amax, uin
       store_scales(i, Mj);
     }
   } else {
-    int64_t group = -1;
-    float Mj = 0.0f;
-    for (int i = 0; i < have; ++i) {
-      if ((first + i) / d.K != group) {                // the same for every thread
-        group = (first + i) / d.K;
-        float m = 0.0f;
-        for (int k = threadIdx.x; k < d.K; k += 32 * kTallWarps) m = fmaxf(m, amax[group * d.K + k]);
+    // one super-group of the CTA's blocks after the other: its maximum by all threads, then a thread per block
+    for (int i0 = 0; i0 < have;) {                     // the same for every thread
+      const int64_t group = (first + i0) / d.K;
+      const int i1 = (int)min((int64_t)have, (group + 1) * d.K - first);
+      float m = 0.0f;
+      for (int k = threadIdx.x; k < d.K; k += 32 * kTallWarps) m = fmaxf(m, amax[group * d.K + k]);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        __syncthreads();
-        if (lane == 0) red[warp] = m;
-        __syncthreads();
-        Mj = red[0];
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      __syncthreads();
+      if (lane == 0) red[warp] = m;
+      __syncthreads();
+      float Mj = red[0];
 #pragma unroll
-        for (int w = 1; w < kTallWarps; ++w) Mj = fmaxf(Mj, red[w]);
-      }
-      if (threadIdx.x == 0) store_scales(i, Mj);
+      for (int w = 1; w < kTallWarps; ++w) Mj = fmaxf(Mj, red[w]);
+      for (int i = i0 + threadIdx.x; i < i1; i += 32 * kTallWarps) store_scales(i, Mj);
+      i0 = i1;
     }
   }
   __syncthreads();

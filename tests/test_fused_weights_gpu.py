@@ -27,7 +27,8 @@ def test_fake_quantize_with_its_scales(built_lib, shape, dtype):
 
 
 @pytest.mark.parametrize("shape,grid", [((128, 128), (128, 128)), ((384, 640), (128, 128)), ((2048, 128), (128, 1)), ((128, 132), (128, 1)),
-                                        ((192, 320), (64, 64)), ((3, 128, 272), (128, 16)), ((64, 260), (64, 4)), ((100, 256), (50, 128)), ((128, 6), (128, 1))])
+                                        ((192, 320), (64, 64)), ((3, 128, 272), (128, 16)), ((64, 260), (64, 4)), ((100, 256), (50, 128)), ((128, 6), (128, 1)),
+                                        ((1024, 320), (1024, 1)), ((768, 144), (768, 1)), ((2, 1024, 192), (1024, 1))])
 def test_fake_quantize_on_a_weights_grid(built_lib, shape, grid):
     x = to_torch(synth(shape, seed=shape[-1], scale=1e-3))
     x.view(-1)[::41] = -0.0

@@ -14,6 +14,7 @@ CASES = [
     ((128, 128), (128, 128)), ((384, 640), (128, 128)), ((2048, 1152), (128, 128)),                   # bf16: an odd number of 128-column blocks
     ((128, 272), (128, 16)), ((64, 264), (64, 8)), ((192, 320), (64, 64)), ((1024, 2048), (64, 32)),  # several blocks per warp, K above and below 32
     ((100, 256), (100, 128)), ((66, 128), (66, 64)), ((3, 128, 256), (128, 128)), ((2, 256, 136), (64, 1)),
+    ((1024, 320), (1024, 1)), ((768, 144), (768, 1)), ((2, 1024, 192), (1024, 1)), ((1024, 2048), (512, 64)),      # K above 32, with super-groups that end inside a CTA's blocks
     ((63, 128), (63, 64)), ((128, 6), (128, 1)), ((128, 96), (128, 48)),                              # the three-kernel form's side of the rule
 ]
 
