@@ -225,7 +225,9 @@ PB_API int pb_fake_quantize_scales(const void* x, int x_dtype, int64_t batch, in
                             int out_format, void* out, int out_dtype, uint8_t* sc8, float* sc32, void* stream);
 /* The same for a weight's gradient on its own grid (matmul_impl_bwd quantizes it there and it is read back, :637-640, :522-526):
  * f32 in and out, e4m3, blocks of 64 rows or more that are one column wide or 4, 8, ... 128 columns, x 16-byte aligned and
- * cols a multiple of 4; anything else PB_ERR_UNSUPPORTED.  Workspace: 4 bytes per block. */
+ * cols a multiple of 4; anything else PB_ERR_UNSUPPORTED.  Workspace: 4 bytes per block; the size entry gives them where this is also
+ * the faster way, and 0 where it is not taken or pb_quantize + pb_dequantize are faster (blocks of many rows, few of them). */
+PB_API size_t pb_fake_quantize_blocks_workspace_size(int64_t batch, int64_t rows, int64_t cols, int a, int b);
 PB_API int pb_fake_quantize_blocks(const float* x, int64_t batch, int64_t rows, int64_t cols, int a, int b, float* out,
                             void* workspace, size_t workspace_bytes, void* stream);
 /* Reads (and clears) the device status words of the kernels that wait on mbarriers (the GEMM kernels, the

@@ -186,17 +186,18 @@ def fake_quantize_impl(x: torch.Tensor, tgrid, dtype, out_format: str = "e4m3") 
     lib = _lib.load()
     if not _fake_quantize_fused(x, tgrid, dtype):
         a, b = int(tgrid[0]), int(tgrid[1])
-        # a weight's gradient on its own grid: the tall-block kernels, without the triple in between
-        if (a >= 64 and (b == 1 or b in (4, 8, 16, 32, 64, 128)) and x.dim() >= 2 and x.dtype == torch.float32 and dtype == torch.float32
-                and out_format == "e4m3" and x.numel() > 0 and x.shape[-1] % 4 == 0 and x.shape[-2] % a == 0 and x.shape[-1] % b == 0
+        # a weight's gradient on its own grid: the tall-block kernels, without the triple in between, where the library takes the grid
+        if (x.dim() >= 2 and x.dtype == torch.float32 and dtype == torch.float32 and out_format == "e4m3" and x.numel() > 0
                 and x.is_contiguous() and x.data_ptr() % 16 == 0):
             rows, cols = x.shape[-2:]
+            batch = math.prod(x.shape[:-2])
             with _lib.on_device(x.device):
-                out = torch.empty_like(x)
-                ws = torch.empty(x.numel() // (a * b), dtype=torch.float32, device=x.device)
-                check(lib.pb_fake_quantize_blocks(x.data_ptr(), math.prod(x.shape[:-2]), rows, cols, a, b, out.data_ptr(),
-                                                  ws.data_ptr(), ws.numel() * 4, _stream(x)))
-            return out
+                ws_bytes = lib.pb_fake_quantize_blocks_workspace_size(batch, rows, cols, a, b)
+                if ws_bytes:
+                    out = torch.empty_like(x)
+                    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device)
+                    check(lib.pb_fake_quantize_blocks(x.data_ptr(), batch, rows, cols, a, b, out.data_ptr(), ws.data_ptr(), ws_bytes, _stream(x)))
+                    return out
         return dequantize_impl(*quantize_impl(x, tgrid, out_format), dtype, tgrid)
     shape = _as_2d(tuple(x.shape))
     x = x.contiguous()

@@ -926,15 +926,30 @@ tall_apply_kernel(const InT* __restrict__ x, const float* __restrict__ amax, uin
   }
 }
 
-// Whether the two-kernel form takes this grid: blocks of kTallMinRows rows or more, one column wide or a power-of-two number
-// of vectors that fits a warp's row, whole vectors in a row of x and q, and a CTA count that a launch can hold.
+// CTAs of the two-kernel form, or 0 where it does not take the grid: blocks of kTallMinRows rows or more, one column wide or a
+// power-of-two number of vectors that fits a warp's row, whole vectors in a row, and a CTA count that a launch can hold.
 template <typename InT>
-bool tall_eligible(const InT* x, const uint8_t* q, const Geometry& g, int64_t batch) {
+int64_t tall_ctas(const Geometry& g, int64_t batch) {
   constexpr int N = TallVec<InT>::kN;
-  if (g.a < kTallMinRows || g.cols % N != 0 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(q) & (N - 1))) return false;
-  if (g.b != 1 && (g.b % N != 0 || (32 * N) % g.b != 0)) return false;
-  const int64_t col_groups = (g.cols + 32 * N - 1) / (32 * N);
-  return batch * g.nbr * col_groups <= kMaxIndexed && g.nbc <= kMaxIndexed;
+  if (g.a < kTallMinRows || g.cols % N != 0) return 0;
+  if (g.b != 1 && (g.b % N != 0 || (32 * N) % g.b != 0)) return 0;
+  const int64_t ctas = batch * g.nbr * ((g.cols + 32 * N - 1) / (32 * N));
+  return ctas <= kMaxIndexed && g.nbc <= kMaxIndexed ? ctas : 0;
+}
+
+// Where it is the faster form.  A CTA walks the rows of its blocks alone (0.029 us a row in f32, 0.042 in bf16), so more rows want more
+// CTAs beside it, and a walk of thousands of rows that lie far apart falls to a third of its rate; the three-kernel form
+// spreads any grid, at an atomicMax per vector: the wider the block the more of them meet.  Both, us, one call:
+//   128 rows, f32: 8.7 | 8.6 (three | two kernels) with one CTA, 22 | 9 with 74.  bf16, (128,128): 9.7 | 10.3 with 4, 14 | 11 with 16
+//   (1024,128) f32: 31 | 34 with 16, 42 | 34 with 24, 107 | 37 with 148.  (4096,128), 64 CTAs: 364 | 306 in f32, 373 | 431 in bf16
+//   (1024,1) f32: 30 | 44 with 48, 45 | 45 with 74, 86 | 49 with 148.  (2048,1) f32, 148 CTAs: 172 | 211
+//   (512,16) f32: 17 | 20 with 74, 60 | 65 with 592.
+template <typename InT>
+bool tall_pays(const Geometry& g, int64_t ctas) {
+  if (g.a <= (sizeof(InT) == 4 ? 128 : 96)) return true;
+  if (g.a <= 128) return ctas >= 16;
+  if (g.b >= 128) return g.a <= 2048 && 6 * ctas >= sm_count();
+  return g.b == 1 && g.a <= 1024 && 2 * ctas >= sm_count();
 }
 
 template <typename InT>
@@ -987,7 +1002,9 @@ int grid_for(int64_t work_items, int threads, int ctas_per_sm) {
 template <typename InT, int VEC>
 int launch_generic(const InT* x, const Geometry& g, int64_t batch, int fmt, uint8_t* q, uint8_t* sc8, float* sc32,
                    void* workspace, cudaStream_t st) {
-  if (tall_eligible(x, q, g, batch)) return launch_tall(x, g, batch, fmt, q, sc8, sc32, workspace, st);
+  const int64_t ctas = tall_ctas<InT>(g, batch);
+  if (ctas > 0 && tall_pays<InT>(g, ctas) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & (TallVec<InT>::kN - 1)) == 0)
+    return launch_tall(x, g, batch, fmt, q, sc8, sc32, workspace, st);
   const int64_t nblk = batch * g.Nb;
   uint32_t* amax_bits = static_cast<uint32_t*>(workspace);
   float* divisor = reinterpret_cast<float*>(amax_bits + nblk);
@@ -1301,6 +1318,13 @@ extern "C" int pb_fake_quantize_scales(const void* x, int x_dtype, int64_t batch
   return fake_quantize_entry(x, x_dtype, batch, rows, cols, a, b, out_format, out, out_dtype, sc8, sc32, stream);
 }
 
+extern "C" size_t pb_fake_quantize_blocks_workspace_size(int64_t batch, int64_t rows, int64_t cols, int a, int b) {
+  Geometry g;
+  if (batch <= 0 || make_geometry(rows, cols, a, b, &g) != PB_OK) return 0;
+  const int64_t ctas = tall_ctas<float>(g, batch);
+  return ctas > 0 && tall_pays<float>(g, ctas) ? (size_t)(batch * g.Nb) * 4 : 0;
+}
+
 extern "C" int pb_fake_quantize_blocks(const float* x, int64_t batch, int64_t rows, int64_t cols, int a, int b, float* out,
                                        void* workspace, size_t workspace_bytes, void* stream) {
   if (!x || !out) return fail(PB_ERR_NULL_POINTER, "pb_fake_quantize_blocks: x and out must be non-null");
@@ -1308,7 +1332,7 @@ extern "C" int pb_fake_quantize_blocks(const float* x, int64_t batch, int64_t ro
   Geometry g;
   if (int s = make_geometry(rows, cols, a, b, &g)) return s;
   if (reinterpret_cast<uintptr_t>(out) & 15) return fail(PB_ERR_MISALIGNED, "pb_fake_quantize_blocks: out must be 16-byte aligned");
-  if (!tall_eligible(x, static_cast<const uint8_t*>(nullptr), g, batch))
+  if (tall_ctas<float>(g, batch) == 0 || (reinterpret_cast<uintptr_t>(x) & 15))
     return fail(PB_ERR_UNSUPPORTED, "pb_fake_quantize_blocks: grid (%d,%d) on [%lld, %lld]: use pb_quantize + pb_dequantize", a, b, (long long)rows, (long long)cols);
   const size_t need = (size_t)(batch * g.Nb) * 4;
   if (!workspace || workspace_bytes < need)

@@ -35,3 +35,16 @@ def test_fake_quantize_on_a_weights_grid(built_lib, shape, grid):
     x.view(-1)[: shape[-1]] = 0.0
     got, want = _ops.fake_quantize_impl(x, grid, torch.float32), dequantize_impl(*quantize_impl(x, grid), torch.float32, grid)
     assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("rows,cols,grid,one_call", [(128, 128, (128, 128), True), (128, 4, (128, 1), True), (1024, 3840, (1024, 128), True), (2048, 128, (2048, 128), False),
+                                                     (4096, 256, (4096, 1), False), (1024, 2048, (512, 16), False)])
+def test_tall_blocks_that_few_ctas_would_walk_go_by_two_calls(built_lib, rows, cols, grid, one_call):
+    """The library's rule, and the same bits on both sides of it; the one call still takes what the rule sends elsewhere."""
+    x = to_torch(synth((rows, cols), seed=cols, scale=1e-3))
+    blocks = rows * cols // (grid[0] * grid[1])
+    assert built_lib.pb_fake_quantize_blocks_workspace_size(1, rows, cols, *grid) == (4 * blocks if one_call else 0)
+    want = dequantize_impl(*quantize_impl(x, grid), torch.float32, grid)
+    out, ws = torch.empty_like(x), torch.empty(blocks, device="cuda")
+    assert built_lib.pb_fake_quantize_blocks(x.data_ptr(), 1, rows, cols, *grid, out.data_ptr(), ws.data_ptr(), 4 * blocks, torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(out, want) and torch.equal(_ops.fake_quantize_impl(x, grid, torch.float32), want)

@@ -15,6 +15,8 @@ CASES = [
     ((128, 272), (128, 16)), ((64, 264), (64, 8)), ((192, 320), (64, 64)), ((1024, 2048), (64, 32)),  # several blocks per warp, K above and below 32
     ((100, 256), (100, 128)), ((66, 128), (66, 64)), ((3, 128, 256), (128, 128)), ((2, 256, 136), (64, 1)),
     ((1024, 320), (1024, 1)), ((768, 144), (768, 1)), ((2, 1024, 192), (1024, 1)), ((1024, 2048), (512, 64)),      # K above 32, with super-groups that end inside a CTA's blocks
+    ((2048, 3200), (2048, 128)), ((1024, 9472), (512, 1)), ((192, 3200), (96, 128)),                  # many rows on many CTAs
+    ((4096, 256), (4096, 128)), ((2048, 256), (2048, 1)), ((512, 2048), (256, 32)), ((128, 128), (128, 1)),      # ... and on few: three kernels
     ((63, 128), (63, 64)), ((128, 6), (128, 1)), ((128, 96), (128, 48)),                              # the three-kernel form's side of the rule
 ]
 
