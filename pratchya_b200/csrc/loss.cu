@@ -12,24 +12,9 @@
 namespace pb {
 namespace {
 
-// Threads per row: 256, six rows at a time on an SM (40 registers); 1024 where there are too few rows for that (wide_rows).
+// Threads per row: 256, or 1024 where there are few long rows (wide_forward, wide_backward).
 constexpr int kLossThreads = 256, kWideThreads = 1024;
 constexpr int kLoads = 4;             // 16-byte loads that a thread has in flight
-
-template <int THREADS>
-__device__ __forceinline__ float block_reduce(float v, bool take_max, float* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float other = __shfl_xor_sync(0xffffffffu, v, o);
-    v = take_max ? fmaxf(v, other) : v + other;
-  }
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float r = red[0];
-  for (int w = 1; w < THREADS / 32; ++w) r = take_max ? fmaxf(r, red[w]) : r + red[w];
-  __syncthreads();
-  return r;
-}
 
 // A thread's maximum, sum of exp(z - maximum) and sum of z.  While the maximum is -inf (nothing but -inf seen) the
 // exponentials are taken from 0, so that -inf - -inf does not make a NaN of a logit that only weighs nothing.
@@ -38,7 +23,7 @@ struct RowTerms {
   __device__ __forceinline__ void raise(float top) {
     const float m2 = fmaxf(m, top);
     if (m2 > m) {
-      s *= expf(m - m2);               // m = -inf: 0 * 0
+      if (s != 0.0f) s *= expf(m - m2);      // the first logits have nothing to rescale
       m = m2;
     }
   }
@@ -47,18 +32,33 @@ struct RowTerms {
     s += (expf(v.x - base) + expf(v.y - base)) + (expf(v.z - base) + expf(v.w - base));
     zs += (v.x + v.y) + (v.z + v.w);
   }
+  // the terms of LANES lanes of a warp together, in each of them
+  template <int LANES>
+  __device__ __forceinline__ void over_lanes() {
+    float top = m;
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    s *= expf(m - (top == -INFINITY ? 0.0f : top));      // m = -inf: 0 * 0
+    m = top;
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+      zs += __shfl_xor_sync(0xffffffffu, zs, o);
+    }
+  }
 };
 __device__ __forceinline__ float top4(const float4& v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); }
 
 // row_loss[r] = weight[r] * loss_row, lse[r] kept for the backward pass.  One CTA per row, one read of it: a thread keeps a
-// running maximum and rescales its sum of exponentials where the maximum rises; the threads' terms meet at the end.
+// running maximum and rescales its sum of exponentials where the maximum rises; the threads' terms meet at the end, in their
+// warps and then in the first one, behind one barrier.
 // Bound by the 4 bytes per logit.  The form before read the row twice, maximum and sum of z first and the exponentials on
 // a second read from L2, with one 16-byte load of a thread in flight:
 // 4096 x 65536 logits 0.316 ms, now 0.17 ms (6.3 TB/s; the loss and its gradient 0.684 -> 0.537 ms).
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) smoothed_xent_fwd_kernel(const float* logits, const int64_t* target, const float* weight,
+template <int THREADS, int PER_SM>
+__global__ void __launch_bounds__(THREADS, PER_SM) smoothed_xent_fwd_kernel(const float* logits, const int64_t* target, const float* weight,
                                                                    float* row_loss, float* lse, int64_t vocab, float alpha) {
-  __shared__ float red[THREADS / 32];
+  __shared__ float red[3][THREADS / 32];
   const int64_t row = blockIdx.x;
   const float4* z4 = reinterpret_cast<const float4*>(logits + row * vocab);
   const int64_t quads = vocab / 4, whole = quads - quads % (THREADS * kLoads);
@@ -79,13 +79,18 @@ __global__ void __launch_bounds__(THREADS) smoothed_xent_fwd_kernel(const float*
     t.raise(top4(v));
     t.add(v);
   }
-  const float m = block_reduce<THREADS>(t.m, true, red);
-  const float s = block_reduce<THREADS>(t.s * expf(t.m - m), false, red);       // a row of -inf only: NaN, as its softmax is
-  const float zs = block_reduce<THREADS>(t.zs, false, red);
-  if (threadIdx.x == 0) {
-    const float l = m + logf(s);
+  t.over_lanes<32>();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) { red[0][warp] = t.m; red[1][warp] = t.s; red[2][warp] = t.zs; }
+  __syncthreads();
+  if (warp != 0) return;
+  RowTerms r;
+  if (lane < THREADS / 32) { r.m = red[0][lane]; r.s = red[1][lane]; r.zs = red[2][lane]; }
+  r.over_lanes<THREADS / 32>();
+  if (lane == 0) {
+    const float l = r.m + logf(r.s * expf(r.m - r.m));      // a row of -inf only: NaN, as its softmax is
     lse[row] = l;
-    row_loss[row] = weight[row] * (l - (1.0f - alpha) * logits[row * vocab + target[row]] - alpha * (zs / (float)vocab));
+    row_loss[row] = weight[row] * (l - (1.0f - alpha) * logits[row * vocab + target[row]] - alpha * (r.zs / (float)vocab));
   }
 }
 
@@ -111,8 +116,15 @@ __global__ void __launch_bounds__(THREADS) smoothed_xent_bwd_kernel(const float*
   }
 }
 
-// Fewer rows than the SMs hold at 256 threads each: four times the threads per row, where a row has loads for them.
-bool wide_rows(int64_t rows, int64_t vocab) { return rows < (int64_t)sm_count() * 6 && vocab >= kWideThreads * 4; }
+// Where 1024 threads a row are faster than 256.  A CTA of 1024 has an SM to itself in the forward pass, and a thread's few
+// loads do not pay for meeting at the end.  Forward, us, 256 | 1024 threads: 65536 logits 10.3 | 7.5 with 148 rows, 12.2 | 13.1
+// with 222; 16384 logits 4.4 | 4.2 with 148 rows; 8192 3.6 | 3.8; 4096 logits 4.3 | 11.6 with 740 rows.
+bool wide_forward(int64_t rows, int64_t vocab) { return rows <= sm_count() && vocab >= 16384; }
+// Backward: 4096 logits 3.0 | 2.6 with 148 rows, 3.4 | 3.4 with 296, 3.6 | 4.2 with 444; 16384 logits 7.3 | 5.9 with 296 rows,
+// 14.6 | 15.7 with 740; 32768 logits 38 | 35 with 740 rows; 65536 18.9 | 9.1 with 148 rows, 73 | 66 with 740.
+bool wide_backward(int64_t rows, int64_t vocab) {
+  return (vocab >= 4096 && rows <= 2 * (int64_t)sm_count()) || (vocab >= 32768 && rows < 6 * (int64_t)sm_count());
+}
 
 }  // namespace
 }  // namespace pb
@@ -126,10 +138,14 @@ extern "C" int pb_smoothed_xent(const float* logits, const int64_t* target, cons
     return fail(PB_ERR_BAD_SHAPE, "pb_smoothed_xent: rows=%lld vocab=%lld (vocab must be a multiple of 4)", (long long)rows, (long long)vocab);
   if (reinterpret_cast<uintptr_t>(logits) & 15) return fail(PB_ERR_MISALIGNED, "pb_smoothed_xent: logits must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (wide_rows(rows, vocab))
-    smoothed_xent_fwd_kernel<kWideThreads><<<(unsigned)rows, kWideThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
+  // eight CTAs on an SM (32 registers) where no thread has a whole round of loads, six otherwise: 4096 rows, 2048 logits 12.1 us with
+  // six and 11.5 with eight, 65536 logits 157 and 161
+  if (wide_forward(rows, vocab))
+    smoothed_xent_fwd_kernel<kWideThreads, 1><<<(unsigned)rows, kWideThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
+  else if (vocab < kLossThreads * kLoads * 4)
+    smoothed_xent_fwd_kernel<kLossThreads, 8><<<(unsigned)rows, kLossThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
   else
-    smoothed_xent_fwd_kernel<kLossThreads><<<(unsigned)rows, kLossThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
+    smoothed_xent_fwd_kernel<kLossThreads, 6><<<(unsigned)rows, kLossThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
   PB_LAUNCH_CHECK("smoothed_xent_fwd_kernel");
   return PB_OK;
 }
@@ -142,7 +158,7 @@ extern "C" int pb_smoothed_xent_bwd(const float* logits, const int64_t* target, 
   if ((reinterpret_cast<uintptr_t>(logits) & 15) || (reinterpret_cast<uintptr_t>(dlogits) & 15))
     return fail(PB_ERR_MISALIGNED, "pb_smoothed_xent_bwd: logits and dlogits must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (wide_rows(rows, vocab))
+  if (wide_backward(rows, vocab))
     smoothed_xent_bwd_kernel<kWideThreads><<<(unsigned)rows, kWideThreads, 0, st>>>(logits, target, weight, lse, upstream, 1.0f / denominator, dlogits, vocab, alpha);
   else
     smoothed_xent_bwd_kernel<kLossThreads><<<(unsigned)rows, kLossThreads, 0, st>>>(logits, target, weight, lse, upstream, 1.0f / denominator, dlogits, vocab, alpha);

@@ -19,7 +19,7 @@ def _run(z, target, weight, alpha):
     return loss, lse, dz
 
 
-@pytest.mark.parametrize("rows,vocab", [(3, 4), (2, 1020), (5, 4092), (5, 4096), (3, 4100), (2, 16384), (2, 16388), (1, 65536), (1000, 4096), (1000, 4100), (1000, 8)])
+@pytest.mark.parametrize("rows,vocab", [(3, 4), (2, 1020), (5, 4092), (5, 4096), (3, 4100), (2, 16384), (2, 16388), (1, 65536), (1000, 4096), (1000, 4100), (1000, 8), (400, 4092), (400, 8192), (500, 32768)])
 def test_rows_of_any_length(built_lib, rows, vocab):
     g = torch.Generator(device="cuda").manual_seed(rows + vocab)
     z = torch.randn(rows, vocab, generator=g, device="cuda") * 4
