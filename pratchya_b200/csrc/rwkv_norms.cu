@@ -184,35 +184,44 @@ template <> struct Chans<4> {
 };
 template <int V> __device__ __forceinline__ void load_chans(const float* p, float (&o)[V]) { Chans<V>::get(__ldg(reinterpret_cast<const typename Chans<V>::T*>(p)), o); }
 
-// One CTA per token: first the bonus dot product over all channels, then the output.  Bound by its five reads and one write of
-// [tokens, channels], or, four bytes at a time (V = 1: arrays off the 16-byte alignment), by the number of its loads, the
-// parameters' among them.  One warp per token (64 dependent rounds, and a warp for every token of a short prompt) came
-// before: 8 x 1024 tokens of 2048 channels 115 -> 73 us, 512 tokens 33 -> 7.5 us.
-template <int V>
+// WARPS of a CTA's eight per token, by its channels (see the launch): first the bonus dot product over all channels, then the
+// output.  Bound by its five reads and one write of [tokens, channels], or, four bytes at a time (V = 1: arrays off the 16-byte
+// alignment), by the number of its loads, the parameters' among them.  One warp per token whatever its channels (64 dependent
+// rounds for 2048 of them, and a warp for every token of a short prompt) came before: 8 x 1024 tokens of 2048 channels
+// 115 -> 73 us, 512 tokens 33 -> 7.5 us.
+template <int V, int WARPS>
 __global__ void __launch_bounds__(kThreads) wkv_finish_fwd_kernel(const FinishParams p) {
+  constexpr int kTokens = kWarps / WARPS, kGroup = 32 * WARPS;
   __shared__ float red[2][kWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = warp / WARPS, tid = threadIdx.x % kGroup;
   const int C = p.N * kH;
   int turn = 0;
-  for (int64_t row = blockIdx.x; row < p.R; row += gridDim.x, turn ^= 1) {
+  for (int64_t row0 = (int64_t)blockIdx.x * kTokens; row0 < p.R; row0 += (int64_t)gridDim.x * kTokens, turn ^= 1) {
+    const int64_t row = row0 + slot;
+    const bool mine = row < p.R;
     const size_t base = (size_t)row * C;
     float dot = 0.0f;
+    if (mine) {
 #pragma unroll 4
-    for (int c = threadIdx.x * V; c < C; c += kThreads * V) {
-      float r[V], k[V], m[V];
-      load_chans<V>(p.r + base + c, r); load_chans<V>(p.k + base + c, k); load_chans<V>(p.bonus_mult + c, m);
+      for (int c = tid * V; c < C; c += kGroup * V) {
+        float r[V], k[V], m[V];
+        load_chans<V>(p.r + base + c, r); load_chans<V>(p.k + base + c, k); load_chans<V>(p.bonus_mult + c, m);
 #pragma unroll
-      for (int e = 0; e < V; ++e) dot = fmaf(__fmul_rn(r[e], k[e]), m[e], dot);
+        for (int e = 0; e < V; ++e) dot = fmaf(__fmul_rn(r[e], k[e]), m[e], dot);
+      }
     }
     dot = warp_sum(dot);
-    if (lane == 0) red[turn][warp] = dot;
-    __syncthreads();              // the other half of `red` is written next, this one again only behind the next barrier
-    dot = red[turn][0];
+    if constexpr (WARPS > 1) {
+      if (lane == 0) red[turn][warp] = dot;
+      __syncthreads();            // the other half of `red` is written next, this one again only behind the next barrier
+      dot = red[turn][slot * WARPS];
 #pragma unroll
-    for (int w = 1; w < kWarps; ++w) dot += red[turn][w];
+      for (int w = 1; w < WARPS; ++w) dot += red[turn][slot * WARPS + w];
+    }
+    if (!mine) continue;
     const float* stats = p.stats + 2 * (size_t)(row / p.T) * p.N;
 #pragma unroll 4
-    for (int c = threadIdx.x * V; c < C; c += kThreads * V) {
+    for (int c = tid * V; c < C; c += kGroup * V) {
       const float mean = __ldg(stats + 2 * (c / kH)), rstd = __ldg(stats + 2 * (c / kH) + 1);      // V channels are of one head
       float y[V], v[V], gate[V], gs[V], gb[V], o[V];
       load_chans<V>(p.y + base + c, y); load_chans<V>(p.v + base + c, v); load_chans<V>(p.gate + base + c, gate);
@@ -444,8 +453,25 @@ extern "C" int pb_wkv_finish(const float* y, const float* r, const float* k, con
   group_stats_kernel<<<(groups + 127) / 128, 128, 0, st>>>(static_cast<const float*>(workspace), stats, groups, tiles, (float)steps * (float)kH, eps);
   PB_LAUNCH_CHECK("group_stats_kernel");
   FinishParams p{y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, stats, out, batch * steps, (int)steps, (int)heads};
-  if (any_misaligned({y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, out})) wkv_finish_fwd_kernel<1><<<blocks_for(p.R, 1), kThreads, 0, st>>>(p);
-  else wkv_finish_fwd_kernel<4><<<blocks_for(p.R, 1), kThreads, 0, st>>>(p);
+  // One head is no more than a warp's channels: four bytes at a time use all of its lanes.
+  const bool wide = heads > 1 && !any_misaligned({y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, out});
+  // A warp per four heads, and twice as many (all eight, four bytes at a time) where there are too few tokens to fill the SMs.
+  // Eight whatever the heads left most lanes without a load: 32768 tokens of two heads 116 us (one warp 41), of eight 150 (two
+  // warps 95); 8192 tokens of 16 heads 59 (four 56), of 32 heads 95.  One token of four heads: 5.8 us with one warp, 5.3 with two,
+  // of eight heads 7.2, 5.8 and 5.5 (four).
+  const int per_token = (heads <= 4 ? 1 : heads <= 8 ? 2 : heads <= 16 ? 4 : kWarps) * (p.R > 8 * sm_count() ? 1 : wide ? 2 : kWarps);
+  const int warps = per_token < kWarps ? per_token : kWarps;
+  const int grid = blocks_for(p.R, kWarps / warps);
+#define PB_FINISH_LAUNCH(V)                                                                    \
+  do {                                                                                         \
+    if (warps == 1)      wkv_finish_fwd_kernel<V, 1><<<grid, kThreads, 0, st>>>(p);            \
+    else if (warps == 2) wkv_finish_fwd_kernel<V, 2><<<grid, kThreads, 0, st>>>(p);            \
+    else if (warps == 4) wkv_finish_fwd_kernel<V, 4><<<grid, kThreads, 0, st>>>(p);            \
+    else                 wkv_finish_fwd_kernel<V, kWarps><<<grid, kThreads, 0, st>>>(p);       \
+  } while (0)
+  if (wide) PB_FINISH_LAUNCH(4);
+  else      PB_FINISH_LAUNCH(1);
+#undef PB_FINISH_LAUNCH
   PB_LAUNCH_CHECK("wkv_finish_fwd_kernel");
   return PB_OK;
 }

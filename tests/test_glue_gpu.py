@@ -5,6 +5,8 @@ ChannelMix, pratchya/_nnx_impl/_module.py:129-258), values and gradients.
 Forward values: bit-equal where the kernel performs the same f32 operations in the same order (lerps, rotary
 embedding, sigmoid, exp); 1e-6 of the largest magnitude where a 64-term sum is formed in another order (normalized).
 Gradients: 2e-5 of each gradient's largest magnitude against torch.autograd (sums over tokens in another order)."""
+import math
+
 import pytest
 import torch
 
@@ -252,3 +254,27 @@ def test_fused_cross_entropy_matches_torch(built_lib, bsz, steps, vocab):
     work = scratch * 1.0                                           # a non-leaf array that nothing else reads
     g_inplace, = torch.autograd.grad(fused(work, labels, reuse_logits=True) * 1.7, scratch)
     assert torch.equal(g_inplace, g_got)
+
+
+@pytest.mark.parametrize("n_head", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("bsz,steps", [(1, 1), (2, 7), (1, 1187)])       # fewer tokens than a CTA takes, a remainder, more than eight per SM
+@pytest.mark.parametrize("offset", [0, 1])
+def test_wkv_finish_for_any_number_of_heads_and_alignment(built_lib, n_head, bsz, steps, offset):
+    """Every split of a CTA over tokens, with 16-byte loads and (arrays one float off their alignment) with 4-byte ones."""
+    from pratchya_b200._nnx_impl._glue import wkv_finish
+    gen = torch.Generator(device="cuda").manual_seed(steps + n_head)
+    c = n_head * 64
+
+    def mk(*shape, scale=1.0, mean=0.0):
+        t = torch.empty(math.prod(shape) + offset, device="cuda")[offset:].view(shape)
+        return t.copy_(mean + scale * torch.randn(shape, device="cuda", generator=gen))
+
+    y, r, k, v, gate = mk(bsz, steps, c, scale=2.0, mean=0.3), *(mk(bsz, steps, c) for _ in range(4))
+    gs, gb, bm = mk(c, scale=0.1, mean=1.0), mk(c, scale=0.1), mk(c, scale=0.05)
+    got = wkv_finish(y, r, k, v, gate, gs, gb, bm, n_head * 1e-5, n_head)
+    y, r, k, v, gate, gs, gb, bm = (t.double() for t in (y, r, k, v, gate, gs, gb, bm))
+    g = y.view(bsz, steps, n_head, 64)
+    mean = g.mean(dim=(1, 3), keepdim=True)
+    var = (g * g).mean(dim=(1, 3), keepdim=True) - mean * mean
+    want = ((((g - mean) * torch.rsqrt(var + n_head * 1e-5)).view(bsz, steps, c) * gs + gb) + (r * k * bm).sum(-1, keepdim=True) * v) * gate
+    close(got, want, "wkv_finish", 2e-6)
