@@ -146,7 +146,8 @@ _SAME_DEVICE = contextlib.nullcontext()
 
 
 def on_device(device):
-    """`torch.cuda.device(device)` where that is not the current device already: the usual case costs a comparison."""
+    """`torch.cuda.device(device)` for a device with an index (a tensor's) where that is not the current one already: the usual
+    case costs a comparison."""
     return _SAME_DEVICE if torch._C._cuda_getDevice() == device.index else torch.cuda.device(device)
 
 

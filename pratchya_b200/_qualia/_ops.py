@@ -346,8 +346,11 @@ def _operand(q, sc8, sc32, rows, depth, grid, transposed_blocks=0) -> Operand:
 
 
 def gemm_tn(a: Operand, b: Operand, out_dtype, device, keep_alive=()) -> torch.Tensor:
-    """D[m, n] = sum_k dq(A)[m, k] * dq(B)[n, k] on the tcgen05 kernel."""
+    """D[m, n] = sum_k dq(A)[m, k] * dq(B)[n, k] on the tcgen05 kernel.  `device`: as torch takes it ("cuda" is the current one)."""
     lib = _lib.load()
+    device = torch.device(device)
+    if device.index is None:
+        device = torch.device(device.type, torch.cuda.current_device())
     with _lib.on_device(device):
         d = torch.empty((a.rows, b.rows), dtype=out_dtype, device=device)
         ws_bytes = lib.pb_gemm_workspace_size(a, b)

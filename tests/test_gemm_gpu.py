@@ -254,3 +254,12 @@ def test_low_rank_ffn_matches_the_oracle_chain(built_lib):
     # tanh differs in the last bit between numpy and the device, which can move an element of the second
     # quantization across an fp8 rounding boundary: 5e-3 of the maximum leaves room for a few of those
     assert np.abs(got - want).max() <= 5e-3 * scale, f"LowRankFFN differs from the oracle chain by {np.abs(got - want).max() / scale:.2e} of its maximum"
+
+
+def test_gemm_tn_takes_any_spelling_of_the_device(built_lib):
+    m, n, k = 128, 128, 1024
+    xq, wq = gpu_triple(synth((m, k), seed=1), (1, 128)), gpu_triple(synth((n, k), seed=2), (1, 128))
+    op = lambda t, rows: _ops._operand(t[0], t[1], t[2], rows, k, (1, 128))
+    want = _ops.gemm_tn(op(xq, m), op(wq, n), torch.float32, xq[0].device)
+    for device in (torch.device("cuda"), "cuda", "cuda:0", 0):
+        assert torch.equal(_ops.gemm_tn(op(xq, m), op(wq, n), torch.float32, device), want)
