@@ -939,19 +939,19 @@ int64_t tall_ctas(const Geometry& g, int64_t batch) {
   return ctas <= kMaxIndexed && g.nbc <= kMaxIndexed ? ctas : 0;
 }
 
-// Where it is the faster form.  A CTA walks the rows of its blocks alone (0.029 us a row in f32, 0.042 in bf16), so more rows want more
+// Where it is the faster form.  A CTA walks the rows of its blocks alone (0.025 us a row in f32, 0.032 in bf16), so more rows want more
 // CTAs beside it, and a walk of thousands of rows that lie far apart falls to a third of its rate; the three-kernel form
-// spreads any grid, at an atomicMax per vector: the wider the block the more of them meet.  Both, us, one call:
-//   128 rows, f32: 8.7 | 8.6 (three | two kernels) with one CTA, 22 | 9 with 74.  bf16, (128,128): 9.7 | 10.3 with 4, 14 | 11 with 16
-//   (1024,128) f32: 31 | 34 with 16, 42 | 34 with 24, 107 | 37 with 148.  (4096,128), 64 CTAs: 364 | 306 in f32, 373 | 431 in bf16
-//   (1024,1) f32: 30 | 44 with 48, 45 | 45 with 74, 86 | 49 with 148.  (2048,1) f32, 148 CTAs: 172 | 211
-//   (512,16) f32: 17 | 20 with 74, 60 | 65 with 592.
-template <typename InT>
+// spreads any grid, at an atomicMax per vector: the wider the block the more of them meet.  Three | two kernels, us:
+//   128 rows: 8.5 | 7.9 with one CTA, 22 | 8 with 74 (f32, (128,128)); bf16 9.1 | 8.6 and 23 | 10; (128,16) bf16 8.3 | 9.0 with 74
+//   (1024,128) f32: 15 | 29 with 4 CTAs, 31 | 29 with 16, 105 | 32 with 148.  bf16: 20 | 36, 49 | 36, 202 | 49
+//   (1024,1) f32: 24 | 30 with 25, 40 | 31 with 48, 82 | 33 with 148.  bf16: 35 | 44, 57 | 45, 176 | 60
+//   (2048,1) f32: 40 | 54 with 25, 60 | 55 with 48, 187 | 132 with 148.  (4096,1): 200 | 242 with 74
+//   (4096,128), 48 CTAs: 271 | 231 in f32, 358 | 261 in bf16; (16384,128), 16: 374 | 1054 before this kernel's last 10 %
+//   (512,16) f32: 17 | 17 with 74, 58 | 61 with 592.
 bool tall_pays(const Geometry& g, int64_t ctas) {
-  if (g.a <= (sizeof(InT) == 4 ? 128 : 96)) return true;
-  if (g.a <= 128) return ctas >= 16;
-  if (g.b >= 128) return g.a <= 2048 && 6 * ctas >= sm_count();
-  return g.b == 1 && g.a <= 1024 && 2 * ctas >= sm_count();
+  if (g.a <= 128) return true;
+  if (g.a > 2048) return false;
+  return g.b >= 128 ? 9 * ctas >= sm_count() : g.b == 1 && 3 * ctas >= sm_count();
 }
 
 template <typename InT>
@@ -1005,7 +1005,7 @@ template <typename InT, int VEC>
 int launch_generic(const InT* x, const Geometry& g, int64_t batch, int fmt, uint8_t* q, uint8_t* sc8, float* sc32,
                    void* workspace, cudaStream_t st) {
   const int64_t ctas = tall_ctas<InT>(g, batch);
-  if (ctas > 0 && tall_pays<InT>(g, ctas) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & (TallVec<InT>::kN - 1)) == 0)
+  if (ctas > 0 && tall_pays(g, ctas) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(q) & (TallVec<InT>::kN - 1)) == 0)
     return launch_tall(x, g, batch, fmt, q, sc8, sc32, workspace, st);
   const int64_t nblk = batch * g.Nb;
   uint32_t* amax_bits = static_cast<uint32_t*>(workspace);
@@ -1324,7 +1324,7 @@ extern "C" size_t pb_fake_quantize_blocks_workspace_size(int64_t batch, int64_t 
   Geometry g;
   if (batch <= 0 || make_geometry(rows, cols, a, b, &g) != PB_OK) return 0;
   const int64_t ctas = tall_ctas<float>(g, batch);
-  return ctas > 0 && tall_pays<float>(g, ctas) ? (size_t)(batch * g.Nb) * 4 : 0;
+  return ctas > 0 && tall_pays(g, ctas) ? (size_t)(batch * g.Nb) * 4 : 0;
 }
 
 extern "C" int pb_fake_quantize_blocks(const float* x, int64_t batch, int64_t rows, int64_t cols, int a, int b, float* out,
