@@ -470,8 +470,8 @@ _LITERAL_DOT_TF32 = False
 def set_literal_dot_precision(precision: str) -> None:
     """Precision of the f32 dots behind the grids the block-scaled kernel cannot take (the reference's literal recipe
     there: dequantize, then an f32 dot).  "f32" (default) keeps full f32 products (`literal_dots`: on the tensor cores
-    where it can, else the library matmul); "tf32" lets the library round the operands to 10 mantissa bits, which is what an f32 dot gets on a GPU under XLA's default
-    precision, and is several times faster."""
+    where it can, else the library matmul); "tf32" lets the library round the operands to 10 mantissa bits, which is
+    what an f32 dot gets on a GPU under XLA's default precision, and is several times faster."""
     global _LITERAL_DOT_TF32
     if precision not in ("f32", "tf32"):
         raise ValueError(f"precision must be 'f32' or 'tf32', got {precision!r}")

@@ -25,12 +25,13 @@
 // while the other fills, and one lane of theirs issues tcgen05.mma.  Where the tiles do not fill the SMs the contraction is
 // cut, and the parts are added in order by a second kernel.
 //
-// What bounds it: no one part.  A stage takes 2800 cycles, of which the tensor core works 768; before the loads moved behind the
+// What bounds it: no one part.  A stage of dX takes 2800 cycles (of dW 3500), of which the tensor core works 768; before the loads moved behind the
 // fence, dX took 17 % less with the split left out, 14 with the loads, 13 with the emptying, 8 with eleven of the twelve
-// products (dW: 28, 40, 11, 5), and sixteen converting warps were no faster than eight.  Against the library's SGEMM alone (the
-// dequantization of both operands came on top), 3000 tokens, 2048 x 2048: dX 488 -> 155 us, dW 430 -> 202; 8192 tokens,
-// 2048 x 128: 100 -> 67 and 124 -> 45; 64 tokens, 1024 x 1024: 22 -> 25, 16 -> 16.  A bf16 g is read as it is: 146 and 186 us for the
-// 3000 tokens, and no f32 copy of it.
+// products (dW: 28, 40, 11, 5), and sixteen converting warps were no faster than eight.  Against dequantizing and the library's
+// SGEMM (inside a CUDA graph): 3000 tokens, 2048 x 2048, dX 491 -> 143 us, dW 432 -> 175 (bf16 g, read as it is: 507 -> 142 and
+// 448 -> 179); 8192 tokens, 2048 x 128, 100 -> 62 and 139 -> 37; 64 tokens, 1024 x 1024, 22 -> 14 and 9 -> 8.5.  Where there is less
+// than that to do the library's kernels are shorter (64 tokens, 2048 x 128, 8 | 10 and 7 | 8), but a call of it is not: one after
+// the other the two dots take 48 us there and these 24, for the host's part of four library calls.
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
