@@ -70,6 +70,7 @@ _SIGNATURES = {
     "pb_gemm_check": (_int, [_ptr]),
     "pb_transpose_bytes": (_int, [_ptr, _i64, _i64, _ptr, _ptr]),
     "pb_dense_dot_workspace_size": (_sz, [_int, _i64, _i64, _int, _int, _i64]),
+    "pb_dense_dot_workspace_best": (_sz, [_int, _i64, _i64, _int, _int, _i64, _int]),
     "pb_dense_dot": (_int, [_int, _ptr, _ptr, _ptr, _i64, _i64, _int, _int, _ptr, _int, _i64, _ptr, _ptr, _sz, _ptr]),
     "pb_token_shift_lerp": (_int, [_ptr, _ptr, _ptr, _i64, _i64, _i64, _int, _ptr, _ptr]),
     "pb_token_shift_lerp_bwd_workspace_size": (_sz, [_i64, _i64, _i64, _int]),

@@ -32,11 +32,16 @@
 // 448 -> 179); 8192 tokens, 2048 x 128, 100 -> 62 and 139 -> 37; 64 tokens, 1024 x 1024, 22 -> 14 and 9 -> 8.5.  Where there is less
 // than that to do the library's kernels are shorter (64 tokens, 2048 x 128, 8 | 10 and 7 | 8), but a call of it is not: one after
 // the other the two dots take 48 us there and these 24, for the host's part of four library calls.
+//
+// Every tile converts what it reads, so an operand that many tiles share is converted many times: where 512 columns or more share
+// it and there is enough to do, split_dot.cu makes it ready once (split_dot_pays: 3000 tokens, 2048 x 2048, bf16 cotangent, dX 141 -> 75 us,
+// dW 178 -> 68).  Left to this form are few tokens, the low-rank layers' f32 cotangents and callers without the workspace.
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
+#include "split_dot.cuh"
 
 namespace pb {
 namespace {
@@ -485,6 +490,9 @@ int dense_dot_status_fetch(unsigned int* out) {
   const unsigned int zero = 0;
   PB_CUDA_TRY(cudaMemcpyFromSymbol(out, g_dot_status, sizeof(*out)));
   if (*out != 0) PB_CUDA_TRY(cudaMemcpyToSymbol(g_dot_status, &zero, sizeof(zero)));
+  unsigned int split = 0;
+  if (int s = split_dot_status_fetch(&split)) return s;
+  if (split != 0) *out = split;
   return PB_OK;
 }
 }  // namespace pb
@@ -495,6 +503,15 @@ extern "C" size_t pb_dense_dot_workspace_size(int tokens, int64_t rows, int64_t 
   if (!dot_shape_ok(tokens, rows, cols, a, b, g_free)) return 0;
   const DotPlan d = make_plan(tokens, rows, cols, g_free);
   return d.splits > 1 ? (size_t)d.splits * d.I * d.J * sizeof(float) : 0;
+}
+
+extern "C" size_t pb_dense_dot_workspace_best(int tokens, int64_t rows, int64_t cols, int a, int b, int64_t g_free, int g_dtype) {
+  const size_t least = pb_dense_dot_workspace_size(tokens, rows, cols, a, b, g_free);
+  SplitDotPlan split;
+  if ((g_dtype != PB_F32 && g_dtype != PB_BF16) || !dot_shape_ok(tokens, rows, cols, a, b, g_free) ||
+      !split_dot_plan(tokens, rows, cols, a, b, g_free, g_dtype == PB_BF16, &split))
+    return least;
+  return std::max(least, split.bytes);
 }
 
 extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, const float* sc32, int64_t rows, int64_t cols, int a, int b,
@@ -516,6 +533,9 @@ extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, co
   if (need && (!workspace || workspace_bytes < need))
     return fail(PB_ERR_WORKSPACE_TOO_SMALL, "pb_dense_dot: needs %zu bytes of workspace, got %zu", need, workspace_bytes);
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return fail(PB_ERR_MISALIGNED, "pb_dense_dot: workspace must be 16-byte aligned");
+  SplitDotPlan split;
+  if (workspace && !(reinterpret_cast<uintptr_t>(workspace) & 31) && split_dot_plan(tokens, rows, cols, a, b, g_free, g_dtype == PB_BF16, &split) && workspace_bytes >= split.bytes)
+    return split_dot_run(split, tokens, q, sc8, sc32, rows, cols, a, b, g, g_dtype == PB_BF16, g_free, out, workspace, static_cast<cudaStream_t>(stream));
   uint32_t log2_K = 0;                  // K divides 8, or 1024 for (128,128)
   while ((1ll << log2_K) < geo.K) ++log2_K;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -544,6 +564,7 @@ extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, co
 extern "C" PB_API int pb_debug_dot_control(unsigned int polls, int withhold) {
   g_dot_polls.store(polls ? polls : kWaitPolls);
   g_dot_withhold.store(withhold);
+  split_dot_control(polls, withhold);
   return PB_OK;
 }
 #endif

@@ -1,0 +1,25 @@
+// The form of the literal f32 dots whose operands are made ready for the tensor core once (split_dot.cu), for dense_dot.cu.
+#pragma once
+
+#include <cstddef>
+#include <cstdint>
+
+#include <cuda_runtime.h>
+
+namespace pb {
+
+struct SplitDotPlan {
+  int n, tiles, row_tiles, splits, units, units_per_split, variants, nbc, log2_K;
+  int64_t slab;                       // rows of the three-term operand at a time
+  size_t off_other, off_parts, bytes; // of the workspace, which starts with the terms
+};
+// False where dense_dot_kernel takes the call: shapes this form does not take, and those it is not faster for.
+bool split_dot_plan(int tokens, int64_t rows, int64_t cols, int a, int b, int64_t g_free, bool g_bf16, SplitDotPlan* d);
+int split_dot_run(const SplitDotPlan& d, int tokens, const uint8_t* q, const uint8_t* sc8, const float* sc32, int64_t rows, int64_t cols, int a, int b,
+                  const void* g, bool g_bf16, int64_t g_free, float* out, void* workspace, cudaStream_t st);
+int split_dot_status_fetch(unsigned int* out);
+#ifdef PB_DIAGNOSTICS
+void split_dot_control(uint32_t polls, int withhold);
+#endif
+
+}  // namespace pb

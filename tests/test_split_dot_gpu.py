@@ -1,0 +1,133 @@
+"""pb_dense_dot's form for operands that many tiles share (the fastest workspace), against 64-bit products and against the form that
+needs no workspace: remainders of its tiles in every direction, every tile width, contractions cut and not, several sets and
+several rounds of terms, powers of two that bf16 does not hold, infinities and NaNs."""
+import pytest
+import torch
+
+from pratchya_b200 import _lib
+from pratchya_b200._qualia import dequantize_impl, quantize_impl
+
+pytestmark = pytest.mark.gpu
+
+F32, BF16 = torch.float32, torch.bfloat16
+PB_ERR_DEVICE_TIMEOUT = 7
+
+
+def _dot(lib, tokens, triple, grid, g, best=True):
+    """(out, whether the workspace is the fastest form's)"""
+    q, sc8, sc32 = triple
+    rows, cols = q.shape
+    free, code = g.shape[1] if tokens else g.shape[0], _lib.PB_BF16 if g.dtype == BF16 else _lib.PB_F32
+    least = lib.pb_dense_dot_workspace_size(tokens, rows, cols, *grid, free)
+    size = lib.pb_dense_dot_workspace_best(tokens, rows, cols, *grid, free, code) if best else least
+    ws = torch.full((max(size, 16),), 0xff, dtype=torch.uint8, device="cuda")          # NaNs, as bf16 and as f32
+    out = torch.full((cols, free) if tokens else (free, rows), float("nan"), device="cuda")
+    status = lib.pb_dense_dot(tokens, q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), rows, cols, *grid, g.data_ptr(), code, free, out.data_ptr(),
+                              ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream)
+    assert status == 0, lib.pb_last_error()
+    return out, size > least
+
+
+def _sums(tokens, triple, grid, g):
+    d = dequantize_impl(*triple, F32, grid).double()
+    return (d.t(), g.double()) if tokens else (g.double(), d.t())
+
+
+def _bound(a, b):
+    """Per element, |a| @ |b| times the roundings of this form: one of an operand (2^-24), up to two of a factor on the finished sum, the
+    tensor core's within 64 of the contraction (twelve additions of at most 2^-23, of which eight make the low terms) and one
+    addition per 64 of it or per part."""
+    return (a.abs() @ b.abs()) * 2.0 ** -24 * (27 + (a.shape[1] + 63) // 64 + 16)
+
+
+def _inputs(rows, cols, grid, free, tokens, dtype, amp=1.0):
+    g = torch.Generator(device="cuda").manual_seed(rows + 3 * cols + free)
+    x = torch.randn(rows, cols, generator=g, device="cuda") * torch.randn(rows, 1, generator=g, device="cuda").exp() * 0.02
+    cot = torch.randn(rows if tokens else free, free if tokens else cols, generator=g, device="cuda") * 1e-3 * amp
+    return quantize_impl(x, grid), cot.to(dtype)
+
+
+# tokens, rows, cols, grid, free: the widths of a tile are chosen by how the tiles fill 148 SMs
+CASES = [(0, 2048, 2048, (128, 128), 3001), (0, 1024, 1024, (128, 128), 1031), (0, 512, 2048, (128, 128), 777), (0, 4096, 528, (128, 1), 600), (0, 1024, 4096, (128, 128), 260),
+         (0, 1152, 640, (128, 1), 2050), (1, 3001, 2048, (1, 128), 2048), (1, 193, 1024, (1, 128), 1032), (1, 1000, 512, (1, 128), 520), (1, 401, 3072, (1, 128), 648),
+         (1, 4100, 2048, (1, 128), 128), (1, 777, 640, (1, 128), 1024), (1, 256, 1024, (1, 128), 2056)]
+
+
+@pytest.mark.parametrize("tokens,rows,cols,grid,free", CASES)
+@pytest.mark.parametrize("dtype", [F32, BF16])
+def test_sums_against_64_bits_and_the_other_form(built_lib, tokens, rows, cols, grid, free, dtype):
+    triple, g = _inputs(rows, cols, grid, free, tokens, dtype)
+    got, shared = _dot(built_lib, tokens, triple, grid, g)
+    plain, _ = _dot(built_lib, tokens, triple, grid, g, best=False)
+    a, b = _sums(tokens, triple, grid, g)
+    want, bound = a @ b, _bound(a, b)
+    assert ((got.double() - want).abs() <= bound + 1e-37).all()
+    assert ((got - plain).abs().double() <= 2 * bound + 1e-37).all()
+    error = lambda o: ((o.double() - want).norm() / want.norm()).item()
+    assert error(got) <= error(plain) * 1.02                     # never the less precise of the two
+    again, _ = _dot(built_lib, tokens, triple, grid, g)
+    assert torch.equal(got, again)
+    assert built_lib.pb_gemm_check(torch.cuda.current_stream().cuda_stream) == 0
+
+
+def test_the_cases_reach_this_form(built_lib):
+    """A changed rule that leaves these cases to the other form would leave this one untested."""
+    size = lambda c, code: built_lib.pb_dense_dot_workspace_best(c[0], c[1], c[2], *c[3], c[4], code) - built_lib.pb_dense_dot_workspace_size(c[0], c[1], c[2], *c[3], c[4])
+    assert sum(size(c, _lib.PB_BF16) > 0 for c in CASES) >= 11 and sum(size(c, _lib.PB_F32) > 0 for c in CASES) >= 8
+    assert size((0, 4096, 528, (128, 1), 600), _lib.PB_F32) == 0           # a factor per column of the contraction
+    assert size((1, 777, 640, (1, 128), 1024), _lib.PB_F32) == 0           # super-groups that end inside a row
+
+
+@pytest.mark.parametrize("tokens,rows,cols,grid,free,dtype", [(1, 8200, 2048, (1, 128), 8192, F32), (1, 8200, 11264, (1, 128), 512, BF16), (0, 11264, 8208, (128, 1), 512, BF16)])
+def test_several_rounds_of_terms(built_lib, tokens, rows, cols, grid, free, dtype):
+    triple, g = _inputs(rows, cols, grid, free, tokens, dtype)
+    got, shared = _dot(built_lib, tokens, triple, grid, g)
+    assert shared
+    a, b = _sums(tokens, triple, grid, g)
+    assert ((got.double() - a @ b).abs() <= _bound(a, b) + 1e-37).all()
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("tokens", [0, 1])
+def test_infinities_nans_and_blocks_far_below_their_group(built_lib, tokens, dtype):
+    """Blocks 2^-118 and less of their super-group's largest value (their power of two times an fp8 value has no normal bf16), an
+    infinite and a NaN cotangent: what the form without a workspace gives, whose sums are f32 products where they are not finite."""
+    rows, cols, grid, free = (512, 1024, (1, 128), 1024) if tokens else (1024, 1024, (128, 128), 600)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(rows, cols, generator=g, device="cuda")
+    x[:, 128:256] *= 2.0 ** -118
+    if not tokens:
+        x[256:384] *= 2.0 ** -120
+    triple = quantize_impl(x, grid)
+    cot = (torch.randn(rows if tokens else free, free if tokens else cols, generator=g, device="cuda") * 1e20).to(dtype)
+    got, shared = _dot(built_lib, tokens, triple, grid, cot)
+    assert shared
+    a, b = _sums(tokens, triple, grid, cot)
+    want = a @ b
+    assert ((got.double() - want).abs() <= (a.abs() @ b.abs()) * 2.0 ** -24 * (a.shape[1] + 4) + a.shape[1] * 2.0 ** -149).all()
+    cot = cot * 1e-20
+    cot[(5, 17) if tokens else (17, 5)], cot[(9, 33) if tokens else (33, 9)] = float("inf"), float("nan")
+    got = _dot(built_lib, tokens, triple, grid, cot)[0]
+    got = got if tokens else got.t()                             # [i, j]: the cotangents' rows j are 17 and 33
+    rest = [j for j in range(got.shape[1]) if j not in (17, 33)]
+    assert torch.isnan(got[:, 33]).all() and not torch.isfinite(got[:, 17]).any() and torch.isfinite(got[:, rest]).all()
+
+
+@pytest.mark.parametrize("tokens", [0, 1])
+def test_a_wait_that_runs_out_is_reported_and_the_next_launch_is_clean(built_lib, diag_lib, tokens):
+    """The diagnostics build leaves the first stage of a launch unfilled, with a poll budget of about two milliseconds per wait."""
+    rows, cols, grid, free = (600, 1024, (1, 128), 512) if tokens else (1024, 1024, (128, 128), 600)
+    triple, g = _inputs(rows, cols, grid, free, tokens, F32)
+    st = torch.cuda.current_stream().cuda_stream
+    before, shared = _dot(diag_lib, tokens, triple, grid, g)
+    assert shared and diag_lib.pb_gemm_check(st) == 0
+    try:
+        assert diag_lib.pb_debug_dot_control(1 << 10, 1) == 0
+        _dot(diag_lib, tokens, triple, grid, g)
+        assert diag_lib.pb_gemm_check(st) == PB_ERR_DEVICE_TIMEOUT and b"dense-dot" in diag_lib.pb_last_error()
+        assert diag_lib.pb_gemm_check(st) == 0                   # reading the status clears it
+    finally:
+        diag_lib.pb_debug_dot_control(0, 0)
+    after, _ = _dot(diag_lib, tokens, triple, grid, g)
+    assert diag_lib.pb_gemm_check(st) == 0 and torch.equal(before, after)
+    assert built_lib.pb_gemm_check(st) == 0
