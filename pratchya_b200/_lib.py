@@ -143,6 +143,24 @@ def load_diagnostics():
     return _diag_lib
 
 
+_native = None
+
+
+def native():
+    """The extension that runs the ops' host side (csrc/native.cc); raises if it has not been built."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from .csrc import _native as module
+        except ImportError as e:
+            raise RuntimeError("pratchya_b200/csrc/_native.so is missing or does not load: build it with "
+                               "`python -m pratchya_b200.csrc.build` (there is no other host path for the ops)") from e
+        module.set_error(PbError)
+        _native = module
+    return _native
+
+
 _SAME_DEVICE = contextlib.nullcontext()
 
 

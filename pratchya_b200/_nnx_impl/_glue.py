@@ -9,48 +9,37 @@ import ctypes as C
 import torch
 
 from .. import _lib
-from .._lib import check
+from ._nograph import run
+
+_E4M3, _E8M0 = torch.float8_e4m3fn, torch.float8_e8m0fnu
 
 
 def _f32c(t):
-    return t.to(torch.float32).contiguous()
-
-
-def _stream(dev):
-    return _lib.current_stream(dev)
+    return t if t.dtype is torch.float32 and t.is_contiguous() else t.to(torch.float32).contiguous()
 
 
 class _ShiftLerpFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, state, mu):
-        lib = _lib.load()
+        nat = _lib.native()
         bsz, steps, chans = x.shape
         n_mix = mu.shape[0]
-        out = torch.empty((n_mix, bsz, steps, chans), dtype=torch.float32, device=x.device)
-        with _lib.on_device(x.device):
-            check(lib.pb_token_shift_lerp(x.data_ptr(), state.data_ptr() if state is not None else None, mu.data_ptr(),
-                                          bsz, steps, chans, n_mix, out.data_ptr(), _stream(x.device)))
+        out = nat.empty((n_mix, bsz, steps, chans), torch.float32, x)
+        nat.pb_token_shift_lerp(x, state, mu, bsz, steps, chans, n_mix, out)
         ctx.save_for_backward(x, state, mu)
         return tuple(out.unbind(0))          # separate outputs: their cotangents arrive separately, with no stacking copy
 
     @staticmethod
     def backward(ctx, *gs):
         x, state, mu = ctx.saved_tensors
-        lib = _lib.load()
+        nat = _lib.native()
         bsz, steps, chans = x.shape
         n_mix = mu.shape[0]
-        dev = x.device
-        with _lib.on_device(dev):
-            gs = [_f32c(g) if g is not None else torch.zeros_like(x) for g in gs]
-            g_ptrs = (C.c_void_p * n_mix)(*[g.data_ptr() for g in gs])
-            dx = torch.empty_like(x)
-            dstate = torch.empty_like(state) if state is not None else None
-            dmu = torch.empty_like(mu)
-            ws_bytes = lib.pb_token_shift_lerp_bwd_workspace_size(bsz, steps, chans, n_mix)
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-            check(lib.pb_token_shift_lerp_bwd(g_ptrs, x.data_ptr(), state.data_ptr() if state is not None else None, mu.data_ptr(),
-                                              bsz, steps, chans, n_mix, dx.data_ptr(), dstate.data_ptr() if dstate is not None else None,
-                                              dmu.data_ptr(), ws.data_ptr(), ws_bytes, _stream(dev)))
+        gs = [_f32c(g) if g is not None else torch.zeros_like(x) for g in gs]
+        g_ptrs = (C.c_void_p * n_mix)(*[g.data_ptr() for g in gs])
+        dx, dstate, dmu = nat.empties(x, 1)[0], nat.empties(state, 1)[0] if state is not None else None, nat.empties(mu, 1)[0]
+        ws_bytes = nat.pb_token_shift_lerp_bwd_workspace_size(bsz, steps, chans, n_mix)
+        nat.pb_token_shift_lerp_bwd(g_ptrs, x, state, mu, bsz, steps, chans, n_mix, dx, dstate, dmu, nat.empty((ws_bytes,), torch.uint8, x), ws_bytes)
         return dx, dstate, dmu
 
 
@@ -66,7 +55,7 @@ def token_shift_lerp(x, state, mu):
         if tuple(state.shape) != (x.shape[0], 1, x.shape[2]):
             raise ValueError(f"token_shift_lerp: state {tuple(state.shape)} for x {tuple(x.shape)}")
         st = _f32c(state)
-    return _ShiftLerpFn.apply(_f32c(x), st, _f32c(mu))
+    return run(_ShiftLerpFn, _f32c(x), st, _f32c(mu))
 
 
 class QuantizedMix:
@@ -87,24 +76,17 @@ class QuantizedMix:
 class _ShiftLerpQuantFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, state, mu, mask):
-        lib = _lib.load()
+        nat = _lib.native()
         bsz, steps, chans = x.shape
         n_mix, rows = mu.shape[0], bsz * steps
         n_t = bin(mask).count("1")
-        dev = x.device
         groups = rows * chans // 1024
-        with _lib.on_device(dev):
-            q = torch.empty((n_mix, rows, chans), dtype=torch.float8_e4m3fn, device=dev)
-            sc8 = torch.empty((n_mix, groups, 8), dtype=torch.float8_e8m0fnu, device=dev)
-            sc32 = torch.empty((n_mix, groups, 1, 1), dtype=torch.float32, device=dev)
-            q_t = torch.empty((n_t, chans, rows), dtype=torch.float8_e4m3fn, device=dev)
-            sc8_t = torch.empty((n_t, groups, 8), dtype=torch.float8_e8m0fnu, device=dev)
-            sc32_t = torch.empty((n_t, groups, 1, 1), dtype=torch.float32, device=dev)
-            check(lib.pb_shift_lerp_quantize(x.data_ptr(), state.data_ptr() if state is not None else None, mu.data_ptr(), bsz, steps, chans, n_mix,
-                                             q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), mask,
-                                             q_t.data_ptr() if n_t else None, sc8_t.data_ptr() if n_t else None, sc32_t.data_ptr() if n_t else None,
-                                             _stream(dev)))
-            handles = tuple(torch.zeros(1, dtype=torch.float32, device=dev).expand(bsz, steps, chans) for _ in range(n_mix))
+        q, sc8, sc32 = nat.empty((n_mix, rows, chans), _E4M3, x), nat.empty((n_mix, groups, 8), _E8M0, x), nat.empty((n_mix, groups, 1, 1), torch.float32, x)
+        q_t, sc8_t, sc32_t = nat.empty((n_t, chans, rows), _E4M3, x), nat.empty((n_t, groups, 8), _E8M0, x), nat.empty((n_t, groups, 1, 1), torch.float32, x)
+        nat.pb_shift_lerp_quantize(x, state, mu, bsz, steps, chans, n_mix, q, sc8, sc32, mask,
+                                   q_t if n_t else None, sc8_t if n_t else None, sc32_t if n_t else None)
+        zero = torch.zeros(1, dtype=torch.float32, device=x.device)
+        handles = tuple(zero.expand(bsz, steps, chans) for _ in range(n_mix))
         ctx.save_for_backward(x, state, mu)
         ctx.mark_non_differentiable(q, sc8, sc32, q_t, sc8_t, sc32_t)
         ctx.set_materialize_grads(False)      # no zero-filled fp8 arrays for the triples' absent cotangents
@@ -137,7 +119,7 @@ def token_shift_lerp_quantized(x, state, mu, transposed=()):
         if not 0 <= k < n_mix:
             raise ValueError(f"token_shift_lerp_quantized: transposed index {k} of {n_mix} mixes")
         mask |= 1 << k
-    out = _ShiftLerpQuantFn.apply(_f32c(x), st, _f32c(mu), mask)
+    out = run(_ShiftLerpQuantFn, _f32c(x), st, _f32c(mu), mask)
     handles, (q, sc8, sc32, q_t, sc8_t, sc32_t) = out[:n_mix], out[n_mix:]
     mixes, slot = [], 0
     for k in range(n_mix):
@@ -156,14 +138,10 @@ def can_quantize_mixes(x, want_transposed):
 class _WkvPrepareFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, r_raw, k_raw, d, iclr_raw, v_prime, v0, nu_raw, cos_tab, sin_tab, rk_mult, mix_amt, n_head):
-        lib = _lib.load()
+        nat = _lib.native()
         bsz, steps, chans = r_raw.shape
-        outs = [torch.empty_like(r_raw) for _ in range(7)]
-        with _lib.on_device(r_raw.device):
-            check(lib.pb_wkv_prepare(r_raw.data_ptr(), k_raw.data_ptr(), d.data_ptr(), iclr_raw.data_ptr(), v_prime.data_ptr(),
-                                     v0.data_ptr() if v0 is not None else None, nu_raw.data_ptr() if nu_raw is not None else None,
-                                     cos_tab.data_ptr(), sin_tab.data_ptr(), rk_mult.data_ptr(), mix_amt.data_ptr(),
-                                     bsz, steps, n_head, chans // n_head, *[o.data_ptr() for o in outs], _stream(r_raw.device)))
+        outs = nat.empties(r_raw, 7)
+        nat.pb_wkv_prepare(r_raw, k_raw, d, iclr_raw, v_prime, v0, nu_raw, cos_tab, sin_tab, rk_mult, mix_amt, bsz, steps, n_head, chans // n_head, *outs)
         ctx.save_for_backward(r_raw, k_raw, d, iclr_raw, v_prime, v0, nu_raw, cos_tab, sin_tab, rk_mult, mix_amt)
         ctx.n_head = n_head
         return tuple(outs)
@@ -171,25 +149,16 @@ class _WkvPrepareFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *grads):
         r_raw, k_raw, d, iclr_raw, v_prime, v0, nu_raw, cos_tab, sin_tab, rk_mult, mix_amt = ctx.saved_tensors
-        lib = _lib.load()
+        nat = _lib.native()
         bsz, steps, chans = r_raw.shape
         n_head = ctx.n_head
-        dev = r_raw.device
-        with _lib.on_device(dev):
-            gs = [_f32c(g) if g is not None else torch.zeros_like(r_raw) for g in grads]
-            douts = [torch.empty_like(r_raw) for _ in range(5)]
-            d_v0 = torch.empty_like(r_raw) if v0 is not None else None
-            d_nu = torch.empty_like(r_raw) if v0 is not None else None
-            d_rk, d_mix = torch.empty_like(rk_mult), torch.empty_like(mix_amt)
-            ws_bytes = lib.pb_wkv_prepare_bwd_workspace_size(bsz, steps, n_head, chans // n_head)
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-            check(lib.pb_wkv_prepare_bwd(r_raw.data_ptr(), k_raw.data_ptr(), d.data_ptr(), iclr_raw.data_ptr(), v_prime.data_ptr(),
-                                         v0.data_ptr() if v0 is not None else None, nu_raw.data_ptr() if nu_raw is not None else None,
-                                         cos_tab.data_ptr(), sin_tab.data_ptr(), rk_mult.data_ptr(), mix_amt.data_ptr(),
-                                         bsz, steps, n_head, chans // n_head, *[g.data_ptr() for g in gs],
-                                         *[o.data_ptr() for o in douts], d_v0.data_ptr() if d_v0 is not None else None,
-                                         d_nu.data_ptr() if d_nu is not None else None, d_rk.data_ptr(), d_mix.data_ptr(),
-                                         ws.data_ptr(), ws_bytes, _stream(dev)))
+        gs = [_f32c(g) if g is not None else torch.zeros_like(r_raw) for g in grads]
+        douts = nat.empties(r_raw, 5)
+        d_v0, d_nu = nat.empties(r_raw, 2) if v0 is not None else (None, None)
+        d_rk, d_mix = nat.empties(rk_mult, 1)[0], nat.empties(mix_amt, 1)[0]
+        ws_bytes = nat.pb_wkv_prepare_bwd_workspace_size(bsz, steps, n_head, chans // n_head)
+        nat.pb_wkv_prepare_bwd(r_raw, k_raw, d, iclr_raw, v_prime, v0, nu_raw, cos_tab, sin_tab, rk_mult, mix_amt, bsz, steps, n_head, chans // n_head,
+                               *gs, *douts, d_v0, d_nu, d_rk, d_mix, nat.empty((ws_bytes,), torch.uint8, r_raw), ws_bytes)
         d_r_raw, d_k_raw, d_d, d_iclr_raw, d_v_prime = douts
         return d_r_raw, d_k_raw, d_d, d_iclr_raw, d_v_prime, d_v0, d_nu, None, None, d_rk, d_mix, None
 
@@ -210,36 +179,29 @@ def wkv_prepare(r_raw, k_raw, d, iclr_raw, v_prime, v0, nu_raw, cos_tab, sin_tab
         raise ValueError(f"wkv_prepare: angle tables must be [{shape[1]}, 32]")
     ins = [_f32c(t) for t in ins]
     opt = [_f32c(t) if t is not None else None for t in (v0, nu_raw)]
-    return _WkvPrepareFn.apply(*ins, *opt, _f32c(cos_tab), _f32c(sin_tab), _f32c(rk_mult).reshape(-1), _f32c(mix_amt).reshape(-1), n_head)
+    return run(_WkvPrepareFn, *ins, *opt, _f32c(cos_tab), _f32c(sin_tab), _f32c(rk_mult).reshape(-1), _f32c(mix_amt).reshape(-1), n_head)
 
 
 class _RmsNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, scale, eps):
-        lib = _lib.load()
+        nat = _lib.native()
         chans = x.shape[-1]
         rows = x.numel() // chans
-        y = torch.empty_like(x)
-        inv = torch.empty(rows, dtype=torch.float32, device=x.device)
-        with _lib.on_device(x.device):
-            check(lib.pb_rms_norm(x.data_ptr(), scale.data_ptr(), rows, chans, eps, y.data_ptr(), inv.data_ptr(), _stream(x.device)))
+        y, inv = nat.empties(x, 1)[0], nat.empty((rows,), torch.float32, x)
+        nat.pb_rms_norm(x, scale, rows, chans, eps, y, inv)
         ctx.save_for_backward(x, scale, inv)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         x, scale, inv = ctx.saved_tensors
-        lib = _lib.load()
+        nat = _lib.native()
         chans = x.shape[-1]
         rows = x.numel() // chans
-        dy = _f32c(dy)
-        dev = x.device
-        with _lib.on_device(dev):
-            dx, dscale = torch.empty_like(x), torch.empty_like(scale)
-            ws_bytes = lib.pb_rms_norm_bwd_workspace_size(rows, chans)
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-            check(lib.pb_rms_norm_bwd(dy.data_ptr(), x.data_ptr(), scale.data_ptr(), inv.data_ptr(), rows, chans,
-                                      dx.data_ptr(), dscale.data_ptr(), ws.data_ptr(), ws_bytes, _stream(dev)))
+        dx, dscale = nat.empties(x, 1)[0], nat.empties(scale, 1)[0]
+        ws_bytes = nat.pb_rms_norm_bwd_workspace_size(rows, chans)
+        nat.pb_rms_norm_bwd(_f32c(dy), x, scale, inv, rows, chans, dx, dscale, nat.empty((ws_bytes,), torch.uint8, x), ws_bytes)
         return dx, dscale, None
 
 
@@ -250,27 +212,24 @@ def rms_norm(x, scale, eps: float):
         raise RuntimeError("rms_norm needs CUDA tensors: pratchya_b200 has no CPU path")
     if scale.numel() != x.shape[-1] or x.shape[-1] % 128 != 0:
         raise ValueError(f"rms_norm: x {tuple(x.shape)}, scale {tuple(scale.shape)} (the last dimension must be a multiple of 128)")
-    return _RmsNormFn.apply(_f32c(x), _f32c(scale).reshape(-1), float(eps))
+    return run(_RmsNormFn, _f32c(x), _f32c(scale).reshape(-1), float(eps))
 
 
 class _Relu2Fn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x):
-        lib = _lib.load()
-        y = torch.empty_like(x)
-        with _lib.on_device(x.device):
-            check(lib.pb_relu2(x.data_ptr(), x.numel(), y.data_ptr(), _stream(x.device)))
+        nat = _lib.native()
+        y = nat.empties(x, 1)[0]
+        nat.pb_relu2(x, x.numel(), y)
         ctx.save_for_backward(x)
         return y
 
     @staticmethod
     def backward(ctx, g):
         (x,) = ctx.saved_tensors
-        lib = _lib.load()
-        g = _f32c(g)
-        dx = torch.empty_like(x)
-        with _lib.on_device(x.device):
-            check(lib.pb_relu2_bwd(g.data_ptr(), x.data_ptr(), x.numel(), dx.data_ptr(), _stream(x.device)))
+        nat = _lib.native()
+        dx = nat.empties(x, 1)[0]
+        nat.pb_relu2_bwd(_f32c(g), x, x.numel(), dx)
         return dx
 
 
@@ -278,27 +237,20 @@ def relu2(x):
     """relu(x) ** 2, _module.py:249; the element count must be a multiple of 4."""
     if not x.is_cuda:
         raise RuntimeError("relu2 needs CUDA tensors: pratchya_b200 has no CPU path")
-    return _Relu2Fn.apply(_f32c(x))
+    return run(_Relu2Fn, _f32c(x))
 
 
 class _Relu2QuantFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, k):
-        lib = _lib.load()
+        nat = _lib.native()
         cols = k.shape[-1]
         rows = k.numel() // cols
         groups = rows * cols // 1024
-        dev = k.device
-        with _lib.on_device(dev):
-            q = torch.empty((rows, cols), dtype=torch.float8_e4m3fn, device=dev)
-            sc8 = torch.empty((groups, 8), dtype=torch.float8_e8m0fnu, device=dev)
-            sc32 = torch.empty((groups, 1, 1), dtype=torch.float32, device=dev)
-            q_t = torch.empty((cols, rows), dtype=torch.float8_e4m3fn, device=dev)
-            sc8_t = torch.empty((groups, 8), dtype=torch.float8_e8m0fnu, device=dev)
-            sc32_t = torch.empty((groups, 1, 1), dtype=torch.float32, device=dev)
-            check(lib.pb_relu2_quantize_dual(k.data_ptr(), rows, cols, q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(),
-                                             q_t.data_ptr(), sc8_t.data_ptr(), sc32_t.data_ptr(), _stream(dev)))
-            handle = torch.zeros(1, dtype=torch.float32, device=dev).expand(k.shape)
+        q, sc8, sc32 = nat.empty((rows, cols), _E4M3, k), nat.empty((groups, 8), _E8M0, k), nat.empty((groups, 1, 1), torch.float32, k)
+        q_t, sc8_t, sc32_t = nat.empty((cols, rows), _E4M3, k), nat.empty((groups, 8), _E8M0, k), nat.empty((groups, 1, 1), torch.float32, k)
+        nat.pb_relu2_quantize_dual(k, rows, cols, q, sc8, sc32, q_t, sc8_t, sc32_t)
+        handle = torch.zeros(1, dtype=torch.float32, device=k.device).expand(k.shape)
         ctx.save_for_backward(k)
         ctx.mark_non_differentiable(q, sc8, sc32, q_t, sc8_t, sc32_t)
         ctx.set_materialize_grads(False)
@@ -317,7 +269,7 @@ def relu2_quantized(k):
     with C and the number of rows multiples of 1024.  The bytes are those of relu2 + quantize_impl / quantize_transposed_impl."""
     if not k.is_cuda:
         raise RuntimeError("relu2_quantized needs CUDA tensors: pratchya_b200 has no CPU path")
-    out = _Relu2QuantFn.apply(_f32c(k))
+    out = run(_Relu2QuantFn, _f32c(k))
     return QuantizedMix(out[0], (out[1], out[2], out[3]), (out[4], out[5], out[6]))
 
 
@@ -328,17 +280,12 @@ def can_quantize_relu2(k):
 class _WkvFinishFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, eps, n_head):
-        lib = _lib.load()
+        nat = _lib.native()
         bsz, steps, chans = y.shape
-        dev = y.device
-        out = torch.empty_like(y)
-        stats = torch.empty((bsz * n_head, 2), dtype=torch.float32, device=dev)
-        with _lib.on_device(dev):
-            ws_bytes = lib.pb_wkv_finish_workspace_size(bsz, steps, n_head, chans // n_head)
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-            check(lib.pb_wkv_finish(y.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), gate.data_ptr(), gn_scale.data_ptr(),
-                                    gn_bias.data_ptr(), bonus_mult.data_ptr(), eps, bsz, steps, n_head, chans // n_head,
-                                    out.data_ptr(), stats.data_ptr(), ws.data_ptr(), ws_bytes, _stream(dev)))
+        out, stats = nat.empties(y, 1)[0], nat.empty((bsz * n_head, 2), torch.float32, y)
+        ws_bytes = nat.pb_wkv_finish_workspace_size(bsz, steps, n_head, chans // n_head)
+        nat.pb_wkv_finish(y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, eps, bsz, steps, n_head, chans // n_head, out, stats,
+                          nat.empty((ws_bytes,), torch.uint8, y), ws_bytes)
         ctx.save_for_backward(y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, stats)
         ctx.n_head = n_head
         return out
@@ -346,22 +293,14 @@ class _WkvFinishFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, stats = ctx.saved_tensors
-        lib = _lib.load()
+        nat = _lib.native()
         bsz, steps, chans = y.shape
         n_head = ctx.n_head
-        dev = y.device
-        g = _f32c(g)
-        with _lib.on_device(dev):
-            d_y, d_r, d_k, d_v, d_gate = (torch.empty_like(y) for _ in range(5))
-            d_gs, d_gb, d_bm = torch.empty_like(gn_scale), torch.empty_like(gn_bias), torch.empty_like(bonus_mult)
-            ws_bytes = lib.pb_wkv_finish_bwd_workspace_size(bsz, steps, n_head, chans // n_head)
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-            check(lib.pb_wkv_finish_bwd(g.data_ptr(), y.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), gate.data_ptr(),
-                                        gn_scale.data_ptr(), gn_bias.data_ptr(), bonus_mult.data_ptr(), stats.data_ptr(),
-                                        bsz, steps, n_head, chans // n_head, d_y.data_ptr(), d_r.data_ptr(), d_k.data_ptr(),
-                                        d_v.data_ptr(), d_gate.data_ptr(), d_gs.data_ptr(), d_gb.data_ptr(), d_bm.data_ptr(),
-                                        ws.data_ptr(), ws_bytes, _stream(dev)))
-        return d_y, d_r, d_k, d_v, d_gate, d_gs, d_gb, d_bm, None, None
+        grads = [*nat.empties(y, 5), nat.empties(gn_scale, 1)[0], nat.empties(gn_bias, 1)[0], nat.empties(bonus_mult, 1)[0]]      # in the order of the inputs
+        ws_bytes = nat.pb_wkv_finish_bwd_workspace_size(bsz, steps, n_head, chans // n_head)
+        nat.pb_wkv_finish_bwd(_f32c(g), y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, stats, bsz, steps, n_head, chans // n_head, *grads,
+                              nat.empty((ws_bytes,), torch.uint8, y), ws_bytes)
+        return (*grads, None, None)
 
 
 def wkv_finish(y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, eps: float, n_head: int):
@@ -374,21 +313,17 @@ def wkv_finish(y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, eps: float, n_he
         raise ValueError(f"wkv_finish: inputs must share a shape [B, T, {n_head} * 64], got {[tuple(t.shape) for t in ins]}")
     if not y.is_cuda:
         raise RuntimeError("wkv_finish needs CUDA tensors: pratchya_b200 has no CPU path")
-    return _WkvFinishFn.apply(*[_f32c(t) for t in ins], _f32c(gn_scale).reshape(-1), _f32c(gn_bias).reshape(-1),
+    return run(_WkvFinishFn, *[_f32c(t) for t in ins], _f32c(gn_scale).reshape(-1), _f32c(gn_bias).reshape(-1),
                               _f32c(bonus_mult).reshape(-1), float(eps), n_head)
 
 
 class _SmoothedXentFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, target, weight, alpha, denominator, reuse_logits=False):
-        lib = _lib.load()
+        nat = _lib.native()
         rows, vocab = logits.shape
-        dev = logits.device
-        row_loss = torch.empty(rows, dtype=torch.float32, device=dev)
-        lse = torch.empty(rows, dtype=torch.float32, device=dev)
-        with _lib.on_device(dev):
-            check(lib.pb_smoothed_xent(logits.data_ptr(), target.data_ptr(), weight.data_ptr(), rows, vocab, alpha,
-                                       row_loss.data_ptr(), lse.data_ptr(), _stream(dev)))
+        row_loss, lse = nat.empty((rows,), torch.float32, logits), nat.empty((rows,), torch.float32, logits)
+        nat.pb_smoothed_xent(logits, target, weight, rows, vocab, alpha, row_loss, lse)
         ctx.save_for_backward(logits, target, weight, lse)
         ctx.alpha, ctx.denominator, ctx.reuse_logits = alpha, denominator, bool(reuse_logits)
         return row_loss.sum() / denominator
@@ -396,15 +331,12 @@ class _SmoothedXentFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         logits, target, weight, lse = ctx.saved_tensors
-        lib = _lib.load()
+        nat = _lib.native()
         rows, vocab = logits.shape
-        dev = logits.device
         g = g.to(torch.float32).reshape(1).contiguous()
         # every element of the cotangent depends on its own logit only: with reuse_logits it is written over the logits
-        dlogits = logits if ctx.reuse_logits else torch.empty_like(logits)
-        with _lib.on_device(dev):
-            check(lib.pb_smoothed_xent_bwd(logits.data_ptr(), target.data_ptr(), weight.data_ptr(), lse.data_ptr(), g.data_ptr(),
-                                           ctx.denominator, rows, vocab, ctx.alpha, dlogits.data_ptr(), _stream(dev)))
+        dlogits = logits if ctx.reuse_logits else nat.empties(logits, 1)[0]
+        nat.pb_smoothed_xent_bwd(logits, target, weight, lse, g, ctx.denominator, rows, vocab, ctx.alpha, dlogits)
         return dlogits, None, None, None, None, None
 
 
@@ -424,4 +356,4 @@ def smoothed_cross_entropy(logits, labels, alpha: float = 0.1, reuse_logits: boo
     weight[:, -1] = 0.0
     flat = _f32c(logits).reshape(bsz * steps, vocab)
     reuse = bool(reuse_logits) and flat.data_ptr() == logits.data_ptr()          # only the caller's own array, never a converted copy's alias
-    return _SmoothedXentFn.apply(flat, target, weight.reshape(-1), float(alpha), float(bsz * (steps - 1)), reuse)
+    return run(_SmoothedXentFn, flat, target, weight.reshape(-1), float(alpha), float(bsz * (steps - 1)), reuse)

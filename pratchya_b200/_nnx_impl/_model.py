@@ -22,6 +22,7 @@ from .._qualia import _ops
 from ._glue import QuantizedMix, can_quantize_mixes, can_quantize_relu2, relu2, relu2_quantized, rms_norm, token_shift_lerp, token_shift_lerp_quantized, wkv_finish, wkv_prepare
 from ._glue import smoothed_cross_entropy as fused_cross_entropy
 from ._module import linear_fp8
+from ._nograph import no_graph
 from ._wkv7 import wkv_state_scan
 
 
@@ -67,7 +68,7 @@ class FakeQuant(torch.autograd.Function):
 
 
 def read_param(p, tgrid, dtype=torch.float32):
-    return FakeQuant.apply(p, tgrid, dtype)
+    return _ops.fake_quantize_impl(p, tgrid, dtype) if no_graph() else FakeQuant.apply(p, tgrid, dtype)
 
 
 def _lecun(fan_in, shape, gen, device):

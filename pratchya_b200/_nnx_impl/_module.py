@@ -11,6 +11,7 @@ import torch
 from .. import _lib
 from .._qualia import _ops
 from .._qualia._qarr import QArrayImpl
+from ._nograph import NoContext, no_graph
 
 
 def lecun_normal(fan_in: int, fan_out: int, *, generator=None, device="cuda", dtype=torch.float32):
@@ -146,6 +147,35 @@ class LowRankFFN:
         return self.up(torch.tanh(self.down(x)))
 
 
+def _weight_triple(weight, grid, prepared):
+    """The fp8 triple of a weight, from what the caller keeps of it (`prepared`) where it is there."""
+    wq = prepared.get("wq") if prepared is not None else None
+    if wq is None:
+        wq = _ops.quantize_impl(weight, grid)
+        if prepared is not None:
+            prepared["wq"] = wq
+    return wq
+
+
+def _weight_bytes_t(wq, prepared):
+    w_t = prepared.get("w_t") if prepared is not None else None
+    if w_t is None:
+        w_t = _ops.transpose_bytes(wq[0])
+        if prepared is not None:
+            prepared["w_t"] = w_t
+    return w_t
+
+
+def _forward_only(x, weight, grid, fake_quant_output, prepared, prepared_x):
+    """The layer's output in one call of the extension, or None where it does not apply (_LinearFn.forward then says why)."""
+    a, b = grid
+    if a != 128 or weight.dim() != 2 or not weight.is_cuda or not x.is_cuda or weight.shape[0] % 128 or (b == 128 and weight.shape[1] % 128) or weight.shape[1] % 16:
+        return None
+    wq = _weight_triple(weight, grid, prepared)
+    row = prepared_x[0] if prepared_x is not None else (None, None, None)
+    return _lib.native().linear(x, *row, wq[1], wq[2], _weight_bytes_t(wq, prepared), b, fake_quant_output)
+
+
 class _LinearFn(torch.autograd.Function):
     """Differentiable FP8 linear layer: forward and the custom-VJP chain of the reference
     (dequantize_impl_bwd -> quantize_impl_bwd -> matmul_impl_bwd -> quantize_impl_bwd,
@@ -162,12 +192,7 @@ class _LinearFn(torch.autograd.Function):
     def forward(ctx, x, weight, grid, fake_quant_output, recipe, grad_format, for_backward=True, prepared=None, prepared_x=None):
         a, b = grid
         x2 = x.reshape(-1, x.shape[-1])
-        if prepared is not None and "wq" in prepared:
-            wq = prepared["wq"]
-        else:
-            wq = _ops.quantize_impl(weight, grid)
-            if prepared is not None:
-                prepared["wq"] = wq
+        wq = _weight_triple(weight, grid, prepared)
         # the tensor-core backward needs the weight as a K-major operand in both directions: (128,128) blocks only.
         # A (128,1) weight (LoRA, gate, lm_head) has one scale per column and 128 rows, which no 128-deep block
         # along its columns can carry: its forward runs on the tensor cores, its backward on the literal recipe.
@@ -182,14 +207,10 @@ class _LinearFn(torch.autograd.Function):
         else:
             xq, xt = _ops.quantize_impl(x2, (1, a)), None
         eligible = _ops._tensor_core_eligible(xq[0], wq[0], (1, a), grid)
-        w_t = None
         if eligible:
-            w_t = prepared.get("w_t") if prepared is not None else None
-            if w_t is None:
-                w_t = _ops.transpose_bytes(wq[0])
-                if prepared is not None:
-                    prepared["w_t"] = w_t
-        y = _ops.matmul_impl(*xq, *wq, (1, a), grid, y_fp8_t=w_t, out_dtype=torch.float32)
+            y = _ops.gemm(xq, (_weight_bytes_t(wq, prepared), *wq[1:]), (b, 128), torch.float32, 1)
+        else:
+            y = _ops.matmul_impl(*xq, *wq, (1, a), grid, out_dtype=torch.float32)
         ctx.grid, ctx.recipe, ctx.grad_format, ctx.fake = grid, recipe, grad_format, fake_quant_output
         ctx.x_shape, ctx.x_dtype, ctx.w_dtype = x.shape, x.dtype, weight.dtype
         saved = [*xq, *wq]
@@ -198,7 +219,9 @@ class _LinearFn(torch.autograd.Function):
             ctx.have_xt = True
         else:
             ctx.have_xt = False
-        if fake_quant_output:
+        if fake_quant_output and not for_backward:
+            y = _ops.fake_quantize_impl(y, (1, b), x.dtype)
+        elif fake_quant_output:
             y, y_sc8, y_sc32 = _ops.fake_quantize_scales_impl(y, (1, b), x.dtype)
             saved += [y_sc8, y_sc32]
         else:
@@ -216,8 +239,6 @@ class _LinearFn(torch.autograd.Function):
         if ctx.have_xt:
             xt, pos = saved[6:9], 9
         g = g_y.reshape(-1, g_y.shape[-1]).contiguous()
-        m, k = xq[0].shape
-        n = wq[0].shape[1]
         if ctx.fake and xt is not None and b == 128:
             # the cotangent of the output's dequantize (:575-601) as the prologue of dY's two quantizers
             gq, gt = _ops.dequantize_bwd_quantize_dual_impl(saved[pos], saved[pos + 1], g, out_format=ctx.grad_format)
@@ -227,9 +248,8 @@ class _LinearFn(torch.autograd.Function):
             if xt is not None:
                 gq, gt = _ops.quantize_dual_impl(g, out_format=ctx.grad_format)
         if xt is not None:
-            op = _ops._operand
-            gx = _ops.gemm_tn(op(gq[0], gq[1], gq[2], m, n, (1, 128)), op(wq[0], wq[1], wq[2], k, n, (128, 128)), torch.float32, g.device)
-            gw = _ops.gemm_tn(op(xt[0], xt[1], xt[2], k, m, (1, 128)), op(gt[0], gt[1], gt[2], n, m, (1, 128)), torch.float32, g.device)
+            gx = _ops.gemm(gq, wq, (128, 128), torch.float32)
+            gw = _ops.gemm(xt, gt, (1, 128), torch.float32)
         else:
             gx, gw = _ops.literal_dots(xq, wq, (1, a), ctx.grid, g)
         gx = _ops.fake_quantize_impl(gx, (1, a), torch.float32)                                  # :637 then :522-526
@@ -251,5 +271,9 @@ def linear_fp8(x, weight: torch.Tensor, tgrid=(128, 128), *, fake_quant_output: 
     prepared_x = None
     if hasattr(x, "handle"):          # a QuantizedMix: the input's fp8 triples from the kernel that produced it
         x, prepared_x = x.handle, (x.row, x.tokens)
+    grid = (int(tgrid[0]), int(tgrid[1]))
+    if no_graph():
+        y = _forward_only(x, weight, grid, fake_quant_output, prepared, prepared_x)
+        return y if y is not None else _LinearFn.forward(NoContext(), x, weight, grid, fake_quant_output, recipe, grad_format, False, prepared, prepared_x)
     for_backward = torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)
-    return _LinearFn.apply(x, weight, (int(tgrid[0]), int(tgrid[1])), fake_quant_output, recipe, grad_format, for_backward, prepared, prepared_x)
+    return _LinearFn.apply(x, weight, grid, fake_quant_output, recipe, grad_format, for_backward, prepared, prepared_x)

@@ -1,0 +1,24 @@
+"""The forward pass of a torch.autograd.Function without the Function around it, where nothing can ask for a derivative of it."""
+from __future__ import annotations
+
+import torch
+from torch.autograd import forward_ad
+
+
+class NoContext:
+    """What a forward pass is given in place of its context: everything it puts there is dropped."""
+    def save_for_backward(self, *tensors): pass
+    def mark_non_differentiable(self, *tensors): pass
+    def set_materialize_grads(self, value): pass
+
+
+def no_graph() -> bool:
+    """Gradients are off, no level of forward-mode differentiation is open, no function transform (vmap, grad, jvp) is
+    running and nothing is being traced: each of these sees an op only through its autograd.Function."""
+    return (not torch.is_grad_enabled() and forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
+            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
+
+
+def run(function, *args):
+    """function.apply(*args), or its forward pass alone: the call through apply costs 8 us of host time per op."""
+    return function.forward(NoContext(), *args) if no_graph() else function.apply(*args)

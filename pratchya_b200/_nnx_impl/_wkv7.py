@@ -7,7 +7,6 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from .._lib import check
 
 
 def _check_inputs(ins, n_head):
@@ -25,22 +24,16 @@ def _check_inputs(ins, n_head):
 def _forward(state_in, ins, n_head, want_checkpoints):
     bsz, steps, chans = ins[0].shape
     head_dim = chans // n_head
-    dev = ins[0].device
-    lib = _lib.load()
-    with _lib.on_device(dev):
-        out = torch.empty((bsz, steps, chans), dtype=torch.float32, device=dev)
-        state_out = torch.empty((bsz, n_head, head_dim, head_dim), dtype=torch.float32, device=dev)
-        ckpt = sa = None
-        if want_checkpoints:
-            n_floats = lib.pb_wkv7_checkpoint_floats(bsz, steps, n_head, head_dim)
-            if n_floats == 0:
-                raise _lib.PbError(_lib.PB_ERR_UNSUPPORTED, f"wkv_state_scan: head size {head_dim} is not supported")
-            ckpt = torch.empty(n_floats, dtype=torch.float32, device=dev)
-            sa = torch.empty((bsz, steps, chans), dtype=torch.float32, device=dev)
-        check(lib.pb_wkv7_forward(*[t.data_ptr() for t in ins], state_in.data_ptr() if state_in is not None else None,
-                                  bsz, steps, n_head, head_dim, out.data_ptr(), state_out.data_ptr(),
-                                  ckpt.data_ptr() if ckpt is not None else None, sa.data_ptr() if sa is not None else None,
-                                  _lib.current_stream(dev)))
+    nat, like = _lib.native(), ins[0]
+    out = nat.empty((bsz, steps, chans), torch.float32, like)
+    state_out = nat.empty((bsz, n_head, head_dim, head_dim), torch.float32, like)
+    ckpt = sa = None
+    if want_checkpoints:
+        n_floats = nat.pb_wkv7_checkpoint_floats(bsz, steps, n_head, head_dim)
+        if n_floats == 0:
+            raise _lib.PbError(_lib.PB_ERR_UNSUPPORTED, f"wkv_state_scan: head size {head_dim} is not supported")
+        ckpt, sa = nat.empty((n_floats,), torch.float32, like), nat.empty((bsz, steps, chans), torch.float32, like)
+    nat.pb_wkv7_forward(*ins, state_in, bsz, steps, n_head, head_dim, out, state_out, ckpt, sa)
     return state_out, out, ckpt, sa
 
 
@@ -59,18 +52,12 @@ class _WkvScanFn(torch.autograd.Function):
         bsz, steps, chans = ins[0].shape
         n_head = ctx.n_head
         head_dim = chans // n_head
-        dev = ins[0].device
-        lib = _lib.load()
-        with _lib.on_device(dev):
-            d_out = d_out.to(torch.float32).contiguous() if d_out is not None else torch.zeros_like(ins[0])
-            d_state = d_state_out.to(torch.float32).contiguous() if d_state_out is not None else None
-            grads = [torch.empty_like(ins[0]) for _ in range(6)]
-            d_state_in = torch.empty((bsz, n_head, head_dim, head_dim), dtype=torch.float32, device=dev) if ctx.has_state else None
-            check(lib.pb_wkv7_backward(*[t.data_ptr() for t in ins], ckpt.data_ptr(), sa.data_ptr(), d_out.data_ptr(),
-                                       d_state.data_ptr() if d_state is not None else None,
-                                       bsz, steps, n_head, head_dim, *[g.data_ptr() for g in grads],
-                                       d_state_in.data_ptr() if d_state_in is not None else None,
-                                       _lib.current_stream(dev)))
+        nat, like = _lib.native(), ins[0]
+        d_out = d_out.to(torch.float32).contiguous() if d_out is not None else torch.zeros_like(like)
+        d_state = d_state_out.to(torch.float32).contiguous() if d_state_out is not None else None
+        grads = nat.empties(like, 6)
+        d_state_in = nat.empty((bsz, n_head, head_dim, head_dim), torch.float32, like) if ctx.has_state else None
+        nat.pb_wkv7_backward(*ins, ckpt, sa, d_out, d_state, bsz, steps, n_head, head_dim, *grads, d_state_in)
         return (d_state_in, *grads, None)
 
 
@@ -82,7 +69,7 @@ def wkv_state_scan(wkv_state, decay, iclr, removal_k, replacement_k, v, r, n_hea
     shape = _check_inputs(ins, n_head)
     bsz, steps, chans = shape
     head_dim = chans // n_head
-    ins = [t.to(torch.float32).contiguous() for t in ins]            # the reference casts to f32 before the scan (:153-184)
+    ins = [t if t.dtype is torch.float32 and t.is_contiguous() else t.to(torch.float32).contiguous() for t in ins]      # the reference casts to f32 before the scan (:153-184)
     state_in = None
     if wkv_state is not None:
         state_in = wkv_state.to(torch.float32).contiguous()

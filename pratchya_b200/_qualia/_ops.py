@@ -66,6 +66,9 @@ def quantize_impl(x: torch.Tensor, tgrid=(128, 128), out_format: str = "e4m3"):
     only the final cast.
     """
     _require_cuda(x, "quantize_impl input")
+    out = _lib.native().quantize(x, tgrid[0], tgrid[1], _FMT_CODE[out_format])
+    if out is not None:
+        return out
     lib = _lib.load()
     orig_shape = tuple(x.shape)
     shape = _as_2d(orig_shape)
@@ -93,6 +96,9 @@ def quantize_transposed_impl(x: torch.Tensor, b: int = 128, out_format: str = "e
     """The triple of quantize_impl(swapaxes(x, -1, -2), (1, b)) without materialising the
     transpose (the operands fp8_matmul_bwd builds, _qarr.py:784-789)."""
     _require_cuda(x, "quantize_transposed_impl input")
+    out = _lib.native().quantize_transposed(x, b, _FMT_CODE[out_format])
+    if out is not None:
+        return out
     lib = _lib.load()
     if x.dim() < 2:
         raise ValueError("quantize_transposed_impl needs at least 2 dims")
@@ -125,32 +131,27 @@ def quantize_dual_impl(x: torch.Tensor, out_format: str = "e4m3"):
     rows, cols = x.shape[-2], x.shape[-1]
     if not (x.dtype == torch.bfloat16 and rows % 128 == 0 and cols % 1024 == 0 and x.numel() > 0):
         return quantize_impl(x, (1, 128), out_format), quantize_transposed_impl(x, 128, out_format)
-    lib = _lib.load()
+    nat = _lib.native()
     lead = tuple(x.shape[:-2])
     batch = math.prod(lead)
     m, k = group_geometry(rows, cols, (1, 128))
     mt, kt = group_geometry(cols, rows, (1, 128))
     x = x.contiguous()
-    dev = x.device
-    with _lib.on_device(dev):
-        fmt = _FMT_DTYPE[out_format]
-        q = torch.empty(tuple(x.shape), dtype=fmt, device=dev)
-        sc8 = torch.empty((*lead, m, k), dtype=E8M0, device=dev)
-        sc32 = torch.empty((*lead, m, 1, 1), dtype=torch.float32, device=dev)
-        q_t = torch.empty((*lead, cols, rows), dtype=fmt, device=dev)
-        sc8_t = torch.empty((*lead, mt, kt), dtype=E8M0, device=dev)
-        sc32_t = torch.empty((*lead, mt, 1, 1), dtype=torch.float32, device=dev)
-        ws_bytes = lib.pb_quantize_transposed_workspace_size(batch, rows, cols, 128)
-        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-        check(lib.pb_quantize_dual(x.data_ptr(), _DENSE_CODE[x.dtype], batch, rows, cols, _FMT_CODE[out_format],
-                                   q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), q_t.data_ptr(), sc8_t.data_ptr(), sc32_t.data_ptr(),
-                                   ws.data_ptr(), ws_bytes, _stream(x)))
+    fmt = _FMT_DTYPE[out_format]
+    q, sc8, sc32 = nat.empty(tuple(x.shape), fmt, x), nat.empty((*lead, m, k), E8M0, x), nat.empty((*lead, m, 1, 1), torch.float32, x)
+    q_t, sc8_t, sc32_t = nat.empty((*lead, cols, rows), fmt, x), nat.empty((*lead, mt, kt), E8M0, x), nat.empty((*lead, mt, 1, 1), torch.float32, x)
+    ws_bytes = nat.pb_quantize_transposed_workspace_size(batch, rows, cols, 128)
+    nat.pb_quantize_dual(x, _DENSE_CODE[x.dtype], batch, rows, cols, _FMT_CODE[out_format], q, sc8, sc32, q_t, sc8_t, sc32_t,
+                         nat.empty((ws_bytes,), torch.uint8, x), ws_bytes)
     return (q, sc8, sc32), (q_t, sc8_t, sc32_t)
 
 
 def dequantize_impl(x_fp8: torch.Tensor, sc_fp8: torch.Tensor, sc_fp32: torch.Tensor, dtype, tgrid):
     """_qarr.py:541-569.  (M, K) come from sc_fp8's last two dims, as in the reference (:550)."""
     _require_cuda(x_fp8, "dequantize_impl input")
+    out = _lib.native().dequantize(x_fp8, sc_fp8, sc_fp32, dtype, tgrid[0], tgrid[1])
+    if out is not None:
+        return out
     lib = _lib.load()
     orig_shape = tuple(x_fp8.shape)
     shape = _as_2d(orig_shape)
@@ -183,6 +184,9 @@ def fake_quantize_impl(x: torch.Tensor, tgrid, dtype, out_format: str = "e4m3") 
     _qarr.py:29 and :339-342 -- in one call where the library has one (f32 input on the (1,128) grid with
     whole 8-block super-groups, or f32 in and out on a weight's grid), otherwise by the two calls.  Same bits either way."""
     _require_cuda(x, "fake_quantize_impl input")
+    out = _lib.native().fake_quantize(x, tgrid[0], tgrid[1], dtype, _FMT_CODE[out_format], False)
+    if out is not None:
+        return out
     lib = _lib.load()
     if not _fake_quantize_fused(x, tgrid, dtype):
         a, b = int(tgrid[0]), int(tgrid[1])
@@ -212,6 +216,9 @@ def fake_quantize_scales_impl(x: torch.Tensor, tgrid, dtype):
     """(fake_quantize_impl(x, tgrid, dtype), sc_fp8, sc_fp32): the value a Linear returns and the scales of its triple, which the
     cotangent rule of that value needs (_qarr.py:575-601); the fp8 bytes in between are not written where one kernel does it."""
     _require_cuda(x, "fake_quantize_scales_impl input")
+    out = _lib.native().fake_quantize(x, tgrid[0], tgrid[1], dtype, PB_E4M3, True)
+    if out is not None:
+        return out
     if not _fake_quantize_fused(x, tgrid, dtype):
         q, sc8, sc32 = quantize_impl(x, tgrid)
         return dequantize_impl(q, sc8, sc32, dtype, tgrid), sc8, sc32
@@ -237,22 +244,21 @@ def relu2_requantize_impl(y: torch.Tensor):
     _require_cuda(y, "relu2_requantize_impl input")
     if y.dtype != torch.float32 or y.dim() < 2 or y.shape[-1] % 1024 != 0 or y.numel() == 0:
         raise ValueError(f"relu2_requantize_impl: f32 input with a last dim that is a multiple of 1024, got {y.dtype} {tuple(y.shape)}")
-    lib = _lib.load()
+    nat = _lib.native()
     y = y.contiguous()
     cols = y.shape[-1]
     rows = y.numel() // cols
-    with _lib.on_device(y.device):
-        q = torch.empty((rows, cols), dtype=E4M3, device=y.device)
-        sc8 = torch.empty((rows * cols // 1024, 8), dtype=E8M0, device=y.device)
-        sc32 = torch.empty((rows * cols // 1024, 1, 1), dtype=torch.float32, device=y.device)
-        check(lib.pb_relu2_requantize(y.data_ptr(), rows, cols, _FMT_CODE["e4m3"], q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(),
-                                      None, None, 0, _stream(y)))
+    q, sc8, sc32 = nat.empty((rows, cols), E4M3, y), nat.empty((rows * cols // 1024, 8), E8M0, y), nat.empty((rows * cols // 1024, 1, 1), torch.float32, y)
+    nat.pb_relu2_requantize(y, rows, cols, PB_E4M3, q, sc8, sc32, None, None, 0)
     return q, sc8, sc32
 
 
 def dequantize_impl_bwd(sc_fp8: torch.Tensor, sc_fp32: torch.Tensor, g_out: torch.Tensor, tgrid):
     """Cotangent of the fp8 value: g * x_sc / 128 in g's dtype, _qarr.py:575-601."""
     _require_cuda(g_out, "dequantize_impl_bwd input")
+    out = _lib.native().dequantize_bwd(sc_fp8, sc_fp32, g_out, tgrid[0], tgrid[1])
+    if out is not None:
+        return out
     lib = _lib.load()
     orig_shape = tuple(g_out.shape)
     shape = _as_2d(orig_shape)
@@ -278,20 +284,12 @@ def dequantize_bwd_quantize_dual_impl(sc_fp8: torch.Tensor, sc_fp32: torch.Tenso
     rows, cols = g_out.shape[-2], g_out.shape[-1]
     if not (g_out.dim() == 2 and g_out.dtype == torch.float32 and rows % 1024 == 0 and cols % 1024 == 0 and g_out.numel() > 0):
         return quantize_dual_impl(dequantize_impl_bwd(sc_fp8, sc_fp32, g_out, (1, 128)), out_format=out_format)
-    lib = _lib.load()
+    nat = _lib.native()
     g = g_out.contiguous()
-    groups = rows * cols // 1024
-    dev = g.device
-    with _lib.on_device(dev):
-        q = torch.empty((rows, cols), dtype=_FMT_DTYPE[out_format], device=dev)
-        sc8 = torch.empty((groups, 8), dtype=E8M0, device=dev)
-        sc32 = torch.empty((groups, 1, 1), dtype=torch.float32, device=dev)
-        q_t = torch.empty((cols, rows), dtype=_FMT_DTYPE[out_format], device=dev)
-        sc8_t = torch.empty((groups, 8), dtype=E8M0, device=dev)
-        sc32_t = torch.empty((groups, 1, 1), dtype=torch.float32, device=dev)
-        check(lib.pb_dequantize_bwd_quantize_dual(g.data_ptr(), sc_fp8.contiguous().data_ptr(), sc_fp32.contiguous().data_ptr(), rows, cols,
-                                                  _FMT_CODE[out_format], q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(),
-                                                  q_t.data_ptr(), sc8_t.data_ptr(), sc32_t.data_ptr(), _stream(g)))
+    groups, fmt = rows * cols // 1024, _FMT_DTYPE[out_format]
+    q, sc8, sc32 = nat.empty((rows, cols), fmt, g), nat.empty((groups, 8), E8M0, g), nat.empty((groups, 1, 1), torch.float32, g)
+    q_t, sc8_t, sc32_t = nat.empty((cols, rows), fmt, g), nat.empty((groups, 8), E8M0, g), nat.empty((groups, 1, 1), torch.float32, g)
+    nat.pb_dequantize_bwd_quantize_dual(g, sc_fp8.contiguous(), sc_fp32.contiguous(), rows, cols, _FMT_CODE[out_format], q, sc8, sc32, q_t, sc8_t, sc32_t)
     return (q, sc8, sc32), (q_t, sc8_t, sc32_t)
 
 
@@ -331,6 +329,9 @@ def _tensor_core_eligible(x_fp8, y_fp8, grid_x, grid_y) -> bool:
 
 def transpose_bytes(q: torch.Tensor) -> torch.Tensor:
     """[rows, cols] fp8 bytes -> [cols, rows] (a weight prepared for the forward GEMM)."""
+    out = _lib.native().transpose_bytes(q)
+    if out is not None:
+        return out
     lib = _lib.load()
     rows, cols = q.shape
     q = q.contiguous()
@@ -357,6 +358,16 @@ def gemm_tn(a: Operand, b: Operand, out_dtype, device, keep_alive=()) -> torch.T
         ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=device)
         check(lib.pb_gemm_tn(a, b, d.data_ptr(), _DENSE_CODE[out_dtype], b.rows, ws.data_ptr(), ws_bytes,
                              _lib.current_stream(device)))
+    return d
+
+
+def gemm(a, b, grid_b, out_dtype, b_transposed=0):
+    """D[m, n] = sum_k dq(A)[m, k] * dq(B)[n, k] of two 2-D triples, A on (1,128) and B in blocks of grid_b[0] rows and 128."""
+    d = _lib.native().gemm(*a, 1, *b, grid_b[0], b_transposed, out_dtype)
+    if d is None:
+        (m, k), n = a[0].shape, b[0].shape[0]
+        a, b = [t.contiguous() for t in a], [t.contiguous() for t in b]
+        d = gemm_tn(_operand(*a, m, k, (1, 128)), _operand(*b, n, k, (grid_b[0], 128), b_transposed), out_dtype, a[0].device)
     return d
 
 
@@ -404,6 +415,12 @@ class LinearStep:
         """`relu2_of_fake_quantized`: x is the f32 product of a previous Linear, and this layer's input
         is relu(dq(q(x, (1,128))))**2 (the middle of ChannelMix, _module.py:246-251), computed and
         quantized in the same pass."""
+        if out is None and triple is None:
+            done = _lib.native().linear_step(x, self.rows, self.k, self.n, self.out_dtype, _FMT_CODE[self.out_format], self.b, self.ws, self._b_ready,
+                                             relu2_of_fake_quantized)
+            if done is not None:
+                self._b_ready = True
+                return done[0], done[1:]
         lib = _lib.load()
         x = _dense_input(x)
         if relu2_of_fake_quantized and x.dtype != torch.float32:
@@ -452,10 +469,13 @@ def matmul_impl(x_fp8, x_sc8, x_sc32, y_fp8, y_sc8, y_sc32, block_grid_x, block_
         nn = y_fp8.shape[1]
         if y_fp8_t is None:
             y_fp8_t = transpose_bytes(y_fp8)
+        # the weight's scales were produced on its stored [K, N] view: blocks (128, 128) or (128, 1) there
+        d = _lib.native().gemm(x_fp8, x_sc8, x_sc32, 1, y_fp8_t, y_sc8, y_sc32, block_grid_y[1], 1, out_dtype)
+        if d is not None:
+            return d
         x_fp8, x_sc8, x_sc32 = x_fp8.contiguous(), x_sc8.contiguous(), x_sc32.contiguous()
         y_sc8, y_sc32 = y_sc8.contiguous(), y_sc32.contiguous()
         a = _operand(x_fp8, x_sc8, x_sc32, mm, kk, (1, 128))
-        # the weight's scales were produced on its stored [K, N] view: blocks (128, 128) or (128, 1) there
         b = _operand(y_fp8_t, y_sc8, y_sc32, nn, kk, (block_grid_y[1], 128), transposed_blocks=1)
         d = gemm_tn(a, b, out_dtype, x_fp8.device)
         return d.reshape(*lead, x_fp8.shape[-2], nn) if lead else d
@@ -490,6 +510,9 @@ def _matmul_f32(x, y):
 def _dense_dot(tokens: int, q, sc8, sc32, grid, g: torch.Tensor):
     """g @ dq(Q)^T (`tokens` 0) or dq(Q)^T @ g (`tokens` 1) of a 2-D e4m3 triple and a contiguous f32 or bf16 g
     on pb_dense_dot."""
+    out = _lib.native().dense_dot(tokens, q, sc8, sc32, grid[0], grid[1], g)
+    if out is not None:
+        return out
     lib = _lib.load()
     rows, cols = q.shape
     free = g.shape[0] if tokens == 0 else g.shape[1]

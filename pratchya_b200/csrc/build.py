@@ -2,7 +2,7 @@
 
     python -m pratchya_b200.csrc.build [--force] [-v]
 
-libpratchya_b200.so is the product.  libpratchya_b200_diag.so is the same sources compiled with
+libpratchya_b200.so is the product, _native.so the host side of its ops for torch (native.cc, a CPython extension).  libpratchya_b200_diag.so is the same sources compiled with
 -DPB_DIAGNOSTICS plus selftest.cu: cycle counters, timing experiments, environment switches, the
 fault injection of the abort-path test and the device self-checks live there only, and only the
 tests load it.  Both are kept in-tree next to their sources; nothing is installed anywhere.
@@ -19,6 +19,7 @@ HERE = Path(__file__).resolve().parent
 INCLUDE = HERE.parent.parent / "include"
 LIB = HERE / "libpratchya_b200.so"
 DIAG_LIB = HERE / "libpratchya_b200_diag.so"
+NATIVE = HERE / "_native.so"
 SOURCES = ["api.cu", "quantize.cu", "dequantize.cu", "transpose_quantize.cu", "optimizer.cu", "gemm_sm100.cu", "dense_dot.cu", "split_dot.cu", "wkv7.cu", "rwkv_glue.cu", "rwkv_norms.cu", "loss.cu"]
 DIAG_SOURCES = SOURCES + ["selftest.cu"]
 NVCC_FLAGS = [
@@ -74,7 +75,32 @@ def build(force: bool = False, verbose: bool = False, diagnostics: bool = False)
         r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}")
+    if not diagnostics:
+        build_native(force, verbose)
     return lib
+
+
+def build_native(force: bool = False, verbose: bool = False) -> Path:
+    """Compiles native.cc against torch's headers (the library it calls, libpratchya_b200.so, is found next to it)."""
+    import sysconfig
+
+    import torch
+    src = HERE / "native.cc"
+    if not (force or _stale(NATIVE, [src, INCLUDE / "pratchya_b200.h"])):
+        return NATIVE
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include", f"-I{INCLUDE}",
+           str(src), "-o", str(NATIVE), f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
+           f"-L{HERE}", "-l:libpratchya_b200.so", "-Wl,-rpath,$ORIGIN"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed on native.cc:\n{r.stdout}")
+    return NATIVE
 
 
 def build_all(force: bool = False, verbose: bool = False):
