@@ -20,6 +20,7 @@
 // a device status word, all roles leave their loops, TMEM is released and the kernel returns.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
@@ -47,15 +48,17 @@ constexpr int UMMA_K = 32;     // depth of one tcgen05.mma for 8-bit operands
 constexpr int kMaxChunk = 8;   // k-blocks per promotion at most (1024-deep)
 constexpr uint32_t kTmemCols = 512;
 
-// Tile widths.  224 is the default: two 224-column accumulators plus the scale-factor columns fit
+// Tile widths of the single-CTA kernel, which serves few rows and weights of few columns (choose_kernel).  A k-block costs its MMA
+// thread the same whatever the width, so narrow tiles on many CTAs finish first; 32 and 64 columns also allow the contraction to
+// be cut over a cluster whose ranks' sums meet in rank 0's shared memory.  Of the wide ones 224: two 224-column accumulators plus the scale-factor columns fit
 // the 512 TMEM columns (two 256-column ones do not), so the epilogue drains one chunk while the
 // tensor core fills the next, and a 44 KB stage leaves room for five pipeline stages.
 template <int BN>
 struct Cfg {
-  static_assert(BN == 128 || BN == 224 || BN == 256, "tile width");
-  static constexpr int kStages = BN == 128 ? 5 : (BN == 224 ? 4 : 3);
+  static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 224 || BN == 256, "tile width");
+  static constexpr int kStages = BN <= 64 ? 6 : (BN == 128 ? 5 : (BN == 224 ? 4 : 3));
   static constexpr int kAccBufs = BN == 256 ? 1 : 2;
-  static constexpr int kEpiWarps = BN == 128 ? 4 : 8;
+  static constexpr int kEpiWarps = BN <= 128 ? 4 : 8;
   static constexpr int kThreads = 128 + 32 * kEpiWarps;   // warpgroup 0: producer, MMA, two idle warps; then the epilogue warpgroups
   static constexpr int kABytes = BM * BK;
   static constexpr int kBBytes = BN * BK;
@@ -74,9 +77,14 @@ struct Cfg {
   static constexpr int kOffSf = kOffB + kStages * kBBytes;
   static constexpr int kOffStore = ((kOffSf + kSfSlots * kSfSlot + 1023) / 1024) * 1024;   // epilogue staging, 4 KB per warp
   static constexpr int kOffBar = kOffStore + kEpiWarps * 4096;
-  static constexpr int kNumBars = 2 * kStages + 2 * kAccBufs;
-  static constexpr int kSmemBytes = kOffBar + kNumBars * 8 + 16 + 1024;   // +1024: manual alignment slack
-  static_assert(kSmemBytes <= 232448, "shared memory budget");
+  static constexpr int kNumBars = 2 * kStages + 2 * kAccBufs + 1;
+  // A contraction cut over the CTAs of a cluster: what the other ranks' partial products land in, behind the barriers of rank 0.
+  static constexpr int kOffParts = kOffBar + ((kNumBars * 8 + 16 + 127) / 128) * 128;
+  static constexpr int kPartBytes = BM * BN * 4;
+  static constexpr int kMaxSplit = BN == 32 ? 4 : (BN == 64 ? 2 : 1);
+  static constexpr int kMaxParts = BN == 32 ? 4 : (BN == 64 ? 1 : 0);
+  static constexpr int smem_bytes(int parts) { return kOffParts + parts * kPartBytes + 1024; }   // +1024: manual alignment slack
+  static_assert(smem_bytes(kMaxParts) <= 232448, "shared memory budget");
 };
 
 __device__ unsigned int g_gemm_status;   // 0, or PB_ERR_DEVICE_TIMEOUT once any bounded wait ran out
@@ -208,7 +216,8 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 // acc[off .. off+15] += r * fa * fb[column]; `off` is a constant after unrolling.  `uniform`: 1 = one factor for the
 // whole tile (s_uni = fa * fb), 2 = one factor per eight adjacent columns, lane l of the warp holding that of the
-// warp's column group l in fb8 (a weight on the (128,1) grid), 0 = a factor per column, read from fbp.
+// warp's column group l in fb8 (a weight on the (128,1) grid), 0 = a factor per column, read from fbp, 3 = the same with the two
+// factors multiplied first, which gives the bits of 2.
 __device__ __forceinline__ void promote16(float (&acc)[128], int off, const uint32_t (&r)[16], float fa, float s_uni, const float* fbp, int uniform,
                                           float fb8 = 0.0f) {
   if (uniform == 2) {
@@ -219,12 +228,23 @@ __device__ __forceinline__ void promote16(float (&acc)[128], int off, const uint
       const float2 v = __ffma2_rn(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), make_float2(sj, sj), make_float2(acc[off + j], acc[off + j + 1]));
       acc[off + j] = v.x; acc[off + j + 1] = v.y;
     }
-  } else if (uniform) {
+  } else if (uniform == 1) {
     const float2 s2 = make_float2(s_uni, s_uni);
 #pragma unroll
     for (int j = 0; j < 16; j += 2) {
       const float2 v = __ffma2_rn(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), s2, make_float2(acc[off + j], acc[off + j + 1]));
       acc[off + j] = v.x; acc[off + j + 1] = v.y;
+    }
+  } else if (uniform == 3) {
+    const float2 fa2 = make_float2(fa, fa);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 fb = ld_factors(fbp + off + 4 * j);
+      const float2 v0 = __ffma2_rn(make_float2(__uint_as_float(r[4 * j + 0]), __uint_as_float(r[4 * j + 1])), __fmul2_rn(fa2, make_float2(fb.x, fb.y)),
+                                   make_float2(acc[off + 4 * j + 0], acc[off + 4 * j + 1]));
+      const float2 v1 = __ffma2_rn(make_float2(__uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])), __fmul2_rn(fa2, make_float2(fb.z, fb.w)),
+                                   make_float2(acc[off + 4 * j + 2], acc[off + 4 * j + 3]));
+      acc[off + 4 * j + 0] = v0.x; acc[off + 4 * j + 1] = v0.y; acc[off + 4 * j + 2] = v1.x; acc[off + 4 * j + 3] = v1.y;
     }
   } else {
     const float2 fa2 = make_float2(fa, fa);
@@ -243,16 +263,16 @@ __device__ __forceinline__ void promote16(float (&acc)[128], int off, const uint
 // part i+1 in flight under the arithmetic of part i.  128 accumulators + 32 staging registers leave the
 // epilogue's 216-register budget with room to spare (with two 32-register buffers the kernel spilled).
 // `release` hands the TMEM buffer back as soon as the last load has landed.
-template <typename Release>
+template <int PARTS = 8, typename Release>
 __device__ __forceinline__ void drain_later_chunk(float (&acc)[128], uint32_t t_addr, bool four_parts, float fa, float s_uni,
                                                   const float* fbp, int uniform, Release&& release, float fb8 = 0.0f) {
   uint32_t r[2][16];
   tc_ld16(t_addr, r[0]);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int j = 0; j < PARTS; ++j) {
     if (j < 6 || four_parts) {
       tc_wait_ld();
-      const bool more = j + 1 < 6 || (four_parts && j + 1 < 8);
+      const bool more = j + 1 < PARTS && (j + 1 < 6 || four_parts);
       if (more) tc_ld16(t_addr + 16 * (j + 1), r[(j + 1) & 1]);
       else release();
       promote16(acc, 16 * j, r[j & 1], fa, s_uni, fbp, uniform, fb8);
@@ -310,10 +330,13 @@ struct GemmParams {
   int tiles_m, tiles_n;
   int a_fmt, b_fmt;
   int d_dtype;
-  int diag;         // diagnostics build only (PB_DIAGNOSTICS), pair kernel: 1 skips the loads of B, 2 those of A, 4 those of the scale
+  int diag;         // diagnostics build only (PB_DIAGNOSTICS); 8 in both kernels, the others in the pair kernel: 1 skips the loads of B, 2 those of A, 4 those of the scale
                     // factors (timing experiments); 8 leaves the first pipeline slot unfilled and unarmed, so that every bounded
                     // wait of the launch runs out (the test of the abort path).  Always 0 in the product build.
-  int splitk;       // pair kernel: 1, or 2 = each tile's chunks are shared by two work units that add into a zeroed f32 D
+  int splitk;       // pair kernel: 1, or 2 = each tile's chunks are shared by two work units that add into a zeroed f32 D; single-CTA
+                    // kernel: CTAs of a cluster that share a tile's chunks
+  int split_chunks; // single-CTA kernel: chunks of a rank
+  int add_sums;     // single-CTA kernel, two ranks: the second rank's sum is added to the first's; else the other ranks' chunks are promoted in order
   int band;         // pair kernel: tile rows per band; a band's tiles are visited column by column before the next band
   int fb_uniform;   // B's fp32 factor is the same for all rows of B within a chunk (selects the kernel instantiation)
   int fb_groups8;   // ... or the same within aligned runs of eight rows of B (a weight on the (128,1) grid)
@@ -425,7 +448,41 @@ __device__ __forceinline__ void store_row_segment(const GemmParams& p, const flo
   }
 }
 
-template <int BN, bool PROF, bool UNI>
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// shared::cluster address of the same shared-memory offset in CTA `rank` of this cluster
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// A bounded wait for what another CTA of the cluster announced (as mbar_wait, with the ordering of the whole cluster)
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t polls) {
+  for (uint32_t n = 0; n < polls; ++n) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 2000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (ok) return true;
+  }
+  *abort_flag = 1;
+  atomicExch(&g_gemm_status, (unsigned int)PB_ERR_DEVICE_TIMEOUT);
+  return false;
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// UNI: how B's fp32 factor varies over a tile's columns within a chunk, as promote16's `uniform`: 1, 0 or 3.
+template <int BN, bool PROF, int UNI>
 __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_d, const __grid_constant__ GemmParams p) {
@@ -438,6 +495,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   auto bar_empty = [&](int s) { return s_bar + 8u * (C::kStages + s); };
   auto bar_acc_full = [&](int b) { return s_bar + 8u * (2 * C::kStages + b); };
   auto bar_acc_empty = [&](int b) { return s_bar + 8u * (2 * C::kStages + C::kAccBufs + b); };
+  const uint32_t bar_parts = s_bar + 8u * (2 * C::kStages + 2 * C::kAccBufs);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kOffBar + C::kNumBars * 8);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -446,6 +504,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), 1); }
     for (int b = 0; b < C::kAccBufs; ++b) { mbar_init(bar_acc_full(b), 1); mbar_init(bar_acc_empty(b), C::kEpiWarps); }
+    if (C::kMaxSplit > 1 && p.splitk > 1) mbar_init(bar_parts, (p.splitk - 1) * C::kEpiWarps);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -455,10 +514,16 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
+  if (C::kMaxSplit > 1 && p.splitk > 1) cluster_sync_all();      // rank 0's barrier is there before any other rank signals it
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
   const int num_tiles = p.tiles_m * p.tiles_n;
+  // The ranks of a cluster share a tile, p.split_chunks chunks of its contraction each.
+  const int split = C::kMaxSplit > 1 ? p.splitk : 1, part = split > 1 ? (int)cluster_ctarank() : 0;
+  const int first_tile = blockIdx.x / split, tile_step = gridDim.x / split;
+  const int c_begin = part * (split > 1 ? p.split_chunks : 0), c_end = split > 1 ? min(p.nchunks, c_begin + p.split_chunks) : p.nchunks;
+  const int kb_begin = c_begin * p.P, kb_stop = min(p.KB, c_end * p.P);
   const long long t_cta0 = PROF ? clock64() : 0;
   // With eight epilogue warps 384 threads start with 168 registers each; the epilogue needs ~220
   // (128 accumulators + two 32-register load buffers), warpgroup 0 almost none.
@@ -470,15 +535,17 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       uint32_t sf_fills = 0;
       long long waited = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
         const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN;
-        for (int kb = 0; kb < p.KB; ++kb, ++it) {
+        for (int kb = kb_begin; kb < kb_stop; ++kb, ++it) {
           const int s = it % C::kStages;
           const long long t0 = PROF ? clock64() : 0;
           if (!mbar_wait(bar_empty(s), ((it / C::kStages) & 1u) ^ 1u, abort_flag, p.wait_polls)) { ok = false; break; }
           if (PROF) waited += clock64() - t0;
+          // diagnostics build: the first stage of the last rank is neither armed nor filled; its own waits run out, and rank 0's for its sums
+          if (PROF && (p.diag & 8) && it == 0 && part == split - 1) continue;
           // the scale-factor atom of a stage covers 4 k-blocks: only the first of them carries it
-          const bool with_sf = (kb & 3) == 0;
+          const bool with_sf = (kb & 3) == 0 || kb == kb_begin;      // a rank that starts inside a group of four fetches its atom too
           mbar_arrive_expect_tx(bar_full(s), C::kABytes + C::kBBytes + (with_sf ? C::kSfSlot : 0));
           tma_load_2d(s_a + s * C::kABytes, &map_a, kb * BK, m0, bar_full(s));
           tma_load_2d(s_b + s * C::kBBytes, &map_b, kb * BK, n0, bar_full(s));
@@ -489,7 +556,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int kg = kb >> 2;
             const uint32_t slot = s_sf + (sf_fills % C::kSfSlots) * C::kSfSlot;
             ++sf_fills;
-            bulk_load(slot, p.sfa + ((size_t)kg * p.tiles_m + tile % p.tiles_m) * 512, C::kSfaBytes, bar_full(s));
+            bulk_load(slot, p.sfa + ((size_t)kg * (p.Mpad / BM) + tile % p.tiles_m) * 512, C::kSfaBytes, bar_full(s));
             bulk_load(slot + C::kSfaBytes, p.sfb + ((size_t)kg * p.tiles_n + tile / p.tiles_m) * C::kSfbBytes, C::kSfbBytes, bar_full(s));
           }
         }
@@ -498,7 +565,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // kStages fills are the ones that can still be in flight.
       const uint32_t issued = it;
       for (uint32_t j = (issued > (uint32_t)C::kStages ? issued - C::kStages : 0); j < issued; ++j)
-        (void)mbar_wait(bar_full(j % C::kStages), (j / C::kStages) & 1u, abort_flag, p.wait_polls);
+        if (!(PROF && (p.diag & 8) && j == 0 && part == split - 1)) (void)mbar_wait(bar_full(j % C::kStages), (j / C::kStages) & 1u, abort_flag, p.wait_polls);
       if (PROF) atomicAdd(&g_gemm_prof[0], (unsigned long long)waited);
     } else if (warp == 1 && lane == 0) {
       // ------------------------------------------------------------- MMA issuer
@@ -506,7 +573,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // every dependent instruction costs its full latency, and a tcgen05.mma takes ~75 cycles to
       // issue: the four of a k-block leave ~200 of the tensor core's 512 cycles for everything
       // else.  Hence: no divisions, 32-bit descriptor arithmetic, incremental stage state.
-      const int KB = p.KB, P = p.P, nchunks = p.nchunks;
+      const int P = p.P;
       const uint32_t idesc0 = instr_desc(BN, p.a_fmt, p.b_fmt, 0u);
       const uint32_t a_lo0 = operand_desc_lo(s_a), b_lo0 = operand_desc_lo(s_b);
       const uint32_t sf_tmem0 = tmem_base + C::kSfColBase;
@@ -518,15 +585,15 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       long long wait_full = 0, wait_acc = 0;
       const long long t_begin = PROF ? clock64() : 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        for (int c = 0; c < nchunks && ok; ++c, ++g) {
+      for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
+        for (int c = c_begin; c < c_end && ok; ++c, ++g) {
           const int buf = g % C::kAccBufs;
           long long t0 = PROF ? clock64() : 0;
           if (!mbar_wait(bar_acc_empty(buf), ((g / C::kAccBufs) & 1u) ^ 1u, abort_flag, p.wait_polls)) { ok = false; break; }
           if (PROF) wait_acc += clock64() - t0;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + buf * BN;
-          const int kb_end = min(KB, (c + 1) * P);
+          const int kb_end = min(kb_stop, (c + 1) * P);
           uint32_t accumulate = 0;
           for (int kb = c * P; kb < kb_end; ++kb) {
             if (PROF) t0 = clock64();
@@ -534,7 +601,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             if (PROF) wait_full += clock64() - t0;
             // the scale factors of k-blocks 4j..4j+3 go to the TMEM set of their fill; the MMAs that read that set's
             // last contents were kSfSlots fills ago: k-blocks whose commits this stage's producer has waited for
-            if ((kb & 3) == 0) {
+            if ((kb & 3) == 0 || kb == kb_begin) {
               const uint32_t turn = sf_reads % C::kSfSlots;
               const uint32_t sf_lo = sf_lo0 + turn * (C::kSfSlot >> 4);
               sf_col = sf_tmem0 + turn * C::kSfCols;
@@ -571,17 +638,18 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int ew = warp - 4;
     const int quarter = warp & 3;             // TMEM lanes this warp may touch
     const int col_half = ew >> 2;             // which column slice of the tile: [0,128) or [128,BN)
-    const int ncols = col_half == 0 ? (BN < 128 ? BN : 128) : BN - 128;      // 128, or 96 for the 224-wide tile
-    const bool four_parts = ncols == 128;     // 32-column parts this warp drains per chunk (else three)
+    constexpr int kCols = BN < 128 ? BN : 128;        // columns of a warp at most
+    const int ncols = col_half == 0 ? kCols : BN - 128;      // 96 for the second half of the 224-wide tile
+    const bool four_parts = ncols == 128;     // 32-column parts this warp drains per chunk, of a tile of 128 columns or more (else three)
     const int row_in_tile = quarter * 32 + lane;
     uint32_t g = 0, stores = 0;
     bool ok = true;
     long long wait_chunk = 0;
     const long long t_begin = PROF ? clock64() : 0;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+    for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
       const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN + col_half * 128;
       float acc[128];
-      for (int c = 0; c < p.nchunks; ++c, ++g) {
+      for (int c = c_begin; c < c_end; ++c, ++g) {
         const int buf = g % C::kAccBufs;
         // the chunk's fp32 factors do not depend on the MMAs: fetch them before waiting
         const float fa = __ldg(p.fa + (size_t)c * p.Mpad + m0 + row_in_tile);
@@ -598,40 +666,98 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           __syncwarp();
           if (lane == 0) mbar_arrive(bar_acc_empty(buf));
         };
+        if constexpr (C::kMaxSplit > 1) {
+          if (part > 0 && !p.add_sums) {        // the chunk as the tensor core left it, for rank 0 to promote
+            const uint32_t dst = map_to_cta(s_base + C::kOffParts + (uint32_t)((c - p.split_chunks) * C::kPartBytes + row_in_tile * 16), 0);
+            uint32_t r[16];
+#pragma unroll
+            for (int j = 0; j < kCols / 16; ++j) {
+              tc_ld16(t_addr + 16 * j, r);
+              tc_wait_ld();
+              if (j + 1 == kCols / 16) release();
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                st_cluster_v4(dst + (4 * j + e) * BM * 16, __uint_as_float(r[4 * e]), __uint_as_float(r[4 * e + 1]), __uint_as_float(r[4 * e + 2]), __uint_as_float(r[4 * e + 3]));
+            }
+            continue;
+          }
+        }
         if (PB_EPI_SKIP_DRAIN) { release(); continue; }      // diagnostics build: handshake only
-        if (c == 0) {
+        if (c == c_begin) {
           // First chunk of a tile: straight into the accumulator registers, so the buffer goes
           // back to the MMA warp before any arithmetic.
-          tc_ld32f<0>(t_addr, acc); tc_ld32f<32>(t_addr + 32, acc); tc_ld32f<64>(t_addr + 64, acc);
-          if (four_parts) tc_ld32f<96>(t_addr + 96, acc);
+          tc_ld32f<0>(t_addr, acc);
+          if constexpr (kCols >= 64) tc_ld32f<32>(t_addr + 32, acc);
+          if constexpr (kCols >= 128) {
+            tc_ld32f<64>(t_addr + 64, acc);
+            if (four_parts) tc_ld32f<96>(t_addr + 96, acc);
+          }
           tc_wait_ld();
           release();
-          if (UNI) {
+          if (UNI == 1) {
 #pragma unroll
-            for (int j = 0; j < 128; ++j) acc[j] *= s_uni;
+            for (int j = 0; j < kCols; ++j) acc[j] *= s_uni;
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
+            for (int j = 0; j < kCols / 4; ++j) {
               if (j < 24 || four_parts) {
                 const float4 fb = ld_factors(fbp + 4 * j);
-                acc[4 * j + 0] = acc[4 * j + 0] * fa * fb.x; acc[4 * j + 1] = acc[4 * j + 1] * fa * fb.y;
-                acc[4 * j + 2] = acc[4 * j + 2] * fa * fb.z; acc[4 * j + 3] = acc[4 * j + 3] * fa * fb.w;
+                if (UNI == 3) {
+                  acc[4 * j + 0] *= fa * fb.x; acc[4 * j + 1] *= fa * fb.y; acc[4 * j + 2] *= fa * fb.z; acc[4 * j + 3] *= fa * fb.w;
+                } else {
+                  acc[4 * j + 0] = acc[4 * j + 0] * fa * fb.x; acc[4 * j + 1] = acc[4 * j + 1] * fa * fb.y;
+                  acc[4 * j + 2] = acc[4 * j + 2] * fa * fb.z; acc[4 * j + 3] = acc[4 * j + 3] * fa * fb.w;
+                }
               }
             }
           }
         } else {
-          drain_later_chunk(acc, t_addr, four_parts, fa, s_uni, fbp, UNI, release);
+          drain_later_chunk<kCols / 16>(acc, t_addr, four_parts, fa, s_uni, fbp, UNI, release);
         }
       }
       if (!ok) break;
+      if constexpr (C::kMaxSplit > 1) {
+        if (split > 1) {
+          // The other ranks' chunks, or their sums of them (p.add_sums), are in rank 0's shared memory, sixteen bytes of a row beside the
+          // same of the next; rank 0 goes on with them in their order.
+          const uint32_t mine = s_base + C::kOffParts + (uint32_t)row_in_tile * 16;
+          if (part > 0) {
+            if (p.add_sums) {
+              const uint32_t dst = map_to_cta(mine, 0);
+#pragma unroll
+              for (int j = 0; j < kCols / 4; ++j) st_cluster_v4(dst + j * BM * 16, acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(bar_parts, 0));
+            continue;
+          }
+          if (!mbar_wait_cluster(bar_parts, 0, abort_flag, p.wait_polls)) { ok = false; break; }
+          for (int c = c_end; c < (p.add_sums ? c_end + 1 : p.nchunks); ++c) {
+            const uint32_t src = mine + (uint32_t)(c - c_end) * C::kPartBytes;
+            const float fa = p.add_sums ? 1.0f : __ldg(p.fa + (size_t)c * p.Mpad + m0 + row_in_tile);
+            const float* fbp = p.fb + (size_t)(p.add_sums ? 0 : c) * p.Npad + n0;
+            const float s_uni = p.add_sums ? 1.0f : fa * __ldg(fbp);
+#pragma unroll
+            for (int j = 0; j < kCols / 16; ++j) {
+              uint32_t r[16];
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[4 * e]), "=r"(r[4 * e + 1]), "=r"(r[4 * e + 2]), "=r"(r[4 * e + 3]) : "r"(src + (4 * j + e) * BM * 16));
+              promote16(acc, 16 * j, r, fa, s_uni, fbp, p.add_sums ? 1 : UNI);
+            }
+          }
+        }
+      }
       if (PB_EPI_SKIP_STORE) continue;       // diagnostics build: no stores of D
       if (p.tma_store) {
         const uint32_t stage = s_base + C::kOffStore + ew * 4096;
         const int row0 = m0 + quarter * 32;
         stage_and_store<0>(&map_d, acc, stage, lane, p.d_dtype, n0, row0, stores);
-        stage_and_store<32>(&map_d, acc, stage, lane, p.d_dtype, n0, row0, stores);
-        stage_and_store<64>(&map_d, acc, stage, lane, p.d_dtype, n0, row0, stores);
-        if (four_parts) stage_and_store<96>(&map_d, acc, stage, lane, p.d_dtype, n0, row0, stores);
+        if constexpr (kCols >= 64) stage_and_store<32>(&map_d, acc, stage, lane, p.d_dtype, n0, row0, stores);
+        if constexpr (kCols >= 128) {
+          stage_and_store<64>(&map_d, acc, stage, lane, p.d_dtype, n0, row0, stores);
+          if (four_parts) stage_and_store<96>(&map_d, acc, stage, lane, p.d_dtype, n0, row0, stores);
+        }
       } else {
         store_row_segment(p, acc, m0 + row_in_tile, n0, ncols);
       }
@@ -645,6 +771,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   tc_fence_before();
   __syncthreads();
+  if (C::kMaxSplit > 1 && p.splitk > 1) cluster_sync_all();      // rank 0 stays until every rank's stores to its memory are done
   if (PROF && threadIdx.x == 0) {
     atomicAdd(&g_gemm_prof[5], (unsigned long long)(clock64() - t_cta0));
     atomicAdd(&g_gemm_prof[7], 1ull);
@@ -687,23 +814,6 @@ struct Cfg2 {
   static_assert(kSfSlots >= kSlots && kSfColBase + kSfSlots * kSfCols <= 512, "scale-factor slots and TMEM budget");
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// shared::cluster address of the same shared-memory offset in CTA `rank` of this cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
 // TMA tile load whose completion is signalled on a barrier of either CTA of the pair
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t cluster_bar) {
   asm volatile(
@@ -1241,7 +1351,7 @@ struct GemmPlan {
   OperandPlan pa, pb;
   int P, KB, KG, nchunks, Mpad, Npad, BN;
   int tiles_m, tiles_n, atoms_b;      // A tiles of 128 rows, B tiles of BN rows, scale-factor atoms per B tile
-  bool pair;      // CTA-pair kernel (256 x 256 tiles) instead of the single-CTA one
+  bool pair;      // CTA-pair kernel (256 x 224 tiles) instead of the single-CTA one
   size_t off_sfa, off_sfb, off_fa, off_fb, total;
 };
 
@@ -1250,8 +1360,8 @@ bool pick_pair() {      // the CTA-pair kernel is the default; PB_GEMM_SINGLE=1 
   return pair;
 }
 
-int pick_bn() {      // PB_GEMM_BN=128|224|256: tile width of the single-CTA kernel
-  static const int bn = [] { const int v = env_switch("PB_GEMM_BN", 224); return (v == 128 || v == 256) ? v : 224; }();
+int forced_bn() {    // PB_GEMM_BN=32|64|128|224|256: tile width of the single-CTA kernel; 0: by size
+  static const int bn = env_switch("PB_GEMM_BN", 0);
   return bn;
 }
 
@@ -1275,19 +1385,95 @@ constexpr int diag_bits() { return 0; }
 constexpr uint32_t wait_polls() { return kDefaultWaitPolls; }
 #endif
 
+// Whether an f32 product of m rows on pairs of CTAs is run as two halves of its chunks per tile (where that fills the chip better),
+// each tile then the sum of two sums.  The order of a product's f32 additions is this rule's in every form.
+bool in_halves(int64_t m, int64_t n, int nchunks) {
+  if (m <= 128 || nchunks < 4) return false;
+  const int64_t tiles = (m + 255) / 256 * ((n + Cfg2::BN - 1) / Cfg2::BN), pairs = sm_count() / 2;
+  auto efficiency = [&](int64_t units) { return (double)units / (double)(((units + pairs - 1) / pairs) * pairs); };
+  return efficiency(tiles) < 0.8 && efficiency(2 * tiles) > efficiency(tiles) + 0.1;
+}
+
+int ranks_that_fit(int64_t tiles) {      // clusters of two pack every SM, of four most of them
+  const int sms = sm_count();
+  return 4 * tiles <= sms * 7 / 8 ? 4 : (2 * tiles <= sms ? 2 : 1);
+}
+
+// CTAs of a cluster that share a tile's chunks in the single-CTA kernel, and the chunks of each: two halves whose sums are added
+// where the product is run in halves, else up to `most` ranks, whose chunks rank 0 promotes in their order as if they were its own.
+void cut_contraction(int bn, int most, bool halves, int nchunks, int* split, int* chunks) {
+  *split = 1; *chunks = nchunks;
+  const int max_split = bn == 32 ? Cfg<32>::kMaxSplit : (bn == 64 ? Cfg<64>::kMaxSplit : 1), max_parts = bn == 32 ? Cfg<32>::kMaxParts : Cfg<64>::kMaxParts;
+  if (halves && max_split > 1) {
+    *split = 2; *chunks = (nchunks + 1) / 2;
+    return;
+  }
+  for (int s = 2; s <= std::min(max_split, most); s *= 2) {
+    const int per = (nchunks + s - 1) / s, ranks = (nchunks + per - 1) / per;
+    if (ranks < 2 || nchunks - per > max_parts) continue;
+    *split = ranks; *chunks = per;
+  }
+}
+
+// Which kernel, by how long each would take in us: what a launch costs whatever its depth, and per wave of tiles the k-blocks of one,
+// with a drain of the accumulator every P of them.  A k-block takes 570 cycles in every form where the chip is not full (the MMA
+// thread's waits, commits and issues, not the tensor core), so few rows want many narrow tiles, and where those are still few the
+// contraction cut over a cluster; full waves want the widest.  Fitted to a sweep of 1 to 16384 rows over twenty weights.  us in a graph with the
+// scales made ready (2), f32 out, the form before (a pair above 128 rows, 224 columns below) | this choice, the bits the same:
+// 2048 x 2048: 64 rows 12.6 | 10.0, 500 14.3 | 12.0, 1000 14.7 | 12.8; 1024 x 1024: 8 rows 9.1 | 8.0, 500 11.5 | 8.3, 2048 12.0 | 10.1;
+// 4096 x 512: 64 rows 17.1 | 10.4, 1000 16.1 | 13.6; 8192 x 2048: 64 rows 27.9 | 19.3; 2048 x 8192 the pair from 129 rows; (128,1) weights:
+// 2048 x 128: 64 rows 30.6 | 14.2, 1000 26.0 | 14.8, 4096 19.1 | 14.0; 128 x 2048: 512 rows 9.4 | 6.5; 2048 x 8192: 64 rows 31.3 | 16.5, the
+// pair from 129 rows (27.0 against 43.0 at 512).
+void choose_kernel(GemmPlan* gp, int64_t m, int64_t n) {
+  if (forced_bn() || !pick_pair()) {
+    gp->pair = pick_pair() && m > 128;
+    gp->BN = gp->pair ? Cfg2::BN : (forced_bn() ? forced_bn() : 224);
+    return;
+  }
+  struct Form { int bn; double launch, block, drain, wave; int max_waves; };
+  static constexpr Form forms[] = {{128, 4.8, 0.30, 0.76, 0.8, 2}, {64, 3.7, 0.30, 0.24, 0.4, 2}, {32, 3.1, 0.30, 0.21, 0.3, 1}};
+  const int sms = sm_count();
+  const double drains = gp->P < kMaxChunk ? 1.0 / gp->P : 0.0;
+  const bool halves = in_halves(m, n, gp->nchunks);
+  auto waves = [](int64_t tiles, int64_t at_once) { return (double)((tiles + at_once - 1) / at_once); };
+  double best;
+  if (m > 128) {
+    const double w = waves((m + 255) / 256 * ((n + Cfg2::BN - 1) / Cfg2::BN) * (halves ? 2 : 1), sms / 2);
+    // nothing is changed for what the fit may be off by
+    best = 0.88 * (7.1 + (halves ? 2.0 : 0.0) + w * gp->KB * (halves ? 0.5 : 1.0) * (0.31 + 0.74 * drains) + (w - 1) * 1.6) - 0.2;
+    gp->pair = true; gp->BN = Cfg2::BN;
+  } else {
+    const double w = waves((n + 223) / 224, sms);
+    best = 5.8 + w * gp->KB * (0.33 + 1.03 * drains) + (w - 1) * 1.6 - 0.2;
+    gp->pair = false; gp->BN = 224;
+  }
+  for (const Form& f : forms) {
+    const int64_t tiles = (m + 127) / 128 * ((n + f.bn - 1) / f.bn);
+    int split, chunks;
+    cut_contraction(f.bn, ranks_that_fit(tiles), halves, gp->nchunks, &split, &chunks);
+    if (halves && (split != 2 || 2 * tiles > sms)) continue;
+    const double w = waves(tiles, sms);
+    if (w > f.max_waves) continue;
+    double t = f.launch + w * std::min<double>(gp->KB, (double)chunks * gp->P) * (f.block + f.drain * drains) + (w - 1) * f.wave + (split > 1 ? 2.0 : 0.0);
+    // the few rows of A are the same few lines of L2 for every CTA: 8 rows, 2048 x 8192: 64 CTAs 9.5, 128 10.2, 256 16.6
+    if (m < 48 && tiles * split > sms / 2) t += m < 16 ? 0.1 * gp->KB : 0.7;
+    if (m > 128 && w > 1) t += 1.0;
+    if (t < best) { best = t; gp->pair = false; gp->BN = f.bn; }
+  }
+}
+
 int make_plan(const pb_operand* a, const pb_operand* b, GemmPlan* gp) {
   if (!a || !b) return fail(PB_ERR_NULL_POINTER, "pb_gemm_tn: operands must be non-null");
   if (int s = plan_operand(a, "A", &gp->pa)) return s;
   if (int s = plan_operand(b, "B", &gp->pb)) return s;
   if (a->depth != b->depth)
     return fail(PB_ERR_BAD_SHAPE, "pb_gemm_tn: contraction lengths differ (%lld vs %lld)", (long long)a->depth, (long long)b->depth);
-  gp->pair = pick_pair() && a->rows > 128;
-  gp->BN = gp->pair ? Cfg2::BN : pick_bn();
   gp->P = gp->pa.P < gp->pb.P ? gp->pa.P : gp->pb.P;
   gp->KB = (int)(a->depth / BK);
   if (gp->P > gp->KB) gp->P = gp->KB;
   gp->KG = (gp->KB + 3) / 4;
   gp->nchunks = (gp->KB + gp->P - 1) / gp->P;
+  choose_kernel(gp, a->rows, b->rows);
   gp->Mpad = (int)((a->rows + 255) / 256 * 256);
   gp->tiles_m = gp->Mpad / 128;
   gp->tiles_n = (int)((b->rows + gp->BN - 1) / gp->BN);
@@ -1321,7 +1507,7 @@ int launch_prep(const PrepParams* a, const PrepParams* b, cudaStream_t st) {
   return PB_OK;
 }
 
-template <int BN, bool PROF, bool UNI>
+template <int BN, bool PROF, int UNI>
 int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, const GemmParams& p, cudaStream_t st) {
   static std::mutex mu;
   static bool configured[64] = {false};
@@ -1330,19 +1516,30 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
   {
     std::lock_guard<std::mutex> lock(mu);
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-      PB_CUDA_TRY(cudaFuncSetAttribute(gemm_tn_kernel<BN, PROF, UNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmemBytes));
+      PB_CUDA_TRY(cudaFuncSetAttribute(gemm_tn_kernel<BN, PROF, UNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::smem_bytes(Cfg<BN>::kMaxParts)));
       configured[dev] = true;
     }
   }
   const int tiles = p.tiles_m * p.tiles_n;
-  const int grid = tiles < sm_count() ? tiles : sm_count();
-  gemm_tn_kernel<BN, PROF, UNI><<<grid, Cfg<BN>::kThreads, Cfg<BN>::kSmemBytes, st>>>(ma, mb, md, p);
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((unsigned)(p.splitk > 1 ? tiles * p.splitk : (tiles < sm_count() ? tiles : sm_count())));
+  config.blockDim = dim3(Cfg<BN>::kThreads);
+  config.dynamicSmemBytes = Cfg<BN>::smem_bytes(p.splitk == 1 ? 0 : (p.add_sums ? 1 : p.nchunks - p.split_chunks));
+  config.stream = st;
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = (unsigned)p.splitk; cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  config.attrs = &cluster;
+  config.numAttrs = p.splitk > 1 ? 1 : 0;
+  PB_CUDA_TRY(cudaLaunchKernelEx(&config, gemm_tn_kernel<BN, PROF, UNI>, ma, mb, md, p));
   PB_LAUNCH_CHECK("gemm_tn_kernel");
   return PB_OK;
 }
 template <int BN, bool PROF>
 int launch_gemm_uni(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, const GemmParams& p, cudaStream_t st) {
-  return p.fb_uniform ? launch_gemm<BN, PROF, true>(ma, mb, md, p, st) : launch_gemm<BN, PROF, false>(ma, mb, md, p, st);
+  if (p.fb_uniform) return launch_gemm<BN, PROF, 1>(ma, mb, md, p, st);
+  // a (128,1) weight: rows that fill a pair are multiplied as the pair kernel does, whose bits do not depend on the form then
+  return p.fb_groups8 && p.M > 128 ? launch_gemm<BN, PROF, 3>(ma, mb, md, p, st) : launch_gemm<BN, PROF, 0>(ma, mb, md, p, st);
 }
 
 template <bool PROF, int UNI>
@@ -1445,7 +1642,7 @@ extern "C" int pb_gemm_tn_ex(const pb_operand* a, const pb_operand* b, void* d, 
   p.d = d; p.ldd = ldd;
   p.M = (int)a->rows; p.N = (int)b->rows; p.KB = gp.KB; p.P = gp.P; p.nchunks = gp.nchunks;
   p.Mpad = gp.Mpad; p.Npad = gp.Npad;
-  p.tiles_m = gp.pair ? gp.Mpad / 256 : gp.tiles_m; p.tiles_n = gp.tiles_n;
+  p.tiles_m = gp.pair ? gp.Mpad / 256 : (int)((a->rows + BM - 1) / BM); p.tiles_n = gp.tiles_n;
   p.a_fmt = a->format; p.b_fmt = b->format; p.d_dtype = d_dtype;
   p.fb_uniform = gp.pb.row_uniform ? 1 : 0;
   p.fb_groups8 = gp.pb.row_groups8 ? 1 : 0;
@@ -1460,6 +1657,8 @@ extern "C" int pb_gemm_tn_ex(const pb_operand* a, const pb_operand* b, void* d, 
   }
   p.tma_store = 0;
   p.splitk = 1;
+  p.split_chunks = gp.nchunks;
+  p.add_sums = 0;
   p.profile = profile_level();
   p.diag = diag_bits();
   p.wait_polls = wait_polls();
@@ -1470,14 +1669,17 @@ extern "C" int pb_gemm_tn_ex(const pb_operand* a, const pb_operand* b, void* d, 
   if (p.tma_store) {
     if (int s = make_store_map(&md, d, d_dtype, a->rows, b->rows, ldd)) return s;
   }
+  const bool halves = d_dtype == PB_F32 && p.tma_store && in_halves(a->rows, b->rows, gp.nchunks);
+  if (!gp.pair) {
+    cut_contraction(gp.BN, ranks_that_fit((int64_t)p.tiles_m * p.tiles_n), halves, gp.nchunks, &p.splitk, &p.split_chunks);
+    p.add_sums = halves && p.splitk > 1 ? 1 : 0;
+  }
   if (gp.pair) {
     // Few tiles for the 74 CTA pairs (a 2048 x 2048 weight gradient is 80): give each tile's chunks to
     // two work units that add their halves into D.  Needs f32 output through TMA (the reduction is
     // an f32 TMA add into zeros, so the two orders give the same bits) and at least two chunks a half.
     static const int split_env = env_switch("PB_GEMM_SPLITK", 0);
-    const int pairs = sm_count() / 2, tiles = p.tiles_m * p.tiles_n;
-    auto efficiency = [&](int units) { return (double)units / (double)(((units + pairs - 1) / pairs) * pairs); };
-    bool split = d_dtype == PB_F32 && p.tma_store && gp.nchunks >= 4 && efficiency(tiles) < 0.8 && efficiency(2 * tiles) > efficiency(tiles) + 0.1;
+    bool split = halves;
     if (split_env == 1) split = false;
     if (split_env == 2) split = d_dtype == PB_F32 && p.tma_store && gp.nchunks >= 2;
     if (split) {
@@ -1493,13 +1695,17 @@ extern "C" int pb_gemm_tn_ex(const pb_operand* a, const pb_operand* b, void* d, 
     return launch_gemm_pair_uni<false>(ma, mb, msfa, msfb, md, p, st);
   }
 #ifdef PB_DIAGNOSTICS
-  if (p.profile) {
+  if (p.profile || p.diag) {
+    if (gp.BN == 32) return launch_gemm_uni<32, true>(ma, mb, md, p, st);
+    if (gp.BN == 64) return launch_gemm_uni<64, true>(ma, mb, md, p, st);
     if (gp.BN == 224) return launch_gemm_uni<224, true>(ma, mb, md, p, st);
     return gp.BN == 256 ? launch_gemm_uni<256, true>(ma, mb, md, p, st) : launch_gemm_uni<128, true>(ma, mb, md, p, st);
   }
   if (gp.BN == 256) return launch_gemm_uni<256, false>(ma, mb, md, p, st);
-  if (gp.BN == 128) return launch_gemm_uni<128, false>(ma, mb, md, p, st);
 #endif
+  if (gp.BN == 32) return launch_gemm_uni<32, false>(ma, mb, md, p, st);
+  if (gp.BN == 64) return launch_gemm_uni<64, false>(ma, mb, md, p, st);
+  if (gp.BN == 128) return launch_gemm_uni<128, false>(ma, mb, md, p, st);
   return launch_gemm_uni<224, false>(ma, mb, md, p, st);
 }
 

@@ -486,17 +486,16 @@ int launch_prepare(const PrepareParams& p, cudaStream_t st) {
   return PB_OK;
 }
 
-// Where this form is the faster one.  What it makes ready has to be shared, the terms by `shared` columns of the other operand,
+// Where this form is the faster one.  What it makes ready has to be shared,
 // and its two launches and the passes over the operands want something to do.  us, dense_dot_kernel | this form, inside a graph:
 // dX, 2048 x 2048: f32 100 rows 14.9 | 15.8, 200 20.1 | 18.9, 3000 142 | 84; bf16 300 rows 23.8 | 23.0, 500 30.6 | 27.4, 3000 141 | 75;
-// 1024 x 1024, bf16: 500 rows 14.4 | 14.6, 700 16.9 | 16.2; 2048 x 128, bf16: 1000 rows 9.3 | 10.3, 2000 17.2 | 14.1.
+// 1024 x 1024, bf16: 500 rows 14.4 | 14.6, 700 16.9 | 16.2; 2048 x 128, bf16: 1000 rows 9.3 | 10.3.
 // dW, 1024 x 1024: 64 rows 8.3 | 8.7, 200 13.5 | 10.8, 3000 52 | 33; 2048 x 2048: 64 rows 15.0 | 13.5, 3000 178 | 68; f32 174 | 79;
-// 4096 x 512: 100 rows 10.1 | 10.6, 200 14.2 | 12.1.  Terms that one tile uses: 8192 rows, 2048 x 128, bf16 36.6 | 42.8;
-// 128 x 2048, f32 35.6 | 48.4.
-bool split_dot_pays(int tokens, int64_t I, int64_t J, int64_t C, bool g_bf16) {
-  const int64_t shared = g_bf16 ? J : I;
+// 4096 x 512: 100 rows 10.1 | 10.6, 200 14.2 | 12.1.  Operands that one tile uses: 8192 rows, 2048 x 128, f32 35.5 | 32.5, bf16
+// 36.6 | 42.8; 128 x 2048, f32 35.6 | 48.4.
+bool split_dot_pays(int tokens, int64_t I, int64_t J, int64_t C) {
   const double products = (double)I * (double)J * (double)C;
-  if (shared < 512) return false;
+  if (I < 512 || J < 512) return false;
   if (tokens) return C >= 192 || products >= 0x1p28;
   return products >= 0x1p29 && J >= 192;
 }
@@ -546,7 +545,7 @@ bool split_dot_plan(int tokens, int64_t rows, int64_t cols, int a, int b, int64_
   d->off_other = align((size_t)row_bytes * d->slab);
   d->off_parts = d->off_other + (g_bf16 ? 0 : align((size_t)rows * cols * 2));
   d->bytes = d->off_parts + (d->splits > 1 ? (size_t)d->splits * I * J * 4 : 0);
-  return split_dot_pays(tokens, I, J, C, g_bf16);
+  return split_dot_pays(tokens, I, J, C);
 }
 
 int split_dot_run(const SplitDotPlan& d, int tokens, const uint8_t* q, const uint8_t* sc8, const float* sc32, int64_t rows, int64_t cols, int a, int b,

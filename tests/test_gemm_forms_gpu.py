@@ -1,0 +1,85 @@
+"""The forms of the GEMM that its size chooses between (tiles of 128 x 32, 64, 128 and 224 on one CTA, 256 x 224 on a pair, the
+contraction cut over a cluster of two and four): remainders in every direction against a 64-bit product, and their abort paths."""
+import pytest
+import torch
+
+from pratchya_b200 import _lib
+from pratchya_b200._qualia import _ops, dequantize_impl, quantize_impl
+
+pytestmark = pytest.mark.gpu
+
+PB_ERR_DEVICE_TIMEOUT = 7
+
+
+def _triples(m, k, n, grid):
+    g = torch.Generator(device="cuda").manual_seed(m + k + n)
+    x = torch.randn(m, k, generator=g, device="cuda") * torch.randn(m, 1, generator=g, device="cuda").exp()
+    w = torch.randn(k, n, generator=g, device="cuda") * 0.02
+    return quantize_impl(x, (1, 128)), quantize_impl(w, grid)
+
+
+@pytest.mark.parametrize("m,k,n,grid", [
+    (1, 1024, 1024, (128, 128)), (8, 2048, 2048, (128, 128)), (127, 2304, 128, (128, 128)), (128, 4096, 512, (128, 128)), (33, 5120, 256, (128, 128)), (100, 3072, 1024, (128, 128)),
+    (5, 2048, 8192, (128, 128)), (129, 2048, 2048, (128, 128)), (255, 8192, 2048, (128, 128)), (257, 1024, 896, (128, 128)), (520, 2048, 2048, (128, 128)), (1000, 1024, 1152, (128, 128)),
+    (2000, 1024, 1024, (128, 128)), (1031, 2048, 8192, (128, 128)), (8, 256, 640, (128, 128)), (16, 384, 384, (128, 128)), (640, 1280, 256, (128, 128)),
+    (1, 2048, 128, (128, 1)), (64, 2048, 48, (128, 1)), (300, 1024, 144, (128, 1)), (1000, 2048, 128, (128, 1)), (72, 640, 16, (128, 1)), (8, 128, 2064, (128, 1)), (8192, 2048, 128, (128, 1)),
+    (129, 1152, 4096, (128, 1)), (2056, 128, 1040, (128, 1)), (40, 2048, 8208, (128, 1))])
+def test_products_against_64_bits(built_lib, m, k, n, grid):
+    xq, wq = _triples(m, k, n, grid)
+    if xq[1].shape[-1] != 8:
+        xq, _ = _triples(m + 8 - m % 8, k, n, grid)         # whole super-groups
+    xd, wd = dequantize_impl(*xq, torch.float32, (1, 128)).double(), dequantize_impl(*wq, torch.float32, grid).double()
+    want = xd @ wd
+    # per element, |x| @ |w| times what the tensor core's additions of 128 products (2^-23 each k-block at most, of which eight meet in an
+    # accumulator) and the f32 additions of the blocks and parts behind them may be off by
+    bound = (xd.abs() @ wd.abs()) * 2.0 ** -23 * (k / 128 + 12)
+    got = _ops.matmul_impl(*xq, *wq, (1, 128), grid)
+    assert got.shape == want.shape and ((got.double() - want).abs() <= bound + 1e-30).all()
+    half = _ops.matmul_impl(*xq, *wq, (1, 128), grid, out_dtype=torch.bfloat16)
+    assert ((half.double() - want).abs() <= bound + want.abs() * 2.0 ** -8 + 1e-30).all()
+    assert torch.equal(got, _ops.matmul_impl(*xq, *wq, (1, 128), grid))
+    assert built_lib.pb_gemm_check(torch.cuda.current_stream().cuda_stream) == 0
+
+
+def test_outputs_with_longer_rows_and_off_the_store_alignment(built_lib):
+    """ldd beyond n, and rows that are no multiple of 16 bytes: nothing but [m, n] is written."""
+    for m, k, n, ldd in [(40, 4096, 512, 640), (40, 2048, 512, 513), (130, 1024, 256, 300), (7, 1024, 128, 129)]:
+        xq, wq = _triples(m, k, n, (128, 128))
+        wt = _ops.transpose_bytes(wq[0])
+        a, b = _ops._operand(*xq, m, k, (1, 128)), _ops._operand(wt, wq[1], wq[2], n, k, (128, 128), 1)
+        size = built_lib.pb_gemm_workspace_size(a, b)
+        ws = torch.full((size,), 0xff, dtype=torch.uint8, device="cuda")
+        want = dequantize_impl(*xq, torch.float32, (1, 128)).double() @ dequantize_impl(*wq, torch.float32, (128, 128)).double()
+        for dtype, code in ((torch.float32, _lib.PB_F32), (torch.bfloat16, _lib.PB_BF16)):
+            d = torch.full((m + 1, ldd), 7.0, dtype=dtype, device="cuda")
+            _lib.check(built_lib.pb_gemm_tn(a, b, d.data_ptr(), code, ldd, ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream))
+            assert (d[:m, n:] == 7).all() and (d[m:] == 7).all()
+            assert ((d[:m, :n].double() - want).norm() / want.norm()).item() <= (1e-6 if code == _lib.PB_F32 else 4e-3)
+
+
+@pytest.mark.parametrize("m,k,n", [(40, 4096, 512), (40, 2048, 2048), (40, 1024, 256), (200, 8192, 2048), (100, 1024, 8192), (2048, 2048, 2048)])
+def test_a_wait_that_runs_out_is_reported_and_the_next_launch_is_clean(built_lib, diag_lib, m, k, n):
+    """The diagnostics build leaves a launch's first stage (of a cluster's last rank) unfilled, with a poll budget of about two milliseconds."""
+    xq, wq = _triples(m, k, n, (128, 128))
+    wt = _ops.transpose_bytes(wq[0])
+    a, b = _ops._operand(*xq, m, k, (1, 128)), _ops._operand(wt, wq[1], wq[2], n, k, (128, 128), 1)
+    size, st = diag_lib.pb_gemm_workspace_size(a, b), torch.cuda.current_stream().cuda_stream
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+
+    def run():
+        d = torch.zeros(m, n, device="cuda")
+        assert diag_lib.pb_gemm_tn(a, b, d.data_ptr(), _lib.PB_F32, n, ws.data_ptr(), size, st) == 0
+        return d
+
+    before = run()
+    assert diag_lib.pb_gemm_check(st) == 0 and before.abs().max().item() > 0
+    try:
+        assert diag_lib.pb_debug_gemm_control(1 << 10, 8) == 0
+        run()
+        assert diag_lib.pb_gemm_check(st) == PB_ERR_DEVICE_TIMEOUT
+        assert diag_lib.pb_gemm_check(st) == 0               # reading the status clears it
+    finally:
+        diag_lib.pb_debug_gemm_control(0, 0)
+    after = run()
+    assert diag_lib.pb_gemm_check(st) == 0 and torch.equal(before, after)
+    assert built_lib.pb_gemm_check(st) == 0
