@@ -57,12 +57,16 @@ __device__ __forceinline__ int ckpt_quad(int P, int Q) { return (2 * (P & 3) + (
 // warp, the output's one nothing).  No barrier inside a chunk of eight timesteps: the chunk's vectors arrive by cp.async two
 // chunks ahead, a step's are in registers one step ahead, and S * w is formed while sa's shuffles are under way.  v kt^T comes
 // last: added to a state that is about to be erased, its low bits would go with it.
-// What bounds it: with few heads the latency of a timestep (dot product, three shuffles, update: 310 cycles); with many the
+// What bounds it: with few heads the latency of a timestep (dot product, three shuffles, update: 250 cycles); with many the
 // f32x2 products, three cycles each where their operands are three different registers, and the 4 * (40 + ROWS) bytes per lane
 // and timestep that the vector reads return, which more rows per lane spread over more of them.
-// 1024 timesteps, against one row per thread and both dot products inside it: 32 heads 377 -> 172 us, 64 heads 379 -> 188,
-// 128 heads 379 -> 246, 256 heads 437 -> 387 (with sa and checkpoints 490 -> 474).  y reduced in its own timestep, behind sa's
-// shuffles, cost a fifth with 32 heads; v kt^T formed into the state before sa was known saved a twentieth with 64 heads and more.
+// The order within a timestep keeps everything but that chain off it: sa of the next timestep is formed from the new state before
+// y of this one, the vectors of the next are read behind sa's shuffles (in front of them the shuffles queue behind the reads), y's
+// shuffles come a timestep late and behind the state's update, a lane stores a row's outputs once in 8 / ROWS timesteps, and the
+// next chunk's first vectors are read before this one's last update, so that no chunk starts with an empty pipeline.
+// 1024 timesteps, against y's dot product and the reads in front of sa's and a pipeline emptied every chunk: 16 heads 172 -> 125 us,
+// 32 heads 173 -> 139 (with sa and checkpoints 197 -> 160), 60 heads 188 -> 165, 128 heads 247 -> 214, 256 heads 387 -> 347
+// (474 -> 422).
 constexpr int kFwdChunk = 8;      // timesteps between barriers
 constexpr int kFwdBufs = 3;       // chunks in shared memory
 
@@ -90,6 +94,8 @@ struct StepVecs {
     if constexpr (ROWS == 4) {
       const float4 t = *reinterpret_cast<const float4*>(buf[4] + row0);
       v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else if constexpr (ROWS == 1) {
+      v[0] = buf[4][row0];
     } else {
       const float2 t = *reinterpret_cast<const float2*>(buf[4] + row0);
       v[0] = t.x; v[1] = t.y;
@@ -98,38 +104,33 @@ struct StepVecs {
 };
 
 // The sums over the eight lanes of a tile row that a timestep ends with: sa for every lane (the state's update waits for it),
-// and the output of the timestep BEFORE, each lane ending with row own_row(tj): that one's shuffles run beside sa's instead of
-// behind them.
+// y for the lanes that keep it, each lane ending with row own of its ROWS
 template <int ROWS>
-__device__ __forceinline__ float reduce_rows(float (&sa)[ROWS], const float (&y)[ROWS], int tj) {
-  const bool hi = tj & 4;
-  float y_row;
-  if constexpr (ROWS == 4) {
-    const bool mid = tj & 2;
-    const float s0 = hi ? y[0] : y[2], s1 = hi ? y[1] : y[3];
-    float k0 = hi ? y[2] : y[0], k1 = hi ? y[3] : y[1];
+__device__ __forceinline__ void reduce_sa(float (&sa)[ROWS]) {
 #pragma unroll
-    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 1);
+  for (int m = 1; m <= 4; m *= 2)
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], m);
+}
+template <int ROWS>
+__device__ __forceinline__ float reduce_y(const float (&y)[ROWS], int tj) {
+  const bool hi = tj & 4, mid = tj & 2;
+  float k0;
+  if constexpr (ROWS == 1) {
+    k0 = y[0] + __shfl_xor_sync(0xffffffffu, y[0], 4);
+    k0 += __shfl_xor_sync(0xffffffffu, k0, 2);
+  } else if constexpr (ROWS == 2) {
+    k0 = (hi ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, hi ? y[0] : y[1], 4);
+    k0 += __shfl_xor_sync(0xffffffffu, k0, 2);
+  } else {
+    const float s0 = hi ? y[0] : y[2], s1 = hi ? y[1] : y[3];
+    k0 = hi ? y[2] : y[0];
+    float k1 = hi ? y[3] : y[1];
     k0 += __shfl_xor_sync(0xffffffffu, s0, 4);
     k1 += __shfl_xor_sync(0xffffffffu, s1, 4);
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 2);
-    y_row = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, 2);
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 4);
-    y_row += __shfl_xor_sync(0xffffffffu, y_row, 1);
-  } else {
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 1);
-    y_row = (hi ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, hi ? y[0] : y[1], 4);
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 2);
-    y_row += __shfl_xor_sync(0xffffffffu, y_row, 2);
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], 4);
-    y_row += __shfl_xor_sync(0xffffffffu, y_row, 1);
+    k0 = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, 2);
   }
-  return y_row;
+  return k0 + __shfl_xor_sync(0xffffffffu, k0, 1);
 }
 template <int ROWS>
 __device__ __forceinline__ float pick_row(const float (&v)[ROWS], int a) {
@@ -154,11 +155,10 @@ __device__ __forceinline__ void row_dots(const float2 (&S)[ROWS][4], const float
   for (int a = 0; a < ROWS; ++a) out[a] = (p[a].x + p[a].y) + (q[a].x + q[a].y);
 }
 
-// One timestep on a lane's tile.  In: y of the timestep before, unsummed.  Out: this one's, and the finished row of that one.
+
+// S_t from S_{t-1} and sa
 template <int ROWS>
-__device__ __forceinline__ float wkv_step(float2 (&S)[ROWS][4], StepVecs<ROWS>& x, int tj, float (&y)[ROWS], float (&sa)[ROWS]) {
-  row_dots<ROWS>(S, x.kap, sa);
-  const float y_before = reduce_rows<ROWS>(sa, y, tj);
+__device__ __forceinline__ void update_state(float2 (&S)[ROWS][4], StepVecs<ROWS>& x, const float (&sa)[ROWS]) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) x.b[k] = __fmul2_rn(x.b[k], x.kap[k]);
 #pragma unroll
@@ -175,8 +175,6 @@ __device__ __forceinline__ float wkv_step(float2 (&S)[ROWS][4], StepVecs<ROWS>& 
   for (int a = 0; a < ROWS; ++a)
 #pragma unroll
     for (int k = 0; k < 4; ++k) S[a][k] = __ffma2_rn(dup(x.v[a]), x.kt[k], S[a][k]);
-  row_dots<ROWS>(S, x.r, y);
-  return y_before;
 }
 
 // SAVE: checkpoints and sa are wanted (a backward pass follows).
@@ -185,6 +183,7 @@ __global__ void __launch_bounds__(32 * WARPS)
 wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
   constexpr int kFwdThreads = 32 * WARPS;
   constexpr int kCtaRows = 4 * ROWS * WARPS, kCtasPerHead = kH / kCtaRows;
+  static_assert(kFwdThreads <= 16 * kFwdChunk && kH % kCtaRows == 0, "sixteen threads a timestep of a chunk; a head's rows in whole CTAs");
   __shared__ __align__(16) float ring[kFwdBufs][kFwdChunk][kVecs][kH];
   const int head = blockIdx.x / kCtasPerHead;
   const int n = head % p.N, b = head / p.N;
@@ -223,49 +222,91 @@ wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
       for (int k = 0; k < 4; ++k) S[a][k] = make_float2(0.0f, 0.0f);
     }
   }
-  // of the lanes that end up with a row's y one stores it, and its neighbour sa, both a timestep late
+  // four rows a lane: of the two lanes that end up with a row's y one stores it, and its neighbour sa, both a timestep late
   constexpr int kSame = 8 / ROWS;              // lanes with the same row
   const int own = tj / kSame, part = tj % kSame;
   float* const out = part == 0 ? p.y : (SAVE && part == 1 ? p.sa : nullptr);
   float* dst = out ? out + head_base + row0 + own : nullptr;
-  float y[ROWS], sa[ROWS], sa_before = 0.0f;
+  float y[ROWS], sa[ROWS], sa_before = 0.0f, y_keep = 0.0f, sa_keep = 0.0f;
+  constexpr bool kKeep = ROWS < 4;     // eight timesteps' stores of a lane become ROWS (two arrays: no fewer with four rows)
+  // with kKeep: a row's kSame lanes keep one timestep each of kSame and store together
+  float* const yp = p.y + head_base + row0 + own;
+  float* const sp = SAVE && p.sa ? p.sa + head_base + row0 + own : nullptr;
 #pragma unroll
   for (int a = 0; a < ROWS; ++a) y[a] = 0.0f;
 
   issue(0);
   issue(1);
+  issue(2);
+  cp_async_wait<2>();
+  __syncthreads();
+  StepVecs<ROWS> cur;
+  cur.load(ring[0][0], col0, row0);
+  row_dots<ROWS>(S, cur.kap, sa);
   for (int c = 0; c < n_chunks; ++c) {
-    cp_async_wait<1>();               // this thread's copies for this chunk have landed
-    __syncthreads();                  // ... and everyone's; every warp is also done with the chunk before this one
-    issue(c + 2);                     // into the buffer that chunk used
     const float (*buf)[kVecs][kH] = ring[c % kFwdBufs];
-    if (SAVE && p.ckpt) {             // the state before the chunk (kCk == kFwdChunk), in the backward kernel's layout
-      float4* ck = p.ckpt + ((size_t)head * n_chunks + c) * kTileQuads;
+    const float (*buf_next)[kVecs][kH] = ring[(c + 1) % kFwdBufs];
+    if constexpr (SAVE && ROWS > 1) {
+      if (p.ckpt) {                   // the state before the chunk (kCk == kFwdChunk), in the backward kernel's layout
+        float4* ck = p.ckpt + ((size_t)head * n_chunks + c) * kTileQuads;
 #pragma unroll
-      for (int a = 0; a < ROWS; a += 2)
+        for (int a = 0; a < ROWS; a += 2)
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          ck[ckpt_quad((row0 + a) >> 1, (col0 >> 1) + (k & 1) + 16 * (k >> 1))] = make_float4(S[a][k].x, S[a + 1][k].x, S[a][k].y, S[a + 1][k].y);
+          for (int k = 0; k < 4; ++k)
+            ck[ckpt_quad((row0 + a) >> 1, (col0 >> 1) + (k & 1) + 16 * (k >> 1))] = make_float4(S[a][k].x, S[a + 1][k].x, S[a][k].y, S[a + 1][k].y);
+      }
     }
     const int steps = min(kFwdChunk, p.T - c * kFwdChunk);
-    StepVecs<ROWS> cur;
-    cur.load(buf[0], col0, row0);
 #pragma unroll
     for (int s = 0; s < kFwdChunk; ++s) {
       if (s >= steps) break;
       StepVecs<ROWS> next;
-      if (s + 1 < kFwdChunk) next.load(buf[s + 1], col0, row0);
-      const float y_before = wkv_step<ROWS>(S, cur, tj, y, sa);
-      if (dst && (s > 0 || c > 0)) {
+      const bool last_step = s + 1 == kFwdChunk;
+      if (last_step) {
+        cp_async_wait<1>();
+        __syncthreads();
+      }
+      const float (*from)[kH] = last_step ? buf_next[0] : buf[(s + 1) % kFwdChunk];
+      if (last_step) issue(c + 3);
+      reduce_sa<ROWS>(sa);
+      next.load(from, col0, row0);
+      float y_old[ROWS];
+#pragma unroll
+      for (int a = 0; a < ROWS; ++a) y_old[a] = y[a];
+      update_state<ROWS>(S, cur, sa);
+      float sa_next[ROWS];
+      row_dots<ROWS>(S, next.kap, sa_next);
+      row_dots<ROWS>(S, cur.r, y);
+      const float y_before = reduce_y<ROWS>(y_old, tj);
+      if constexpr (kKeep) {
+        constexpr int kLast = kSame - 1;
+        const int u = (s + kFwdChunk - 1) % kSame;           // of timestep c * 8 + s - 1
+        if (part == u) { y_keep = y_before; if (SAVE) sa_keep = sa_before; }
+        if (u == kLast && (s > 0 || c > 0)) {
+          const long at = (long)(c * kFwdChunk + s - kSame + part) * C;
+          yp[at] = y_keep;
+          if (SAVE) if (sp) sp[at] = sa_keep;
+        }
+      } else if (dst && (s > 0 || c > 0)) {
         *dst = SAVE && part != 0 ? sa_before : y_before;
         dst += C;
       }
       if (SAVE) sa_before = pick_row<ROWS>(sa, own);
-      if (s + 1 < kFwdChunk) cur = next;
+      cur = next;
+#pragma unroll
+      for (int a = 0; a < ROWS; ++a) sa[a] = sa_next[a];
     }
   }
-  const float y_last = reduce_rows<ROWS>(sa, y, tj);
-  if (dst) *dst = SAVE && part != 0 ? sa_before : y_last;
+  const float y_last = reduce_y<ROWS>(y, tj);
+  if constexpr (kKeep) {
+    const int last = (p.T - 1) % kSame;
+    if (part == last) { y_keep = y_last; if (SAVE) sa_keep = sa_before; }
+    if (part <= last) {
+      const long at = (long)(p.T - 1 - last + part) * C;
+      yp[at] = y_keep;
+      if (SAVE) if (sp) sp[at] = sa_keep;
+    }
+  } else if (dst) *dst = SAVE && part != 0 ? sa_before : y_last;
   cp_async_wait<0>();
   if (p.state_out) {
 #pragma unroll
@@ -279,8 +320,14 @@ wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
 template <int ROWS, int WARPS>
 int launch_forward(const WkvParams& p, int64_t heads, cudaStream_t st) {
   const unsigned grid = (unsigned)(heads * (kH / (4 * ROWS * WARPS)));
-  if (p.ckpt || p.sa) wkv7_forward_kernel<ROWS, WARPS, true><<<grid, 32 * WARPS, 0, st>>>(p);
-  else                wkv7_forward_kernel<ROWS, WARPS, false><<<grid, 32 * WARPS, 0, st>>>(p);
+  if constexpr (ROWS > 1) {       // a lane of one row has no row pair to put into a checkpoint
+    if (p.ckpt || p.sa) {
+      wkv7_forward_kernel<ROWS, WARPS, true><<<grid, 32 * WARPS, 0, st>>>(p);
+      PB_LAUNCH_CHECK("wkv7_forward_kernel");
+      return PB_OK;
+    }
+  }
+  wkv7_forward_kernel<ROWS, WARPS, false><<<grid, 32 * WARPS, 0, st>>>(p);
   PB_LAUNCH_CHECK("wkv7_forward_kernel");
   return PB_OK;
 }
@@ -660,10 +707,14 @@ extern "C" int pb_wkv7_forward(const float* decay, const float* iclr, const floa
     if (reinterpret_cast<uintptr_t>(ptr) & 15) return fail(PB_ERR_MISALIGNED, "pb_wkv7_forward: every array must be 16-byte aligned");
   WkvParams p{{decay, iclr, removal_k, replacement_k, v, r}, state_in, y, state_out, reinterpret_cast<float4*>(checkpoints), sa, (int)steps, (int)heads};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // 16, 32 or 64 rows of a head per CTA: as many CTAs as there are SMs, and no more of them on one (each reads the head's vectors)
+  // 8 (one row a lane: no pair of rows for a checkpoint), 16, 32 or 64 rows of a head per CTA: as many CTAs as there are SMs, and no
+  // more of them on one (each reads the head's vectors); 16 heads x 1024: 125 us with 8 rows, 139 with 16
   const int64_t n = batch * heads;
+  if (8 * n <= sm_count() && !checkpoints && !sa) return launch_forward<1, 2>(p, n, st);
   if (4 * n <= sm_count()) return launch_forward<2, 2>(p, n, st);
   if (2 * n <= sm_count()) return launch_forward<2, 4>(p, n, st);
+  // just over a wave of whole heads: quarters of them fill SMs more evenly (160 heads x 1024: 326 us for 350, with saves 358 for 425)
+  if (n > sm_count() && 4 * n <= 5 * sm_count()) return launch_forward<2, 2>(p, n, st);
   return launch_forward<4, 4>(p, n, st);
 }
 
