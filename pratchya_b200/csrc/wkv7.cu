@@ -66,7 +66,7 @@ __device__ __forceinline__ int ckpt_quad(int P, int Q) { return (2 * (P & 3) + (
 // next chunk's first vectors are read before this one's last update, so that no chunk starts with an empty pipeline.
 // 1024 timesteps, against y's dot product and the reads in front of sa's and a pipeline emptied every chunk: 16 heads 172 -> 125 us,
 // 32 heads 173 -> 139 (with sa and checkpoints 197 -> 160), 60 heads 188 -> 165, 128 heads 247 -> 214, 256 heads 387 -> 347
-// (474 -> 422).
+// (474 -> 422) in graphs of repeated calls; 32 heads x 4096, called with L2 flushed in between, 685 -> 571.
 constexpr int kFwdChunk = 8;      // timesteps between barriers
 constexpr int kFwdBufs = 3;       // chunks in shared memory
 
