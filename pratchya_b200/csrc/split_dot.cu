@@ -12,7 +12,7 @@
 // Every f32 product is then exact in three tensor-core products, and the accumulator is emptied into f32 registers every 32 of c,
 // as in dense_dot.cu (the tensor core's own additions do not round to nearest).  The terms carry an exact 2^40, which keeps
 // them above bf16's subnormals.  A sum that is not finite, for an infinity or a NaN in the operands, an overflow of a scaled
-// term or a power of two that bf16 does not hold, is made again with f32 products of dequantized values.
+// term or a power of two that bf16 does not hold, is made again with f32 products of dequantized values, behind the last tile.
 //
 // Element-wise kernel: bound by its bytes.  Main kernel: persistent, one CTA per SM; a tile is 128 rows of the three-term operand
 // by N of the other; a stage is 32 of c of both, by TMA, K-major (64-byte swizzle) for tokens == 0 and with c outermost, as
@@ -54,7 +54,7 @@ struct DotSource {
   const void* g;
   int64_t ldq, ldg;
   uint32_t nbc, log2_K, log2_a, log2_b;      // blocks per block row, of log2 sizes
-  int C, tokens, g_bf16;
+  int C;
 };
 
 struct SplitParams {
@@ -215,20 +215,48 @@ __global__ void __launch_bounds__(256) split_prepare_kernel(const __grid_constan
 }
 
 // ---- the products -------------------------------------------------------------------------------------------------
-// one sum with f32 products of dequantized values, one after the other
-__device__ __noinline__ float plain_dot(const DotSource& s, int i, int j, int c_begin, int c_end) {
-  float acc = 0.0f;
-#pragma unroll 1
-  for (int c = c_begin; c < c_end; ++c) {
-    const uint32_t row = s.tokens ? c : i, col = s.tokens ? i : c;
-    const uint32_t id = (row >> s.log2_a) * s.nbc + (col >> s.log2_b);
+// The sums of this warp's part of a tile (rows p.row_first + 32 quad .., columns cb .. cb + kCols) that are not finite, made again with f32
+// products of dequantized values, one after the other in c: sixteen columns a pass over c.  A lane holds its row's value of a c
+// and one column's, which goes round by shuffles.  All of 2048 x 2048 sums: 4.2 ms over 3000 of c,
+// 32 to 40 over 16384 (dense_dot_kernel 7.4 to 8.4 and 58 to 61).
+template <int N, bool TOKENS, bool G32>
+__device__ __noinline__ void remake_sums(const SplitParams& p, float* out, int row0, int cb, int c_begin, int c_end) {
+  constexpr bool kLanes = TOKENS == G32;
+  const DotSource& s = p.src;
+  const int lane = threadIdx.x & 31, row = row0 + lane, at_row = min(row, p.rows - 1);
+  auto q_value = [&](int i, int c) {
+    const uint32_t r = TOKENS ? c : i, col = TOKENS ? i : c;
+    const uint32_t id = (r >> s.log2_a) * s.nbc + (col >> s.log2_b);
     const float x_sc = __fmul_rn(e8m0_to_f32(__ldg(s.sc8 + id)), __ldg(s.sc32 + (id >> s.log2_K)));
-    const float x = __fmul_rn(__fmul_rn(fp8x2_to_f32x2<PB_E4M3>((uint16_t)__ldg(s.q + (int64_t)row * s.ldq + col)).x, x_sc), 0.0078125f);
-    const int64_t at = s.tokens ? (int64_t)c * s.ldg + j : (int64_t)j * s.ldg + c;
-    const float g = s.g_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(s.g)[at]) : static_cast<const float*>(s.g)[at];
-    acc = fmaf(g, x, acc);
+    return __fmul_rn(__fmul_rn(fp8x2_to_f32x2<PB_E4M3>((uint16_t)__ldg(s.q + (int64_t)r * s.ldq + col)).x, x_sc), 0.0078125f);
+  };
+  auto g_value = [&](int j, int c) {
+    const int64_t at = TOKENS ? (int64_t)c * s.ldg + j : (int64_t)j * s.ldg + c;
+    return G32 ? __ldg(static_cast<const float*>(s.g) + at) : __bfloat162float(static_cast<const __nv_bfloat16*>(s.g)[at]);
+  };
+#pragma unroll 1
+  for (int c0 = cb; c0 < cb + N / 2 && c0 < p.cols; c0 += 16) {
+    auto place = [&](int n) { return out + (kLanes ? (int64_t)(c0 + n) * p.ld + row : (int64_t)row * p.ld + c0 + n); };
+    uint32_t odd = 0;
+#pragma unroll 1
+    for (int n = 0; n < 16; ++n)
+      if (row < p.rows && c0 + n < p.cols) odd |= (__float_as_uint(*place(n)) << 1 >= 2 * 0x7f800000u ? 1u : 0u) << n;
+    if (!__any_sync(0xffffffffu, odd != 0)) continue;
+    const int at_col = min(c0 + (lane & 15), p.cols - 1);
+    float acc[16];
+#pragma unroll
+    for (int n = 0; n < 16; ++n) acc[n] = 0.0f;
+#pragma unroll 4
+    for (int c = c_begin; c < c_end; ++c) {
+      const float mine = G32 ? g_value(p.row_first + at_row, c) : q_value(p.row_first + at_row, c);
+      const float theirs = G32 ? q_value(at_col, c) : g_value(at_col, c);
+#pragma unroll
+      for (int n = 0; n < 16; ++n) acc[n] = fmaf(mine, __shfl_sync(0xffffffffu, theirs, n), acc[n]);
+    }
+#pragma unroll
+    for (int n = 0; n < 16; ++n)
+      if (odd >> n & 1) *place(n) = acc[n];
   }
-  return acc;
 }
 
 // N columns per tile; TOKENS: c is the operands' outer dimension; G32: the terms are g's (rows are j, columns i), else Q's (rows i, columns j).
@@ -345,11 +373,10 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
   } else {
     const int quad = warp & 3, half = (warp - 2) >> 2;      // rows 32 quad .., columns kCols half ..
     uint32_t group = 0;
-    bool ok = true;
+    bool ok = true, odd = false;        // odd: some sum of this thread is not finite
     for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
       int row0, col0, u, u_end;
       const int split = item_of(w, row0, col0, u, u_end);
-      const int c_begin = u * kDepth, c_end = min(p.src.C, u_end * kDepth);
       float acc[kCols];
 #pragma unroll
       for (int n = 0; n < kCols; ++n) acc[n] = 0.0f;
@@ -381,9 +408,7 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
       if (!ok) break;
       const int row = row0 + quad * 32 + lane, cb = col0 + half * kCols;
       float* out = p.out + (int64_t)split * p.part;
-      uint32_t odd[(kCols + 31) / 32];          // the sums that are not finite
-#pragma unroll
-      for (int k = 0; k < (kCols + 31) / 32; ++k) odd[k] = 0;
+      uint32_t most = 0;                        // twice the largest magnitude's bits
 #pragma unroll
       for (int k = 0; k < kCols / 16; ++k) {
         if (cb + 16 * k >= p.cols) break;
@@ -393,7 +418,7 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
 #pragma unroll
         for (int n = 16 * k; n < 16 * k + 16; ++n) {
           acc[n] = !TOKENS && G32 ? acc[n] * big * small : acc[n] * kScaleDown;
-          odd[n >> 5] |= (__float_as_uint(acc[n]) << 1 >= 2 * 0x7f800000u ? 1u : 0u) << (n & 31);
+          most = max(most, __float_as_uint(acc[n]) << 1);
         }
         if (row < p.rows) {
           if (kLanes) {
@@ -407,20 +432,16 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
           }
         }
       }
-      if (row < p.rows) {
+      odd |= row < p.rows && most >= 2 * 0x7f800000u;
+    }
+    // Sums that are not finite are made again when the CTA's tiles are done: nothing waits for these warps any more, however long it takes
+    // (with all of a long contraction's sums to make, longer than a bounded wait lasts).
+    if (__all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, odd)) {
 #pragma unroll 1
-        for (int k = 0; k < (kCols + 31) / 32; ++k) {
-          uint32_t left = odd[0];
-#pragma unroll
-          for (int q = 1; q < (kCols + 31) / 32; ++q) left = k == q ? odd[q] : left;
-          while (left) {
-            const int n = 32 * k + __ffs(left) - 1, col = cb + n;
-            left &= left - 1;
-            if (col >= p.cols) continue;
-            const int i = G32 ? col : p.row_first + row, j = G32 ? p.row_first + row : col;
-            out[kLanes ? (int64_t)col * p.ld + row : (int64_t)row * p.ld + col] = plain_dot(p.src, i, j, c_begin, c_end);
-          }
-        }
+      for (int w = blockIdx.x; w < items; w += gridDim.x) {
+        int row0, col0, u, u_end;
+        const int split = item_of(w, row0, col0, u, u_end);
+        remake_sums<N, TOKENS, G32>(p, p.out + (int64_t)split * p.part, row0 + quad * 32, col0 + half * kCols, u * kDepth, min(p.src.C, u_end * kDepth));
       }
     }
   }
@@ -590,7 +611,7 @@ int split_dot_run(const SplitDotPlan& d, int tokens, const uint8_t* q, const uin
       if (int s = make_map(&other, other_at, C, oc, C, 1, oc * C, kDepth, d.n, false)) return s;
     }
     SplitParams p{};
-    p.src = DotSource{q, sc8, sc32, g, cols, tokens ? J : C, (uint32_t)d.nbc, (uint32_t)d.log2_K, (uint32_t)log2_of(a), (uint32_t)log2_of(b), (int)C, tokens, g_bf16 ? 1 : 0};
+    p.src = DotSource{q, sc8, sc32, g, cols, tokens ? J : C, (uint32_t)d.nbc, (uint32_t)d.log2_K, (uint32_t)log2_of(a), (uint32_t)log2_of(b), (int)C};
     p.ld = tokens ? J : I;
     p.out = d.splits > 1 ? parts : out + (g_bf16 ? (tokens ? r0 * J : r0) : (tokens ? r0 : r0 * I));
     p.part = I * J;

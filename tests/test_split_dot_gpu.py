@@ -113,6 +113,27 @@ def test_infinities_nans_and_blocks_far_below_their_group(built_lib, tokens, dty
     assert torch.isnan(got[:, 33]).all() and not torch.isfinite(got[:, 17]).any() and torch.isfinite(got[:, rest]).all()
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("tokens", [0, 1])
+def test_no_wait_runs_out_while_every_sum_is_made_again(built_lib, diag_lib, tokens, dtype):
+    """Cotangents whose sums pass f32's largest number with the terms' 2^40 and do not without it: all sums of every tile are made again.
+    Three tiles a CTA, 8192 of the contraction, and waits of eight milliseconds at most: the tiles behind do not wait for it."""
+    rows, cols, grid, free = (8192, 2048, (1, 128), 5000) if tokens else (2048, 8192, (128, 128), 5000)
+    triple, g = _inputs(rows, cols, grid, free, tokens, dtype, amp=1e32)
+    st = torch.cuda.current_stream().cuda_stream
+    try:
+        assert diag_lib.pb_debug_dot_control(1 << 12, 0) == 0
+        got, shared = _dot(diag_lib, tokens, triple, grid, g)
+        assert shared and diag_lib.pb_gemm_check(st) == 0
+    finally:
+        diag_lib.pb_debug_dot_control(0, 0)
+    a, b = _sums(tokens, triple, grid, g)
+    # f32 products, one after the other: a rounding a term, and those of an operand
+    assert ((got.double() - a @ b).abs() <= (a.abs() @ b.abs()) * 2.0 ** -24 * (a.shape[1] + 4)).all()
+    wild = torch.full_like(g, float("nan"))
+    assert torch.isnan(_dot(built_lib, tokens, triple, grid, wild)[0]).all() and built_lib.pb_gemm_check(st) == 0
+
+
 @pytest.mark.parametrize("tokens", [0, 1])
 def test_a_wait_that_runs_out_is_reported_and_the_next_launch_is_clean(built_lib, diag_lib, tokens):
     """The diagnostics build leaves the first stage of a launch unfilled, with a poll budget of about two milliseconds per wait."""
