@@ -9,8 +9,14 @@
 //   g in f32:   the fp8 values times their block's power of two (exact; where it is not, a NaN, see below); g as three terms, times
 //               the super-group's f32 factor where that varies along c (tokens == 1, one set of terms per 1024 columns of
 //               Q; one f32 rounding), while a factor that belongs to a column of dX goes to the finished sum.
-// Every f32 product is then exact in three tensor-core products, and the accumulator is emptied into f32 registers every 32 of c,
-// as in dense_dot.cu (the tensor core's own additions do not round to nearest).  The terms carry an exact 2^40, which keeps
+// Every f32 product is then exact in three tensor-core products, and the accumulator is emptied into f32 registers every 64 of c
+// (the tensor core's own additions do not round to nearest; dense_dot.cu empties every 32): the low terms of all 64 go first, so that
+// four additions meet a sum of full size, as many as there, and half as many f32 additions follow.  Contractions of a few hundred have
+// few of those to save, and where the low terms are the fp8 operand's the four are all that is left: bf16 g over fewer than
+// 384 of c empties every 32.  2-norm errors against 64 bits, dense_dot_kernel | every 64 | every 32, dW of 2048 x 2048, bf16 g: operands of
+// one sign, 128 of c 8.4e-8 | 8.7e-8 | 6.3e-8, 256 8.7e-8 | 8.8e-8 | 6.7e-8, 384 9.5e-8 | 9.1e-8 | 7.6e-8, 2048 13.8e-8 | 11.4e-8 | 12.6e-8; of mixed signs, 128
+// 11.3e-8 | 8.3e-8 | 7.0e-8, 2048 18.1e-8 | 13.1e-8 | 15.8e-8.  f32 g, one sign, 128: 8.5e-8 | 5.6e-8 | 5.6e-8, 2048 13.8e-8 | 9.4e-8 | 12.3e-8.
+// The terms carry an exact 2^40, which keeps
 // them above bf16's subnormals.  A sum that is not finite, for an infinity or a NaN in the operands, an overflow of a scaled
 // term or a power of two that bf16 does not hold, is made again with f32 products of dequantized values, behind the last tile.
 //
@@ -31,7 +37,8 @@ namespace {
 
 constexpr int kTermRows = 128;        // of the three-term operand, per tile
 constexpr int kDepth = 32;            // c per stage
-constexpr int kGroup = 2;             // stages per accumulator
+constexpr int kGroup = 2;             // stages per accumulator, at most
+constexpr int kShortDepth = 384;      // of c, from which bf16 g takes that many
 constexpr int kTermBytes = kTermRows * kDepth * 2;
 constexpr int kDrainWarps = 8;
 constexpr int kThreads = 64 + 32 * kDrainWarps;
@@ -66,6 +73,7 @@ struct SplitParams {
   int row_first;                      // the first of these rows, for the sums that are made again
   int row_tiles, tiles, splits, units, units_per_split;
   int cols_per_variant;               // columns of Q that share a set of terms
+  int group;                          // stages per accumulator: 1 or kGroup
   uint32_t polls;
   int withhold;                       // diagnostics build: the first stage is never filled
 };
@@ -338,8 +346,8 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
       for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
         int row0, col0, u, u_end;
         item_of(w, row0, col0, u, u_end);
-        for (; u < u_end; u += kGroup, ++group) {
-          const int ab = group & 1, depth = min(kGroup, u_end - u);
+        for (; u < u_end; u += p.group, ++group) {
+          const int ab = group & 1, depth = min(p.group, u_end - u);
           if (!bar_wait(acc_empty(ab), ((group >> 1) & 1) ^ 1, p.polls)) { ok = false; break; }
           uint32_t at[kGroup], freed[kGroup];
 #pragma unroll
@@ -380,7 +388,7 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
       float acc[kCols];
 #pragma unroll
       for (int n = 0; n < kCols; ++n) acc[n] = 0.0f;
-      for (; u < u_end; u += kGroup, ++group) {
+      for (; u < u_end; u += p.group, ++group) {
         const int ab = group & 1;
         if (!bar_wait(acc_full(ab), (group >> 1) & 1, p.polls)) { ok = false; break; }
         __syncwarp();
@@ -622,6 +630,7 @@ int split_dot_run(const SplitDotPlan& d, int tokens, const uint8_t* q, const uin
     p.tiles = p.row_tiles * (int)((oc + d.n - 1) / d.n);
     p.splits = d.splits; p.units = d.units; p.units_per_split = d.units_per_split;
     p.cols_per_variant = (int)(I / d.variants);
+    p.group = g_bf16 && C < kShortDepth ? 1 : kGroup;
     p.polls = kWaitPolls;
 #ifdef PB_DIAGNOSTICS
     p.polls = g_split_polls.load(); p.withhold = g_split_withhold.load();

@@ -70,6 +70,23 @@ def test_sums_against_64_bits_and_the_other_form(built_lib, tokens, rows, cols, 
     assert built_lib.pb_gemm_check(torch.cuda.current_stream().cuda_stream) == 0
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("tokens,depth", [(0, 128), (0, 256), (0, 512), (1, 128), (1, 200), (1, 256), (1, 320), (1, 376), (1, 384), (1, 512), (1, 1000)])
+def test_short_sums_of_one_sign_are_no_less_precise_than_the_other_form(built_lib, tokens, depth, dtype):
+    """Where nothing cancels, what the tensor core's additions drop adds up, and few f32 additions follow that could hide it."""
+    rows, cols, grid = (depth, 2048, (1, 128)) if tokens else (2048, depth, (128, 128))
+    gen = torch.Generator(device="cuda").manual_seed(depth)
+    triple = quantize_impl(torch.randn(rows, cols, generator=gen, device="cuda").abs() * 0.02, grid)
+    g = (torch.randn(depth, 2048, generator=gen, device="cuda").abs() * 1e-3).to(dtype)
+    g = g if tokens else g.t().contiguous()
+    got, shared = _dot(built_lib, tokens, triple, grid, g)
+    assert shared
+    a, b = _sums(tokens, triple, grid, g)
+    want = a @ b
+    assert ((got.double() - want).abs() <= _bound(a, b)).all()
+    assert (got.double() - want).norm() <= (_dot(built_lib, tokens, triple, grid, g, best=False)[0].double() - want).norm()
+
+
 def test_the_cases_reach_this_form(built_lib):
     """A changed rule that leaves these cases to the other form would leave this one untested."""
     size = lambda c, code: built_lib.pb_dense_dot_workspace_best(c[0], c[1], c[2], *c[3], c[4], code) - built_lib.pb_dense_dot_workspace_size(c[0], c[1], c[2], *c[3], c[4])
