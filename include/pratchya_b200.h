@@ -184,6 +184,8 @@ typedef struct pb_operand {
                              pratchya/_nnx_impl/_module.py:82-84, 326), used without re-quantizing; 0 otherwise */
 } pb_operand;
 
+/* What the fastest kernel for these shapes takes.  A workspace that was sized for more rows of A also serves fewer: where it is too
+ * small for the kernel that is faster there, pb_gemm_tn takes another, with the same bits. */
 PB_API size_t pb_gemm_workspace_size(const pb_operand* a, const pb_operand* b);
 PB_API int pb_gemm_tn(const pb_operand* a, const pb_operand* b,
                void* d, int d_dtype, int64_t ldd,

@@ -1415,6 +1415,11 @@ void cut_contraction(int bn, int most, bool halves, int nchunks, int* split, int
   }
 }
 
+void take_wide(GemmPlan* gp, int64_t m) {
+  gp->pair = m > 128;
+  gp->BN = gp->pair ? Cfg2::BN : 224;
+}
+
 // Which kernel, by how long each would take in us: what a launch costs whatever its depth, and per wave of tiles the k-blocks of one,
 // with a drain of the accumulator every P of them.  A k-block takes 570 cycles in every form where the chip is not full (the MMA
 // thread's waits, commits and issues, not the tensor core), so few rows want many narrow tiles, and where those are still few the
@@ -1441,12 +1446,11 @@ void choose_kernel(GemmPlan* gp, int64_t m, int64_t n) {
     const double w = waves((m + 255) / 256 * ((n + Cfg2::BN - 1) / Cfg2::BN) * (halves ? 2 : 1), sms / 2);
     // nothing is changed for what the fit may be off by
     best = 0.88 * (7.1 + (halves ? 2.0 : 0.0) + w * gp->KB * (halves ? 0.5 : 1.0) * (0.31 + 0.74 * drains) + (w - 1) * 1.6) - 0.2;
-    gp->pair = true; gp->BN = Cfg2::BN;
   } else {
     const double w = waves((n + 223) / 224, sms);
     best = 5.8 + w * gp->KB * (0.33 + 1.03 * drains) + (w - 1) * 1.6 - 0.2;
-    gp->pair = false; gp->BN = 224;
   }
+  take_wide(gp, m);
   for (const Form& f : forms) {
     const int64_t tiles = (m + 127) / 128 * ((n + f.bn - 1) / f.bn);
     int split, chunks;
@@ -1462,7 +1466,23 @@ void choose_kernel(GemmPlan* gp, int64_t m, int64_t n) {
   }
 }
 
-int make_plan(const pb_operand* a, const pb_operand* b, GemmPlan* gp) {
+// Where the prepared scales lie in the workspace.  A's come first: the same place whatever the kernel.
+void lay_out(GemmPlan* gp, int64_t n) {
+  gp->tiles_n = (int)((n + gp->BN - 1) / gp->BN);
+  gp->atoms_b = (gp->BN + 127) / 128;
+  gp->Npad = (gp->tiles_n * gp->BN + 255) / 256 * 256;
+  auto align = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  size_t off = 0;
+  gp->off_sfa = off; off = align(off + (size_t)gp->KG * gp->tiles_m * 512);
+  gp->off_fa = off;  off = align(off + (size_t)gp->nchunks * gp->Mpad * 4);
+  gp->off_sfb = off; off = align(off + (size_t)gp->KG * gp->tiles_n * gp->atoms_b * 512);
+  gp->off_fb = off;  off = align(off + (size_t)gp->nchunks * gp->Npad * 4);
+  gp->total = off;
+}
+
+// workspace_bytes: what there is of it.  Narrow tiles have more scale-factor atoms, so a workspace that was sized for more rows of A
+// can be too small for them: the product then takes the wide ones, with the same bits.
+int make_plan(const pb_operand* a, const pb_operand* b, GemmPlan* gp, size_t workspace_bytes = SIZE_MAX) {
   if (!a || !b) return fail(PB_ERR_NULL_POINTER, "pb_gemm_tn: operands must be non-null");
   if (int s = plan_operand(a, "A", &gp->pa)) return s;
   if (int s = plan_operand(b, "B", &gp->pb)) return s;
@@ -1476,16 +1496,11 @@ int make_plan(const pb_operand* a, const pb_operand* b, GemmPlan* gp) {
   choose_kernel(gp, a->rows, b->rows);
   gp->Mpad = (int)((a->rows + 255) / 256 * 256);
   gp->tiles_m = gp->Mpad / 128;
-  gp->tiles_n = (int)((b->rows + gp->BN - 1) / gp->BN);
-  gp->atoms_b = (gp->BN + 127) / 128;
-  gp->Npad = (gp->tiles_n * gp->BN + 255) / 256 * 256;
-  auto align = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  size_t off = 0;
-  gp->off_sfa = off; off = align(off + (size_t)gp->KG * gp->tiles_m * 512);
-  gp->off_sfb = off; off = align(off + (size_t)gp->KG * gp->tiles_n * gp->atoms_b * 512);
-  gp->off_fa = off;  off = align(off + (size_t)gp->nchunks * gp->Mpad * 4);
-  gp->off_fb = off;  off = align(off + (size_t)gp->nchunks * gp->Npad * 4);
-  gp->total = off;
+  lay_out(gp, b->rows);
+  if (gp->total > workspace_bytes && !forced_bn() && pick_pair()) {
+    take_wide(gp, a->rows);
+    lay_out(gp, b->rows);
+  }
   return PB_OK;
 }
 
@@ -1578,7 +1593,7 @@ int launch_gemm_pair_uni(const CUtensorMap& ma, const CUtensorMap& mb, const CUt
 int gemm_a_prep_location(const pb_operand* a, const pb_operand* b, void* workspace, size_t workspace_bytes,
                          uint8_t** sf, float** f, uint32_t* tiles, uint32_t* Mpad) {
   GemmPlan gp;
-  if (int s = make_plan(a, b, &gp)) return s;
+  if (int s = make_plan(a, b, &gp, workspace_bytes)) return s;
   if (gp.P != kMaxChunk)
     return fail(PB_ERR_UNSUPPORTED, "pb_quantize_for_gemm: this operand pair promotes every %d k-blocks, the fused preparation needs %d", gp.P, kMaxChunk);
   if (!workspace || workspace_bytes < gp.total)
@@ -1611,7 +1626,7 @@ extern "C" int pb_gemm_tn(const pb_operand* a, const pb_operand* b, void* d, int
 extern "C" int pb_gemm_tn_ex(const pb_operand* a, const pb_operand* b, void* d, int d_dtype, int64_t ldd,
                              void* workspace, size_t workspace_bytes, unsigned int flags, void* stream) {
   GemmPlan gp;
-  if (int s = make_plan(a, b, &gp)) return s;
+  if (int s = make_plan(a, b, &gp, workspace_bytes)) return s;
   if (flags & ~(unsigned)(PB_GEMM_A_PREPARED | PB_GEMM_B_PREPARED))
     return fail(PB_ERR_UNSUPPORTED, "pb_gemm_tn_ex: unknown flag bits 0x%x", flags);
   if ((flags & PB_GEMM_A_PREPARED) && gp.P != kMaxChunk)

@@ -41,6 +41,36 @@ def test_products_against_64_bits(built_lib, m, k, n, grid):
     assert built_lib.pb_gemm_check(torch.cuda.current_stream().cuda_stream) == 0
 
 
+@pytest.mark.parametrize("m,k,n,grid", [(8, 2048, 8192, (128, 1)), (64, 2048, 2048, (128, 128)), (100, 2048, 8192, (128, 128)), (136, 2048, 2048, (128, 128)), (500, 1024, 1024, (128, 128))])
+def test_a_workspace_for_more_rows_serves_fewer(built_lib, m, k, n, grid):
+    """A host with one workspace for all of its batch sizes: what the largest takes is enough for every other, and the bits are the same."""
+    xq, wq = _triples(m, k, n, grid)
+    wt, st = _ops.transpose_bytes(wq[0]), torch.cuda.current_stream().cuda_stream
+    b = _ops._operand(wt, wq[1], wq[2], n, k, (grid[1], 128), 1)
+    a = _ops._operand(*xq, m, k, (1, 128))
+    large = _ops._operand(*xq, 1024, k, (1, 128))                      # describes a size: nothing is read through it
+    own, size = built_lib.pb_gemm_workspace_size(a, b), built_lib.pb_gemm_workspace_size(large, b)
+
+    def run(size, x=None):
+        ws, d = torch.full((size + 512,), 0xa5, dtype=torch.uint8, device="cuda"), torch.full((m, n), float("nan"), device="cuda")
+        if x is not None:                                              # A's scales by the quantizer, into the same workspace
+            q, s8, s32 = [torch.empty_like(t) for t in xq]
+            _lib.check(built_lib.pb_quantize_for_gemm(x.data_ptr(), _lib.PB_F32, m, k, _lib.PB_E4M3, q.data_ptr(), s8.data_ptr(), s32.data_ptr(), b, ws.data_ptr(), size, st))
+            _lib.check(built_lib.pb_gemm_tn_ex(_ops._operand(q, s8, s32, m, k, (1, 128)), b, d.data_ptr(), _lib.PB_F32, n, ws.data_ptr(), size, 1, st))
+        else:
+            _lib.check(built_lib.pb_gemm_tn(a, b, d.data_ptr(), _lib.PB_F32, n, ws.data_ptr(), size, st))
+        assert (ws[size:] == 0xa5).all()
+        return d
+
+    want = run(own)
+    assert torch.equal(run(size), want)
+    if grid == (128, 128):
+        g = torch.Generator(device="cuda").manual_seed(m + k + n)      # as _triples
+        x = torch.randn(m, k, generator=g, device="cuda") * torch.randn(m, 1, generator=g, device="cuda").exp()
+        assert torch.equal(run(size, x), want)
+    assert built_lib.pb_gemm_check(st) == 0
+
+
 def test_outputs_with_longer_rows_and_off_the_store_alignment(built_lib):
     """ldd beyond n, and rows that are no multiple of 16 bytes: nothing but [m, n] is written."""
     for m, k, n, ldd in [(40, 4096, 512, 640), (40, 2048, 512, 513), (130, 1024, 256, 300), (7, 1024, 128, 129)]:
