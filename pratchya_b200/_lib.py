@@ -161,6 +161,14 @@ def native():
     return _native
 
 
+def gemm_workspace_bound(rows: int, depth: int, n: int) -> int:
+    """An upper bound of pb_gemm_workspace_size for a (1,128) operand of `rows` against a (128,128) one of `n`, for hosts that
+    declare their scratch before the library is asked: scale-factor atoms (two per tile of 224 columns, one per tile of 32) and
+    fp32 factors of both operands."""
+    kb = depth // 128
+    return 4096 + ((kb + 3) // 4) * 512 * ((rows + 255) // 128 + max(2 * ((n + 223) // 224), (n + 31) // 32) + 2) + 4 * kb * (rows + n + 1024)
+
+
 _SAME_DEVICE = contextlib.nullcontext()
 
 

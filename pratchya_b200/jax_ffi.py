@@ -86,9 +86,7 @@ def matmul_impl_forward(x_fp8, x_sc8, x_sc32, w_t_fp8, w_sc8, w_sc32):
     n = w_t_fp8.shape[0]
     rows = math.prod(x_fp8.shape[:-1])
     depth = x_fp8.shape[-1]
-    # an upper bound of pb_gemm_workspace_size: scale-factor atoms and fp32 factors of both operands
-    kb = depth // 128
-    scratch = 4096 + ((kb + 3) // 4) * 512 * ((rows + 255) // 128 + 2 * ((n + 223) // 224) + 2) + 4 * kb * (rows + n + 1024)
+    scratch = _lib.gemm_workspace_bound(rows, depth, n)
     y, _ = jax.ffi.ffi_call("pb_matmul", (
         jax.ShapeDtypeStruct((*x_fp8.shape[:-1], n), jnp.float32),
         jax.ShapeDtypeStruct((scratch,), jnp.uint8),

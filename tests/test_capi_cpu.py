@@ -74,3 +74,12 @@ def test_argument_errors_of_the_fused_entry_points(built_lib):
     a = _lib.Operand(4096, 4096, 4096, 256, 1024, 1, 128, 0, 0)
     assert built_lib.pb_gemm_tn_ex(a, op, one, 0, 1024, one, 1 << 20, 8, None) == _lib.PB_ERR_UNSUPPORTED
     assert b"flag" in built_lib.pb_last_error()
+
+
+def test_the_bound_of_the_gemm_workspace_is_one(built_lib):
+    """What a host declares before it can ask the library (an XLA call's scratch) holds every form that a size can take."""
+    for rows in (1, 8, 27, 44, 64, 107, 128, 129, 200, 500, 1000, 1024, 4096, 30000):
+        for depth in (128, 256, 640, 1024, 2048, 4096, 10240):
+            for n in (128, 256, 1920, 2048, 6656, 8064, 17792, 65536):
+                a, b = _lib.Operand(256, 256, 256, rows, depth, 1, 128, 0, 0), _lib.Operand(256, 256, 256, n, depth, 128, 128, 0, 1)
+                assert built_lib.pb_gemm_workspace_size(a, b) <= _lib.gemm_workspace_bound(rows, depth, n), (rows, depth, n)
