@@ -520,7 +520,14 @@ def _dense_dot(tokens: int, q, sc8, sc32, grid, g: torch.Tensor):
     with _lib.on_device(g.device):
         out = torch.empty((free, rows) if tokens == 0 else (cols, free), dtype=torch.float32, device=g.device)
         ws_bytes = lib.pb_dense_dot_workspace_best(tokens, rows, cols, grid[0], grid[1], free, _DENSE_CODE[g.dtype])
-        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=g.device) if ws_bytes else None
+        try:
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=g.device) if ws_bytes else None
+        except torch.OutOfMemoryError:                   # the form that takes less of it
+            least = lib.pb_dense_dot_workspace_size(tokens, rows, cols, grid[0], grid[1], free)
+            if least == ws_bytes:
+                raise
+            ws_bytes = least
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=g.device) if ws_bytes else None
         check(lib.pb_dense_dot(tokens, q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), rows, cols, grid[0], grid[1], g.data_ptr(), _DENSE_CODE[g.dtype], free,
                                out.data_ptr(), ws.data_ptr() if ws is not None else None, ws_bytes, _stream(g)))
     return out

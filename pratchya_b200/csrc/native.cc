@@ -433,8 +433,15 @@ OP(dense_dot) {
   const int type = code(g->scalar_type());
   const c10::cuda::CUDAGuard guard(g->device());
   at::Tensor out = tokens ? empty({cols, free}, at::kFloat, *g) : empty({free, rows}, at::kFloat, *g), ws;
-  const size_t bytes = pb_dense_dot_workspace_best(tokens, rows, cols, a, b, free, type);
-  if (bytes) ws = scratch(bytes, *g);
+  size_t bytes = pb_dense_dot_workspace_best(tokens, rows, cols, a, b, free, type);
+  try {
+    if (bytes) ws = scratch(bytes, *g);
+  } catch (const c10::OutOfMemoryError&) {      // the form that takes less of it
+    const size_t least = pb_dense_dot_workspace_size(tokens, rows, cols, a, b, free);
+    if (least == bytes) throw;
+    bytes = least;
+    if (bytes) ws = scratch(bytes, *g);
+  }
   RUN(pb_dense_dot(tokens, (const uint8_t*)q->data_ptr(), (const uint8_t*)sc8->data_ptr(), (const float*)sc32->data_ptr(), rows, cols, a, b, g->data_ptr(), type, free,
                    (float*)out.data_ptr(), bytes ? ws.data_ptr() : nullptr, bytes, current_stream(g->device())));
   return wrap(out);

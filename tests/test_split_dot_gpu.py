@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from pratchya_b200 import _lib
-from pratchya_b200._qualia import dequantize_impl, quantize_impl
+from pratchya_b200._qualia import _ops, dequantize_impl, quantize_impl
 
 pytestmark = pytest.mark.gpu
 
@@ -149,6 +149,26 @@ def test_no_wait_runs_out_while_every_sum_is_made_again(built_lib, diag_lib, tok
     assert ((got.double() - a @ b).abs() <= (a.abs() @ b.abs()) * 2.0 ** -24 * (a.shape[1] + 4)).all()
     wild = torch.full_like(g, float("nan"))
     assert torch.isnan(_dot(built_lib, tokens, triple, grid, wild)[0]).all() and built_lib.pb_gemm_check(st) == 0
+
+
+@pytest.mark.parametrize("whole_op", [True, False])
+@pytest.mark.parametrize("tokens,dtype", [(0, F32), (1, F32), (1, BF16)])
+def test_where_its_workspace_does_not_fit_the_other_form_runs(built_lib, monkeypatch, tokens, dtype, whole_op):
+    """Torch's allocator is held to 48 MB more than it has: room for out and the least workspace, not for the terms."""
+    rows, cols, grid, free = (8192, 2048, (1, 128), 2048) if tokens else (2048, 8192, (128, 128), 2048)
+    triple, g = _inputs(rows, cols, grid, free, tokens, dtype)
+    want = _dot(built_lib, tokens, triple, grid, g, best=False)[0]
+    if not whole_op:                                             # the Python text
+        real = _lib.native()
+        monkeypatch.setattr(_lib, "_native", type("Declining", (), {"dense_dot": lambda self, *args: None, "__getattr__": lambda self, name: getattr(real, name)})())
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (48 << 20)) / total)
+        got = _ops._dense_dot(tokens, *triple, grid, g)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("tokens", [0, 1])
