@@ -388,7 +388,8 @@ PB_API int pb_smoothed_xent_bwd(const float* logits, const int64_t* target, cons
  * with f32 products and sums over the whole f32 range (every f32 product as three exact bf16 tensor-core products; sums that
  * are not finite that way are made again with plain f32 products).  q, g, out and the workspace are 16-byte aligned.  Any other grid or shape: PB_ERR_UNSUPPORTED, and a workspace size of 0.
  * pb_dense_dot_workspace_size is the least workspace; pb_dense_dot_workspace_best what the fastest form for this size and type of g
- * (PB_F32, PB_BF16) takes, which pb_dense_dot chooses where the workspace allows it. */
+ * (PB_F32, PB_BF16) takes, which pb_dense_dot chooses where workspace_bytes allow it.  The two forms add in different orders: a result's
+ * last bits depend on which of the two sizes the workspace has, and on nothing else of it. */
 PB_API size_t pb_dense_dot_workspace_size(int tokens, int64_t rows, int64_t cols, int a, int b, int64_t g_free);
 PB_API size_t pb_dense_dot_workspace_best(int tokens, int64_t rows, int64_t cols, int a, int b, int64_t g_free, int g_dtype);
 PB_API int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, const float* sc32, int64_t rows, int64_t cols, int a, int b,

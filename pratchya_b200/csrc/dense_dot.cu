@@ -511,7 +511,7 @@ extern "C" size_t pb_dense_dot_workspace_best(int tokens, int64_t rows, int64_t 
   if ((g_dtype != PB_F32 && g_dtype != PB_BF16) || !dot_shape_ok(tokens, rows, cols, a, b, g_free) ||
       !split_dot_plan(tokens, rows, cols, a, b, g_free, g_dtype == PB_BF16, &split))
     return least;
-  return std::max(least, split.bytes);
+  return std::max(least, split.bytes + kSplitAlign - 16);
 }
 
 extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, const float* sc32, int64_t rows, int64_t cols, int a, int b,
@@ -534,8 +534,10 @@ extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, co
     return fail(PB_ERR_WORKSPACE_TOO_SMALL, "pb_dense_dot: needs %zu bytes of workspace, got %zu", need, workspace_bytes);
   if (reinterpret_cast<uintptr_t>(workspace) & 15) return fail(PB_ERR_MISALIGNED, "pb_dense_dot: workspace must be 16-byte aligned");
   SplitDotPlan split;
-  if (workspace && !(reinterpret_cast<uintptr_t>(workspace) & 31) && split_dot_plan(tokens, rows, cols, a, b, g_free, g_dtype == PB_BF16, &split) && workspace_bytes >= split.bytes)
-    return split_dot_run(split, tokens, q, sc8, sc32, rows, cols, a, b, g, g_dtype == PB_BF16, g_free, out, workspace, static_cast<cudaStream_t>(stream));
+  const size_t skip = (size_t)(-reinterpret_cast<uintptr_t>(workspace)) & (kSplitAlign - 1);
+  if (workspace && split_dot_plan(tokens, rows, cols, a, b, g_free, g_dtype == PB_BF16, &split) && workspace_bytes >= split.bytes + skip)
+    return split_dot_run(split, tokens, q, sc8, sc32, rows, cols, a, b, g, g_dtype == PB_BF16, g_free, out, static_cast<unsigned char*>(workspace) + skip,
+                         static_cast<cudaStream_t>(stream));
   uint32_t log2_K = 0;                  // K divides 8, or 1024 for (128,128)
   while ((1ll << log2_K) < geo.K) ++log2_K;
   cudaStream_t st = static_cast<cudaStream_t>(stream);

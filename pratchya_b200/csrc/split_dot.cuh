@@ -8,6 +8,8 @@
 
 namespace pb {
 
+constexpr size_t kSplitAlign = 32;    // of the workspace: the terms are stored 32 bytes at a time
+
 struct SplitDotPlan {
   int n, tiles, row_tiles, splits, units, units_per_split, variants, nbc, log2_K;
   int64_t slab;                       // rows of the three-term operand at a time

@@ -87,6 +87,24 @@ def test_short_sums_of_one_sign_are_no_less_precise_than_the_other_form(built_li
     assert (got.double() - want).norm() <= (_dot(built_lib, tokens, triple, grid, g, best=False)[0].double() - want).norm()
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+def test_a_workspace_off_32_bytes_gives_the_same_form(built_lib, dtype):
+    """The workspace's alignment is 16 bytes; the bits do not depend on more of it, and nothing beyond its size is written."""
+    rows, cols, grid, free = 1000, 1024, (1, 128), 1032
+    (q, sc8, sc32), g = _inputs(rows, cols, grid, free, 1, dtype)
+    want, shared = _dot(built_lib, 1, (q, sc8, sc32), grid, g)
+    assert shared
+    code = _lib.PB_BF16 if dtype == BF16 else _lib.PB_F32
+    size = built_lib.pb_dense_dot_workspace_best(1, rows, cols, *grid, free, code)
+    room = torch.full((size + 96,), 0xa5, dtype=torch.uint8, device="cuda")
+    assert room.data_ptr() % 32 == 0
+    for off in (16, 32, 48):
+        out = torch.empty_like(want)
+        _lib.check(built_lib.pb_dense_dot(1, q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), rows, cols, *grid, g.data_ptr(), code, free, out.data_ptr(),
+                                          room.data_ptr() + off, size, torch.cuda.current_stream().cuda_stream))
+        assert torch.equal(out, want) and (room[:16] == 0xa5).all() and (room[off + size:] == 0xa5).all()
+
+
 def test_the_cases_reach_this_form(built_lib):
     """A changed rule that leaves these cases to the other form would leave this one untested."""
     size = lambda c, code: built_lib.pb_dense_dot_workspace_best(c[0], c[1], c[2], *c[3], c[4], code) - built_lib.pb_dense_dot_workspace_size(c[0], c[1], c[2], *c[3], c[4])
