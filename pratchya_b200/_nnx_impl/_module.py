@@ -167,13 +167,14 @@ def _weight_bytes_t(wq, prepared):
 
 
 def _forward_only(x, weight, grid, fake_quant_output, prepared, prepared_x):
-    """The layer's output in one call of the extension, or None where it does not apply (_LinearFn.forward then says why)."""
-    a, b = grid
-    if a != 128 or weight.dim() != 2 or not weight.is_cuda or not x.is_cuda or weight.shape[0] % 128 or (b == 128 and weight.shape[1] % 128) or weight.shape[1] % 16:
+    """The layer's output in one call of the extension, or None where it does not apply (_LinearFn.forward then says why), asked
+    before anything is made of the weight.  What is made of it is in `prepared`."""
+    nat, (a, b) = _lib.native(), grid
+    row = prepared_x[0] if prepared_x is not None else (None, None, None)
+    if a != 128 or not nat.linear_takes(x, row[0], weight, b, fake_quant_output):
         return None
     wq = _weight_triple(weight, grid, prepared)
-    row = prepared_x[0] if prepared_x is not None else (None, None, None)
-    return _lib.native().linear(x, *row, wq[1], wq[2], _weight_bytes_t(wq, prepared), b, fake_quant_output)
+    return nat.linear(x, *row, wq[1], wq[2], _weight_bytes_t(wq, prepared), b, fake_quant_output)
 
 
 class _LinearFn(torch.autograd.Function):
@@ -273,6 +274,7 @@ def linear_fp8(x, weight: torch.Tensor, tgrid=(128, 128), *, fake_quant_output: 
         x, prepared_x = x.handle, (x.row, x.tokens)
     grid = (int(tgrid[0]), int(tgrid[1]))
     if no_graph():
+        prepared = {} if prepared is None else prepared          # what the extension's call makes of the weight is there if it then declines
         y = _forward_only(x, weight, grid, fake_quant_output, prepared, prepared_x)
         return y if y is not None else _LinearFn.forward(NoContext(), x, weight, grid, fake_quant_output, recipe, grad_format, False, prepared, prepared_x)
     for_backward = torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)

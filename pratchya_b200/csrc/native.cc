@@ -340,6 +340,27 @@ OP(gemm) {
   END_HANDLE_TH_ERRORS
 }
 
+// Whether `linear` takes an x (with x_q given, of its quantized rows) for a weight of [depth, cols] on (128, b)
+bool linear_fits(PyObject* o, bool given, int64_t depth, int64_t cols, int b, bool fake, c10::Device device) {
+  if (!THPVariable_CheckExact(o) || watched() || depth <= 0 || depth % 128 || (b != 128 && b != 1)) return false;
+  const at::Tensor& x = THPVariable_Unpack(o);
+  if (!dense(x.scalar_type()) || x.dim() < 2 || x.size(-1) != depth || x.numel() == 0) return false;
+  const int64_t rows = x.numel() / depth;
+  if ((rows * (depth / 128)) % 8 || (b == 128 ? cols % 128 : cols % 16)) return false;
+  if (fake ? b != 128 || (rows * (cols / 128)) % 8 : x.scalar_type() != at::kFloat) return false;
+  return given || (plain(o) && x.device() == device);
+}
+// linear_takes(x, x_q, weight, b, fake): the same before the weight is quantized and turned for the call
+OP(linear_takes) {
+  HANDLE_TH_ERRORS
+  NARGS(5);
+  if (!THPVariable_Check(args[2])) Py_RETURN_FALSE;
+  const at::Tensor& w = THPVariable_Unpack(args[2]);
+  if (!w.is_cuda() || w.dim() != 2) Py_RETURN_FALSE;
+  return PyBool_FromLong(linear_fits(args[0], args[1] != Py_None, w.size(0), w.size(1), (int)integer(args[3]), PyObject_IsTrue(args[4]) == 1, w.device()));
+  END_HANDLE_TH_ERRORS
+}
+
 // linear(x, x_q, x_sc8, x_sc32, w_sc8, w_sc32, w_t, b, fake) -> y: a Linear whose weight is on (128, b) and whose gradient nobody wants.  With
 // x_q given x only lends its shape and type.  fake: the product is re-quantized on (1, b) and read back.
 OP(linear) {
@@ -348,13 +369,9 @@ OP(linear) {
   const bool given = args[1] != Py_None, fake = PyObject_IsTrue(args[8]) == 1;
   const at::Tensor *w8 = plain(args[4]), *w32 = plain(args[5]), *wt = plain(args[6]);
   const int b = (int)integer(args[7]);
-  if (!THPVariable_CheckExact(args[0]) || !w8 || !w32 || !wt || watched() || wt->dim() != 2 || !fp8(*wt) || (b != 128 && b != 1)) return none();
+  if (!w8 || !w32 || !wt || wt->dim() != 2 || !fp8(*wt) || !linear_fits(args[0], given, wt->size(1), wt->size(0), b, fake, wt->device())) return none();
   const at::Tensor& x = THPVariable_Unpack(args[0]);
-  const int64_t depth = wt->size(1), cols = wt->size(0);
-  if (!dense(x.scalar_type()) || x.dim() < 2 || x.size(-1) != depth || depth % 128 || x.numel() == 0) return none();
-  const int64_t rows = x.numel() / depth, blocks = rows * (depth / 128);
-  if (blocks % 8 || (b == 128 ? cols % 128 : cols % 16)) return none();
-  if (fake ? b != 128 || (rows * (cols / 128)) % 8 : x.scalar_type() != at::kFloat) return none();
+  const int64_t depth = wt->size(1), cols = wt->size(0), rows = x.numel() / depth, blocks = rows * (depth / 128);
   at::Tensor q, s8, s32;
   const c10::cuda::CUDAGuard guard(wt->device());
   void* st = current_stream(wt->device());
@@ -363,7 +380,6 @@ OP(linear) {
     if (!gq || !g8 || !g32 || gq->dim() != 2 || gq->size(0) != rows || gq->size(1) != depth || !fp8(*gq)) return none();
     q = *gq; s8 = *g8; s32 = *g32;
   } else {
-    if (!plain(args[0]) || x.device() != wt->device()) return none();
     q = empty({rows, depth}, kE4M3, x); s8 = empty({blocks / 8, 8}, kE8M0, x); s32 = empty({blocks / 8, 1, 1}, at::kFloat, x);
     at::Tensor ws;
     const size_t bytes = pb_quantize_workspace_size(1, rows, depth, 1, 128);
@@ -489,7 +505,7 @@ PyObject* set_error(PyObject*, PyObject* cls) {
 #define ENTRY(name) METHOD(#name, &Entry<&name>::call)
 PyMethodDef methods[] = {
     METHOD("quantize", quantize), METHOD("quantize_transposed", quantize_transposed), METHOD("dequantize", dequantize), METHOD("dequantize_bwd", dequantize_bwd),
-    METHOD("fake_quantize", fake_quantize), METHOD("transpose_bytes", transpose_bytes), METHOD("gemm", gemm), METHOD("linear_step", linear_step), METHOD("linear", linear),
+    METHOD("fake_quantize", fake_quantize), METHOD("transpose_bytes", transpose_bytes), METHOD("gemm", gemm), METHOD("linear_step", linear_step), METHOD("linear", linear), METHOD("linear_takes", linear_takes),
     METHOD("dense_dot", dense_dot), METHOD("empty", empty_on), METHOD("empties", empties),
     ENTRY(pb_quantize_dual), ENTRY(pb_dequantize_bwd_quantize_dual), ENTRY(pb_relu2_requantize), ENTRY(pb_quantize_transposed_workspace_size),
     ENTRY(pb_wkv7_forward), ENTRY(pb_wkv7_backward), ENTRY(pb_wkv7_checkpoint_floats),

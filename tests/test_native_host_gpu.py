@@ -124,6 +124,28 @@ def test_a_linear_without_a_graph_gives_the_bits_of_one_with_it(built_lib, both,
         assert all(torch.equal(k, mine) for k in kept) and set(keep) == {"wq", "w_t"}
 
 
+@pytest.mark.parametrize("prepared", [False, True])
+def test_a_linear_without_a_graph_prepares_its_weight_once(built_lib, monkeypatch, prepared):
+    """The calls that the extension leaves to the Python text, too: one quantization of the weight, and no byte transpose that no product reads."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    calls = []
+    for name in ("quantize_impl", "transpose_bytes"):
+        monkeypatch.setattr(_ops, name, lambda t, *args, _f=getattr(_ops, name), _n=name: (calls.append((_n, t.shape)), _f(t, *args))[1])
+    for w, grid, x, fake, turned in [
+            (r(1024, 128), (128, 1), r(64, 1024), True, 1), (r(1024, 128), (128, 1), r(64, 1024), False, 1), (r(1024, 512), (128, 128), r(1024, 64).t(), True, 1),
+            (r(1024, 512), (128, 128), r(64, 1024).bfloat16(), False, 1), (r(1024, 512), (128, 128), r(64, 1024).half(), True, 1), (r(1024, 512), (128, 128), r(64, 1024), True, 1),
+            (r(128, 256), (128, 128), r(3, 128), True, 0), (r(1024, 24), (128, 1), r(64, 1024), True, 0), (r(256, 256), (16, 16), r(64, 256), True, 0)]:
+        keep = {} if prepared else None
+        with torch.no_grad():
+            for again in (False, True):
+                calls.clear()
+                _module.linear_fp8(x, w, grid, fake_quant_output=fake, prepared=keep)
+                n = 0 if again and prepared else 1
+                assert sum(name == "quantize_impl" and shape == w.shape for name, shape in calls) == n, (tuple(w.shape), grid, calls)
+                assert sum(name == "transpose_bytes" for name, _ in calls) == n * turned, (tuple(w.shape), grid, calls)
+
+
 def test_ops_keep_their_function_where_a_derivative_can_be_asked_for(built_lib):
     x, w = torch.randn(8, 1024, device="cuda"), torch.randn(1024, 256, device="cuda") * 0.02
     scale = torch.ones(1024, device="cuda")
