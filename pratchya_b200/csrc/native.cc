@@ -195,12 +195,18 @@ long long integer(PyObject* o) {
   return v;
 }
 
+// the same for what the C entries take as an int: beyond one it is left, too, not cut to its low bits
+int small(PyObject* o) {
+  const long long v = integer(o);
+  return v == (int)v ? (int)v : 0;
+}
+
 // quantize(x, a, b, format) -> (q, sc8, sc32): quantize_impl
 OP(quantize) {
   HANDLE_TH_ERRORS
   NARGS(4);
   const at::Tensor* x = plain(args[0]);
-  const int a = (int)integer(args[1]), b = (int)integer(args[2]), fmt = (int)integer(args[3]);
+  const int a = small(args[1]), b = small(args[2]), fmt = small(args[3]);
   Grid g;
   if (!x || watched() || !dense(x->scalar_type()) || !g.of(x->sizes(), a, b)) return none();
   const c10::cuda::CUDAGuard guard(x->device());
@@ -218,7 +224,7 @@ OP(quantize_transposed) {
   HANDLE_TH_ERRORS
   NARGS(3);
   const at::Tensor* x = plain(args[0]);
-  const int b = (int)integer(args[1]), fmt = (int)integer(args[2]);
+  const int b = small(args[1]), fmt = small(args[2]);
   if (!x || watched() || !dense(x->scalar_type()) || x->dim() < 2) return none();
   c10::SmallVector<int64_t, 8> s(x->sizes().begin(), x->sizes().end());
   const int64_t rows = s[s.size() - 2], cols = s[s.size() - 1];
@@ -240,7 +246,7 @@ OP(dequantize) {
   HANDLE_TH_ERRORS
   NARGS(6);
   const at::Tensor *q = plain(args[0]), *sc8 = plain(args[1]), *sc32 = plain(args[2]);
-  const int a = (int)integer(args[4]), b = (int)integer(args[5]);
+  const int a = small(args[4]), b = small(args[5]);
   if (!q || !sc8 || !sc32 || watched() || !THPDtype_Check(args[3]) || !fp8(*q) || sc8->dim() < 2) return none();
   const at::ScalarType type = reinterpret_cast<THPDtype*>(args[3])->scalar_type;
   Grid g;
@@ -258,7 +264,7 @@ OP(dequantize_bwd) {
   HANDLE_TH_ERRORS
   NARGS(5);
   const at::Tensor *sc8 = plain(args[0]), *sc32 = plain(args[1]), *g_out = plain(args[2]);
-  const int a = (int)integer(args[3]), b = (int)integer(args[4]);
+  const int a = small(args[3]), b = small(args[4]);
   Grid g;
   if (!sc8 || !sc32 || !g_out || watched() || !dense(g_out->scalar_type()) || !g.of(g_out->sizes(), a, b)) return none();
   const c10::cuda::CUDAGuard guard(g_out->device());
@@ -274,7 +280,7 @@ OP(fake_quantize) {
   HANDLE_TH_ERRORS
   NARGS(6);
   const at::Tensor* x = plain(args[0]);
-  const int a = (int)integer(args[1]), b = (int)integer(args[2]), fmt = (int)integer(args[4]);
+  const int a = small(args[1]), b = small(args[2]), fmt = small(args[4]);
   const bool scales = PyObject_IsTrue(args[5]) == 1;
   if (!x || watched() || !THPDtype_Check(args[3]) || x->scalar_type() != at::kFloat) return none();
   const at::ScalarType type = reinterpret_cast<THPDtype*>(args[3])->scalar_type;
@@ -327,8 +333,8 @@ OP(gemm) {
   const at::ScalarType type = reinterpret_cast<THPDtype*>(args[9])->scalar_type;
   if (!dense(type)) return none();
   const int64_t depth = aq.size(-1), rows = aq.numel() / depth, cols = bq.size(0);
-  const pb_operand a{aq.data_ptr(), (const uint8_t*)t[1]->data_ptr(), (const float*)t[2]->data_ptr(), rows, depth, (int)integer(args[3]), 128, format(aq), 0};
-  const pb_operand b{bq.data_ptr(), (const uint8_t*)t[4]->data_ptr(), (const float*)t[5]->data_ptr(), cols, depth, (int)integer(args[7]), 128, format(bq), (int)integer(args[8])};
+  const pb_operand a{aq.data_ptr(), (const uint8_t*)t[1]->data_ptr(), (const float*)t[2]->data_ptr(), rows, depth, small(args[3]), 128, format(aq), 0};
+  const pb_operand b{bq.data_ptr(), (const uint8_t*)t[4]->data_ptr(), (const float*)t[5]->data_ptr(), cols, depth, small(args[7]), 128, format(bq), small(args[8])};
   const c10::cuda::CUDAGuard guard(aq.device());
   c10::SmallVector<int64_t, 8> shape(aq.sizes().begin(), aq.sizes().end());
   shape.back() = cols;
@@ -357,7 +363,7 @@ OP(linear_takes) {
   if (!THPVariable_Check(args[2])) Py_RETURN_FALSE;
   const at::Tensor& w = THPVariable_Unpack(args[2]);
   if (!w.is_cuda() || w.dim() != 2) Py_RETURN_FALSE;
-  return PyBool_FromLong(linear_fits(args[0], args[1] != Py_None, w.size(0), w.size(1), (int)integer(args[3]), PyObject_IsTrue(args[4]) == 1, w.device()));
+  return PyBool_FromLong(linear_fits(args[0], args[1] != Py_None, w.size(0), w.size(1), small(args[3]), PyObject_IsTrue(args[4]) == 1, w.device()));
   END_HANDLE_TH_ERRORS
 }
 
@@ -368,7 +374,7 @@ OP(linear) {
   NARGS(9);
   const bool given = args[1] != Py_None, fake = PyObject_IsTrue(args[8]) == 1;
   const at::Tensor *w8 = plain(args[4]), *w32 = plain(args[5]), *wt = plain(args[6]);
-  const int b = (int)integer(args[7]);
+  const int b = small(args[7]);
   if (!w8 || !w32 || !wt || wt->dim() != 2 || !fp8(*wt) || !linear_fits(args[0], given, wt->size(1), wt->size(0), b, fake, wt->device())) return none();
   const at::Tensor& x = THPVariable_Unpack(args[0]);
   const int64_t depth = wt->size(1), cols = wt->size(0), rows = x.numel() / depth, blocks = rows * (depth / 128);
@@ -408,7 +414,7 @@ OP(linear_step) {
   NARGS(10);
   const at::Tensor *x = plain(args[0]), *ws = plain(args[7]);
   const int64_t rows = integer(args[1]), k = integer(args[2]), cols = integer(args[3]);
-  const int fmt = (int)integer(args[5]);
+  const int fmt = small(args[5]);
   const bool ready = PyObject_IsTrue(args[8]) == 1, relu2 = PyObject_IsTrue(args[9]) == 1;
   if (!x || !ws || watched() || !THPDtype_Check(args[4]) || !dense(x->scalar_type()) || (relu2 && x->scalar_type() != at::kFloat) || x->dim() < 1 || x->numel() != rows * k ||
       x->size(-1) != k || x->numel() == 0 || x->device() != ws->device())
@@ -441,7 +447,7 @@ OP(dense_dot) {
   HANDLE_TH_ERRORS
   NARGS(7);
   const at::Tensor *q = plain(args[1]), *sc8 = plain(args[2]), *sc32 = plain(args[3]), *g = plain(args[6]);
-  const int tokens = (int)integer(args[0]), a = (int)integer(args[4]), b = (int)integer(args[5]);
+  const int tokens = small(args[0]), a = small(args[4]), b = small(args[5]);
   if (!q || !sc8 || !sc32 || !g || watched() || q->dim() != 2 || g->dim() != 2 || !dense(g->scalar_type()) || q->scalar_type() != kE4M3 ||
       g->size(tokens ? 0 : 1) != q->size(tokens ? 0 : 1))
     return none();

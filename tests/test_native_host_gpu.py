@@ -124,6 +124,18 @@ def test_a_linear_without_a_graph_gives_the_bits_of_one_with_it(built_lib, both,
         assert all(torch.equal(k, mine) for k in kept) and set(keep) == {"wq", "w_t"}
 
 
+@pytest.mark.parametrize("grid", [(2 ** 32 + 1, 128), (1, 2 ** 32 + 128), (2 ** 64 + 1, 128), (-1, 128), (1, -(2 ** 32) + 128)])
+def test_block_sizes_beyond_an_int_are_refused(built_lib, both, grid):
+    """Block sizes whose low 32 bits are (1, 128) divide no array."""
+    x = torch.randn(8, 1024, device="cuda")
+    triple = _ops.quantize_impl(x, (1, 128))
+    for f in (lambda: _ops.quantize_impl(x, grid), lambda: _ops.quantize_transposed_impl(x.repeat(16, 1), grid[1]) if grid[1] != 128 else ValueError,
+              lambda: _ops.fake_quantize_impl(x, grid, torch.float32), lambda: _ops.fake_quantize_scales_impl(x, grid, torch.float32),
+              lambda: _ops.dequantize_impl(*triple, torch.float32, grid)):
+        mine, text = both(f)
+        assert mine is text and isinstance(mine, type) and issubclass(mine, Exception), (grid, mine, text)
+
+
 @pytest.mark.parametrize("prepared", [False, True])
 def test_a_linear_without_a_graph_prepares_its_weight_once(built_lib, monkeypatch, prepared):
     """The calls that the extension leaves to the Python text, too: one quantization of the weight, and no byte transpose that no product reads."""
