@@ -49,16 +49,22 @@ PyObject* raise_status(int status) {
 
 template <typename F>
 auto without_gil(F&& f) {
-  PyThreadState* state = PyEval_SaveThread();
-  auto r = f();
-  PyEval_RestoreThread(state);
-  return r;
+  struct Released {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Released() { PyEval_RestoreThread(state); }
+  } released;
+  return f();
 }
 
 void* current_stream(c10::Device dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
 
 // ---- the C entries --------------------------------------------------------------------------------------------------
-struct Taken { std::optional<c10::Device> device; Py_buffer buffers[4]; int n_buffers = 0; };
+struct Taken {
+  std::optional<c10::Device> device;
+  Py_buffer buffers[4];
+  int n_buffers = 0;
+  ~Taken() { for (int i = 0; i < n_buffers; ++i) PyBuffer_Release(&buffers[i]); }
+};
 
 bool take(PyObject* o, Taken& t, void** out) {
   if (o == Py_None) { *out = nullptr; return true; }
@@ -114,7 +120,6 @@ struct Entry<Fn> {
         result = PyLong_FromSize_t(r);
       }
     }
-    for (int i = 0; i < t.n_buffers; ++i) PyBuffer_Release(&t.buffers[i]);
     return result;
     END_HANDLE_TH_ERRORS
   }
@@ -424,8 +429,7 @@ OP(linear_step) {
   Taken taken;
   void* bp = nullptr;
   if (!take(args[6], taken, &bp)) return nullptr;
-  const pb_operand b = *static_cast<const pb_operand*>(bp);      // the caller's structure outlives the call; its buffer need not stay locked
-  for (int i = 0; i < taken.n_buffers; ++i) PyBuffer_Release(&taken.buffers[i]);
+  const pb_operand b = *static_cast<const pb_operand*>(bp);
   const c10::cuda::CUDAGuard guard(x->device());
   const int64_t groups = rows * k / 1024;
   at::Tensor q = empty({rows, k}, fmt == PB_E4M3 ? kE4M3 : kE5M2, *x), sc8 = empty({groups, 8}, kE8M0, *x), sc32 = empty({groups, 1, 1}, at::kFloat, *x);

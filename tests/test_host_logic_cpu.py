@@ -50,3 +50,14 @@ def test_unquantized_box_and_qx_lookup():
     assert isinstance(out, QArrayImpl) and out.get_value().tolist() == [0.0, 2.0]
     with pytest.raises(AttributeError):
         qx.definitely_not_a_function
+
+
+def test_the_extension_gives_back_the_buffers_of_a_call_that_raises(built_lib):
+    """A tensor without memory raises in the middle of the arguments; the structure before it must not stay locked."""
+    from pratchya_b200 import _lib
+    structure, sparse = bytearray(16), torch.zeros(4, 4).to_sparse()
+    with pytest.raises(RuntimeError):
+        _lib.native().pb_relu2(structure, 4, sparse, 0)
+    with pytest.raises(TypeError):
+        _lib.native().pb_relu2(structure, "4", None, 0)
+    structure.append(1)                                  # BufferError while an export is held
