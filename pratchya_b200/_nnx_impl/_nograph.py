@@ -14,9 +14,15 @@ class NoContext:
 
 def no_graph() -> bool:
     """Gradients are off, no level of forward-mode differentiation is open, no function transform (vmap, grad, jvp) is
-    running and nothing is being traced: each of these sees an op only through its autograd.Function."""
-    return (not torch.is_grad_enabled() and forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
-            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
+    running and nothing is being traced: each of these sees an op only through its autograd.Function.  Torch has no public
+    names for the first two of them; where its own are gone, the answer is no."""
+    if torch.is_grad_enabled():
+        return False
+    try:
+        return (forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
+                and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
+    except AttributeError:
+        return False
 
 
 def run(function, *args):

@@ -61,3 +61,14 @@ def test_the_extension_gives_back_the_buffers_of_a_call_that_raises(built_lib):
     with pytest.raises(TypeError):
         _lib.native().pb_relu2(structure, "4", None, 0)
     structure.append(1)                                  # BufferError while an export is held
+
+
+@pytest.mark.parametrize("owner,name", [("torch.autograd.forward_ad", "_current_level"), ("torch._C._functorch", "peek_interpreter_stack"), ("torch._C", "_get_tracing_state")])
+def test_without_torchs_own_names_an_op_keeps_its_function(monkeypatch, owner, name):
+    import importlib
+
+    from pratchya_b200._nnx_impl._nograph import no_graph
+    with torch.no_grad():
+        assert no_graph()
+        monkeypatch.delattr(importlib.import_module(owner), name)
+        assert not no_graph()
