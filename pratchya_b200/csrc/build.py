@@ -80,13 +80,27 @@ def build(force: bool = False, verbose: bool = False, diagnostics: bool = False)
     return lib
 
 
+NATIVE_MADE_FOR = HERE / "build" / "native.made_for"
+
+
+def _native_made_for() -> str:
+    """The torch and the Python that native.cc is compiled against: another of either needs another _native.so."""
+    import torch
+    return f"torch {torch.__version__} {torch.version.git_version}, python {sys.version}"
+
+
+def native_stale() -> bool:
+    return (_stale(NATIVE, [HERE / "native.cc", INCLUDE / "pratchya_b200.h"]) or not NATIVE_MADE_FOR.exists()
+            or NATIVE_MADE_FOR.read_text() != _native_made_for())
+
+
 def build_native(force: bool = False, verbose: bool = False) -> Path:
     """Compiles native.cc against torch's headers (the library it calls, libpratchya_b200.so, is found next to it)."""
     import sysconfig
 
     import torch
     src = HERE / "native.cc"
-    if not (force or _stale(NATIVE, [src, INCLUDE / "pratchya_b200.h"])):
+    if not (force or native_stale()):
         return NATIVE
     root = Path(torch.__file__).resolve().parent
     cuda = Path(_nvcc()).resolve().parent.parent
@@ -100,6 +114,8 @@ def build_native(force: bool = False, verbose: bool = False) -> Path:
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"{cmd[0]} failed on native.cc:\n{r.stdout}")
+    NATIVE_MADE_FOR.parent.mkdir(exist_ok=True)
+    NATIVE_MADE_FOR.write_text(_native_made_for())
     return NATIVE
 
 

@@ -72,3 +72,15 @@ def test_without_torchs_own_names_an_op_keeps_its_function(monkeypatch, owner, n
         assert no_graph()
         monkeypatch.delattr(importlib.import_module(owner), name)
         assert not no_graph()
+
+
+def test_the_extension_is_rebuilt_for_another_torch_or_python(built_lib, monkeypatch):
+    import sys
+
+    from pratchya_b200.csrc import build
+    assert not build.native_stale()
+    for owner, name in ((torch, "__version__"), (torch.version, "git_version"), (sys, "version")):
+        with monkeypatch.context() as m:
+            m.setattr(owner, name, "0")
+            assert build.native_stale(), name
+    assert not build.native_stale()
