@@ -485,6 +485,13 @@ bool dot_shape_ok(int tokens, int64_t rows, int64_t cols, int a, int b, int64_t 
 
 }  // namespace
 
+int add_parts(const float* parts, float* out, int64_t n, int splits, cudaStream_t st) {
+  const int64_t n4 = n / 4;
+  add_parts_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4*>(parts), reinterpret_cast<float4*>(out), n4, splits);
+  PB_LAUNCH_CHECK("add_parts_kernel");
+  return PB_OK;
+}
+
 // Reads and clears this file's device status word (see pb_gemm_check).
 int dense_dot_status_fetch(unsigned int* out) {
   const unsigned int zero = 0;
@@ -552,12 +559,7 @@ extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, co
   const int status = tokens ? (g_dtype == PB_F32 ? launch_dot<true, float>(p, grid, st) : launch_dot<true, __nv_bfloat16>(p, grid, st))
                             : (g_dtype == PB_F32 ? launch_dot<false, float>(p, grid, st) : launch_dot<false, __nv_bfloat16>(p, grid, st));
   if (status) return status;
-  if (d.splits > 1) {
-    const int64_t n4 = out_elems / 4;                 // I is a multiple of 128
-    add_parts_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4*>(dst), reinterpret_cast<float4*>(out), n4, d.splits);
-    PB_LAUNCH_CHECK("add_parts_kernel");
-  }
-  return PB_OK;
+  return d.splits > 1 ? add_parts(dst, out, out_elems, d.splits, st) : PB_OK;      // I is a multiple of 128
 }
 
 #ifdef PB_DIAGNOSTICS

@@ -461,17 +461,6 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
   }
 }
 
-__global__ void __launch_bounds__(256) sum_parts_kernel(const float4* parts, float4* out, int64_t n4, int splits) {
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n4) return;
-  float4 s = parts[i];
-  for (int k = 1; k < splits; ++k) {
-    const float4 v = parts[(int64_t)k * n4 + i];
-    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-  }
-  out[i] = s;
-}
-
 // ---- host side ----------------------------------------------------------------------------------------------------
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -638,11 +627,8 @@ int split_dot_run(const SplitDotPlan& d, int tokens, const uint8_t* q, const uin
     const int status = tokens ? (g_bf16 ? launch_n<true, false>(d.n, terms, other, p, st) : launch_n<true, true>(d.n, terms, other, p, st))
                               : (g_bf16 ? launch_n<false, false>(d.n, terms, other, p, st) : launch_n<false, true>(d.n, terms, other, p, st));
     if (status) return status;
-    if (d.splits > 1) {       // there is one round then
-      const int64_t n4 = I * J / 4;
-      sum_parts_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4*>(parts), reinterpret_cast<float4*>(out), n4, d.splits);
-      PB_LAUNCH_CHECK("sum_parts_kernel");
-    }
+    if (d.splits > 1)         // there is one round then
+      if (int s = add_parts(parts, out, I * J, d.splits, st)) return s;
   }
   return PB_OK;
 }

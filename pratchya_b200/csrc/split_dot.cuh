@@ -19,6 +19,8 @@ struct SplitDotPlan {
 bool split_dot_plan(int tokens, int64_t rows, int64_t cols, int a, int b, int64_t g_free, bool g_bf16, SplitDotPlan* d);
 int split_dot_run(const SplitDotPlan& d, int tokens, const uint8_t* q, const uint8_t* sc8, const float* sc32, int64_t rows, int64_t cols, int a, int b,
                   const void* g, bool g_bf16, int64_t g_free, float* out, void* workspace, cudaStream_t st);
+// dense_dot.cu: out = the sum of `splits` parts of n elements (a multiple of 4), in their order
+int add_parts(const float* parts, float* out, int64_t n, int splits, cudaStream_t st);
 int split_dot_status_fetch(unsigned int* out);
 #ifdef PB_DIAGNOSTICS
 void split_dot_control(uint32_t polls, int withhold);
