@@ -1,14 +1,15 @@
-"""The forward scan's forms by head count give the bits of one head's call: a head's sums have one order in all of them."""
+"""The forward scan's forms by head count give the bits of one head's call, in what they leave for the backward pass too: a head's sums
+have one order in all of them."""
 import pytest
 import torch
 
-from pratchya_b200._nnx_impl._wkv7 import wkv_state_scan
+from pratchya_b200._nnx_impl._wkv7 import _forward, wkv_state_scan
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("heads", [18, 19, 37, 38, 74, 75, 148, 149, 185, 186])
-@pytest.mark.parametrize("steps", [1, 7, 8, 9, 16, 26])
+@pytest.mark.parametrize("steps", [1, 7, 8, 9, 11, 12, 13, 14, 16, 26])
 @pytest.mark.parametrize("with_grad", [False, True])
 def test_head_counts_agree(built_lib, heads, steps, with_grad):
     g = torch.Generator(device="cuda").manual_seed(heads + steps)
@@ -18,6 +19,12 @@ def test_head_counts_agree(built_lib, heads, steps, with_grad):
     state = torch.randn(1, heads, 64, 64, generator=g, device="cuda")
     full = [t.clone().requires_grad_(with_grad) for t in ins]
     s_all, y_all = wkv_state_scan(state, *full, heads)
+    if with_grad:
+        _, _, ckpt_all, sa_all = _forward(state, ins, heads, True)
     for h in {0, 1, heads // 2, heads - 1}:
-        s_one, y_one = wkv_state_scan(state[:, h:h + 1].contiguous(), *[t[..., h * 64:(h + 1) * 64].contiguous() for t in ins], 1)
+        one = [t[..., h * 64:(h + 1) * 64].contiguous() for t in ins]
+        s_one, y_one = wkv_state_scan(state[:, h:h + 1].contiguous(), *one, 1)
+        if with_grad:
+            _, _, ckpt_one, sa_one = _forward(state[:, h:h + 1].contiguous(), one, 1, True)
+            assert torch.equal(sa_all[..., h * 64:(h + 1) * 64], sa_one) and torch.equal(ckpt_all.view(heads, -1)[h], ckpt_one)
         assert torch.equal(y_all[..., h * 64:(h + 1) * 64], y_one) and torch.equal(s_all[:, h:h + 1], s_one)
