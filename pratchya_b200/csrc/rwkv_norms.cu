@@ -417,7 +417,8 @@ extern "C" int pb_rms_norm(const float* x, const float* scale, int64_t rows, int
     return fail(PB_ERR_BAD_SHAPE, "pb_rms_norm: rows=%lld channels=%lld (channels must be a multiple of 128)", (long long)rows, (long long)channels);
   if (any_misaligned({x, scale, y})) return fail(PB_ERR_MISALIGNED, "pb_rms_norm: x, scale and y must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (!launch_rms_norm_rows(std::make_integer_sequence<int, kRowQuads>{}, x, scale, y, inv_rms, rows, (int)channels, eps, st))
+  // PB_RMS_LOOP=1 (diagnostics build): the loop over a row for every width
+  if (env_switch("PB_RMS_LOOP", 0) || !launch_rms_norm_rows(std::make_integer_sequence<int, kRowQuads>{}, x, scale, y, inv_rms, rows, (int)channels, eps, st))
     rms_norm_fwd_kernel<<<blocks_for(rows, kWarps), kThreads, 0, st>>>(x, scale, y, inv_rms, rows, (int)channels, eps);
   PB_LAUNCH_CHECK("rms_norm_fwd_kernel");
   return PB_OK;

@@ -17,3 +17,22 @@ def test_rms_norm_rows(built_lib, rows, channels):
     # a lane adds 3 + channels / 128 positive terms and five levels of lanes follow; half of that on the root, and eight more roundings
     bound = (0.5 * (8 + channels / 128) + 8) * 2.0 ** -24
     assert ((got.double() - want).abs() <= bound * want.abs()).all()
+
+
+@pytest.mark.parametrize("channels", [128 * q for q in range(1, 33)])
+def test_both_forms_give_the_same_bits(built_lib, diag_lib, monkeypatch, channels):
+    """The diagnostics build's switch gives every width to the kernel that loops over a row."""
+    rows = 37
+    g = torch.Generator(device="cuda").manual_seed(channels)
+    x = torch.randn(rows, channels, generator=g, device="cuda") * torch.randn(rows, 1, generator=g, device="cuda").exp()
+    scale = torch.randn(channels, generator=g, device="cuda")
+
+    def run(lib):
+        y, inv = torch.empty_like(x), torch.empty(rows, device="cuda")
+        assert lib.pb_rms_norm(x.data_ptr(), scale.data_ptr(), rows, channels, 1e-6, y.data_ptr(), inv.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        return y, inv
+
+    want = run(built_lib)
+    assert all(torch.equal(a, b) for a, b in zip(run(diag_lib), want))
+    monkeypatch.setenv("PB_RMS_LOOP", "1")
+    assert all(torch.equal(a, b) for a, b in zip(run(diag_lib), want))
