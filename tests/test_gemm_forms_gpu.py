@@ -1,5 +1,11 @@
 """The forms of the GEMM that its size chooses between (tiles of 128 x 32, 64, 128 and 224 on one CTA, 256 x 224 on a pair, the
-contraction cut over a cluster of two and four): remainders in every direction against a 64-bit product, and their abort paths."""
+contraction cut over a cluster of two and four): remainders in every direction against a 64-bit product, the same bits from all of
+them, and their abort paths."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -69,6 +75,50 @@ def test_a_workspace_for_more_rows_serves_fewer(built_lib, m, k, n, grid):
         x = torch.randn(m, k, generator=g, device="cuda") * torch.randn(m, 1, generator=g, device="cuda").exp()
         assert torch.equal(run(size, x), want)
     assert built_lib.pb_gemm_check(st) == 0
+
+
+# remainders of 128 and 256 rows, of 32, 64, 128 and 224 columns, of a chunk of eight k-blocks; contractions cut and not, in halves and not
+FORM_SIZES = [(1, 1024, 1024, (128, 128)), (40, 4096, 512, (128, 128)), (127, 2304, 128, (128, 128)), (128, 5120, 384, (128, 128)), (129, 2048, 2048, (128, 128)), (200, 8192, 2048, (128, 128)),
+              (257, 4096, 896, (128, 128)), (500, 1024, 1024, (128, 128)), (1000, 3072, 1152, (128, 128)), (2048, 1024, 640, (128, 128)),
+              (8, 2048, 144, (128, 1)), (64, 640, 48, (128, 1)), (136, 2048, 128, (128, 1)), (300, 1024, 2064, (128, 1)), (1000, 2048, 240, (128, 1)), (2056, 128, 1040, (128, 1))]
+
+
+def _products(lib):
+    out = {}
+    for m, k, n, grid in FORM_SIZES:
+        xq, wq = _triples(m, k, n, grid)
+        wt = _ops.transpose_bytes(wq[0])
+        a, b = _ops._operand(*xq, m, k, (1, 128)), _ops._operand(wt, wq[1], wq[2], n, k, (grid[1], 128), 1)
+        size, st = lib.pb_gemm_workspace_size(a, b), torch.cuda.current_stream().cuda_stream
+        ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+        out[m, k, n, grid, "workspace"] = torch.tensor([size])
+        for dtype, code in ((torch.float32, _lib.PB_F32), (torch.bfloat16, _lib.PB_BF16)):
+            d = torch.full((m, n), float("nan"), dtype=dtype, device="cuda")
+            assert lib.pb_gemm_tn(a, b, d.data_ptr(), code, n, ws.data_ptr(), size, st) == 0, lib.pb_last_error()
+            out[m, k, n, grid, code] = d.cpu()
+        assert lib.pb_gemm_check(st) == 0
+    return out
+
+
+@pytest.mark.parametrize("form", ["32", "64", "128", "224", "pair"])
+def test_every_form_gives_the_same_bits(built_lib, diag_lib, tmp_path, form):
+    """The diagnostics build's switches force one form on every size, in a process of its own (they are read once)."""
+    env = dict(os.environ, PB_GEMM_BN="224" if form == "pair" else form, PB_GEMM_SINGLE="0" if form == "pair" else "1")
+    here = Path(__file__).resolve().parent
+    code = "import sys; sys.path[:0] = sys.argv[2:]\nimport test_gemm_forms_gpu as t, torch\ntorch.save(t._products(t._lib.load_diagnostics()), sys.argv[1])"
+    r = subprocess.run([sys.executable, "-c", code, str(tmp_path / "d.pt"), str(here), str(here.parent)], env=env, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:]
+    forced = torch.load(tmp_path / "d.pt")
+    chosen, compared = _products(built_lib), 0
+    sizes = [key for key in chosen if key[-1] == "workspace"]
+    assert sum(not torch.equal(forced[key], chosen[key]) for key in sizes) >= 5            # the switch is heard: another tile width, another layout
+    for key, want in ((key, d) for key, d in chosen.items() if key not in sizes):
+        # an f32 product of more than 128 rows may be the sum of two halves, which the wide single tiles do not make
+        if form in ("128", "224") and key[0] > 128 and key[-1] == _lib.PB_F32:
+            continue
+        assert torch.equal(forced[key].view(torch.uint8), want.view(torch.uint8)), (form, key)
+        compared += 1
+    assert compared >= 20
 
 
 def test_outputs_with_longer_rows_and_off_the_store_alignment(built_lib):
