@@ -52,7 +52,7 @@ constexpr uint32_t kTmemCols = 512;
 // thread the same whatever the width, so narrow tiles on many CTAs finish first; 32 and 64 columns also allow the contraction to
 // be cut over a cluster whose ranks' sums meet in rank 0's shared memory.  Of the wide ones 224: two 224-column accumulators plus the scale-factor columns fit
 // the 512 TMEM columns (two 256-column ones do not), so the epilogue drains one chunk while the
-// tensor core fills the next, and a 44 KB stage leaves room for five pipeline stages.
+// tensor core fills the next, and a 44 KB stage leaves room for four pipeline stages beside the epilogue's staging.
 template <int BN>
 struct Cfg {
   static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 224 || BN == 256, "tile width");
