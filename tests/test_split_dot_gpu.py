@@ -120,6 +120,11 @@ def test_several_rounds_of_terms(built_lib, tokens, rows, cols, grid, free, dtyp
     assert shared
     a, b = _sums(tokens, triple, grid, g)
     assert ((got.double() - a @ b).abs() <= _bound(a, b) + 1e-37).all()
+    # the sums of one cotangent made again, in the last round too: f32 products, a rounding a term and those of an operand
+    (g[:, -7] if tokens else g[-7]).mul_(1e32)
+    a, b = _sums(tokens, triple, grid, g)
+    got = _dot(built_lib, tokens, triple, grid, g)[0]
+    assert ((got.double() - a @ b).abs() <= (a.abs() @ b.abs()) * 2.0 ** -24 * (a.shape[1] + 4) + 1e-37).all()
 
 
 @pytest.mark.parametrize("dtype", [F32, BF16])
