@@ -40,11 +40,6 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 
 __device__ __forceinline__ float2 dup(float x) { return make_float2(x, x); }
 
-// a lane's eight columns of a shared-memory vector (four at p, four at p + 32) as four float2
-__device__ __forceinline__ void ld8(const float* p, float2 (&out)[4]) {
-  const float4 lo = *reinterpret_cast<const float4*>(p), hi = *reinterpret_cast<const float4*>(p + 32);
-  out[0] = make_float2(lo.x, lo.y); out[1] = make_float2(lo.z, lo.w); out[2] = make_float2(hi.x, hi.y); out[3] = make_float2(hi.z, hi.w);
-}
 // A state in the kernels' own layout (checkpoints in global memory, kept states in shared memory): 1024 quads, a quad the
 // rows 2P, 2P + 1 of the columns 2Q, 2Q + 1 as ((2P, 2Q), (2P+1, 2Q), (2P, 2Q+1), (2P+1, 2Q+1)).  Backward thread
 // 16 * (P >> 2) + (Q >> 1) keeps it as its quad 2 * (P & 3) + (Q & 1): consecutive threads, consecutive 16 bytes.
@@ -52,23 +47,38 @@ __device__ __forceinline__ int ckpt_quad(int P, int Q) { return (2 * (P & 3) + (
 
 // ---- forward ---------------------------------------------------------------------------------------------------
 // The rows of a head's state are independent of one another given the timestep's vectors, so a head's 64 rows are cut over
-// warps, and where there are few heads over CTAs as well.  A warp owns 4 * ROWS rows on the backward pass's 4 x 8 lane grid:
-// a lane keeps ROWS rows x 8 columns, a row's two dot products end in three xor-shuffles (the state's one only delays the
-// warp, the output's one nothing).  No barrier inside a chunk of eight timesteps: the chunk's vectors arrive by cp.async two
-// chunks ahead, a step's are in registers one step ahead, and S * w is formed while sa's shuffles are under way.  v kt^T comes
-// last: added to a state that is about to be erased, its low bits would go with it.
-// What bounds it: with few heads the latency of a timestep (dot product, three shuffles, update: 250 cycles); with many the
-// f32x2 products, three cycles each where their operands are three different registers, and the 4 * (40 + ROWS) bytes per lane
-// and timestep that the vector reads return, which more rows per lane spread over more of them.
-// The order within a timestep keeps everything but that chain off it: sa of the next timestep is formed from the new state before
-// y of this one, the vectors of the next are read behind sa's shuffles (in front of them the shuffles queue behind the reads), y's
-// shuffles come a timestep late and behind the state's update, a lane stores a row's outputs once in 8 / ROWS timesteps, and the
-// next chunk's first vectors are read before this one's last update, so that no chunk starts with an empty pipeline.
-// 1024 timesteps, against y's dot product and the reads in front of sa's and a pipeline emptied every chunk: 16 heads 172 -> 125 us,
-// 32 heads 173 -> 139 (with sa and checkpoints 197 -> 160), 60 heads 188 -> 165, 128 heads 247 -> 214, 256 heads 387 -> 347
-// (474 -> 422) in graphs of repeated calls; 32 heads x 4096, called with L2 flushed in between, 685 -> 571.
+// warps, and where there are few heads over CTAs as well.  A warp's lanes are a grid of 2 x 16 or 4 x 8; a lane keeps ROWS rows x 4
+// or 8 columns, and a row's dot products end in shuffles.
+//
+// The chain.  sa_{t+1} = S_t kap_{t+1} taken as it stands makes every timestep wait for a dot product, its shuffles and the
+// update in turn.  With S_t written out it is
+//     sa_{t+1} = S_{t-1} (w_t o kap_{t+1}) - (b_t . kap_{t+1}) sa_t + (kt_t . kap_{t+1}) v_t         (b = a o kap)
+// whose only sum along the state's rows is over the state a timestep earlier: two timesteps' sums are under way at once, and
+// sa_t enters through two products.  The first timestep of every chunk of eight takes S kap as it stands, so that a scan cut at
+// multiples of eight and continued from its state gives the bits of the whole one.  What the form needs that does not depend on
+// the state (b, w_t o kap_{t+1}, the two scalars) warps of their own make a chunk ahead, once per CTA, from the chunk's vectors as
+// they arrive by cp.async; one barrier per chunk.
+//
+// Sums.  p, the dot product that sa is made of, and y, the output's, are summed together: of two lanes half a row apart one keeps p
+// and hands over its part of y, the other the reverse (each reads its two vectors in that order); a lane's rows are in an order
+// of its own (register a holds row a ^ its lane bits), so that every further halving hands over the upper registers and no value
+// is selected.  A row's p ends on lanes that make sa of it and broadcast that; its y on as many, which store it.  A sum's levels
+// have the same order in every form, so the bits do not depend on the number of heads.
+//
+// The update is (S o w - sa b^T) + v kt^T with the erasure's product rounded and the other two fused: v kt^T comes last (added
+// to a state that is about to be erased, its low bits would go with it), and of the three roundings one is of the erased part's
+// size instead of the state's: 2-norm errors against 64 bits 9.8e-8 -> 9.1e-8 of y, 7.1e-8 -> 6.1e-8 of the state (500 timesteps;
+// keys that repeat or hardly decay: below the step-by-step form's too).
+//
+// What bounds it: with few heads what reads and shuffles return to the registers (146 of a timestep's 205 cycles on an SM of four
+// warps; one row group more per warp or per lane costs more in latency than it saves there), with many the f32x2 products,
+// three cycles each where their operands are three different registers, on top of those reads.  Two CTAs of a whole head an SM: four
+// preparing warps, one a scheduler (one alone made its scheduler the slowest: 128 heads 233 -> 212 us), which hand their registers over.
+// 1024 timesteps, against one timestep after the other with each lane's own b: 16 heads 125 -> 105 us (with saves 160 -> 114), 32 heads 147 -> 106
+// (163 -> 114), 60 heads 165 -> 134 (185 -> 149), 128 heads 221 -> 196 (257 -> 231), 160 heads 329 -> 333 (360 -> 364), 192 heads 358 -> 335
+// (428 -> 367), 256 heads 357 -> 346 (425 -> 395); 32 heads x 4096 572 -> 419.
 constexpr int kFwdChunk = 8;      // timesteps between barriers
-constexpr int kFwdBufs = 3;       // chunks in shared memory
+constexpr int kFwdBufs = 5;       // chunks in shared memory: the one before, the one computed with, the one prepared, two under way
 
 struct WkvParams {
   const float* in[kVecs];
@@ -80,256 +90,398 @@ struct WkvParams {
   int T, N;                       // timesteps, heads
 };
 
-// a lane's share of one timestep's vectors
-template <int ROWS>
-struct StepVecs {
-  float2 w[4], b[4], kap[4], kt[4], r[4];
-  float v[ROWS];
-  __device__ __forceinline__ void load(const float (*buf)[kH], int col0, int row0) {
-    ld8(buf[2] + col0, kap);
-    ld8(buf[0] + col0, w);
-    ld8(buf[3] + col0, kt);
-    ld8(buf[1] + col0, b);
-    ld8(buf[5] + col0, r);
-    if constexpr (ROWS == 4) {
-      const float4 t = *reinterpret_cast<const float4*>(buf[4] + row0);
-      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    } else if constexpr (ROWS == 1) {
-      v[0] = buf[4][row0];
-    } else {
-      const float2 t = *reinterpret_cast<const float2*>(buf[4] + row0);
-      v[0] = t.x; v[1] = t.y;
-    }
-  }
+// the preparing warps and the others arrive from different places
+__device__ __forceinline__ void cta_meet() { asm volatile("bar.sync 0;" ::: "memory"); }
+
+struct WkvFwdChunk {
+  // decay, b (iclr as it arrives), removal_k, replacement_k, v, r, and what the state of timestep s is multiplied with for sa of
+  // timestep s + 2: w_{s+1} o kap_{s+2}.  (The last two hold what the state before the chunk meets: kap_0, w_0 o kap_1.)
+  float vec[kFwdChunk][kVecs + 1][kH];
+  float2 mix[kFwdChunk];                // (b_s . kap_{s+1}, kt_s . kap_{s+1}); the last one is not used
 };
 
-// The sums over the eight lanes of a tile row that a timestep ends with: sa for every lane (the state's update waits for it),
-// y for the lanes that keep it, each lane ending with row own of its ROWS
-template <int ROWS>
-__device__ __forceinline__ void reduce_sa(float (&sa)[ROWS]) {
-#pragma unroll
-  for (int m = 1; m <= 4; m *= 2)
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) sa[a] += __shfl_xor_sync(0xffffffffu, sa[a], m);
-}
-template <int ROWS>
-__device__ __forceinline__ float reduce_y(const float (&y)[ROWS], int tj) {
-  const bool hi = tj & 4, mid = tj & 2;
-  float k0;
-  if constexpr (ROWS == 1) {
-    k0 = y[0] + __shfl_xor_sync(0xffffffffu, y[0], 4);
-    k0 += __shfl_xor_sync(0xffffffffu, k0, 2);
-  } else if constexpr (ROWS == 2) {
-    k0 = (hi ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, hi ? y[0] : y[1], 4);
-    k0 += __shfl_xor_sync(0xffffffffu, k0, 2);
-  } else {
-    const float s0 = hi ? y[0] : y[2], s1 = hi ? y[1] : y[3];
-    k0 = hi ? y[2] : y[0];
-    float k1 = hi ? y[3] : y[1];
-    k0 += __shfl_xor_sync(0xffffffffu, s0, 4);
-    k1 += __shfl_xor_sync(0xffffffffu, s1, 4);
-    k0 = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, 2);
+// a lane's share of one timestep's vectors
+template <int ROWS, int PAIRS>
+struct StepVecs {
+  float2 w[PAIRS], b[PAIRS], kt[PAIRS];
+  float v[ROWS];                  // register 0 is the row whose sums the lane ends with
+  float2 mix;
+};
+// a lane's columns of a shared-memory vector: four, or four and four 32 further on
+template <int PAIRS>
+__device__ __forceinline__ void ld_cols(const float* p, float2 (&out)[PAIRS]) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  out[0] = make_float2(t.x, t.y); out[1] = make_float2(t.z, t.w);
+  if constexpr (PAIRS == 4) {
+    const float4 u = *reinterpret_cast<const float4*>(p + 32);
+    out[2] = make_float2(u.x, u.y); out[3] = make_float2(u.z, u.w);
   }
-  return k0 + __shfl_xor_sync(0xffffffffu, k0, 1);
 }
-template <int ROWS>
-__device__ __forceinline__ float pick_row(const float (&v)[ROWS], int a) {
-  float r = v[0];
-#pragma unroll
-  for (int k = 1; k < ROWS; ++k) r = a == k ? v[k] : r;
-  return r;
-}
-// sum over a lane's columns of S * x, row by row.  Loops over columns outside, rows inside: consecutive products share x.
-template <int ROWS>
-__device__ __forceinline__ void row_dots(const float2 (&S)[ROWS][4], const float2 (&x)[4], float (&out)[ROWS]) {
+
+// sum over a lane's columns of S * x, row by row: four columns' sum, or two of those added as two lanes' are
+template <int ROWS, int PAIRS>
+__device__ __forceinline__ void row_dots(const float2 (&S)[ROWS][PAIRS], const float2 (&x)[PAIRS], float (&out)[ROWS]) {
   float2 p[ROWS], q[ROWS];
 #pragma unroll
   for (int a = 0; a < ROWS; ++a) p[a] = __fmul2_rn(S[a][0], x[0]);
 #pragma unroll
-  for (int a = 0; a < ROWS; ++a) q[a] = __fmul2_rn(S[a][2], x[2]);
-#pragma unroll
   for (int a = 0; a < ROWS; ++a) p[a] = __ffma2_rn(S[a][1], x[1], p[a]);
+  if constexpr (PAIRS == 4) {
 #pragma unroll
-  for (int a = 0; a < ROWS; ++a) q[a] = __ffma2_rn(S[a][3], x[3], q[a]);
+    for (int a = 0; a < ROWS; ++a) q[a] = __fmul2_rn(S[a][2], x[2]);
 #pragma unroll
-  for (int a = 0; a < ROWS; ++a) out[a] = (p[a].x + p[a].y) + (q[a].x + q[a].y);
-}
-
-
-// S_t from S_{t-1} and sa
-template <int ROWS>
-__device__ __forceinline__ void update_state(float2 (&S)[ROWS][4], StepVecs<ROWS>& x, const float (&sa)[ROWS]) {
+    for (int a = 0; a < ROWS; ++a) q[a] = __ffma2_rn(S[a][3], x[3], q[a]);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) x.b[k] = __fmul2_rn(x.b[k], x.kap[k]);
+    for (int a = 0; a < ROWS; ++a) out[a] = (p[a].x + p[a].y) + (q[a].x + q[a].y);
+  } else {
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) S[a][k] = __fmul2_rn(S[a][k], x.w[k]);
-#pragma unroll
-  for (int a = 0; a < ROWS; ++a) {
-    const float2 nsa = dup(-sa[a]);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) S[a][k] = __ffma2_rn(nsa, x.b[k], S[a][k]);
+    for (int a = 0; a < ROWS; ++a) out[a] = p[a].x + p[a].y;
   }
-#pragma unroll
-  for (int a = 0; a < ROWS; ++a)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) S[a][k] = __ffma2_rn(dup(x.v[a]), x.kt[k], S[a][k]);
 }
+template <int V> struct Int { static constexpr int value = V; };
 
-// SAVE: checkpoints and sa are wanted (a backward pass follows).
-template <int ROWS, int WARPS, bool SAVE>
-__global__ void __launch_bounds__(32 * WARPS)
+// A warp's lanes are a grid of 32 / LANES x LANES.  SAVE: checkpoints and sa are wanted (a backward pass follows).  PREP warps prepare the
+// chunks.
+template <int ROWS, int LANES, int WARPS, int PREP, int PER_SM, bool SAVE>
+__global__ void __launch_bounds__(32 * (WARPS + PREP), PER_SM)
 wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
-  constexpr int kFwdThreads = 32 * WARPS;
-  constexpr int kCtaRows = 4 * ROWS * WARPS, kCtasPerHead = kH / kCtaRows;
-  static_assert(kFwdThreads <= 16 * kFwdChunk && kH % kCtaRows == 0, "sixteen threads a timestep of a chunk; a head's rows in whole CTAs");
-  __shared__ __align__(16) float ring[kFwdBufs][kFwdChunk][kVecs][kH];
+  constexpr int kWarpRows = ROWS * (32 / LANES), kCtaRows = kWarpRows * WARPS, kCtasPerHead = kH / kCtaRows;
+  constexpr int kPairs = kH / LANES / 2;        // float2 of a lane's row
+  constexpr int kPrepSteps = kFwdChunk / PREP;
+  constexpr int kSame = LANES / 2 / ROWS;       // lanes that end with the same row's sum
+  constexpr int kSameBits = kSame == 1 ? 0 : (kSame == 2 ? 1 : 2);
+  static_assert(kH % kCtaRows == 0 && kFwdChunk % PREP == 0 && (LANES == 8 || LANES == 16) && (ROWS << kSameBits) * 2 == LANES, "whole CTAs of rows, whole timesteps");
+  extern __shared__ __align__(16) unsigned char wkv_fwd_smem[];
+  WkvFwdChunk* const ring = reinterpret_cast<WkvFwdChunk*>(wkv_fwd_smem);
   const int head = blockIdx.x / kCtasPerHead;
   const int n = head % p.N, b = head / p.N;
   const int C = p.N * kH;
-  const int tid = threadIdx.x, lane = tid & 31, ti = lane >> 3, tj = lane & 7;
-  const int row0 = (blockIdx.x % kCtasPerHead) * kCtaRows + 4 * ROWS * (tid >> 5) + ROWS * ti, col0 = 4 * tj;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t head_base = (size_t)b * p.T * C + (size_t)n * kH;      // element (b, t = 0, channel n*H)
-  const int n_chunks = (p.T + kFwdChunk - 1) / kFwdChunk;
+  const int full = p.T / kFwdChunk, n_chunks = (p.T + kFwdChunk - 1) / kFwdChunk;
 
-  // a chunk is 8 x 6 vectors of 16 quarters of 16 bytes; every thread commits one (possibly empty) group per call
-  auto issue = [&](int chunk) {
-    constexpr int kStepsAtOnce = kFwdThreads / 16;
+  constexpr bool kMoveRegs = WARPS == 4 && PREP == 4 && PER_SM == 2 && ROWS * LANES == 32;      // two CTAs of 256 threads: 128 registers each at launch
+  if (warp >= WARPS) {
+    if constexpr (kMoveRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    // every thread commits one (possibly empty) group per chunk: its warp's timesteps, 6 vectors of 16 quarters of 16 bytes each
+    const int s0 = (warp - WARPS) * kPrepSteps;
+    auto issue = [&](int chunk) {
+      WkvFwdChunk& to = ring[chunk % kFwdBufs];
 #pragma unroll
-    for (int s0 = 0; s0 < kFwdChunk; s0 += kStepsAtOnce) {
-      const int s = s0 + (tid >> 4), t = chunk * kFwdChunk + s;
-      if (t < p.T) {
-        const size_t at = head_base + (size_t)t * C + (tid & 15) * 4;
-#pragma unroll
-        for (int v = 0; v < kVecs; ++v)
-          cp_async16((uint32_t)__cvta_generic_to_shared(&ring[chunk % kFwdBufs][s][v][(tid & 15) * 4]), p.in[v] + at);
+      for (int i = 0; i < kPrepSteps * 3; ++i) {
+        const int s = s0 + i / 3, v = 2 * (i % 3) + (lane >> 4), t = chunk * kFwdChunk + s;
+        if (t < p.T) {
+          const float* src = i % 3 == 0 ? (lane < 16 ? p.in[0] : p.in[1]) : (i % 3 == 1 ? (lane < 16 ? p.in[2] : p.in[3]) : (lane < 16 ? p.in[4] : p.in[5]));
+          cp_async16((uint32_t)__cvta_generic_to_shared(&to.vec[s][v][(lane & 15) * 4]), src + head_base + (size_t)t * C + (lane & 15) * 4);
+        }
       }
+      cp_async_commit();
+    };
+    // what a chunk's timesteps need beside its vectors; a lane two columns.  (Timesteps past the sequence's end: what the buffer
+    // holds, which nothing reads.)
+    auto prepare = [&](int chunk) {
+      WkvFwdChunk& at = ring[chunk % kFwdBufs];
+      const int j = 2 * lane;
+      float dots[2 * kPrepSteps];
+      float2 kap = *reinterpret_cast<const float2*>(&at.vec[s0][2][j]);
+      if (s0 == 0) *reinterpret_cast<float2*>(&at.vec[kFwdChunk - 2][kVecs][j]) = kap;
+#pragma unroll
+      for (int i = 0; i < kPrepSteps; ++i) {
+        const int s = s0 + i;
+        const float2 w = *reinterpret_cast<const float2*>(&at.vec[s][0][j]), a = *reinterpret_cast<const float2*>(&at.vec[s][1][j]);
+        const float2 kt = *reinterpret_cast<const float2*>(&at.vec[s][3][j]);
+        const float2 bb = make_float2(a.x * kap.x, a.y * kap.y);
+        *reinterpret_cast<float2*>(&at.vec[s][1][j]) = bb;
+        const bool more = s + 1 < kFwdChunk;
+        const float2 nxt = *reinterpret_cast<const float2*>(&at.vec[more ? s + 1 : s][2][j]);
+        if (more) *reinterpret_cast<float2*>(&at.vec[(s + kFwdChunk - 1) % kFwdChunk][kVecs][j]) = make_float2(w.x * nxt.x, w.y * nxt.y);
+        dots[2 * i] = __fmaf_rn(bb.y, nxt.y, bb.x * nxt.x);
+        dots[2 * i + 1] = __fmaf_rn(kt.y, nxt.y, kt.x * nxt.x);
+        kap = nxt;
+      }
+      // 2 * kPrepSteps sums over the warp, over lane bits 4, 3, 2, 1, 0 in turn whatever their number
+      int nv = 2 * kPrepSteps, index = 0;
+#pragma unroll
+      for (int m = 16; m >= 1; m /= 2) {
+        if (nv > 1) {
+          nv /= 2;
+          const bool hi = lane & m;
+#pragma unroll
+          for (int q = 0; q < kPrepSteps; ++q)
+            if (q < nv) {
+              const float keep = hi ? dots[q + nv] : dots[q], send = hi ? dots[q] : dots[q + nv];
+              dots[q] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+            }
+          index += hi ? nv : 0;
+        } else {
+          dots[0] += __shfl_xor_sync(0xffffffffu, dots[0], m);
+        }
+      }
+      reinterpret_cast<float*>(&at.mix[s0])[index] = dots[0];      // lanes with the same index hold the same sum
+    };
+    auto producers_meet = [] {
+      if constexpr (PREP == 1) __syncwarp();
+      else asm volatile("bar.sync 1, %0;" ::"n"(32 * PREP) : "memory");
+    };
+#pragma unroll
+    for (int c = 0; c < kFwdBufs - 1; ++c) issue(c);
+    cp_async_wait<kFwdBufs - 2>();
+    producers_meet();
+    prepare(0);
+    cta_meet();
+    for (int c = 0; c < full; ++c) {
+      cp_async_wait<kFwdBufs - 3>();
+      producers_meet();                         // everyone's vectors of chunk c + 1
+      if (c + 1 < n_chunks) prepare(c + 1);
+      cta_meet();                               // chunk c + 1 is ready, chunk c - 1 has been read
+      issue(c + kFwdBufs - 1);
     }
-    cp_async_commit();
-  };
+    cp_async_wait<0>();
+    return;
+  }
 
-  float2 S[ROWS][4];
+  if constexpr (kMoveRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");      // 128 * (56 + 200) = 256 * 128
+  const int tj = lane & (LANES - 1), own_row = (tj & (LANES / 2 - 1)) >> kSameBits, part = tj & (kSame - 1);
+  const bool for_y = tj & (LANES / 2);
+  const int row0 = (blockIdx.x % kCtasPerHead) * kCtaRows + kWarpRows * warp + ROWS * (lane / LANES), col0 = 4 * tj;
+  float2 S[ROWS][kPairs];
   const size_t shead = (size_t)head * kH * kH;
 #pragma unroll
   for (int a = 0; a < ROWS; ++a) {
     if (p.state_in) {
-      const float4 lo = __ldg(reinterpret_cast<const float4*>(p.state_in + shead + (row0 + a) * kH + col0));
-      const float4 hi = __ldg(reinterpret_cast<const float4*>(p.state_in + shead + (row0 + a) * kH + col0 + 32));
-      S[a][0] = make_float2(lo.x, lo.y); S[a][1] = make_float2(lo.z, lo.w); S[a][2] = make_float2(hi.x, hi.y); S[a][3] = make_float2(hi.z, hi.w);
+#pragma unroll
+      for (int k = 0; k < kPairs; k += 2) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p.state_in + shead + (row0 + (a ^ own_row)) * kH + col0 + 16 * k));
+        S[a][k] = make_float2(t.x, t.y); S[a][k + 1] = make_float2(t.z, t.w);
+      }
     } else {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) S[a][k] = make_float2(0.0f, 0.0f);
+      for (int k = 0; k < kPairs; ++k) S[a][k] = make_float2(0.0f, 0.0f);
     }
   }
-  // four rows a lane: of the two lanes that end up with a row's y one stores it, and its neighbour sa, both a timestep late
-  constexpr int kSame = 8 / ROWS;              // lanes with the same row
-  const int own = tj / kSame, part = tj % kSame;
-  float* const out = part == 0 ? p.y : (SAVE && part == 1 ? p.sa : nullptr);
-  float* dst = out ? out + head_base + row0 + own : nullptr;
-  float y[ROWS], sa[ROWS], sa_before = 0.0f, y_keep = 0.0f, sa_keep = 0.0f;
-  constexpr bool kKeep = ROWS < 4;     // eight timesteps' stores of a lane become ROWS (two arrays: no fewer with four rows)
-  // with kKeep: a row's kSame lanes keep one timestep each of kSame and store together
-  float* const yp = p.y + head_base + row0 + own;
-  float* const sp = SAVE && p.sa ? p.sa + head_base + row0 + own : nullptr;
+  // A row's kSame lanes keep one timestep each of kSame and store together: y, and with a backward pass to follow sa
+  const bool stores = for_y || (SAVE && p.sa);
+  const long out_step = (long)kSame * C;
+  float* out = (SAVE && stores && !for_y ? p.sa : p.y) + head_base + row0 + own_row + (long)part * C;      // of the next kSame timesteps the one that this lane keeps
+  float keep = 0.0f;
+  int from[ROWS];                               // the lane that makes sa of register a's row
 #pragma unroll
-  for (int a = 0; a < ROWS; ++a) y[a] = 0.0f;
+  for (int a = 0; a < ROWS; ++a) from[a] = (lane & ~(LANES - 1)) | ((tj & (LANES / 2 - 1)) ^ (a << kSameBits));
 
-  issue(0);
-  issue(1);
-  issue(2);
-  cp_async_wait<2>();
-  __syncthreads();
-  StepVecs<ROWS> cur;
-  cur.load(ring[0][0], col0, row0);
-  row_dots<ROWS>(S, cur.kap, sa);
-  for (int c = 0; c < n_chunks; ++c) {
-    const float (*buf)[kVecs][kH] = ring[c % kFwdBufs];
-    const float (*buf_next)[kVecs][kH] = ring[(c + 1) % kFwdBufs];
-    if constexpr (SAVE && ROWS > 1) {
-      if (p.ckpt) {                   // the state before the chunk (kCk == kFwdChunk), in the backward kernel's layout
+  using Vecs = StepVecs<ROWS, kPairs>;
+  auto load = [&](Vecs& x, const WkvFwdChunk& at, int s) {
+    ld_cols(at.vec[s][0] + col0, x.w); ld_cols(at.vec[s][1] + col0, x.b); ld_cols(at.vec[s][3] + col0, x.kt);
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) x.v[a] = at.vec[s][4][row0 + (a ^ own_row)];
+    x.mix = at.mix[s];
+  };
+  // Parts of the sums that a state takes part in, not yet summed over lanes: pa the lane's kept one (p or y), pb the other,
+  // pc the second p of a chunk's first state.  half: the sums of the state before, but for their last level.
+  float pa[ROWS], pb[ROWS], pc[ROWS], half[1];
+  const int first_at = (for_y ? kVecs - 1 : kVecs) * kH + col0, second_at = (for_y ? kVecs : kVecs - 1) * kH + col0;
+  auto both_dots = [&](const float* x, const float* y) {
+    float2 x1[kPairs], x2[kPairs];
+    ld_cols(x, x1);
+    ld_cols(y, x2);
+    row_dots(S, x2, pb);
+    row_dots(S, x1, pa);
+  };
+  auto one_dot = [&](const float* x, float (&to)[ROWS]) {
+    float2 v[kPairs];
+    ld_cols(x + col0, v);
+    row_dots(S, v, to);
+  };
+  // The levels of a row's sum over lanes: with N registers left, the upper half of them goes to the lane that keeps those rows;
+  // with one, it is added.  A level is asked for and, when other work has passed, added.
+  float got[ROWS];
+  auto ask = [&](const float (&k)[ROWS], auto bit, auto regs) {
+    constexpr int M = decltype(bit)::value, N = decltype(regs)::value;
+    if constexpr (N > 1) {
+#pragma unroll
+      for (int a = 0; a < N / 2; ++a) got[a] = __shfl_xor_sync(0xffffffffu, k[a + N / 2], M);
+    } else {
+      got[0] = __shfl_xor_sync(0xffffffffu, k[0], M);
+    }
+  };
+  auto add = [&](float (&k)[ROWS], auto regs) {
+    constexpr int N = decltype(regs)::value;
+#pragma unroll
+    for (int a = 0; a < (N > 1 ? N / 2 : 1); ++a) k[a] += got[a];
+  };
+  constexpr Int<ROWS> n2;
+  constexpr Int<ROWS / 2> n3;                   // sixteen lanes have one more level
+  constexpr Int<LANES == 16 ? (ROWS == 8 ? 2 : 1) : (ROWS == 4 ? 2 : 1)> n4;
+  constexpr Int<LANES / 4> m2;
+  constexpr Int<2> m3;
+  constexpr Int<1> m4;
+  auto first_level = [&](const float (&from_other)[ROWS]) {
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) got[a] = __shfl_xor_sync(0xffffffffu, from_other[a], LANES / 2);
+  };
+  auto add_first = [&](float (&k)[ROWS]) {
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) k[a] += got[a];
+  };
+  auto other_levels = [&](float (&k)[ROWS]) {   // with nothing in between
+    ask(k, m2, n2); add(k, n2);
+    if constexpr (LANES == 16) { ask(k, m3, n3); add(k, n3); }
+    ask(k, m4, n4); add(k, n4);
+    return k[0];
+  };
+
+  float nsa[ROWS];                              // -sa of the timestep, of the lane's rows
+  float own = 0.0f, own_before = 0.0f;          // of the row whose sums the lane ends with: the timestep's, the one's before
+  float y_held = 0.0f, v_before = 0.0f;
+  float2 mix_before = make_float2(0.0f, 0.0f);
+  auto put = [&](int u, float val) {            // val: of a timestep, u = t % kSame
+    if (part == u) keep = val;
+    if (u == kSame - 1) {
+      if (stores) *out = keep;
+      out += out_step;
+    }
+  };
+  Vecs cur, next;
+  float last_got[2];                            // the last level of the sum that makes the next timestep's sa, asked for
+  auto ask_last = [&](const float (&k)[ROWS]) {
+    half[0] = k[0];
+    last_got[0] = __shfl_xor_sync(0xffffffffu, k[decltype(n4)::value / 2], 1);
+  };
+  // Timestep s of chunk c.  Two sums over lanes are under way: the one over the state before the last, whose last level makes this
+  // timestep's sa (and y of two timesteps ago), and the one over the last state, whose levels are asked for between the products
+  // of the update, which wait for sa.
+  auto step = [&](int c, int s, auto is_first) {
+    constexpr bool first = decltype(is_first)::value;       // s == 0
+    const WkvFwdChunk& at = ring[c % kFwdBufs];
+    const WkvFwdChunk& after = ring[(c + 1) % kFwdBufs];
+    const float* const rec = &at.vec[0][0][0] + s * (kVecs + 1) * kH;
+    float y_done = half[0] + last_got[0];       // y of two timesteps ago, on the lanes that store it
+    const float sa_done = -own_before;
+    own_before = own;
+    if constexpr (first) {
+      first_level(pb);
+      add_first(pa);
+      first_level(pc);
+      add_first(pc);
+      y_held = other_levels(pa);
+      own = -y_held;                            // the lanes that do not store y: sa as it stands
+    } else {
+      const float x = y_done;
+      if (s == 1) y_done = y_held;
+      own = __fmaf_rn(-v_before, mix_before.y, __fmaf_rn(-own_before, mix_before.x, -x));
+    }
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) nsa[a] = __shfl_sync(0xffffffffu, own, from[a]);
+    float (&k)[ROWS] = first ? pc : pa;
+    if constexpr (!first) {
+      if (s + 1 == kFwdChunk) first_level(pa);
+      else first_level(pb);
+    }
+    if (s + 1 == kFwdChunk) {
+      cta_meet();
+      load(next, after, 0);
+    } else {
+      load(next, at, s + 1);
+    }
+    if (s > 1 || c > 0) put((s + kFwdChunk - 2) % kSame, SAVE && !for_y ? sa_done : y_done);
+    if constexpr (!first) add_first(k);
+    ask(k, m2, n2);
+    float2 m[ROWS][kPairs];
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a)
+#pragma unroll
+      for (int j = 0; j < kPairs; ++j) m[a][j] = __fmul2_rn(dup(nsa[a]), cur.b[j]);
+#pragma unroll
+    for (int j = 0; j < kPairs; ++j)
+#pragma unroll
+      for (int a = 0; a < ROWS; ++a) S[a][j] = __ffma2_rn(S[a][j], cur.w[j], m[a][j]);
+    add(k, n2);
+    if constexpr (LANES == 16) ask(k, m3, n3);
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a)
+#pragma unroll
+      for (int j = 0; j < kPairs; ++j) S[a][j] = __ffma2_rn(dup(cur.v[a]), cur.kt[j], S[a][j]);
+    if constexpr (LANES == 16) add(k, n3);
+    ask_last(k);
+    if (s + 2 < kFwdChunk) {
+      both_dots(rec + first_at, rec + second_at);
+    } else if (s + 2 == kFwdChunk) {
+      one_dot(at.vec[s][kVecs - 1], pa);
+    } else {
+      const float *kap = after.vec[kFwdChunk - 2][kVecs] + col0, *r = at.vec[s][kVecs - 1] + col0;
+      both_dots(for_y ? r : kap, for_y ? kap : r);
+      one_dot(after.vec[kFwdChunk - 1][kVecs], pc);
+    }
+    v_before = cur.v[0];
+    mix_before = cur.mix;
+    cur = next;
+  };
+  auto checkpoint = [&](int c) {                // the state before the chunk (kCk == kFwdChunk), in the backward kernel's layout
+    if constexpr (SAVE) {
+      if (p.ckpt) {
         float4* ck = p.ckpt + ((size_t)head * n_chunks + c) * kTileQuads;
 #pragma unroll
         for (int a = 0; a < ROWS; a += 2)
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            ck[ckpt_quad((row0 + a) >> 1, (col0 >> 1) + (k & 1) + 16 * (k >> 1))] = make_float4(S[a][k].x, S[a + 1][k].x, S[a][k].y, S[a + 1][k].y);
+          for (int k = 0; k < kPairs; ++k) {
+            const float2 e = own_row & 1 ? S[a + 1][k] : S[a][k], o = own_row & 1 ? S[a][k] : S[a + 1][k];
+            ck[ckpt_quad((row0 + (a ^ own_row)) >> 1, (col0 >> 1) + (k & 1) + 16 * (k >> 1))] = make_float4(e.x, o.x, e.y, o.y);
+          }
       }
     }
-    const int steps = min(kFwdChunk, p.T - c * kFwdChunk);
+  };
+
+  cta_meet();
+  load(cur, ring[0], 0);
+  half[0] = last_got[0] = 0.0f;                       // y of no timestep, here and in the next
+  one_dot(ring[0].vec[kFwdChunk - 2][kVecs], pa);
 #pragma unroll
-    for (int s = 0; s < kFwdChunk; ++s) {
-      if (s >= steps) break;
-      StepVecs<ROWS> next;
-      const bool last_step = s + 1 == kFwdChunk;
-      if (last_step) {
-        cp_async_wait<1>();
-        __syncthreads();
-      }
-      const float (*from)[kH] = last_step ? buf_next[0] : buf[(s + 1) % kFwdChunk];
-      if (last_step) issue(c + 3);
-      reduce_sa<ROWS>(sa);
-      next.load(from, col0, row0);
-      float y_old[ROWS];
+  for (int a = 0; a < ROWS; ++a) pb[a] = pa[a];
+  one_dot(ring[0].vec[kFwdChunk - 1][kVecs], pc);
+  for (int c = 0; c < full; ++c) {
+    checkpoint(c);
+    step(c, 0, Int<1>());
 #pragma unroll
-      for (int a = 0; a < ROWS; ++a) y_old[a] = y[a];
-      update_state<ROWS>(S, cur, sa);
-      float sa_next[ROWS];
-      row_dots<ROWS>(S, next.kap, sa_next);
-      row_dots<ROWS>(S, cur.r, y);
-      const float y_before = reduce_y<ROWS>(y_old, tj);
-      if constexpr (kKeep) {
-        constexpr int kLast = kSame - 1;
-        const int u = (s + kFwdChunk - 1) % kSame;           // of timestep c * 8 + s - 1
-        if (part == u) { y_keep = y_before; if (SAVE) sa_keep = sa_before; }
-        if (u == kLast && (s > 0 || c > 0)) {
-          const long at = (long)(c * kFwdChunk + s - kSame + part) * C;
-          yp[at] = y_keep;
-          if (SAVE) if (sp) sp[at] = sa_keep;
-        }
-      } else if (dst && (s > 0 || c > 0)) {
-        *dst = SAVE && part != 0 ? sa_before : y_before;
-        dst += C;
-      }
-      if (SAVE) sa_before = pick_row<ROWS>(sa, own);
-      cur = next;
-#pragma unroll
-      for (int a = 0; a < ROWS; ++a) sa[a] = sa_next[a];
-    }
+    for (int s = 1; s < kFwdChunk; ++s) step(c, s, Int<0>());
   }
-  const float y_last = reduce_y<ROWS>(y, tj);
-  if constexpr (kKeep) {
-    const int last = (p.T - 1) % kSame;
-    if (part == last) { y_keep = y_last; if (SAVE) sa_keep = sa_before; }
-    if (part <= last) {
-      const long at = (long)(p.T - 1 - last + part) * C;
-      yp[at] = y_keep;
-      if (SAVE) if (sp) sp[at] = sa_keep;
-    }
-  } else if (dst) *dst = SAVE && part != 0 ? sa_before : y_last;
-  cp_async_wait<0>();
+  const int tail = p.T - full * kFwdChunk;
+  if (tail) {
+    checkpoint(full);
+    step(full, 0, Int<1>());
+#pragma unroll 1
+    for (int s = 1; s < tail; ++s) step(full, s, Int<0>());
+  }
+  // the last two timesteps' outputs are still open
+  const int t = p.T - 1, s_last = t % kFwdChunk, u = t % kSame;
+  if (t > 0) {
+    put((t - 1) % kSame, SAVE && !for_y ? -own_before : (s_last == 0 ? y_held : half[0] + last_got[0]));
+  }
+  if (s_last + 2 == kFwdChunk) first_level(pa);
+  else first_level(pb);
+  add_first(pa);
+  const float y_last = other_levels(pa);
+  if (part == u) keep = SAVE && !for_y ? -own : y_last;
+  if (part <= u && stores) *out = keep;
   if (p.state_out) {
 #pragma unroll
-    for (int a = 0; a < ROWS; ++a) {
-      *reinterpret_cast<float4*>(p.state_out + shead + (row0 + a) * kH + col0) = make_float4(S[a][0].x, S[a][0].y, S[a][1].x, S[a][1].y);
-      *reinterpret_cast<float4*>(p.state_out + shead + (row0 + a) * kH + col0 + 32) = make_float4(S[a][2].x, S[a][2].y, S[a][3].x, S[a][3].y);
-    }
+    for (int a = 0; a < ROWS; ++a)
+#pragma unroll
+      for (int k = 0; k < kPairs; k += 2)
+        *reinterpret_cast<float4*>(p.state_out + shead + (row0 + (a ^ own_row)) * kH + col0 + 16 * k) = make_float4(S[a][k].x, S[a][k].y, S[a][k + 1].x, S[a][k + 1].y);
   }
 }
 
-template <int ROWS, int WARPS>
+template <int ROWS, int LANES, int WARPS, int PREP, int PER_SM>
 int launch_forward(const WkvParams& p, int64_t heads, cudaStream_t st) {
-  const unsigned grid = (unsigned)(heads * (kH / (4 * ROWS * WARPS)));
-  if constexpr (ROWS > 1) {       // a lane of one row has no row pair to put into a checkpoint
-    if (p.ckpt || p.sa) {
-      wkv7_forward_kernel<ROWS, WARPS, true><<<grid, 32 * WARPS, 0, st>>>(p);
-      PB_LAUNCH_CHECK("wkv7_forward_kernel");
-      return PB_OK;
-    }
-  }
-  wkv7_forward_kernel<ROWS, WARPS, false><<<grid, 32 * WARPS, 0, st>>>(p);
-  PB_LAUNCH_CHECK("wkv7_forward_kernel");
-  return PB_OK;
+  const unsigned grid = (unsigned)(heads * (kH / (ROWS * (32 / LANES) * WARPS)));
+  const int smem = kFwdBufs * (int)sizeof(WkvFwdChunk);
+  auto go = [&](auto kernel) {
+    PB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));   // per device
+    kernel<<<grid, 32 * (WARPS + PREP), smem, st>>>(p);
+    PB_LAUNCH_CHECK("wkv7_forward_kernel");
+    return (int)PB_OK;
+  };
+  if (p.ckpt || p.sa) return go(wkv7_forward_kernel<ROWS, LANES, WARPS, PREP, PER_SM, true>);
+  return go(wkv7_forward_kernel<ROWS, LANES, WARPS, PREP, PER_SM, false>);
 }
 
 // ---- backward of the scan ------------------------------------------------------------------------------------
@@ -462,7 +614,7 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
     }
     cp_async_commit();
   };
-  // to = from * w - sa b^T + v kt^T on the tile
+  // to = from * w - sa b^T + v kt^T on the tile, rounded as the forward pass rounds it
   auto update = [&](const float (*buf)[kH], const BwdTile& from, BwdTile& to) {
     const float4 w4 = *reinterpret_cast<const float4*>(buf[0] + col0), a4 = *reinterpret_cast<const float4*>(buf[1] + col0);
     const float4 k4 = *reinterpret_cast<const float4*>(buf[2] + col0), t4 = *reinterpret_cast<const float4*>(buf[3] + col0);
@@ -473,11 +625,7 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-      for (int rp = 0; rp < 4; ++rp) to[rp][c] = __fmul2_rn(from[rp][c], w[c]);
-#pragma unroll
-    for (int rp = 0; rp < 4; ++rp)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) to[rp][c] = __ffma2_rn(sa[rp], nb[c], to[rp][c]);
+      for (int rp = 0; rp < 4; ++rp) to[rp][c] = __ffma2_rn(from[rp][c], w[c], __fmul2_rn(sa[rp], nb[c]));
 #pragma unroll
     for (int rp = 0; rp < 4; ++rp)
 #pragma unroll
@@ -707,15 +855,15 @@ extern "C" int pb_wkv7_forward(const float* decay, const float* iclr, const floa
     if (reinterpret_cast<uintptr_t>(ptr) & 15) return fail(PB_ERR_MISALIGNED, "pb_wkv7_forward: every array must be 16-byte aligned");
   WkvParams p{{decay, iclr, removal_k, replacement_k, v, r}, state_in, y, state_out, reinterpret_cast<float4*>(checkpoints), sa, (int)steps, (int)heads};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // 8 (one row a lane: no pair of rows for a checkpoint), 16, 32 or 64 rows of a head per CTA: as many CTAs as there are SMs, and no
-  // more of them on one (each reads the head's vectors); 16 heads x 1024: 125 us with 8 rows, 139 with 16
   const int64_t n = batch * heads;
-  if (8 * n <= sm_count() && !checkpoints && !sa) return launch_forward<1, 2>(p, n, st);
-  if (4 * n <= sm_count()) return launch_forward<2, 2>(p, n, st);
-  if (2 * n <= sm_count()) return launch_forward<2, 4>(p, n, st);
-  // just over a wave of whole heads: quarters of them fill SMs more evenly (160 heads x 1024: 326 us for 350, with saves 358 for 425)
-  if (n > sm_count() && 4 * n <= 5 * sm_count()) return launch_forward<2, 2>(p, n, st);
-  return launch_forward<4, 4>(p, n, st);
+  // Rows of a head per CTA: 16, 32 or 64, as many CTAs as there are SMs and no more of them on one (each reads the head's vectors);
+  // from a wave of whole heads to one and a half, three halves on an SM instead of two heads.  1024 timesteps, us, of the forms 16 |
+  // 32 | halves | 64: 32 heads 106 | 133 | 171 | 195, 74 heads 171 | 134 | 173 | 196, 96 heads 268 | 218 | 305 | 196, 160 heads 431 | 334 |
+  // 333 | 348 (with saves 466 | 437 | 364 | 397), 222 heads 501 | 334 | 335 | 347 (544 | 438 | 367 | 395), 256 heads 595 | 426 | 432 | 346.
+  if (4 * n <= sm_count()) return launch_forward<2, 16, 4, 4, 1>(p, n, st);
+  if (2 * n <= sm_count()) return launch_forward<4, 16, 4, 4, 1>(p, n, st);
+  if (n > sm_count() && 2 * n <= 3 * sm_count()) return launch_forward<4, 8, 2, 2, 3>(p, n, st);
+  return launch_forward<4, 8, 4, 4, 2>(p, n, st);
 }
 
 extern "C" size_t pb_wkv7_checkpoint_floats(int64_t batch, int64_t steps, int64_t heads, int head_dim) {
