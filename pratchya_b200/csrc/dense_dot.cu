@@ -19,19 +19,19 @@
 // their infinities and NaNs are then an f32 dot's).  The look at the sums is free, behind their stores; ranges kept by
 // the converting warps instead cost 5 % (3000 tokens, 2048 x 2048, f32: dW 173 -> 182 us).
 //
-// A CTA makes a 128 x 128 tile of out: eight warps convert (global loads into registers, scale, split, 128-byte
-// swizzled K-major tiles in shared memory; where i and j are the contiguous dimensions the eight c of a 16-byte chunk come from
-// eight rows, so the transpose is in the loads), eight warps empty one pair of accumulators
-// while the other fills, and one lane of theirs issues tcgen05.mma.  Where the tiles do not fill the SMs the contraction is
-// cut, and the parts are added in order by a second kernel.
+// A CTA makes 128 x 128 tiles of out, one after the other: eight warps convert (global loads into registers, scale, split, 128-byte
+// swizzled tiles in shared memory: K-major for dX, with c outermost, as the operands lie in memory, for dW), four warps empty one pair of
+// accumulators while the other fills, and a lane of a warp of its own issues tcgen05.mma: as a lane of an emptying warp it was what
+// a stage waited for (1200 cycles to issue a stage's twelve, 700 to empty one). A finished tile leaves by bulk copies from shared
+// memory.  Where the tiles do not fill the SMs the contraction is cut, and the parts are added in order by a second kernel.
 //
-// What bounds it: no one part.  A stage of dX takes 2800 cycles (of dW 3500), of which the tensor core works 768; before the loads moved behind the
-// fence, dX took 17 % less with the split left out, 14 with the loads, 13 with the emptying, 8 with eleven of the twelve
-// products (dW: 28, 40, 11, 5), and sixteen converting warps were no faster than eight.  Against dequantizing and the library's
-// SGEMM (inside a CUDA graph): 3000 tokens, 2048 x 2048, dX 491 -> 143 us, dW 432 -> 175 (bf16 g, read as it is: 507 -> 142 and
-// 448 -> 179); 8192 tokens, 2048 x 128, 100 -> 62 and 139 -> 37; 64 tokens, 1024 x 1024, 22 -> 14 and 9 -> 8.5.  Where there is less
-// than that to do the library's kernels are shorter (64 tokens, 2048 x 128, 8 | 10 and 7 | 8), but a call of it is not: one after
-// the other the two dots take 48 us there and these 24, for the host's part of four library calls.
+// What bounds it: shared memory's data path.  A stage takes 2400 cycles, of which the converting warps' stores, loads and shuffles hold
+// it for 1000 and the tensor core's reads of both operands (three terms against the same fp8 tile) for 770; their shuffles
+// queue behind the stores.  Prefetching g into L2 gained 2 us where g streams from HBM and lost one where it does not; two stages' loads
+// under way, other orders of the conversions: nothing.  Against the first form (emptying warps that issued, stores of a tile from
+// registers, whose instructions had to be fetched for one use: 15000 cycles of a 58000-cycle CTA), us in a CUDA graph: 8192 tokens, f32, 2048 x 128
+// dX 62 -> 31, dW 40 -> 30, 128 x 2048 38 -> 35 and 41 -> 31; 704 tokens, 128 x 1024 15.0 -> 12.0, 19.0 -> 13.4; 64 tokens, 2048 x 128 9.6 -> 7.6, 8.5 -> 7.0;
+// the same bits.
 //
 // Every tile converts what it reads, so an operand that many tiles share is converted many times: where 512 columns or more share
 // it and there is enough to do, split_dot.cu makes it ready once (split_dot_pays: 3000 tokens, 2048 x 2048, bf16 cotangent, dX 141 -> 75 us,
@@ -48,13 +48,14 @@ namespace {
 
 constexpr int kTile = 128;            // i and j per CTA
 constexpr int kDepth = 64;            // c per stage; an accumulator takes 32 of them
-constexpr int kStages = 3;
+constexpr int kStages = 2;
 constexpr int kMinSplitDepth = 256;   // c per part: below this a part is mostly prologue
-constexpr int kConvWarps = 8, kDrainWarps = 8;
-constexpr int kDotThreads = 32 * (kConvWarps + kDrainWarps);       // 128 registers each: a seventeenth warp for the MMAs leaves 96, and spills
+constexpr int kConvWarps = 8, kDrainWarps = 4, kIssueWarp = kConvWarps + kDrainWarps;
+constexpr int kDotThreads = 512;      // 128 registers each at launch; the emptying warpgroup takes 216, the issuing one's three other warps have nothing to do
 constexpr int kOpBytes = kTile * kDepth * 2;            // one bf16 operand tile: 128 rows of 128 bytes
 constexpr int kStageBytes = 4 * kOpBytes;               // q, then f's lo, mid and hi
-constexpr int kDotSmem = kStages * kStageBytes + 1024 + 128;      // 1024: the tiles start on a swizzle atom
+constexpr int kOutPitch = 4 * kTile + 16;                // bytes of a finished tile's row in shared memory
+constexpr int kDotSmem = kStages * kStageBytes + kTile * kOutPitch + 1024;      // 1024: the tiles start on a swizzle atom
 constexpr uint32_t kAccCols = 4 * kTile;                // tensor memory: two stages of two accumulators, each of half a stage's c
 constexpr float kScaleUp = 0x1p40f, kScaleDown = 0x1p-40f;      // of f, and of its sums (see above)
 constexpr uint32_t kWaitPolls = 1u << 21;               // a poll parks for up to 2 us: about four seconds at most
@@ -69,7 +70,7 @@ struct DotParams {
   int I, J, C;                        // extents: i and j of out, and the contraction
   uint32_t nbc, log2_K;               // blocks per block row of the triple; blocks per super-group, a power of two
   int per_column;                     // tokens == 0: the blocks are (128,1), not (128,128)
-  int i_tiles, tiles, split_depth;
+  int i_tiles, tiles, items, split_depth;
 #ifdef PB_DIAGNOSTICS
   uint32_t polls;                     // poll budget of every wait
   int withhold;                       // the first stage is filled and never announced: every role runs out of patience
@@ -100,22 +101,31 @@ __device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_
 __device__ __forceinline__ void commit_to(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// K-major tile, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart (descriptor version 1, layout 2)
+// Operand tiles, 128-byte swizzle (descriptor version 1, layout 2).  TOKENS == false, K-major: rows of 128 bytes (64 of c), 8-row groups
+// 1024 bytes apart.  TOKENS, c outermost, as the operands lie in memory: 64 rows of 128 bytes (64 of i or j), eight c 1024 bytes apart,
+// the next 64 of i or j 8192.
+template <bool TOKENS>
 __device__ __forceinline__ uint64_t tile_desc(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr & 0x3ffffu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+  return (uint64_t)((smem_addr & 0x3ffffu) >> 4) | ((uint64_t)(TOKENS ? 8192 >> 4 : 1) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-// kind::f16: f32 accumulator, both operands bf16 and K-major, N = M = 128
-constexpr uint32_t kDotInstr = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTile >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
+template <bool TOKENS> constexpr uint32_t kStep16 = TOKENS ? 16 * 128 / 16 : 32 / 16;      // 16 of c further, in descriptor units
+// kind::f16: f32 accumulator, both operands bf16, both K-major or both not, N = M = 128
+template <bool TOKENS>
+constexpr uint32_t kDotInstr = (1u << 4) | (1u << 7) | (1u << 10) | (TOKENS ? 3u << 15 : 0u) | ((uint32_t)(kTile >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
+template <bool TOKENS>
 __device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-               ::"r"(d), "l"(a), "l"(b), "r"(kDotInstr), "r"(accumulate) : "memory");
+               ::"r"(d), "l"(a), "l"(b), "r"(kDotInstr<TOKENS>), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void ld_acc16(uint32_t taddr, uint32_t (&r)[16]) {
+__device__ __forceinline__ void ld_acc32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr) : "memory");
 }
 
@@ -138,28 +148,32 @@ __device__ __forceinline__ void split_chunk(const float (&g)[8], const float (&s
 #pragma unroll
   for (int e = 0; e < 4; ++e) split3(__fmul2_rn(make_float2(g[2 * e], g[2 * e + 1]), make_float2(s[2 * e], s[2 * e + 1])), hi[e], mid[e], lo[e]);
 }
-// byte offset of the 16-byte chunk (eight c) of a row in a swizzled tile
-__device__ __forceinline__ uint32_t chunk_at(int row, int chunk) { return (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4); }
+// byte offset of a 16-byte chunk of a swizzled tile: eight c of row i or j, or eight i or j of row c
+template <bool TOKENS>
+__device__ __forceinline__ uint32_t chunk_at(int row, int chunk) {
+  if (TOKENS) return (uint32_t)(chunk >> 3) * 8192u + (uint32_t)row * 128u + (uint32_t)(((chunk & 7) ^ (row & 7)) << 4);
+  return (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4);
+}
 __device__ __forceinline__ void st_chunk(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d));      // ordered by the fence at the stage's end
 }
 
-// What a converting thread holds of a stage: four chunks (eight c each) of g for rows j, its share of q, the scales of its c.
+// What a converting thread holds of a stage: four chunks of g, two pairs of chunks of q, the scales of their c.
 template <bool TOKENS, typename G>
 struct StageRegs {
-  static constexpr int kWords = sizeof(G) == 4 || TOKENS ? 8 : 4;
-  uint32_t g[4][kWords];              // as loaded: f32, or a bf16 in the low half, or two bf16
+  static constexpr int kWords = sizeof(G) == 4 ? 8 : 4;
+  static constexpr int kScales = TOKENS ? 4 : 8;      // it uses: TOKENS, of the rows of its chunks of g; else of the eight c of all of them
+  uint32_t g[4][kWords];              // as loaded: f32, or two bf16
   __device__ __forceinline__ void chunk(int k, float (&f)[8]) const {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       if constexpr (sizeof(G) == 4) f[e] = __uint_as_float(g[k][e]);
-      else if constexpr (TOKENS) f[e] = __uint_as_float(g[k][e] << 16);
       else f[e] = __uint_as_float(e & 1 ? g[k][e / 2] & 0xffff0000u : g[k][e / 2] << 16);
     }
   }
-  uint32_t q[TOKENS ? 16 : 8];        // TOKENS: [half][c] two i each; else 32 bytes of a row
-  uint32_t e8[TOKENS ? 1 : 8];        // TOKENS: lanes 0-7 a c each, handed round; else this thread's
-  float e32[TOKENS ? 1 : 8];
+  uint32_t q[8];                      // TOKENS: sixteen i of two c; else 32 c of a row
+  uint32_t e8[2];                     // of the two c of a stage whose scales this lane makes for its warp
+  float e32[2];
 };
 
 // what dequantizing multiplies a block's values by, before the exact 1/128
@@ -195,17 +209,25 @@ __device__ __noinline__ void plain_dots(const DotParams& p, float* out, int i, i
   }
 }
 
+// Where an item of the grid's work lies: a tile, and a part of the contraction.
+struct DotItem {
+  int it, i0, j0, c_begin, c_end, n_stages, split;
+  __device__ __forceinline__ DotItem(const DotParams& p, int w) {
+    split = w / p.tiles;
+    const int tile = w - split * p.tiles;
+    it = tile % p.i_tiles; i0 = it * kTile; j0 = (tile / p.i_tiles) * kTile;
+    c_begin = split * p.split_depth; c_end = min(p.C, c_begin + p.split_depth);
+    n_stages = (c_end - c_begin + kDepth - 1) / kDepth;
+  }
+};
+
 template <bool TOKENS, typename G>
 __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_constant__ DotParams p) {
   extern __shared__ unsigned char dot_smem[];
   __shared__ __align__(8) uint64_t bars[2 * kStages + 4];
   __shared__ uint32_t tmem_slot;
-  const uint32_t tiles_base = (dot_smem_u32(dot_smem) + 1023u) & ~1023u;
+  const uint32_t tiles_base = (dot_smem_u32(dot_smem) + 1023u) & ~1023u, out_base = tiles_base + kStages * kStageBytes;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int split = blockIdx.x / p.tiles, tile = blockIdx.x - split * p.tiles;
-  const int it = tile % p.i_tiles, i0 = it * kTile, j0 = (tile / p.i_tiles) * kTile;
-  const int c_begin = split * p.split_depth, c_end = min(p.C, c_begin + p.split_depth);
-  const int n_stages = (c_end - c_begin + kDepth - 1) / kDepth;
   auto full = [&](int s) { return dot_smem_u32(&bars[s]); };
   auto empty = [&](int s) { return dot_smem_u32(&bars[kStages + s]); };
   auto acc_full = [&](int a) { return dot_smem_u32(&bars[2 * kStages + a]); };
@@ -216,7 +238,7 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
     for (int a = 0; a < 2; ++a) { bar_init(acc_full(a), 1); bar_init(acc_empty(a), kDrainWarps); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == kConvWarps) {
+  if (warp == kIssueWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dot_smem_u32(&tmem_slot)), "r"(kAccCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -226,31 +248,41 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
   const uint32_t tmem = *(volatile uint32_t*)&tmem_slot;
 
   if (warp < kConvWarps) {
-    const int chunk = TOKENS ? warp : tid & 7;              // this thread's eight c of a stage
+    // a thread's chunks: TOKENS, eight j of rows c = (tid >> 4) + 16 k; else eight c of rows j = (tid >> 3) + 32 k
+    const int chunk = TOKENS ? tid & 15 : tid & 7, row = TOKENS ? tid >> 4 : tid >> 3;
+    constexpr int kRows = TOKENS ? 16 : 32, kScales = StageRegs<TOKENS, G>::kScales;
     StageRegs<TOKENS, G> r;
-    auto row_of = [&](int k) { return TOKENS ? 32 * k + lane : 32 * k + (tid >> 3); };
-    // Offsets from a stage's first element, the same for every stage: one add per load.  Rows past J are read again from the
-    // last one: what they make is never stored.  c past the end are zeros (only a last stage has them: `whole`).
+    const bool whole_chunks = p.J % 8 == 0;       // TOKENS: else the last chunk of a row of g ends in its middle
+    // Offsets from a stage's first element, the same for every stage of an item.  Rows past J are read again from the last one:
+    // what they make is never stored.  c past the end, and j past J where those are what is contiguous, are zeros.
     uint32_t g_row[4];
+    const uint32_t ldg = (uint32_t)p.ldg, q_step = TOKENS ? 32u * (uint32_t)p.ldq : 16u;
+    const uint32_t q_at = TOKENS ? (uint32_t)(tid >> 3) * (uint32_t)p.ldq + 16u * (tid & 7) : (uint32_t)(tid >> 1) * (uint32_t)p.ldq + (tid & 1) * 32;
+    auto set_rows = [&](const DotItem& w) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t j = (uint32_t)min(row_of(k), p.J - 1 - j0);
-      g_row[k] = TOKENS ? j : j * (uint32_t)p.ldg + 8 * chunk;
-    }
-    const uint32_t ldg = (uint32_t)p.ldg, ldq = (uint32_t)p.ldq;
-    const uint32_t q_at = TOKENS ? 8 * chunk * ldq + 2 * lane : (uint32_t)(tid >> 1) * ldq + (tid & 1) * 32;
-    auto load_g = [&](int st, int k) {
-      const int c0 = c_begin + st * kDepth;
-      const bool whole = c0 + kDepth <= c_end;
+      for (int k = 0; k < 4; ++k)
+        g_row[k] = TOKENS ? (uint32_t)(row + kRows * k) * ldg + 8u * chunk : (uint32_t)min(row + kRows * k, p.J - 1 - w.j0) * ldg + 8u * chunk;
+    };
+    auto load_g = [&](const DotItem& w, int c0, int k) {
       if constexpr (TOKENS) {
-        const G* src = static_cast<const G*>(p.g) + (int64_t)c0 * p.ldg + j0;
-        using Word = typename std::conditional<sizeof(G) == 4, uint32_t, uint16_t>::type;
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          r.g[k][e] = (whole || c0 + 8 * chunk + e < c_end) ? (uint32_t)__ldg(reinterpret_cast<const Word*>(src) + (8 * chunk + e) * ldg + g_row[k]) : 0u;
+        const G* src = static_cast<const G*>(p.g) + (int64_t)c0 * p.ldg + w.j0 + g_row[k];
+        const bool lo = c0 + row + kRows * k < w.c_end && w.j0 + 8 * chunk < p.J, hi = c0 + row + kRows * k < w.c_end && w.j0 + 8 * chunk + 4 < p.J;
+        if constexpr (sizeof(G) == 4) {
+          const uint4 zero = make_uint4(0, 0, 0, 0);
+          const uint4 a = lo ? __ldg(reinterpret_cast<const uint4*>(src)) : zero, b = hi ? __ldg(reinterpret_cast<const uint4*>(src) + 1) : zero;
+          r.g[k][0] = a.x; r.g[k][1] = a.y; r.g[k][2] = a.z; r.g[k][3] = a.w;
+          r.g[k][4] = b.x; r.g[k][5] = b.y; r.g[k][6] = b.z; r.g[k][7] = b.w;
+        } else if (whole_chunks) {
+          const uint4 a = lo ? __ldg(reinterpret_cast<const uint4*>(src)) : make_uint4(0, 0, 0, 0);
+          r.g[k][0] = a.x; r.g[k][1] = a.y; r.g[k][2] = a.z; r.g[k][3] = a.w;
+        } else {                                  // rows of whole 8-byte units
+          const uint2 zero = make_uint2(0, 0);
+          const uint2 a = lo ? __ldg(reinterpret_cast<const uint2*>(src)) : zero, b = hi ? __ldg(reinterpret_cast<const uint2*>(src) + 1) : zero;
+          r.g[k][0] = a.x; r.g[k][1] = a.y; r.g[k][2] = b.x; r.g[k][3] = b.y;
+        }
       } else {
-        const bool in = whole || c0 + 8 * chunk < c_end;    // C is a multiple of 16: a chunk is in or out together
-        const uint4* src = reinterpret_cast<const uint4*>(static_cast<const G*>(p.g) + (int64_t)j0 * p.ldg + c0 + g_row[k]);
+        const bool in = c0 + 8 * chunk < w.c_end;           // C is a multiple of 16: a chunk is in or out together
+        const uint4* src = reinterpret_cast<const uint4*>(static_cast<const G*>(p.g) + (int64_t)w.j0 * p.ldg + c0 + g_row[k]);
 #pragma unroll
         for (int h = 0; h < StageRegs<TOKENS, G>::kWords / 4; ++h) {
           const uint4 v = in ? __ldg(src + h) : make_uint4(0, 0, 0, 0);
@@ -258,178 +290,218 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
         }
       }
     };
-    auto load_q = [&](int st) {
-      const int c0 = c_begin + st * kDepth;
-      const bool whole = c0 + kDepth <= c_end;
-      if constexpr (TOKENS) {
-        const uint8_t* src = p.q + (int64_t)c0 * p.ldq + i0;
+    auto load_q = [&](const DotItem& w, int c0) {
+      const uint8_t* src = (TOKENS ? p.q + (int64_t)c0 * p.ldq + w.i0 : p.q + (int64_t)w.i0 * p.ldq + c0) + q_at;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const bool in = whole || c0 + 8 * chunk + e < c_end;
-          r.q[e] = in ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(src + q_at + e * ldq)) : 0u;
-          r.q[8 + e] = in ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(src + q_at + e * ldq + 64)) : 0u;
-        }
-      } else {
-        const uint8_t* src = p.q + (int64_t)i0 * p.ldq + c0;
+      for (int h = 0; h < 2; ++h) {
+        const int c = TOKENS ? (tid >> 3) + 32 * h : (tid & 1) * 32 + 16 * h;
+        const uint4 v = c0 + c < w.c_end ? __ldg(reinterpret_cast<const uint4*>(src + h * q_step)) : make_uint4(0, 0, 0, 0);
+        r.q[4 * h] = v.x; r.q[4 * h + 1] = v.y; r.q[4 * h + 2] = v.z; r.q[4 * h + 3] = v.w;
+      }
+    };
+    // A lane makes the scales of two of a stage's c and the warp hands them round: which register a thread takes one from is fixed.
+    auto load_scales = [&](const DotItem& w, int c0) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint4 v = whole || c0 + (tid & 1) * 32 + 16 * h < c_end ? __ldg(reinterpret_cast<const uint4*>(src + q_at) + h) : make_uint4(0, 0, 0, 0);
-          r.q[4 * h] = v.x; r.q[4 * h + 1] = v.y; r.q[4 * h + 2] = v.z; r.q[4 * h + 3] = v.w;
+      for (int h = 0; h < 2; ++h) {
+        const int c = c0 + (TOKENS ? lane + 32 * h : 2 * lane + h);
+        r.e8[h] = 0u; r.e32[h] = 0.0f;
+        if (c < w.c_end) {
+          const uint32_t id = TOKENS ? (uint32_t)c * p.nbc + w.it : (uint32_t)w.it * p.nbc + (p.per_column ? c : c / 128);
+          r.e8[h] = __ldg(p.sc8 + id); r.e32[h] = __ldg(p.sc32 + (id >> p.log2_K));
         }
       }
     };
-    auto load_scales = [&](int st) {
-      const int c = c_begin + st * kDepth + 8 * chunk;
+    int at = blockIdx.x, st = 0;
+    DotItem w(p, at);
+    int c0 = w.c_begin;
+    set_rows(w);
+    load_scales(w, c0);
+    load_q(w, c0);
 #pragma unroll
-      for (int e = 0; e < (TOKENS ? 1 : 8); ++e) { r.e8[e] = 0u; r.e32[e] = 0.0f; }
-      if constexpr (TOKENS) {
-        const int own = c + (lane & 7);
-        if (own < c_end) {
-          const uint32_t id = (uint32_t)own * p.nbc + it;
-          r.e8[0] = __ldg(p.sc8 + id); r.e32[0] = __ldg(p.sc32 + (id >> p.log2_K));
-        }
-      } else if (c < c_end) {
-        const uint32_t id = (uint32_t)it * p.nbc + (p.per_column ? c : c / 128);
-        r.e8[0] = __ldg(p.sc8 + id); r.e32[0] = __ldg(p.sc32 + (id >> p.log2_K));
-        if (p.per_column) {           // else 64 of c lie in one block
-#pragma unroll
-          for (int e = 1; e < 8; ++e) { r.e8[e] = __ldg(p.sc8 + id + e); r.e32[e] = __ldg(p.sc32 + ((id + e) >> p.log2_K)); }
+    for (int k = 0; k < 4; ++k) load_g(w, c0, k);
+    // The next stage's loads are asked for as their registers become free.  The fence that makes the stores visible to the tensor core
+    // is the issuing lane's: a thread's own waits for all that it has under way, loads too.
+    for (uint32_t n = 0;; ++n) {
+      if (++st == w.n_stages) {
+        at += gridDim.x;
+        st = 0;
+        if (at < p.items) {
+          w = DotItem(p, at);
+          set_rows(w);
         }
       }
-    };
-    auto load_stage = [&](int st) {
-      load_scales(st);
-      load_q(st);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) load_g(st, k);
-    };
-    load_stage(0);
-    for (int st = 0; st < n_stages; ++st) {
-      const int buf = st % kStages;
-      if (!bar_wait(empty(buf), ((st / kStages) & 1) ^ 1, wait_polls(p))) break;
+      const bool more = at < p.items;
+      c0 = w.c_begin + st * kDepth;
+      const int buf = n % kStages;
+      if (!bar_wait(empty(buf), ((n / kStages) & 1) ^ 1, wait_polls(p))) break;
       const uint32_t base = tiles_base + buf * kStageBytes;
-      const bool more = st + 1 < n_stages;
-      if constexpr (TOKENS) {
+      float s[kScales];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t lo[4], hi[4];      // the chunks of i = 64 h + 2 lane and the next
+      for (int h = 0; h < 2; ++h) {
+        const float own = __fmul_rn(block_multiplier(r.e8[h], r.e32[h]), kScaleUp * 0.0078125f);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint32_t a = r.q[8 * h + 2 * e], b = r.q[8 * h + 2 * e + 1];
-            lo[e] = fp8x2_to_bf16x2(__byte_perm(a, b, 0x0040)); hi[e] = fp8x2_to_bf16x2(__byte_perm(a, b, 0x0051));
+        for (int e = 0; e < kScales / 2; ++e) {
+          if constexpr (TOKENS) s[2 * h + e] = __shfl_sync(0xffffffffu, own, row + kRows * e);
+          else s[2 * e + h] = __shfl_sync(0xffffffffu, own, 4 * chunk + e);
+        }
+      }
+      if (more) load_scales(w, c0);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t o[2][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { o[e >> 1][2 * (e & 1)] = fp8x2_to_bf16x2(r.q[4 * h + e]); o[e >> 1][2 * (e & 1) + 1] = fp8x2_to_bf16x2(r.q[4 * h + e] >> 16); }
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          if constexpr (TOKENS) {       // the lanes of the second 64 of i store their second chunk first: else two lanes meet in every bank
+            const int x = tid & 7, which = b ^ (x >> 2);
+            st_chunk(base + chunk_at<TOKENS>((tid >> 3) + 32 * h, 2 * x + which), which ? o[1][0] : o[0][0], which ? o[1][1] : o[0][1], which ? o[1][2] : o[0][2], which ? o[1][3] : o[0][3]);
+          } else {
+            st_chunk(base + chunk_at<TOKENS>(tid >> 1, 4 * (tid & 1) + 2 * h + b), o[b][0], o[b][1], o[b][2], o[b][3]);
           }
-          st_chunk(base + chunk_at(64 * h + 2 * lane, chunk), lo[0], lo[1], lo[2], lo[3]);
-          st_chunk(base + chunk_at(64 * h + 2 * lane + 1, chunk), hi[0], hi[1], hi[2], hi[3]);
-        }
-      } else {
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          uint32_t o[4];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) { o[2 * e] = fp8x2_to_bf16x2(r.q[2 * h + e]); o[2 * e + 1] = fp8x2_to_bf16x2(r.q[2 * h + e] >> 16); }
-          st_chunk(base + chunk_at(tid >> 1, 4 * (tid & 1) + h), o[0], o[1], o[2], o[3]);
         }
       }
-      float s[8];
-      auto scale = [](uint32_t e8, float e32) { return __fmul_rn(block_multiplier(e8, e32), kScaleUp * 0.0078125f); };
-      if constexpr (TOKENS) {
-        const float own = scale(r.e8[0], r.e32[0]);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) s[e] = __shfl_sync(0xffffffffu, own, e);
-      } else {
-        s[0] = scale(r.e8[0], r.e32[0]);
-#pragma unroll
-        for (int e = 1; e < 8; ++e) s[e] = p.per_column ? scale(r.e8[e], r.e32[e]) : s[0];
-      }
+      if (more) load_q(w, c0);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         uint32_t hi[4], mid[4], lo[4];
-        float g[8];
+        float g[8], f[8];
         r.chunk(k, g);
-        split_chunk(g, s, hi, mid, lo);
-        const uint32_t at = base + chunk_at(row_of(k), chunk);
-        st_chunk(at + kOpBytes, lo[0], lo[1], lo[2], lo[3]);
-        st_chunk(at + 2 * kOpBytes, mid[0], mid[1], mid[2], mid[3]);
-        st_chunk(at + 3 * kOpBytes, hi[0], hi[1], hi[2], hi[3]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = TOKENS ? s[k % kScales] : s[e % kScales];
+        split_chunk(g, f, hi, mid, lo);
+        const uint32_t to = base + chunk_at<TOKENS>(row, chunk) + (uint32_t)(kRows * k) * 128u;      // eight rows further the same swizzle
+        st_chunk(to + kOpBytes, lo[0], lo[1], lo[2], lo[3]);
+        st_chunk(to + 2 * kOpBytes, mid[0], mid[1], mid[2], mid[3]);
+        st_chunk(to + 3 * kOpBytes, hi[0], hi[1], hi[2], hi[3]);
+        if (more) load_g(w, c0, k);
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the tensor core reads what was stored
       __syncwarp();
 #ifdef PB_DIAGNOSTICS
-      if (lane == 0 && !(p.withhold && st == 0)) bar_arrive(full(buf));
+      if (lane == 0 && !(p.withhold && n == 0)) bar_arrive(full(buf));
 #else
       if (lane == 0) bar_arrive(full(buf));
 #endif
-      // The next stage's loads go behind the fence, which waits for the thread's accesses that are under way: asked for as
-      // their registers became free, they held every stage up at its fence (dX 155 -> 150 us, dW 174 -> 160, 2368 tokens).
-      if (more) load_stage(st + 1);
+      if (!more) break;
+    }
+  } else if (warp >= kIssueWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == kIssueWarp && lane == 0) {
+      bool ok = true;
+      uint32_t n = 0;
+      for (int at = blockIdx.x; at < p.items && ok; at += gridDim.x)
+        for (int left = DotItem(p, at).n_stages; left > 0 && ok; --left, ++n) {
+          const int buf = n % kStages, ab = n & 1;
+          ok = bar_wait(full(buf), (n / kStages) & 1, wait_polls(p)) && bar_wait(acc_empty(ab), ((n >> 1) & 1) ^ 1, wait_polls(p));
+          if (!ok) break;
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the tensor core reads what the converting threads stored
+          tc_after();
+          const uint64_t a = tile_desc<TOKENS>(tiles_base + buf * kStageBytes);
+#pragma unroll
+          for (int kk = 0; kk < kDepth / 16; ++kk)            // smallest terms first
+#pragma unroll
+            for (int t = 1; t <= 3; ++t)
+              mma_f16<TOKENS>(tmem + (2 * ab + (kk >> 1)) * kTile, a + kk * kStep16<TOKENS>, a + (uint64_t)(t * (kOpBytes >> 4)) + kk * kStep16<TOKENS>, (kk & 1) || t > 1);
+          commit_to(empty(buf));
+          commit_to(acc_full(ab));
+        }
     }
   } else {
-    const int quad = warp & 3, half = (warp - kConvWarps) >> 2;      // rows 32 quad .., columns 64 half ..
-    // The first of these warps has one lane issue a stage's products, always a stage ahead of the one the warp empties.
-    auto issue = [&](int st) {
-      const int buf = st % kStages, ab = st & 1;
-      if (!bar_wait(full(buf), (st / kStages) & 1, wait_polls(p)) || !bar_wait(acc_empty(ab), ((st >> 1) & 1) ^ 1, wait_polls(p))) return false;
-      tc_after();
-      const uint64_t a = tile_desc(tiles_base + buf * kStageBytes);
-#pragma unroll
-      for (int kk = 0; kk < kDepth / 16; ++kk)              // smallest terms first; 16 of c are 32 bytes of a row
-#pragma unroll
-        for (int t = 1; t <= 3; ++t)
-          mma_f16(tmem + (2 * ab + (kk >> 1)) * kTile, a + 2 * kk, a + (uint64_t)(t * (kOpBytes >> 4)) + 2 * kk, (kk & 1) || t > 1);
-      commit_to(empty(buf));
-      commit_to(acc_full(ab));
-      return true;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");      // 128 * (2 * 128 + 216 + 40) = 512 * 128
+    const int quad = warp & 3, r = quad * 32 + lane;         // the thread's row of the tile, an i
+    auto drains_meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kDrainWarps) : "memory"); };
+    auto drains_any = [](bool mine) {
+      uint32_t any;
+      asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(any) : "r"((uint32_t)mine), "n"(32 * kDrainWarps) : "memory");
+      return any != 0;
     };
-    bool issuing = warp == kConvWarps && lane == 0;
-    if (issuing) issuing = issue(0);
-    __syncwarp();
-    float acc[64];
+    bool ok = true, odd = false;        // odd: some sum of this thread is not finite
+    uint32_t n = 0;
+    for (int at = blockIdx.x; at < p.items && ok; at += gridDim.x) {
+      const DotItem w(p, at);
+      float acc[kTile];
 #pragma unroll
-    for (int n = 0; n < 64; ++n) acc[n] = 0.0f;
-    for (int st = 0; st < n_stages; ++st) {
-      const int ab = st & 1;
-      if (issuing && st + 1 < n_stages) issuing = issue(st + 1);
-      __syncwarp();
-      if (!bar_wait(acc_full(ab), (st >> 1) & 1, wait_polls(p))) break;
-      tc_after();
-      const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + 2 * ab * kTile + half * 64;
-      uint32_t v[2][16];
-      ld_acc16(at, v[0]);
+      for (int e = 0; e < kTile; ++e) acc[e] = 0.0f;
+      for (int st = 0; st < w.n_stages; ++st, ++n) {
+        const int ab = n & 1;
+        ok = __all_sync(0xffffffffu, bar_wait(acc_full(ab), (n >> 1) & 1, wait_polls(p)));
+        if (!ok) break;
+        tc_after();
+        const uint32_t from = tmem + ((uint32_t)(quad * 32) << 16) + 2 * ab * kTile;
+        uint32_t v[2][32];
+        ld_acc32(from, v[0]);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {   // 16 columns of one accumulator, then of the other
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (k + 1 < 8) {
-          ld_acc16(at + ((k + 1) & 3) * 16 + ((k + 1) >> 2) * kTile, v[(k + 1) & 1]);
-        } else {
-          tc_before();
-          __syncwarp();
-          if (lane == 0) bar_arrive(acc_empty(ab));
+        for (int k = 0; k < 8; ++k) {   // 32 columns of one accumulator, then of the other
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (k + 1 < 8) {
+            ld_acc32(from + (k + 1) * 32, v[(k + 1) & 1]);
+          } else {
+            tc_before();
+            __syncwarp();
+            if (lane == 0) bar_arrive(acc_empty(ab));
+          }
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            float* to = acc + 32 * (k & 3) + e;
+            const float2 t = __fadd2_rn(make_float2(to[0], to[1]), make_float2(__uint_as_float(v[k & 1][e]), __uint_as_float(v[k & 1][e + 1])));
+            to[0] = t.x; to[1] = t.y;
+          }
         }
-#pragma unroll
-        for (int n = 0; n < 16; ++n) acc[16 * (k & 3) + n] += __uint_as_float(v[k & 1][n]);
       }
-    }
-    float* out = p.out + (int64_t)split * p.part;
-    const int i = i0 + quad * 32 + lane, jb = j0 + half * 64;
-    if constexpr (TOKENS) {
+      // The tile leaves by way of shared memory, a bulk copy per row of out: stores from registers were hundreds of instructions
+      // that a warp runs through once, most of whose time went into fetching them (8192 rows, 2048 x 128: 15000 cycles a tile).
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the tile before has left
+      ok = !drains_any(!ok);              // all of these warps give up, or none: they wait for one another below
+      if (!ok) break;
+      float2 zero = make_float2(0.0f, 0.0f);            // times 0: NaN where a sum is not finite
 #pragma unroll
-      for (int n = 0; n < 64; n += 4)
-        if (jb + n < p.J)             // J is a multiple of 4
-          *reinterpret_cast<float4*>(out + (int64_t)i * p.ldo + jb + n) =
-              make_float4(acc[n] * kScaleDown, acc[n + 1] * kScaleDown, acc[n + 2] * kScaleDown, acc[n + 3] * kScaleDown);
+      for (int e = 0; e < kTile; e += 2) {
+        zero = __ffma2_rn(make_float2(acc[e], acc[e + 1]), make_float2(0.0f, 0.0f), zero);
+        const float2 t = __fmul2_rn(make_float2(acc[e], acc[e + 1]), make_float2(kScaleDown, kScaleDown));
+        acc[e] = t.x; acc[e + 1] = t.y;
+      }
+      odd |= !(zero.x + zero.y == 0.0f);
+#pragma unroll
+      for (int e = 0; e < kTile; e += 4) {
+        if constexpr (TOKENS) {
+          asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(out_base + r * kOutPitch + e * 4), "f"(acc[e]), "f"(acc[e + 1]), "f"(acc[e + 2]), "f"(acc[e + 3]) : "memory");
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) asm volatile("st.shared.f32 [%0], %1;" ::"r"(out_base + (e + k) * kOutPitch + r * 4), "f"(acc[e + k]) : "memory");
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      drains_meet();
+      // row r of the tile in shared memory: an i (TOKENS) or a j; J is a multiple of 4 (TOKENS)
+      const int bytes = TOKENS ? 4 * min(kTile, p.J - w.j0) : (w.j0 + r < p.J ? 4 * kTile : 0);
+      float* to = p.out + (int64_t)w.split * p.part + (TOKENS ? (int64_t)(w.i0 + r) * p.ldo + w.j0 : (int64_t)(w.j0 + r) * p.ldo + w.i0);
+      if (bytes) asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(to), "r"(out_base + r * kOutPitch), "r"(bytes) : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    // Sums that are not finite are made again when the CTA's tiles are done: nothing waits for these warps any more, however long it takes.
+    if (drains_any(odd && ok)) {
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");           // what is made again lies in out already
+      drains_meet();
+#pragma unroll 1
+      for (int at = blockIdx.x; at < p.items; at += gridDim.x) {
+        const DotItem w(p, at);
+        float* out = p.out + (int64_t)w.split * p.part;
+        const int i = w.i0 + r;
+#pragma unroll 1
+        for (int jb = w.j0; jb < w.j0 + kTile; jb += 64) {
+          bool again = false;
+#pragma unroll 1
+          for (int j = jb; j < min(jb + 64, p.J); ++j) again |= __float_as_uint(out[TOKENS ? (int64_t)i * p.ldo + j : (int64_t)j * p.ldo + i]) << 1 >= 2 * 0x7f800000u;
+          if (again) plain_dots<TOKENS, G>(p, out, i, jb, w.it, w.c_begin, w.c_end);
+        }
+      }
     } else {
-#pragma unroll
-      for (int n = 0; n < 64; ++n)
-        if (jb + n < p.J) out[(int64_t)(jb + n) * p.ldo + i] = acc[n] * kScaleDown;
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // shared memory is the CTA's until the last tile has left it
     }
-    uint32_t most = 0;                // twice the largest magnitude's bits
-#pragma unroll
-    for (int n = 0; n < 64; ++n) most = max(most, __float_as_uint(acc[n]) << 1);
-    if (most >= 2 * 0x7f800000u) plain_dots<TOKENS, G>(p, out, i, jb, it, c_begin, c_end);
   }
   tc_before();
   __syncthreads();
-  if (warp == kConvWarps) {
+  if (warp == kIssueWarp) {
     tc_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kAccCols) : "memory");
   }
@@ -550,12 +622,12 @@ extern "C" int pb_dense_dot(int tokens, const uint8_t* q, const uint8_t* sc8, co
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   float* dst = d.splits > 1 ? static_cast<float*>(workspace) : out;
   DotParams p{q, sc8, sc32, g, dst, cols, tokens ? g_free : cols, tokens ? g_free : (int64_t)d.I, out_elems, d.I, d.J, d.C,
-              (uint32_t)geo.nbc, log2_K, b == 1, d.i_tiles, d.tiles, d.split_depth};
+              (uint32_t)geo.nbc, log2_K, b == 1, d.i_tiles, d.tiles, d.tiles * d.splits, d.split_depth};
 #ifdef PB_DIAGNOSTICS
   p.polls = g_dot_polls.load();
   p.withhold = g_dot_withhold.load();
 #endif
-  const unsigned grid = (unsigned)(d.tiles * d.splits);
+  const unsigned grid = (unsigned)std::min(p.items, sm_count());
   const int status = tokens ? (g_dtype == PB_F32 ? launch_dot<true, float>(p, grid, st) : launch_dot<true, __nv_bfloat16>(p, grid, st))
                             : (g_dtype == PB_F32 ? launch_dot<false, float>(p, grid, st) : launch_dot<false, __nv_bfloat16>(p, grid, st));
   if (status) return status;

@@ -3,6 +3,7 @@ or column, a contraction shorter than a stage, parts of it on several CTAs, and 
 import pytest
 import torch
 
+from pratchya_b200 import _lib
 from pratchya_b200._qualia import _ops
 from pratchya_b200._qualia import dequantize_impl, quantize_impl
 
@@ -101,3 +102,38 @@ def test_other_shapes_take_the_library_route(built_lib):
         gx, gw = _ops.literal_dots(xq, wq, gx_, gw_, dy)
         xh, wh = dequantize_impl(*xq, torch.float32, gx_).double(), dequantize_impl(*wq, torch.float32, gw_).double()
         assert (gx.double() - dy.double() @ wh.t()).abs().max() <= 1e-4 and (gw.double() - xh.t() @ dy.double()).abs().max() <= 1e-4
+
+
+@pytest.mark.parametrize("tokens,rows,cols,grid,free", [(0, 2048, 128, (128, 1), 2433), (0, 3072, 48, (128, 1), 1030), (0, 256, 4112, (128, 1), 129), (1, 100, 2048, (1, 128), 1316), (1, 65, 1024, (1, 128), 2500),
+                                                        (1, 1090, 256, (1, 128), 4), (1, 200, 384, (1, 128), 132)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_several_tiles_per_cta_and_ragged_ends(built_lib, tokens, rows, cols, grid, free, dtype):
+    """More tiles than SMs (a tile leaves while the next is made), parts of a contraction that end inside a stage, rows of g that end inside
+    a chunk of eight; then the sums of one cotangent, in the last tile, that are not finite and made again."""
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols + free)
+    q, sc8, sc32 = quantize_impl(torch.randn(rows, cols, generator=gen, device="cuda") * 0.02, grid)
+    g = (torch.randn(rows if tokens else free, free if tokens else cols, generator=gen, device="cuda") * 1e-3).to(dtype)
+    code = _lib.PB_F32 if dtype is torch.float32 else _lib.PB_BF16
+    size = built_lib.pb_dense_dot_workspace_size(tokens, rows, cols, *grid, free)
+    ws = torch.full((max(size, 16),), 0xff, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    d = dequantize_impl(q, sc8, sc32, torch.float32, grid).double()
+
+    def run():
+        out = torch.full(((cols, free) if tokens else (free, rows)), float("nan"), device="cuda")
+        _lib.check(built_lib.pb_dense_dot(tokens, q.data_ptr(), sc8.data_ptr(), sc32.data_ptr(), rows, cols, *grid, g.data_ptr(), code, free, out.data_ptr(), ws.data_ptr(), size, stream))
+        a, b = (d.t(), g.double()) if tokens else (g.double(), d.t())
+        return out.double(), a @ b, _bound(a, b)
+
+    got, want, bound = run()
+    assert ((got - want).abs() <= bound + 1e-30).all()
+    (g[:, -1] if tokens else g[-1]).mul_(1e33)
+    got, want, bound = run()
+    finite = torch.ones(free, dtype=torch.bool, device="cuda")
+    finite[-1] = False
+    got_f, want_f, bound_f = (t[:, finite] if tokens else t[finite] for t in (got, want, bound))
+    assert ((got_f - want_f).abs() <= bound_f + 1e-30).all()
+    last, want_l = (got[:, -1], want[:, -1]) if tokens else (got[-1], want[-1])      # f32 products one after the other
+    bound_l = (bound[:, -1] if tokens else bound[-1]) * (rows if tokens else cols)
+    assert ((last - want_l).abs() <= bound_l).all()
+    assert built_lib.pb_gemm_check(stream) == 0
