@@ -21,16 +21,15 @@
 //
 // A CTA makes 128 x 128 tiles of out, one after the other: eight warps convert (global loads into registers, scale, split, 128-byte
 // swizzled tiles in shared memory: K-major for dX, with c outermost, as the operands lie in memory, for dW), four warps empty one pair of
-// accumulators while the other fills, and a lane of a warp of its own issues tcgen05.mma: as a lane of an emptying warp it was what
-// a stage waited for (1200 cycles to issue a stage's twelve, 700 to empty one). A finished tile leaves by bulk copies from shared
-// memory.  Where the tiles do not fill the SMs the contraction is cut, and the parts are added in order by a second kernel.
+// accumulators while the other fills and store finished tiles, and a lane of a warp of its own issues tcgen05.mma: as a lane of an
+// emptying warp it was what a stage waited for (1200 cycles to issue a stage's twelve, 700 to empty one).  Where the tiles do not
+// fill the SMs the contraction is cut, and the parts are added in order by a second kernel.
 //
 // What bounds it: shared memory's data path.  A stage takes 2400 cycles, of which the converting warps' stores, loads and shuffles hold
 // it for 1000 and the tensor core's reads of both operands (three terms against the same fp8 tile) for 770; their shuffles
 // queue behind the stores.  Prefetching g into L2 gained 2 us where g streams from HBM and lost one where it does not; two stages' loads
-// under way, other orders of the conversions: nothing.  Against the first form (emptying warps that issued, stores of a tile from
-// registers, whose instructions had to be fetched for one use: 15000 cycles of a 58000-cycle CTA), us in a CUDA graph: 8192 tokens, f32, 2048 x 128
-// dX 62 -> 31, dW 40 -> 30, 128 x 2048 38 -> 35 and 41 -> 31; 704 tokens, 128 x 1024 15.0 -> 12.0, 19.0 -> 13.4; 64 tokens, 2048 x 128 9.6 -> 7.6, 8.5 -> 7.0;
+// under way, other orders of the conversions: nothing.  Against the first form (emptying warps that issued, an address computed for every store
+// of a tile: 15000 cycles of a 58000-cycle CTA), us in a CUDA graph: 8192 tokens, f32, 2048 x 128 dX 62 -> 28, dW 40 -> 30, 128 x 2048 38 -> 35 and 41 -> 31; 704 tokens, 128 x 1024 15.0 -> 12.0, 19.0 -> 13.4; 64 tokens, 2048 x 128 9.6 -> 7.6, 8.5 -> 7.0;
 // the same bits.
 //
 // Every tile converts what it reads, so an operand that many tiles share is converted many times: where 512 columns or more share
@@ -409,12 +408,6 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");      // 128 * (2 * 128 + 216 + 40) = 512 * 128
     const int quad = warp & 3, r = quad * 32 + lane;         // the thread's row of the tile, an i
-    auto drains_meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kDrainWarps) : "memory"); };
-    auto drains_any = [](bool mine) {
-      uint32_t any;
-      asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(any) : "r"((uint32_t)mine), "n"(32 * kDrainWarps) : "memory");
-      return any != 0;
-    };
     bool ok = true, odd = false;        // odd: some sum of this thread is not finite
     uint32_t n = 0;
     for (int at = blockIdx.x; at < p.items && ok; at += gridDim.x) {
@@ -448,10 +441,6 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
           }
         }
       }
-      // The tile leaves by way of shared memory, a bulk copy per row of out: stores from registers were hundreds of instructions
-      // that a warp runs through once, most of whose time went into fetching them (8192 rows, 2048 x 128: 15000 cycles a tile).
-      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the tile before has left
-      ok = !drains_any(!ok);              // all of these warps give up, or none: they wait for one another below
       if (!ok) break;
       float2 zero = make_float2(0.0f, 0.0f);            // times 0: NaN where a sum is not finite
 #pragma unroll
@@ -461,27 +450,31 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
         acc[e] = t.x; acc[e + 1] = t.y;
       }
       odd |= !(zero.x + zero.y == 0.0f);
+      float* out = p.out + (int64_t)w.split * p.part;
+      if constexpr (TOKENS) {           // a thread's row of out, by way of shared memory: whole lines (of 16 bytes a lane: 1 us more)
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");    // the tile before has left
 #pragma unroll
-      for (int e = 0; e < kTile; e += 4) {
-        if constexpr (TOKENS) {
+        for (int e = 0; e < kTile; e += 4)
           asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(out_base + r * kOutPitch + e * 4), "f"(acc[e]), "f"(acc[e + 1]), "f"(acc[e + 2]), "f"(acc[e + 3]) : "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                     ::"l"(out + (int64_t)(w.i0 + r) * p.ldo + w.j0), "r"(out_base + r * kOutPitch), "r"(4 * min(kTile, p.J - w.j0)) : "memory");      // J is a multiple of 4
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      } else {                          // one address, moved on: with an address per store the code took 15000 cycles to fetch for one use
+        float* to = out + (int64_t)w.j0 * p.ldo + w.i0 + r;
+        if (w.j0 + kTile <= p.J) {
+#pragma unroll
+          for (int e = 0; e < kTile; ++e, to += p.ldo) *to = acc[e];
         } else {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) asm volatile("st.shared.f32 [%0], %1;" ::"r"(out_base + (e + k) * kOutPitch + r * 4), "f"(acc[e + k]) : "memory");
+          for (int e = 0; e < kTile; ++e, to += p.ldo)
+            if (w.j0 + e < p.J) *to = acc[e];
         }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      drains_meet();
-      // row r of the tile in shared memory: an i (TOKENS) or a j; J is a multiple of 4 (TOKENS)
-      const int bytes = TOKENS ? 4 * min(kTile, p.J - w.j0) : (w.j0 + r < p.J ? 4 * kTile : 0);
-      float* to = p.out + (int64_t)w.split * p.part + (TOKENS ? (int64_t)(w.i0 + r) * p.ldo + w.j0 : (int64_t)(w.j0 + r) * p.ldo + w.i0);
-      if (bytes) asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(to), "r"(out_base + r * kOutPitch), "r"(bytes) : "memory");
-      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
     // Sums that are not finite are made again when the CTA's tiles are done: nothing waits for these warps any more, however long it takes.
-    if (drains_any(odd && ok)) {
-      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");           // what is made again lies in out already
-      drains_meet();
+    if (odd && ok) {
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");           // what the thread makes again lies in out already
 #pragma unroll 1
       for (int at = blockIdx.x; at < p.items; at += gridDim.x) {
         const DotItem w(p, at);
@@ -495,9 +488,8 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
           if (again) plain_dots<TOKENS, G>(p, out, i, jb, w.it, w.c_begin, w.c_end);
         }
       }
-    } else {
-      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // shared memory is the CTA's until the last tile has left it
     }
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");        // shared memory is the CTA's until the last tile has left it
   }
   tc_before();
   __syncthreads();

@@ -5,11 +5,13 @@
 //   tokens == 1:  out[i, j] = sum_c dq(Q)[c, i] * g[c, j]      (dW = X^T g,  :621)
 //
 // One operand is exact in bf16 as it is, the other is kept as three bf16 terms, hi + mid + lo, which hold all 24 bits of an f32:
-//   g in bf16:  g as it is; the dequantized values (the one f32 rounding that dequantizing makes) as three terms.  Any grid.
+//   g in bf16:  g as it is; the dequantized values (the one f32 rounding that dequantizing makes) as three terms.  Any grid.  For dX with
+//               a super-group's factor that belongs to rows of Q (out's columns) the fp8 values times their block's power of two, one term:
+//               that factor goes to the finished sum, and every product is one tensor-core product.
 //   g in f32:   the fp8 values times their block's power of two (exact; where it is not, a NaN, see below); g as three terms, times
 //               the super-group's f32 factor where that varies along c (tokens == 1, one set of terms per 1024 columns of
 //               Q; one f32 rounding), while a factor that belongs to a column of dX goes to the finished sum.
-// Every f32 product is then exact in three tensor-core products, and the accumulator is emptied into f32 registers every 64 of c
+// Every f32 product is then exact in its tensor-core products, and the accumulator is emptied into f32 registers every 64 of c
 // (the tensor core's own additions do not round to nearest; dense_dot.cu empties every 32): the low terms of all 64 go first, so that
 // four additions meet a sum of full size, as many as there, and half as many f32 additions follow.  Contractions of a few hundred have
 // few of those to save, and where the low terms are the fp8 operand's the four are all that is left: bf16 g over fewer than
@@ -20,9 +22,14 @@
 // them above bf16's subnormals.  A sum that is not finite, for an infinity or a NaN in the operands, an overflow of a scaled
 // term or a power of two that bf16 does not hold, is made again with f32 products of dequantized values, behind the last tile.
 //
+// One term for three, us in a CUDA graph: 3000 tokens, 2048 x 2048 79 -> 39, 1000 tokens 40 -> 23; 2-norm errors 1.31e-7 -> 1.06e-7.  What it is bound
+// by then is waits and issuing, so its stages hold 64 of c, not 32 (53 -> 44 us), and the stores of a finished tile: one address that
+// moves on, where sixteen columns a time through shared memory and bulk copies took 44 -> 39, and an address and a look at every sum more
+// (f32 dW of 300 tokens, 2048 x 4096: 30.5 -> 26.6).
+//
 // Element-wise kernel: bound by its bytes.  Main kernel: persistent, one CTA per SM; a tile is 128 rows of the three-term operand
 // by N of the other; a stage is 32 of c of both, by TMA, K-major (64-byte swizzle) for tokens == 0 and with c outermost, as
-// it lies in memory, for tokens == 1 (128-byte swizzle): no transpose anywhere.  Warp 0 loads, warp 1 issues six
+// it lies in memory, for tokens == 1 (128-byte swizzle): no transpose anywhere.  Warp 0 loads, warp 1 issues six (four)
 // tcgen05.mma a stage, eight warps empty one accumulator while the other fills.  N is 256, 192 or 128, whichever fills whole waves of SMs best.
 #include <cuda.h>
 
@@ -39,18 +46,22 @@ constexpr int kTermRows = 128;        // of the three-term operand, per tile
 constexpr int kDepth = 32;            // c per stage
 constexpr int kGroup = 2;             // stages per accumulator, at most
 constexpr int kShortDepth = 384;      // of c, from which bf16 g takes that many
-constexpr int kTermBytes = kTermRows * kDepth * 2;
 constexpr int kDrainWarps = 8;
 constexpr int kThreads = 64 + 32 * kDrainWarps;
 constexpr uint32_t kWaitPolls = 1u << 21;               // a poll parks for up to 2 us: about four seconds at most
 constexpr float kScaleUp = 0x1p40f, kScaleDown = 0x1p-40f;
 constexpr size_t kMaxTerms = (size_t)512 << 20;         // bytes of three-term operand at a time: more of it takes several rounds (1024 of its rows at least)
 
-template <int N>
+constexpr int kOutCols = 16;           // of a finished tile that a thread stores at a time
+
+template <int N, bool TOKENS, bool G32, int TERMS>
 struct Cfg {
-  static constexpr int kStages = N == 256 ? 5 : 6;
-  static constexpr int kStageBytes = 3 * kTermBytes + N * kDepth * 2;
+  static constexpr int kUnits = TERMS == 1 ? 2 : 1;    // of kDepth, per stage: one term's stages are otherwise more waiting and issuing than products
+  static constexpr int kTermBytes = kTermRows * kDepth * 2 * kUnits;
+  static constexpr int kStageBytes = TERMS * kTermBytes + N * kDepth * 2 * kUnits;
+  static constexpr int kStages = TERMS == 1 ? (N == 256 ? 4 : (N == 192 ? 5 : 6)) : (N == 256 ? 5 : 6);
   static constexpr int kSmem = kStages * kStageBytes + 1024;      // 1024: the tiles start on a swizzle atom
+  static_assert(kSmem + 512 <= 232448, "an SM's shared memory");
 };
 
 __device__ unsigned int g_split_status; // 0, or PB_ERR_DEVICE_TIMEOUT once a bounded wait ran out
@@ -67,7 +78,7 @@ struct DotSource {
 struct SplitParams {
   DotSource src;
   float* out;                         // or the parts, [splits][out]
-  const float* col_factor;            // tokens == 0, f32 g: sc32, one factor per 128 columns of a tile's N; else null
+  const float* factor;                // tokens == 0, one factor per 128 of i for the finished sums (sc32): of the tile's columns with f32 g, of its rows with one term
   int64_t ld, part;                   // row stride of out, elements of a part
   int rows, cols;                     // extents of the three-term operand and of the other
   int row_first;                      // the first of these rows, for the sums that are made again
@@ -104,13 +115,14 @@ __device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_
 __device__ __forceinline__ void commit_to(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// Operand tiles (descriptor version 1).  K-major: rows of 64 bytes (32 of c), 8-row groups 512 bytes apart, 64-byte swizzle.
-// c outermost: 32 rows of 128 bytes (64 of the operand's rows), eight c 1024 bytes apart, the next 64 rows 4096, 128-byte swizzle.
-template <bool TOKENS>
+// Operand tiles (descriptor version 1).  K-major: rows of 64 bytes (32 of c), 8-row groups 512 bytes apart, 64-byte swizzle; with 64 of c
+// (UNITS == 2) twice of each.  c outermost: 32 rows of 128 bytes (64 of the operand's rows), eight c 1024 bytes apart, the next 64 rows 4096,
+// 128-byte swizzle.
+template <bool TOKENS, int UNITS>
 __device__ __forceinline__ uint64_t tile_desc(uint32_t addr) {
   const uint64_t start = (uint64_t)((addr & 0x3ffffu) >> 4) | (1ull << 46);
   if (TOKENS) return start | ((uint64_t)(4096 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (2ull << 61);
-  return start | (1ull << 16) | ((uint64_t)(512 >> 4) << 32) | (4ull << 61);
+  return start | (1ull << 16) | ((uint64_t)(512 * UNITS >> 4) << 32) | ((UNITS == 2 ? 2ull : 4ull) << 61);
 }
 template <bool TOKENS> constexpr uint32_t kStep16 = TOKENS ? 16 * 128 / 16 : 32 / 16;      // 16 of c further, in descriptor units
 // kind::f16: f32 accumulator, both operands bf16, both K-major or both not
@@ -158,16 +170,16 @@ struct PrepareParams {
   int variants;                       // tokens == 1: sets of terms of g, K blocks of a row of Q each
 };
 
-// sixteen values of Q from their bytes: terms of the dequantized values (TERMS), or value times its block's power of two
+// sixteen values of Q from their bytes: terms of the dequantized values (TERMS), or value times its block's power of two (times `up`)
 template <bool TERMS>
-__device__ __forceinline__ void prepare_q(const PrepareParams& p, uint32_t v) {
+__device__ __forceinline__ void prepare_q(const PrepareParams& p, uint32_t v, float up) {
   const uint32_t in_row = p.q_vecs.div(v), row = p.q_row0 + in_row, col = p.q_col0 + (v - in_row * p.q_vecs.d) * 16;
   const uint4 bytes = __ldg(reinterpret_cast<const uint4*>(p.q + (int64_t)row * p.ldq + col));
   const uint32_t words[4] = {bytes.x, bytes.y, bytes.z, bytes.w};
   const uint32_t id0 = (row >> p.log2_a) * p.nbc + (col >> p.log2_b);
   auto multiplier = [&](uint32_t id) {
     const float two = e8m0_to_f32(__ldg(p.sc8 + id));
-    return TERMS ? __fmul_rn(__fmul_rn(two, __ldg(p.sc32 + (id >> p.log2_K))), kScaleUp * 0.0078125f) : two;
+    return TERMS ? __fmul_rn(__fmul_rn(two, __ldg(p.sc32 + (id >> p.log2_K))), kScaleUp * 0.0078125f) : two * up;
   };
   const float m0 = multiplier(id0);
   uint32_t hi[8], mid[8], lo[8];
@@ -210,12 +222,12 @@ __device__ __forceinline__ void prepare_g(const PrepareParams& p, uint32_t v) {
   }
 }
 
-// G32: f32 g.  Blocks [0, q_blocks) work on Q, the others on g.
-template <bool TOKENS, bool G32>
+// G32: f32 g.  TERMS: of Q, where g is used as it is.  Blocks [0, q_blocks) work on Q, the others on g.
+template <bool TOKENS, bool G32, int TERMS>
 __global__ void __launch_bounds__(256) split_prepare_kernel(const __grid_constant__ PrepareParams p) {
   if (blockIdx.x < p.q_blocks) {
     const uint32_t v = blockIdx.x * 256 + threadIdx.x;
-    if (v < p.n_q) prepare_q<!G32>(p, v);
+    if (v < p.n_q) prepare_q<!G32 && TERMS == 3>(p, v, G32 ? 1.0f : kScaleUp);
   } else if (G32) {
     const uint32_t v = (blockIdx.x - p.q_blocks) * 256 + threadIdx.x;
     if (v < p.n_g) prepare_g<TOKENS>(p, v);
@@ -267,11 +279,12 @@ __device__ __noinline__ void remake_sums(const SplitParams& p, float* out, int r
   }
 }
 
-// N columns per tile; TOKENS: c is the operands' outer dimension; G32: the terms are g's (rows are j, columns i), else Q's (rows i, columns j).
-template <int N, bool TOKENS, bool G32>
+// N columns per tile; TOKENS: c is the operands' outer dimension; G32: the terms are g's (rows are j, columns i), else Q's (rows i, columns j);
+// TERMS: 3, or 1 where Q's exact values are multiplied and its super-group's factor goes to the finished sums.
+template <int N, bool TOKENS, bool G32, int TERMS>
 __global__ void __launch_bounds__(kThreads, 1)
 split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_constant__ CUtensorMap map_other, const __grid_constant__ SplitParams p) {
-  using C = Cfg<N>;
+  using C = Cfg<N, TOKENS, G32, TERMS>;
   constexpr bool kLanes = TOKENS == G32;        // out is contiguous along the tile's rows, that is across the lanes of a warp
   constexpr int kCols = N / 2;                  // of an emptying thread
   extern __shared__ unsigned char split_smem[];
@@ -312,19 +325,19 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
         int row0, col0, u, u_end;
         item_of(w, row0, col0, u, u_end);
         const int set = TOKENS && G32 ? 3 * (col0 / p.cols_per_variant) : 0;
-        for (; u < u_end; ++u, ++it) {
+        for (; u < u_end; u += C::kUnits, ++it) {      // a last stage that ends behind c is filled with zeros
           const int s = it % C::kStages;
           if (!bar_wait(empty(s), ((it / C::kStages) & 1) ^ 1, p.polls)) { ok = false; break; }
           if (p.withhold && it == 0) continue;
-          const uint32_t bar = full(s), at = base + s * C::kStageBytes, other = at + 3 * kTermBytes;
+          const uint32_t bar = full(s), at = base + s * C::kStageBytes, other = at + TERMS * C::kTermBytes;
           bar_expect(bar, C::kStageBytes);
 #pragma unroll
-          for (int t = 0; t < 3; ++t) {
+          for (int t = 0; t < TERMS; ++t) {
             if (TOKENS) {
-              load_box(at + t * kTermBytes, &map_terms, row0, u * kDepth, set + t, bar);
-              load_box(at + t * kTermBytes + 4096, &map_terms, row0 + 64, u * kDepth, set + t, bar);
+              load_box(at + t * C::kTermBytes, &map_terms, row0, u * kDepth, set + t, bar);
+              load_box(at + t * C::kTermBytes + 4096, &map_terms, row0 + 64, u * kDepth, set + t, bar);
             } else {
-              load_box(at + t * kTermBytes, &map_terms, u * kDepth, row0, t, bar);
+              load_box(at + t * C::kTermBytes, &map_terms, u * kDepth, row0, t, bar);
             }
           }
           if (TOKENS) {
@@ -347,11 +360,12 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
         int row0, col0, u, u_end;
         item_of(w, row0, col0, u, u_end);
         for (; u < u_end; u += p.group, ++group) {
-          const int ab = group & 1, depth = min(p.group, u_end - u);
+          const int ab = group & 1, depth = C::kUnits == 2 ? 1 : min(p.group, u_end - u);      // stages
           if (!bar_wait(acc_empty(ab), ((group >> 1) & 1) ^ 1, p.polls)) { ok = false; break; }
-          uint32_t at[kGroup], freed[kGroup];
+          constexpr int kMost = kGroup / C::kUnits;
+          uint32_t at[kMost], freed[kMost];
 #pragma unroll
-          for (int h = 0; h < kGroup; ++h) {
+          for (int h = 0; h < kMost; ++h) {
             if (h >= depth) break;
             const int s = it % C::kStages;
             if (!bar_wait(full(s), (it / C::kStages) & 1, p.polls)) { ok = false; break; }
@@ -362,17 +376,17 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
           tc_after();
           // Smallest terms first, over all of the group: only the last few additions meet a sum of full size.
 #pragma unroll
-          for (int t = 2; t >= 0; --t)
+          for (int t = TERMS - 1; t >= 0; --t)
 #pragma unroll
-            for (int h = 0; h < kGroup; ++h) {
+            for (int h = 0; h < kMost; ++h) {
               if (h >= depth) break;
-              const uint64_t a = tile_desc<TOKENS>(at[h]), b = tile_desc<TOKENS>(at[h] + 3 * kTermBytes);
+              const uint64_t a = tile_desc<TOKENS, C::kUnits>(at[h]), b = tile_desc<TOKENS, C::kUnits>(at[h] + TERMS * C::kTermBytes);
 #pragma unroll
-              for (int k = 0; k < kDepth / 16; ++k)
-                mma_f16<N, TOKENS>(tmem + ab * N, a + (uint64_t)(t * (kTermBytes >> 4) + k * kStep16<TOKENS>), b + (uint64_t)(k * kStep16<TOKENS>), h > 0 || k > 0 || t < 2);
+              for (int k = 0; k < C::kUnits * kDepth / 16; ++k)
+                mma_f16<N, TOKENS>(tmem + ab * N, a + (uint64_t)(t * (C::kTermBytes >> 4) + k * kStep16<TOKENS>), b + (uint64_t)(k * kStep16<TOKENS>), h > 0 || k > 0 || t < TERMS - 1);
             }
 #pragma unroll
-          for (int h = 0; h < kGroup; ++h)
+          for (int h = 0; h < kMost; ++h)
             if (h < depth) commit_to(freed[h]);
           commit_to(acc_full(ab));
         }
@@ -380,6 +394,7 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
     }
   } else {
     const int quad = warp & 3, half = (warp - 2) >> 2;      // rows 32 quad .., columns kCols half ..
+    const int r = quad * 32 + lane;             // the thread's row of the tile
     uint32_t group = 0;
     bool ok = true, odd = false;        // odd: some sum of this thread is not finite
     for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
@@ -390,8 +405,8 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
       for (int n = 0; n < kCols; ++n) acc[n] = 0.0f;
       for (; u < u_end; u += p.group, ++group) {
         const int ab = group & 1;
-        if (!bar_wait(acc_full(ab), (group >> 1) & 1, p.polls)) { ok = false; break; }
-        __syncwarp();
+        ok = __all_sync(0xffffffffu, bar_wait(acc_full(ab), (group >> 1) & 1, p.polls));
+        if (!ok) break;
         tc_after();
         const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + ab * N + half * kCols;
         uint32_t v[2][16];
@@ -414,37 +429,49 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
         }
       }
       if (!ok) break;
-      const int row = row0 + quad * 32 + lane, cb = col0 + half * kCols;
+      const int cb = col0 + half * kCols;
       float* out = p.out + (int64_t)split * p.part;
-      uint32_t most = 0;                        // twice the largest magnitude's bits
+      constexpr bool kFactor = TERMS == 1 || (!TOKENS && G32);
+      float row_factor = 1.0f;
+      if (TERMS == 1) row_factor = __ldg(p.factor + (((uint32_t)(p.row_first + row0) / 128 * p.src.nbc) >> p.src.log2_K));
+      float2 zero = make_float2(0.0f, 0.0f);    // times 0: NaN where a sum is not finite
 #pragma unroll
-      for (int k = 0; k < kCols / 16; ++k) {
-        if (cb + 16 * k >= p.cols) break;
-        float f = 1.0f;
-        if (!TOKENS && G32) f = __ldg(p.col_factor + (((uint32_t)(cb + 16 * k) / 128 * p.src.nbc) >> p.src.log2_K));
-        const float big = f >= 1.0f ? f * (kScaleDown * 0.0078125f) : kScaleDown * 0.0078125f, small = f >= 1.0f ? 1.0f : f;
+      for (int k = 0; k < kCols / kOutCols; ++k) {
+        const int c0 = cb + k * kOutCols;
+        if (c0 >= p.cols) break;
+        const float f = TERMS == 1 ? row_factor : (kFactor ? __ldg(p.factor + (((uint32_t)c0 / 128 * p.src.nbc) >> p.src.log2_K)) : 1.0f);
+        const float big = kFactor ? (f >= 1.0f ? f * (kScaleDown * 0.0078125f) : kScaleDown * 0.0078125f) : kScaleDown, small = f >= 1.0f ? 1.0f : f;
 #pragma unroll
-        for (int n = 16 * k; n < 16 * k + 16; ++n) {
-          acc[n] = !TOKENS && G32 ? acc[n] * big * small : acc[n] * kScaleDown;
-          most = max(most, __float_as_uint(acc[n]) << 1);
+        for (int n = kOutCols * k; n < kOutCols * (k + 1); n += 2) {
+          zero = __ffma2_rn(make_float2(acc[n], acc[n + 1]), make_float2(0.0f, 0.0f), zero);
+          float2 v = __fmul2_rn(make_float2(acc[n], acc[n + 1]), make_float2(big, big));
+          if (kFactor) v = __fmul2_rn(v, make_float2(small, small));
+          acc[n] = v.x; acc[n + 1] = v.y;
         }
-        if (row < p.rows) {
-          if (kLanes) {
+        const float* v = acc + kOutCols * k;
+        if (row0 + r >= p.rows) continue;
+        if constexpr (kLanes) {
+          float* to = out + (int64_t)c0 * p.ld + row0 + r;
+          if (c0 + kOutCols <= p.cols) {
 #pragma unroll
-            for (int n = 16 * k; n < 16 * k + 16; ++n)
-              if (cb + n < p.cols) out[(int64_t)(cb + n) * p.ld + row] = acc[n];
+            for (int n = 0; n < kOutCols; ++n, to += p.ld) *to = v[n];
           } else {
 #pragma unroll
-            for (int n = 16 * k; n < 16 * k + 16; n += 4)
-              if (cb + n < p.cols) *reinterpret_cast<float4*>(out + (int64_t)row * p.ld + cb + n) = make_float4(acc[n], acc[n + 1], acc[n + 2], acc[n + 3]);
+            for (int n = 0; n < kOutCols; ++n, to += p.ld)
+              if (c0 + n < p.cols) *to = v[n];
           }
+        } else {
+          float* to = out + (int64_t)(row0 + r) * p.ld + c0;
+#pragma unroll
+          for (int n = 0; n < kOutCols; n += 4)
+            if (c0 + n < p.cols) *reinterpret_cast<float4*>(to + n) = make_float4(v[n], v[n + 1], v[n + 2], v[n + 3]);
         }
       }
-      odd |= row < p.rows && most >= 2 * 0x7f800000u;
+      odd |= row0 + r < p.rows && !(zero.x + zero.y == 0.0f);
     }
     // Sums that are not finite are made again when the CTA's tiles are done: nothing waits for these warps any more, however long it takes
     // (with all of a long contraction's sums to make, longer than a bounded wait lasts).
-    if (__all_sync(0xffffffffu, ok) && __any_sync(0xffffffffu, odd)) {
+    if (__any_sync(0xffffffffu, ok && odd)) {
 #pragma unroll 1
       for (int w = blockIdx.x; w < items; w += gridDim.x) {
         int row0, col0, u, u_end;
@@ -467,14 +494,14 @@ using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, voi
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 // planes of [outer, inner] bf16
-int make_map(CUtensorMap* map, const void* base, int64_t inner, int64_t outer, int64_t ld, int64_t planes, int64_t plane, int box_inner, int box_outer, bool tokens) {
+int make_map(CUtensorMap* map, const void* base, int64_t inner, int64_t outer, int64_t ld, int64_t planes, int64_t plane, int box_inner, int box_outer) {
   EncodeFn encode = reinterpret_cast<EncodeFn>(tensor_map_encoder());
   if (!encode) return fail(PB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   const cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)outer, (cuuint64_t)planes};
   const cuuint64_t strides[2] = {(cuuint64_t)(ld * 2), (cuuint64_t)(plane * 2)};
   const cuuint32_t box[3] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer, 1}, step[3] = {1, 1, 1};
   const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            tokens ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                            box_inner == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(PB_ERR_CUDA, "cuTensorMapEncodeTiled (split dot) failed with CUresult %d", (int)r);
   return PB_OK;
 }
@@ -484,22 +511,22 @@ std::atomic<uint32_t> g_split_polls{kWaitPolls};
 std::atomic<int> g_split_withhold{0};
 #endif
 
-template <int N, bool TOKENS, bool G32>
+template <int N, bool TOKENS, bool G32, int TERMS>
 int launch(const CUtensorMap& terms, const CUtensorMap& other, const SplitParams& p, cudaStream_t st) {
-  PB_CUDA_TRY(cudaFuncSetAttribute(split_dot_kernel<N, TOKENS, G32>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<N>::kSmem));      // per device
+  PB_CUDA_TRY(cudaFuncSetAttribute(split_dot_kernel<N, TOKENS, G32, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<N, TOKENS, G32, TERMS>::kSmem));      // per device
   const int items = p.tiles * p.splits;
-  split_dot_kernel<N, TOKENS, G32><<<items < sm_count() ? items : sm_count(), kThreads, Cfg<N>::kSmem, st>>>(terms, other, p);
+  split_dot_kernel<N, TOKENS, G32, TERMS><<<items < sm_count() ? items : sm_count(), kThreads, Cfg<N, TOKENS, G32, TERMS>::kSmem, st>>>(terms, other, p);
   PB_LAUNCH_CHECK("split_dot_kernel");
   return PB_OK;
 }
-template <bool TOKENS, bool G32>
+template <bool TOKENS, bool G32, int TERMS>
 int launch_n(int n, const CUtensorMap& terms, const CUtensorMap& other, const SplitParams& p, cudaStream_t st) {
-  if (n == 256) return launch<256, TOKENS, G32>(terms, other, p, st);
-  return n == 192 ? launch<192, TOKENS, G32>(terms, other, p, st) : launch<128, TOKENS, G32>(terms, other, p, st);
+  if (n == 256) return launch<256, TOKENS, G32, TERMS>(terms, other, p, st);
+  return n == 192 ? launch<192, TOKENS, G32, TERMS>(terms, other, p, st) : launch<128, TOKENS, G32, TERMS>(terms, other, p, st);
 }
-template <bool TOKENS, bool G32>
+template <bool TOKENS, bool G32, int TERMS>
 int launch_prepare(const PrepareParams& p, cudaStream_t st) {
-  split_prepare_kernel<TOKENS, G32><<<p.q_blocks + (G32 ? (p.n_g + 255) / 256 : 0), 256, 0, st>>>(p);
+  split_prepare_kernel<TOKENS, G32, TERMS><<<p.q_blocks + (G32 ? (p.n_g + 255) / 256 : 0), 256, 0, st>>>(p);
   PB_LAUNCH_CHECK("split_prepare_kernel");
   return PB_OK;
 }
@@ -511,8 +538,11 @@ int launch_prepare(const PrepareParams& p, cudaStream_t st) {
 // dW, 1024 x 1024: 64 rows 8.3 | 8.7, 200 13.5 | 10.8, 3000 52 | 33; 2048 x 2048: 64 rows 15.0 | 13.5, 3000 178 | 68; f32 174 | 79;
 // 4096 x 512: 100 rows 10.1 | 10.6, 200 14.2 | 12.1.  Operands that one tile uses: 8192 rows, 2048 x 128, f32 35.5 | 32.5, bf16
 // 36.6 | 42.8; 128 x 2048, f32 35.6 | 48.4.
-bool split_dot_pays(int tokens, int64_t I, int64_t J, int64_t C) {
+// One term (a bf16 cotangent's dX): 2048 x 2048 64 rows 12.5 | 12.7, 150 rows 16.6 | 14.5, 1000 rows 39 | 22; 4096 x 1024 100 rows 12.3 | 12.5, 1000 rows
+// 41 | 18; 1024 x 1024 64 rows 11.5 | 10.4; 128 x 2048 64 rows 11.1 | 9.7; 8192 x 2048 64 rows 24.4 | 23.4, 2000 rows 275 | 86.
+bool split_dot_pays(int tokens, bool exact, int64_t I, int64_t J, int64_t C) {
   const double products = (double)I * (double)J * (double)C;
+  if (exact) return J > 128 || I * C <= (1ll << 21);
   if (I < 512 || J < 512) return false;
   if (tokens) return C >= 192 || products >= 0x1p28;
   return products >= 0x1p29 && J >= 192;
@@ -543,14 +573,15 @@ bool split_dot_plan(int tokens, int64_t rows, int64_t cols, int a, int b, int64_
   d->log2_K = log2_of(geo.K); d->nbc = (int)geo.nbc;
   d->units = (int)((C + kDepth - 1) / kDepth);
   // The three-term operand's rows are the tile's 128, the other's columns its N.
-  const int64_t R = g_bf16 ? I : J, S = g_bf16 ? J : I, row_bytes = 6 * (int64_t)d->variants * C;
+  d->exact = g_bf16 && !tokens && b == 128 && geo.K % geo.nbc == 0;      // a factor per 128 of i
+  const int64_t R = g_bf16 ? I : J, S = g_bf16 ? J : I, row_bytes = (d->exact ? 2 : 6) * (int64_t)d->variants * C;
   d->slab = std::min(R, std::max<int64_t>(1024, (int64_t)kMaxTerms / row_bytes / 1024 * 1024));
   d->row_tiles = (int)((d->slab + kTermRows - 1) / kTermRows);
   const int sms = sm_count();
   int64_t best = -1;
   for (int n : {256, 192, 128}) {
     if (d->variants > 1 && I / d->variants % n != 0) continue;      // a tile's columns share their set of terms
-    const int64_t tiles = d->row_tiles * ((S + n - 1) / n), waves = (tiles + sms - 1) / sms, cost = waves * n;
+    const int64_t tiles = d->row_tiles * ((S + n - 1) / n), waves = (tiles + sms - 1) / sms, cost = waves * (d->exact ? n + kTermRows : n);
     if (best < 0 || cost < best) { best = cost; d->n = n; d->tiles = (int)tiles; }
     if (tiles > kMaxIndexed / 64) return false;
   }
@@ -563,7 +594,7 @@ bool split_dot_plan(int tokens, int64_t rows, int64_t cols, int a, int b, int64_
   d->off_other = align((size_t)row_bytes * d->slab);
   d->off_parts = d->off_other + (g_bf16 ? 0 : align((size_t)rows * cols * 2));
   d->bytes = d->off_parts + (d->splits > 1 ? (size_t)d->splits * I * J * 4 : 0);
-  return split_dot_pays(tokens, I, J, C);
+  return split_dot_pays(tokens, d->exact, I, J, C);
 }
 
 int split_dot_run(const SplitDotPlan& d, int tokens, const uint8_t* q, const uint8_t* sc8, const float* sc32, int64_t rows, int64_t cols, int a, int b,
@@ -595,37 +626,39 @@ int split_dot_run(const SplitDotPlan& d, int tokens, const uint8_t* q, const uin
     pp.q_vecs = FastDiv((uint32_t)(q_cols / 16));
     pp.n_q = g_bf16 || r0 == 0 ? (uint32_t)(q_rows * q_cols / 16) : 0u;      // the exact values serve all rounds
     pp.q_blocks = (pp.n_q + 255) / 256;
-    if (int s = g_bf16 ? launch_prepare<false, false>(pp, st) : (tokens ? launch_prepare<true, true>(pp, st) : launch_prepare<false, true>(pp, st))) return s;
+    if (int s = d.exact ? launch_prepare<false, false, 1>(pp, st) : g_bf16 ? launch_prepare<false, false, 3>(pp, st) : (tokens ? launch_prepare<true, true, 3>(pp, st) : launch_prepare<false, true, 3>(pp, st))) return s;
 
     CUtensorMap terms, other;
     const void* other_at = g_bf16 ? g : static_cast<const void*>(q_exact);
-    const int64_t planes = 3 * (int64_t)d.variants, plane = tr * C;
+    const int64_t planes = (d.exact ? 1 : 3) * (int64_t)d.variants, plane = tr * C;
+    const int deep = d.exact ? 2 * kDepth : kDepth;       // c per stage
     if (tokens) {
-      if (int s = make_map(&terms, terms_at, tr, C, tr, planes, plane, 64, kDepth, true)) return s;
-      if (int s = make_map(&other, other_at, oc, C, oc, 1, oc * C, 64, kDepth, true)) return s;
+      if (int s = make_map(&terms, terms_at, tr, C, tr, planes, plane, 64, kDepth)) return s;
+      if (int s = make_map(&other, other_at, oc, C, oc, 1, oc * C, 64, kDepth)) return s;
     } else {
-      if (int s = make_map(&terms, terms_at, C, tr, C, planes, plane, kDepth, kTermRows, false)) return s;
-      if (int s = make_map(&other, other_at, C, oc, C, 1, oc * C, kDepth, d.n, false)) return s;
+      if (int s = make_map(&terms, terms_at, C, tr, C, planes, plane, deep, kTermRows)) return s;
+      if (int s = make_map(&other, other_at, C, oc, C, 1, oc * C, deep, d.n)) return s;
     }
     SplitParams p{};
     p.src = DotSource{q, sc8, sc32, g, cols, tokens ? J : C, (uint32_t)d.nbc, (uint32_t)d.log2_K, (uint32_t)log2_of(a), (uint32_t)log2_of(b), (int)C};
     p.ld = tokens ? J : I;
     p.out = d.splits > 1 ? parts : out + (g_bf16 ? (tokens ? r0 * J : r0) : (tokens ? r0 : r0 * I));
     p.part = I * J;
-    p.col_factor = sc32;
+    p.factor = sc32;
     p.rows = (int)tr; p.cols = (int)oc;
     p.row_first = (int)r0;
     p.row_tiles = (int)((tr + kTermRows - 1) / kTermRows);
     p.tiles = p.row_tiles * (int)((oc + d.n - 1) / d.n);
     p.splits = d.splits; p.units = d.units; p.units_per_split = d.units_per_split;
     p.cols_per_variant = (int)(I / d.variants);
-    p.group = g_bf16 && C < kShortDepth ? 1 : kGroup;
+    p.group = g_bf16 && !d.exact && C < kShortDepth ? 1 : kGroup;
     p.polls = kWaitPolls;
 #ifdef PB_DIAGNOSTICS
     p.polls = g_split_polls.load(); p.withhold = g_split_withhold.load();
 #endif
-    const int status = tokens ? (g_bf16 ? launch_n<true, false>(d.n, terms, other, p, st) : launch_n<true, true>(d.n, terms, other, p, st))
-                              : (g_bf16 ? launch_n<false, false>(d.n, terms, other, p, st) : launch_n<false, true>(d.n, terms, other, p, st));
+    const int status = d.exact ? launch_n<false, false, 1>(d.n, terms, other, p, st)
+                     : tokens ? (g_bf16 ? launch_n<true, false, 3>(d.n, terms, other, p, st) : launch_n<true, true, 3>(d.n, terms, other, p, st))
+                              : (g_bf16 ? launch_n<false, false, 3>(d.n, terms, other, p, st) : launch_n<false, true, 3>(d.n, terms, other, p, st));
     if (status) return status;
     if (d.splits > 1)         // there is one round then
       if (int s = add_parts(parts, out, I * J, d.splits, st)) return s;

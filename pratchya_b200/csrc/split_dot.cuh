@@ -13,6 +13,7 @@ constexpr size_t kSplitAlign = 32;    // of the workspace: the terms are stored 
 struct SplitDotPlan {
   int n, tiles, row_tiles, splits, units, units_per_split, variants, nbc, log2_K;
   int64_t slab;                       // rows of the three-term operand at a time
+  bool exact;                         // that operand is one term: the fp8 values times their block's power of two
   size_t off_other, off_parts, bytes; // of the workspace, which starts with the terms
 };
 // False where dense_dot_kernel takes the call: shapes this form does not take, and those it is not faster for.

@@ -212,3 +212,20 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_launch_is_clean(built_lib
     after, _ = _dot(diag_lib, tokens, triple, grid, g)
     assert diag_lib.pb_gemm_check(st) == 0 and torch.equal(before, after)
     assert built_lib.pb_gemm_check(st) == 0
+
+
+@pytest.mark.parametrize("rows,cols,free,amp", [(128, 128, 1, 1.0), (128, 2048, 63, 1.0), (512, 512, 5, 1.0), (1024, 1024, 64, 1e-30), (2048, 2048, 129, 1.0), (8192, 4096, 150, 1.0), (384, 2048, 1000, 1e30),
+                                                (640, 640, 200, 1.0), (1152, 896, 333, 1.0), (2048, 1024, 2400, 1.0)])
+def test_one_term_for_a_bf16_cotangent(built_lib, rows, cols, free, amp):
+    """dX of a bf16 cotangent: the fp8 values times their powers of two, the super-group's factor on the finished sums (of one group, of
+    two, of one per row of blocks; 640 and 1152 rows: groups that end inside a row, three terms), few tokens and no whole tile of them."""
+    triple, g = _inputs(rows, cols, (128, 128), free, 0, BF16, amp)
+    got, _ = _dot(built_lib, 0, triple, (128, 128), g)
+    plain, _ = _dot(built_lib, 0, triple, (128, 128), g, best=False)
+    a, b = _sums(0, triple, (128, 128), g)
+    want, bound = a @ b, _bound(a, b)
+    assert ((got.double() - want).abs() <= bound + 1e-37).all()
+    if amp == 1.0:
+        assert (got.double() - want).norm() <= (plain.double() - want).norm() * 1.02
+    assert torch.equal(got, _dot(built_lib, 0, triple, (128, 128), g)[0])
+    assert built_lib.pb_gemm_check(torch.cuda.current_stream().cuda_stream) == 0
