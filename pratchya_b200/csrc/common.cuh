@@ -25,6 +25,21 @@ int fail(int status, const char* fmt, ...);
       return ::pb::fail(PB_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(_e)); \
   } while (0)
 
+// Launched behind the kernel before it on the stream: the grid is set up while that one's last CTAs finish, and its threads go on past
+// grid_wait(), which every kernel launched this way begins with, when all of that one's memory operations have been performed.
+template <typename... Params, typename... Args>
+cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid; config.blockDim = block; config.dynamicSmemBytes = smem; config.stream = st;
+  cudaLaunchAttribute behind;
+  behind.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  behind.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &behind;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 #define PB_LAUNCH_CHECK(name)                                                      \
   do {                                                                             \
     cudaError_t _e = cudaGetLastError();                                           \

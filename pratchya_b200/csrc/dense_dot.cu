@@ -245,6 +245,7 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
   __syncthreads();
   tc_after();
   const uint32_t tmem = *(volatile uint32_t*)&tmem_slot;
+  grid_wait();
 
   if (warp < kConvWarps) {
     // a thread's chunks: TOKENS, eight j of rows c = (tid >> 4) + 16 k; else eight c of rows j = (tid >> 3) + 32 k
@@ -500,6 +501,7 @@ __global__ void __launch_bounds__(kDotThreads, 1) dense_dot_kernel(const __grid_
 }
 
 __global__ void __launch_bounds__(256) add_parts_kernel(const float4* parts, float4* out, int64_t n4, int splits) {
+  grid_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= n4) return;
   float4 s = parts[i];
@@ -536,7 +538,7 @@ std::atomic<int> g_dot_withhold{0};
 template <bool TOKENS, typename G>
 int launch_dot(const DotParams& p, unsigned grid, cudaStream_t st) {
   PB_CUDA_TRY(cudaFuncSetAttribute(dense_dot_kernel<TOKENS, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDotSmem));      // per device
-  dense_dot_kernel<TOKENS, G><<<grid, kDotThreads, kDotSmem, st>>>(p);
+  launch_behind(dense_dot_kernel<TOKENS, G>, grid, kDotThreads, kDotSmem, st, p);
   PB_LAUNCH_CHECK("dense_dot_kernel");
   return PB_OK;
 }
@@ -551,7 +553,7 @@ bool dot_shape_ok(int tokens, int64_t rows, int64_t cols, int a, int b, int64_t 
 
 int add_parts(const float* parts, float* out, int64_t n, int splits, cudaStream_t st) {
   const int64_t n4 = n / 4;
-  add_parts_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4*>(parts), reinterpret_cast<float4*>(out), n4, splits);
+  launch_behind(add_parts_kernel, (unsigned)((n4 + 255) / 256), 256, 0, st, reinterpret_cast<const float4*>(parts), reinterpret_cast<float4*>(out), n4, splits);
   PB_LAUNCH_CHECK("add_parts_kernel");
   return PB_OK;
 }

@@ -69,6 +69,7 @@ template <typename OutT, int FMT, int VEC>
 __global__ void __launch_bounds__(256)
 dequantize_kernel(const uint8_t* __restrict__ q, const uint8_t* __restrict__ sc8, const float* __restrict__ sc32,
                   OutT* __restrict__ out, DqDims d) {
+  grid_wait();
   const uint32_t stride = gridDim.x * blockDim.x;
   if constexpr (VEC == 16) {
     // two 16-byte vectors per iteration: both loads (and their scale lookups) are in flight together
@@ -99,6 +100,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(256)
 dequantize_bwd_kernel(const T* __restrict__ g, const uint8_t* __restrict__ sc8, const float* __restrict__ sc32,
                       T* __restrict__ out, DqDims d) {
+  grid_wait();
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < d.total_vecs; i += stride) {
     const float x_sc = block_multiplier(d, sc8, sc32, i);
@@ -115,6 +117,7 @@ template <typename OutT, int FMT>
 __global__ void __launch_bounds__(256)
 dequantize_row128_kernel(const uint4* __restrict__ q, const uint8_t* __restrict__ sc8, const float* __restrict__ sc32,
                          OutT* __restrict__ out, int64_t n_groups) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * 8;
   int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -196,7 +199,7 @@ int launch_dq(const uint8_t* q, const uint8_t* sc8, const float* sc32, OutT* out
   if (vec16 && g.a == 1 && g.b == 128 && g.K == 8) {
     const int64_t n_groups = batch * g.M;
     const int64_t need = (n_groups + 7) / 8, cap = (int64_t)sm_count() * 16;
-    dequantize_row128_kernel<OutT, FMT><<<(int)(need < cap ? need : cap), 256, 0, st>>>((const uint4*)q, sc8, sc32, out, n_groups);
+    launch_behind(dequantize_row128_kernel<OutT, FMT>, (int)(need < cap ? need : cap), 256, 0, st, (const uint4*)q, sc8, sc32, out, n_groups);
     PB_LAUNCH_CHECK("dequantize_row128_kernel");
     return PB_OK;
   }
@@ -204,8 +207,8 @@ int launch_dq(const uint8_t* q, const uint8_t* sc8, const float* sc32, OutT* out
   if (total / vec > kMaxIndexed || batch * g.rows > kMaxIndexed)
     return fail(PB_ERR_UNSUPPORTED, "pb_dequantize: %lld elements exceed the 31-bit index range of this kernel", (long long)total);
   DqDims d{VecIndexer(g.cols, g.a, g.b, vec), FastDiv((uint32_t)g.K), (uint32_t)(total / vec)};
-  if (vec16) dequantize_kernel<OutT, FMT, 16><<<dq_grid(d.total_vecs), 256, 0, st>>>(q, sc8, sc32, out, d);
-  else       dequantize_kernel<OutT, FMT, 1><<<dq_grid(d.total_vecs), 256, 0, st>>>(q, sc8, sc32, out, d);
+  if (vec16) launch_behind(dequantize_kernel<OutT, FMT, 16>, dq_grid(d.total_vecs), 256, 0, st, q, sc8, sc32, out, d);
+  else       launch_behind(dequantize_kernel<OutT, FMT, 1>, dq_grid(d.total_vecs), 256, 0, st, q, sc8, sc32, out, d);
   PB_LAUNCH_CHECK("dequantize_kernel");
   return PB_OK;
 }
@@ -295,11 +298,11 @@ extern "C" int pb_dequantize_bwd(const void* gin, int dtype, const uint8_t* sc8,
   DqDims d{VecIndexer(g.cols, g.a, g.b, vec), FastDiv((uint32_t)g.K), (uint32_t)(total / vec)};
   const int grid = dq_grid(d.total_vecs);
   if (dtype == PB_F32) {
-    if (vec4) dequantize_bwd_kernel<float, 4><<<grid, 256, 0, st>>>((const float*)gin, sc8, sc32, (float*)out, d);
-    else      dequantize_bwd_kernel<float, 1><<<grid, 256, 0, st>>>((const float*)gin, sc8, sc32, (float*)out, d);
+    if (vec4) launch_behind(dequantize_bwd_kernel<float, 4>, grid, 256, 0, st, (const float*)gin, sc8, sc32, (float*)out, d);
+    else      launch_behind(dequantize_bwd_kernel<float, 1>, grid, 256, 0, st, (const float*)gin, sc8, sc32, (float*)out, d);
   } else {
-    if (vec4) dequantize_bwd_kernel<__nv_bfloat16, 4><<<grid, 256, 0, st>>>((const __nv_bfloat16*)gin, sc8, sc32, (__nv_bfloat16*)out, d);
-    else      dequantize_bwd_kernel<__nv_bfloat16, 1><<<grid, 256, 0, st>>>((const __nv_bfloat16*)gin, sc8, sc32, (__nv_bfloat16*)out, d);
+    if (vec4) launch_behind(dequantize_bwd_kernel<__nv_bfloat16, 4>, grid, 256, 0, st, (const __nv_bfloat16*)gin, sc8, sc32, (__nv_bfloat16*)out, d);
+    else      launch_behind(dequantize_bwd_kernel<__nv_bfloat16, 1>, grid, 256, 0, st, (const __nv_bfloat16*)gin, sc8, sc32, (__nv_bfloat16*)out, d);
   }
   PB_LAUNCH_CHECK("dequantize_bwd_kernel");
   return PB_OK;

@@ -517,6 +517,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (C::kMaxSplit > 1 && p.splitk > 1) cluster_sync_all();      // rank 0's barrier is there before any other rank signals it
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_wait();
 
   const int num_tiles = p.tiles_m * p.tiles_n;
   // The ranks of a cluster share a tile, p.split_chunks chunks of its contraction each.
@@ -899,6 +900,7 @@ gemm_tn_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   cluster_sync_all();          // both CTAs' barriers are initialised before any remote signal
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_wait();
 
   const int num_tiles = p.tiles_m * p.tiles_n;          // 256 x 224 tiles
   const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
@@ -1193,6 +1195,7 @@ struct PrepPair {
 };
 
 __global__ void __launch_bounds__(256) gemm_prep_kernel(const __grid_constant__ PrepPair pair) {
+  grid_wait();
   const bool second = blockIdx.x >= pair.first;
   const PrepParams& q = pair.q[second];
   const unsigned block = second ? blockIdx.x - pair.first : blockIdx.x, blocks = second ? gridDim.x - pair.first : pair.first;
@@ -1517,7 +1520,7 @@ unsigned prep_blocks(const PrepParams& q) {
 // `a`, `b`: the operands to prepare; either may be null, not both
 int launch_prep(const PrepParams* a, const PrepParams* b, cudaStream_t st) {
   PrepPair pair{{a ? *a : *b, b ? *b : *a}, a ? prep_blocks(*a) : 0u};
-  gemm_prep_kernel<<<pair.first + (b ? prep_blocks(*b) : 0u), 256, 0, st>>>(pair);
+  launch_behind(gemm_prep_kernel, pair.first + (b ? prep_blocks(*b) : 0u), 256, 0, st, pair);
   PB_LAUNCH_CHECK("gemm_prep_kernel");
   return PB_OK;
 }
@@ -1541,11 +1544,13 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
   config.blockDim = dim3(Cfg<BN>::kThreads);
   config.dynamicSmemBytes = Cfg<BN>::smem_bytes(p.splitk == 1 ? 0 : (p.add_sums ? 1 : p.nchunks - p.split_chunks));
   config.stream = st;
-  cudaLaunchAttribute cluster;
-  cluster.id = cudaLaunchAttributeClusterDimension;
-  cluster.val.clusterDim.x = (unsigned)p.splitk; cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-  config.attrs = &cluster;
-  config.numAttrs = p.splitk > 1 ? 1 : 0;
+  cudaLaunchAttribute attrs[2];           // see launch_behind
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = (unsigned)p.splitk; attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+  config.attrs = attrs;
+  config.numAttrs = p.splitk > 1 ? 2 : 1;
   PB_CUDA_TRY(cudaLaunchKernelEx(&config, gemm_tn_kernel<BN, PROF, UNI>, ma, mb, md, p));
   PB_LAUNCH_CHECK("gemm_tn_kernel");
   return PB_OK;
@@ -1574,7 +1579,7 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
   const int tiles = p.tiles_m * p.tiles_n * p.splitk;
   const int pairs = sm_count() / 2;
   const int grid = 2 * (tiles < pairs ? tiles : pairs);
-  gemm_tn_pair_kernel<PROF, UNI><<<grid, Cfg2::kThreads, Cfg2::kSmemBytes, st>>>(ma, mb, msfa, msfb, md, p);
+  PB_CUDA_TRY(launch_behind(gemm_tn_pair_kernel<PROF, UNI>, grid, Cfg2::kThreads, Cfg2::kSmemBytes, st, ma, mb, msfa, msfb, md, p));
   PB_LAUNCH_CHECK("gemm_tn_pair_kernel");
   return PB_OK;
 }

@@ -58,6 +58,7 @@ __device__ __forceinline__ float top4(const float4& v) { return fmaxf(fmaxf(v.x,
 template <int THREADS, int PER_SM>
 __global__ void __launch_bounds__(THREADS, PER_SM) smoothed_xent_fwd_kernel(const float* logits, const int64_t* target, const float* weight,
                                                                    float* row_loss, float* lse, int64_t vocab, float alpha) {
+  grid_wait();
   __shared__ float red[3][THREADS / 32];
   const int64_t row = blockIdx.x;
   const float4* z4 = reinterpret_cast<const float4*>(logits + row * vocab);
@@ -99,6 +100,7 @@ template <int THREADS>
 __global__ void __launch_bounds__(THREADS) smoothed_xent_bwd_kernel(const float* logits, const int64_t* target, const float* weight,
                                                                    const float* lse, const float* upstream, float inv_denominator,
                                                                    float* dlogits, int64_t vocab, float alpha) {
+  grid_wait();
   const int64_t row = blockIdx.x;
   const float* z = logits + row * vocab;
   float* dz = dlogits + row * vocab;
@@ -141,11 +143,11 @@ extern "C" int pb_smoothed_xent(const float* logits, const int64_t* target, cons
   // eight CTAs on an SM (32 registers) where no thread has a whole round of loads, six otherwise: 4096 rows, 2048 logits 12.1 us with
   // six and 11.5 with eight, 65536 logits 157 and 161
   if (wide_forward(rows, vocab))
-    smoothed_xent_fwd_kernel<kWideThreads, 1><<<(unsigned)rows, kWideThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
+    launch_behind(smoothed_xent_fwd_kernel<kWideThreads, 1>, (unsigned)rows, kWideThreads, 0, st, logits, target, weight, row_loss, lse, vocab, alpha);
   else if (vocab < kLossThreads * kLoads * 4)
-    smoothed_xent_fwd_kernel<kLossThreads, 8><<<(unsigned)rows, kLossThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
+    launch_behind(smoothed_xent_fwd_kernel<kLossThreads, 8>, (unsigned)rows, kLossThreads, 0, st, logits, target, weight, row_loss, lse, vocab, alpha);
   else
-    smoothed_xent_fwd_kernel<kLossThreads, 6><<<(unsigned)rows, kLossThreads, 0, st>>>(logits, target, weight, row_loss, lse, vocab, alpha);
+    launch_behind(smoothed_xent_fwd_kernel<kLossThreads, 6>, (unsigned)rows, kLossThreads, 0, st, logits, target, weight, row_loss, lse, vocab, alpha);
   PB_LAUNCH_CHECK("smoothed_xent_fwd_kernel");
   return PB_OK;
 }
@@ -159,9 +161,9 @@ extern "C" int pb_smoothed_xent_bwd(const float* logits, const int64_t* target, 
     return fail(PB_ERR_MISALIGNED, "pb_smoothed_xent_bwd: logits and dlogits must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (wide_backward(rows, vocab))
-    smoothed_xent_bwd_kernel<kWideThreads><<<(unsigned)rows, kWideThreads, 0, st>>>(logits, target, weight, lse, upstream, 1.0f / denominator, dlogits, vocab, alpha);
+    launch_behind(smoothed_xent_bwd_kernel<kWideThreads>, (unsigned)rows, kWideThreads, 0, st, logits, target, weight, lse, upstream, 1.0f / denominator, dlogits, vocab, alpha);
   else
-    smoothed_xent_bwd_kernel<kLossThreads><<<(unsigned)rows, kLossThreads, 0, st>>>(logits, target, weight, lse, upstream, 1.0f / denominator, dlogits, vocab, alpha);
+    launch_behind(smoothed_xent_bwd_kernel<kLossThreads>, (unsigned)rows, kLossThreads, 0, st, logits, target, weight, lse, upstream, 1.0f / denominator, dlogits, vocab, alpha);
   PB_LAUNCH_CHECK("smoothed_xent_bwd_kernel");
   return PB_OK;
 }

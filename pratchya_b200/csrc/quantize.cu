@@ -85,6 +85,7 @@ template <int FMT, int MINB, bool PREP>
 __global__ void __launch_bounds__(kRowThreads, MINB)
 quantize_row128_bf16_wide_kernel(const uint8_t* __restrict__ x, uint4* __restrict__ q,
                                  uint8_t* __restrict__ sc8, float* __restrict__ sc32, int64_t n_groups, const GemmPrepOut prep) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * (kRowThreads / 32);
   for (int64_t g = (int64_t)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); g < n_groups; g += warps_total) {
@@ -142,6 +143,7 @@ template <int FMT, int MINB, bool PREP>
 __global__ void __launch_bounds__(kRowThreads, MINB)
 quantize_row128_bf16_kernel(const uint4* __restrict__ x, uint2* __restrict__ q,
                             uint8_t* __restrict__ sc8, float* __restrict__ sc32, int64_t n_groups, const GemmPrepOut prep) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * (kRowThreads / 32);
   for (int64_t g = (int64_t)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); g < n_groups; g += warps_total) {
@@ -203,6 +205,7 @@ template <int FMT, bool PREP>
 __global__ void __launch_bounds__(kRowThreads)
 quantize_row128_f32_kernel(const float4* __restrict__ x, uint32_t* __restrict__ q,
                            uint8_t* __restrict__ sc8, float* __restrict__ sc32, int64_t n_groups, const GemmPrepOut prep) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * (kRowThreads / 32);
   for (int64_t g = (int64_t)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); g < n_groups; g += warps_total) {
@@ -356,6 +359,7 @@ template <int FMT, typename OutT, bool SCALES>
 __global__ void __launch_bounds__(kRowThreads)
 fake_quantize_row128_f32_kernel(const float4* __restrict__ x, typename Out4<OutT>::vec* __restrict__ out, uint8_t* __restrict__ sc8,
                                 float* __restrict__ sc32, int64_t n_groups) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * (kRowThreads / 32);
   for (int64_t g = (int64_t)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); g < n_groups; g += warps_total) {
@@ -412,6 +416,7 @@ template <int FMT, bool RELU2>
 __global__ void __launch_bounds__(kRowThreads)
 scaled_quantize_row128_f32_kernel(const float4* __restrict__ g, const uint8_t* __restrict__ y_sc8, const float* __restrict__ y_sc32,
                                   uint32_t* __restrict__ q, uint8_t* __restrict__ sc8, float* __restrict__ sc32, int64_t n_groups) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * (kRowThreads / 32);
   for (int64_t gi = (int64_t)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); gi < n_groups; gi += warps_total) {
@@ -471,6 +476,7 @@ __global__ void __launch_bounds__(kRowThreads)
 shift_lerp_quantize_row128_kernel(const float4* __restrict__ x, const float4* __restrict__ state, const float4* __restrict__ mu,
                                   uint32_t* __restrict__ q, uint8_t* __restrict__ sc8, float* __restrict__ sc32,
                                   int64_t n_groups, int segs, int steps, int n_mix) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * (kRowThreads / 32);
   for (int64_t g = (int64_t)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); g < n_groups; g += warps_total) {
@@ -536,6 +542,7 @@ template <int FMT, bool PREP>
 __global__ void __launch_bounds__(kRowThreads)
 relu2_requantize_row128_f32_kernel(const float4* __restrict__ y, uint32_t* __restrict__ q, uint8_t* __restrict__ sc8,
                                    float* __restrict__ sc32, int64_t n_groups, const GemmPrepOut prep) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps_total = (int64_t)gridDim.x * (kRowThreads / 32);
   for (int64_t g = (int64_t)blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5); g < n_groups; g += warps_total) {
@@ -641,6 +648,7 @@ __device__ __forceinline__ void load_vec(const InT* p, float (&v)[VEC]) {
 template <typename InT, int VEC>
 __global__ void __launch_bounds__(256)
 generic_amax_kernel(const InT* __restrict__ x, int* __restrict__ amax_bits, GenericDims d) {
+  grid_wait();
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; ; i += stride) {
     // whole warps leave together: lane 0 holds the warp's smallest index
@@ -672,6 +680,7 @@ template <bool WARP_PER_GROUP>
 __global__ void __launch_bounds__(256)
 generic_scale_kernel(const uint32_t* __restrict__ amax_bits, float* __restrict__ divisor,
                      uint8_t* __restrict__ sc8, float* __restrict__ sc32, int64_t n_groups, int64_t K) {
+  grid_wait();
   if constexpr (WARP_PER_GROUP) {
     const int lane = threadIdx.x & 31;
     const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -708,9 +717,9 @@ generic_scale_kernel(const uint32_t* __restrict__ amax_bits, float* __restrict__
 // transposed quantizer).
 int launch_group_scales(const uint32_t* amax_bits, float* divisor, uint8_t* sc8, float* sc32, int64_t n_groups, int64_t K, cudaStream_t st) {
   if (K >= 32) {
-    generic_scale_kernel<true><<<(unsigned)((n_groups * 32 + 255) / 256), 256, 0, st>>>(amax_bits, divisor, sc8, sc32, n_groups, K);
+    launch_behind(generic_scale_kernel<true>, (unsigned)((n_groups * 32 + 255) / 256), 256, 0, st, amax_bits, divisor, sc8, sc32, n_groups, K);
   } else {
-    generic_scale_kernel<false><<<(unsigned)((n_groups + 255) / 256), 256, 0, st>>>(amax_bits, divisor, sc8, sc32, n_groups, K);
+    launch_behind(generic_scale_kernel<false>, (unsigned)((n_groups + 255) / 256), 256, 0, st, amax_bits, divisor, sc8, sc32, n_groups, K);
   }
   PB_LAUNCH_CHECK("generic_scale_kernel");
   return PB_OK;
@@ -722,6 +731,7 @@ template <typename InT, int VEC, int FMT>
 __global__ void __launch_bounds__(256)
 generic_apply_kernel(const InT* __restrict__ x, const float* __restrict__ divisor,
                      uint8_t* __restrict__ q, GenericDims d) {
+  grid_wait();
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < d.total_vecs; i += stride) {
     float v[VEC];
@@ -788,6 +798,7 @@ struct TallDims {
 template <typename InT, bool PER_COLUMN>
 __global__ void __launch_bounds__(32 * kTallWarps)
 tall_amax_kernel(const InT* __restrict__ x, float* __restrict__ amax, const TallDims d) {
+  grid_wait();
   constexpr int N = TallVec<InT>::kN;
   __shared__ float red[kTallWarps][32 * N];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -841,6 +852,7 @@ template <typename InT, bool PER_COLUMN, int FMT, bool FAKE>
 __global__ void __launch_bounds__(32 * kTallWarps, 4)
 tall_apply_kernel(const InT* __restrict__ x, const float* __restrict__ amax, uint8_t* __restrict__ q,
                   uint8_t* __restrict__ sc8, float* __restrict__ sc32, float* __restrict__ fake, const TallDims d) {
+  grid_wait();
   constexpr int N = TallVec<InT>::kN;
   constexpr int kMost = PER_COLUMN ? 32 * N : 32;      // blocks of a CTA
   __shared__ float divisor[kMost], multiplier[FAKE ? kMost : 1];
@@ -962,15 +974,15 @@ int launch_tall(const InT* x, const Geometry& g, int64_t batch, int fmt, uint8_t
   const unsigned grid = (unsigned)(batch * g.nbr * d.col_groups);
   const int threads = 32 * kTallWarps;
   if (g.b == 1) {
-    tall_amax_kernel<InT, true><<<grid, threads, 0, st>>>(x, amax, d);
+    launch_behind(tall_amax_kernel<InT, true>, grid, threads, 0, st, x, amax, d);
     PB_LAUNCH_CHECK("tall_amax_kernel");
-    if (fmt == PB_E4M3) tall_apply_kernel<InT, true, PB_E4M3, false><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, nullptr, d);
-    else                tall_apply_kernel<InT, true, PB_E5M2, false><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, nullptr, d);
+    if (fmt == PB_E4M3) launch_behind(tall_apply_kernel<InT, true, PB_E4M3, false>, grid, threads, 0, st, x, amax, q, sc8, sc32, nullptr, d);
+    else                launch_behind(tall_apply_kernel<InT, true, PB_E5M2, false>, grid, threads, 0, st, x, amax, q, sc8, sc32, nullptr, d);
   } else {
-    tall_amax_kernel<InT, false><<<grid, threads, 0, st>>>(x, amax, d);
+    launch_behind(tall_amax_kernel<InT, false>, grid, threads, 0, st, x, amax, d);
     PB_LAUNCH_CHECK("tall_amax_kernel");
-    if (fmt == PB_E4M3) tall_apply_kernel<InT, false, PB_E4M3, false><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, nullptr, d);
-    else                tall_apply_kernel<InT, false, PB_E5M2, false><<<grid, threads, 0, st>>>(x, amax, q, sc8, sc32, nullptr, d);
+    if (fmt == PB_E4M3) launch_behind(tall_apply_kernel<InT, false, PB_E4M3, false>, grid, threads, 0, st, x, amax, q, sc8, sc32, nullptr, d);
+    else                launch_behind(tall_apply_kernel<InT, false, PB_E5M2, false>, grid, threads, 0, st, x, amax, q, sc8, sc32, nullptr, d);
   }
   PB_LAUNCH_CHECK("tall_apply_kernel");
   return PB_OK;
@@ -983,13 +995,13 @@ int launch_tall_fake(const float* x, const Geometry& g, int64_t batch, float* ou
   const unsigned grid = (unsigned)(batch * g.nbr * d.col_groups);
   const int threads = 32 * kTallWarps;
   if (g.b == 1) {
-    tall_amax_kernel<float, true><<<grid, threads, 0, st>>>(x, amax, d);
+    launch_behind(tall_amax_kernel<float, true>, grid, threads, 0, st, x, amax, d);
     PB_LAUNCH_CHECK("tall_amax_kernel");
-    tall_apply_kernel<float, true, PB_E4M3, true><<<grid, threads, 0, st>>>(x, amax, nullptr, nullptr, nullptr, out, d);
+    launch_behind(tall_apply_kernel<float, true, PB_E4M3, true>, grid, threads, 0, st, x, amax, nullptr, nullptr, nullptr, out, d);
   } else {
-    tall_amax_kernel<float, false><<<grid, threads, 0, st>>>(x, amax, d);
+    launch_behind(tall_amax_kernel<float, false>, grid, threads, 0, st, x, amax, d);
     PB_LAUNCH_CHECK("tall_amax_kernel");
-    tall_apply_kernel<float, false, PB_E4M3, true><<<grid, threads, 0, st>>>(x, amax, nullptr, nullptr, nullptr, out, d);
+    launch_behind(tall_apply_kernel<float, false, PB_E4M3, true>, grid, threads, 0, st, x, amax, nullptr, nullptr, nullptr, out, d);
   }
   PB_LAUNCH_CHECK("tall_apply_kernel");
   return PB_OK;
@@ -1016,11 +1028,11 @@ int launch_generic(const InT* x, const Geometry& g, int64_t batch, int fmt, uint
   GenericDims d{VecIndexer(g.cols, g.a, g.b, VEC), (uint32_t)(total / VEC)};
   PB_CUDA_TRY(cudaMemsetAsync(amax_bits, 0xff, nblk * sizeof(uint32_t), st));      // -1: a block of nothing but NaNs keeps it
   const int grid = grid_for(d.total_vecs, 256, 8);
-  generic_amax_kernel<InT, VEC><<<grid, 256, 0, st>>>(x, reinterpret_cast<int*>(amax_bits), d);
+  launch_behind(generic_amax_kernel<InT, VEC>, grid, 256, 0, st, x, reinterpret_cast<int*>(amax_bits), d);
   PB_LAUNCH_CHECK("generic_amax_kernel");
   if (int s = launch_group_scales(amax_bits, divisor, sc8, sc32, batch * g.M, g.K, st)) return s;
-  if (fmt == PB_E4M3) generic_apply_kernel<InT, VEC, PB_E4M3><<<grid, 256, 0, st>>>(x, divisor, q, d);
-  else                generic_apply_kernel<InT, VEC, PB_E5M2><<<grid, 256, 0, st>>>(x, divisor, q, d);
+  if (fmt == PB_E4M3) launch_behind(generic_apply_kernel<InT, VEC, PB_E4M3>, grid, 256, 0, st, x, divisor, q, d);
+  else                launch_behind(generic_apply_kernel<InT, VEC, PB_E5M2>, grid, 256, 0, st, x, divisor, q, d);
   PB_LAUNCH_CHECK("generic_apply_kernel");
   return PB_OK;
 }
@@ -1080,7 +1092,7 @@ static int quantize_entry(const void* x, int x_dtype, int64_t batch, int64_t row
     // 40 registers per thread (6 CTAs of 256 threads per SM) measures the same as the compiler's
     // unconstrained 49; an unconstrained single CTA per SM (96 registers) is 15 % slower.
     const bool e4 = out_format == PB_E4M3;
-#define PB_ROW128_LAUNCH(KERNEL, XT, QT) KERNEL<<<grid, kRowThreads, 0, st>>>((const XT*)x, (QT*)q, sc8, sc32, n_groups, prep)
+#define PB_ROW128_LAUNCH(KERNEL, XT, QT) launch_behind(KERNEL, grid, kRowThreads, 0, st, (const XT*)x, (QT*)q, sc8, sc32, n_groups, prep)
     static const bool wide = env_switch("PB_QUANT_WIDE", 1) != 0;
     if (x_dtype == PB_BF16 && wide && (reinterpret_cast<uintptr_t>(x) & 31) == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
       if (prep.sf) {
@@ -1173,11 +1185,11 @@ extern "C" int pb_relu2_requantize(const void* y, int64_t rows, int64_t cols, in
   const int grid = grid_for(n_groups * 32, kRowThreads, 8);
   const bool e4 = out_format == PB_E4M3;
   if (prep.sf) {
-    if (e4) relu2_requantize_row128_f32_kernel<PB_E4M3, true><<<grid, kRowThreads, 0, st>>>((const float4*)y, (uint32_t*)q, sc8, sc32, n_groups, prep);
-    else    relu2_requantize_row128_f32_kernel<PB_E5M2, true><<<grid, kRowThreads, 0, st>>>((const float4*)y, (uint32_t*)q, sc8, sc32, n_groups, prep);
+    if (e4) launch_behind(relu2_requantize_row128_f32_kernel<PB_E4M3, true>, grid, kRowThreads, 0, st, (const float4*)y, (uint32_t*)q, sc8, sc32, n_groups, prep);
+    else    launch_behind(relu2_requantize_row128_f32_kernel<PB_E5M2, true>, grid, kRowThreads, 0, st, (const float4*)y, (uint32_t*)q, sc8, sc32, n_groups, prep);
   } else {
-    if (e4) relu2_requantize_row128_f32_kernel<PB_E4M3, false><<<grid, kRowThreads, 0, st>>>((const float4*)y, (uint32_t*)q, sc8, sc32, n_groups, prep);
-    else    relu2_requantize_row128_f32_kernel<PB_E5M2, false><<<grid, kRowThreads, 0, st>>>((const float4*)y, (uint32_t*)q, sc8, sc32, n_groups, prep);
+    if (e4) launch_behind(relu2_requantize_row128_f32_kernel<PB_E4M3, false>, grid, kRowThreads, 0, st, (const float4*)y, (uint32_t*)q, sc8, sc32, n_groups, prep);
+    else    launch_behind(relu2_requantize_row128_f32_kernel<PB_E5M2, false>, grid, kRowThreads, 0, st, (const float4*)y, (uint32_t*)q, sc8, sc32, n_groups, prep);
   }
   PB_LAUNCH_CHECK("relu2_requantize_row128_f32_kernel");
   return PB_OK;
@@ -1202,9 +1214,9 @@ extern "C" int pb_dequantize_bwd_quantize_dual(const float* g, const uint8_t* y_
   const int64_t n_groups = rows * (cols / 1024);
   const int grid = grid_for(n_groups * 32, kRowThreads, 8);
   if (out_format == PB_E4M3)
-    scaled_quantize_row128_f32_kernel<PB_E4M3, false><<<grid, kRowThreads, 0, st>>>(reinterpret_cast<const float4*>(g), y_sc8, y_sc32, reinterpret_cast<uint32_t*>(q), sc8, sc32, n_groups);
+    launch_behind(scaled_quantize_row128_f32_kernel<PB_E4M3, false>, grid, kRowThreads, 0, st, reinterpret_cast<const float4*>(g), y_sc8, y_sc32, reinterpret_cast<uint32_t*>(q), sc8, sc32, n_groups);
   else
-    scaled_quantize_row128_f32_kernel<PB_E5M2, false><<<grid, kRowThreads, 0, st>>>(reinterpret_cast<const float4*>(g), y_sc8, y_sc32, reinterpret_cast<uint32_t*>(q), sc8, sc32, n_groups);
+    launch_behind(scaled_quantize_row128_f32_kernel<PB_E5M2, false>, grid, kRowThreads, 0, st, reinterpret_cast<const float4*>(g), y_sc8, y_sc32, reinterpret_cast<uint32_t*>(q), sc8, sc32, n_groups);
   PB_LAUNCH_CHECK("scaled_quantize_row128_f32_kernel");
   return pb::launch_scaled_transposed(g, y_sc8, y_sc32, out_format, q_t, sc8_t, sc32_t, rows, cols, st);
 }
@@ -1224,7 +1236,7 @@ extern "C" int pb_relu2_quantize_dual(const float* k, int64_t rows, int64_t cols
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t n_groups = rows * (cols / 1024);
   const int grid = grid_for(n_groups * 32, kRowThreads, 8);
-  scaled_quantize_row128_f32_kernel<PB_E4M3, true><<<grid, kRowThreads, 0, st>>>(reinterpret_cast<const float4*>(k), nullptr, nullptr,
+  launch_behind(scaled_quantize_row128_f32_kernel<PB_E4M3, true>, grid, kRowThreads, 0, st, reinterpret_cast<const float4*>(k), nullptr, nullptr,
                                                                                reinterpret_cast<uint32_t*>(q), sc8, sc32, n_groups);
   PB_LAUNCH_CHECK("scaled_quantize_row128_f32_kernel");
   return pb::launch_relu2_transposed(k, q_t, sc8_t, sc32_t, rows, cols, st);
@@ -1260,7 +1272,7 @@ extern "C" int pb_shift_lerp_quantize(const float* x, const float* state, const 
   const int segs = (int)(channels / 1024);
   const int64_t n_groups = rows * segs;
   const int grid = grid_for(n_groups * 32, kRowThreads, 4);
-  shift_lerp_quantize_row128_kernel<PB_E4M3><<<grid, kRowThreads, 0, st>>>(
+  launch_behind(shift_lerp_quantize_row128_kernel<PB_E4M3>, grid, kRowThreads, 0, st, 
       reinterpret_cast<const float4*>(x), reinterpret_cast<const float4*>(state), reinterpret_cast<const float4*>(mu),
       reinterpret_cast<uint32_t*>(q), sc8, sc32, n_groups, segs, (int)steps, n_mix);
   PB_LAUNCH_CHECK("shift_lerp_quantize_row128_kernel");
@@ -1294,8 +1306,8 @@ static int fake_quantize_entry(const void* x, int x_dtype, int64_t batch, int64_
   const bool e4 = out_format == PB_E4M3;
 #define PB_FAKE_LAUNCH(FMT, OT, VT)                                                                                                              \
   do {                                                                                                                                           \
-    if (sc8) fake_quantize_row128_f32_kernel<FMT, OT, true><<<grid, kRowThreads, 0, st>>>((const float4*)x, (VT*)out, sc8, sc32, n_groups);       \
-    else     fake_quantize_row128_f32_kernel<FMT, OT, false><<<grid, kRowThreads, 0, st>>>((const float4*)x, (VT*)out, nullptr, nullptr, n_groups); \
+    if (sc8) launch_behind(fake_quantize_row128_f32_kernel<FMT, OT, true>, grid, kRowThreads, 0, st, (const float4*)x, (VT*)out, sc8, sc32, n_groups);       \
+    else     launch_behind(fake_quantize_row128_f32_kernel<FMT, OT, false>, grid, kRowThreads, 0, st, (const float4*)x, (VT*)out, nullptr, nullptr, n_groups); \
   } while (0)
   if (out_dtype == PB_F32) {
     if (e4) PB_FAKE_LAUNCH(PB_E4M3, float, float4);

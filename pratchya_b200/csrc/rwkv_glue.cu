@@ -36,6 +36,7 @@ struct ShiftLerpParams {
 };
 
 __global__ void __launch_bounds__(kGlueThreads) shift_lerp_fwd_kernel(const ShiftLerpParams p) {
+  grid_wait();
   const int C4 = p.C >> 2;
   const int64_t total = p.R * C4, stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
@@ -67,6 +68,7 @@ struct ShiftLerpBwdParams {
 
 template <int NMIX>
 __global__ void __launch_bounds__(kGlueThreads) shift_lerp_bwd_kernel(const ShiftLerpBwdParams p) {
+  grid_wait();
   const int c = (blockIdx.x * kGlueThreads + threadIdx.x) << 2;
   if (c >= p.C) return;
   const int64_t r0 = (int64_t)blockIdx.y * kLerpTileRows, r1 = min(p.R, r0 + kLerpTileRows);
@@ -118,6 +120,7 @@ __global__ void __launch_bounds__(kGlueThreads) shift_lerp_bwd_kernel(const Shif
 // out[j] = sum over tiles of partial[tile][j]: eight partial sums per column (tiles g, g + 8, ...), added in a fixed order.
 // A block takes 32 columns; out may be the first tile's slot of partial (a column is read and written by its block only).
 __global__ void __launch_bounds__(kGlueThreads) reduce_partials_kernel(const float* partial, float* out, int tiles, int64_t n) {
+  grid_wait();
   __shared__ float red[kGlueThreads / 32][32];
   const int cx = threadIdx.x & 31, gy = threadIdx.x >> 5;
   const int64_t j = (int64_t)blockIdx.x * 32 + cx;
@@ -157,6 +160,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 __global__ void __launch_bounds__(kGlueThreads) wkv_prepare_fwd_kernel(const PrepareParams p) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int C = p.N * kGlueH;
   const int64_t warps = (int64_t)gridDim.x * (kGlueThreads / 32), total = p.R * p.N;
@@ -200,6 +204,7 @@ struct PrepareBwdParams {
 };
 
 __global__ void __launch_bounds__(kGlueThreads) wkv_prepare_bwd_kernel(const PrepareBwdParams p) {
+  grid_wait();
   const PrepareParams& f = p.f;
   const int lane = threadIdx.x & 31;
   const int C = f.N * kGlueH;
@@ -288,7 +293,7 @@ extern "C" int pb_token_shift_lerp(const float* x, const float* state, const flo
   if (n_mix <= 0 || n_mix > kMaxMix) return fail(PB_ERR_UNSUPPORTED, "pb_token_shift_lerp: n_mix=%d (1..%d)", n_mix, kMaxMix);
   if (misaligned({x, state, mu, out})) return fail(PB_ERR_MISALIGNED, "pb_token_shift_lerp: every array must be 16-byte aligned");
   ShiftLerpParams p{x, state, mu, out, batch * steps, (int)steps, (int)channels, n_mix};
-  shift_lerp_fwd_kernel<<<grid_stride_blocks(p.R * (channels / 4)), kGlueThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  launch_behind(shift_lerp_fwd_kernel, grid_stride_blocks(p.R * (channels / 4)), kGlueThreads, 0, static_cast<cudaStream_t>(stream), p);
   PB_LAUNCH_CHECK("shift_lerp_fwd_kernel");
   return PB_OK;
 }
@@ -318,11 +323,11 @@ extern "C" int pb_token_shift_lerp_bwd(const float* const* g, const float* x, co
   ShiftLerpBwdParams p{{}, x, state, mu, dx, dstate, static_cast<float*>(workspace), R, (int)steps, (int)channels, n_mix};
   for (int k = 0; k < n_mix; ++k) p.g[k] = g[k];
   const dim3 grid((unsigned)((channels / 4 + kGlueThreads - 1) / kGlueThreads), (unsigned)tiles);
-  if (n_mix == 6) shift_lerp_bwd_kernel<6><<<grid, kGlueThreads, 0, st>>>(p);
-  else shift_lerp_bwd_kernel<1><<<grid, kGlueThreads, 0, st>>>(p);
+  if (n_mix == 6) launch_behind(shift_lerp_bwd_kernel<6>, grid, kGlueThreads, 0, st, p);
+  else launch_behind(shift_lerp_bwd_kernel<1>, grid, kGlueThreads, 0, st, p);
   PB_LAUNCH_CHECK("shift_lerp_bwd_kernel");
   const int64_t n = (int64_t)n_mix * channels;
-  reduce_partials_kernel<<<(unsigned)((n + 31) / 32), kGlueThreads, 0, st>>>(p.partial, dmu, tiles, n);
+  launch_behind(reduce_partials_kernel, (unsigned)((n + 31) / 32), kGlueThreads, 0, st, p.partial, dmu, tiles, n);
   PB_LAUNCH_CHECK("reduce_partials_kernel");
   return PB_OK;
 }
@@ -345,7 +350,7 @@ extern "C" int pb_wkv_prepare(const float* r_raw, const float* k_raw, const floa
   if ((v0 == nullptr) != (nu_raw == nullptr)) return fail(PB_ERR_NULL_POINTER, "pb_wkv_prepare: v0 and nu_raw come together");
   PrepareParams p{r_raw, k_raw, d, iclr_raw, v_prime, v0, nu_raw, cos_tab, sin_tab, rk_mult, mix_amt,
                   decay, iclr, removal_k, replacement_k, v, r, k, batch * steps, (int)steps, (int)heads};
-  wkv_prepare_fwd_kernel<<<grid_stride_blocks(p.R * heads * 32), kGlueThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  launch_behind(wkv_prepare_fwd_kernel, grid_stride_blocks(p.R * heads * 32), kGlueThreads, 0, static_cast<cudaStream_t>(stream), p);
   PB_LAUNCH_CHECK("wkv_prepare_fwd_kernel");
   return PB_OK;
 }
@@ -382,11 +387,11 @@ extern "C" int pb_wkv_prepare_bwd(const float* r_raw, const float* k_raw, const 
                      g_decay, g_iclr, g_removal_k, g_replacement_k, g_v, g_r, g_k,
                      d_r_raw, d_k_raw, d_d, d_iclr_raw, d_v_prime, d_v0, d_nu_raw, static_cast<float*>(workspace)};
   const int64_t warps = (int64_t)tiles * heads;
-  wkv_prepare_bwd_kernel<<<(unsigned)((warps + kGlueThreads / 32 - 1) / (kGlueThreads / 32)), kGlueThreads, 0, st>>>(p);
+  launch_behind(wkv_prepare_bwd_kernel, (unsigned)((warps + kGlueThreads / 32 - 1) / (kGlueThreads / 32)), kGlueThreads, 0, st, p);
   PB_LAUNCH_CHECK("wkv_prepare_bwd_kernel");
   // partial is [tiles][2][C]: the two parameters' sums come out as one [2][C] array, split below
   float* sums = static_cast<float*>(workspace);      // reduced in place into the first tile's slot after the reduction reads it
-  reduce_partials_kernel<<<(unsigned)((2 * C + 31) / 32), kGlueThreads, 0, st>>>(p.partial, sums, tiles, 2 * C);
+  launch_behind(reduce_partials_kernel, (unsigned)((2 * C + 31) / 32), kGlueThreads, 0, st, p.partial, sums, tiles, 2 * C);
   PB_LAUNCH_CHECK("reduce_partials_kernel");
   PB_CUDA_TRY(cudaMemcpyAsync(d_rk_mult, sums, (size_t)C * sizeof(float), cudaMemcpyDeviceToDevice, st));
   PB_CUDA_TRY(cudaMemcpyAsync(d_mix_amt, sums + C, (size_t)C * sizeof(float), cudaMemcpyDeviceToDevice, st));

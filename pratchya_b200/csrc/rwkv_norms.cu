@@ -33,6 +33,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // out[j] = sum over tiles of partial[tile][j]: eight partial sums per column (tiles g, g + 8, ...), added in a fixed order.
 // A block takes 32 columns; out may be the first tile's slot of partial (a column is read and written by its block only).
 __global__ void __launch_bounds__(kThreads) reduce_tiles_kernel(const float* partial, float* out, int tiles, int64_t n) {
+  grid_wait();
   __shared__ float red[kWarps][32];
   const int cx = threadIdx.x & 31, gy = threadIdx.x >> 5;
   const int64_t j = (int64_t)blockIdx.x * 32 + cx;
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(kThreads) reduce_tiles_kernel(const float* par
 // ---- RMSNorm: y = (x * rsqrt(mean(x^2) + eps)) * scale, one warp per row --------------------------------------
 __global__ void __launch_bounds__(kThreads) rms_norm_fwd_kernel(const float* x, const float* scale, float* y, float* inv_rms,
                                                                int64_t R, int C, float eps) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * kWarps;
   for (int64_t row = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5); row < R; row += warps) {
@@ -80,6 +82,7 @@ constexpr int kRowWarps = 4;
 template <int QUADS>
 __global__ void __launch_bounds__(32 * kRowWarps) rms_norm_fwd_row_kernel(const float* __restrict__ x, const float* __restrict__ scale, float* __restrict__ y,
                                                                         float* __restrict__ inv_rms, int64_t R, float eps) {
+  grid_wait();
   constexpr int C = 128 * QUADS;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * kRowWarps;
@@ -105,6 +108,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) rms_norm_fwd_row_kernel(const 
 // dx = inv * (dy * scale) - x * (inv^3 * sum_c(dy * scale * x) / C)
 __global__ void __launch_bounds__(kThreads) rms_norm_bwd_dx_kernel(const float* dy, const float* x, const float* scale, const float* inv_rms,
                                                                   float* dx, int64_t R, int C) {
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * kWarps;
   for (int64_t row = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5); row < R; row += warps) {
@@ -129,6 +133,7 @@ __global__ void __launch_bounds__(kThreads) rms_norm_bwd_dx_kernel(const float* 
 // partial[tile][c] = sum over the tile's rows of dy * x * inv_rms
 __global__ void __launch_bounds__(kThreads) rms_norm_bwd_dscale_kernel(const float* dy, const float* x, const float* inv_rms, float* partial,
                                                                       int64_t R, int C) {
+  grid_wait();
   const int c = (blockIdx.x * kThreads + threadIdx.x) << 2;
   if (c >= C) return;
   const int64_t r0 = (int64_t)blockIdx.y * kTileRows, r1 = min(R, r0 + kTileRows);
@@ -144,6 +149,7 @@ __global__ void __launch_bounds__(kThreads) rms_norm_bwd_dscale_kernel(const flo
 
 // ---- relu(x)^2 -----------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads) relu2_fwd_kernel(const float4* x, float4* y, int64_t n4) {
+  grid_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
     const float4 v = x[i];
@@ -152,6 +158,7 @@ __global__ void __launch_bounds__(kThreads) relu2_fwd_kernel(const float4* x, fl
   }
 }
 __global__ void __launch_bounds__(kThreads) relu2_bwd_kernel(const float4* g, const float4* x, float4* dx, int64_t n4) {
+  grid_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) {
     const float4 v = x[i], gg = g[i];
@@ -164,6 +171,7 @@ __global__ void __launch_bounds__(kThreads) relu2_bwd_kernel(const float4* g, co
 // the mean and the variance E[x^2] - E[x]^2 (clamped at 0) over the T x 64 values.
 // group_sums_kernel: partial[b][n][tile][2] = (sum, sum of squares) over a tile of kStatTileSteps timesteps.
 __global__ void __launch_bounds__(kThreads) group_sums_kernel(const float* y, float* partial, int T, int N, int tiles) {
+  grid_wait();
   __shared__ float red[kWarps][2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int bn = blockIdx.x, tile = blockIdx.y;
@@ -189,6 +197,7 @@ __global__ void __launch_bounds__(kThreads) group_sums_kernel(const float* y, fl
 }
 // stats[bn] = (mean, rstd)
 __global__ void group_stats_kernel(const float* partial, float* stats, int groups, int tiles, float count, float eps) {
+  grid_wait();
   const int bn = blockIdx.x * blockDim.x + threadIdx.x;
   if (bn >= groups) return;
   float s = 0.f, q = 0.f;
@@ -223,6 +232,7 @@ template <int V> __device__ __forceinline__ void load_chans(const float* p, floa
 // 115 -> 73 us, 512 tokens 33 -> 7.5 us.
 template <int V, int WARPS>
 __global__ void __launch_bounds__(kThreads) wkv_finish_fwd_kernel(const FinishParams p) {
+  grid_wait();
   constexpr int kTokens = kWarps / WARPS, kGroup = 32 * WARPS;
   __shared__ float red[2][kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = warp / WARPS, tid = threadIdx.x % kGroup;
@@ -281,6 +291,7 @@ struct FinishBwdParams {
 };
 
 __global__ void __launch_bounds__(kThreads) wkv_finish_bwd_scalars_kernel(const FinishBwdParams p) {
+  grid_wait();
   const FinishParams& f = p.f;
   const int lane = threadIdx.x & 31;
   const int C = f.N * kH;
@@ -312,6 +323,7 @@ __global__ void __launch_bounds__(kThreads) wkv_finish_bwd_scalars_kernel(const 
 
 // group_terms[bn] = (sum_t head_sums[b, t, n, 0], sum_t head_sums[b, t, n, 1]) / (T * 64); one CTA per (b, n)
 __global__ void __launch_bounds__(kThreads) group_terms_kernel(const float* head_sums, float* group_terms, int T, int N) {
+  grid_wait();
   __shared__ float red[kWarps][2];
   const int bn = blockIdx.x, b = bn / N, n = bn - b * N;
   float s1 = 0.f, s2 = 0.f;
@@ -335,6 +347,7 @@ __global__ void __launch_bounds__(kThreads) group_terms_kernel(const float* head
 // adds up their share of the three parameter gradients over the tile's tokens.  The arrays are read through __ldg so that a
 // token's loads need not wait for the stores of the one before.
 __global__ void __launch_bounds__(kThreads) wkv_finish_bwd_main_kernel(const FinishBwdParams p) {
+  grid_wait();
   const FinishParams& f = p.f;
   const int lane = threadIdx.x & 31;
   const int C = f.N * kH;
@@ -395,7 +408,7 @@ bool launch_rms_norm_rows(std::integer_sequence<int, I...>, const float* x, cons
                           float eps, cudaStream_t st) {
   const unsigned blocks = blocks_for(rows, kRowWarps);
   return ((channels == 128 * (I + 1) &&
-           (rms_norm_fwd_row_kernel<I + 1><<<blocks, 32 * kRowWarps, 0, st>>>(x, scale, y, inv_rms, rows, eps), true)) || ...);
+           (launch_behind(rms_norm_fwd_row_kernel<I + 1>, blocks, 32 * kRowWarps, 0, st, x, scale, y, inv_rms, rows, eps), true)) || ...);
 }
 
 bool any_misaligned(std::initializer_list<const void*> ptrs) {
@@ -419,7 +432,7 @@ extern "C" int pb_rms_norm(const float* x, const float* scale, int64_t rows, int
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // PB_RMS_LOOP=1 (diagnostics build): the loop over a row for every width
   if (env_switch("PB_RMS_LOOP", 0) || !launch_rms_norm_rows(std::make_integer_sequence<int, kRowQuads>{}, x, scale, y, inv_rms, rows, (int)channels, eps, st))
-    rms_norm_fwd_kernel<<<blocks_for(rows, kWarps), kThreads, 0, st>>>(x, scale, y, inv_rms, rows, (int)channels, eps);
+    launch_behind(rms_norm_fwd_kernel, blocks_for(rows, kWarps), kThreads, 0, st, x, scale, y, inv_rms, rows, (int)channels, eps);
   PB_LAUNCH_CHECK("rms_norm_fwd_kernel");
   return PB_OK;
 }
@@ -438,13 +451,13 @@ extern "C" int pb_rms_norm_bwd(const float* dy, const float* x, const float* sca
   if (!workspace || workspace_bytes < need) return fail(PB_ERR_WORKSPACE_TOO_SMALL, "pb_rms_norm_bwd: needs %zu bytes of workspace, got %zu", need, workspace_bytes);
   if (any_misaligned({dy, x, scale, dx, workspace})) return fail(PB_ERR_MISALIGNED, "pb_rms_norm_bwd: arrays must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  rms_norm_bwd_dx_kernel<<<blocks_for(rows, kWarps), kThreads, 0, st>>>(dy, x, scale, inv_rms, dx, rows, (int)channels);
+  launch_behind(rms_norm_bwd_dx_kernel, blocks_for(rows, kWarps), kThreads, 0, st, dy, x, scale, inv_rms, dx, rows, (int)channels);
   PB_LAUNCH_CHECK("rms_norm_bwd_dx_kernel");
   const int tiles = (int)((rows + kTileRows - 1) / kTileRows);
   const dim3 grid((unsigned)((channels / 4 + kThreads - 1) / kThreads), (unsigned)tiles);
-  rms_norm_bwd_dscale_kernel<<<grid, kThreads, 0, st>>>(dy, x, inv_rms, static_cast<float*>(workspace), rows, (int)channels);
+  launch_behind(rms_norm_bwd_dscale_kernel, grid, kThreads, 0, st, dy, x, inv_rms, static_cast<float*>(workspace), rows, (int)channels);
   PB_LAUNCH_CHECK("rms_norm_bwd_dscale_kernel");
-  reduce_tiles_kernel<<<(unsigned)((channels + 31) / 32), kThreads, 0, st>>>(static_cast<const float*>(workspace), dscale, tiles, channels);
+  launch_behind(reduce_tiles_kernel, (unsigned)((channels + 31) / 32), kThreads, 0, st, static_cast<const float*>(workspace), dscale, tiles, channels);
   PB_LAUNCH_CHECK("reduce_tiles_kernel");
   return PB_OK;
 }
@@ -453,7 +466,7 @@ extern "C" int pb_relu2(const float* x, int64_t n, float* y, void* stream) {
   if (!x || !y) return fail(PB_ERR_NULL_POINTER, "pb_relu2: x and y must be non-null");
   if (n <= 0 || n % 4 != 0) return fail(PB_ERR_BAD_SHAPE, "pb_relu2: n=%lld must be a positive multiple of 4", (long long)n);
   if (any_misaligned({x, y})) return fail(PB_ERR_MISALIGNED, "pb_relu2: x and y must be 16-byte aligned");
-  relu2_fwd_kernel<<<blocks_for(n / 4, kThreads), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(y), n / 4);
+  launch_behind(relu2_fwd_kernel, blocks_for(n / 4, kThreads), kThreads, 0, static_cast<cudaStream_t>(stream), reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(y), n / 4);
   PB_LAUNCH_CHECK("relu2_fwd_kernel");
   return PB_OK;
 }
@@ -462,7 +475,7 @@ extern "C" int pb_relu2_bwd(const float* g, const float* x, int64_t n, float* dx
   if (!g || !x || !dx) return fail(PB_ERR_NULL_POINTER, "pb_relu2_bwd: g, x and dx must be non-null");
   if (n <= 0 || n % 4 != 0) return fail(PB_ERR_BAD_SHAPE, "pb_relu2_bwd: n=%lld must be a positive multiple of 4", (long long)n);
   if (any_misaligned({g, x, dx})) return fail(PB_ERR_MISALIGNED, "pb_relu2_bwd: g, x and dx must be 16-byte aligned");
-  relu2_bwd_kernel<<<blocks_for(n / 4, kThreads), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_behind(relu2_bwd_kernel, blocks_for(n / 4, kThreads), kThreads, 0, static_cast<cudaStream_t>(stream), 
       reinterpret_cast<const float4*>(g), reinterpret_cast<const float4*>(x), reinterpret_cast<float4*>(dx), n / 4);
   PB_LAUNCH_CHECK("relu2_bwd_kernel");
   return PB_OK;
@@ -493,9 +506,9 @@ extern "C" int pb_wkv_finish(const float* y, const float* r, const float* k, con
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int tiles = (int)((steps + kStatTileSteps - 1) / kStatTileSteps);
   const int groups = (int)(batch * heads);
-  group_sums_kernel<<<dim3((unsigned)groups, (unsigned)tiles), kThreads, 0, st>>>(y, static_cast<float*>(workspace), (int)steps, (int)heads, tiles);
+  launch_behind(group_sums_kernel, dim3((unsigned)groups, (unsigned)tiles), kThreads, 0, st, y, static_cast<float*>(workspace), (int)steps, (int)heads, tiles);
   PB_LAUNCH_CHECK("group_sums_kernel");
-  group_stats_kernel<<<(groups + 127) / 128, 128, 0, st>>>(static_cast<const float*>(workspace), stats, groups, tiles, (float)steps * (float)kH, eps);
+  launch_behind(group_stats_kernel, (groups + 127) / 128, 128, 0, st, static_cast<const float*>(workspace), stats, groups, tiles, (float)steps * (float)kH, eps);
   PB_LAUNCH_CHECK("group_stats_kernel");
   FinishParams p{y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, stats, out, batch * steps, (int)steps, (int)heads};
   // One head is no more than a warp's channels: four bytes at a time use all of its lanes.
@@ -509,10 +522,10 @@ extern "C" int pb_wkv_finish(const float* y, const float* r, const float* k, con
   const int grid = blocks_for(p.R, kWarps / warps);
 #define PB_FINISH_LAUNCH(V)                                                                    \
   do {                                                                                         \
-    if (warps == 1)      wkv_finish_fwd_kernel<V, 1><<<grid, kThreads, 0, st>>>(p);            \
-    else if (warps == 2) wkv_finish_fwd_kernel<V, 2><<<grid, kThreads, 0, st>>>(p);            \
-    else if (warps == 4) wkv_finish_fwd_kernel<V, 4><<<grid, kThreads, 0, st>>>(p);            \
-    else                 wkv_finish_fwd_kernel<V, kWarps><<<grid, kThreads, 0, st>>>(p);       \
+    if (warps == 1)      launch_behind(wkv_finish_fwd_kernel<V, 1>, grid, kThreads, 0, st, p);            \
+    else if (warps == 2) launch_behind(wkv_finish_fwd_kernel<V, 2>, grid, kThreads, 0, st, p);            \
+    else if (warps == 4) launch_behind(wkv_finish_fwd_kernel<V, 4>, grid, kThreads, 0, st, p);            \
+    else                 launch_behind(wkv_finish_fwd_kernel<V, kWarps>, grid, kThreads, 0, st, p);       \
   } while (0)
   if (wide) PB_FINISH_LAUNCH(4);
   else      PB_FINISH_LAUNCH(1);
@@ -551,14 +564,14 @@ extern "C" int pb_wkv_finish_bwd(const float* g, const float* y, const float* r,
   float* partial = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(group_terms) + align256((size_t)batch * heads * 2 * 4));
   FinishBwdParams p{{y, r, k, v, gate, gn_scale, gn_bias, bonus_mult, stats, nullptr, R, (int)steps, (int)heads},
                     g, scalars, head_sums, group_terms, d_y, d_r, d_k, d_v, d_gate, partial};
-  wkv_finish_bwd_scalars_kernel<<<blocks_for(R, kWarps), kThreads, 0, st>>>(p);
+  launch_behind(wkv_finish_bwd_scalars_kernel, blocks_for(R, kWarps), kThreads, 0, st, p);
   PB_LAUNCH_CHECK("wkv_finish_bwd_scalars_kernel");
-  group_terms_kernel<<<(unsigned)(batch * heads), kThreads, 0, st>>>(head_sums, group_terms, (int)steps, (int)heads);
+  launch_behind(group_terms_kernel, (unsigned)(batch * heads), kThreads, 0, st, head_sums, group_terms, (int)steps, (int)heads);
   PB_LAUNCH_CHECK("group_terms_kernel");
   const int64_t warps = (int64_t)tiles * heads;
-  wkv_finish_bwd_main_kernel<<<(unsigned)((warps + kWarps - 1) / kWarps), kThreads, 0, st>>>(p);
+  launch_behind(wkv_finish_bwd_main_kernel, (unsigned)((warps + kWarps - 1) / kWarps), kThreads, 0, st, p);
   PB_LAUNCH_CHECK("wkv_finish_bwd_main_kernel");
-  reduce_tiles_kernel<<<(unsigned)((3 * C + 31) / 32), kThreads, 0, st>>>(partial, partial, tiles, 3 * C);
+  launch_behind(reduce_tiles_kernel, (unsigned)((3 * C + 31) / 32), kThreads, 0, st, partial, partial, tiles, 3 * C);
   PB_LAUNCH_CHECK("reduce_tiles_kernel");
   PB_CUDA_TRY(cudaMemcpyAsync(d_gn_scale, partial, (size_t)C * 4, cudaMemcpyDeviceToDevice, st));
   PB_CUDA_TRY(cudaMemcpyAsync(d_gn_bias, partial + C, (size_t)C * 4, cudaMemcpyDeviceToDevice, st));

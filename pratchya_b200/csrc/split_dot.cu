@@ -225,6 +225,7 @@ __device__ __forceinline__ void prepare_g(const PrepareParams& p, uint32_t v) {
 // G32: f32 g.  TERMS: of Q, where g is used as it is.  Blocks [0, q_blocks) work on Q, the others on g.
 template <bool TOKENS, bool G32, int TERMS>
 __global__ void __launch_bounds__(256) split_prepare_kernel(const __grid_constant__ PrepareParams p) {
+  grid_wait();
   if (blockIdx.x < p.q_blocks) {
     const uint32_t v = blockIdx.x * 256 + threadIdx.x;
     if (v < p.n_q) prepare_q<!G32 && TERMS == 3>(p, v, G32 ? 1.0f : kScaleUp);
@@ -309,6 +310,7 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
   __syncthreads();
   tc_after();
   const uint32_t tmem = *(volatile uint32_t*)&tmem_slot;
+  grid_wait();
   const int items = p.tiles * p.splits;
   auto item_of = [&](int w, int& row0, int& col0, int& u_begin, int& u_end) {
     const int split = w / p.tiles, tile = w - split * p.tiles;
@@ -515,7 +517,7 @@ template <int N, bool TOKENS, bool G32, int TERMS>
 int launch(const CUtensorMap& terms, const CUtensorMap& other, const SplitParams& p, cudaStream_t st) {
   PB_CUDA_TRY(cudaFuncSetAttribute(split_dot_kernel<N, TOKENS, G32, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<N, TOKENS, G32, TERMS>::kSmem));      // per device
   const int items = p.tiles * p.splits;
-  split_dot_kernel<N, TOKENS, G32, TERMS><<<items < sm_count() ? items : sm_count(), kThreads, Cfg<N, TOKENS, G32, TERMS>::kSmem, st>>>(terms, other, p);
+  launch_behind(split_dot_kernel<N, TOKENS, G32, TERMS>, items < sm_count() ? items : sm_count(), kThreads, Cfg<N, TOKENS, G32, TERMS>::kSmem, st, terms, other, p);
   PB_LAUNCH_CHECK("split_dot_kernel");
   return PB_OK;
 }
@@ -526,7 +528,7 @@ int launch_n(int n, const CUtensorMap& terms, const CUtensorMap& other, const Sp
 }
 template <bool TOKENS, bool G32, int TERMS>
 int launch_prepare(const PrepareParams& p, cudaStream_t st) {
-  split_prepare_kernel<TOKENS, G32, TERMS><<<p.q_blocks + (G32 ? (p.n_g + 255) / 256 : 0), 256, 0, st>>>(p);
+  launch_behind(split_prepare_kernel<TOKENS, G32, TERMS>, p.q_blocks + (G32 ? (p.n_g + 255) / 256 : 0), 256, 0, st, p);
   PB_LAUNCH_CHECK("split_prepare_kernel");
   return PB_OK;
 }

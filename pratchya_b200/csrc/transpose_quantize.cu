@@ -208,6 +208,7 @@ template <typename InT, int FMT>
 __global__ void __launch_bounds__(OnePass<InT>::kThreads)
 transpose_quantize1024_kernel(const InT* __restrict__ x, uint8_t* __restrict__ q_t, uint8_t* __restrict__ sc8,
                               float* __restrict__ sc32, int rows, int cols) {
+  grid_wait();
   constexpr int kCols = OnePass<InT>::kCols, kThreads = OnePass<InT>::kThreads;
   extern __shared__ __align__(16) uint8_t tile_raw[];
   InT* tile = reinterpret_cast<InT*>(tile_raw);                // [1024][kCols]
@@ -275,6 +276,7 @@ template <int FMT>
 __global__ void __launch_bounds__(512, 2)
 transpose_quantize1024_bf16_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q_t, uint8_t* __restrict__ sc8,
                                    float* __restrict__ sc32, int rows, int cols) {
+  grid_wait();
   extern __shared__ __align__(16) uint8_t tile_raw[];              // [1024 rows][64 bytes]
   __shared__ uint32_t part_amax[32][16];                            // [block*4 + quarter][column pair], bf16 pairs
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 1024;
@@ -366,7 +368,7 @@ int launch_one_pass_bf16(const void* x, uint8_t* q_t, uint8_t* sc8, float* sc32,
     }
   }
   const dim3 grid((unsigned)(cols / 32), (unsigned)(rows / 1024), (unsigned)batch);
-  transpose_quantize1024_bf16_kernel<FMT><<<grid, 512, 1024 * 64, st>>>((const __nv_bfloat16*)x, q_t, sc8, sc32, (int)rows, (int)cols);
+  launch_behind(transpose_quantize1024_bf16_kernel<FMT>, grid, 512, 1024 * 64, st, (const __nv_bfloat16*)x, q_t, sc8, sc32, (int)rows, (int)cols);
   PB_LAUNCH_CHECK("transpose_quantize1024_bf16_kernel");
   return PB_OK;
 }
@@ -436,6 +438,7 @@ template <int FMT>
 __global__ void __launch_bounds__(1024, 1)
 transpose_quantize1024_bf16_ring_kernel(const __grid_constant__ CUtensorMap map_x, uint8_t* __restrict__ q_t, uint8_t* __restrict__ sc8,
                                         float* __restrict__ sc32, int rows, int cols, int tiles_x, int tiles_y, int n_tiles) {
+  grid_wait();
   extern __shared__ uint8_t ring_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ring_raw) + 1023) & ~(uintptr_t)1023);
   uint32_t (*part_amax)[32][16] = reinterpret_cast<uint32_t (*)[32][16]>(smem + kRingBufs * kRingTileBytes);   // [group * 2 + parity]
@@ -575,6 +578,7 @@ __global__ void __launch_bounds__(1024, 1)
 transpose_quantize1024_f32_ring_kernel(const __grid_constant__ CUtensorMap map_x, uint8_t* __restrict__ q_t, uint8_t* __restrict__ sc8,
                                        float* __restrict__ sc32, int rows, int cols, int tiles_x, int tiles_y, int n_tiles,
                                        const LerpPrologue lerp) {
+  grid_wait();
   extern __shared__ uint8_t ring_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ring_raw) + 1023) & ~(uintptr_t)1023);
   float (*part_amax)[32][16] = reinterpret_cast<float (*)[32][16]>(smem + kRingBufs * kRingTileBytes);   // [group * 2 + parity]
@@ -758,7 +762,7 @@ int launch_one_pass_f32_ring(const void* x, uint8_t* q_t, uint8_t* sc8, float* s
   const int tiles_x = (int)(cols / 16), tiles_y = (int)(rows / 1024);
   const int64_t n_tiles = (int64_t)tiles_x * tiles_y * batch;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  transpose_quantize1024_f32_ring_kernel<FMT, LERP><<<grid, 1024, kRingSmem + kRingScaleBytes, st>>>(map, q_t, sc8, sc32, (int)rows, (int)cols, tiles_x, tiles_y, (int)n_tiles, lerp);
+  launch_behind(transpose_quantize1024_f32_ring_kernel<FMT, LERP>, grid, 1024, kRingSmem + kRingScaleBytes, st, map, q_t, sc8, sc32, (int)rows, (int)cols, tiles_x, tiles_y, (int)n_tiles, lerp);
   PB_LAUNCH_CHECK("transpose_quantize1024_f32_ring_kernel");
   return PB_OK;
 }
@@ -793,7 +797,7 @@ int launch_one_pass_bf16_ring(const void* x, uint8_t* q_t, uint8_t* sc8, float* 
   const int tiles_x = (int)(cols / 32), tiles_y = (int)(rows / 1024);
   const int64_t n_tiles = (int64_t)tiles_x * tiles_y * batch;
   const int grid = (int)(n_tiles < sm_count() ? n_tiles : sm_count());
-  transpose_quantize1024_bf16_ring_kernel<FMT><<<grid, 1024, kRingSmem, st>>>(map, q_t, sc8, sc32, (int)rows, (int)cols, tiles_x, tiles_y, (int)n_tiles);
+  launch_behind(transpose_quantize1024_bf16_ring_kernel<FMT>, grid, 1024, kRingSmem, st, map, q_t, sc8, sc32, (int)rows, (int)cols, tiles_x, tiles_y, (int)n_tiles);
   PB_LAUNCH_CHECK("transpose_quantize1024_bf16_ring_kernel");
   return PB_OK;
 }
@@ -812,7 +816,7 @@ int launch_one_pass(const void* x, uint8_t* q_t, uint8_t* sc8, float* sc32, int6
     }
   }
   const dim3 grid((unsigned)(cols / OnePass<InT>::kCols), (unsigned)(rows / 1024), (unsigned)batch);
-  transpose_quantize1024_kernel<InT, FMT><<<grid, OnePass<InT>::kThreads, OnePass<InT>::kSmem, st>>>((const InT*)x, q_t, sc8, sc32, (int)rows, (int)cols);
+  launch_behind(transpose_quantize1024_kernel<InT, FMT>, grid, OnePass<InT>::kThreads, OnePass<InT>::kSmem, st, (const InT*)x, q_t, sc8, sc32, (int)rows, (int)cols);
   PB_LAUNCH_CHECK("transpose_quantize1024_kernel");
   return PB_OK;
 }
@@ -837,6 +841,7 @@ transpose_bytes_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ ds
 // each column; eight lanes write 128 consecutive bytes.  2048 x 2048: 11.1 -> 3.6 us.
 __global__ void __launch_bounds__(256)
 transpose_bytes16_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int rows, int cols) {
+  grid_wait();
   __shared__ uint32_t tile[128][33];
   const int r0 = blockIdx.y * 128, c0 = blockIdx.x * 128;
 #pragma unroll
@@ -1037,7 +1042,7 @@ extern "C" int pb_transpose_bytes(const void* src, int64_t rows, int64_t cols, v
     return fail(PB_ERR_BAD_SHAPE, "pb_transpose_bytes: bad shape [%lld, %lld]", (long long)rows, (long long)cols);
   if (rows % 16 == 0 && cols % 16 == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
     const dim3 grid16((unsigned)((cols + 127) / 128), (unsigned)((rows + 127) / 128));      // fewer rows of tiles than the other's
-    transpose_bytes16_kernel<<<grid16, 256, 0, static_cast<cudaStream_t>(stream)>>>((const uint8_t*)src, (uint8_t*)dst, (int)rows, (int)cols);
+    launch_behind(transpose_bytes16_kernel, grid16, 256, 0, static_cast<cudaStream_t>(stream), (const uint8_t*)src, (uint8_t*)dst, (int)rows, (int)cols);
     PB_LAUNCH_CHECK("transpose_bytes16_kernel");
     return PB_OK;
   }

@@ -145,6 +145,7 @@ template <int V> struct Int { static constexpr int value = V; };
 template <int ROWS, int LANES, int WARPS, int PREP, int PER_SM, bool SAVE>
 __global__ void __launch_bounds__(32 * (WARPS + PREP), PER_SM)
 wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
+  grid_wait();
   constexpr int kWarpRows = ROWS * (32 / LANES), kCtaRows = kWarpRows * WARPS, kCtasPerHead = kH / kCtaRows;
   constexpr int kPairs = kH / LANES / 2;        // float2 of a lane's row
   constexpr int kPrepSteps = kFwdChunk / PREP;
@@ -476,7 +477,7 @@ int launch_forward(const WkvParams& p, int64_t heads, cudaStream_t st) {
   const int smem = kFwdBufs * (int)sizeof(WkvFwdChunk);
   auto go = [&](auto kernel) {
     PB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));   // per device
-    kernel<<<grid, 32 * (WARPS + PREP), smem, st>>>(p);
+    launch_behind(kernel, grid, 32 * (WARPS + PREP), smem, st, p);
     PB_LAUNCH_CHECK("wkv7_forward_kernel");
     return (int)PB_OK;
   };
@@ -569,6 +570,7 @@ __device__ __forceinline__ float2 cols_reduce_scatter(const float2 (&v)[4], int 
 
 __global__ void __launch_bounds__(kThreads, 2)
 wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char wkv_bwd_smem[];
   WkvBwdSmem& sm = *reinterpret_cast<WkvBwdSmem*>(wkv_bwd_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -888,7 +890,7 @@ extern "C" int pb_wkv7_backward(const float* decay, const float* iclr, const flo
   WkvBwdParams p{{decay, iclr, removal_k, replacement_k, v, r}, dy, sa, reinterpret_cast<const float4*>(checkpoints), dstate_out,
                  {d_decay, d_iclr, d_removal_k, d_replacement_k, d_v, d_r}, dstate_in, (int)steps, (int)heads};
   PB_CUDA_TRY(cudaFuncSetAttribute(wkv7_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WkvBwdSmem)));   // per device
-  wkv7_backward_kernel<<<(unsigned)(batch * heads), kThreads, sizeof(WkvBwdSmem), static_cast<cudaStream_t>(stream)>>>(p);
+  launch_behind(wkv7_backward_kernel, (unsigned)(batch * heads), kThreads, sizeof(WkvBwdSmem), static_cast<cudaStream_t>(stream), p);
   PB_LAUNCH_CHECK("wkv7_backward_kernel");
   return PB_OK;
 }
