@@ -198,6 +198,15 @@ class _LinearFn(torch.autograd.Function):
         # A (128,1) weight (LoRA, gate, lm_head) has one scale per column and 128 rows, which no 128-deep block
         # along its columns can carry: its forward runs on the tensor cores, its backward on the literal recipe.
         want_xt = for_backward and recipe == "fp8" and (a, b) == (128, 128) and x2.shape[0] % 1024 == 0
+        ctx.grid, ctx.recipe, ctx.grad_format, ctx.fake = grid, recipe, grad_format, fake_quant_output
+        ctx.x_shape, ctx.x_dtype, ctx.w_dtype = x.shape, x.dtype, weight.dtype
+        if for_backward and prepared_x is None and a == 128 and _lib.native().linear_takes(x, None, weight, b, fake_quant_output):
+            # the steps below in one call of the extension, where it takes them
+            out = _lib.native().linear_forward(x, wq[1], wq[2], _weight_bytes_t(wq, prepared), b, fake_quant_output, want_xt)
+            if out is not None:
+                ctx.have_xt = want_xt
+                ctx.save_for_backward(*out[1:4], *wq, *out[4:])
+                return out[0]
         if prepared_x is not None:      # x arrives quantized (its producer wrote the triples); x itself is a handle that is not read
             xq, xt = prepared_x
             if a != 128 or xq[0].shape != x2.shape or (want_xt and xt is None):
@@ -212,8 +221,6 @@ class _LinearFn(torch.autograd.Function):
             y = _ops.gemm(xq, (_weight_bytes_t(wq, prepared), *wq[1:]), (b, 128), torch.float32, 1)
         else:
             y = _ops.matmul_impl(*xq, *wq, (1, a), grid, out_dtype=torch.float32)
-        ctx.grid, ctx.recipe, ctx.grad_format, ctx.fake = grid, recipe, grad_format, fake_quant_output
-        ctx.x_shape, ctx.x_dtype, ctx.w_dtype = x.shape, x.dtype, weight.dtype
         saved = [*xq, *wq]
         if want_xt and eligible:
             saved += list(xt)                                           # X^T on (1,128) for wgrad
@@ -239,6 +246,11 @@ class _LinearFn(torch.autograd.Function):
         xt = None
         if ctx.have_xt:
             xt, pos = saved[6:9], 9
+        if a == 128 and ctx.w_dtype is torch.float32 and (xt is not None or not _ops._LITERAL_DOT_TF32):
+            out = _lib.native().linear_backward(g_y, *xq, *wq, *(xt or (None, None, None)), *(saved[pos:pos + 2] if ctx.fake else (None, None)), b,
+                                                _ops._FMT_CODE[ctx.grad_format], ctx.x_dtype)
+            if out is not None:
+                return out[0].reshape(ctx.x_shape), out[1], None, None, None, None, None, None, None
         g = g_y.reshape(-1, g_y.shape[-1]).contiguous()
         if ctx.fake and xt is not None and b == 128:
             # the cotangent of the output's dequantize (:575-601) as the prologue of dY's two quantizers

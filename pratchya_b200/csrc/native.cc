@@ -413,6 +413,178 @@ OP(linear) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---- a Linear's training step: what _LinearFn's two passes call one by one, each in one call ----
+struct Triple { at::Tensor q, s8, s32; };
+
+int rows_form(const at::Tensor& x, int64_t rows, int64_t cols, int fmt, Triple* t, void* st) {       // on (1,128), whole groups of eight blocks
+  const int64_t groups = rows * (cols / 128) / 8;
+  *t = {empty({rows, cols}, fmt == PB_E4M3 ? kE4M3 : kE5M2, x), empty({groups, 8}, kE8M0, x), empty({groups, 1, 1}, at::kFloat, x)};
+  at::Tensor ws;
+  const size_t bytes = pb_quantize_workspace_size(1, rows, cols, 1, 128);
+  if (bytes) ws = scratch(bytes, x);
+  return without_gil([&] {
+    return pb_quantize(x.data_ptr(), code(x.scalar_type()), 1, rows, cols, 1, 128, fmt, t->q.data_ptr(), (uint8_t*)t->s8.data_ptr(), (float*)t->s32.data_ptr(),
+                       bytes ? ws.data_ptr() : nullptr, bytes, st);
+  });
+}
+// x^T on (1,128): rows are a multiple of 1024
+Triple tokens_form(const at::Tensor& x, int64_t rows, int64_t cols, int fmt) {
+  const int64_t groups = rows * cols / 1024;
+  return {empty({cols, rows}, fmt == PB_E4M3 ? kE4M3 : kE5M2, x), empty({groups, 8}, kE8M0, x), empty({groups, 1, 1}, at::kFloat, x)};
+}
+// both forms: quantize_dual_impl
+int dual_form(const at::Tensor& x, int64_t rows, int64_t cols, int fmt, Triple* t, Triple* tt, void* st) {
+  const size_t bytes = pb_quantize_transposed_workspace_size(1, rows, cols, 128);
+  at::Tensor ws = scratch(bytes ? bytes : 1, x);
+  if (x.scalar_type() == at::kBFloat16 && cols % 1024 == 0) {
+    const int64_t groups = rows * cols / 1024;
+    *t = {empty({rows, cols}, fmt == PB_E4M3 ? kE4M3 : kE5M2, x), empty({groups, 8}, kE8M0, x), empty({groups, 1, 1}, at::kFloat, x)};
+    *tt = tokens_form(x, rows, cols, fmt);
+    return without_gil([&] {
+      return pb_quantize_dual(x.data_ptr(), PB_BF16, 1, rows, cols, fmt, t->q.data_ptr(), (uint8_t*)t->s8.data_ptr(), (float*)t->s32.data_ptr(), tt->q.data_ptr(),
+                              (uint8_t*)tt->s8.data_ptr(), (float*)tt->s32.data_ptr(), ws.data_ptr(), bytes, st);
+    });
+  }
+  if (int status = rows_form(x, rows, cols, fmt, t, st)) return status;
+  *tt = tokens_form(x, rows, cols, fmt);
+  return without_gil([&] {
+    return pb_quantize_transposed(x.data_ptr(), code(x.scalar_type()), 1, rows, cols, 128, fmt, tt->q.data_ptr(), (uint8_t*)tt->s8.data_ptr(), (float*)tt->s32.data_ptr(),
+                                  bytes ? ws.data_ptr() : nullptr, bytes, st);
+  });
+}
+// d [rows of a, rows of b] f32, of operands whose blocks are 128 deep
+int product(const Triple& a, const Triple& b, int b_height, int b_transposed, at::Tensor* d, void* st) {
+  const int64_t depth = a.q.size(1), rows = a.q.size(0), cols = b.q.size(0);
+  const pb_operand oa{a.q.data_ptr(), (const uint8_t*)a.s8.data_ptr(), (const float*)a.s32.data_ptr(), rows, depth, 1, 128, format(a.q), 0};
+  const pb_operand ob{b.q.data_ptr(), (const uint8_t*)b.s8.data_ptr(), (const float*)b.s32.data_ptr(), cols, depth, b_height, 128, format(b.q), b_transposed};
+  *d = empty({rows, cols}, at::kFloat, a.q);
+  const size_t bytes = pb_gemm_workspace_size(&oa, &ob);
+  at::Tensor ws = scratch(bytes ? bytes : 1, a.q);
+  return without_gil([&] { return pb_gemm_tn(&oa, &ob, d->data_ptr(), PB_F32, cols, ws.data_ptr(), bytes, st); });
+}
+int literal_dot(int tokens, const Triple& t, int a, int b, const at::Tensor& g, int64_t g_rows, int64_t g_cols, at::Tensor* out, void* st) {
+  const int64_t rows = t.q.size(0), cols = t.q.size(1), free = tokens ? g_cols : g_rows;
+  const int type = code(g.scalar_type());
+  *out = tokens ? empty({cols, free}, at::kFloat, g) : empty({free, rows}, at::kFloat, g);
+  at::Tensor ws;
+  size_t bytes = pb_dense_dot_workspace_best(tokens, rows, cols, a, b, free, type);
+  try {
+    if (bytes) ws = scratch(bytes, g);
+  } catch (const c10::OutOfMemoryError&) {      // the form that takes less of it
+    const size_t least = pb_dense_dot_workspace_size(tokens, rows, cols, a, b, free);
+    if (least == bytes) throw;
+    bytes = least;
+    if (bytes) ws = scratch(bytes, g);
+  }
+  return without_gil([&] {
+    return pb_dense_dot(tokens, (const uint8_t*)t.q.data_ptr(), (const uint8_t*)t.s8.data_ptr(), (const float*)t.s32.data_ptr(), rows, cols, a, b, g.data_ptr(), type, free,
+                        (float*)out->data_ptr(), bytes ? ws.data_ptr() : nullptr, bytes, st);
+  });
+}
+
+// linear_forward(x, w_sc8, w_sc32, w_t, b, fake, tokens) -> (y, x's triple[, the triple of x^T][, the scales of y]): _LinearFn.forward for a weight
+// on (128, b).  tokens: the triple of x^T is wanted (rows a multiple of 1024).
+OP(linear_forward) {
+  HANDLE_TH_ERRORS
+  NARGS(7);
+  const bool fake = PyObject_IsTrue(args[5]) == 1, tokens = PyObject_IsTrue(args[6]) == 1;
+  const at::Tensor *w8 = plain(args[1]), *w32 = plain(args[2]), *wt = plain(args[3]);
+  const int b = small(args[4]);
+  if (!w8 || !w32 || !wt || wt->dim() != 2 || !fp8(*wt) || !linear_fits(args[0], false, wt->size(1), wt->size(0), b, fake, wt->device())) return none();
+  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  const int64_t depth = wt->size(1), cols = wt->size(0), rows = x.numel() / depth;
+  if (tokens && rows % 1024) return none();
+  const c10::cuda::CUDAGuard guard(wt->device());
+  void* st = current_stream(wt->device());
+  Triple q, t;
+  int status = tokens ? dual_form(x, rows, depth, PB_E4M3, &q, &t, st) : rows_form(x, rows, depth, PB_E4M3, &q, st);
+  if (status != PB_OK) return raise_status(status);
+  at::Tensor d, s8, s32;
+  if ((status = product(q, {*wt, *w8, *w32}, b, 1, &d, st)) != PB_OK) return raise_status(status);
+  c10::SmallVector<int64_t, 8> shape(x.sizes().begin(), x.sizes().end());
+  shape.back() = cols;
+  at::Tensor y;
+  if (fake) {
+    const int64_t groups = rows * (cols / 128) / 8;
+    y = empty(shape, x.scalar_type(), x);
+    s8 = empty({groups, 8}, kE8M0, x); s32 = empty({groups, 1, 1}, at::kFloat, x);
+    RUN(pb_fake_quantize_scales(d.data_ptr(), PB_F32, 1, rows, cols, 1, 128, PB_E4M3, y.data_ptr(), code(x.scalar_type()), (uint8_t*)s8.data_ptr(), (float*)s32.data_ptr(), st));
+  } else {
+    y = d.view(shape);
+  }
+  if (tokens && fake) return wrap({y, q.q, q.s8, q.s32, t.q, t.s8, t.s32, s8, s32});
+  if (tokens) return wrap({y, q.q, q.s8, q.s32, t.q, t.s8, t.s32});
+  if (fake) return wrap({y, q.q, q.s8, q.s32, s8, s32});
+  return wrap({y, q.q, q.s8, q.s32});
+  END_HANDLE_TH_ERRORS
+}
+
+// linear_backward(g, x_q, x_sc8, x_sc32, w_q, w_sc8, w_sc32, t_q, t_sc8, t_sc32, y_sc8, y_sc32, b, format, x_dtype) -> (gx [rows, depth], gw):
+// _LinearFn.backward for a weight on (128, b).  t: the triple of x^T, for products of fp8 gradients in `format`, or None: literal dots.  y: the
+// scales of a fake-quantized output, or None.
+OP(linear_backward) {
+  HANDLE_TH_ERRORS
+  NARGS(15);
+  const at::Tensor* in[12];
+  for (int i = 0; i < 12; ++i) {
+    const bool may_miss = i >= 7;
+    if (may_miss && args[i] == Py_None) { in[i] = nullptr; continue; }
+    if (!(in[i] = plain(args[i]))) return none();
+  }
+  const bool tokens = in[7] && in[8] && in[9], fake = in[10] && in[11];
+  const int b = small(args[12]), fmt = small(args[13]);
+  const at::Tensor &xq = *in[1], &wq = *in[4];
+  if (watched() || !THPDtype_Check(args[14]) || (b != 128 && b != 1) || (fake && b != 128) || (tokens && b != 128) || xq.dim() != 2 || wq.dim() != 2 || xq.scalar_type() != kE4M3 ||
+      wq.scalar_type() != kE4M3 || xq.numel() == 0 || wq.numel() == 0 || !dense(in[0]->scalar_type()))
+    return none();
+  const at::ScalarType x_type = reinterpret_cast<THPDtype*>(args[14])->scalar_type;
+  const int64_t rows = xq.size(0), depth = xq.size(1), cols = wq.size(1);
+  if (!dense(x_type) || wq.size(0) != depth || depth % 128 || cols % (b == 128 ? 128 : 16) || (rows * (depth / 128)) % 8 || (fake && (rows * (cols / 128)) % 8) ||
+      in[0]->dim() < 1 || in[0]->size(-1) != cols || in[0]->numel() != rows * cols || (tokens && (rows % 1024 || !fp8(*in[7]))) ||
+      ((reinterpret_cast<uintptr_t>(in[0]->data_ptr()) | reinterpret_cast<uintptr_t>(xq.data_ptr()) | reinterpret_cast<uintptr_t>(wq.data_ptr())) & 15))
+    return none();
+  const size_t w_bytes = pb_fake_quantize_blocks_workspace_size(1, depth, cols, 128, b);
+  if (!w_bytes) return none();
+  const c10::cuda::CUDAGuard guard(xq.device());
+  void* st = current_stream(xq.device());
+  at::Tensor g = *in[0], gx, gw;
+  int status = PB_OK;
+  if (tokens) {
+    Triple q, t;
+    if (fake && g.scalar_type() == at::kFloat && cols % 1024 == 0) {
+      const int64_t groups = rows * cols / 1024;
+      q = {empty({rows, cols}, fmt == PB_E4M3 ? kE4M3 : kE5M2, g), empty({groups, 8}, kE8M0, g), empty({groups, 1, 1}, at::kFloat, g)};
+      t = tokens_form(g, rows, cols, fmt);
+      RUN(pb_dequantize_bwd_quantize_dual((const float*)g.data_ptr(), (const uint8_t*)in[10]->data_ptr(), (const float*)in[11]->data_ptr(), rows, cols, fmt, (uint8_t*)q.q.data_ptr(),
+                                          (uint8_t*)q.s8.data_ptr(), (float*)q.s32.data_ptr(), (uint8_t*)t.q.data_ptr(), (uint8_t*)t.s8.data_ptr(), (float*)t.s32.data_ptr(), st));
+    } else {
+      if (fake) {
+        at::Tensor scaled = empty(g.sizes(), g.scalar_type(), g);
+        RUN(pb_dequantize_bwd(g.data_ptr(), code(g.scalar_type()), (const uint8_t*)in[10]->data_ptr(), (const float*)in[11]->data_ptr(), 1, rows, cols, 1, 128, scaled.data_ptr(), st));
+        g = scaled;
+      }
+      if ((status = dual_form(g, rows, cols, fmt, &q, &t, st)) != PB_OK) return raise_status(status);
+    }
+    if ((status = product(q, {wq, *in[5], *in[6]}, 128, 0, &gx, st)) != PB_OK || (status = product({*in[7], *in[8], *in[9]}, t, 1, 0, &gw, st)) != PB_OK) return raise_status(status);
+  } else {
+    if (fake) {
+      at::Tensor scaled = empty(g.sizes(), g.scalar_type(), g);
+      RUN(pb_dequantize_bwd(g.data_ptr(), code(g.scalar_type()), (const uint8_t*)in[10]->data_ptr(), (const float*)in[11]->data_ptr(), 1, rows, cols, 1, 128, scaled.data_ptr(), st));
+      g = scaled;
+    }
+    if ((status = literal_dot(0, {wq, *in[5], *in[6]}, 128, b, g, rows, cols, &gx, st)) != PB_OK ||
+        (status = literal_dot(1, {xq, *in[2], *in[3]}, 1, 128, g, rows, cols, &gw, st)) != PB_OK)
+      return raise_status(status);
+  }
+  at::Tensor dx = empty({rows, depth}, x_type, xq);
+  RUN(pb_fake_quantize(gx.data_ptr(), PB_F32, 1, rows, depth, 1, 128, PB_E4M3, dx.data_ptr(), code(x_type), st));
+  gx.reset();
+  at::Tensor dw = empty({depth, cols}, at::kFloat, xq), ws = scratch(w_bytes, xq);
+  RUN(pb_fake_quantize_blocks((const float*)gw.data_ptr(), 1, depth, cols, 128, b, (float*)dw.data_ptr(), ws.data_ptr(), w_bytes, st));
+  return wrap({dx, dw});
+  END_HANDLE_TH_ERRORS
+}
+
 // linear_step(x, rows, k, n, dtype, format, b operand, workspace, b prepared, relu2) -> (d, q, sc8, sc32): LinearStep.__call__
 OP(linear_step) {
   HANDLE_TH_ERRORS
@@ -516,6 +688,7 @@ PyObject* set_error(PyObject*, PyObject* cls) {
 PyMethodDef methods[] = {
     METHOD("quantize", quantize), METHOD("quantize_transposed", quantize_transposed), METHOD("dequantize", dequantize), METHOD("dequantize_bwd", dequantize_bwd),
     METHOD("fake_quantize", fake_quantize), METHOD("transpose_bytes", transpose_bytes), METHOD("gemm", gemm), METHOD("linear_step", linear_step), METHOD("linear", linear), METHOD("linear_takes", linear_takes),
+    METHOD("linear_forward", linear_forward), METHOD("linear_backward", linear_backward),
     METHOD("dense_dot", dense_dot), METHOD("empty", empty_on), METHOD("empties", empties),
     ENTRY(pb_quantize_dual), ENTRY(pb_dequantize_bwd_quantize_dual), ENTRY(pb_relu2_requantize), ENTRY(pb_quantize_transposed_workspace_size),
     ENTRY(pb_wkv7_forward), ENTRY(pb_wkv7_backward), ENTRY(pb_wkv7_checkpoint_floats),
