@@ -172,8 +172,8 @@ __device__ __forceinline__ float2 div_hoisted_unsigned2(float2 x, float2 nD2, fl
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi);
 __device__ __forceinline__ uint32_t div_hoisted_pack2(float x0, float x1, float2 nD2, float2 r2) {
   const float2 q = div_hoisted_unsigned2(make_float2(x0, x1), nD2, r2);
-  const uint32_t sign = ((__float_as_uint(x0) >> 16) & 0x8000u) | (__float_as_uint(x1) & 0x80000000u);
-  return (pack_bf16x2(q.x, q.y) & 0x7fff7fffu) | sign;
+  const uint32_t upper = __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632);      // the halves that hold the signs
+  return (pack_bf16x2(q.x, q.y) & 0x7fff7fffu) | (upper & 0x80008000u);
 }
 __device__ __forceinline__ float div_hoisted(float x, float D, float r) {
   const float q = div_hoisted_unsigned(x, D, r);

@@ -664,10 +664,12 @@ transpose_quantize1024_f32_ring_kernel(const __grid_constant__ CUtensorMap map_x
       }
     } else if (LERP == 2) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int r = row_first + (i ^ swap);
-        w[i] = __fmul_rn(__fmul_rn(*reinterpret_cast<const float*>(tile + r * 64 + cp * 4), xs[r + (r >> 7)]), 0.0078125f);
-        cm = fmaxf(cm, fabsf(w[i]));
+      for (int i = 0; i < 32; i += 2) {
+        const int r = row_first + (i ^ swap), r1 = row_first + ((i + 1) ^ swap);
+        const float2 x = make_float2(*reinterpret_cast<const float*>(tile + r * 64 + cp * 4), *reinterpret_cast<const float*>(tile + r1 * 64 + cp * 4));
+        const float2 v = __fmul2_rn(__fmul2_rn(x, make_float2(xs[r + (r >> 7)], xs[r1 + (r1 >> 7)])), make_float2(0.0078125f, 0.0078125f));
+        w[i] = v.x; w[i + 1] = v.y;
+        cm = fmaxf(cm, fmaxf(fabsf(v.x), fabsf(v.y)));
       }
     } else if (LERP == 1) {
       if (row_first != 0) before = *reinterpret_cast<const float*>(tile + (row_first - 1) * 64 + cp * 4);
@@ -690,7 +692,7 @@ transpose_quantize1024_f32_ring_kernel(const __grid_constant__ CUtensorMap map_x
         cm = fmaxf(cm, fabsf(w[i]));
       }
     }
-    const int qswap = LERP == 1 ? 0 : swap;       // the lerp prologue leaves the registers in row order
+    const uint32_t bytes = LERP != 1 && swap ? 0x4501u : 0x5410u;      // the lerp prologue leaves the registers in row order
     float (*pa)[16] = part_amax[grp * 2 + (local & 1)];
     pa[blk * 4 + quarter][cp] = cm;
     int give_up;
@@ -720,10 +722,9 @@ transpose_quantize1024_f32_ring_kernel(const __grid_constant__ CUtensorMap map_x
     uint32_t out[8];
 #pragma unroll
     for (int i = 0; i < 32; i += 4) {
-      // rows i..i+3 of the column; the registers of the upper half-warp hold each pair of rows swapped
-      const uint32_t p0 = div_hoisted_pack2(qswap ? w[i + 1] : w[i], qswap ? w[i] : w[i + 1], nD2, r2);
-      const uint32_t p1 = div_hoisted_pack2(qswap ? w[i + 3] : w[i + 2], qswap ? w[i + 2] : w[i + 3], nD2, r2);
-      out[i >> 2] = bf16x2_to_fp8x2<FMT>(p0) | (bf16x2_to_fp8x2<FMT>(p1) << 16);
+      // rows i..i+3 of the column; the registers of the upper half-warp hold each pair of rows swapped, and their bytes are swapped back
+      const uint32_t p0 = div_hoisted_pack2(w[i], w[i + 1], nD2, r2), p1 = div_hoisted_pack2(w[i + 2], w[i + 3], nD2, r2);
+      out[i >> 2] = __byte_perm(bf16x2_to_fp8x2<FMT>(p0), bf16x2_to_fp8x2<FMT>(p1), bytes);
     }
     uint8_t* o = q_t + col * rows + r0 + row_first;
     asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
