@@ -30,6 +30,8 @@ constexpr int kVecs = 6;          // decay, iclr, removal_k, replacement_k, v, r
 constexpr int kCk = 8;            // spacing of the state checkpoints the backward pass restarts from
 constexpr int kSub = 4;           // timesteps whose recomputed states the backward pass keeps at once
 constexpr int kBwdVecs = kVecs + 2;      // the six inputs, dy and sa
+constexpr int kNegB = kBwdVecs;          // and -b = -(a o kap), made from them
+constexpr int kBwdSlots = kBwdVecs + 1;
 constexpr int kTileQuads = kH * kH / 4;  // float4 per state
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
@@ -492,8 +494,9 @@ int launch_forward(const WkvParams& p, int64_t heads, cudaStream_t st) {
 //     dkap_t = S_{t-1}^T dsa_t + db_t * a_t  da_t  = db_t * kap_t             dS_{t-1} = G_t diag(w_t) + dsa_t kap_t^T
 // Warp q owns rows 16q .. 16q+15; its lanes form a 2 x 16 grid and a lane keeps 8 rows (as float2 row pairs) x 4 columns of dS
 // and of S_{t-1}: per timestep it reads 4 elements of five vectors and 8 of three, and a column's sum needs one shuffle.  dsa,
-// the only sum that the recurrence waits for, is reduced first (a reduce-scatter over the sixteen lanes and eight
-// broadcasts), and everything that only leaves the kernel is formed behind it.  dr_t = S_t^T dy_t is formed a timestep later
+// the only sum that the recurrence waits for, goes first, and dv with it: the upper eight of a row's sixteen lanes hand over
+// their parts of dsa for those of dv, four levels of shuffles instead of twice four, between the products of the sums that only
+// leave the kernel, whose own shuffles go out together.  dr_t = S_t^T dy_t is formed a timestep later
 // in the walk, where S_t is the state at hand: put together from S_{t-1} instead, w o (S_{t-1}^T dy) - b (sa . dy) + kt (v . dy),
 // it loses what a timestep writes where it has just erased something larger.
 //
@@ -505,9 +508,11 @@ int launch_forward(const WkvParams& p, int64_t heads, cudaStream_t st) {
 // column sums of four timesteps wait in shared memory for one block barrier.  The chunk's eight vectors per timestep
 // arrive by cp.async one chunk ahead, and the next checkpoint into the slot that the upper half has emptied.
 //
-// Bound by the bytes its shared-memory reads and shuffles return and by its f32x2 products, both near 1300 of the 1950 cycles
-// a timestep takes with two heads on an SM.  8 x 32 heads x 1024 timesteps 1577 -> 1030 us, 32 heads 1035 -> 698 us, against
-// 4 x 8 tiles with every state in shared memory and a barrier per timestep.
+// Bound by its f32x2 products, three cycles each where their operands are three different registers (some 1450 of the 1850
+// cycles a timestep takes with two heads on an SM), and by what shuffles and shared memory return (half of their rate).
+// 8 x 32 heads x 1024 timesteps 1577 -> 1030 us, 32 heads 1035 -> 698 us, against 4 x 8 tiles with every state in shared memory
+// and a barrier per timestep; 256 heads 1016 -> 994, 32 heads 685 -> 663 by the sums' shuffles as above, 988 and 661 by stores of
+// column sums to all banks, 979 and 650 by -b made once per chunk, 965 and 635 by the erasure's products (below).
 struct WkvBwdParams {
   const float* in[kVecs];
   const float* dy;                // [B, T, C]
@@ -521,7 +526,7 @@ struct WkvBwdParams {
 
 struct WkvBwdSmem {
   float4 slot[2][kTileQuads];               // every thread its own quads: the chunk's checkpoint, and the state before its timestep 4
-  float vec[2][kCk][kBwdVecs][kH];          // the chunk's vectors, two chunks
+  float vec[2][kCk][kBwdSlots][kH];         // the chunk's vectors and -b, two chunks
   float col_part[2][kSub][kWarps][5][kH];   // two halves of a chunk: [timestep][warp][S^T dy of the timestep before, dkt, sum G sa, dw, S^T dsa][column]
   float dy_before[2][kH];                   // dy of the timestep before the chunk, two chunks (the first has none: what it reads is dropped)
   float last_part[kWarps][kH];              // S^T dy of the last timestep, a warp's rows each
@@ -549,23 +554,34 @@ __device__ __forceinline__ void ld_rows(const float* p, float2 (&out)[4]) {
   const float4 lo = *reinterpret_cast<const float4*>(p), hi = *reinterpret_cast<const float4*>(p + 4);
   out[0] = make_float2(lo.x, lo.y); out[1] = make_float2(lo.z, lo.w); out[2] = make_float2(hi.x, hi.y); out[3] = make_float2(hi.z, hi.w);
 }
-// Eight row values over the sixteen lanes of a tile row: lane tj ends with the sum of row tj >> 1.
-__device__ __forceinline__ float rows_reduce_scatter(const float2 (&v)[4], int tj) {
-  const bool b3 = tj & 8, b2 = tj & 4, b1 = tj & 2;
-  float2 k0 = b3 ? v[2] : v[0], k1 = b3 ? v[3] : v[1];
-  const float2 s0 = b3 ? v[0] : v[2], s1 = b3 ? v[1] : v[3];
-  k0.x += __shfl_xor_sync(0xffffffffu, s0.x, 8); k0.y += __shfl_xor_sync(0xffffffffu, s0.y, 8);
-  k1.x += __shfl_xor_sync(0xffffffffu, s1.x, 8); k1.y += __shfl_xor_sync(0xffffffffu, s1.y, 8);
-  float2 k = b2 ? k1 : k0;
-  const float2 s = b2 ? k0 : k1;
-  k.x += __shfl_xor_sync(0xffffffffu, s.x, 4); k.y += __shfl_xor_sync(0xffffffffu, s.y, 4);
-  float r = (b1 ? k.y : k.x) + __shfl_xor_sync(0xffffffffu, b1 ? k.x : k.y, 2);
-  return r + __shfl_xor_sync(0xffffffffu, r, 1);
+// sum over a lane's rows of M * x, column by column, each still as a row pair
+__device__ __forceinline__ void column_sums(const BwdTile& M, const float2 (&x)[4], float2 (&sum)[4]) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(M[0][c], x[0]);
+#pragma unroll
+  for (int rp = 1; rp < 4; ++rp)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(M[rp][c], x[rp], sum[c]);
 }
-// Four column sums (each still as a row pair) over the two lanes of a tile column: lane ti ends with columns 2 ti, 2 ti + 1.
-__device__ __forceinline__ float2 cols_reduce_scatter(const float2 (&v)[4], int ti) {
-  const float c0 = v[0].x + v[0].y, c1 = v[1].x + v[1].y, c2 = v[2].x + v[2].y, c3 = v[3].x + v[3].y;
-  return make_float2((ti ? c2 : c0) + __shfl_xor_sync(0xffffffffu, ti ? c0 : c2, 16), (ti ? c3 : c1) + __shfl_xor_sync(0xffffffffu, ti ? c1 : c3, 16));
+// sum over a lane's columns of M * x, row by row
+__device__ __forceinline__ void row_sums(const BwdTile& M, float4 x, float2 (&sum)[4]) {
+  const float2 x2[4] = {dup(x.x), dup(x.y), dup(x.z), dup(x.w)};
+#pragma unroll
+  for (int rp = 0; rp < 4; ++rp) sum[rp] = __fmul2_rn(M[rp][0], x2[0]);
+#pragma unroll
+  for (int c = 1; c < 4; ++c)
+#pragma unroll
+    for (int rp = 0; rp < 4; ++rp) sum[rp] = __ffma2_rn(M[rp][c], x2[c], sum[rp]);
+}
+__device__ __forceinline__ float2 from_lane_xor(float2 v, int mask) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, mask), __shfl_xor_sync(0xffffffffu, v.y, mask));
+}
+__device__ __forceinline__ float2 plus(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+// Four column sums over the two lanes of a tile column: a lane ends with columns 2 tc, 2 tc + 1, and gives the other two away.
+struct ColumnPair { float2 keep, give; };
+__device__ __forceinline__ ColumnPair split_columns(const float2 (&v)[4], int tc) {
+  const float2 lo = make_float2(v[0].x + v[0].y, v[1].x + v[1].y), hi = make_float2(v[2].x + v[2].y, v[3].x + v[3].y);
+  return tc ? ColumnPair{hi, lo} : ColumnPair{lo, hi};
 }
 
 __global__ void __launch_bounds__(kThreads, 2)
@@ -575,6 +591,7 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
   WkvBwdSmem& sm = *reinterpret_cast<WkvBwdSmem*>(wkv_bwd_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ti = lane >> 4, tj = lane & 15, row0 = 16 * warp + 8 * ti, col0 = 4 * tj;
+  const int tc = ti ^ (tj >> 3);  // which two of its four columns a lane's sums end with: sixteen lanes then store to all banks
   const int n = blockIdx.x % p.N, b = blockIdx.x / p.N;
   const int C = p.N * kH;
   const size_t head_base = (size_t)b * p.T * C + (size_t)n * kH;
@@ -616,129 +633,97 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
     }
     cp_async_commit();
   };
-  // to = from * w - sa b^T + v kt^T on the tile, rounded as the forward pass rounds it
+  // to = from * w - sa b^T + v kt^T on the tile, rounded as the forward pass rounds it.  The erasure's products one at a time: a
+  // packed one wants its column twice, and 256 heads x 1024 timesteps were then 976 us against 957 (other products
+  // one at a time as well: 956 to 1011).
   auto update = [&](const float (*buf)[kH], const BwdTile& from, BwdTile& to) {
-    const float4 w4 = *reinterpret_cast<const float4*>(buf[0] + col0), a4 = *reinterpret_cast<const float4*>(buf[1] + col0);
-    const float4 k4 = *reinterpret_cast<const float4*>(buf[2] + col0), t4 = *reinterpret_cast<const float4*>(buf[3] + col0);
+    const float4 w4 = *reinterpret_cast<const float4*>(buf[0] + col0), b4 = *reinterpret_cast<const float4*>(buf[kNegB] + col0);
+    const float4 t4 = *reinterpret_cast<const float4*>(buf[3] + col0);
     const float2 w[4] = {dup(w4.x), dup(w4.y), dup(w4.z), dup(w4.w)}, kt[4] = {dup(t4.x), dup(t4.y), dup(t4.z), dup(t4.w)};
-    const float2 nb[4] = {dup(-(a4.x * k4.x)), dup(-(a4.y * k4.y)), dup(-(a4.z * k4.z)), dup(-(a4.w * k4.w))};
+    const float nb[4] = {b4.x, b4.y, b4.z, b4.w};
     float2 v[4], sa[4];
     ld_rows(buf[4] + row0, v); ld_rows(buf[kVecs + 1] + row0, sa);
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-      for (int rp = 0; rp < 4; ++rp) to[rp][c] = __ffma2_rn(from[rp][c], w[c], __fmul2_rn(sa[rp], nb[c]));
+      for (int rp = 0; rp < 4; ++rp) to[rp][c] = __ffma2_rn(from[rp][c], w[c], make_float2(sa[rp].x * nb[c], sa[rp].y * nb[c]));
 #pragma unroll
     for (int rp = 0; rp < 4; ++rp)
 #pragma unroll
       for (int c = 0; c < 4; ++c) to[rp][c] = __ffma2_rn(v[rp], kt[c], to[rp][c]);
   };
+  const bool upper = tj & 8;        // of the sixteen lanes of a tile row
+  const int mine_at = (upper ? 3 : kNegB) * kH + col0, theirs_at = (upper ? kNegB : 3) * kH + col0, col = col0 + 2 * tc;
   float2 dy[4];                     // of the timestep that goes backwards next
-  // one timestep backwards, S the state before it, which is also the one after the timestep before: dr of that one, whose dy
+  // One timestep backwards, S the state before it, which is also the one after the timestep before: dr of that one, whose dy
   // is at `dy_below`
   auto back = [&](const float (*buf)[kH], const float* dy_below, const BwdTile& S, float (*part)[kH], size_t out) {
-    float2 nb[4], kap[4], rds[4];
-    {
-      const float4 a4 = *reinterpret_cast<const float4*>(buf[1] + col0), k4 = *reinterpret_cast<const float4*>(buf[2] + col0);
-      const float4 r4 = *reinterpret_cast<const float4*>(buf[5] + col0);
-      kap[0] = dup(k4.x); kap[1] = dup(k4.y); kap[2] = dup(k4.z); kap[3] = dup(k4.w);
-      nb[0] = dup(-(a4.x * k4.x)); nb[1] = dup(-(a4.y * k4.y)); nb[2] = dup(-(a4.z * k4.z)); nb[3] = dup(-(a4.w * k4.w));
-      const float2 r[4] = {dup(r4.x), dup(r4.y), dup(r4.z), dup(r4.w)};
-      // G = dS + dy r^T, and dsa = -G b: the only sum the recurrence waits for, so it goes first
+    const float4 k4 = *reinterpret_cast<const float4*>(buf[2] + col0), r4 = *reinterpret_cast<const float4*>(buf[5] + col0);
+    const float2 kap[4] = {dup(k4.x), dup(k4.y), dup(k4.z), dup(k4.w)}, r[4] = {dup(r4.x), dup(r4.y), dup(r4.z), dup(r4.w)};
+    // G = dS + dy r^T
 #pragma unroll
-      for (int rp = 0; rp < 4; ++rp)
+    for (int rp = 0; rp < 4; ++rp)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) dS[rp][c] = __ffma2_rn(dy[rp], r[c], dS[rp][c]);
+      for (int c = 0; c < 4; ++c) dS[rp][c] = __ffma2_rn(dy[rp], r[c], dS[rp][c]);
+    // dsa = -G b and dv = G kt, summed over the sixteen lanes of a tile row together: the lower eight lanes keep dsa, the upper ones dv,
+    // and every further level halves the rows.  The levels wait for shuffles between the products of the sums that only leave.
+    float2 rows[4], away[4];
+    row_sums(dS, *reinterpret_cast<const float4*>(buf[0] + theirs_at), away);
 #pragma unroll
-      for (int rp = 0; rp < 4; ++rp) rds[rp] = __fmul2_rn(dS[rp][0], nb[0]);
+    for (int rp = 0; rp < 4; ++rp) away[rp] = from_lane_xor(away[rp], 8);
+    row_sums(dS, *reinterpret_cast<const float4*>(buf[0] + mine_at), rows);
 #pragma unroll
-      for (int c = 1; c < 4; ++c)
+    for (int rp = 0; rp < 4; ++rp) rows[rp] = plus(rows[rp], away[rp]);
+    const bool b2 = tj & 4, b1 = tj & 2, b0 = tj & 1;
+    const float2 away0 = from_lane_xor(b2 ? rows[0] : rows[2], 4), away1 = from_lane_xor(b2 ? rows[1] : rows[3], 4);
+    float2 x[4], dkt[4], db[4], dr[4], dw[4];
+    ld_rows(buf[4] + row0, x);
+    column_sums(dS, x, dkt);
+    const float2 four0 = plus(b2 ? rows[2] : rows[0], away0), four1 = plus(b2 ? rows[3] : rows[1], away1);
+    const float2 away2 = from_lane_xor(b1 ? four0 : four1, 2);
+    ld_rows(buf[kVecs + 1] + row0, x);
+    column_sums(dS, x, db);
+    const float2 two = plus(b1 ? four1 : four0, away2);
+    const float row_sum = (b0 ? two.y : two.x) + __shfl_xor_sync(0xffffffffu, b0 ? two.x : two.y, 1);       // of row tj & 7
 #pragma unroll
-        for (int rp = 0; rp < 4; ++rp) rds[rp] = __ffma2_rn(dS[rp][c], nb[c], rds[rp]);
-    }
-    const float dsa_row = rows_reduce_scatter(rds, tj);
+    for (int c = 0; c < 4; ++c) dw[c] = __fmul2_rn(S[0][c], dS[0][c]);
+#pragma unroll
+    for (int rp = 1; rp < 4; ++rp)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) dw[c] = __ffma2_rn(S[rp][c], dS[rp][c], dw[c]);
     float2 dsa[4];
 #pragma unroll
     for (int rp = 0; rp < 4; ++rp) {
-      dsa[rp].x = __shfl_sync(0xffffffffu, dsa_row, (lane & 16) + 4 * rp);
-      dsa[rp].y = __shfl_sync(0xffffffffu, dsa_row, (lane & 16) + 4 * rp + 2);
+      dsa[rp].x = __shfl_sync(0xffffffffu, row_sum, (lane & 16) + 2 * rp);
+      dsa[rp].y = __shfl_sync(0xffffffffu, row_sum, (lane & 16) + 2 * rp + 1);
     }
-    const int col = col0 + 2 * ti;
-    // the sums that only leave: dv along the rows, the others along the columns
-    {
-      float2 v[4], sum[4], dvp[4];
-      ld_rows(buf[4] + row0, v);
-      const float4 t4 = *reinterpret_cast<const float4*>(buf[3] + col0);
-      const float2 kt[4] = {dup(t4.x), dup(t4.y), dup(t4.z), dup(t4.w)};
+    if (upper) p.din[4][out + row0 + (tj & 7)] = row_sum;
+    ld_rows(dy_below + row0, dy);
+    column_sums(S, dy, dr);
+    const ColumnPair left[4] = {split_columns(dr, tc), split_columns(dkt, tc), split_columns(db, tc), split_columns(dw, tc)};
+    float2 got[4];
 #pragma unroll
-      for (int rp = 0; rp < 4; ++rp) dvp[rp] = __fmul2_rn(dS[rp][0], kt[0]);
+    for (int q = 0; q < 4; ++q) got[q] = from_lane_xor(left[q].give, 16);
+    const float4 w4 = *reinterpret_cast<const float4*>(buf[0] + col0);
+    const float2 w[4] = {dup(w4.x), dup(w4.y), dup(w4.z), dup(w4.w)};
+    float2 dkap[4];
 #pragma unroll
-      for (int c = 1; c < 4; ++c)
+    for (int rp = 0; rp < 4; ++rp)
 #pragma unroll
-        for (int rp = 0; rp < 4; ++rp) dvp[rp] = __ffma2_rn(dS[rp][c], kt[c], dvp[rp]);
-      const float dv = rows_reduce_scatter(dvp, tj);
-      if (!(tj & 1)) p.din[4][out + row0 + (tj >> 1)] = dv;
+      for (int c = 0; c < 4; ++c) dS[rp][c] = __fmul2_rn(dS[rp][c], w[c]);
+    column_sums(S, dsa, dkap);
+    const ColumnPair last = split_columns(dkap, tc);
+    *reinterpret_cast<float2*>(part[4] + col) = plus(last.keep, from_lane_xor(last.give, 16));
 #pragma unroll
-      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(dS[0][c], v[0]);
+    for (int rp = 0; rp < 4; ++rp)
 #pragma unroll
-      for (int rp = 1; rp < 4; ++rp)
+      for (int c = 0; c < 4; ++c) dS[rp][c] = __ffma2_rn(dsa[rp], kap[c], dS[rp][c]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(dS[rp][c], v[rp], sum[c]);
-      *reinterpret_cast<float2*>(part[1] + col) = cols_reduce_scatter(sum, ti);
-    }
-    {
-      float2 sa[4], sum[4];
-      ld_rows(buf[kVecs + 1] + row0, sa);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(dS[0][c], sa[0]);
-#pragma unroll
-      for (int rp = 1; rp < 4; ++rp)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(dS[rp][c], sa[rp], sum[c]);
-      *reinterpret_cast<float2*>(part[2] + col) = cols_reduce_scatter(sum, ti);
-    }
-    {
-      float2 sum[4], dw[4];
-      ld_rows(dy_below + row0, dy);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(S[0][c], dy[0]);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) dw[c] = __fmul2_rn(S[0][c], dS[0][c]);
-#pragma unroll
-      for (int rp = 1; rp < 4; ++rp) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(S[rp][c], dy[rp], sum[c]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) dw[c] = __ffma2_rn(S[rp][c], dS[rp][c], dw[c]);
-      }
-      *reinterpret_cast<float2*>(part[0] + col) = cols_reduce_scatter(sum, ti);
-      *reinterpret_cast<float2*>(part[3] + col) = cols_reduce_scatter(dw, ti);
-    }
-    {
-      const float4 w4 = *reinterpret_cast<const float4*>(buf[0] + col0);
-      const float2 w[4] = {dup(w4.x), dup(w4.y), dup(w4.z), dup(w4.w)};
-      float2 sum[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int rp = 0; rp < 4; ++rp) dS[rp][c] = __fmul2_rn(dS[rp][c], w[c]);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(S[0][c], dsa[0]);
-#pragma unroll
-      for (int rp = 0; rp < 4; ++rp) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) dS[rp][c] = __ffma2_rn(dsa[rp], kap[c], dS[rp][c]);
-        if (rp > 0) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(S[rp][c], dsa[rp], sum[c]);
-        }
-      }
-      *reinterpret_cast<float2*>(part[4] + col) = cols_reduce_scatter(sum, ti);
-    }
+    for (int q = 0; q < 4; ++q) *reinterpret_cast<float2*>(part[q] + col) = plus(left[q].keep, got[q]);
   };
   // The column sums of the half chunk's timesteps [lo, hi): every warp's part is in shared memory behind the barrier.  (The
   // other buffer is written by the next half, and this one again only behind that half's barrier.)
-  auto finish_columns = [&](const float (*V)[kBwdVecs][kH], const float (*part)[kWarps][5][kH], int t0, int lo, int hi) {
+  auto finish_columns = [&](const float (*V)[kBwdSlots][kH], const float (*part)[kWarps][5][kH], int t0, int lo, int hi) {
     __syncthreads();
     const int j = tid & (kH - 1);
     for (int s = lo + (tid >> 6); s < hi; s += 2) {
@@ -759,7 +744,7 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
     }
   };
   // Timesteps lo .. lo + count - 1 backwards, `first` holding the state before lo; the later ones' states stay in registers.
-  auto run_half = [&](const float (*V)[kBwdVecs][kH], const float* dy_below, const float4* first, int t0, int lo, int count, int half, BwdTile& S1) {
+  auto run_half = [&](const float (*V)[kBwdSlots][kH], const float* dy_below, const float4* first, int t0, int lo, int count, int half, BwdTile& S1) {
     float (*part)[kWarps][5][kH] = sm.col_part[half];
     const size_t out = head_base + (size_t)(t0 + lo) * C;
     BwdTile S2, S3;                   // S1 comes as the state before lo
@@ -783,8 +768,13 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
     __syncthreads();              // everyone is done with the vectors of the chunk after this one
     issue_vec(ck - 1);            // into the buffer that chunk used
     cp_async_wait<1>();           // this thread's copies of chunk ck, and of its checkpoint, have landed
+    if (t0 + (tid >> 4) < p.T) {  // a thread's own copies: -b of those columns
+      float (*mine)[kH] = sm.vec[ck & 1][tid >> 4];
+      const float4 a4 = *reinterpret_cast<const float4*>(&mine[1][(tid & 15) * 4]), k4 = *reinterpret_cast<const float4*>(&mine[2][(tid & 15) * 4]);
+      *reinterpret_cast<float4*>(&mine[kNegB][(tid & 15) * 4]) = make_float4(-(a4.x * k4.x), -(a4.y * k4.y), -(a4.z * k4.z), -(a4.w * k4.w));
+    }
     __syncthreads();              // ... and everyone's vectors
-    const float (*V)[kBwdVecs][kH] = sm.vec[ck & 1];
+    const float (*V)[kBwdSlots][kH] = sm.vec[ck & 1];
     if (ck == n_ck - 1) {         // the last timestep's dr takes the final state
       BwdTile S;
       load_quads(sm.slot[ck_slot], tid, S);
@@ -792,13 +782,9 @@ wkv7_backward_kernel(const __grid_constant__ WkvBwdParams p) {
       for (int s = 0; s < steps; ++s) update(V[s], S, S);
       ld_rows(V[steps - 1][kVecs] + row0, dy);
       float2 sum[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) sum[c] = __fmul2_rn(S[0][c], dy[0]);
-#pragma unroll
-      for (int rp = 1; rp < 4; ++rp)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) sum[c] = __ffma2_rn(S[rp][c], dy[rp], sum[c]);
-      *reinterpret_cast<float2*>(sm.last_part[warp] + col0 + 2 * ti) = cols_reduce_scatter(sum, ti);
+      column_sums(S, dy, sum);
+      const ColumnPair pair = split_columns(sum, tc);
+      *reinterpret_cast<float2*>(sm.last_part[warp] + col) = plus(pair.keep, from_lane_xor(pair.give, 16));
       __syncthreads();
       if (tid < kH) {
         float r = sm.last_part[0][tid];
