@@ -385,7 +385,7 @@ PB_API int pb_smoothed_xent_bwd(const float* logits, const int64_t* target, cons
  * (or bf16, widened exactly) cotangent g, for the Linears whose cotangent no 128-deep scale block can carry:
  *   tokens == 0:  out[g_free, rows] = g[g_free, cols] . dq(Q)[rows, cols]^T     Q on (128,128) or (128,1), cols % 16 == 0
  *   tokens == 1:  out[cols, g_free] = dq(Q)[rows, cols]^T . g[rows, g_free]     Q on (1,128), g_free % 4 == 0
- * with f32 products and sums over the whole f32 range (every f32 product as three exact bf16 tensor-core products; sums that
+ * with f32 products and sums over the whole f32 range (every f32 product as three exact bf16 tensor-core products, or as one where g is bf16 and the rest of a scale goes to the finished sum; sums that
  * are not finite that way are made again with plain f32 products).  q, g, out and the workspace are 16-byte aligned.  Any other grid or shape: PB_ERR_UNSUPPORTED, and a workspace size of 0.
  * pb_dense_dot_workspace_size is the least workspace; pb_dense_dot_workspace_best what the fastest form for this size and type of g
  * (PB_F32, PB_BF16) takes, which pb_dense_dot chooses where workspace_bytes allow it.  The two forms add in different orders: a result's

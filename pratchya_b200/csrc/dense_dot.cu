@@ -33,7 +33,7 @@
 // the same bits.
 //
 // Every tile converts what it reads, so an operand that many tiles share is converted many times: where 512 columns or more share
-// it and there is enough to do, split_dot.cu makes it ready once (split_dot_pays: 3000 tokens, 2048 x 2048, bf16 cotangent, dX 141 -> 75 us,
+// it and there is enough to do, split_dot.cu makes it ready once (split_dot_pays: 3000 tokens, 2048 x 2048, bf16 cotangent, dX 141 -> 38 us,
 // dW 178 -> 68).  Left to this form are few tokens, the low-rank layers' f32 cotangents and callers without the workspace.
 #include <algorithm>
 #include <atomic>
