@@ -263,6 +263,7 @@ PB_API int pb_quantize_dual(const void* x, int x_dtype, int64_t batch, int64_t r
  *      are f32 [batch, steps, heads*head_dim]; state_in / state_out are f32 [batch, heads, head_dim, head_dim]
  *      (state_in may be null for a zero state, state_out may be null); y is f32 [batch, steps, heads*head_dim],
  *      the order the reference has after its transpose (:210).  head_dim must be 64.  16-byte aligned arrays.
+ *      A sequence cut after any timestep and continued from state_out gives the bits of the whole one.
  *      `checkpoints` (may be null) receives the state before timesteps 0, 8, 16, ... as f32
  *      [batch, heads, ceil(steps/8), head_dim, head_dim] (pb_wkv7_checkpoint_floats elements): what
  *      pb_wkv7_backward restarts from.  `sa` (may be null) receives, for every timestep, the state before the step times

@@ -64,7 +64,8 @@ class _WkvScanFn(torch.autograd.Function):
 def wkv_state_scan(wkv_state, decay, iclr, removal_k, replacement_k, v, r, n_head: int):
     """(wkv_state', out): the scan of :187-207 over the T timesteps of six f32 [B, T, C] inputs from the
     initial state wkv_state [B, N, H, H] (None: zeros), with C = N * H and H = 64.  `out` is [B, T, C]
-    (the reference's order after its transpose, :210).  Differentiable in the six inputs and the state."""
+    (the reference's order after its transpose, :210).  Differentiable in the six inputs and the state.  A sequence cut after any
+    timestep and continued from wkv_state' gives the bits of the whole one."""
     ins = [decay, iclr, removal_k, replacement_k, v, r]
     shape = _check_inputs(ins, n_head)
     bsz, steps, chans = shape

@@ -52,33 +52,30 @@ __device__ __forceinline__ int ckpt_quad(int P, int Q) { return (2 * (P & 3) + (
 // warps, and where there are few heads over CTAs as well.  A warp's lanes are a grid of 2 x 16 or 4 x 8; a lane keeps ROWS rows x 4
 // or 8 columns, and a row's dot products end in shuffles.
 //
-// The chain.  sa_{t+1} = S_t kap_{t+1} taken as it stands makes every timestep wait for a dot product, its shuffles and the
-// update in turn.  With S_t written out it is
-//     sa_{t+1} = S_{t-1} (w_t o kap_{t+1}) - (b_t . kap_{t+1}) sa_t + (kt_t . kap_{t+1}) v_t         (b = a o kap)
-// whose only sum along the state's rows is over the state a timestep earlier: two timesteps' sums are under way at once, and
-// sa_t enters through two products.  The first timestep of every chunk of eight takes S kap as it stands, so that a scan cut at
-// multiples of eight and continued from its state gives the bits of the whole one.  What the form needs that does not depend on
-// the state (b, w_t o kap_{t+1}, the two scalars) warps of their own make a chunk ahead, once per CTA, from the chunk's vectors as
-// they arrive by cp.async; one barrier per chunk.
+// The chain.  sa_t = S_{t-1} kap_t waits for the timestep before, and everything else hangs on it: a dot product, a sum over lanes, the
+// update.  sa is taken of the state as it is stored, at every timestep: what rounding left in it is then read and erased with it, and a scan cut after
+// any timestep and continued from its state gives the bits of the whole one.  (Written with S_{t-1} in terms of S_{t-2}, whose sum could start a timestep
+// earlier, 16 heads take 101 us instead of 125, but a timestep behind one that has erased something large is off by 2^-24 of what was erased: one
+// key repeated, a value of 64 among others of size one, that timestep's y 4e-6 instead of 5e-8.)  b = a o kap is made a chunk ahead, once per CTA, by warps
+// of their own, from the chunk's vectors as they arrive by cp.async; one barrier per chunk.
 //
-// Sums.  p, the dot product that sa is made of, and y, the output's, are summed together: of two lanes half a row apart one keeps p
+// Sums.  sa of a timestep and y of the one before, both of the same state, are summed together: of two lanes half a row apart one keeps sa's part
 // and hands over its part of y, the other the reverse (each reads its two vectors in that order); a lane's rows are in an order
 // of its own (register a holds row a ^ its lane bits), so that every further halving hands over the upper registers and no value
-// is selected.  A row's p ends on lanes that make sa of it and broadcast that; its y on as many, which store it.  A sum's levels
+// is selected.  A row's sa ends on lanes that broadcast it; its y on as many, which store it.  A sum's levels
 // have the same order in every form, so the bits do not depend on the number of heads.
 //
 // The update is (S o w - sa b^T) + v kt^T with the erasure's product rounded and the other two fused: v kt^T comes last (added
 // to a state that is about to be erased, its low bits would go with it), and of the three roundings one is of the erased part's
-// size instead of the state's: 2-norm errors against 64 bits 9.8e-8 -> 9.1e-8 of y, 7.1e-8 -> 6.1e-8 of the state (500 timesteps;
-// keys that repeat or hardly decay: below the step-by-step form's too).
+// size instead of the state's: 2-norm errors against 64 bits 9.8e-8 -> 9.1e-8 of y, 7.1e-8 -> 6.0e-8 of the state (500 timesteps).
 //
-// What bounds it: with few heads what reads and shuffles return to the registers (146 of a timestep's 205 cycles on an SM of four
-// warps; one row group more per warp or per lane costs more in latency than it saves there), with many the f32x2 products,
-// three cycles each where their operands are three different registers, on top of those reads.  Two CTAs of a whole head an SM: four
-// preparing warps, one a scheduler (one alone made its scheduler the slowest: 128 heads 233 -> 212 us), which hand their registers over.
-// 1024 timesteps, against one timestep after the other with each lane's own b: 16 heads 125 -> 105 us (with saves 160 -> 114), 32 heads 147 -> 106
-// (163 -> 114), 60 heads 165 -> 134 (185 -> 149), 128 heads 221 -> 196 (257 -> 231), 160 heads 329 -> 333 (360 -> 364), 192 heads 358 -> 335
-// (428 -> 367), 256 heads 357 -> 346 (425 -> 395); 32 heads x 4096 572 -> 419.
+// What bounds it: with few heads the chain (235 cycles a timestep: five shuffles behind one another, the dot product and the update; sums that every
+// lane of a row makes, four shuffles but twice as many of them, 125 -> 129 us; vectors read in front of the shuffles, or between them, the same), with many
+// the f32x2 products, three cycles each where their operands are three different registers, on top of the reads.  Two CTAs of a whole head
+// an SM: four preparing warps, one a scheduler (one alone makes its scheduler the slowest), which hand their registers over.
+// 1024 timesteps, us, against each lane's own b and sums of sa and y one after the other: 16 heads 122 -> 125 (with saves 159 -> 131), 32 heads 144 -> 125
+// (160 -> 131), 60 heads 162 -> 145 (183 -> 157), 128 heads 218 -> 198 (254 -> 235), 160 heads 326 -> 327 (356 -> 360), 222 heads 354 -> 327 (424 -> 360),
+// 256 heads 353 -> 335 (423 -> 389); 32 heads x 4096 571 -> 492.
 constexpr int kFwdChunk = 8;      // timesteps between barriers
 constexpr int kFwdBufs = 5;       // chunks in shared memory: the one before, the one computed with, the one prepared, two under way
 
@@ -96,10 +93,7 @@ struct WkvParams {
 __device__ __forceinline__ void cta_meet() { asm volatile("bar.sync 0;" ::: "memory"); }
 
 struct WkvFwdChunk {
-  // decay, b (iclr as it arrives), removal_k, replacement_k, v, r, and what the state of timestep s is multiplied with for sa of
-  // timestep s + 2: w_{s+1} o kap_{s+2}.  (The last two hold what the state before the chunk meets: kap_0, w_0 o kap_1.)
-  float vec[kFwdChunk][kVecs + 1][kH];
-  float2 mix[kFwdChunk];                // (b_s . kap_{s+1}, kt_s . kap_{s+1}); the last one is not used
+  float vec[kFwdChunk][kVecs][kH];      // decay, b (iclr as it arrives), removal_k, replacement_k, v, r
 };
 
 // a lane's share of one timestep's vectors
@@ -107,7 +101,6 @@ template <int ROWS, int PAIRS>
 struct StepVecs {
   float2 w[PAIRS], b[PAIRS], kt[PAIRS];
   float v[ROWS];                  // register 0 is the row whose sums the lane ends with
-  float2 mix;
 };
 // a lane's columns of a shared-memory vector: four, or four and four 32 further on
 template <int PAIRS>
@@ -140,7 +133,6 @@ __device__ __forceinline__ void row_dots(const float2 (&S)[ROWS][PAIRS], const f
     for (int a = 0; a < ROWS; ++a) out[a] = p[a].x + p[a].y;
   }
 }
-template <int V> struct Int { static constexpr int value = V; };
 
 // A warp's lanes are a grid of 32 / LANES x LANES.  SAVE: checkpoints and sa are wanted (a backward pass follows).  PREP warps prepare the
 // chunks.
@@ -180,61 +172,24 @@ wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
       }
       cp_async_commit();
     };
-    // what a chunk's timesteps need beside its vectors; a lane two columns.  (Timesteps past the sequence's end: what the buffer
-    // holds, which nothing reads.)
+    // b of the warp's own timesteps; a lane two columns.  (Timesteps past the sequence's end: what the buffer holds, which nothing reads.)
     auto prepare = [&](int chunk) {
       WkvFwdChunk& at = ring[chunk % kFwdBufs];
-      const int j = 2 * lane;
-      float dots[2 * kPrepSteps];
-      float2 kap = *reinterpret_cast<const float2*>(&at.vec[s0][2][j]);
-      if (s0 == 0) *reinterpret_cast<float2*>(&at.vec[kFwdChunk - 2][kVecs][j]) = kap;
 #pragma unroll
-      for (int i = 0; i < kPrepSteps; ++i) {
-        const int s = s0 + i;
-        const float2 w = *reinterpret_cast<const float2*>(&at.vec[s][0][j]), a = *reinterpret_cast<const float2*>(&at.vec[s][1][j]);
-        const float2 kt = *reinterpret_cast<const float2*>(&at.vec[s][3][j]);
-        const float2 bb = make_float2(a.x * kap.x, a.y * kap.y);
-        *reinterpret_cast<float2*>(&at.vec[s][1][j]) = bb;
-        const bool more = s + 1 < kFwdChunk;
-        const float2 nxt = *reinterpret_cast<const float2*>(&at.vec[more ? s + 1 : s][2][j]);
-        if (more) *reinterpret_cast<float2*>(&at.vec[(s + kFwdChunk - 1) % kFwdChunk][kVecs][j]) = make_float2(w.x * nxt.x, w.y * nxt.y);
-        dots[2 * i] = __fmaf_rn(bb.y, nxt.y, bb.x * nxt.x);
-        dots[2 * i + 1] = __fmaf_rn(kt.y, nxt.y, kt.x * nxt.x);
-        kap = nxt;
+      for (int s = s0; s < s0 + kPrepSteps; ++s) {
+        const float2 a = *reinterpret_cast<const float2*>(&at.vec[s][1][2 * lane]), kap = *reinterpret_cast<const float2*>(&at.vec[s][2][2 * lane]);
+        *reinterpret_cast<float2*>(&at.vec[s][1][2 * lane]) = make_float2(a.x * kap.x, a.y * kap.y);
       }
-      // 2 * kPrepSteps sums over the warp, over lane bits 4, 3, 2, 1, 0 in turn whatever their number
-      int nv = 2 * kPrepSteps, index = 0;
-#pragma unroll
-      for (int m = 16; m >= 1; m /= 2) {
-        if (nv > 1) {
-          nv /= 2;
-          const bool hi = lane & m;
-#pragma unroll
-          for (int q = 0; q < kPrepSteps; ++q)
-            if (q < nv) {
-              const float keep = hi ? dots[q + nv] : dots[q], send = hi ? dots[q] : dots[q + nv];
-              dots[q] = keep + __shfl_xor_sync(0xffffffffu, send, m);
-            }
-          index += hi ? nv : 0;
-        } else {
-          dots[0] += __shfl_xor_sync(0xffffffffu, dots[0], m);
-        }
-      }
-      reinterpret_cast<float*>(&at.mix[s0])[index] = dots[0];      // lanes with the same index hold the same sum
-    };
-    auto producers_meet = [] {
-      if constexpr (PREP == 1) __syncwarp();
-      else asm volatile("bar.sync 1, %0;" ::"n"(32 * PREP) : "memory");
     };
 #pragma unroll
     for (int c = 0; c < kFwdBufs - 1; ++c) issue(c);
     cp_async_wait<kFwdBufs - 2>();
-    producers_meet();
+    __syncwarp();                               // the warp's vectors of chunk 0
     prepare(0);
     cta_meet();
     for (int c = 0; c < full; ++c) {
       cp_async_wait<kFwdBufs - 3>();
-      producers_meet();                         // everyone's vectors of chunk c + 1
+      __syncwarp();                             // the warp's vectors of chunk c + 1
       if (c + 1 < n_chunks) prepare(c + 1);
       cta_meet();                               // chunk c + 1 is ready, chunk c - 1 has been read
       issue(c + kFwdBufs - 1);
@@ -276,66 +231,34 @@ wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
     ld_cols(at.vec[s][0] + col0, x.w); ld_cols(at.vec[s][1] + col0, x.b); ld_cols(at.vec[s][3] + col0, x.kt);
 #pragma unroll
     for (int a = 0; a < ROWS; ++a) x.v[a] = at.vec[s][4][row0 + (a ^ own_row)];
-    x.mix = at.mix[s];
   };
-  // Parts of the sums that a state takes part in, not yet summed over lanes: pa the lane's kept one (p or y), pb the other,
-  // pc the second p of a chunk's first state.  half: the sums of the state before, but for their last level.
-  float pa[ROWS], pb[ROWS], pc[ROWS], half[1];
-  const int first_at = (for_y ? kVecs - 1 : kVecs) * kH + col0, second_at = (for_y ? kVecs : kVecs - 1) * kH + col0;
-  auto both_dots = [&](const float* x, const float* y) {
-    float2 x1[kPairs], x2[kPairs];
-    ld_cols(x, x1);
-    ld_cols(y, x2);
-    row_dots(S, x2, pb);
-    row_dots(S, x1, pa);
-  };
-  auto one_dot = [&](const float* x, float (&to)[ROWS]) {
-    float2 v[kPairs];
-    ld_cols(x + col0, v);
-    row_dots(S, v, to);
-  };
-  // The levels of a row's sum over lanes: with N registers left, the upper half of them goes to the lane that keeps those rows;
-  // with one, it is added.  A level is asked for and, when other work has passed, added.
-  float got[ROWS];
-  auto ask = [&](const float (&k)[ROWS], auto bit, auto regs) {
-    constexpr int M = decltype(bit)::value, N = decltype(regs)::value;
-    if constexpr (N > 1) {
+  // A state's parts of sa of the next timestep and of y of its own, not yet summed over lanes: pa the lane's kept one, pb the other.
+  float pa[ROWS], pb[ROWS];
+  const int kept_at = (for_y ? kVecs - 1 : kVecs + 2) * kH + col0, other_at = (for_y ? kVecs + 2 : kVecs - 1) * kH + col0;      // from r's or the next timestep's kap
+  // A row's sum over lanes: y's part goes to the lanes that keep y and sa's to the others, then the upper half of the registers left to
+  // the lane that keeps those rows; the last one is added.
+  auto sum_over_lanes = [&] {
+    float got[ROWS];
 #pragma unroll
-      for (int a = 0; a < N / 2; ++a) got[a] = __shfl_xor_sync(0xffffffffu, k[a + N / 2], M);
-    } else {
-      got[0] = __shfl_xor_sync(0xffffffffu, k[0], M);
+    for (int a = 0; a < ROWS; ++a) got[a] = __shfl_xor_sync(0xffffffffu, pb[a], LANES / 2);
+#pragma unroll
+    for (int a = 0; a < ROWS; ++a) pa[a] += got[a];
+    int left = ROWS;
+#pragma unroll
+    for (int m = LANES / 4; m >= 1; m /= 2) {
+      const int gives = left > 1 ? left / 2 : 0;          // the first register that goes
+      left = left > 1 ? left / 2 : 1;
+#pragma unroll
+      for (int a = 0; a < ROWS; ++a)
+        if (a < left) got[a] = __shfl_xor_sync(0xffffffffu, pa[(a + gives) % ROWS], m);
+#pragma unroll
+      for (int a = 0; a < ROWS; ++a)
+        if (a < left) pa[a] += got[a];
     }
-  };
-  auto add = [&](float (&k)[ROWS], auto regs) {
-    constexpr int N = decltype(regs)::value;
-#pragma unroll
-    for (int a = 0; a < (N > 1 ? N / 2 : 1); ++a) k[a] += got[a];
-  };
-  constexpr Int<ROWS> n2;
-  constexpr Int<ROWS / 2> n3;                   // sixteen lanes have one more level
-  constexpr Int<LANES == 16 ? (ROWS == 8 ? 2 : 1) : (ROWS == 4 ? 2 : 1)> n4;
-  constexpr Int<LANES / 4> m2;
-  constexpr Int<2> m3;
-  constexpr Int<1> m4;
-  auto first_level = [&](const float (&from_other)[ROWS]) {
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) got[a] = __shfl_xor_sync(0xffffffffu, from_other[a], LANES / 2);
-  };
-  auto add_first = [&](float (&k)[ROWS]) {
-#pragma unroll
-    for (int a = 0; a < ROWS; ++a) k[a] += got[a];
-  };
-  auto other_levels = [&](float (&k)[ROWS]) {   // with nothing in between
-    ask(k, m2, n2); add(k, n2);
-    if constexpr (LANES == 16) { ask(k, m3, n3); add(k, n3); }
-    ask(k, m4, n4); add(k, n4);
-    return k[0];
+    return pa[0];
   };
 
-  float nsa[ROWS];                              // -sa of the timestep, of the lane's rows
-  float own = 0.0f, own_before = 0.0f;          // of the row whose sums the lane ends with: the timestep's, the one's before
-  float y_held = 0.0f, v_before = 0.0f;
-  float2 mix_before = make_float2(0.0f, 0.0f);
+  float own = 0.0f;                             // -sa of the timestep before, of the row whose sums the lane ends with
   auto put = [&](int u, float val) {            // val: of a timestep, u = t % kSame
     if (part == u) keep = val;
     if (u == kSame - 1) {
@@ -344,50 +267,31 @@ wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
     }
   };
   Vecs cur, next;
-  float last_got[2];                            // the last level of the sum that makes the next timestep's sa, asked for
-  auto ask_last = [&](const float (&k)[ROWS]) {
-    half[0] = k[0];
-    last_got[0] = __shfl_xor_sync(0xffffffffu, k[decltype(n4)::value / 2], 1);
-  };
-  // Timestep s of chunk c.  Two sums over lanes are under way: the one over the state before the last, whose last level makes this
-  // timestep's sa (and y of two timesteps ago), and the one over the last state, whose levels are asked for between the products
-  // of the update, which wait for sa.
-  auto step = [&](int c, int s, auto is_first) {
-    constexpr bool first = decltype(is_first)::value;       // s == 0
+  // Timestep s of chunk c: the sums over lanes of the last state's parts, sa to all lanes, the update, the new state's parts.  The
+  // vectors that these want are read behind the shuffles (in front of them the shuffles queue behind the reads).
+  auto step = [&](int c, int s) {
     const WkvFwdChunk& at = ring[c % kFwdBufs];
     const WkvFwdChunk& after = ring[(c + 1) % kFwdBufs];
-    const float* const rec = &at.vec[0][0][0] + s * (kVecs + 1) * kH;
-    float y_done = half[0] + last_got[0];       // y of two timesteps ago, on the lanes that store it
-    const float sa_done = -own_before;
-    own_before = own;
-    if constexpr (first) {
-      first_level(pb);
-      add_first(pa);
-      first_level(pc);
-      add_first(pc);
-      y_held = other_levels(pa);
-      own = -y_held;                            // the lanes that do not store y: sa as it stands
-    } else {
-      const float x = y_done;
-      if (s == 1) y_done = y_held;
-      own = __fmaf_rn(-v_before, mix_before.y, __fmaf_rn(-own_before, mix_before.x, -x));
-    }
+    const float* const rec = &at.vec[s][0][0];
+    const float sum = sum_over_lanes();         // y of the timestep before, or sa
+    const float done = SAVE && !for_y ? -own : sum;
+    own = -sum;
+    float nsa[ROWS];                            // -sa of the lane's rows
 #pragma unroll
     for (int a = 0; a < ROWS; ++a) nsa[a] = __shfl_sync(0xffffffffu, own, from[a]);
-    float (&k)[ROWS] = first ? pc : pa;
-    if constexpr (!first) {
-      if (s + 1 == kFwdChunk) first_level(pa);
-      else first_level(pb);
-    }
+    float2 kept[kPairs], other[kPairs];
     if (s + 1 == kFwdChunk) {
       cta_meet();
+      const float *kap = after.vec[0][2] + col0, *r = rec + (kVecs - 1) * kH + col0;
+      ld_cols(for_y ? r : kap, kept);
+      ld_cols(for_y ? kap : r, other);
       load(next, after, 0);
     } else {
+      ld_cols(rec + kept_at, kept);
+      ld_cols(rec + other_at, other);
       load(next, at, s + 1);
     }
-    if (s > 1 || c > 0) put((s + kFwdChunk - 2) % kSame, SAVE && !for_y ? sa_done : y_done);
-    if constexpr (!first) add_first(k);
-    ask(k, m2, n2);
+    if (s > 0 || c > 0) put((s + kFwdChunk - 1) % kSame, done);
     float2 m[ROWS][kPairs];
 #pragma unroll
     for (int a = 0; a < ROWS; ++a)
@@ -397,25 +301,12 @@ wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
     for (int j = 0; j < kPairs; ++j)
 #pragma unroll
       for (int a = 0; a < ROWS; ++a) S[a][j] = __ffma2_rn(S[a][j], cur.w[j], m[a][j]);
-    add(k, n2);
-    if constexpr (LANES == 16) ask(k, m3, n3);
 #pragma unroll
     for (int a = 0; a < ROWS; ++a)
 #pragma unroll
       for (int j = 0; j < kPairs; ++j) S[a][j] = __ffma2_rn(dup(cur.v[a]), cur.kt[j], S[a][j]);
-    if constexpr (LANES == 16) add(k, n3);
-    ask_last(k);
-    if (s + 2 < kFwdChunk) {
-      both_dots(rec + first_at, rec + second_at);
-    } else if (s + 2 == kFwdChunk) {
-      one_dot(at.vec[s][kVecs - 1], pa);
-    } else {
-      const float *kap = after.vec[kFwdChunk - 2][kVecs] + col0, *r = at.vec[s][kVecs - 1] + col0;
-      both_dots(for_y ? r : kap, for_y ? kap : r);
-      one_dot(after.vec[kFwdChunk - 1][kVecs], pc);
-    }
-    v_before = cur.v[0];
-    mix_before = cur.mix;
+    row_dots(S, other, pb);
+    row_dots(S, kept, pa);
     cur = next;
   };
   auto checkpoint = [&](int c) {                // the state before the chunk (kCk == kFwdChunk), in the backward kernel's layout
@@ -435,33 +326,27 @@ wkv7_forward_kernel(const __grid_constant__ WkvParams p) {
 
   cta_meet();
   load(cur, ring[0], 0);
-  half[0] = last_got[0] = 0.0f;                       // y of no timestep, here and in the next
-  one_dot(ring[0].vec[kFwdChunk - 2][kVecs], pa);
+  {
+    float2 kap[kPairs];
+    ld_cols(ring[0].vec[0][2] + col0, kap);
+    row_dots(S, kap, pa);
 #pragma unroll
-  for (int a = 0; a < ROWS; ++a) pb[a] = pa[a];
-  one_dot(ring[0].vec[kFwdChunk - 1][kVecs], pc);
+    for (int a = 0; a < ROWS; ++a) pb[a] = pa[a];         // y of no timestep: not stored
+  }
   for (int c = 0; c < full; ++c) {
     checkpoint(c);
-    step(c, 0, Int<1>());
 #pragma unroll
-    for (int s = 1; s < kFwdChunk; ++s) step(c, s, Int<0>());
+    for (int s = 0; s < kFwdChunk; ++s) step(c, s);
   }
   const int tail = p.T - full * kFwdChunk;
   if (tail) {
     checkpoint(full);
-    step(full, 0, Int<1>());
 #pragma unroll 1
-    for (int s = 1; s < tail; ++s) step(full, s, Int<0>());
+    for (int s = 0; s < tail; ++s) step(full, s);
   }
-  // the last two timesteps' outputs are still open
-  const int t = p.T - 1, s_last = t % kFwdChunk, u = t % kSame;
-  if (t > 0) {
-    put((t - 1) % kSame, SAVE && !for_y ? -own_before : (s_last == 0 ? y_held : half[0] + last_got[0]));
-  }
-  if (s_last + 2 == kFwdChunk) first_level(pa);
-  else first_level(pb);
-  add_first(pa);
-  const float y_last = other_levels(pa);
+  // the last timestep's outputs are still open
+  const float y_last = sum_over_lanes();
+  const int u = (p.T - 1) % kSame;
   if (part == u) keep = SAVE && !for_y ? -own : y_last;
   if (part <= u && stores) *out = keep;
   if (p.state_out) {
@@ -846,8 +731,8 @@ extern "C" int pb_wkv7_forward(const float* decay, const float* iclr, const floa
   const int64_t n = batch * heads;
   // Rows of a head per CTA: 16, 32 or 64, as many CTAs as there are SMs and no more of them on one (each reads the head's vectors);
   // from a wave of whole heads to one and a half, three halves on an SM instead of two heads.  1024 timesteps, us, of the forms 16 |
-  // 32 | halves | 64: 32 heads 106 | 133 | 171 | 195, 74 heads 171 | 134 | 173 | 196, 96 heads 268 | 218 | 305 | 196, 160 heads 431 | 334 |
-  // 333 | 348 (with saves 466 | 437 | 364 | 397), 222 heads 501 | 334 | 335 | 347 (544 | 438 | 367 | 395), 256 heads 595 | 426 | 432 | 346.
+  // 32 | halves | 64: 37 heads 125 | 144 | 177 | 199, 74 heads 171 | 145 | 177 | 198, 96 heads 289 | 217 | 302 | 198, 160 heads 451 | 346 |
+  // 327 | 338 (with saves 479 | 378 | 359 | 391), 222 heads 507 | 345 | 327 | 336 (537 | 378 | 360 | 389), 256 heads 616 | 428 | 434 | 335.
   if (4 * n <= sm_count()) return launch_forward<2, 16, 4, 4, 1>(p, n, st);
   if (2 * n <= sm_count()) return launch_forward<4, 16, 4, 4, 1>(p, n, st);
   if (n > sm_count() && 2 * n <= 3 * sm_count()) return launch_forward<4, 8, 2, 2, 3>(p, n, st);

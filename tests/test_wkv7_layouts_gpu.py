@@ -69,3 +69,28 @@ def test_what_a_timestep_writes_where_it_erases_something_larger(built_lib, head
     for t in range(steps):
         got = dr[:, t, :, (5 * t) % 64]
         assert ((got - (v64[:, t] * dy64[:, t]).sum(-1)).abs() <= 65 * 2.0 ** -24 * (v64[:, t] * dy64[:, t]).abs().sum(-1)).all(), t
+
+
+@pytest.mark.parametrize("heads", [1, 60, 100, 160, 230])
+@pytest.mark.parametrize("iclr,decay,outlier", [(1.0, 1.0, 64.0), (1.0, 1.0, 1e6), (0.95, 0.99, 64.0), (0.95, 0.99, 1e4)])
+def test_the_timesteps_after_a_large_value_is_erased(built_lib, heads, iclr, decay, outlier):
+    """One key for all timesteps, read by itself, and a value far larger than the others in one of them.  The timestep behind it erases
+    what it wrote and keeps that write's rounding, 2^-24 of its size, which the next one reads in the stored state and erases with
+    it.  From there on each timestep is as accurate as its own sums: some twenty roundings of what it reads and of what it writes,
+    as a 2-norm over the rows no more than 8 * 2^-24 of both (1 to 2 seen)."""
+    steps = 24
+    g = torch.Generator(device="cuda").manual_seed(heads)
+    shape = (1, steps, heads * 64)
+    key = torch.nn.functional.normalize(torch.randn(1, 1, heads, 64, generator=g, device="cuda"), dim=-1).expand(1, steps, heads, 64).reshape(shape).contiguous()
+    full = lambda x: torch.full(shape, x, device="cuda")
+    v0 = torch.randn(shape, generator=g, device="cuda")
+    norm = lambda x: x.view(steps, heads, 64).double().norm(dim=-1)
+    for at in range(5, 13):           # wherever in a chunk of eight it comes
+        v = v0.clone()
+        v[:, at] *= outlier
+        ins = [full(decay), full(iclr), key, key, v, key]
+        _, y = wkv_state_scan(None, *ins, heads)
+        _, ref = _recurrence(torch.zeros(1, heads, 64, 64, device="cuda", dtype=torch.float64), [x.double() for x in ins], heads)
+        error, size = norm(y - ref), norm(ref)
+        for t in [*range(1, at), *range(at + 2, steps)]:
+            assert (error[t] <= 8 * 2.0 ** -24 * (size[t] + size[t - 1])).all(), (at, t, (error[t] / (size[t] + size[t - 1])).max().item())
