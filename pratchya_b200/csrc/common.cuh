@@ -25,10 +25,14 @@ int fail(int status, const char* fmt, ...);
       return ::pb::fail(PB_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(_e)); \
   } while (0)
 
-// Launched behind the kernel before it on the stream: the grid is set up while that one's last CTAs finish, and its threads go on past
-// grid_wait(), which every kernel launched this way begins with, when all of that one's memory operations have been performed.
-template <typename... Params, typename... Args>
-cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+template <typename T> struct As { using type = T; };      // a parameter that no type is deduced from
+// Launched behind the kernel before it on the stream: the launch is under way while that one's last stores are, and the grid's threads go
+// on past grid_wait(), which every kernel launched this way begins with, when all of that one's memory operations have been performed.  (No
+// kernel here lets the next one in early: a grid's CTAs start when the last one of the grid before it has ended.)  Memory that a
+// kernel reads as const __restrict__ or by __ldg is therefore written by nobody between its first read and its end.
+// Arguments convert to the kernel's parameters as in a call: no pointer to another type, no dropped const.
+template <typename... Params>
+cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, typename As<Params>::type... args) {
   cudaLaunchConfig_t config{};
   config.gridDim = grid; config.blockDim = block; config.dynamicSmemBytes = smem; config.stream = st;
   cudaLaunchAttribute behind;
@@ -36,7 +40,7 @@ cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, dim3 block, size
   behind.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &behind;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+  return cudaLaunchKernelEx(&config, kernel, args...);
 }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
