@@ -6,11 +6,12 @@
 //
 // One operand is exact in bf16 as it is, the other is kept as three bf16 terms, hi + mid + lo, which hold all 24 bits of an f32:
 //   g in bf16:  g as it is; the dequantized values (the one f32 rounding that dequantizing makes) as three terms.  Any grid.  For dX with
-//               a super-group's factor that belongs to rows of Q (out's columns) the fp8 values times their block's power of two, one term:
-//               that factor goes to the finished sum, and every product is one tensor-core product.
+//               a super-group's factor that belongs to rows of Q (out's columns) the fp8 values times their block's power of two and the factor's,
+//               one term: the rest of that factor, a number in [1, 2), goes to the finished sum, and every product is one tensor-core product.
 //   g in f32:   the fp8 values times their block's power of two (exact; where it is not, a NaN, see below); g as three terms, times
 //               the super-group's f32 factor where that varies along c (tokens == 1, one set of terms per 1024 columns of
-//               Q; one f32 rounding), while a factor that belongs to a column of dX goes to the finished sum.
+//               Q; one f32 rounding), while of a factor that belongs to a column of dX the power of two goes to Q's values and the rest to the finished sum
+//               (all of it there, and rows 2^-60 and less of a large super-group leave f32's range before the sum is scaled back).
 // Every f32 product is then exact in its tensor-core products, and the accumulator is emptied into f32 registers every 64 of c
 // (the tensor core's own additions do not round to nearest; dense_dot.cu empties every 32): the low terms of all 64 go first, so that
 // four additions meet a sum of full size, as many as there, and half as many f32 additions follow.  Contractions of a few hundred have
@@ -50,6 +51,7 @@ constexpr int kDrainWarps = 8;
 constexpr int kThreads = 64 + 32 * kDrainWarps;
 constexpr uint32_t kWaitPolls = 1u << 21;               // a poll parks for up to 2 us: about four seconds at most
 constexpr float kScaleUp = 0x1p40f, kScaleDown = 0x1p-40f;
+constexpr float kQScaleUp = 0x1p10f;  // of it, Q's share where g is f32 and Q's values hold their super-group's power of two
 constexpr size_t kMaxTerms = (size_t)512 << 20;         // bytes of three-term operand at a time: more of it takes several rounds (1024 of its rows at least)
 
 constexpr int kOutCols = 16;           // of a finished tile that a thread stores at a time
@@ -78,7 +80,7 @@ struct DotSource {
 struct SplitParams {
   DotSource src;
   float* out;                         // or the parts, [splits][out]
-  const float* factor;                // tokens == 0, one factor per 128 of i for the finished sums (sc32): of the tile's columns with f32 g, of its rows with one term
+  const float* factor;                // tokens == 0, one factor per 128 of i (sc32), whose rest the finished sums take: of the tile's columns with f32 g, of its rows with one term
   int64_t ld, part;                   // row stride of out, elements of a part
   int rows, cols;                     // extents of the three-term operand and of the other
   int row_first;                      // the first of these rows, for the sums that are made again
@@ -170,8 +172,17 @@ struct PrepareParams {
   int variants;                       // tokens == 1: sets of terms of g, K blocks of a row of Q each
 };
 
-// sixteen values of Q from their bytes: terms of the dequantized values (TERMS), or value times its block's power of two (times `up`)
-template <bool TERMS>
+// A super-group's factor as a power of two and what is left of it, in [1, 2) (below for a subnormal one).  An infinite one is left to the
+// power, and the sums that meet it are made again.
+__device__ __forceinline__ float power_of(float f) { return __uint_as_float(max(__float_as_uint(f) & 0x7f800000u, 0x00800000u)); }
+__device__ __forceinline__ float rest_of(float f) {
+  const uint32_t bits = __float_as_uint(f);
+  return bits & 0x7f800000u ? __uint_as_float((bits & 0x807fffffu) | 0x3f800000u) : f * 0x1p126f;
+}
+
+// sixteen values of Q from their bytes: terms of the dequantized values (TERMS), or value times its block's power of two, and with POWER
+// (the finished sums take the rest of the super-group's factor) times that one's and `up`
+template <bool TERMS, bool POWER>
 __device__ __forceinline__ void prepare_q(const PrepareParams& p, uint32_t v, float up) {
   const uint32_t in_row = p.q_vecs.div(v), row = p.q_row0 + in_row, col = p.q_col0 + (v - in_row * p.q_vecs.d) * 16;
   const uint4 bytes = __ldg(reinterpret_cast<const uint4*>(p.q + (int64_t)row * p.ldq + col));
@@ -179,7 +190,9 @@ __device__ __forceinline__ void prepare_q(const PrepareParams& p, uint32_t v, fl
   const uint32_t id0 = (row >> p.log2_a) * p.nbc + (col >> p.log2_b);
   auto multiplier = [&](uint32_t id) {
     const float two = e8m0_to_f32(__ldg(p.sc8 + id));
-    return TERMS ? __fmul_rn(__fmul_rn(two, __ldg(p.sc32 + (id >> p.log2_K))), kScaleUp * 0.0078125f) : two * up;
+    if (!TERMS && !POWER) return two;
+    const float group = __ldg(p.sc32 + (id >> p.log2_K));
+    return TERMS ? __fmul_rn(__fmul_rn(two, group), kScaleUp * 0.0078125f) : two * (up * 0.0078125f) * power_of(group);
   };
   const float m0 = multiplier(id0);
   uint32_t hi[8], mid[8], lo[8];
@@ -211,7 +224,7 @@ __device__ __forceinline__ void prepare_g(const PrepareParams& p, uint32_t v) {
   const float4 a = __ldg(src), b = __ldg(src + 1);
   const float2 x[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)};
   for (int set = 0; set < (TOKENS ? p.variants : 1); ++set) {
-    const float m = TOKENS ? __fmul_rn(__ldg(p.sc32 + ((row * p.nbc) >> p.log2_K) + set), kScaleUp * 0.0078125f) : kScaleUp;
+    const float m = TOKENS ? __fmul_rn(__ldg(p.sc32 + ((row * p.nbc) >> p.log2_K) + set), kScaleUp * 0.0078125f) : kScaleUp / kQScaleUp;
     uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) split3(__fmul2_rn(x[e], make_float2(m, m)), hi[e], mid[e], lo[e]);
@@ -228,7 +241,7 @@ __global__ void __launch_bounds__(256) split_prepare_kernel(const __grid_constan
   grid_wait();
   if (blockIdx.x < p.q_blocks) {
     const uint32_t v = blockIdx.x * 256 + threadIdx.x;
-    if (v < p.n_q) prepare_q<!G32 && TERMS == 3>(p, v, G32 ? 1.0f : kScaleUp);
+    if (v < p.n_q) prepare_q<!G32 && TERMS == 3, !TOKENS>(p, v, G32 ? kQScaleUp : kScaleUp);
   } else if (G32) {
     const uint32_t v = (blockIdx.x - p.q_blocks) * 256 + threadIdx.x;
     if (v < p.n_g) prepare_g<TOKENS>(p, v);
@@ -281,7 +294,7 @@ __device__ __noinline__ void remake_sums(const SplitParams& p, float* out, int r
 }
 
 // N columns per tile; TOKENS: c is the operands' outer dimension; G32: the terms are g's (rows are j, columns i), else Q's (rows i, columns j);
-// TERMS: 3, or 1 where Q's exact values are multiplied and its super-group's factor goes to the finished sums.
+// TERMS: 3, or 1 where Q's exact values are multiplied and the rest of their super-group's factor goes to the finished sums.
 template <int N, bool TOKENS, bool G32, int TERMS>
 __global__ void __launch_bounds__(kThreads, 1)
 split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_constant__ CUtensorMap map_other, const __grid_constant__ SplitParams p) {
@@ -435,19 +448,17 @@ split_dot_kernel(const __grid_constant__ CUtensorMap map_terms, const __grid_con
       float* out = p.out + (int64_t)split * p.part;
       constexpr bool kFactor = TERMS == 1 || (!TOKENS && G32);
       float row_factor = 1.0f;
-      if (TERMS == 1) row_factor = __ldg(p.factor + (((uint32_t)(p.row_first + row0) / 128 * p.src.nbc) >> p.src.log2_K));
+      if (TERMS == 1) row_factor = rest_of(__ldg(p.factor + (((uint32_t)(p.row_first + row0) / 128 * p.src.nbc) >> p.src.log2_K)));
       float2 zero = make_float2(0.0f, 0.0f);    // times 0: NaN where a sum is not finite
 #pragma unroll
       for (int k = 0; k < kCols / kOutCols; ++k) {
         const int c0 = cb + k * kOutCols;
         if (c0 >= p.cols) break;
-        const float f = TERMS == 1 ? row_factor : (kFactor ? __ldg(p.factor + (((uint32_t)c0 / 128 * p.src.nbc) >> p.src.log2_K)) : 1.0f);
-        const float big = kFactor ? (f >= 1.0f ? f * (kScaleDown * 0.0078125f) : kScaleDown * 0.0078125f) : kScaleDown, small = f >= 1.0f ? 1.0f : f;
+        const float down = kScaleDown * (TERMS == 1 ? row_factor : (kFactor ? rest_of(__ldg(p.factor + (((uint32_t)c0 / 128 * p.src.nbc) >> p.src.log2_K))) : 1.0f));
 #pragma unroll
         for (int n = kOutCols * k; n < kOutCols * (k + 1); n += 2) {
           zero = __ffma2_rn(make_float2(acc[n], acc[n + 1]), make_float2(0.0f, 0.0f), zero);
-          float2 v = __fmul2_rn(make_float2(acc[n], acc[n + 1]), make_float2(big, big));
-          if (kFactor) v = __fmul2_rn(v, make_float2(small, small));
+          const float2 v = __fmul2_rn(make_float2(acc[n], acc[n + 1]), make_float2(down, down));
           acc[n] = v.x; acc[n + 1] = v.y;
         }
         const float* v = acc + kOutCols * k;

@@ -229,3 +229,19 @@ def test_one_term_for_a_bf16_cotangent(built_lib, rows, cols, free, amp):
         assert (got.double() - want).norm() <= (plain.double() - want).norm() * 1.02
     assert torch.equal(got, _dot(built_lib, 0, triple, (128, 128), g)[0])
     assert built_lib.pb_gemm_check(torch.cuda.current_stream().cuda_stream) == 0
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("power", [60, 100, -60])
+def test_rows_far_below_a_large_super_group(built_lib, dtype, power):
+    """dX of a weight whose super-group's largest value is 2^power, with rows of size one in it, and a cotangent of 2^-power: the sums of
+    those rows are as far from f32's ends as an f32 dot's."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn(1024, 1024, generator=g, device="cuda") * 2.0 ** power
+    x[256:384] = torch.randn(128, 1024, generator=g, device="cuda") * 2.0 ** min(power, 0)
+    triple = quantize_impl(x, (128, 128))
+    cot = (torch.randn(600, 1024, generator=g, device="cuda") * 2.0 ** -power).to(dtype)
+    got, shared = _dot(built_lib, 0, triple, (128, 128), cot)
+    assert shared
+    a, b = _sums(0, triple, (128, 128), cot)
+    assert ((got.double() - a @ b).abs() <= _bound(a, b)).all()
