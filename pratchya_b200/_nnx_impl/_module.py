@@ -246,9 +246,10 @@ class _LinearFn(torch.autograd.Function):
         xt = None
         if ctx.have_xt:
             xt, pos = saved[6:9], 9
-        if a == 128 and ctx.w_dtype is torch.float32 and (xt is not None or not _ops._LITERAL_DOT_TF32):
+        fmt = _ops._FMT_CODE.get(ctx.grad_format)        # read where dY is quantized only
+        if a == 128 and ctx.w_dtype is torch.float32 and (fmt is not None if xt is not None else not _ops._LITERAL_DOT_TF32):
             out = _lib.native().linear_backward(g_y, *xq, *wq, *(xt or (None, None, None)), *(saved[pos:pos + 2] if ctx.fake else (None, None)), b,
-                                                _ops._FMT_CODE[ctx.grad_format], ctx.x_dtype)
+                                                fmt if fmt is not None else 0, ctx.x_dtype)
             if out is not None:
                 return out[0].reshape(ctx.x_shape), out[1], None, None, None, None, None, None, None
         g = g_y.reshape(-1, g_y.shape[-1]).contiguous()

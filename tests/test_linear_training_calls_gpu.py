@@ -67,3 +67,14 @@ def test_training_step_in_two_calls_gives_the_bits_of_its_ops(built_lib, monkeyp
     finally:
         _ops.set_literal_dot_precision("f32")
     assert _same(mine, text), (mine, text)
+
+
+@pytest.mark.parametrize("grid,n,fake", [((128, 128), 512, True), ((128, 1), 48, False)])
+def test_a_gradient_format_that_nothing_is_stored_in_is_not_asked_for(built_lib, grid, n, fake):
+    """The literal dots store no gradient in fp8: what `grad_format` says is not read there, and refused where it is."""
+    x, w = torch.randn(64, 1024, device="cuda", requires_grad=True), (torch.randn(1024, n, device="cuda") * 0.02).requires_grad_(True)
+    step = lambda x, fmt: torch.autograd.grad(_module.linear_fp8(x, w, grid, fake_quant_output=fake, grad_format=fmt).sum(), (x, w))
+    assert all(torch.equal(a, b) for a, b in zip(step(x, "none"), step(x, "e4m3")))
+    if grid == (128, 128):
+        with pytest.raises(KeyError):
+            step(torch.randn(1024, 1024, device="cuda", requires_grad=True), "none")
