@@ -462,8 +462,9 @@ int product(const Triple& a, const Triple& b, int b_height, int b_transposed, at
   at::Tensor ws = scratch(bytes ? bytes : 1, a.q);
   return without_gil([&] { return pb_gemm_tn(&oa, &ob, d->data_ptr(), PB_F32, cols, ws.data_ptr(), bytes, st); });
 }
-int literal_dot(int tokens, const Triple& t, int a, int b, const at::Tensor& g, int64_t g_rows, int64_t g_cols, at::Tensor* out, void* st) {
-  const int64_t rows = t.q.size(0), cols = t.q.size(1), free = tokens ? g_cols : g_rows;
+// _dense_dot; free: g's extent that is not summed over
+int literal_dot(int tokens, const Triple& t, int a, int b, const at::Tensor& g, int64_t free, at::Tensor* out, void* st) {
+  const int64_t rows = t.q.size(0), cols = t.q.size(1);
   const int type = code(g.scalar_type());
   *out = tokens ? empty({cols, free}, at::kFloat, g) : empty({free, rows}, at::kFloat, g);
   at::Tensor ws;
@@ -572,8 +573,8 @@ OP(linear_backward) {
       RUN(pb_dequantize_bwd(g.data_ptr(), code(g.scalar_type()), (const uint8_t*)in[10]->data_ptr(), (const float*)in[11]->data_ptr(), 1, rows, cols, 1, 128, scaled.data_ptr(), st));
       g = scaled;
     }
-    if ((status = literal_dot(0, {wq, *in[5], *in[6]}, 128, b, g, rows, cols, &gx, st)) != PB_OK ||
-        (status = literal_dot(1, {xq, *in[2], *in[3]}, 1, 128, g, rows, cols, &gw, st)) != PB_OK)
+    if ((status = literal_dot(0, {wq, *in[5], *in[6]}, 128, b, g, rows, &gx, st)) != PB_OK ||
+        (status = literal_dot(1, {xq, *in[2], *in[3]}, 1, 128, g, cols, &gw, st)) != PB_OK)
       return raise_status(status);
   }
   at::Tensor dx = empty({rows, depth}, x_type, xq);
@@ -627,21 +628,9 @@ OP(dense_dot) {
   if (!q || !sc8 || !sc32 || !g || watched() || q->dim() != 2 || g->dim() != 2 || !dense(g->scalar_type()) || q->scalar_type() != kE4M3 ||
       g->size(tokens ? 0 : 1) != q->size(tokens ? 0 : 1))
     return none();
-  const int64_t rows = q->size(0), cols = q->size(1), free = g->size(tokens ? 1 : 0);
-  const int type = code(g->scalar_type());
   const c10::cuda::CUDAGuard guard(g->device());
-  at::Tensor out = tokens ? empty({cols, free}, at::kFloat, *g) : empty({free, rows}, at::kFloat, *g), ws;
-  size_t bytes = pb_dense_dot_workspace_best(tokens, rows, cols, a, b, free, type);
-  try {
-    if (bytes) ws = scratch(bytes, *g);
-  } catch (const c10::OutOfMemoryError&) {      // the form that takes less of it
-    const size_t least = pb_dense_dot_workspace_size(tokens, rows, cols, a, b, free);
-    if (least == bytes) throw;
-    bytes = least;
-    if (bytes) ws = scratch(bytes, *g);
-  }
-  RUN(pb_dense_dot(tokens, (const uint8_t*)q->data_ptr(), (const uint8_t*)sc8->data_ptr(), (const float*)sc32->data_ptr(), rows, cols, a, b, g->data_ptr(), type, free,
-                   (float*)out.data_ptr(), bytes ? ws.data_ptr() : nullptr, bytes, current_stream(g->device())));
+  at::Tensor out;
+  if (const int status = literal_dot(tokens, {*q, *sc8, *sc32}, a, b, *g, g->size(tokens ? 1 : 0), &out, current_stream(g->device()))) return raise_status(status);
   return wrap(out);
   END_HANDLE_TH_ERRORS
 }
