@@ -78,3 +78,73 @@ def test_a_gradient_format_that_nothing_is_stored_in_is_not_asked_for(built_lib,
     if grid == (128, 128):
         with pytest.raises(KeyError):
             step(torch.randn(1024, 1024, device="cuda", requires_grad=True), "none")
+
+
+class _Counting:
+    """The extension, with what its two calls were asked and answered."""
+    def __init__(self, native):
+        self.native, self.taken, self.left = native, [], []
+
+    def __getattr__(self, name):
+        call = getattr(self.native, name)
+        if name not in ("linear_forward", "linear_backward"):
+            return call
+
+        def counted(*args):
+            out = call(*args)
+            (self.left if out is None else self.taken).append(name)
+            return out
+        return counted
+
+
+def _training_step(x, w, grid, fake, **options):
+    y = _module.linear_fp8(x, w, grid, fake_quant_output=fake, **options)
+    return (y.detach(), *torch.autograd.grad(y, (x, w), torch.ones_like(y) * 1e-3))
+
+
+BOTH = ["linear_forward", "linear_backward"]
+
+
+@pytest.mark.parametrize("rows,k,n,grid,fake,dtype,taken", [
+    (64, 1024, 512, (128, 128), True, torch.float32, BOTH), (1000, 512, 1024, (128, 128), True, torch.bfloat16, BOTH), (1024, 1024, 1024, (128, 128), True, torch.bfloat16, BOTH),
+    (1024, 512, 384, (128, 128), False, torch.float32, BOTH), (704, 128, 1024, (128, 1), False, torch.float32, BOTH), (7, 1024, 48, (128, 1), False, torch.float32, BOTH),
+    (5, 384, 128, (128, 128), True, torch.float32, []), (24, 256, 256, (64, 64), True, torch.float32, []), (64, 1024, 512, (128, 128), True, torch.float16, [])])
+def test_which_steps_the_calls_take(built_lib, monkeypatch, rows, k, n, grid, fake, dtype, taken):
+    counting = _Counting(_lib.native())
+    monkeypatch.setattr(_lib, "_native", counting)
+    x, w = torch.randn(rows, k, device="cuda").to(dtype).requires_grad_(True), (torch.randn(k, n, device="cuda") * 0.02).requires_grad_(True)
+    _training_step(x, w, grid, fake)
+    assert counting.taken == taken
+
+
+@pytest.mark.parametrize("rows,k,n,grid,fake,dtype", [(600, 1024, 1024, (128, 128), True, torch.bfloat16), (1024, 512, 1024, (128, 128), True, torch.float32), (704, 128, 1024, (128, 1), False, torch.float32)])
+def test_the_calls_under_hooks_on_another_stream_and_in_a_graph(built_lib, monkeypatch, rows, k, n, grid, fake, dtype):
+    counting = _Counting(_lib.native())
+    monkeypatch.setattr(_lib, "_native", counting)
+    xs = [torch.randn(rows, k, device="cuda").to(dtype).requires_grad_(True) for _ in range(3)]
+    w = (torch.randn(k, n, device="cuda") * 0.02).requires_grad_(True)
+    want = [_training_step(x, w, grid, fake) for x in xs]
+    packed = []
+
+    def pack(t):
+        packed.append(t)
+        return t.cpu()
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        got = _training_step(xs[0], w, grid, fake)
+    assert _same(got, want[0]) and len(packed) == (11 if fake and rows % 1024 == 0 else 8 if fake else 6)      # x's triple, the weight's, x^T's, the output's scales
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = [_training_step(x, w, grid, fake) for x in xs]
+    torch.cuda.current_stream().wait_stream(side)
+    assert all(_same(a, b) for a, b in zip(got, want))
+    static = xs[0].detach().clone().requires_grad_(True)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = _training_step(static, w, grid, fake)
+    for x, ref in zip(xs, want):
+        with torch.no_grad():
+            static.copy_(x)
+        graph.replay()
+        assert _same(out, ref)
+    assert not counting.left
