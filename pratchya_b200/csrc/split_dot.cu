@@ -544,18 +544,20 @@ int launch_prepare(const PrepareParams& p, cudaStream_t st) {
   return PB_OK;
 }
 
-// Where this form is the faster one.  What it makes ready has to be shared,
-// and its two launches and the passes over the operands want something to do.  us, dense_dot_kernel | this form, inside a graph:
-// dX, 2048 x 2048: f32 100 rows 14.9 | 15.8, 200 20.1 | 18.9, 3000 142 | 84; bf16 300 rows 23.8 | 23.0, 500 30.6 | 27.4, 3000 141 | 75;
-// 1024 x 1024, bf16: 500 rows 14.4 | 14.6, 700 16.9 | 16.2; 2048 x 128, bf16: 1000 rows 9.3 | 10.3.
-// dW, 1024 x 1024: 64 rows 8.3 | 8.7, 200 13.5 | 10.8, 3000 52 | 33; 2048 x 2048: 64 rows 15.0 | 13.5, 3000 178 | 68; f32 174 | 79;
-// 4096 x 512: 100 rows 10.1 | 10.6, 200 14.2 | 12.1.  Operands that one tile uses: 8192 rows, 2048 x 128, f32 35.5 | 32.5, bf16
-// 36.6 | 42.8; 128 x 2048, f32 35.6 | 48.4.
-// One term (a bf16 cotangent's dX): 2048 x 2048 64 rows 12.5 | 12.7, 150 rows 16.6 | 14.5, 1000 rows 39 | 22; 4096 x 1024 100 rows 12.3 | 12.5, 1000 rows
-// 41 | 18; 1024 x 1024 64 rows 11.5 | 10.4; 128 x 2048 64 rows 11.1 | 9.7; 8192 x 2048 64 rows 24.4 | 23.4, 2000 rows 275 | 86.
+// Where this form is taken.  What it makes ready has to be shared, and its two launches and the passes over the operands want something to do.
+// us, dense_dot_kernel | this form, inside a graph:
+// One term (a bf16 cotangent's dX), everywhere: 128 x 128 8 rows 7.1 | 5.3, 8000 6.9 | 7.0; 512 x 128 500 rows 6.8 | 6.9; 2048 x 2048 8 rows 11.6 | 10.3,
+// 64 11.4 | 10.5, 128 11.3 | 11.3, 1000 37.5 | 19.8, 3000 104 | 34; 1024 x 4096 128 rows 11.8 | 12.2; 8192 x 2048 8 rows 22.5 | 20.4, 64 22.9 | 20.4, 2000 274 | 80.
+// f32 dX, 2048 x 2048: 100 rows 12.0 | 14.2, 200 16.3 | 17.6, 500 25.1 | 24.6, 1000 39.6 | 35.6, 3000 110 | 83; 1024 x 1024: 500 rows 11.9 | 13.7, 3000 41 | 28;
+// 2048 x 128: 2000 rows 10.6 | 15.7, 8000 25.4 | 34.0; 128 x 2048: 8000 rows 26 | 48.
+// dW, 2048 x 2048, f32: 64 rows 8.9 | 9.8, 200 15.0 | 13.4, 3000 100 | 77, bf16: 64 rows 9.0 | 13.5, 200 14.9 | 16.3, 300 17.2 | 18.0, 500 23.4 | 21.7,
+// 3000 110 | 67; 1024 x 1024, bf16: 200 rows 9.3 | 11.0, 500 13.9 | 13.1, 8000 77 | 67; 4096 x 512, f32: 500 rows 13.6 | 15.1, 16000 323 | 267; 2048 x 128,
+// f32: 8000 rows 21.6 | 29.6.
+// The lines of the last two have sizes on this form's side that take it up to half as long again, next to them: it is the more precise of the
+// two (the errors above), and no size's sums are to become less precise for it.
 bool split_dot_pays(int tokens, bool exact, int64_t I, int64_t J, int64_t C) {
   const double products = (double)I * (double)J * (double)C;
-  if (exact) return J > 128 || I * C <= (1ll << 21);
+  if (exact) return true;
   if (I < 512 || J < 512) return false;
   if (tokens) return C >= 192 || products >= 0x1p28;
   return products >= 0x1p29 && J >= 192;

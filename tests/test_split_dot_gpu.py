@@ -245,3 +245,15 @@ def test_rows_far_below_a_large_super_group(built_lib, dtype, power):
     assert shared
     a, b = _sums(0, triple, (128, 128), cot)
     assert ((got.double() - a @ b).abs() <= _bound(a, b)).all()
+
+
+@pytest.mark.parametrize("rows,cols,free", [(2048, 2048, 8), (4096, 1024, 64), (8192, 2048, 1), (8192, 2048, 100), (8192, 2048, 128)])
+def test_one_term_for_few_rows_of_a_large_weight(built_lib, rows, cols, free):
+    """The faster form there, and the more precise one."""
+    triple, g = _inputs(rows, cols, (128, 128), free, 0, BF16)
+    got, shared = _dot(built_lib, 0, triple, (128, 128), g)
+    assert shared
+    a, b = _sums(0, triple, (128, 128), g)
+    want = a @ b
+    assert ((got.double() - want).abs() <= _bound(a, b)).all()
+    assert (got.double() - want).norm() <= (_dot(built_lib, 0, triple, (128, 128), g, best=False)[0].double() - want).norm() * 1.02
