@@ -29,8 +29,8 @@
 // (f32 dW of 300 tokens, 2048 x 4096: 30.5 -> 26.6).
 //
 // Element-wise kernel: bound by its bytes.  Main kernel: persistent, one CTA per SM; a tile is 128 rows of the three-term operand
-// by N of the other; a stage is 32 of c of both, by TMA, K-major (64-byte swizzle) for tokens == 0 and with c outermost, as
-// it lies in memory, for tokens == 1 (128-byte swizzle): no transpose anywhere.  Warp 0 loads, warp 1 issues six (four)
+// by N of the other; a stage is 32 of c of both (64 with one term), by TMA, K-major (64-byte swizzle, 128 with one term) for tokens == 0 and with c
+// outermost, as it lies in memory, for tokens == 1 (128-byte swizzle): no transpose anywhere.  Warp 0 loads, warp 1 issues six (four)
 // tcgen05.mma a stage, eight warps empty one accumulator while the other fills.  N is 256, 192 or 128, whichever fills whole waves of SMs best.
 #include <cuda.h>
 

@@ -1,5 +1,5 @@
-"""The scan's two forward layouts (16 rows of a head per CTA for few heads, a whole head for many) and the backward kernel's half
-chunks, over lengths around the chunk of eight, against the recurrence in 64 bits."""
+"""The scan's forward layouts (16 or 32 rows of a head per CTA for few heads, halves of a head around one wave of them, a whole head for many)
+and the backward kernel's half chunks, over lengths around the chunk of eight, against the recurrence in 64 bits."""
 import pytest
 import torch
 
